@@ -4,9 +4,9 @@
 //       SFCPartitioner::do_partition (dynamis_state/src/csrc/partition/sfc_partitioner.cpp:166-176)
 //   dynb_halo_mark_from_edges                per-edge pass of extract_halo_info
 //       (dynamis_state/src/csrc/graph/dist_graph_ops_kernels.cu:46-59, 104-188)
-//   dynb_csr_plan / dynb_csr_fill            send / recv CSR of build_halo_maps
-//       (dynamis_state/src/csrc/build_halo_maps.cpp:60-125) and of extract_halo_info, from a
-//       per-atom rank bit mask instead of the reference's [N, W] bool matrix + nonzero + argsort
+//   dynb_halo_lists_plan / _fill             send and recv CSR of build_halo_maps
+//       (dynamis_state/src/csrc/build_halo_maps.cpp:60-125) and of extract_halo_info, from
+//       per-atom rank bit masks instead of the reference's [N, W] bool matrix + nonzero + argsort
 //   dynb_filter_edges_plan / _fill           filter_edges_to_radius
 //       (dist_graph_ops_kernels.cu:16-43, 62-102)
 //
@@ -43,19 +43,66 @@ bincount_i64_kernel(const int64_t* __restrict__ a, int64_t n, int64_t W, unsigne
     }
 }
 
+// Stream compaction in two launches: matches per tile, then every block adds up the tiles in front of its own (a few
+// thousand values out of L2 at most) and writes its matches.  A warp owns 256 consecutive values, so that the order is
+// kept by ballots alone.
+constexpr int SELECT_TILE = 2048;
+
 __global__ void __launch_bounds__(256)
-flag_eq_i64_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, uint32_t* __restrict__ flags)
+select_count_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, uint32_t* __restrict__ tile_count)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) flags[i] = (a[i] == value) ? 1u : 0u;
+    __shared__ uint32_t wsum[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * SELECT_TILE + warp * 256 + lane;
+    int64_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = (base + 32 * k < n) ? a[base + 32 * k] : ~value;
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) c += (v[k] == value) ? 1u : 0u;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) wsum[warp] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t s = 0;
+        for (int w = 0; w < 8; w++) s += wsum[w];
+        tile_count[blockIdx.x] = s;
+    }
 }
 
 __global__ void __launch_bounds__(256)
-scatter_selected_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, const uint32_t* __restrict__ excl,
-                        const int64_t* __restrict__ gather_src, int64_t* __restrict__ out)
+select_fill_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, const uint32_t* __restrict__ tile_count,
+                   const int64_t* __restrict__ gather_src, int64_t* __restrict__ out, int64_t* __restrict__ count_out)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && a[i] == value) out[excl[i]] = gather_src ? gather_src[i] : i;
+    __shared__ uint32_t wsum[8], before[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * SELECT_TILE + warp * 256 + lane;
+    int64_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = (base + 32 * k < n) ? a[base + 32 * k] : ~value;
+    uint32_t s = 0;
+    for (int i = threadIdx.x; i < (int)blockIdx.x; i += 256) s += tile_count[i];
+    s = __reduce_add_sync(0xffffffffu, s);
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) c += (v[k] == value) ? 1u : 0u;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) { before[warp] = s; wsum[warp] = c; }
+    __syncthreads();
+    uint32_t at = 0;
+    for (int w = 0; w < 8; w++) at += before[w];
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count_out = (int64_t)at + tile_count[blockIdx.x];
+    for (int w = 0; w < warp; w++) at += wsum[w];
+    const uint32_t lt = lanemask_lt();
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const uint32_t m = __ballot_sync(0xffffffffu, v[k] == value);
+        if (v[k] == value) {
+            const int64_t i = base + 32 * k;
+            out[at + __popc(m & lt)] = gather_src ? gather_src[i] : i;
+        }
+        at += __popc(m);
+    }
 }
 
 __global__ void u32_total_to_i64_kernel(const uint32_t* t, int64_t* out) { *out = (int64_t)(*t); }
@@ -85,99 +132,221 @@ halo_mark_edges_kernel(const int64_t* __restrict__ src, const int64_t* __restric
     has_remote[d] = 1;
 }
 
-// ------------------------------------------------------------------------------------------ CSR assembly
-// Element a in [0, n) carries a set of peer ranks.  For each peer p, the output segment p lists the
-// elements whose set contains p, ascending in a.  Modes define the set:
-enum { CSR_SEND = 0, CSR_RECV = 1, CSR_RAW = 2 };
-//   CSR_SEND  owner[a] == R ? bits of mask[a] without R : {}        (needed_by rows of my atoms)
-//   CSR_RECV  owner[a] != R and bit R of mask[a] ? {owner[a]} : {}   (foreign atoms I need)
-//   CSR_RAW   bits of mask[a]
-constexpr int CSR_THREADS = 256;
-constexpr int CSR_WARPS = CSR_THREADS / 32;
+// ------------------------------------------------------------------------------------------ halo lists
+// Atom a in [0, n) carries two sets of peer ranks, S(a) and R(a).  Send segment p lists the atoms with p in S(a), recv
+// segment p those with p in R(a), each ascending in a.  Either the sets are given as bit masks (extract_halo_info), or
+// they follow from one "needed by" mask and the owners (build_halo_maps):
+//   S(a) = owner[a] == me ? ranks that need a, without me : {}
+//   R(a) = owner[a] != me and I need a ? {owner[a]} : {}
+// and the own atoms themselves (owner[a] == me, ascending) give the local indices.
+//
+// Both lists, the local indices and the interior mask come out of one counting and one writing pass over the masks; most
+// atoms have empty sets, so a warp (128 consecutive atoms, 32 at a time) works on the peers that occur and on no others.
+// One million atoms, 8 ranks: 8 + 6 + 9 us (count, row scan, fill), where per-list passes that walked all peers took 120.
+constexpr int HL_THREADS = 256;
+constexpr int HL_WARPS = HL_THREADS / 32;
+constexpr int HL_ROUNDS = 4;
+constexpr int HL_TILE = HL_THREADS * HL_ROUNDS;
 
-__device__ __forceinline__ bool csr_has(const uint32_t* __restrict__ mask, int words, const int64_t* __restrict__ owner,
-                                        int64_t a, int64_t R, int mode, int p)
-{
-    if (mode == CSR_RAW) return (mask[a * words + (p >> 5)] >> (p & 31)) & 1u;
-    const int64_t o = owner[a];
-    if (mode == CSR_SEND) return o == R && p != R && ((mask[a * words + (p >> 5)] >> (p & 31)) & 1u);
-    return o != R && o == p && ((mask[a * words + (R >> 5)] >> (R & 31)) & 1u);
-}
+struct HaloSets {
+    const uint32_t* send_mask;   // masks of S(a), or of "needed by" when owner != nullptr
+    const uint32_t* recv_mask;   // masks of R(a); not read when owner != nullptr
+    const int64_t* owner;
+    int64_t n, me;
+    int words;
+};
 
-// bsum[p * nblocks + block] = number of elements of this block whose set contains p
-__global__ void __launch_bounds__(CSR_THREADS)
-csr_count_kernel(const uint32_t* __restrict__ mask, int words, const int64_t* __restrict__ owner, int64_t n, int64_t R,
-                 int mode, int W, int nblocks, uint32_t* __restrict__ bsum)
+__device__ __forceinline__ void halo_sets(const HaloSets& h, int64_t a, int word, uint32_t& s, uint32_t& r, bool& own)
 {
-    __shared__ uint32_t wsum[CSR_WARPS];
-    const int64_t a = (int64_t)blockIdx.x * CSR_THREADS + threadIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int p = 0; p < W; p++) {
-        const bool f = (a < n) && csr_has(mask, words, owner, a, R, mode, p);
-        const uint32_t b = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) wsum[warp] = __popc(b);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t s = 0;
-            for (int w = 0; w < CSR_WARPS; w++) s += wsum[w];
-            bsum[(int64_t)p * nblocks + blockIdx.x] = s;
-        }
-        __syncthreads();
+    s = r = 0u;
+    own = false;
+    if (a >= h.n) return;
+    if (h.owner == nullptr) {
+        s = h.send_mask[a * h.words + word];
+        r = h.recv_mask[a * h.words + word];
+        return;
+    }
+    const int64_t o = h.owner[a];
+    own = o == h.me;
+    if (own) {
+        s = h.send_mask[a * h.words + word];
+        if (word == (int)(h.me >> 5)) s &= ~(1u << (h.me & 31));
+    } else if ((int)(o >> 5) == word && ((h.send_mask[a * h.words + (h.me >> 5)] >> (h.me & 31)) & 1u)) {
+        r = 1u << (o & 31);
     }
 }
 
-// One block per peer: exclusive scan of its row of block sums (in place) and the row total.
+// lane p of the warp adds up how many of the 32 sets contain p
+__device__ __forceinline__ uint32_t halo_count_sets(uint32_t set, int lane)
+{
+    uint32_t c = 0;
+    for (uint32_t any = __reduce_or_sync(0xffffffffu, set); any; any &= any - 1) {
+        const int p = __ffs((int)any) - 1;
+        const uint32_t m = __ballot_sync(0xffffffffu, (set >> p) & 1u);
+        if (lane == p) c = __popc(m);
+    }
+    return c;
+}
+
+// rows of bsum (nblocks entries each): send peers 0..W-1, recv peers 0..W-1, own atoms
+__global__ void __launch_bounds__(HL_THREADS)
+halo_lists_count_kernel(const HaloSets h, int W, int nblocks, uint32_t* __restrict__ bsum)
+{
+    __shared__ uint32_t ws[HL_WARPS][2][32];
+    __shared__ uint32_t wown[HL_WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * HL_TILE + warp * 32 * HL_ROUNDS + lane;
+    for (int word = 0; word < h.words; word++) {
+        uint32_t cs = 0, cr = 0, co = 0;
+#pragma unroll
+        for (int k = 0; k < HL_ROUNDS; k++) {
+            uint32_t s, r;
+            bool own;
+            halo_sets(h, base + 32 * k, word, s, r, own);
+            cs += halo_count_sets(s, lane);
+            cr += halo_count_sets(r, lane);
+            co += __popc(__ballot_sync(0xffffffffu, own));
+        }
+        __syncthreads();
+        ws[warp][0][lane] = cs;
+        ws[warp][1][lane] = cr;
+        if (lane == 0) wown[warp] = co;
+        __syncthreads();
+        if (threadIdx.x < 64) {
+            const int which = threadIdx.x >> 5, p = word * 32 + lane;
+            uint32_t t = 0;
+            for (int w = 0; w < HL_WARPS; w++) t += ws[w][which][lane];
+            if (p < W) bsum[(int64_t)(which * W + p) * nblocks + blockIdx.x] = t;
+        } else if (threadIdx.x == 64 && word == 0) {
+            uint32_t t = 0;
+            for (int w = 0; w < HL_WARPS; w++) t += wown[w];
+            bsum[(int64_t)(2 * W) * nblocks + blockIdx.x] = t;
+        }
+    }
+}
+
+// One block per row: exclusive scan of the row of block sums (in place) and its total; the block that finishes last turns
+// the totals into offsets [send W + 1 | recv W + 1 | number of own atoms].
 __global__ void __launch_bounds__(SCAN_THREADS)
-csr_scan_rows_kernel(uint32_t* __restrict__ bsum, int nblocks, int64_t* __restrict__ totals)
+halo_lists_scan_kernel(uint32_t* __restrict__ bsum, int nblocks, int W, int64_t* __restrict__ totals, uint32_t* __restrict__ arrived,
+                       int64_t* __restrict__ offsets)
 {
     __shared__ uint32_t warp_sums[SCAN_THREADS / 32];
+    __shared__ bool last;
     uint32_t* row = bsum + (int64_t)blockIdx.x * nblocks;
     uint32_t carry = 0;
-    for (int b0 = 0; b0 < nblocks; b0 += SCAN_THREADS) {
-        const int i = b0 + threadIdx.x;
-        const uint32_t v = (i < nblocks) ? row[i] : 0u;
+    for (int b0 = 0; b0 < nblocks; b0 += SCAN_THREADS * 4) {
+        const int i = b0 + threadIdx.x * 4;
+        uint32_t v[4], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) { v[k] = (i + k < nblocks) ? row[i + k] : 0u; sum += v[k]; }
         uint32_t tot;
-        const uint32_t ex = block_excl_scan<uint32_t>(v, &tot, warp_sums);
-        if (i < nblocks) row[i] = carry + ex;
+        uint32_t run = carry + block_excl_scan<uint32_t>(sum, &tot, warp_sums);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (i + k < nblocks) row[i + k] = run;
+            run += v[k];
+        }
         carry += tot;
     }
-    if (threadIdx.x == 0) totals[blockIdx.x] = (int64_t)carry;
-}
-
-__global__ void csr_offsets_kernel(const int64_t* __restrict__ totals, int W, int64_t* __restrict__ offsets)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int64_t run = 0;
-        for (int p = 0; p < W; p++) { offsets[p] = run; run += totals[p]; }
-        offsets[W] = run;
+    if (threadIdx.x == 0) {
+        totals[blockIdx.x] = (int64_t)carry;
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
     }
+    __syncthreads();
+    if (!last || threadIdx.x != 0) return;
+    __threadfence();
+    for (int which = 0; which < 2; which++) {
+        int64_t run = 0;
+        for (int p = 0; p < W; p++) {
+            offsets[which * (W + 1) + p] = run;
+            run += __ldcg(reinterpret_cast<const long long*>(totals) + which * W + p);
+        }
+        offsets[which * (W + 1) + W] = run;
+    }
+    offsets[2 * (W + 1)] = __ldcg(reinterpret_cast<const long long*>(totals) + 2 * W);
 }
 
-__global__ void __launch_bounds__(CSR_THREADS)
-csr_fill_kernel(const uint32_t* __restrict__ mask, int words, const int64_t* __restrict__ owner, int64_t n, int64_t R,
-                int mode, int W, int nblocks, const uint32_t* __restrict__ bsum, const int64_t* __restrict__ offsets,
-                const int64_t* __restrict__ value_map, int64_t* __restrict__ out)
+struct HaloListsOut {
+    const int64_t* value_map;    // send list entry of atom a when the owners are not given (global -> local)
+    const uint8_t* has_foreign;  // by atom; with the owners given
+    int64_t* send_local;
+    int64_t* recv_atom;
+    int64_t* recv_ghost;
+    uint8_t* interior;           // by local index; with the owners given
+    int64_t n_local;
+};
+
+__global__ void __launch_bounds__(HL_THREADS)
+halo_lists_fill_kernel(const HaloSets h, int W, int nblocks, const uint32_t* __restrict__ bsum, const int64_t* __restrict__ offsets,
+                       const HaloListsOut out)
 {
-    __shared__ uint32_t wsum[CSR_WARPS];
-    const int64_t a = (int64_t)blockIdx.x * CSR_THREADS + threadIdx.x;
+    __shared__ uint32_t ws[HL_WARPS][2][32];
+    __shared__ uint32_t wown[HL_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = lanemask_lt();
-    for (int p = 0; p < W; p++) {
-        const bool f = (a < n) && csr_has(mask, words, owner, a, R, mode, p);
-        const uint32_t b = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) wsum[warp] = __popc(b);
+    const int64_t base = (int64_t)blockIdx.x * HL_TILE + warp * 32 * HL_ROUNDS + lane;
+    for (int word = 0; word < h.words; word++) {
+        uint32_t set[2][HL_ROUNDS], own[HL_ROUNDS], c[2] = {0u, 0u}, co = 0;
+#pragma unroll
+        for (int k = 0; k < HL_ROUNDS; k++) {
+            bool o;
+            halo_sets(h, base + 32 * k, word, set[0][k], set[1][k], o);
+            own[k] = __ballot_sync(0xffffffffu, o);
+            c[0] += halo_count_sets(set[0][k], lane);
+            c[1] += halo_count_sets(set[1][k], lane);
+            co += __popc(own[k]);
+        }
         __syncthreads();
-        if (f) {
-            uint32_t before = 0;
-            for (int w = 0; w < warp; w++) before += wsum[w];
-            const int64_t pos = offsets[p] + bsum[(int64_t)p * nblocks + blockIdx.x] + before + __popc(b & lt);
-            out[pos] = value_map ? value_map[a] : a;
+        ws[warp][0][lane] = c[0];
+        ws[warp][1][lane] = c[1];
+        if (lane == 0) wown[warp] = co;
+        __syncthreads();
+        // lane p: place of this warp's first entry in segment p of the send and of the recv list
+        const int p = word * 32 + lane;
+        int64_t at[2] = {0, 0};
+        if (p < W) {
+#pragma unroll
+            for (int which = 0; which < 2; which++) {
+                at[which] = offsets[which * (W + 1) + p] + bsum[(int64_t)(which * W + p) * nblocks + blockIdx.x];
+                for (int w = 0; w < warp; w++) at[which] += ws[w][which][lane];
+            }
+        }
+        int64_t first_own = 0;
+        if (h.owner != nullptr) {
+            first_own = bsum[(int64_t)(2 * W) * nblocks + blockIdx.x];
+            for (int w = 0; w < warp; w++) first_own += wown[w];
+        }
+#pragma unroll
+        for (int k = 0; k < HL_ROUNDS; k++) {
+            const int64_t a = base + 32 * k;
+            const int64_t local = first_own + __popc(own[k] & lt);
+            if (word == 0 && ((own[k] >> lane) & 1u)) out.interior[local] = out.has_foreign[a] ? 0 : 1;
+            first_own += __popc(own[k]);
+#pragma unroll
+            for (int which = 0; which < 2; which++) {
+                const uint32_t mine = set[which][k];
+                for (uint32_t any = __reduce_or_sync(0xffffffffu, mine); any; any &= any - 1) {
+                    const int q = __ffs((int)any) - 1;
+                    const uint32_t m = __ballot_sync(0xffffffffu, (mine >> q) & 1u);
+                    const int64_t e = __shfl_sync(0xffffffffu, (long long)at[which], q) + __popc(m & lt);
+                    if ((mine >> q) & 1u) {
+                        if (which == 0) {
+                            out.send_local[e] = h.owner != nullptr ? local : out.value_map[a];
+                        } else {
+                            out.recv_atom[e] = a;
+                            out.recv_ghost[e] = out.n_local + e;
+                        }
+                    }
+                    if (lane == q) at[which] += __popc(m);
+                }
+            }
         }
         __syncthreads();
     }
 }
 
-// local index of each atom inside its owner's ascending list: excl scan of (owner == R)
 __global__ void __launch_bounds__(256)
 gather_not_u8_kernel(const uint8_t* __restrict__ flags, const int64_t* __restrict__ idx, int64_t n, uint8_t* __restrict__ out)
 {
@@ -261,7 +430,7 @@ extern "C" int dynb_bincount_i64(const int64_t* a_dev, int64_t n, int64_t W, int
 extern "C" int dynb_select_workspace_bytes(int64_t n, int64_t* bytes)
 {
     if (n < 0 || bytes == nullptr) return fail_arg("bad arguments");
-    *bytes = align_up((n + 2) * 4, 256) + align_up((int64_t)(scan_num_tiles(n + 2) + 1) * 8, 256) + 256;
+    *bytes = align_up((n / SELECT_TILE + 1) * 4, 256);
     return DYNB_OK;
 }
 
@@ -276,14 +445,10 @@ extern "C" int dynb_select_eq_i64(const int64_t* a_dev, int64_t n, int64_t value
     int64_t need;
     dynb_select_workspace_bytes(n, &need);
     if (workspace_dev == nullptr || workspace_bytes < need) return fail_arg("workspace too small (see dynb_select_workspace_bytes)");
-    unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
-    uint32_t* flags = reinterpret_cast<uint32_t*>(ws);
-    uint32_t* sums = reinterpret_cast<uint32_t*>(ws + align_up((n + 2) * 4, 256));
-    uint32_t* total = reinterpret_cast<uint32_t*>(ws + need - 256);
-    flag_eq_i64_kernel<<<nblk(n), 256, 0, s>>>(a_dev, n, value, flags);
-    DYNB_CUDA_OK((exclusive_scan<uint32_t, uint32_t>(flags, flags, nullptr, n, sums, total, s)));
-    scatter_selected_kernel<<<nblk(n), 256, 0, s>>>(a_dev, n, value, flags, gather_src_dev, out_dev);
-    u32_total_to_i64_kernel<<<1, 1, 0, s>>>(total, count_dev);
+    uint32_t* tile_count = static_cast<uint32_t*>(workspace_dev);
+    const unsigned tiles = nblk(n, SELECT_TILE);
+    select_count_kernel<<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count);
+    select_fill_kernel<<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count, gather_src_dev, out_dev, count_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -306,53 +471,69 @@ extern "C" int dynb_halo_mark_from_edges(const int64_t* edges_dev, int64_t E, co
     return DYNB_OK;
 }
 
-static inline int csr_blocks(int64_t n) { return (int)((n + CSR_THREADS - 1) / CSR_THREADS); }
+static inline int hl_blocks(int64_t n) { return (int)std::max<int64_t>((n + HL_TILE - 1) / HL_TILE, 1); }
 
-extern "C" int dynb_csr_workspace_bytes(int64_t n, int64_t W, int64_t* bytes)
+extern "C" int dynb_halo_lists_workspace_bytes(int64_t n, int64_t W, int64_t* bytes)
 {
     if (n < 0 || W < 1 || bytes == nullptr) return fail_arg("bad arguments");
-    *bytes = align_up((int64_t)std::max(csr_blocks(n), 1) * W * 4, 256) + align_up(W * 8, 256);
+    *bytes = align_up((int64_t)hl_blocks(n) * (2 * W + 1) * 4, 256) + align_up((2 * W + 1) * 8, 256) + 256;
     return DYNB_OK;
 }
 
-extern "C" int dynb_csr_plan(const uint32_t* mask_dev, const int64_t* owner_dev, int64_t n, int64_t R, int mode, int64_t W,
-                             int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream)
+static int halo_lists_args(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n, int64_t R,
+                           int64_t W, HaloSets& h)
 {
-    if (n < 0 || W < 1 || mode < 0 || mode > 2 || offsets_dev == nullptr) return fail_arg("bad arguments");
-    if (mode != CSR_RAW && owner_dev == nullptr) return fail_arg("owner required");
+    if (n < 0 || W < 1) return fail_arg("bad arguments");
+    if (n > 0 && (send_mask_dev == nullptr || (owner_dev == nullptr && recv_mask_dev == nullptr))) return fail_arg("null pointer");
+    if (owner_dev != nullptr && (R < 0 || R >= W)) return fail_arg("rank out of range");
     if (W > 4096) return fail_arg("world_size above 4096 is not supported");
+    h = HaloSets{send_mask_dev, recv_mask_dev, owner_dev, n, R, (int)((W + 31) / 32)};
+    return DYNB_OK;
+}
+
+extern "C" int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
+                                    int64_t R, int64_t W, int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream)
+{
+    HaloSets h;
+    int rc = halo_lists_args(send_mask_dev, recv_mask_dev, owner_dev, n, R, W, h);
+    if (rc) return rc;
     int64_t need;
-    dynb_csr_workspace_bytes(n, W, &need);
-    if (workspace_dev == nullptr || workspace_bytes < need) return fail_arg("workspace too small (see dynb_csr_workspace_bytes)");
+    dynb_halo_lists_workspace_bytes(n, W, &need);
+    if (offsets_dev == nullptr) return fail_arg("null pointer");
+    if (workspace_dev == nullptr || workspace_bytes < need) return fail_arg("workspace too small (see dynb_halo_lists_workspace_bytes)");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int words = (int)((W + 31) / 32);
-    const int nb = std::max(csr_blocks(n), 1);
-    unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
-    uint32_t* bsum = reinterpret_cast<uint32_t*>(ws);
-    int64_t* totals = reinterpret_cast<int64_t*>(ws + align_up((int64_t)nb * W * 4, 256));
     if (n == 0) {
-        DYNB_CUDA_OK(cudaMemsetAsync(offsets_dev, 0, (size_t)(W + 1) * 8, s));
+        DYNB_CUDA_OK(cudaMemsetAsync(offsets_dev, 0, (size_t)(2 * (W + 1) + 1) * 8, s));
         return DYNB_OK;
     }
-    csr_count_kernel<<<nb, CSR_THREADS, 0, s>>>(mask_dev, words, owner_dev, n, R, mode, (int)W, nb, bsum);
-    csr_scan_rows_kernel<<<(unsigned)W, SCAN_THREADS, 0, s>>>(bsum, nb, totals);
-    csr_offsets_kernel<<<1, 32, 0, s>>>(totals, (int)W, offsets_dev);
+    const int nb = hl_blocks(n);
+    unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
+    uint32_t* bsum = reinterpret_cast<uint32_t*>(ws);
+    int64_t* totals = reinterpret_cast<int64_t*>(ws + align_up((int64_t)nb * (2 * W + 1) * 4, 256));
+    uint32_t* arrived = reinterpret_cast<uint32_t*>(ws + need - 256);
+    DYNB_CUDA_OK(cudaMemsetAsync(arrived, 0, 4, s));
+    halo_lists_count_kernel<<<nb, HL_THREADS, 0, s>>>(h, (int)W, nb, bsum);
+    halo_lists_scan_kernel<<<(unsigned)(2 * W + 1), SCAN_THREADS, 0, s>>>(bsum, nb, (int)W, totals, arrived, offsets_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
 
-extern "C" int dynb_csr_fill(const uint32_t* mask_dev, const int64_t* owner_dev, int64_t n, int64_t R, int mode, int64_t W,
-                             const int64_t* value_map_dev, const int64_t* offsets_dev, int64_t* out_dev,
-                             const void* workspace_dev, void* stream)
+extern "C" int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
+                                    int64_t R, int64_t W, const int64_t* value_map_dev, const uint8_t* has_foreign_dev,
+                                    const int64_t* offsets_dev, int64_t n_local, int64_t* send_local_dev, int64_t* recv_atom_dev,
+                                    int64_t* recv_ghost_dev, uint8_t* interior_dev, const void* workspace_dev, void* stream)
 {
-    if (n < 0 || W < 1 || mode < 0 || mode > 2) return fail_arg("bad arguments");
+    HaloSets h;
+    int rc = halo_lists_args(send_mask_dev, recv_mask_dev, owner_dev, n, R, W, h);
+    if (rc) return rc;
     if (n == 0) return DYNB_OK;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int words = (int)((W + 31) / 32);
-    const int nb = csr_blocks(n);
-    const uint32_t* bsum = reinterpret_cast<const uint32_t*>(workspace_dev);
-    csr_fill_kernel<<<nb, CSR_THREADS, 0, s>>>(mask_dev, words, owner_dev, n, R, mode, (int)W, nb, bsum, offsets_dev,
-                                               value_map_dev, out_dev);
+    if (offsets_dev == nullptr || workspace_dev == nullptr || (owner_dev == nullptr && value_map_dev == nullptr) ||
+        (owner_dev != nullptr && has_foreign_dev == nullptr))
+        return fail_arg("null pointer");
+    const HaloListsOut out{value_map_dev, has_foreign_dev, send_local_dev, recv_atom_dev, recv_ghost_dev, interior_dev, n_local};
+    const int nb = hl_blocks(n);
+    halo_lists_fill_kernel<<<nb, HL_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(h, (int)W, nb, static_cast<const uint32_t*>(workspace_dev),
+                                                                                   offsets_dev, out);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -375,6 +556,13 @@ extern "C" int dynb_scatter_iota(const int64_t* idx_dev, int64_t n, int64_t N, i
     return DYNB_OK;
 }
 
+extern "C" int dynb_filter_edges_workspace_bytes(int64_t E, int64_t* bytes)
+{
+    if (E < 0 || bytes == nullptr) return fail_arg("bad arguments");
+    *bytes = align_up((2 * E + 2) * 4, 256) + align_up((int64_t)(scan_num_tiles(2 * E + 2) + 1) * 8, 256) + 256;
+    return DYNB_OK;
+}
+
 extern "C" int dynb_filter_edges_plan(const int64_t* edges_dev, const float* shifts_f32_dev, const float* pos_dev,
                                       const float* cell_host, double radius, int64_t E, int64_t* count_dev,
                                       void* workspace_dev, int64_t workspace_bytes, void* stream)
@@ -384,8 +572,8 @@ extern "C" int dynb_filter_edges_plan(const int64_t* edges_dev, const float* shi
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (E == 0) { DYNB_CUDA_OK(cudaMemsetAsync(count_dev, 0, 8, s)); return DYNB_OK; }
     int64_t need;
-    dynb_select_workspace_bytes(2 * E, &need);
-    if (workspace_dev == nullptr || workspace_bytes < need) return fail_arg("workspace too small (dynb_select_workspace_bytes(2*E))");
+    dynb_filter_edges_workspace_bytes(E, &need);
+    if (workspace_dev == nullptr || workspace_bytes < need) return fail_arg("workspace too small (see dynb_filter_edges_workspace_bytes)");
     unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
     uint32_t* keep = reinterpret_cast<uint32_t*>(ws);
     uint32_t* excl = keep + (E + 1);

@@ -804,18 +804,7 @@ __device__ __forceinline__ int runs_flags(uint32_t* flags, int run_off, int run_
     return __popc(before);
 }
 
-enum { MODE_COUNT = 0, MODE_FILL = 1, MODE_HALO = 2 };
-
-// MODE_HALO: instead of counting or writing edges, record for every edge src -> dst whose
-// endpoints have different owners that owner(dst) needs src (bit owner(dst) of needed[src]) and
-// that dst has a foreign neighbour.  This is the edge loop of the reference's halo-map builder
-// (dynamis_state/src/csrc/build_halo_maps.cpp:50-58, 127-138) without materialising the graph.
-struct HaloArgs {
-    const long long* owner;   // [n_atoms] rank of each atom
-    uint32_t* needed;         // [n_atoms, words]
-    unsigned char* has_foreign;  // [n_atoms]
-    int words;
-};
+enum { MODE_COUNT = 0, MODE_FILL = 1 };
 
 #ifndef DYNB_COUNT_UNROLL
 #define DYNB_COUNT_UNROLL 1
@@ -910,7 +899,7 @@ rg_group_list_kernel(const PairParams<T>* __restrict__ params_dev, uint32_t* __r
 template <typename T, int MODE, bool BYVAL>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
 rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T> params_val, long long* __restrict__ ei,
-               float* __restrict__ shifts, T* __restrict__ d2out, const long long E, const HaloArgs halo, const int skip_if_masks,
+               float* __restrict__ shifts, T* __restrict__ d2out, const long long E, const int skip_if_masks,
                const GlueArgs glue)
 {
     // BYVAL: the launch has the record at hand and passes it as a kernel argument; its fields are then operands
@@ -1159,22 +1148,14 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
                 const Vec4<T> tpB = p.tpos[has2 ? t + 1 : t];
                 const T ax = tpA.x, ay = tpA.y, az = tpA.z, bx = tpB.x, by = tpB.y, bz = tpB.z;
                 int prodA = 0, prodB = 0;
-                if (chunk != 0 && MODE != MODE_HALO) {
+                if (chunk != 0) {
                     prodA = (int)p.tcount[t];
                     prodB = has2 ? (int)p.tcount[t + 1] : 0;
                 }
                 {
                     int4 tmA = p.tmeta[t];
                     int4 tmB = p.tmeta[has2 ? t + 1 : t];
-                    long long baseA = 0, baseB = 0, ownA = 0, ownB = 0;
-                    bool foreignA = false, foreignB = false;
-                    if (MODE == MODE_FILL) {
-                        baseA = p.toffset[t];
-                        baseB = p.toffset[has2 ? t + 1 : t];
-                    } else {
-                        ownA = halo.owner[tmA.x];
-                        ownB = halo.owner[tmB.x];
-                    }
+                    const long long baseA = p.toffset[t], baseB = p.toffset[has2 ? t + 1 : t];
                     int n = 0, nB = 0;  // parked hits of target A / target B
                     for (int k = 0; k < clen32; k += 32) {
                         const int j = k + lane;
@@ -1183,24 +1164,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
                         const T dB = dist2<T>(bx, by, bz, c.x, c.y, c.z);
                         const bool hitA = (dA <= r2) && (dA > eps);
                         const bool hitB = has2 && (dB <= r2) && (dB > eps);
-                        if (MODE == MODE_HALO) {
-                            if (hitA || hitB) {
-                                const int a = real_to_bits(c.w);
-                                const long long oa = halo.owner[a];
-                                if (hitA && oa != ownA) {
-                                    uint32_t* wd = &halo.needed[(long long)a * halo.words + (ownA >> 5)];
-                                    const uint32_t bit = 1u << (ownA & 31);
-                                    if (!(*wd & bit)) atomicOr(wd, bit);
-                                    foreignA = true;
-                                }
-                                if (hitB && oa != ownB) {
-                                    uint32_t* wd = &halo.needed[(long long)a * halo.words + (ownB >> 5)];
-                                    const uint32_t bit = 1u << (ownB & 31);
-                                    if (!(*wd & bit)) atomicOr(wd, bit);
-                                    foreignB = true;
-                                }
-                            }
-                        } else {
+                        {
                             // each target parks the slots of its hits in its own half of the list; the index in
                             // the half is the position inside the target's edge run since the last write-out
                             const uint32_t mA = __ballot_sync(0xffffffffu, hitA);
@@ -1241,14 +1205,9 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
                             }
                         }
                     }
-                    if (MODE == MODE_FILL) {
-                        if (more_chunks && lane == 0) {
-                            p.tcount[t] = (uint32_t)prodA;
-                            if (has2) p.tcount[t + 1] = (uint32_t)prodB;
-                        }
-                    } else {
-                        if (__any_sync(0xffffffffu, foreignA) && lane == 0) halo.has_foreign[tmA.x] = 1;
-                        if (has2 && __any_sync(0xffffffffu, foreignB) && lane == 0) halo.has_foreign[tmB.x] = 1;
+                    if (more_chunks && lane == 0) {
+                        p.tcount[t] = (uint32_t)prodA;
+                        if (has2) p.tcount[t + 1] = (uint32_t)prodB;
                     }
                 }
             }
@@ -1430,6 +1389,170 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// Halo marking: for every edge src -> dst whose endpoints have different owners, owner(dst) needs src (bit owner(dst)
+// of needed[src]) and dst has a foreign neighbour.  This is the edge loop of the reference's halo-map builder
+// (dynamis_state/src/csrc/build_halo_maps.cpp:50-58, 127-138) without materialising the graph.  With rank >= 0 only
+// the edges that start or end at an atom of that rank are looked at: they are all its send and receive lists need.
+//
+// Bound by instruction issue, so the work is in what is not tested: most of the volume lies inside one subdomain.  The
+// owners of the cell-sorted records and targets are gathered once (rg_halo_owner_kernel); a warp then looks only at the
+// owners of its group's candidates, keeps those that can matter to one of its targets, and tests distances for these
+// alone — lane = candidate, targets broadcast from shared memory, so that the bits a candidate collects stay in a
+// register and go out with one atomic per candidate and group.
+// ------------------------------------------------------------------------------------------
+struct HaloArgs {
+    const long long* owner;      // [n_atoms] rank of each atom
+    unsigned short* sown;        // [M] owner of every source record, [Nt] of every target behind it (sorted orders)
+    unsigned short* town;
+    uint32_t* needed;            // [n_atoms, words]
+    unsigned char* has_foreign;  // [n_atoms]
+    int words;
+    int rank;                    // -1: all ranks
+};
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo, int64_t Nt)
+{
+    const PairParams<T> p = *params_dev;
+    if (p.h->status & RG_FATAL) return;
+    const int64_t M = (int64_t)p.h->M, n = M > Nt ? M : Nt;
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
+        if (j < M) halo.sown[j] = (unsigned short)halo.owner[p.smeta[j].x];
+        if (j < Nt) halo.town[j] = (unsigned short)halo.owner[p.tmeta[j].x];
+    }
+}
+
+constexpr int HALO_LIST = 512;     // candidates kept per warp before they are tested
+constexpr int HALO_TARGETS = 32;   // targets of a group tested together
+template <typename T> struct HaloWarp {
+    Vec4<T> tgt[HALO_TARGETS];     // w = owner
+    int list[HALO_LIST];
+};
+
+// One warp tests its listed candidates against its staged targets.
+template <typename T, bool WIDE>
+__device__ __forceinline__ uint32_t halo_test(const PairParams<T>& p, const HaloArgs& halo, const HaloWarp<T>& w, int n, int nt, int lane)
+{
+    const T r2 = p.r2, eps = (T)1e-8f;
+    uint32_t foreign = 0;  // bit q: target q has a foreign neighbour among these candidates
+    for (int base = 0; base < n; base += 32) {
+        const bool live = base + lane < n;
+        const int rec = w.list[live ? base + lane : 0];
+        const Vec4<T> c = p.spos[rec];
+        const int o = live ? (int)halo.sown[rec] : -1;
+        uint32_t need = 0;
+        for (int q = 0; q < nt; q++) {
+            const Vec4<T> t = w.tgt[q];
+            const int ot = real_to_bits(t.w);
+            const T d = dist2<T>(t.x, t.y, t.z, c.x, c.y, c.z);
+            const bool hit = (d <= r2) && (d > eps) && o >= 0 && o != ot && (halo.rank < 0 || o == halo.rank || ot == halo.rank);
+            if (hit) {
+                if (!WIDE) {
+                    need |= 1u << ot;
+                } else {
+                    uint32_t* wd = &halo.needed[(long long)real_to_bits(c.w) * halo.words + (ot >> 5)];
+                    const uint32_t bit = 1u << (ot & 31);
+                    if (!(*wd & bit)) atomicOr(wd, bit);
+                }
+            }
+            if (__any_sync(0xffffffffu, hit)) foreign |= 1u << q;
+        }
+        if (!WIDE && need) {
+            uint32_t* wd = &halo.needed[real_to_bits(c.w)];
+            if ((*wd & need) != need) atomicOr(wd, need);
+        }
+    }
+    return foreign;
+}
+
+template <typename T, bool WIDE>   // WIDE: more than 32 ranks, several words per atom
+__global__ void __launch_bounds__(PAIR_THREADS, 4)
+rg_halo_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo)
+{
+    const PairParams<T> p = *params_dev;
+    __shared__ HaloWarp<T> warps[PAIR_WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    HaloWarp<T>& w = warps[warp];
+    const DevHeader* hp = p.h;
+    if (hp->status & RG_FATAL) return;
+    const int nx = hp->nx, ny = hp->ny, nz = hp->nz, S = hp->group_cells, Sy = hp->group_cells_y, pad = hp->pad;
+    const uint32_t gx = (uint32_t)hp->gx, gy = (uint32_t)((ny + Sy - 1) / Sy), num_groups = (uint32_t)hp->num_groups;
+    const int Wd = 2 * pad + 1, Wy = Sy + 2 * pad, nrun = Wy * Wd;
+    const int lane_dy = (lane % Wy) - pad, lane_dz = (lane / Wy) - pad;
+    const uint32_t lt = lanemask_lt();
+    const int rank = halo.rank;
+
+    const uint32_t nwarps = gridDim.x * PAIR_WARPS;
+    for (uint32_t grp = blockIdx.x * PAIR_WARPS + warp; grp < num_groups; grp += nwarps) {
+        const uint32_t row = grp / gx;
+        const int ix = (int)(grp - row * gx);
+        const int cz = (int)(row / gy), iy = (int)(row - (uint32_t)cz * gy);
+        const int cx0 = ix * S, cx1 = min(cx0 + S, nx) - 1;
+        const int cy0 = iy * Sy, cy1 = min(cy0 + Sy, ny) - 1;
+        const uint32_t tb0 = p.tcstart[((uint32_t)cz * ny + cy0) * nx + cx0], te0 = p.tcstart[((uint32_t)cz * ny + cy0) * nx + cx1 + 1];
+        uint32_t tb1 = 0, te1 = 0;
+        if (cy1 > cy0) {
+            tb1 = p.tcstart[((uint32_t)cz * ny + cy1) * nx + cx0];
+            te1 = p.tcstart[((uint32_t)cz * ny + cy1) * nx + cx1 + 1];
+        }
+        const int n0 = (int)(te0 - tb0), ntot = n0 + (int)(te1 - tb1);
+        if (ntot == 0) continue;
+        int run_a = 0, run_len = 0;
+        if (lane < nrun) {
+            const int yy = cy0 + lane_dy, zz = cz + lane_dz;
+            if (yy >= 0 && yy < ny && yy <= cy1 + pad && zz >= 0 && zz < nz) {
+                const uint32_t b = ((uint32_t)zz * ny + yy) * nx;
+                run_a = (int)p.cstart[b + max(cx0 - pad, 0)];
+                run_len = (int)(p.cstart[b + min(cx1 + pad, nx - 1) + 1]) - run_a;
+            }
+        }
+        const int longest = __reduce_max_sync(0xffffffffu, run_len);
+        for (int q0 = 0; q0 < ntot; q0 += HALO_TARGETS) {
+            const int nt = min(HALO_TARGETS, ntot - q0);
+            const uint32_t t = (q0 + lane < n0) ? tb0 + q0 + lane : tb1 + (q0 + lane - n0);
+            const int ot = (lane < nt) ? (int)halo.town[t] : 0;
+            const int lo = __reduce_min_sync(0xffffffffu, lane < nt ? ot : 0x7fffffff), hi = __reduce_max_sync(0xffffffffu, ot);
+            const bool uniform = lo == hi, any_rank = rank < 0 || __any_sync(0xffffffffu, lane < nt && ot == rank);
+            bool staged = false;
+            uint32_t foreign = 0;
+            int n = 0;
+            for (int i = 0; i < longest; i++) {
+                bool keep = false;
+                if (i < run_len) {
+                    const int o = (int)halo.sown[run_a + i];
+                    keep = (any_rank || o == rank) && !(uniform && o == lo);
+                }
+                const uint32_t m = __ballot_sync(0xffffffffu, keep);
+                if (m == 0u) continue;
+                if (!staged) {
+                    if (lane < nt) {
+                        Vec4<T> v = p.tpos[t];
+                        v.w = bits_to_real(ot, T());
+                        w.tgt[lane] = v;
+                    }
+                    staged = true;
+                }
+                if (keep) w.list[n + __popc(m & lt)] = run_a + i;
+                n += __popc(m);
+                if (n > HALO_LIST - 32) {
+                    __syncwarp();
+                    foreign |= halo_test<T, WIDE>(p, halo, w, n, nt, lane);
+                    n = 0;
+                    __syncwarp();
+                }
+            }
+            if (n > 0) {
+                __syncwarp();
+                foreign |= halo_test<T, WIDE>(p, halo, w, n, nt, lane);
+            }
+            if (lane < nt && (foreign >> lane) & 1u) halo.has_foreign[p.tmeta[t].x] = 1;
+            __syncwarp();
+        }
+    }
+}
+
 // First launch of a plan: the header block (it travels as a kernel argument: no staging copy of a pageable host
 // buffer), the cell counters, the degree counters and the caller's degree array in one pass.
 struct HeaderBlock { uint32_t words[RG_HEADER_BYTES / 4]; };
@@ -1577,8 +1700,9 @@ static int rg_suggest(int64_t N, const void* cell_host, const uint8_t* pbc_host,
 template <typename T>
 static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const uint8_t* pbc_host, double radius,
                    const int64_t* targets, int64_t Nt, void* ws, int64_t ws_bytes, int64_t src_cap, int64_t cell_cap,
-                   int32_t* counts_out, dynb_rg_header* header_host, cudaStream_t stream)
+                   int32_t* counts_out, dynb_rg_header* header_host, bool bins_only, cudaStream_t stream)
 {
+    // bins_only: the plan ends with the sorted records (all that the halo marking reads)
     Geom<T> g;
     int rc = rg_geometry_checked<T>(cell_host, pbc_host, radius, g);
     if (rc) return rc;
@@ -1671,7 +1795,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         HeaderBlock blk;
         memcpy(blk.words, init, sizeof(init));
         // every region of the layout starts on a 256-byte boundary and is padded to one
-        const int64_t n_a16 = (L.partials - L.ccount) / 16, n_b16 = ((Nt + 1) * 4 + 15) / 16;
+        const int64_t n_a16 = (L.partials - L.ccount) / 16, n_b16 = bins_only ? 0 : ((Nt + 1) * 4 + 15) / 16;
         rg_init_kernel<<<sm_count_cached() * 4, 256, 0, stream>>>(reinterpret_cast<uint32_t*>(w + L.hdr), blk,
                                                                   reinterpret_cast<uint4*>(w + L.ccount), n_a16,
                                                                   reinterpret_cast<uint4*>(w + L.tcount), n_b16, counts_out, Nt);
@@ -1711,12 +1835,18 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     rg_bin_finalize_kernel<T><<<(unsigned)((nf + 255) / 256), 256, 0, stream>>>(
         N, Nt, targets, g, posw, aff, h, ccount, tccount, srec, trec, spos, sxyz, src_cap, scode, smeta, tpos, tmeta);
 
+    if (bins_only) {
+        DYNB_CUDA_OK(cudaGetLastError());
+        if (header_host != nullptr)
+            DYNB_CUDA_OK(cudaMemcpyAsync(header_host, h, sizeof(dynb_rg_header), cudaMemcpyDeviceToHost, stream));
+        return DYNB_OK;
+    }
     if (targets != nullptr)
         rg_group_list_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, tcfill);
     const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
     DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_COUNT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const int grid = sm_count_cached() * 4 * pair_grid_waves();
-    rg_pair_kernel<T, MODE_COUNT, true><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, pp_host, nullptr, nullptr, nullptr, 0, HaloArgs{}, 0, GlueArgs{});
+    rg_pair_kernel<T, MODE_COUNT, true><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, pp_host, nullptr, nullptr, nullptr, 0, 0, GlueArgs{});
     DYNB_CUDA_OK((exclusive_scan<uint32_t, long long>(tcount, toffset, nullptr, Nt + 1, sums64,
                                                        reinterpret_cast<long long*>(&h->E), stream)));
     DYNB_CUDA_OK(cudaGetLastError());
@@ -1752,20 +1882,20 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
     // behind the bit-driven writer this launch only has the listed long groups to do (usually none): two waves keep its cost low
     const int fgrid = use_masks ? sm_count_cached() * 4 * std::min(2, pair_grid_waves()) : grid;
     rg_pair_kernel<T, MODE_FILL, false><<<fgrid, PAIR_THREADS, smem, stream>>>(
-        params_dev, PairParams<T>{}, reinterpret_cast<long long*>(ei), shifts, static_cast<T*>(d2out), (long long)E, HaloArgs{}, use_masks, glue);
+        params_dev, PairParams<T>{}, reinterpret_cast<long long*>(ei), shifts, static_cast<T*>(d2out), (long long)E, use_masks, glue);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
 
 template <typename T>
-static int rg_halo_mark(const void* ws, const HaloArgs& ha, cudaStream_t stream)
+static int rg_halo_mark(const void* ws, HaloArgs ha, int64_t N, cudaStream_t stream)
 {
     const unsigned char* w = static_cast<const unsigned char*>(ws);
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
-    const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
-    DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_HALO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    rg_halo_owner_kernel<T><<<(unsigned)std::min<int64_t>((N + 255) / 256, (int64_t)sm_count_cached() * 8), 256, 0, stream>>>(params_dev, ha, N);
     const int grid = sm_count_cached() * 4 * pair_grid_waves();
-    rg_pair_kernel<T, MODE_HALO, false><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, PairParams<T>{}, nullptr, nullptr, nullptr, 0, ha, 0, GlueArgs{});
+    if (ha.words == 1) rg_halo_kernel<T, false><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
+    else rg_halo_kernel<T, true><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -1798,11 +1928,10 @@ extern "C" int dynb_rg_workspace_bytes(int64_t n_atoms, int64_t n_targets, int64
     return DYNB_OK;
 }
 
-extern "C" int dynb_rg_plan(const void* pos_dev, int dtype, int64_t n_atoms, const void* cell_host,
-                            const uint8_t* pbc_host, double radius, const int64_t* target_indices_dev,
-                            int64_t n_targets, void* workspace_dev, int64_t workspace_bytes, int64_t src_capacity,
-                            int64_t cell_capacity, int32_t* neighbor_counts_dev, dynb_rg_header* header_host,
-                            void* stream)
+static int rg_plan_any(const void* pos_dev, int dtype, int64_t n_atoms, const void* cell_host, const uint8_t* pbc_host, double radius,
+                       const int64_t* target_indices_dev, int64_t n_targets, void* workspace_dev, int64_t workspace_bytes,
+                       int64_t src_capacity, int64_t cell_capacity, int32_t* neighbor_counts_dev, dynb_rg_header* header_host,
+                       bool bins_only, void* stream)
 {
     if (n_atoms <= 0 || n_targets <= 0) return fail_arg("n_atoms and n_targets must be positive (handle empty input in the caller)");
     if (pos_dev == nullptr || workspace_dev == nullptr) return fail_arg("null device pointer");
@@ -1813,11 +1942,29 @@ extern "C" int dynb_rg_plan(const void* pos_dev, int dtype, int64_t n_atoms, con
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (dtype == DYNB_F32)
         return rg_plan<float>(pos_dev, n_atoms, cell_host, pbc_host, radius, target_indices_dev, n_targets, workspace_dev,
-                              workspace_bytes, src_capacity, cell_capacity, neighbor_counts_dev, header_host, s);
+                              workspace_bytes, src_capacity, cell_capacity, neighbor_counts_dev, header_host, bins_only, s);
     if (dtype == DYNB_F64)
         return rg_plan<double>(pos_dev, n_atoms, cell_host, pbc_host, radius, target_indices_dev, n_targets, workspace_dev,
-                               workspace_bytes, src_capacity, cell_capacity, neighbor_counts_dev, header_host, s);
+                               workspace_bytes, src_capacity, cell_capacity, neighbor_counts_dev, header_host, bins_only, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");
+}
+
+extern "C" int dynb_rg_plan(const void* pos_dev, int dtype, int64_t n_atoms, const void* cell_host,
+                            const uint8_t* pbc_host, double radius, const int64_t* target_indices_dev,
+                            int64_t n_targets, void* workspace_dev, int64_t workspace_bytes, int64_t src_capacity,
+                            int64_t cell_capacity, int32_t* neighbor_counts_dev, dynb_rg_header* header_host,
+                            void* stream)
+{
+    return rg_plan_any(pos_dev, dtype, n_atoms, cell_host, pbc_host, radius, target_indices_dev, n_targets, workspace_dev,
+                       workspace_bytes, src_capacity, cell_capacity, neighbor_counts_dev, header_host, false, stream);
+}
+
+extern "C" int dynb_rg_bin(const void* pos_dev, int dtype, int64_t n_atoms, const void* cell_host, const uint8_t* pbc_host,
+                           double radius, void* workspace_dev, int64_t workspace_bytes, int64_t src_capacity, int64_t cell_capacity,
+                           dynb_rg_header* header_host, void* stream)
+{
+    return rg_plan_any(pos_dev, dtype, n_atoms, cell_host, pbc_host, radius, nullptr, n_atoms, workspace_dev, workspace_bytes,
+                       src_capacity, cell_capacity, nullptr, header_host, true, stream);
 }
 
 extern "C" int dynb_rg_fill(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
@@ -1855,20 +2002,25 @@ extern "C" int dynb_rg_fill_glue(const void* workspace_dev, int dtype, int64_t* 
 }
 
 extern "C" int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
-                                 int64_t world_size, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream)
+                                 int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev,
+                                 int64_t src_capacity, void* scratch_dev, int64_t scratch_bytes, void* stream)
 {
-    if (workspace_dev == nullptr || owner_dev == nullptr || needed_dev == nullptr || has_foreign_dev == nullptr)
+    if (workspace_dev == nullptr || owner_dev == nullptr || needed_dev == nullptr || has_foreign_dev == nullptr || scratch_dev == nullptr)
         return fail_arg("null pointer");
-    if (n_atoms <= 0 || world_size < 1) return fail_arg("bad sizes");
+    if (n_atoms <= 0 || world_size < 1 || world_size > 65535 || rank < -1 || rank >= world_size) return fail_arg("bad sizes");
+    if (src_capacity < 1 || scratch_bytes < 2 * (n_atoms + src_capacity)) return fail_arg("scratch must hold 2 * (n_atoms + src_capacity) bytes");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     HaloArgs ha;
     ha.owner = reinterpret_cast<const long long*>(owner_dev);
+    ha.town = static_cast<unsigned short*>(scratch_dev);
+    ha.sown = ha.town + n_atoms;
     ha.needed = needed_dev;
     ha.has_foreign = has_foreign_dev;
     ha.words = (int)((world_size + 31) / 32);
+    ha.rank = (int)rank;
     DYNB_CUDA_OK(cudaMemsetAsync(needed_dev, 0, (size_t)n_atoms * ha.words * 4, s));
     DYNB_CUDA_OK(cudaMemsetAsync(has_foreign_dev, 0, (size_t)n_atoms, s));
-    if (dtype == DYNB_F32) return rg_halo_mark<float>(workspace_dev, ha, s);
-    if (dtype == DYNB_F64) return rg_halo_mark<double>(workspace_dev, ha, s);
+    if (dtype == DYNB_F32) return rg_halo_mark<float>(workspace_dev, ha, n_atoms, s);
+    if (dtype == DYNB_F64) return rg_halo_mark<double>(workspace_dev, ha, n_atoms, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");
 }

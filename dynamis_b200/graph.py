@@ -137,6 +137,76 @@ class RadiusGraphPlan:
         return edge_index, unit, cart
 
 
+def _geometry(st: dict, cell_np, pbc_np, radius: float, N: int, dtype_code: int):
+    """Host-side conversions and capacities of a geometry, kept by value of (cell, pbc, radius, sizes):
+    (key, (cell, pbc, radius, source capacity, cell capacity))."""
+    key = (cell_np.tobytes(), str(cell_np.dtype), pbc_np.tobytes(), float(radius), N, dtype_code)
+    geo = st["geo"].get(key)
+    if geo is None:
+        np_real = np.float64 if dtype_code == _lib.DYNB_F64 else np.float32
+        cell_h = np.ascontiguousarray(cell_np.astype(np_real))
+        pbc_h = np.ascontiguousarray(pbc_np.astype(bool).astype(np.uint8))
+        radius_h = float(np.float32(radius)) if dtype_code == _lib.DYNB_F32 else float(radius)
+        src_cap = ctypes.c_int64()
+        cell_cap = ctypes.c_int64()
+        _lib.check(_lib.lib().dynb_rg_suggest_capacity(N, cell_h.ctypes.data, pbc_h.ctypes.data, radius_h, dtype_code,
+                                                       ctypes.byref(src_cap), ctypes.byref(cell_cap)), "rg_suggest_capacity")
+        if len(st["geo"]) > 64:
+            st["geo"].clear()
+        geo = st["geo"][key] = (cell_h, pbc_h, radius_h, src_cap.value, cell_cap.value)
+    return key, geo
+
+
+def _raise_status(status: int) -> None:
+    if status & _lib.RG_BAD_TARGET:
+        raise RuntimeError("target_indices contains an index outside [0, N)")
+    if status & _lib.RG_NONFINITE:
+        raise RuntimeError("pos contains NaN or Inf")
+    if status & _lib.RG_SHIFT_RANGE:
+        raise RuntimeError("an atom lies too many periodic cells outside the unit cell (limit 511)")
+    if status & _lib.RG_SRC_OVERFLOW:
+        raise RuntimeError("periodic-image capacity overflow")
+
+
+class BinnedAtoms:
+    """The cell-sorted records of all atoms and their periodic images, without degrees (what halo marking reads).
+
+    ``launch()`` queues the work; once the stream has been waited for, ``done()`` says whether the records are
+    there (True), raises for bad input, or returns False after enlarging the image capacity: launch again."""
+
+    def __init__(self, pos, cell, pbc, radius):
+        self.pos = pos.contiguous()
+        self.dtype_code = _lib.DYNB_F64 if pos.dtype == torch.float64 else _lib.DYNB_F32
+        self.st = _dev_state(pos.device)
+        self.hdr_t = torch.empty((64,), dtype=torch.uint8, pin_memory=True)
+        self.hdr = _lib.RgHeader.from_address(self.hdr_t.data_ptr())
+        self.key, geo = _geometry(self.st, cell.detach().to("cpu").numpy(), pbc.detach().to("cpu").numpy(), radius, pos.size(0),
+                                  self.dtype_code)
+        self.cell_h, self.pbc_h, self.radius, self.src_capacity, self.cell_capacity = geo
+        self.attempts = 0
+        self.ws = None
+
+    def launch(self) -> None:
+        L, N, dev = _lib.lib(), self.pos.size(0), self.pos.device
+        nbytes = ctypes.c_int64()
+        _lib.check(L.dynb_rg_workspace_bytes(N, N, self.src_capacity, self.cell_capacity, self.dtype_code, ctypes.byref(nbytes)),
+                   "rg_workspace_bytes")
+        self.ws = _workspace(self.st, nbytes.value, dev)
+        self.attempts += 1
+        _lib.check(L.dynb_rg_bin(self.pos.data_ptr(), self.dtype_code, N, self.cell_h.ctypes.data, self.pbc_h.ctypes.data, self.radius,
+                                 self.ws.data_ptr(), self.ws.numel(), self.src_capacity, self.cell_capacity, self.hdr_t.data_ptr(),
+                                 torch.cuda.current_stream(dev).cuda_stream), "rg_bin")
+
+    def done(self) -> bool:
+        status = int(self.hdr.status)
+        if status & _lib.RG_SRC_OVERFLOW and self.attempts < 3:
+            self.src_capacity = max(int(self.hdr.M) + 1024, 2 * self.src_capacity)
+            self.st["geo"][self.key] = (self.cell_h, self.pbc_h, self.radius, self.src_capacity, self.cell_capacity)
+            return False
+        _raise_status(status)
+        return True
+
+
 def plan_radius_graph(pos, cell, pbc, radius, target_indices=None) -> RadiusGraphPlan:
     """Counting phase (wrap, periodic images, cell binning, degrees, offsets).  Synchronises the
     current stream once to learn the number of edges.  ``pos`` must be non-empty."""
@@ -150,27 +220,12 @@ def plan_radius_graph(pos, cell, pbc, radius, target_indices=None) -> RadiusGrap
     L = _lib.lib()
     dev = pos.device
     dtype_code = _lib.DYNB_F64 if pos.dtype == torch.float64 else _lib.DYNB_F32
-    np_real = np.float64 if pos.dtype == torch.float64 else np.float32
     cell_np = cell.detach().to("cpu").numpy()
     pbc_np = pbc.detach().to("cpu").numpy()
 
     with _lib.on_device(dev):
         st = _dev_state(dev)
-        # the host-side conversions and the capacities of a geometry are kept by value of (cell, pbc, radius, sizes)
-        geo_key = (cell_np.tobytes(), str(cell_np.dtype), pbc_np.tobytes(), float(radius), N, dtype_code)
-        geo = st["geo"].get(geo_key)
-        if geo is None:
-            cell_h = np.ascontiguousarray(cell_np.astype(np_real))
-            pbc_h = np.ascontiguousarray(pbc_np.astype(bool).astype(np.uint8))
-            radius_h = float(np.float32(radius)) if dtype_code == _lib.DYNB_F32 else float(radius)
-            src_cap = ctypes.c_int64()
-            cell_cap = ctypes.c_int64()
-            _lib.check(L.dynb_rg_suggest_capacity(N, cell_h.ctypes.data, pbc_h.ctypes.data, radius_h, dtype_code,
-                                                  ctypes.byref(src_cap), ctypes.byref(cell_cap)), "rg_suggest_capacity")
-            if len(st["geo"]) > 64:
-                st["geo"].clear()
-            geo = st["geo"][geo_key] = (cell_h, pbc_h, radius_h, src_cap.value, cell_cap.value)
-        cell_h, pbc_h, radius, src_cap, cell_cap = geo
+        geo_key, (cell_h, pbc_h, radius, src_cap, cell_cap) = _geometry(st, cell_np, pbc_np, radius, N, dtype_code)
         counts = torch.empty((Nt,), dtype=torch.int32, device=dev)
         stream = torch.cuda.current_stream(dev)
         hdr = st["hdr"]
@@ -190,14 +245,7 @@ def plan_radius_graph(pos, cell, pbc, radius, target_indices=None) -> RadiusGrap
                 st["geo"][geo_key] = (cell_h, pbc_h, radius, src_cap, cell_cap)  # the next call starts with the larger capacity
                 continue
             break
-    if status & _lib.RG_BAD_TARGET:
-        raise RuntimeError("target_indices contains an index outside [0, N)")
-    if status & _lib.RG_NONFINITE:
-        raise RuntimeError("pos contains NaN or Inf")
-    if status & _lib.RG_SHIFT_RANGE:
-        raise RuntimeError("an atom lies too many periodic cells outside the unit cell (limit 511)")
-    if status & _lib.RG_SRC_OVERFLOW:
-        raise RuntimeError("periodic-image capacity overflow")
+    _raise_status(status)
     plan = RadiusGraphPlan()
     plan.ws = ws
     plan.dtype_code = dtype_code

@@ -52,7 +52,7 @@ def filter_edges_to_radius(edges: torch.Tensor, cell_shifts: torch.Tensor, pos: 
     L = _lib.lib()
     with torch.cuda.device(dev):
         nbytes = ctypes.c_int64()
-        _lib.check(L.dynb_select_workspace_bytes(2 * E, ctypes.byref(nbytes)), "select_workspace_bytes")
+        _lib.check(L.dynb_filter_edges_workspace_bytes(E, ctypes.byref(nbytes)), "filter_edges_workspace_bytes")
         ws = scratch(dev, "filter", nbytes.value)
         cnt = torch.empty((1,), dtype=torch.int64, device=dev)
         _lib.check(L.dynb_filter_edges_plan(edges.data_ptr(), shifts_f.data_ptr(), pos.data_ptr(), cell_h.ctypes.data,
@@ -109,26 +109,22 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
         g2l = torch.full((max(N, 1),), -1, dtype=torch.int64, device=dev)
         _lib.check(L.dynb_scatter_iota(mine.data_ptr(), n_local, N, g2l.data_ptr(), bad.data_ptr(), _stream(dev)), "scatter_iota")
         nbytes = ctypes.c_int64()
-        _lib.check(L.dynb_csr_workspace_bytes(N, W, ctypes.byref(nbytes)), "csr_workspace_bytes")
-        ws_s = scratch(dev, "csr_send", nbytes.value)
-        ws_r = scratch(dev, "csr_recv", nbytes.value)
-        offs = torch.empty((2, W + 1), dtype=torch.int64, device=dev)
-        _lib.check(L.dynb_csr_plan(send_mask.data_ptr(), None, N, R, 2, W, offs[0].data_ptr(), ws_s.data_ptr(), ws_s.numel(),
-                                   _stream(dev)), "csr_plan(send)")
-        _lib.check(L.dynb_csr_plan(recv_mask.data_ptr(), None, N, R, 2, W, offs[1].data_ptr(), ws_r.data_ptr(), ws_r.numel(),
-                                   _stream(dev)), "csr_plan(recv)")
+        _lib.check(L.dynb_halo_lists_workspace_bytes(N, W, ctypes.byref(nbytes)), "halo_lists_workspace_bytes")
+        ws = scratch(dev, "halo_lists", nbytes.value)
+        offs = torch.empty((2 * (W + 1) + 1,), dtype=torch.int64, device=dev)
+        _lib.check(L.dynb_halo_lists_plan(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, offs.data_ptr(), ws.data_ptr(),
+                                          ws.numel(), _stream(dev)), "halo_lists_plan")
         offs_h = offs.cpu()
         if int(bad.item()) != 0:
             raise RuntimeError("extract_halo_info: an edge endpoint, partition id or my_outer_atoms entry is out of range")
-        total_send, total_recv = int(offs_h[0, W]), int(offs_h[1, W])
+        total_send, total_recv = int(offs_h[W]), int(offs_h[2 * W + 1])
         send_local = torch.empty((total_send,), dtype=torch.int64, device=dev)
         recv_atom = torch.empty((total_recv,), dtype=torch.int64, device=dev)
-        _lib.check(L.dynb_csr_fill(send_mask.data_ptr(), None, N, R, 2, W, g2l.data_ptr(), offs[0].data_ptr(),
-                                   send_local.data_ptr(), ws_s.data_ptr(), _stream(dev)), "csr_fill(send)")
-        _lib.check(L.dynb_csr_fill(recv_mask.data_ptr(), None, N, R, 2, W, None, offs[1].data_ptr(), recv_atom.data_ptr(),
-                                   ws_r.data_ptr(), _stream(dev)), "csr_fill(recv)")
+        recv_ghost = torch.empty((total_recv,), dtype=torch.int64, device=dev)
+        _lib.check(L.dynb_halo_lists_fill(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, g2l.data_ptr(), None,
+                                          offs.data_ptr(), n_local, send_local.data_ptr(), recv_atom.data_ptr(), recv_ghost.data_ptr(),
+                                          None, ws.data_ptr(), _stream(dev)), "halo_lists_fill")
         interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
         _lib.check(L.dynb_gather_not_u8(has_remote.data_ptr(), mine.data_ptr(), n_local, interior.data_ptr(), _stream(dev)),
                    "gather_not_u8")
-        recv_ghost = torch.arange(n_local, n_local + total_recv, dtype=torch.int64, device=dev)
-        return offs[0].clone(), send_local, offs[1].clone(), recv_ghost, interior, recv_atom
+        return offs[:W + 1], send_local, offs[W + 1:2 * W + 2], recv_ghost, interior, recv_atom

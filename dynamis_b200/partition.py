@@ -8,7 +8,7 @@ bound in dynamis_state/src/dynamis_state_bindings.cpp:75-115): ``SFCPartitioner(
 The compute is in libdynb.so: Morton/"Hilbert" keys, a stable radix sort, the label assignment
 (dynb_sfc_partition), bincount / stream compaction (dynb_bincount_i64, dynb_select_eq_i64), and
 for the halo maps one cell-scan pass at cutoff + buffer that marks which rank needs which atom
-(dynb_rg_halo_mark) followed by CSR assembly (dynb_csr_plan / dynb_csr_fill).  Unlike the
+(dynb_rg_halo_mark) followed by the assembly of the lists (dynb_halo_lists_plan / _fill).  Unlike the
 reference, no [N, W] bool matrix and no edge list are materialised.
 """
 
@@ -21,7 +21,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .graph import plan_radius_graph, radius_graph_pbc, radius_graph_pbc_ex
+from .graph import BinnedAtoms, radius_graph_pbc, radius_graph_pbc_ex
 from .state import DistEnvironment, MolecularInfo, PartitionMessagePassingInfo, SimulationConfig
 
 PARTITION_MAX_NUM_NEIGHBORS = 1000
@@ -176,40 +176,39 @@ class AbstractPartitioner:
         with _lib.on_device(dev):
             needed = torch.empty((max(N, 1), words), dtype=torch.int32, device=dev)
             has_foreign = torch.empty((max(N, 1),), dtype=torch.uint8, device=dev)
-            if N > 0:
-                plan = plan_radius_graph(pos32, cell, pbc, ghost_cutoff)
-                _lib.check(L.dynb_rg_halo_mark(plan.ws.data_ptr(), plan.dtype_code, pid.data_ptr(), N, W, needed.data_ptr(),
-                                               has_foreign.data_ptr(), _stream(dev)), "rg_halo_mark")
-            my_indices = select_eq(pid, R)
-            n_local = my_indices.numel()
-            g2l = torch.empty((max(N, 1),), dtype=torch.int64, device=dev)
-            bad = scratch(dev, "bad", 256)
-            _lib.check(L.dynb_scatter_iota(my_indices.data_ptr(), n_local, N, g2l.data_ptr(), bad.data_ptr(), _stream(dev)),
-                       "scatter_iota")
             nbytes = ctypes.c_int64()
-            _lib.check(L.dynb_csr_workspace_bytes(N, W, ctypes.byref(nbytes)), "csr_workspace_bytes")
-            ws_s = scratch(dev, "csr_send", nbytes.value)
-            ws_r = scratch(dev, "csr_recv", nbytes.value)
-            offs = torch.empty((2, W + 1), dtype=torch.int64, device=dev)
-            _lib.check(L.dynb_csr_plan(needed.data_ptr(), pid.data_ptr(), N, R, 0, W, offs[0].data_ptr(), ws_s.data_ptr(),
-                                       ws_s.numel(), _stream(dev)), "csr_plan(send)")
-            _lib.check(L.dynb_csr_plan(needed.data_ptr(), pid.data_ptr(), N, R, 1, W, offs[1].data_ptr(), ws_r.data_ptr(),
-                                       ws_r.numel(), _stream(dev)), "csr_plan(recv)")
-            offs_h = offs.cpu()
-            total_send, total_recv = int(offs_h[0, W]), int(offs_h[1, W])
+            _lib.check(L.dynb_halo_lists_workspace_bytes(N, W, ctypes.byref(nbytes)), "halo_lists_workspace_bytes")
+            ws = scratch(dev, "halo_lists", nbytes.value)
+            offs = torch.empty((2 * (W + 1) + 1,), dtype=torch.int64, device=dev)
+            offs_h = torch.empty((2 * (W + 1) + 1,), dtype=torch.int64, pin_memory=True)
+            # everything up to the list sizes is queued before the one wait; the header's status is looked at behind it
+            bins = BinnedAtoms(pos32, cell, pbc, ghost_cutoff) if N > 0 else None
+            while True:
+                if bins is not None:
+                    bins.launch()
+                    mark = scratch(dev, "halo_owner", 2 * (N + bins.src_capacity))
+                    _lib.check(L.dynb_rg_halo_mark(bins.ws.data_ptr(), bins.dtype_code, pid.data_ptr(), N, W, R, needed.data_ptr(),
+                                                   has_foreign.data_ptr(), bins.src_capacity, mark.data_ptr(), mark.numel(),
+                                                   _stream(dev)), "rg_halo_mark")
+                _lib.check(L.dynb_halo_lists_plan(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
+                                                  ws.numel(), _stream(dev)), "halo_lists_plan")
+                offs_h.copy_(offs, non_blocking=True)
+                torch.cuda.current_stream(dev).synchronize()
+                if bins is None or bins.done():
+                    break
+            total_send, total_recv, n_local = int(offs_h[W]), int(offs_h[2 * W + 1]), int(offs_h[2 * W + 2])
             send_local = torch.empty((total_send,), dtype=torch.int64, device=dev)
             recv_atom = torch.empty((total_recv,), dtype=torch.int64, device=dev)
-            _lib.check(L.dynb_csr_fill(needed.data_ptr(), pid.data_ptr(), N, R, 0, W, g2l.data_ptr(), offs[0].data_ptr(),
-                                       send_local.data_ptr(), ws_s.data_ptr(), _stream(dev)), "csr_fill(send)")
-            _lib.check(L.dynb_csr_fill(needed.data_ptr(), pid.data_ptr(), N, R, 1, W, None, offs[1].data_ptr(),
-                                       recv_atom.data_ptr(), ws_r.data_ptr(), _stream(dev)), "csr_fill(recv)")
+            recv_ghost = torch.empty((total_recv,), dtype=torch.int64, device=dev)
             interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
-            _lib.check(L.dynb_gather_not_u8(has_foreign.data_ptr(), my_indices.data_ptr(), n_local, interior.data_ptr(),
-                                            _stream(dev)), "gather_not_u8")
-            info.send_offsets = offs[0].clone()
+            _lib.check(L.dynb_halo_lists_fill(needed.data_ptr(), None, pid.data_ptr(), N, R, W, None, has_foreign.data_ptr(),
+                                              offs.data_ptr(), n_local, send_local.data_ptr(), recv_atom.data_ptr(),
+                                              recv_ghost.data_ptr(), interior.data_ptr(), ws.data_ptr(), _stream(dev)),
+                       "halo_lists_fill")
+            info.send_offsets = offs[:W + 1]
             info.send_local_indices = send_local
-            info.recv_offsets = offs[1].clone()
-            info.recv_ghost_indices = torch.arange(n_local, n_local + total_recv, dtype=torch.int64, device=dev)
+            info.recv_offsets = offs[W + 1:2 * W + 2]
+            info.recv_ghost_indices = recv_ghost
             info.recv_atom_global = recv_atom
             info.interior_mask = interior
             # build_halo_maps.cpp:150-154

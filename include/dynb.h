@@ -101,13 +101,22 @@ int dynb_rg_fill_glue(const void* workspace_dev, int dtype, int64_t* edge_index_
                       const float* cell_host /* [9] */, int negate_shifts, const int64_t* id_map_dev,
                       int64_t E, void* stream);
 
-/* Halo marking over a plan (all atoms as targets, radius = cutoff + ghost buffer): for every edge
- * src -> dst whose endpoints have different owners, sets bit owner[dst] of
- * needed_dev[src * words + ...] (words = ceil(world_size / 32)) and has_foreign_dev[dst] = 1.
- * Both outputs are cleared first.  This is the edge loop of build_halo_maps
- * (dynamis_state/src/csrc/build_halo_maps.cpp:50-58, 127-138) without materialising the graph. */
+/* The part of dynb_rg_plan that halo marking needs: wrap, periodic images, cell-sorted records of all atoms; no degrees.
+ * header_host receives M and the status bits (as the plan: on SRC_OVERFLOW repeat with a larger capacity). */
+int dynb_rg_bin(const void* pos_dev, int dtype, int64_t n_atoms, const void* cell_host, const uint8_t* pbc_host, double radius,
+                void* workspace_dev, int64_t workspace_bytes, int64_t src_capacity, int64_t cell_capacity,
+                dynb_rg_header* header_host, void* stream);
+
+/* Halo marking over a plan (all atoms as targets, radius = cutoff + ghost buffer) or over dynb_rg_bin: for every edge
+ * src -> dst whose endpoints have different owners, sets bit owner[dst] of needed_dev[src * words + ...]
+ * (words = ceil(world_size / 32)) and has_foreign_dev[dst] = 1.  rank >= 0: only for edges that start or end at an
+ * atom of that rank (all its own halo lists need); -1: for every edge.  Both outputs are cleared first.
+ * src_capacity is the one of the plan; scratch_dev holds 2 * (n_atoms + src_capacity) bytes.
+ * This is the edge loop of build_halo_maps (dynamis_state/src/csrc/build_halo_maps.cpp:50-58, 127-138) without
+ * materialising the graph. */
 int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
-                      int64_t world_size, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream);
+                      int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev,
+                      int64_t src_capacity, void* scratch_dev, int64_t scratch_bytes, void* stream);
 
 /* ------------------------------------------------------------------ SFC partition
  * Replaces sfc_partition_cuda (dynamis_state/src/csrc/partition/sfc.cpp:9-33,
@@ -164,19 +173,22 @@ int dynb_halo_mark_from_edges(const int64_t* edges_dev, int64_t E, const int64_t
                               int64_t world_size, uint32_t* send_mask_dev, uint32_t* recv_mask_dev,
                               uint8_t* has_remote_dev, uint32_t* bad_dev, void* stream);
 
-/* CSR assembly (build_halo_maps.cpp:60-125; dist_graph_ops_kernels.cu:143-177).  Element a in
- * [0, n) carries a set of peer ranks; segment p of the output lists, ascending in a, the elements
- * whose set contains p.  mode 0 (send): owner[a] == R ? mask bits without R : {};
- * mode 1 (recv): owner[a] != R and bit R of mask[a] ? {owner[a]} : {};  mode 2: the mask bits.
- * dynb_csr_plan writes offsets_dev [W+1]; after reading offsets[W] the caller allocates out_dev and
- * calls dynb_csr_fill with the same arguments and workspace (value_map_dev[a] is written instead
- * of a when given). */
-int dynb_csr_workspace_bytes(int64_t n, int64_t W, int64_t* bytes);
-int dynb_csr_plan(const uint32_t* mask_dev, const int64_t* owner_dev, int64_t n, int64_t R, int mode, int64_t W,
-                  int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream);
-int dynb_csr_fill(const uint32_t* mask_dev, const int64_t* owner_dev, int64_t n, int64_t R, int mode, int64_t W,
-                  const int64_t* value_map_dev, const int64_t* offsets_dev, int64_t* out_dev,
-                  const void* workspace_dev, void* stream);
+/* Send and recv lists of one rank (build_halo_maps.cpp:60-125; dist_graph_ops_kernels.cu:143-177).  Atom a in [0, n)
+ * carries two sets of peer ranks; segment p of the send (recv) list holds, ascending in a, the atoms whose send (recv)
+ * set contains p.  owner_dev == NULL: the sets are the bits of the two masks ([n, ceil(W/32)] uint32).  owner_dev given:
+ * send_mask_dev is the "needed by" mask of dynb_rg_halo_mark (recv_mask_dev is not read), an own atom (owner == R) is sent
+ * to the ranks that need it, a foreign one is received from its owner when R needs it.
+ * dynb_halo_lists_plan writes offsets_dev: send [W+1], recv [W+1], number of own atoms.  After reading them the caller
+ * allocates the outputs and calls dynb_halo_lists_fill with the same arguments and workspace: send_local_dev (local index
+ * of an own atom, or value_map_dev[a] without owners), recv_atom_dev (a), recv_ghost_dev (n_local + place in the list),
+ * and, with owners, interior_dev[local index] = !has_foreign_dev[a]. */
+int dynb_halo_lists_workspace_bytes(int64_t n, int64_t W, int64_t* bytes);
+int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
+                         int64_t R, int64_t W, int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream);
+int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
+                         int64_t R, int64_t W, const int64_t* value_map_dev, const uint8_t* has_foreign_dev,
+                         const int64_t* offsets_dev, int64_t n_local, int64_t* send_local_dev, int64_t* recv_atom_dev,
+                         int64_t* recv_ghost_dev, uint8_t* interior_dev, const void* workspace_dev, void* stream);
 /* interior_mask[i] = !flags[idx[i]] (build_halo_maps.cpp:138). */
 int dynb_gather_not_u8(const uint8_t* flags_dev, const int64_t* idx_dev, int64_t n, uint8_t* out_dev, void* stream);
 /* g2l[idx[i]] = i (dist_graph_ops_kernels.cu:143-144). */
@@ -187,7 +199,8 @@ int dynb_scatter_iota(const int64_t* idx_dev, int64_t n, int64_t N, int64_t* g2l
  * dist_graph_ops_kernels.cu:16-43, 62-102): keeps edge e iff
  * |pos[src] + shift @ cell - pos[dst]|^2 <= radius^2 (float32), order preserving.  The plan writes
  * the number kept to count_dev; the fill compacts edges [2,E] -> [2,E_out] and the shift rows of
- * any element size (shift_row_bytes = 3 * element size).  Workspace: dynb_select_workspace_bytes(2*E). */
+ * any element size (shift_row_bytes = 3 * element size). */
+int dynb_filter_edges_workspace_bytes(int64_t E, int64_t* bytes);
 int dynb_filter_edges_plan(const int64_t* edges_dev, const float* shifts_f32_dev, const float* pos_dev,
                            const float* cell_host, double radius, int64_t E, int64_t* count_dev,
                            void* workspace_dev, int64_t workspace_bytes, void* stream);

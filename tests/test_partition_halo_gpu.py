@@ -297,3 +297,32 @@ def test_halo_ops_vs_reference_kernels(cuda, ref_ops):
         fe, fs = D.filter_edges_to_radius(ei, cs, tp, tc, 6.0)
         re_, rs = ref_ops.filter_edges(ei, cs, tp, tc.to(cuda), 6.0)
         assert torch.equal(fe, re_) and torch.equal(fs, rs)
+
+
+@pytest.mark.parametrize("n,L,W,spatial", [(1, 30.0, 3, True), (1023, 24.0, 2, True), (1025, 24.0, 32, False), (2049, 20.0, 33, True),
+                                           (3000, 12.0, 5, False), (4000, 40.0, 70, False)])
+def test_halo_lists_at_tile_edges(cuda, n, L, W, spatial):
+    """Sizes around the tile of the list passes, more than 32 ranks, owners without any spatial order (every candidate can
+    matter, so candidate batches fill up) and dense cells (more targets in a group than are tested together)."""
+    rng = np.random.default_rng(n + W)
+    pos = (rng.random((n, 3)) * L).astype(np.float32)
+    cell = (np.eye(3) * L).astype(np.float32)
+    owner = np.minimum((pos[:, 0] / (L / W)).astype(np.int64), W - 1) if spatial else rng.integers(0, W, n)
+    g = O.radius_graph(pos, cell, [1, 1, 1], np.float32(5.5))
+    for r in {0, W // 2, W - 1}:
+        info = D.PartitionMessagePassingInfo()
+        info.partition_id = torch.as_tensor(owner, device=cuda)
+        D.SFCPartitioner().build_halo_maps(info, _state(pos, cuda), _env(r, W), _cfg(cell, 5.0, 0.5))
+        ref = O.build_halo_maps(g["src"], g["dst"], owner, r, W)
+        for key in ("send_offsets", "send_local_indices", "recv_offsets", "recv_ghost_indices", "recv_atom_global", "interior_mask"):
+            np.testing.assert_array_equal(getattr(info, key).cpu().numpy(), ref[key])
+
+
+@pytest.mark.parametrize("n", [1, 255, 2047, 2048, 2049, 70_001])
+def test_select_eq_at_tile_edges(cuda, n):
+    from dynamis_b200.partition import select_eq
+
+    v = torch.randint(0, 3, (n,), device=cuda, generator=torch.Generator(device=cuda).manual_seed(n))
+    src = torch.arange(n, device=cuda) * 7
+    assert torch.equal(select_eq(v, 1), torch.nonzero(v == 1).reshape(-1))
+    assert torch.equal(select_eq(v, 2, src), src[v == 2])
