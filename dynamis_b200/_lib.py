@@ -84,7 +84,7 @@ SIGNATURES = {
     "dynb_rg_fill": (_i32, [_p, _i32, _p, _p, _p, _i64, _p]),
     "dynb_rg_fill_glue": (_i32, [_p, _i32, _p, _p, _p, _p, _i32, _p, _i64, _p]),
     "dynb_rg_bin": (_i32, [_p, _i32, _i64, _p, _p, _f64, _p, _i64, _i64, _i64, _p, _p]),
-    "dynb_rg_halo_mark": (_i32, [_p, _i32, _p, _i64, _i64, _i64, _p, _p, _i64, _p, _i64, _p]),
+    "dynb_rg_halo_mark": (_i32, [_p, _i32, _p, _i64, _i64, _i64, _p, _p, _i64, _i64, _p, _i64, _p]),
     "dynb_sfc_workspace_bytes": (_i32, [_i64, ctypes.POINTER(_i64)]),
     "dynb_sfc_partition": (_i32, [_p, _i64, _p, _i64, _i32, _p, _p, _p, _i64, _p]),
     "dynb_sfc_keys": (_i32, [_p, _i64, _i32, _p, _p, _i64, _p]),
@@ -99,7 +99,7 @@ SIGNATURES = {
     "dynb_halo_mark_from_edges": (_i32, [_p, _i64, _p, _i64, _i64, _i64, _p, _p, _p, _p, _p]),
     "dynb_halo_lists_workspace_bytes": (_i32, [_i64, _i64, ctypes.POINTER(_i64)]),
     "dynb_halo_lists_plan": (_i32, [_p, _p, _p, _i64, _i64, _i64, _p, _p, _i64, _p]),
-    "dynb_halo_lists_fill": (_i32, [_p, _p, _p, _i64, _i64, _i64, _p, _p, _p, _i64, _p, _p, _p, _p, _p, _p]),
+    "dynb_halo_lists_fill": (_i32, [_p, _p, _p, _i64, _i64, _i64, _p, _p, _p, _i64, _p, _p, _p, _p, _p, _p, _p]),
     "dynb_gather_not_u8": (_i32, [_p, _p, _i64, _p, _p]),
     "dynb_scatter_iota": (_i32, [_p, _i64, _i64, _p, _p, _p]),
     "dynb_filter_edges_workspace_bytes": (_i32, [_i64, ctypes.POINTER(_i64)]),
@@ -160,6 +160,14 @@ def check(rc: int, what: str = "") -> None:
         msg = lib().dynb_last_error()
         text = msg.decode() if msg else ""
         raise RuntimeError(f"dynb {what} failed (code {rc}): {text}")
+
+
+def stream_of(dev) -> int:
+    """Handle of the current stream of ``dev`` (``torch.cuda.current_stream`` builds a Stream object per call, which
+    costs more host time than a kernel launch)."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(dev.index if dev.index is not None else torch.cuda.current_device())
 
 
 class _NoSwitch:

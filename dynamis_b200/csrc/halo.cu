@@ -142,7 +142,7 @@ halo_mark_edges_kernel(const int64_t* __restrict__ src, const int64_t* __restric
 //
 // Both lists, the local indices and the interior mask come out of one counting and one writing pass over the masks; most
 // atoms have empty sets, so a warp (128 consecutive atoms, 32 at a time) works on the peers that occur and on no others.
-// One million atoms, 8 ranks: 8 + 6 + 9 us (count, row scan, fill), where per-list passes that walked all peers took 120.
+// One million atoms, 8 ranks: 9 + 10 + 18 us (count, row scan, fill), where per-list passes that walked all peers took 120.
 constexpr int HL_THREADS = 256;
 constexpr int HL_WARPS = HL_THREADS / 32;
 constexpr int HL_ROUNDS = 4;
@@ -156,23 +156,33 @@ struct HaloSets {
     int words;
 };
 
-__device__ __forceinline__ void halo_sets(const HaloSets& h, int64_t a, int word, uint32_t& s, uint32_t& r, bool& own)
+// the sets of this lane's HL_ROUNDS atoms (base, base + 32, ...) among the 32 peers of one mask word; all loads first
+__device__ __forceinline__ void halo_sets(const HaloSets& h, int64_t base, int word, uint32_t (&s)[HL_ROUNDS], uint32_t (&r)[HL_ROUNDS],
+                                          uint32_t& own)
 {
-    s = r = 0u;
-    own = false;
-    if (a >= h.n) return;
-    if (h.owner == nullptr) {
-        s = h.send_mask[a * h.words + word];
-        r = h.recv_mask[a * h.words + word];
-        return;
+    uint32_t mw[HL_ROUNDS], mr[HL_ROUNDS];
+    int64_t o[HL_ROUNDS];
+    const bool owners = h.owner != nullptr;
+    const uint32_t* second = owners ? h.send_mask + (h.me >> 5) : h.recv_mask + word;
+#pragma unroll
+    for (int k = 0; k < HL_ROUNDS; k++) {
+        const int64_t a = base + 32 * k;
+        const bool live = a < h.n;
+        mw[k] = live ? h.send_mask[a * h.words + word] : 0u;
+        mr[k] = live ? second[a * h.words] : 0u;
+        o[k] = (live && owners) ? h.owner[a] : -1;
     }
-    const int64_t o = h.owner[a];
-    own = o == h.me;
-    if (own) {
-        s = h.send_mask[a * h.words + word];
-        if (word == (int)(h.me >> 5)) s &= ~(1u << (h.me & 31));
-    } else if ((int)(o >> 5) == word && ((h.send_mask[a * h.words + (h.me >> 5)] >> (h.me & 31)) & 1u)) {
-        r = 1u << (o & 31);
+    own = 0u;
+#pragma unroll
+    for (int k = 0; k < HL_ROUNDS; k++) {
+        s[k] = mw[k];
+        r[k] = mr[k];
+        if (owners) {
+            const bool mine = o[k] == h.me;
+            if (mine) own |= 1u << k;
+            s[k] = !mine ? 0u : (word == (int)(h.me >> 5) ? mw[k] & ~(1u << (h.me & 31)) : mw[k]);
+            r[k] = (!mine && (int)(o[k] >> 5) == word && ((mr[k] >> (h.me & 31)) & 1u)) ? 1u << (o[k] & 31) : 0u;
+        }
     }
 }
 
@@ -197,16 +207,14 @@ halo_lists_count_kernel(const HaloSets h, int W, int nblocks, uint32_t* __restri
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t base = (int64_t)blockIdx.x * HL_TILE + warp * 32 * HL_ROUNDS + lane;
     for (int word = 0; word < h.words; word++) {
-        uint32_t cs = 0, cr = 0, co = 0;
+        uint32_t s[HL_ROUNDS], r[HL_ROUNDS], own, cs = 0, cr = 0;
+        halo_sets(h, base, word, s, r, own);
 #pragma unroll
         for (int k = 0; k < HL_ROUNDS; k++) {
-            uint32_t s, r;
-            bool own;
-            halo_sets(h, base + 32 * k, word, s, r, own);
-            cs += halo_count_sets(s, lane);
-            cr += halo_count_sets(r, lane);
-            co += __popc(__ballot_sync(0xffffffffu, own));
+            cs += halo_count_sets(s[k], lane);
+            cr += halo_count_sets(r[k], lane);
         }
+        const uint32_t co = __reduce_add_sync(0xffffffffu, __popc(own));
         __syncthreads();
         ws[warp][0][lane] = cs;
         ws[warp][1][lane] = cr;
@@ -275,6 +283,7 @@ struct HaloListsOut {
     int64_t* recv_atom;
     int64_t* recv_ghost;
     uint8_t* interior;           // by local index; with the owners given
+    int64_t* matrix_row;         // [W] rows sent to every rank, n_local at the own place; or nullptr
     int64_t n_local;
 };
 
@@ -287,13 +296,14 @@ halo_lists_fill_kernel(const HaloSets h, int W, int nblocks, const uint32_t* __r
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = lanemask_lt();
     const int64_t base = (int64_t)blockIdx.x * HL_TILE + warp * 32 * HL_ROUNDS + lane;
+    if (blockIdx.x == 0 && out.matrix_row != nullptr)
+        for (int p = threadIdx.x; p < W; p += HL_THREADS) out.matrix_row[p] = p == (int)h.me ? out.n_local : offsets[p + 1] - offsets[p];
     for (int word = 0; word < h.words; word++) {
-        uint32_t set[2][HL_ROUNDS], own[HL_ROUNDS], c[2] = {0u, 0u}, co = 0;
+        uint32_t set[2][HL_ROUNDS], mine_own, own[HL_ROUNDS], c[2] = {0u, 0u}, co = 0;
+        halo_sets(h, base, word, set[0], set[1], mine_own);
 #pragma unroll
         for (int k = 0; k < HL_ROUNDS; k++) {
-            bool o;
-            halo_sets(h, base + 32 * k, word, set[0][k], set[1][k], o);
-            own[k] = __ballot_sync(0xffffffffu, o);
+            own[k] = __ballot_sync(0xffffffffu, (mine_own >> k) & 1u);
             c[0] += halo_count_sets(set[0][k], lane);
             c[1] += halo_count_sets(set[1][k], lane);
             co += __popc(own[k]);
@@ -521,7 +531,8 @@ extern "C" int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_
 extern "C" int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
                                     int64_t R, int64_t W, const int64_t* value_map_dev, const uint8_t* has_foreign_dev,
                                     const int64_t* offsets_dev, int64_t n_local, int64_t* send_local_dev, int64_t* recv_atom_dev,
-                                    int64_t* recv_ghost_dev, uint8_t* interior_dev, const void* workspace_dev, void* stream)
+                                    int64_t* recv_ghost_dev, uint8_t* interior_dev, int64_t* matrix_row_dev,
+                                    const void* workspace_dev, void* stream)
 {
     HaloSets h;
     int rc = halo_lists_args(send_mask_dev, recv_mask_dev, owner_dev, n, R, W, h);
@@ -530,7 +541,7 @@ extern "C" int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_
     if (offsets_dev == nullptr || workspace_dev == nullptr || (owner_dev == nullptr && value_map_dev == nullptr) ||
         (owner_dev != nullptr && has_foreign_dev == nullptr))
         return fail_arg("null pointer");
-    const HaloListsOut out{value_map_dev, has_foreign_dev, send_local_dev, recv_atom_dev, recv_ghost_dev, interior_dev, n_local};
+    const HaloListsOut out{value_map_dev, has_foreign_dev, send_local_dev, recv_atom_dev, recv_ghost_dev, interior_dev, matrix_row_dev, n_local};
     const int nb = hl_blocks(n);
     halo_lists_fill_kernel<<<nb, HL_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(h, (int)W, nb, static_cast<const uint32_t*>(workspace_dev),
                                                                                    offsets_dev, out);

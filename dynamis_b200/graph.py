@@ -28,7 +28,7 @@ def _dev_state(device: torch.device) -> dict:
     """Plan workspace and pinned header of one (device, stream): calls on different streams of a device get
     workspaces of their own and so cannot race on one; calls on one stream are ordered by the stream."""
     index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (device.type, index, torch.cuda.current_stream(torch.device("cuda", index)).cuda_stream)
+    key = (index, _lib.stream_of(device))
     st = _STATE.get(key)
     if st is None:
         pinned = torch.empty(64, dtype=torch.uint8).pin_memory()
@@ -195,7 +195,7 @@ class BinnedAtoms:
         self.attempts += 1
         _lib.check(L.dynb_rg_bin(self.pos.data_ptr(), self.dtype_code, N, self.cell_h.ctypes.data, self.pbc_h.ctypes.data, self.radius,
                                  self.ws.data_ptr(), self.ws.numel(), self.src_capacity, self.cell_capacity, self.hdr_t.data_ptr(),
-                                 torch.cuda.current_stream(dev).cuda_stream), "rg_bin")
+                                 _lib.stream_of(dev)), "rg_bin")
 
     def done(self) -> bool:
         status = int(self.hdr.status)

@@ -50,7 +50,7 @@ def filter_edges_to_radius(edges: torch.Tensor, cell_shifts: torch.Tensor, pos: 
     cell_h = np.ascontiguousarray(cell.detach().to("cpu", torch.float32).numpy())
     shifts_f = cell_shifts if cell_shifts.dtype == torch.float32 else cell_shifts.to(torch.float32)
     L = _lib.lib()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_filter_edges_workspace_bytes(E, ctypes.byref(nbytes)), "filter_edges_workspace_bytes")
         ws = scratch(dev, "filter", nbytes.value)
@@ -98,7 +98,7 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
     n_local = mine.numel()
     words = (W + 31) // 32
     L = _lib.lib()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         send_mask = torch.empty((max(N, 1), words), dtype=torch.int32, device=dev)
         recv_mask = torch.empty((max(N, 1), words), dtype=torch.int32, device=dev)
         has_remote = torch.empty((max(N, 1),), dtype=torch.uint8, device=dev)
@@ -123,7 +123,7 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
         recv_ghost = torch.empty((total_recv,), dtype=torch.int64, device=dev)
         _lib.check(L.dynb_halo_lists_fill(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, g2l.data_ptr(), None,
                                           offs.data_ptr(), n_local, send_local.data_ptr(), recv_atom.data_ptr(), recv_ghost.data_ptr(),
-                                          None, ws.data_ptr(), _stream(dev)), "halo_lists_fill")
+                                          None, None, ws.data_ptr(), _stream(dev)), "halo_lists_fill")
         interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
         _lib.check(L.dynb_gather_not_u8(has_remote.data_ptr(), mine.data_ptr(), n_local, interior.data_ptr(), _stream(dev)),
                    "gather_not_u8")

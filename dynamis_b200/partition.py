@@ -18,6 +18,7 @@ import ctypes
 import enum
 from typing import Optional
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -33,7 +34,7 @@ _SCRATCH: dict = {}
 def scratch(device: torch.device, name: str, nbytes: int) -> torch.Tensor:
     """Grow-only named device scratch buffers (uint8), one set per (device, stream): work on different streams of
     a device never shares one."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream, name)
+    key = (device.index, _lib.stream_of(device), name)
     buf = _SCRATCH.get(key)
     if buf is None or buf.numel() < nbytes:
         _SCRATCH.pop(key, None)
@@ -42,8 +43,7 @@ def scratch(device: torch.device, name: str, nbytes: int) -> torch.Tensor:
     return buf
 
 
-def _stream(dev):
-    return torch.cuda.current_stream(dev).cuda_stream
+_stream = _lib.stream_of
 
 
 class SFCCurveType(enum.IntEnum):
@@ -123,25 +123,29 @@ def bincount_labels(labels: torch.Tensor, W: int) -> torch.Tensor:
     return counts
 
 
-def select_eq(values: torch.Tensor, value: int, gather_src: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``gather_src[nonzero(values == value)]`` (or the positions themselves), ascending.  One host sync."""
+def select_eq(values: torch.Tensor, value: int, gather_src: Optional[torch.Tensor] = None,
+              count: Optional[int] = None) -> torch.Tensor:
+    """``gather_src[nonzero(values == value)]`` (or the positions themselves), ascending.  One host sync, none when the
+    caller knows how many there are (``count``)."""
     dev = values.device
     n = values.numel()
     L = _lib.lib()
     with _lib.on_device(dev):
-        out = torch.empty((n,), dtype=torch.int64, device=dev)
+        out = torch.empty((n if count is None else count,), dtype=torch.int64, device=dev)
         cnt = torch.empty((1,), dtype=torch.int64, device=dev)
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_select_workspace_bytes(n, ctypes.byref(nbytes)), "select_workspace_bytes")
         ws = scratch(dev, "select", nbytes.value)
         _lib.check(L.dynb_select_eq_i64(values.data_ptr(), n, int(value), gather_src.data_ptr() if gather_src is not None else None,
                                         out.data_ptr(), cnt.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev)), "select_eq")
-        k = int(cnt.item())
+        k = int(cnt.item()) if count is None else count
     return out[:k]
 
 
-def _finish_partition(labels: torch.Tensor, state: MolecularInfo, env: DistEnvironment) -> PartitionMessagePassingInfo:
-    """partition_indices / atom_counts / matrix from the labels (sfc_partitioner.cpp:164-178)."""
+def _finish_partition(labels: torch.Tensor, state: MolecularInfo, env: DistEnvironment,
+                      n_local: Optional[int] = None) -> PartitionMessagePassingInfo:
+    """partition_indices / atom_counts / matrix from the labels (sfc_partitioner.cpp:164-178).  ``n_local``: the number of
+    atoms with this rank's label where it is known beforehand (saves the wait for it)."""
     info = PartitionMessagePassingInfo()
     W, R = int(env.world_size), int(env.global_rank)
     dev = labels.device
@@ -149,7 +153,7 @@ def _finish_partition(labels: torch.Tensor, state: MolecularInfo, env: DistEnvir
     info.atom_counts = bincount_labels(labels, W)
     vn = state.atom_vertex_numbers
     vn = vn.to(device=dev, dtype=torch.int64).contiguous() if vn is not None else None
-    info.partition_indices = select_eq(labels, R, vn)
+    info.partition_indices = select_eq(labels, R, vn, n_local)
     m = torch.zeros((W, W), dtype=torch.int64, device=dev)
     m[R, R] = info.partition_indices.numel()
     info.global_send_recv_matrix = m
@@ -166,7 +170,7 @@ class AbstractPartitioner:
             raise RuntimeError("pos must be a CUDA tensor")
         dev = pos.device
         N, W, R = int(global_state.num_atoms), int(env.world_size), int(env.global_rank)
-        ghost_cutoff = float(torch.tensor(config.cutoff + config.ghost_cutoff_buffer, dtype=torch.float32).item())
+        ghost_cutoff = float(np.float32(config.cutoff + config.ghost_cutoff_buffer))
         pos32 = pos.to(torch.float32).contiguous()
         cell = config.cell.to(torch.float32)
         pbc = config.pbc.to(torch.bool)
@@ -186,10 +190,10 @@ class AbstractPartitioner:
             while True:
                 if bins is not None:
                     bins.launch()
-                    mark = scratch(dev, "halo_owner", 2 * (N + bins.src_capacity))
+                    mark = scratch(dev, "halo_owner", 2 * (N + bins.src_capacity + bins.cell_capacity))
                     _lib.check(L.dynb_rg_halo_mark(bins.ws.data_ptr(), bins.dtype_code, pid.data_ptr(), N, W, R, needed.data_ptr(),
-                                                   has_foreign.data_ptr(), bins.src_capacity, mark.data_ptr(), mark.numel(),
-                                                   _stream(dev)), "rg_halo_mark")
+                                                   has_foreign.data_ptr(), bins.src_capacity, bins.cell_capacity,
+                                                   mark.data_ptr(), mark.numel(), _stream(dev)), "rg_halo_mark")
                 _lib.check(L.dynb_halo_lists_plan(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
                                                   ws.numel(), _stream(dev)), "halo_lists_plan")
                 offs_h.copy_(offs, non_blocking=True)
@@ -201,21 +205,22 @@ class AbstractPartitioner:
             recv_atom = torch.empty((total_recv,), dtype=torch.int64, device=dev)
             recv_ghost = torch.empty((total_recv,), dtype=torch.int64, device=dev)
             interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
+            matrix = info.global_send_recv_matrix
+            if matrix is None or matrix.device != dev or matrix.dtype != torch.int64 or not matrix.is_contiguous() or N == 0:
+                kept, matrix = matrix, torch.zeros((W, W), dtype=torch.int64, device=dev)
+                if kept is not None:
+                    matrix.copy_(kept)
+                info.global_send_recv_matrix = matrix
             _lib.check(L.dynb_halo_lists_fill(needed.data_ptr(), None, pid.data_ptr(), N, R, W, None, has_foreign.data_ptr(),
                                               offs.data_ptr(), n_local, send_local.data_ptr(), recv_atom.data_ptr(),
-                                              recv_ghost.data_ptr(), interior.data_ptr(), ws.data_ptr(), _stream(dev)),
-                       "halo_lists_fill")
+                                              recv_ghost.data_ptr(), interior.data_ptr(), matrix[R].data_ptr(), ws.data_ptr(),
+                                              _stream(dev)), "halo_lists_fill")
             info.send_offsets = offs[:W + 1]
             info.send_local_indices = send_local
             info.recv_offsets = offs[W + 1:2 * W + 2]
             info.recv_ghost_indices = recv_ghost
             info.recv_atom_global = recv_atom
             info.interior_mask = interior
-            # build_halo_maps.cpp:150-154
-            if info.global_send_recv_matrix is None:
-                info.global_send_recv_matrix = torch.zeros((W, W), dtype=torch.int64, device=dev)
-            info.global_send_recv_matrix[R] = info.send_offsets[1:] - info.send_offsets[:-1]
-            info.global_send_recv_matrix[R, R] = n_local
         info.edge_index_halo = None
         info._edge_index_halo_fn = lambda: radius_graph_pbc(pos32, cell, pbc, ghost_cutoff, HALO_MAX_NUM_NEIGHBORS, False)[0]
 
@@ -235,9 +240,12 @@ class SFCPartitioner(AbstractPartitioner):
         pos32 = pos.to(torch.float32)
         if config is None:
             labels = sfc_partition_labels(pos32, state.edge_counts, W, int(self.curve_type))
-            return _finish_partition(labels, state, env)
+            # equal counts: the first N % W ranks hold one atom more (sfc_kernels.cu:123-134)
+            N = pos32.size(0)
+            n_local = N // W + (1 if int(env.global_rank) < N % W else 0) if state.edge_counts is None else None
+            return _finish_partition(labels, state, env, n_local)
         # mode 3: weights = in-degree at the cutoff; the graph is kept for downstream use
-        cutoff = float(torch.tensor(config.cutoff, dtype=torch.float32).item())
+        cutoff = float(np.float32(config.cutoff))
         cell = config.cell.to(torch.float32)
         ei, _, _, counts = radius_graph_pbc_ex(pos32, cell, config.pbc.to(torch.bool), cutoff, PARTITION_MAX_NUM_NEIGHBORS, False)
         labels = sfc_partition_labels(pos32, counts.to(torch.int64), W, int(self.curve_type))
@@ -293,7 +301,7 @@ class KDTreePartitioner(AbstractPartitioner):
         if config is None:
             labels = kdtree_partition_labels(pos32, state.edge_counts, W)
             return _finish_partition(labels, state, env)
-        cutoff = float(torch.tensor(config.cutoff, dtype=torch.float32).item())
+        cutoff = float(np.float32(config.cutoff))
         cell = config.cell.to(torch.float32)
         ei, _, _, counts = radius_graph_pbc_ex(pos32, cell, config.pbc.to(torch.bool), cutoff, PARTITION_MAX_NUM_NEIGHBORS, False)
         labels = kdtree_partition_labels(pos32, counts.to(torch.int64), W)

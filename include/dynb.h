@@ -111,12 +111,12 @@ int dynb_rg_bin(const void* pos_dev, int dtype, int64_t n_atoms, const void* cel
  * src -> dst whose endpoints have different owners, sets bit owner[dst] of needed_dev[src * words + ...]
  * (words = ceil(world_size / 32)) and has_foreign_dev[dst] = 1.  rank >= 0: only for edges that start or end at an
  * atom of that rank (all its own halo lists need); -1: for every edge.  Both outputs are cleared first.
- * src_capacity is the one of the plan; scratch_dev holds 2 * (n_atoms + src_capacity) bytes.
+ * The capacities are those of the plan; scratch_dev holds 2 * (n_atoms + src_capacity + cell_capacity) bytes.
  * This is the edge loop of build_halo_maps (dynamis_state/src/csrc/build_halo_maps.cpp:50-58, 127-138) without
  * materialising the graph. */
 int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
                       int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev,
-                      int64_t src_capacity, void* scratch_dev, int64_t scratch_bytes, void* stream);
+                      int64_t src_capacity, int64_t cell_capacity, void* scratch_dev, int64_t scratch_bytes, void* stream);
 
 /* ------------------------------------------------------------------ SFC partition
  * Replaces sfc_partition_cuda (dynamis_state/src/csrc/partition/sfc.cpp:9-33,
@@ -181,14 +181,15 @@ int dynb_halo_mark_from_edges(const int64_t* edges_dev, int64_t E, const int64_t
  * dynb_halo_lists_plan writes offsets_dev: send [W+1], recv [W+1], number of own atoms.  After reading them the caller
  * allocates the outputs and calls dynb_halo_lists_fill with the same arguments and workspace: send_local_dev (local index
  * of an own atom, or value_map_dev[a] without owners), recv_atom_dev (a), recv_ghost_dev (n_local + place in the list),
- * and, with owners, interior_dev[local index] = !has_foreign_dev[a]. */
+ * and, with owners, interior_dev[local index] = !has_foreign_dev[a].  matrix_row_dev (optional, may be NULL): [W] rows
+ * sent to every rank, n_local at the own place (build_halo_maps.cpp:150-154). */
 int dynb_halo_lists_workspace_bytes(int64_t n, int64_t W, int64_t* bytes);
 int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
                          int64_t R, int64_t W, int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream);
 int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
                          int64_t R, int64_t W, const int64_t* value_map_dev, const uint8_t* has_foreign_dev,
                          const int64_t* offsets_dev, int64_t n_local, int64_t* send_local_dev, int64_t* recv_atom_dev,
-                         int64_t* recv_ghost_dev, uint8_t* interior_dev, const void* workspace_dev, void* stream);
+                         int64_t* recv_ghost_dev, uint8_t* interior_dev, int64_t* matrix_row_dev, const void* workspace_dev, void* stream);
 /* interior_mask[i] = !flags[idx[i]] (build_halo_maps.cpp:138). */
 int dynb_gather_not_u8(const uint8_t* flags_dev, const int64_t* idx_dev, int64_t n, uint8_t* out_dev, void* stream);
 /* g2l[idx[i]] = i (dist_graph_ops_kernels.cu:143-144). */
