@@ -63,6 +63,8 @@ struct DevHeader {
     double clip_lo[3];  // source images outside [clip_lo, clip_hi] cannot reach any target and are dropped
     double clip_hi[3];
     uint32_t active_groups;  // entries of the list of groups that hold targets (target subsets only)
+    float test_near, test_lo, test_hi;  // double positions: thresholds of the float test (float_test)
+    uint32_t test_equal_is_near;
     uint32_t long_groups;    // entries of the list of groups whose candidate list is too long for the hit bits
 };
 static_assert(offsetof(DevHeader, ncell_plus1) == sizeof(dynb_rg_header), "public header prefix mismatch");
@@ -678,6 +680,39 @@ __device__ __forceinline__ uint32_t pack_shift_code(int ex, int ey, int ez)
     return (uint32_t)(ex + 512) | ((uint32_t)(ey + 512) << 10) | ((uint32_t)(ez + 512) << 20);
 }
 
+// Coordinates as the count pass tests them: float positions as they are, double positions as floats from the grid's origin.
+__device__ __forceinline__ float scan_coord(float x, double) { return x; }
+__device__ __forceinline__ float scan_coord(double x, double origin) { return (float)(x - origin); }
+
+// The count pass in double precision tests floats first.  A float distance d from coordinates relative to the grid's origin
+// (scan_coord) decides a pair when it lies clear of the cutoff; the few others are tested on the double records:
+//   lo >= d > near: a neighbour;   d > hi: none;   else the double test decides (exact_hits).
+// With u = 2^-24 and X the largest coordinate a difference of two coordinates is off by at most eta = 2 u X, so for
+// |delta| near t the float result differs from the true t^2 by less than 2 sqrt(3) t eta + 6 u t^2 + 3 (eta + u t)^2
+// (conversion, three subtractions, three roundings of the sum); twice that is the margin around r^2 and above the
+// self-distance limit.  The thresholds are rounded outwards, a distance that is not a number is never decided here, and
+// coordinates near the end of the float range are left to the double test altogether.
+// Two records with the same three floats lie within 2 u X of one another along each axis: when that puts them inside the
+// self-distance limit, an undecided pair of equal floats (every target meets itself) is no neighbour and needs no double test.
+// 500 k atoms of silicon, 6 A: 364 -> 228 us (32-byte candidates in chunks of 160 and a double test for each of them before;
+// now all 512 places in one chunk and the packed float test, a double test for about one candidate in 10^5).
+__device__ __forceinline__ void float_test(double r2, double X, float& near, float& lo, float& hi, uint32_t& equal_is_near)
+{
+    const double u = 5.9604644775390625e-8, eta = 2.0 * u * X, eps = (double)1e-8f;
+    double margin[2];
+    const double t2[2] = {eps, r2};
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double t = sqrt(t2[k]), e = eta + u * t;
+        margin[k] = 2.0 * (3.5 * t * eta + 6.0 * u * t2[k] + 3.0 * e * e);
+    }
+    const bool in_range = X < 1.0e15 && r2 < 1.0e30;
+    near = __double2float_ru(eps + margin[0]);
+    lo = in_range ? __double2float_rd(r2 - margin[1]) : -1.0f;
+    hi = in_range ? __double2float_ru(r2 + margin[1]) : __int_as_float(0x7f800000);
+    equal_is_near = 3.1 * eta * eta < eps ? 1u : 0u;
+}
+
 // Deterministic order inside each cell (ascending key) and the packed records.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -686,9 +721,13 @@ rg_bin_finalize_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ target
                        DevHeader* __restrict__ hp, const uint32_t* __restrict__ cstart,
                        const uint32_t* __restrict__ tcstart, const uint4* __restrict__ srec, const uint2* __restrict__ trec,
                        Vec4<T>* __restrict__ spos, float* __restrict__ sxyz, long long sxyz_stride,
-                       uint32_t* __restrict__ scode, uint2* __restrict__ smeta, Vec4<T>* __restrict__ tpos, int4* __restrict__ tmeta)
+                       uint32_t* __restrict__ scode, uint2* __restrict__ smeta, Vec4<T>* __restrict__ tpos, float4* __restrict__ tscan,
+                       int4* __restrict__ tmeta, double r2)
 {
     if (hp->status & RG_FATAL) return;
+    if (sizeof(T) == 8 && blockIdx.x == 0 && threadIdx.x == 0)
+        float_test(r2, 1.01 * (double)max(hp->nx, max(hp->ny, hp->nz)) / hp->res_inv + 0.02, hp->test_near, hp->test_lo, hp->test_hi,
+                   hp->test_equal_is_near);
     const unsigned long long M = hp->M;
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool has_s = j < (int64_t)M, has_t = j < Nt;
@@ -734,11 +773,9 @@ rg_bin_finalize_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ target
         r.w = bits_to_real((int32_t)atom, T());
         const uint32_t at = sb + rank;
         spos[at] = r;
-        if (sizeof(T) == 4 && sxyz != nullptr) {
-            sxyz[at] = (float)r.x;
-            sxyz[sxyz_stride + at] = (float)r.y;
-            sxyz[2 * sxyz_stride + at] = (float)r.z;
-        }
+        sxyz[at] = scan_coord(r.x, hp->gmin[0]);
+        sxyz[sxyz_stride + at] = scan_coord(r.y, hp->gmin[1]);
+        sxyz[2 * sxyz_stride + at] = scan_coord(r.z, hp->gmin[2]);
         const int ex = dx - sff.x, ey = dy - sff.y, ez = dz - sff.z;
         uint32_t packed = pack_shift_code(0, 0, 0);
         if (ex < -511 || ex > 511 || ey < -511 || ey > 511 || ez < -511 || ez > 511) atomicOr(&hp->status, DYNB_RG_SHIFT_RANGE);
@@ -753,6 +790,9 @@ rg_bin_finalize_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ target
         Vec4<T> r;
         r.x = tw.x; r.y = tw.y; r.z = tw.z; r.w = bits_to_real((int32_t)ent, T());
         tpos[tb + rank] = r;
+        if (sizeof(T) == 8)
+            tscan[tb + rank] = make_float4(scan_coord(tw.x, hp->gmin[0]), scan_coord(tw.y, hp->gmin[1]), scan_coord(tw.z, hp->gmin[2]),
+                                           __int_as_float((int)ent));
         tmeta[tb + rank] = make_int4((int)ta, tff.x, tff.y, tff.z);
     }
 }
@@ -839,10 +879,11 @@ template <typename T> struct PairParams {
     const uint32_t* cstart;
     const uint32_t* tcstart;
     const Vec4<T>* spos;
-    const float* sxyz;        // fp32 only: coordinates of the source records as three arrays, each sxyz_stride long
+    const float* sxyz;        // coordinates of the source records as three arrays, each sxyz_stride long (scan_coord)
     long long sxyz_stride;
     const uint32_t* scode;    // packed (shift - floor(frac) of the source atom), 10 bits per axis, bias 512
     const Vec4<T>* tpos;
+    const float4* tscan;      // the targets' coordinates as the count pass tests them, and the entry
     const int4* tmeta;
     uint32_t* tcount;         // [Nt+1] degree per sorted target; running cursor in FILL
     const long long* toffset; // [Nt+1]
@@ -896,6 +937,27 @@ rg_group_list_kernel(const PairParams<T>* __restrict__ params_dev, uint32_t* __r
     }
 }
 
+// The undecided candidates of a target (bit s: place 32 s + lane of the staged chunk) by the double test.
+template <typename T>
+__device__ __forceinline__ uint32_t exact_hits(const PairParams<T>& p, uint32_t t, uint32_t undecided, bool equal_is_near, float ax, float ay,
+                                               float az, const float* xs, const int* delta, const uint32_t* flags, const int* wpre, int cbeg,
+                                               int clen, int lane, uint32_t le)
+{
+    constexpr int PK = RG_MASK_SLOTS * 32;
+    uint32_t hits = 0;
+    while (undecided) {
+        const int s = __ffs((int)undecided) - 1, j = 32 * s + lane;
+        undecided &= undecided - 1;
+        if (j >= clen) continue;  // padding
+        const float* x = xs + ((j >> 6) * 64 + lane * 2 + (s & 1));
+        if (equal_is_near && x[0] == ax && x[PK] == ay && x[2 * PK] == az) continue;
+        const Vec4<T> c = p.spos[delta[wpre[s] + __popc(flags[s] & le) - 1] + cbeg + j], a = p.tpos[t];
+        const T d = dist2<T>(a.x, a.y, a.z, c.x, c.y, c.z);
+        if (d <= p.r2 && d > (T)1e-8f) hits |= 1u << s;
+    }
+    return hits;
+}
+
 template <typename T, int MODE, bool BYVAL>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
 rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T> params_val, long long* __restrict__ ei,
@@ -909,17 +971,18 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
     const PairParams<T>& p = BYVAL ? params_val : params_loaded;
     extern __shared__ __align__(32) unsigned char smem_raw[];
     constexpr int CAP = PAIR_CAND_BYTES / (int)sizeof(Vec4<T>);
-    // The fp32 count pass keeps its candidates as three arrays of coordinates (no atom ids, no shift codes: the
+    // The count pass keeps its candidates as three arrays of float coordinates (no atom ids, no shift codes: the
     // space of both holds a whole list with hit bits) laid out for the packed distance test: the 8 bytes that
     // lane l reads for block b hold the coordinate of candidates 64 b + l and 64 b + 32 + l.
-    constexpr bool PACKED = (MODE == MODE_COUNT) && sizeof(T) == 4;
+    constexpr bool PACKED = (MODE == MODE_COUNT);
     constexpr int PK = RG_MASK_SLOTS * 32;
     constexpr int CAPX = PACKED ? PK : CAP;
-    static_assert(3 * 4 * PK <= PAIR_CAND_BYTES + PAIR_CODE_BYTES, "packed candidates must fit the record and code space");
+    static_assert(3 * 4 * PK + 4 * RUN_FLAG_WORDS <= PAIR_CAND_BYTES + PAIR_CODE_BYTES, "packed candidates must fit the record and code space");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char* wbase = smem_raw + warp * PAIR_WARP_BYTES;
     Vec4<T>* cand = reinterpret_cast<Vec4<T>*>(wbase);
     float* xs = reinterpret_cast<float*>(wbase);
+    int* wpre = reinterpret_cast<int*>(wbase + 3 * 4 * PK);  // runs that start in front of each word of flags
     uint32_t* codes = reinterpret_cast<uint32_t*>(wbase + PAIR_CAND_BYTES);
     unsigned short* listA = reinterpret_cast<unsigned short*>(wbase + PAIR_CAND_BYTES + PAIR_CODE_BYTES);
     unsigned short* listB = listA + PAIR_LIST;
@@ -943,6 +1006,10 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
     const T r2 = p.r2;
     const T eps = (T)1e-8f;
     const uint32_t lt = lanemask_lt();
+    constexpr bool FLOAT_FIRST = PACKED && sizeof(T) == 8;
+    const float near = FLOAT_FIRST ? hp->test_near : (float)eps, upto = FLOAT_FIRST ? hp->test_lo : (float)r2;
+    const float beyond = FLOAT_FIRST ? hp->test_hi : 0.0f;
+    const bool equal_is_near = FLOAT_FIRST && hp->test_equal_is_near;
 
     const uint32_t nwarps = gridDim.x * PAIR_WARPS;
     for (uint32_t gi = blockIdx.x * PAIR_WARPS + warp; gi < num_groups; gi += nwarps) {
@@ -991,6 +1058,11 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
             // dense staging: slot j of the list holds flattened candidate cbeg + j; all loads of a chunk are
             // independent
             int rank_base = runs_flags(flags, run_off, run_len, lane, cbeg);
+            if constexpr (FLOAT_FIRST) {
+                int starts;
+                const int before = warp_excl_scan(lane < RUN_FLAG_WORDS ? __popc(flags[lane]) : 0, lane, &starts);
+                if (lane < RUN_FLAG_WORDS) wpre[lane] = rank_base + before;
+            }
             if constexpr (PACKED) {
                 // Per 64 candidates two rounds; in each the lower half-warp takes 16 candidates of the block's
                 // first 32 and the upper half-warp 16 of its second 32, so that the 32 four-byte stores of a
@@ -1052,87 +1124,54 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
                 const uint32_t kb = has2 ? k + 1 : k;
                 const uint32_t tA = (k < n0) ? tb[0] + k : tb[1] + (k - n0);
                 const uint32_t tB = (kb < n0) ? tb[0] + kb : tb[1] + (kb - n0);
-                const Vec4<T> tpA = p.tpos[tA];
-                const Vec4<T> tpB = p.tpos[tB];
-                const T ax = tpA.x, ay = tpA.y, az = tpA.z, bx = tpB.x, by = tpB.y, bz = tpB.z;
+                const float4 tpA = p.tscan[tA];  // w = entry
+                const float4 tpB = p.tscan[tB];
                 // lane l keeps, for each of its candidates l, 32 + l, 64 + l, ..., one hit bit per target; the
                 // bits are stored so that the edge-writing pass need not repeat the distance tests.  A list too
                 // long for the bits is only counted.
                 unsigned short* mrowA = p.hitmask + (size_t)tA * 32;
                 unsigned short* mrowB = p.hitmask + (size_t)tB * 32;
-                uint32_t bitsA = 0, bitsB = 0;
-                int ca = 0, cb = 0;
-                if (chunk != 0) {
-                    if (write_masks) {
-                        bitsA = mrowA[lane];
-                        bitsB = mrowB[lane];
-                    } else {
-                        ca = (int)p.tcount[tA];
-                        cb = has2 ? (int)p.tcount[tB] : 0;
-                    }
-                }
-                uint32_t bit = 1u << (cbeg >> 5);
-                if constexpr (PACKED) {
-                    const unsigned long long ax2 = f32x2_pack(ax, ax), ay2 = f32x2_pack(ay, ay), az2 = f32x2_pack(az, az);
-                    const unsigned long long bx2 = f32x2_pack(bx, bx), by2 = f32x2_pack(by, by), bz2 = f32x2_pack(bz, bz);
-                    const unsigned long long* x2 = reinterpret_cast<const unsigned long long*>(xs) + lane;
-                    const int nblk = (clen + 63) >> 6;
-                    int na = 0, nb = 0;
+                uint32_t bitsA = 0, bitsB = 0, mayA = 0, mayB = 0, bit = 1u;
+                const unsigned long long ax2 = f32x2_pack(tpA.x, tpA.x), ay2 = f32x2_pack(tpA.y, tpA.y), az2 = f32x2_pack(tpA.z, tpA.z);
+                const unsigned long long bx2 = f32x2_pack(tpB.x, tpB.x), by2 = f32x2_pack(tpB.y, tpB.y), bz2 = f32x2_pack(tpB.z, tpB.z);
+                const unsigned long long* x2 = reinterpret_cast<const unsigned long long*>(xs) + lane;
+                const int nblk = (clen + 63) >> 6;
 #pragma unroll COUNT_UNROLL
-                    for (int blk = 0; blk < nblk; blk++) {
-                        const unsigned long long sx2 = x2[blk * 32], sy2 = x2[PK / 2 + blk * 32], sz2 = x2[PK + blk * 32];
-                        float a0, a1, b0, b1;
-                        dist2_x2(ax2, ay2, az2, sx2, sy2, sz2, a0, a1);
-                        dist2_x2(bx2, by2, bz2, sx2, sy2, sz2, b0, b1);
-                        const bool ha0 = (a0 <= r2) && (a0 > eps), ha1 = (a1 <= r2) && (a1 > eps);
-                        const bool hb0 = (b0 <= r2) && (b0 > eps), hb1 = (b1 <= r2) && (b1 > eps);
-                        if (write_masks) {
-                            bitsA |= (ha0 ? bit : 0u) | (ha1 ? (bit << 1) : 0u);
-                            bitsB |= (hb0 ? bit : 0u) | (hb1 ? (bit << 1) : 0u);
-                            bit <<= 2;
-                        } else {
-                            na += (ha0 ? 1 : 0) + (ha1 ? 1 : 0);
-                            nb += (hb0 ? 1 : 0) + (hb1 ? 1 : 0);
-                        }
+                for (int blk = 0; blk < nblk; blk++) {
+                    const unsigned long long sx2 = x2[blk * 32], sy2 = x2[PK / 2 + blk * 32], sz2 = x2[PK + blk * 32];
+                    float a0, a1, b0, b1;
+                    dist2_x2(ax2, ay2, az2, sx2, sy2, sz2, a0, a1);
+                    dist2_x2(bx2, by2, bz2, sx2, sy2, sz2, b0, b1);
+                    const bool ha0 = (a0 <= upto) && (a0 > near), ha1 = (a1 <= upto) && (a1 > near);
+                    const bool hb0 = (b0 <= upto) && (b0 > near), hb1 = (b1 <= upto) && (b1 > near);
+                    bitsA |= (ha0 ? bit : 0u) | (ha1 ? (bit << 1) : 0u);
+                    bitsB |= (hb0 ? bit : 0u) | (hb1 ? (bit << 1) : 0u);
+                    if constexpr (FLOAT_FIRST) {
+                        mayA |= (!(a0 > beyond) ? bit : 0u) | (!(a1 > beyond) ? (bit << 1) : 0u);
+                        mayB |= (!(b0 > beyond) ? bit : 0u) | (!(b1 > beyond) ? (bit << 1) : 0u);
                     }
-                    if (!write_masks) {
-                        ca += __reduce_add_sync(0xffffffffu, na);
-                        cb += __reduce_add_sync(0xffffffffu, nb);
-                    }
-                } else {
-                    int na = 0, nb = 0;
-#pragma unroll COUNT_UNROLL
-                    for (int kk = 0; kk < clen32; kk += 32) {
-                        const Vec4<T> c = cand[kk + lane];
-                        const T dA = dist2<T>(ax, ay, az, c.x, c.y, c.z);
-                        const T dB = dist2<T>(bx, by, bz, c.x, c.y, c.z);
-                        const bool hA = (dA <= r2) && (dA > eps), hB = (dB <= r2) && (dB > eps);
-                        if (write_masks) {
-                            bitsA |= hA ? bit : 0u;
-                            bitsB |= hB ? bit : 0u;
-                            bit <<= 1;
-                        } else {
-                            na += hA ? 1 : 0;
-                            nb += hB ? 1 : 0;
-                        }
-                    }
-                    if (!write_masks) {
-                        ca += __reduce_add_sync(0xffffffffu, na);
-                        cb += __reduce_add_sync(0xffffffffu, nb);
-                    }
+                    bit <<= 2;
                 }
-                if (write_masks) {
+                if constexpr (FLOAT_FIRST) {
+                    bitsA |= exact_hits<T>(p, tA, mayA & ~bitsA, equal_is_near, tpA.x, tpA.y, tpA.z, xs, delta, flags, wpre, cbeg, clen, lane, le);
+                    bitsB |= exact_hits<T>(p, tB, mayB & ~bitsB, equal_is_near, tpB.x, tpB.y, tpB.z, xs, delta, flags, wpre, cbeg, clen, lane, le);
+                }
+                if (write_masks) {  // the list is one chunk
                     mrowA[lane] = (unsigned short)bitsA;
                     if (has2) mrowB[lane] = (unsigned short)bitsB;
-                    ca = __reduce_add_sync(0xffffffffu, __popc(bitsA));
-                    cb = __reduce_add_sync(0xffffffffu, __popc(bitsB));
+                }
+                int ca = __reduce_add_sync(0xffffffffu, __popc(bitsA)), cb = __reduce_add_sync(0xffffffffu, __popc(bitsB));
+                if (chunk != 0) {
+                    ca += (int)p.tcount[tA];
+                    if (has2) cb += (int)p.tcount[tB];
+                    __syncwarp();
                 }
                 if (lane == 0) {
                     p.tcount[tA] = (uint32_t)ca;
                     if (has2) p.tcount[tB] = (uint32_t)cb;
                     if (!more_chunks && p.counts_out != nullptr) {  // degree in caller order (tpos.w = entry)
-                        p.counts_out[real_to_bits(tpA.w)] = ca;
-                        if (has2) p.counts_out[real_to_bits(tpB.w)] = cb;
+                        p.counts_out[__float_as_int(tpA.w)] = ca;
+                        if (has2) p.counts_out[__float_as_int(tpB.w)] = cb;
                     }
                 }
                 if (!more_chunks) warp_max_degree = max(warp_max_degree, max(ca, has2 ? cb : 0));
@@ -1690,7 +1729,7 @@ rg_init_kernel(uint32_t* __restrict__ hdr, const HeaderBlock blk, uint4* __restr
 static int pair_grid_waves() { return PAIR_GRID_WAVES; }
 
 struct RgLayout {
-    int64_t hdr, partials, tpartials, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, scode, smeta, hitmask, trec, tpos, tmeta,
+    int64_t hdr, partials, tpartials, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, scode, smeta, hitmask, trec, tpos, tscan, tmeta,
         tcount, toffset, sums, total;
 };
 
@@ -1712,12 +1751,13 @@ static RgLayout rg_layout(int64_t N, int64_t Nt, int64_t src_cap, int64_t cell_c
     L.aff = take(N * 16);
     L.srec = take(src_cap * 16);  // {key, cell} of every source image, in slot order
     L.spos = take(src_cap * v4);
-    L.sxyz = take(dtype == DYNB_F64 ? 0 : src_cap * 12);  // fp32 only: x[], y[], z[] of the source records for the count pass
+    L.sxyz = take(src_cap * 12);  // float x[], y[], z[] of the source records for the count pass
     L.scode = take(src_cap * 4);
     L.smeta = take(src_cap * 8);
     L.hitmask = take(Nt * 32 * 2);
     L.trec = take(Nt * 8);        // {entry, cell} of every target, in slot order
     L.tpos = take(Nt * v4);
+    L.tscan = dtype == DYNB_F64 ? take(Nt * 16) : L.tpos;  // float positions are tested as they are
     L.tmeta = take(Nt * 16);
     L.tcount = take((Nt + 1) * 4);
     L.toffset = take((Nt + 2) * 8);
@@ -1835,12 +1875,13 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     auto* tcfill = reinterpret_cast<uint32_t*>(w + L.tcfill);
     auto* srec = reinterpret_cast<uint4*>(w + L.srec);
     auto* spos = reinterpret_cast<Vec4<T>*>(w + L.spos);
-    float* sxyz = (sizeof(T) == 4) ? reinterpret_cast<float*>(w + L.sxyz) : nullptr;
+    float* sxyz = reinterpret_cast<float*>(w + L.sxyz);
     auto* scode = reinterpret_cast<uint32_t*>(w + L.scode);
     auto* smeta = reinterpret_cast<uint2*>(w + L.smeta);
     auto* hitmask = reinterpret_cast<unsigned short*>(w + L.hitmask);
     auto* trec = reinterpret_cast<uint2*>(w + L.trec);
     auto* tpos = reinterpret_cast<Vec4<T>*>(w + L.tpos);
+    auto* tscan = reinterpret_cast<float4*>(w + L.tscan);
     auto* tmeta = reinterpret_cast<int4*>(w + L.tmeta);
     auto* tcount = reinterpret_cast<uint32_t*>(w + L.tcount);
     auto* toffset = reinterpret_cast<long long*>(w + L.toffset);
@@ -1900,7 +1941,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         memcpy(init, &hi, sizeof(hi));
         PairParams<T>& pp = pp_host;
         pp.h = h; pp.cstart = ccount; pp.tcstart = tccount; pp.spos = spos; pp.sxyz = sxyz; pp.sxyz_stride = src_cap; pp.scode = scode; pp.smeta = smeta; pp.hitmask = hitmask; pp.counts_out = counts_out; pp.tpos = tpos;
-        pp.tmeta = tmeta; pp.tcount = tcount; pp.toffset = toffset; pp.r2 = (T)radius * (T)radius;
+        pp.tscan = tscan; pp.tmeta = tmeta; pp.tcount = tcount; pp.toffset = toffset; pp.r2 = (T)radius * (T)radius;
         // the targets' fill counters are free once the targets are binned: they hold the list of groups with targets
         pp.glist = (targets != nullptr) ? tcfill : nullptr;
         pp.long_list = cfill;   // likewise free once the sources are binned
@@ -1948,7 +1989,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         host_grid ? PAIR_CAND_BYTES / (int)sizeof(Vec4<T>) : 0);
     const int64_t nf = std::max(src_cap, Nt);
     rg_bin_finalize_kernel<T><<<(unsigned)((nf + 255) / 256), 256, 0, stream>>>(
-        N, Nt, targets, g, posw, aff, h, ccount, tccount, srec, trec, spos, sxyz, src_cap, scode, smeta, tpos, tmeta);
+        N, Nt, targets, g, posw, aff, h, ccount, tccount, srec, trec, spos, sxyz, src_cap, scode, smeta, tpos, tscan, tmeta, (double)pp_host.r2);
 
     if (bins_only) {
         DYNB_CUDA_OK(cudaGetLastError());

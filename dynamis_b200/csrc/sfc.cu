@@ -575,7 +575,7 @@ sel_hist_kernel(const uint64_t* __restrict__ keys, const int64_t* __restrict__ w
     // shared memory and added to the table once at the end -- for keys that crowd into a few digits (the
     // ordered bits of float coordinates) a million atomics on a handful of addresses took 90-150 us.
     // Every atom adds a constant one to a 32-bit shared counter (a native operation that also takes lanes on one address
-    // together) and the coarse counters are summed from the digit counters at the end: 118, 90 and 77 -> 22, 20 and 20 us for the
+    // together) and the coarse counters are summed from the digit counters at the end: 118, 90 and 77 -> 22, 26 and 25 us for the
     // first digits of the three levels of a KD-tree of a million atoms.  Before, lanes were grouped by a warp match and a
     // 64-bit coarse counter, one of two or three in use, was added to in shared memory for every group.
     extern __shared__ unsigned int s_fine[];

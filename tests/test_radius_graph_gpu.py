@@ -294,6 +294,39 @@ def test_float64_triclinic_small(cuda):
     torch.testing.assert_close(d2, (vec * vec).sum(dim=1), rtol=1e-12, atol=1e-12)
 
 
+@pytest.mark.parametrize("case", ["cutoff_ulps", "cutoff_float_margin", "self_limit", "coarse_floats", "outside_float_range", "long_lists", "subset"])
+def test_float64_pairs_near_the_limits(cuda, case):
+    """The double-precision count pass decides by float distances what lies clear of the cutoff and of the self-distance
+    limit (1e-8 A^2) and tests the rest in double: pairs planted a few double ulps, or about a float rounding, from either
+    limit, coordinates whose floats are coarser than the cutoff, coordinates beyond the float range, lists longer than
+    one chunk, a target subset.  Membership must equal the double-precision oracle's pair by pair."""
+    rng = np.random.default_rng(31)
+    n, box, r, targets = 3000, 200.0, 5.0, None
+    if case == "coarse_floats":
+        n, box, r = 1500, 4.0e8, 6.0          # one float step at 4e8 is 32
+    elif case == "outside_float_range":
+        n, box, r = 300, 1.0e17, 5.0e15
+    dist = np.full(n, r)
+    if case == "cutoff_ulps":
+        dist *= 1.0 + rng.integers(-3, 4, n) * 2.0 ** -53
+    elif case == "self_limit":
+        dist = 1.0e-4 * (1.0 + rng.normal(size=n) * np.where(rng.random(n) < 0.5, 1e-15, 1e-3))
+    else:
+        dist *= 1.0 + rng.normal(size=n) * np.where(rng.random(n) < 0.5, 1e-7, 1e-2)
+    if case == "long_lists":
+        pos, box, r = rng.random((3000, 3)) * 10.0, 10.0, 3.0
+    else:
+        dirs = rng.normal(size=(n, 3))
+        dirs /= np.linalg.norm(dirs, axis=1, keepdims=True)
+        base = rng.random((n, 3)) * box
+        if case == "coarse_floats":
+            base[:, 0] = box * 0.7 + rng.random(n) * 400.0   # a filament, so that cells hold several pairs
+        pos = np.concatenate([base, base + dirs * dist[:, None]])
+    if case == "subset":
+        targets = rng.permutation(pos.shape[0])[: pos.shape[0] // 3].astype(np.int64)
+    ei, cs, g = _check_vs_oracle(pos, np.eye(3) * box, [True] * 3, r, cuda, targets, what=case)
+
+
 def test_edge_distances_fp32(cuda):
     import dynamis_b200 as D
 
