@@ -327,6 +327,39 @@ def test_float64_pairs_near_the_limits(cuda, case):
     ei, cs, g = _check_vs_oracle(pos, np.eye(3) * box, [True] * 3, r, cuda, targets, what=case)
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("lists", ["short", "long", "mixed", "subset"])
+def test_distances_from_hit_bits(cuda, dtype, lists):
+    """With distances the edges come from the hit bits too, except for groups whose candidate list has none: lists on
+    either side of that limit, both in one call, and a target subset.  Edges equal the oracle's; each distance equals the
+    one evaluated in float64 from the edge's own atoms and shift (one rounding of each coordinate difference of up to
+    the box's magnitude, three of the sum)."""
+    rng = np.random.default_rng(17)
+    box, r, targets = 24.0, 3.0, None
+    pos = rng.random((1500, 3)) * box
+    if lists == "long":
+        pos = rng.random((2500, 3)) * 10.0
+        box = 10.0
+    elif lists == "mixed":
+        pos = np.concatenate([pos, 9.0 + rng.random((700, 3)) * 5.0])
+    elif lists == "subset":
+        targets = rng.permutation(1500)[:401].astype(np.int64)
+    pos = pos.astype(dtype)
+    cell = (np.eye(3) * box).astype(dtype)
+    tt = torch.as_tensor(targets, device=cuda) if targets is not None else None
+    p, c = torch.as_tensor(pos, device=cuda), torch.as_tensor(cell)
+    ei, cs, nni, counts, d2 = D.radius_graph_pbc_with_dist(p, c, torch.tensor([True] * 3), r, tt)
+    g = O.radius_graph(pos, cell, [True] * 3, r, targets)
+    assert int(nni.item()) == g["E"]
+    assert_same_edges(canon_t(ei, cs), canon_o(g), lists)
+    np.testing.assert_array_equal(counts.cpu().numpy(), g["counts"])
+    vec = p[ei[0]].double() + cs.double() @ c.to(cuda).double() - p[ei[1]].double()
+    u = float(np.finfo(dtype).eps) / 2
+    # wrapped positions and images carry a rounding of up to two boxes per coordinate, twice; d2 of d changes by 2 d of that
+    bound = 2 * r * np.sqrt(3.0) * 8 * u * 2 * box + 6 * u * r * r
+    assert float((d2.double() - (vec * vec).sum(dim=1)).abs().max()) <= bound
+
+
 def test_edge_distances_fp32(cuda):
     import dynamis_b200 as D
 
