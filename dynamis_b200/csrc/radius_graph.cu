@@ -589,13 +589,37 @@ rg_grid_kernel(DevHeader* h, double radius, long long src_capacity, long long ce
 // ------------------------------------------------------------------------------------------
 // binning
 // ------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t pack_shift_code(int ex, int ey, int ez)
+{
+    return (uint32_t)(ex + 512) | ((uint32_t)(ey + 512) << 10) | ((uint32_t)(ez + 512) << 20);
+}
+
+// What the scatter pass leaves in the provisional slot of a source image (key: image order, id: atom, code: shift - floor)
+// or of a target of a subset (key: atom, id: entry, code: floor).  In single precision the position goes along: the ordering
+// pass then reads its own slot and its cell's slots and gathers nothing by atom number, and a slot is one 32-byte sector,
+// written by one store.  In double precision it would be two sectors (48 bytes: 27 us slower for 500 k atoms); there the
+// ordering pass fetches the wrapped position.  Without a subset no target is scattered: the targets of a cell are its images
+// at shift zero, in the same order.  Atoms in random order, scatter and ordering, before and after: 263 + 218 -> 144 + 82 us
+// (4 M), 47 + 37 -> 37 + 20 us (1 M); bound by the sectors of the random writes and the cursors' atomics.
+template <typename T> struct SlotRec;
+template <> struct __align__(32) SlotRec<float> { uint32_t key, id, cell, code; float x, y, z, pad; };
+template <> struct __align__(16) SlotRec<double> { uint32_t key, id, cell, code; };
+__device__ __forceinline__ void store_slot(SlotRec<float>* at, uint32_t key, uint32_t id, uint32_t cell, uint32_t code, float x, float y, float z)
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(at), "r"(key), "r"(id), "r"(cell), "r"(code),
+                 "r"(__float_as_uint(x)), "r"(__float_as_uint(y)), "r"(__float_as_uint(z)), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void store_slot(SlotRec<double>* at, uint32_t key, uint32_t id, uint32_t cell, uint32_t code, double, double, double)
+{
+    *reinterpret_cast<uint4*>(at) = make_uint4(key, id, cell, code);
+}
 template <typename T, bool SCATTER>
 __global__ void __launch_bounds__(256, 5)
 rg_bin_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ targets, Geom<T> g,
-              const Vec4<T>* __restrict__ posw, DevHeader* __restrict__ hp,
+              const Vec4<T>* __restrict__ posw, const int4* __restrict__ aff, DevHeader* __restrict__ hp,
               uint32_t* __restrict__ ccount, uint32_t* __restrict__ cfill,
               uint32_t* __restrict__ tccount, uint32_t* __restrict__ tcfill,
-              uint4* __restrict__ srec, uint2* __restrict__ trec, long long src_capacity, int shape_cand_capacity)
+              SlotRec<T>* __restrict__ srec, SlotRec<T>* __restrict__ trec, long long src_capacity, int shape_cand_capacity)
 {
     const DevHeader h = *hp;
     // the counting pass still runs when only the image capacity is short (it writes nothing but the cell counters): the
@@ -632,6 +656,8 @@ rg_bin_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ targets, Geom<T
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) {
         const Vec4<T> w = posw[i];
+        int4 f = make_int4(0, 0, 0, 0);
+        if (SCATTER) f = aff[i];
         const uint32_t flags = (uint32_t)real_to_bits(w.w);
         const int k1 = 2 * g.rep[1] + 1, k2 = 2 * g.rep[2] + 1;
         // box of needed shifts (see rg_wrap_kernel); same (dx, dy, dz) order as a full walk
@@ -651,14 +677,17 @@ rg_bin_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ targets, Geom<T
                         atomicAdd(&ccount[c], 1u);
                     } else {
                         // the fill cursors start at the cells' first slots (the prefix sum wrote them there too):
-                        // one atomic and one 16-byte record {key, cell} per image
+                        // one atomic and one record per image; (atom, image) orders the images of a cell
                         const uint32_t slot = atomicAdd(&cfill[c], 1u);
-                        const unsigned code = (unsigned)(((dx + g.rep[0]) * k1 + (dy + g.rep[1])) * k2 + (dz + g.rep[2]));
-                        srec[slot] = make_uint4(code, (uint32_t)i, c, 0u);  // (atom, shift code) orders the images of a cell
+                        const unsigned image = (unsigned)(((dx + g.rep[0]) * k1 + (dy + g.rep[1])) * k2 + (dz + g.rep[2]));
+                        const int ex = dx - f.x, ey = dy - f.y, ez = dz - f.z;
+                        if (max(max(abs(ex), abs(ey)), abs(ez)) > 511) atomicOr(&hp->status, DYNB_RG_SHIFT_RANGE);
+                        store_slot(&srec[slot], image, (uint32_t)i, c, pack_shift_code(ex, ey, ez), x, y, z);
                     }
                 }
     }
-    if (i < Nt) {
+    // without a subset the targets are the images at shift zero: the ordering pass finds them among the sources
+    if (i < Nt && (!SCATTER || targets != nullptr)) {
         const int64_t a = targets ? targets[i] : i;
         if (a < 0 || a >= N) {
             atomicOr(&hp->status, DYNB_RG_BAD_TARGET);
@@ -668,16 +697,13 @@ rg_bin_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ targets, Geom<T
             if (!SCATTER) {
                 atomicAdd(&tccount[c], 1u);
             } else {
+                const int4 f = aff[a];
                 const uint32_t slot = atomicAdd(&tcfill[c], 1u);
-                trec[slot] = make_uint2((uint32_t)i, c);
+                // a floor that does not fit its ten bits: the atom's own image has raised the range status
+                store_slot(&trec[slot], (uint32_t)a, (uint32_t)i, c, pack_shift_code(f.x, f.y, f.z), w.x, w.y, w.z);
             }
         }
     }
-}
-
-__device__ __forceinline__ uint32_t pack_shift_code(int ex, int ey, int ez)
-{
-    return (uint32_t)(ex + 512) | ((uint32_t)(ey + 512) << 10) | ((uint32_t)(ez + 512) << 20);
 }
 
 // Coordinates as the count pass tests them: float positions as they are, double positions as floats from the grid's origin.
@@ -716,12 +742,11 @@ __device__ __forceinline__ void float_test(double r2, double X, float& near, flo
 // Deterministic order inside each cell (ascending key) and the packed records.
 template <typename T>
 __global__ void __launch_bounds__(256)
-rg_bin_finalize_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ targets, Geom<T> g,
-                       const Vec4<T>* __restrict__ posw, const int4* __restrict__ aff,
-                       DevHeader* __restrict__ hp, const uint32_t* __restrict__ cstart,
-                       const uint32_t* __restrict__ tcstart, const uint4* __restrict__ srec, const uint2* __restrict__ trec,
+rg_bin_finalize_kernel(int64_t Nt, int subset, Geom<T> g, const Vec4<T>* __restrict__ posw, DevHeader* __restrict__ hp,
+                       const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ tcstart,
+                       const SlotRec<T>* __restrict__ srec, const SlotRec<T>* __restrict__ trec,
                        Vec4<T>* __restrict__ spos, float* __restrict__ sxyz, long long sxyz_stride,
-                       uint32_t* __restrict__ scode, uint2* __restrict__ smeta, Vec4<T>* __restrict__ tpos, float4* __restrict__ tscan,
+                       uint2* __restrict__ smeta, Vec4<T>* __restrict__ tpos, float4* __restrict__ tscan,
                        int4* __restrict__ tmeta, double r2)
 {
     if (hp->status & RG_FATAL) return;
@@ -730,70 +755,72 @@ rg_bin_finalize_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ target
                    hp->test_equal_is_near);
     const unsigned long long M = hp->M;
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool has_s = j < (int64_t)M, has_t = j < Nt;
+    const bool has_s = j < (int64_t)M, has_t = subset && j < Nt;
+    auto put_target = [&](uint32_t at, T x, T y, T z, uint32_t entry, uint32_t atom, int fx, int fy, int fz) {
+        Vec4<T> r;
+        r.x = x; r.y = y; r.z = z; r.w = bits_to_real((int32_t)entry, T());
+        tpos[at] = r;
+        if (sizeof(T) == 8)
+            tscan[at] = make_float4(scan_coord(x, hp->gmin[0]), scan_coord(y, hp->gmin[1]), scan_coord(z, hp->gmin[2]), __int_as_float((int)entry));
+        tmeta[at] = make_int4((int)atom, fx, fy, fz);
+    };
     // The loads are issued level by level for the source image and the target of this thread together: the two
-    // records, then everything that depends only on a record (cell range, position and floor of the atom), then
-    // the records of the cell for the rank; the kernel waits for memory, not for arithmetic.
-    uint4 srj = make_uint4(0u, 0u, 0u, 0u);
-    uint2 trj = make_uint2(0u, 0u);
-    if (has_s) srj = srec[j];
-    if (has_t) trj = trec[j];
+    // slots, then the cell ranges, then the slots of the cell for the rank; the kernel waits for memory, not for arithmetic.
+    SlotRec<T> s{}, t{};
+    if (has_s) s = srec[j];
+    if (has_t) t = trec[j];
     uint32_t sb = 0, se = 0, tb = 0, te = 0;
-    Vec4<T> sw = {}, tw = {};
-    int4 sff = make_int4(0, 0, 0, 0), tff = make_int4(0, 0, 0, 0);
-    int64_t ta = 0;
+    const int k1 = 2 * g.rep[1] + 1, k2 = 2 * g.rep[2] + 1;
+    const uint32_t center = (uint32_t)((g.rep[0] * k1 + g.rep[1]) * k2 + g.rep[2]);  // the image at shift zero
+    Vec4<T> sw{}, tw{};
     if (has_s) {
-        sb = cstart[srj.z];
-        se = cstart[srj.z + 1];
-        sw = posw[srj.y];
-        sff = aff[srj.y];
+        sb = cstart[s.cell];
+        se = cstart[s.cell + 1];
+        if (!subset && s.key == center) tb = tcstart[s.cell];
+        if constexpr (sizeof(T) == 8) {
+            sw = posw[s.id];
+            unsigned image = s.key;
+            const int dz = (int)(image % k2) - g.rep[2]; image /= k2;
+            const int dy = (int)(image % k1) - g.rep[1]; image /= k1;
+            image_pos(g, sw.x, sw.y, sw.z, (int)image - g.rep[0], dy, dz, sw.x, sw.y, sw.z);
+        } else {
+            sw.x = s.x; sw.y = s.y; sw.z = s.z;
+        }
     }
     if (has_t) {
-        tb = tcstart[trj.y];
-        te = tcstart[trj.y + 1];
-        ta = targets ? targets[trj.x] : (int64_t)trj.x;
-        tw = posw[ta];
-        tff = aff[ta];
+        tb = tcstart[t.cell];
+        te = tcstart[t.cell + 1];
+        if constexpr (sizeof(T) == 8) tw = posw[t.key];
+        else { tw.x = t.x; tw.y = t.y; tw.z = t.z; }
     }
     if (has_s) {
-        const unsigned long long key = ((unsigned long long)srj.y << 32) | srj.x;
-        uint32_t rank = 0;
+        // place in the cell: images in front of this one; and, of those, the ones at shift zero
+        const unsigned long long mine = ((unsigned long long)s.id << 32) | s.key;
+        uint32_t rank = 0, trank = 0;
         for (uint32_t q = sb; q < se; q++) {
             const uint2 kq = *reinterpret_cast<const uint2*>(&srec[q]);
-            rank += ((((unsigned long long)kq.y << 32) | kq.x) < key) ? 1u : 0u;
+            const bool before = ((((unsigned long long)kq.y << 32) | kq.x) < mine);
+            rank += before ? 1u : 0u;
+            trank += (before && kq.x == center) ? 1u : 0u;
         }
-        const int k1 = 2 * g.rep[1] + 1, k2 = 2 * g.rep[2] + 1;
-        const uint32_t atom = srj.y;
-        unsigned code = srj.x;
-        const int dz = (int)(code % k2) - g.rep[2]; code /= k2;
-        const int dy = (int)(code % k1) - g.rep[1]; code /= k1;
-        const int dx = (int)code - g.rep[0];
-        Vec4<T> r;
-        image_pos(g, sw.x, sw.y, sw.z, dx, dy, dz, r.x, r.y, r.z);
-        r.w = bits_to_real((int32_t)atom, T());
         const uint32_t at = sb + rank;
+        Vec4<T> r;
+        r.x = sw.x; r.y = sw.y; r.z = sw.z; r.w = bits_to_real((int32_t)s.id, T());
         spos[at] = r;
-        sxyz[at] = scan_coord(r.x, hp->gmin[0]);
-        sxyz[sxyz_stride + at] = scan_coord(r.y, hp->gmin[1]);
-        sxyz[2 * sxyz_stride + at] = scan_coord(r.z, hp->gmin[2]);
-        const int ex = dx - sff.x, ey = dy - sff.y, ez = dz - sff.z;
-        uint32_t packed = pack_shift_code(0, 0, 0);
-        if (ex < -511 || ex > 511 || ey < -511 || ey > 511 || ez < -511 || ez > 511) atomicOr(&hp->status, DYNB_RG_SHIFT_RANGE);
-        else packed = pack_shift_code(ex, ey, ez);
-        scode[at] = packed;
-        smeta[at] = make_uint2(atom, packed);
+        sxyz[at] = scan_coord(sw.x, hp->gmin[0]);
+        sxyz[sxyz_stride + at] = scan_coord(sw.y, hp->gmin[1]);
+        sxyz[2 * sxyz_stride + at] = scan_coord(sw.z, hp->gmin[2]);
+        smeta[at] = make_uint2(s.id, s.code);
+        // its shift is zero: the code is minus the floor
+        if (!subset && s.key == center)
+            put_target(tb + trank, sw.x, sw.y, sw.z, s.id, s.id, 512 - (int)(s.code & 1023u), 512 - (int)((s.code >> 10) & 1023u),
+                       512 - (int)((s.code >> 20) & 1023u));
     }
     if (has_t) {
-        const uint32_t ent = trj.x;
         uint32_t rank = 0;
-        for (uint32_t q = tb; q < te; q++) rank += (trec[q].x < ent) ? 1u : 0u;
-        Vec4<T> r;
-        r.x = tw.x; r.y = tw.y; r.z = tw.z; r.w = bits_to_real((int32_t)ent, T());
-        tpos[tb + rank] = r;
-        if (sizeof(T) == 8)
-            tscan[tb + rank] = make_float4(scan_coord(tw.x, hp->gmin[0]), scan_coord(tw.y, hp->gmin[1]), scan_coord(tw.z, hp->gmin[2]),
-                                           __int_as_float((int)ent));
-        tmeta[tb + rank] = make_int4((int)ta, tff.x, tff.y, tff.z);
+        for (uint32_t q = tb; q < te; q++) rank += (trec[q].id < t.id) ? 1u : 0u;
+        put_target(tb + rank, tw.x, tw.y, tw.z, t.id, t.key, (int)(t.code & 1023u) - 512, (int)((t.code >> 10) & 1023u) - 512,
+                   (int)((t.code >> 20) & 1023u) - 512);
     }
 }
 
@@ -881,7 +908,6 @@ template <typename T> struct PairParams {
     const Vec4<T>* spos;
     const float* sxyz;        // coordinates of the source records as three arrays, each sxyz_stride long (scan_coord)
     long long sxyz_stride;
-    const uint32_t* scode;    // packed (shift - floor(frac) of the source atom), 10 bits per axis, bias 512
     const Vec4<T>* tpos;
     const float4* tscan;      // the targets' coordinates as the count pass tests them, and the entry
     const int4* tmeta;
@@ -1099,7 +1125,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
                         cp_async<16>(&cand[j], &p.spos[gidx]);
                         cp_async<16>(reinterpret_cast<char*>(&cand[j]) + 16, reinterpret_cast<const char*>(&p.spos[gidx]) + 16);
                     }
-                    if (MODE == MODE_FILL) cp_async<4>(&codes[j], &p.scode[gidx]);
+                    if (MODE == MODE_FILL) cp_async<4>(&codes[j], &p.smeta[gidx].y);
                 }
             }
             }
@@ -1376,7 +1402,7 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
                 const uint32_t word = (sw < nslots) ? flags[sw] : 0u;
                 const int r = rank_base + __popc(word & le) - 1;
                 rank_base += __popc(word);
-                if constexpr (DIST) mv[u] = (j < L) ? make_uint2((uint32_t)(delta[r] + j), p.scode[delta[r] + j]) : make_uint2(0u, 0u);
+                if constexpr (DIST) mv[u] = (j < L) ? make_uint2((uint32_t)(delta[r] + j), p.smeta[delta[r] + j].y) : make_uint2(0u, 0u);
                 else mv[u] = (j < L) ? p.smeta[delta[r] + j] : make_uint2(0u, 0u);
             }
 #pragma unroll
@@ -1748,7 +1774,7 @@ rg_init_kernel(uint32_t* __restrict__ hdr, const HeaderBlock blk, uint4* __restr
 static int pair_grid_waves() { return PAIR_GRID_WAVES; }
 
 struct RgLayout {
-    int64_t hdr, partials, tpartials, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, scode, smeta, hitmask, trec, tpos, tscan, tmeta,
+    int64_t hdr, partials, tpartials, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, smeta, hitmask, trec, tpos, tscan, tmeta,
         tcount, toffset, sums, total;
 };
 
@@ -1768,13 +1794,13 @@ static RgLayout rg_layout(int64_t N, int64_t Nt, int64_t src_cap, int64_t cell_c
     L.tpartials = take(((Nt + 255) / 256 + 1) * 64);
     L.posw = take(N * v4);
     L.aff = take(N * 16);
-    L.srec = take(src_cap * 16);  // {key, cell} of every source image, in slot order
+    const int64_t slot = dtype == DYNB_F64 ? sizeof(SlotRec<double>) : sizeof(SlotRec<float>);
+    L.srec = take(src_cap * slot);  // source images in slot order
     L.spos = take(src_cap * v4);
     L.sxyz = take(src_cap * 12);  // float x[], y[], z[] of the source records for the count pass
-    L.scode = take(src_cap * 4);
     L.smeta = take(src_cap * 8);
     L.hitmask = take(Nt * 32 * 2);
-    L.trec = take(Nt * 8);        // {entry, cell} of every target, in slot order
+    L.trec = take(Nt * slot);     // targets in slot order
     L.tpos = take(Nt * v4);
     L.tscan = dtype == DYNB_F64 ? take(Nt * 16) : L.tpos;  // float positions are tested as they are
     L.tmeta = take(Nt * 16);
@@ -1892,13 +1918,12 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     auto* cfill = reinterpret_cast<uint32_t*>(w + L.cfill);
     auto* tccount = reinterpret_cast<uint32_t*>(w + L.tccount);
     auto* tcfill = reinterpret_cast<uint32_t*>(w + L.tcfill);
-    auto* srec = reinterpret_cast<uint4*>(w + L.srec);
+    auto* srec = reinterpret_cast<SlotRec<T>*>(w + L.srec);
     auto* spos = reinterpret_cast<Vec4<T>*>(w + L.spos);
     float* sxyz = reinterpret_cast<float*>(w + L.sxyz);
-    auto* scode = reinterpret_cast<uint32_t*>(w + L.scode);
     auto* smeta = reinterpret_cast<uint2*>(w + L.smeta);
     auto* hitmask = reinterpret_cast<unsigned short*>(w + L.hitmask);
-    auto* trec = reinterpret_cast<uint2*>(w + L.trec);
+    auto* trec = reinterpret_cast<SlotRec<T>*>(w + L.trec);
     auto* tpos = reinterpret_cast<Vec4<T>*>(w + L.tpos);
     auto* tscan = reinterpret_cast<float4*>(w + L.tscan);
     auto* tmeta = reinterpret_cast<int4*>(w + L.tmeta);
@@ -1959,7 +1984,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         }
         memcpy(init, &hi, sizeof(hi));
         PairParams<T>& pp = pp_host;
-        pp.h = h; pp.cstart = ccount; pp.tcstart = tccount; pp.spos = spos; pp.sxyz = sxyz; pp.sxyz_stride = src_cap; pp.scode = scode; pp.smeta = smeta; pp.hitmask = hitmask; pp.counts_out = counts_out; pp.tpos = tpos;
+        pp.h = h; pp.cstart = ccount; pp.tcstart = tccount; pp.spos = spos; pp.sxyz = sxyz; pp.sxyz_stride = src_cap; pp.smeta = smeta; pp.hitmask = hitmask; pp.counts_out = counts_out; pp.tpos = tpos;
         pp.tscan = tscan; pp.tmeta = tmeta; pp.tcount = tcount; pp.toffset = toffset; pp.r2 = (T)radius * (T)radius;
         // the targets' fill counters are free once the targets are binned: they hold the list of groups with targets
         pp.glist = (targets != nullptr) ? tcfill : nullptr;
@@ -1997,18 +2022,18 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
                                                  (int)((N + WRAP_THREADS - 1) / WRAP_THREADS),
                                                  reinterpret_cast<const unsigned long long*>(w + L.tpartials), n_tpart);
         rg_bin_kernel<T, false><<<(unsigned)((nb + 255) / 256), 256, 0, stream>>>(
-            N, Nt, targets, g, posw, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap, 0);
+            N, Nt, targets, g, posw, aff, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap, 0);
     }
     // cell starts of sources and targets in the same two launches (which also set the fill cursors); the total of the source counts is the
     // number of source images actually binned (<= the count of rg_wrap when clipping): it becomes header.M
     DYNB_CUDA_OK((exclusive_scan_pair<uint32_t, uint32_t>(ccount, ccount, reinterpret_cast<uint32_t*>(&h->M), tccount, tccount, nullptr,
                                                            &h->ncell_plus1, cell_cap + 1, sums32, stream, cfill, tcfill)));
     rg_bin_kernel<T, true><<<(unsigned)((nb + 255) / 256), 256, 0, stream>>>(
-        N, Nt, targets, g, posw, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap,
+        N, Nt, targets, g, posw, aff, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap,
         host_grid ? PAIR_CAND_BYTES / (int)sizeof(Vec4<T>) : 0);
     const int64_t nf = std::max(src_cap, Nt);
     rg_bin_finalize_kernel<T><<<(unsigned)((nf + 255) / 256), 256, 0, stream>>>(
-        N, Nt, targets, g, posw, aff, h, ccount, tccount, srec, trec, spos, sxyz, src_cap, scode, smeta, tpos, tscan, tmeta, (double)pp_host.r2);
+        Nt, targets != nullptr ? 1 : 0, g, posw, h, ccount, tccount, srec, trec, spos, sxyz, src_cap, smeta, tpos, tscan, tmeta, (double)pp_host.r2);
 
     if (bins_only) {
         DYNB_CUDA_OK(cudaGetLastError());
