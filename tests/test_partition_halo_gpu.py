@@ -220,6 +220,26 @@ def test_extract_halo_info_equals_build_halo_maps(cuda, W):
         np.testing.assert_array_equal(ra.cpu().numpy(), ora)
 
 
+@pytest.mark.parametrize("n_edges", [1, 31, 32, 33, 1023, 1024, 1025, 5000])
+@pytest.mark.parametrize("kept", ["all", "none", "some"])
+def test_filter_edges_tile_edges(cuda, n_edges, kept):
+    """Edge counts around a word (32) and a tile (1024) of the filter, with all, none and some of them kept."""
+    rng = np.random.default_rng(n_edges)
+    pos = (rng.random((50, 3)) * 10.0).astype(np.float32)
+    cell = (np.eye(3) * 10.0).astype(np.float32)
+    edges = rng.integers(0, 50, (2, n_edges))
+    shifts = rng.integers(-1, 2, (n_edges, 3)).astype(np.float32)
+    radius = {"all": 100.0, "none": 1e-3, "some": 9.0}[kept]
+    if kept == "none":
+        edges[1] = (edges[0] + 1) % 50
+    te, ts, tp, tc = (torch.as_tensor(a, device=cuda) for a in (edges, shifts, pos, cell))
+    fe, fs = D.filter_edges_to_radius(te, ts, tp, tc.cpu(), radius)
+    oe, os_ = O.filter_edges_to_radius(edges, shifts, pos, cell, radius)
+    assert (fe.cpu().numpy() == oe).all() and (fs.cpu().numpy() == os_).all() and fe.shape == oe.shape
+    fe64, fs64 = D.filter_edges_to_radius(te, ts.double(), tp, tc.cpu(), radius)
+    assert torch.equal(fe64, fe) and torch.equal(fs64, fs.double())
+
+
 def test_filter_edges_to_radius(cuda):
     pos, cell = _halo_case(21, 3000, 36.0)
     tp, tc, tb = torch.as_tensor(pos, device=cuda), torch.as_tensor(cell), torch.tensor([True, True, True])
