@@ -149,11 +149,10 @@ struct GridChoice {
 
 // Cells of edge radius/1.99 scanned +-2 (as the reference, :662,776) unless that would need more than
 // cell_capacity cells; then the cells grow, and once they are wider than the cutoff the scan shrinks to +-1.
-__host__ __device__ inline void rg_choose_shape(GridChoice& gc, double avg, int cand_capacity, int force_sx, int force_sy, bool allow_wide);
+__host__ __device__ inline void rg_choose_shape(GridChoice& gc, double avg, int cand_capacity, bool allow_wide);
 // avg: expected sources per cell, for the shape of the work items.
 __host__ __device__ inline void rg_choose_grid(const double lo[3], const double ext[3], double radius, long long cell_capacity,
-                                               int cand_capacity, double M, double sources_per_volume, int force_sx, int force_sy,
-                                               bool allow_wide, GridChoice& gc)
+                                               int cand_capacity, double M, double sources_per_volume, bool allow_wide, GridChoice& gc)
 {
     double res = radius / 1.99;
     long long n[3];
@@ -177,8 +176,7 @@ __host__ __device__ inline void rg_choose_grid(const double lo[3], const double 
     gc.pad = pad;
     for (int k = 0; k < 3; k++) gc.gmin[k] = lo[k];
     gc.res_inv = 1.0 / res;
-    rg_choose_shape(gc, sources_per_volume > 0.0 ? sources_per_volume * res * res * res : M / (double)ncell, cand_capacity, force_sx,
-                    force_sy, allow_wide);
+    rg_choose_shape(gc, sources_per_volume > 0.0 ? sources_per_volume * res * res * res : M / (double)ncell, cand_capacity, allow_wide);
 }
 
 // cells per warp work item (Sx along x, Sy along y): as many target cells as possible while the
@@ -186,35 +184,44 @@ __host__ __device__ inline void rg_choose_grid(const double lo[3], const double 
 // allow_wide: the mean is taken over a box that the sources fill.  With a target subset the grid can span far more
 // cells than hold sources (a subdomain whose wrapped targets sit on both sides of the periodic box), the mean then
 // says nothing about the lists, and the wide shapes — which sit just under the limit of the hit bits — stay out.
-__host__ __device__ inline void rg_choose_shape(GridChoice& gc, double avg, int cand_capacity, int force_sx, int force_sy, bool allow_wide)
+constexpr int RG_SHAPES = 5;   // 4 x 2, 3 x 2, 2 x 2, 2 x 1, 1 x 1
+__host__ __device__ inline void rg_shape(int c, int& sx, int& sy)
 {
-    const int pad = gc.pad;
+    sx = c == 0 ? 4 : (c == 1 ? 3 : (c < 4 ? 2 : 1));
+    sy = c < 3 ? 2 : 1;
+}
+__host__ __device__ inline bool rg_shape_fits(int c, int pad, double avg, int cand_capacity, bool allow_wide)
+{
+    int sx, sy;
+    rg_shape(c, sx, sy);
+    if ((sy + 2 * pad) * (2 * pad + 1) > 32) return false;  // one lane per candidate run
+    if (sx > 2 && !allow_wide) return false;
+    const double Lexp = (double)(sx + 2 * pad) * (double)(sy + 2 * pad) * (double)(2 * pad + 1) * (avg > 1e-6 ? avg : 1e-6);
+    return (sx > 2) ? (1.15 * Lexp + 4.0 * sqrt(Lexp) <= (double)(RG_MASK_SLOTS * 32)) : (Lexp <= 1.5 * (double)cand_capacity);
+}
+__host__ __device__ inline void rg_set_shape(GridChoice& gc, int c)
+{
+    int sx, sy;
+    rg_shape(c, sx, sy);
+    if (sx > gc.nx) sx = gc.nx;
+    if (sy > gc.ny) sy = gc.ny;
+    gc.group_cells = sx;
+    gc.group_cells_y = sy;
+    gc.gx = (gc.nx + sx - 1) / sx;
+    const int gy = (gc.ny + sy - 1) / sy;
+    gc.num_groups = (unsigned long long)gc.gx * (unsigned long long)gy * (unsigned long long)gc.nz;
+}
+__host__ __device__ inline void rg_choose_shape(GridChoice& gc, double avg, int cand_capacity, bool allow_wide)
+{
     // measured on B200 (1 M-atom liquid, 1 M-atom fcc): 2 x 2 cells per warp beat 2 x 1 and 1 x 1 even when the
     // candidate list then needs a second chunk, and wider groups (3 or 4 cells along x, which lengthens every
     // candidate run instead of adding runs) beat 2 x 2 as long as the list keeps its hit bits: the work per group
     // (decode, run table, staging) is shared by more targets.  A list longer than the hit bits sends its group to
     // the slow writer, so the wide shapes are taken only with a margin (15 % on the mean density, four standard
     // deviations of a Poisson count) under that limit.
-    const double budget = 1.5 * (double)cand_capacity;
-    const int shapes[5][2] = {{4, 2}, {3, 2}, {2, 2}, {2, 1}, {1, 1}};
-    int bestx = 1, besty = 1;
-    for (int c = 0; c < 5; c++) {
-        const int sx = shapes[c][0], sy = shapes[c][1];
-        if ((sy + 2 * pad) * (2 * pad + 1) > 32) continue;  // one lane per candidate run
-        if (sx > 2 && !allow_wide) continue;
-        const double Lexp = (double)(sx + 2 * pad) * (double)(sy + 2 * pad) * (double)(2 * pad + 1) * (avg > 1e-6 ? avg : 1e-6);
-        const bool fits = (sx > 2) ? (1.15 * Lexp + 4.0 * sqrt(Lexp) <= (double)(RG_MASK_SLOTS * 32)) : (Lexp <= budget);
-        if (fits || c == 4) { bestx = sx; besty = sy; break; }
-    }
-    if (force_sx > 0) bestx = force_sx;
-    if (force_sy > 0 && (force_sy + 2 * pad) * (2 * pad + 1) <= 32) besty = force_sy;
-    if (bestx > gc.nx) bestx = gc.nx;
-    if (besty > gc.ny) besty = gc.ny;
-    gc.group_cells = bestx;
-    gc.group_cells_y = besty;
-    gc.gx = (gc.nx + bestx - 1) / bestx;
-    const int gy = (gc.ny + besty - 1) / besty;
-    gc.num_groups = (unsigned long long)gc.gx * (unsigned long long)gy * (unsigned long long)gc.nz;
+    int best = 0;
+    while (best < RG_SHAPES - 1 && !rg_shape_fits(best, gc.pad, avg, cand_capacity, allow_wide)) best++;
+    rg_set_shape(gc, best);
 }
 
 __host__ __device__ inline void rg_store_grid(DevHeader& h, const GridChoice& gc)
@@ -484,7 +491,7 @@ rg_target_bbox_kernel(const int64_t* __restrict__ targets, int64_t Nt, int64_t N
 template <typename T>
 __global__ void __launch_bounds__(1024)
 rg_grid_kernel(DevHeader* h, double radius, long long src_capacity, long long cell_capacity, int cand_capacity,
-               int force_sx, int force_sy, const unsigned long long* __restrict__ partials, int num_partials,
+               const unsigned long long* __restrict__ partials, int num_partials,
                const unsigned long long* __restrict__ tpartials, int num_tpartials)
 {
     {   // reduce the per-block partials of rg_wrap_kernel into the header
@@ -582,7 +589,7 @@ rg_grid_kernel(DevHeader* h, double radius, long long src_capacity, long long ce
         ext[k] = hi - lo[k];
     }
     GridChoice gc;
-    rg_choose_grid(lo, ext, radius, cell_capacity, cand_capacity, (double)h->M, 0.0, force_sx, force_sy, num_tpartials == 0, gc);
+    rg_choose_grid(lo, ext, radius, cell_capacity, cand_capacity, (double)h->M, 0.0, num_tpartials == 0, gc);
     rg_store_grid(*h, gc);
 }
 
@@ -631,27 +638,31 @@ rg_bin_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ targets, Geom<T
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&hp->status, DYNB_RG_SRC_OVERFLOW);
         return;
     }
-    if (SCATTER && shape_cand_capacity > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (SCATTER && shape_cand_capacity > 0 && blockIdx.x == 0 && threadIdx.x < 32) {
         // grid chosen on the host: the shape of the work items is settled here, from the number of images and the
         // bounding box they really fill (gathered while wrapping) — an atom cluster in a large periodic box is as
-        // dense in its cells as it is, whatever the volume of the cell
-        double vol_cells = 1.0;
-        const double res = 1.0 / h.res_inv;
-        const int nn[3] = {h.nx, h.ny, h.nz};
-        for (int k = 0; k < 3; k++) {
-            const double ext = unordered_any<T>(h.bb_max[k]) - unordered_any<T>(h.bb_min[k]) + 0.02;
-            double cells = ceil(ext / res);
+        // dense in its cells as it is, whatever the volume of the cell.  One lane per axis, then one per shape: the divisions
+        // and square roots of the five shapes are in flight together (scatter of a thousand atoms 10.1 -> 9.3 us).
+        const int lane = threadIdx.x;
+        double cells = 1.0;
+        if (lane < 3) {
+            const int n = lane == 0 ? h.nx : (lane == 1 ? h.ny : h.nz);
+            cells = ceil((unordered_any<T>(hp->bb_max[lane]) - unordered_any<T>(hp->bb_min[lane]) + 0.02) / (1.0 / h.res_inv));
             if (!(cells >= 1.0)) cells = 1.0;
-            if (cells > (double)nn[k]) cells = (double)nn[k];
-            vol_cells *= cells;
+            if (cells > (double)n) cells = (double)n;
         }
-        GridChoice gc;
-        gc.nx = h.nx; gc.ny = h.ny; gc.nz = h.nz; gc.pad = h.pad;
-        rg_choose_shape(gc, (double)h.M / vol_cells, shape_cand_capacity, 0, 0, true);
-        hp->group_cells = gc.group_cells;
-        hp->group_cells_y = gc.group_cells_y;
-        hp->gx = gc.gx;
-        hp->num_groups = gc.num_groups;
+        const double vol_cells = __shfl_sync(0xffffffffu, cells, 0) * __shfl_sync(0xffffffffu, cells, 1) * __shfl_sync(0xffffffffu, cells, 2);
+        const bool fits = lane >= RG_SHAPES - 1 || rg_shape_fits(lane, h.pad, (double)h.M / vol_cells, shape_cand_capacity, true);
+        const int best = __ffs((int)__ballot_sync(0xffffffffu, fits)) - 1;
+        if (lane == 0) {
+            GridChoice gc;
+            gc.nx = h.nx; gc.ny = h.ny; gc.nz = h.nz;
+            rg_set_shape(gc, best);
+            hp->group_cells = gc.group_cells;
+            hp->group_cells_y = gc.group_cells_y;
+            hp->gx = gc.gx;
+            hp->num_groups = gc.num_groups;
+        }
     }
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) {
@@ -1311,7 +1322,7 @@ constexpr int FM_WARP_BYTES = FM_META * 8 + FM_META * 2 + RUN_INDEX_BYTES;    //
 template <typename T, bool GLUE, bool DIST>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
 rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restrict__ ei, float* __restrict__ shifts,
-                   T* __restrict__ d2out, const long long E, const GlueArgs glue)
+                   T* __restrict__ d2out, const long long E, const GlueArgs glue, long long* __restrict__ total)
 {
     const PairParams<T> p = *params_dev;
     extern __shared__ __align__(32) unsigned char smem_raw[];
@@ -1325,6 +1336,7 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
 
     const DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
+    if (total != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *total = E;
     const int nx = hp->nx, ny = hp->ny, nz = hp->nz, S = hp->group_cells, Sy = hp->group_cells_y, pad = hp->pad;
     const uint32_t gx = (uint32_t)hp->gx;
     const uint32_t gy = (uint32_t)((ny + Sy - 1) / Sy);
@@ -1771,8 +1783,6 @@ rg_init_kernel(uint32_t* __restrict__ hdr, const HeaderBlock blk, uint4* __restr
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
-static int pair_grid_waves() { return PAIR_GRID_WAVES; }
-
 struct RgLayout {
     int64_t hdr, partials, tpartials, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, smeta, hitmask, trec, tpos, tscan, tmeta,
         tcount, toffset, sums, total;
@@ -1969,7 +1979,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         c = cd;
         const double vol = std::fabs(c[0] * (c[4] * c[8] - c[5] * c[7]) - c[1] * (c[3] * c[8] - c[5] * c[6]) + c[2] * (c[3] * c[7] - c[4] * c[6]));
         const double density = vol > 0.0 ? (double)N / vol : 0.0;  // images repeat the atoms: the same density everywhere in the box
-        rg_choose_grid(lo, ext, radius, (long long)cell_cap, PAIR_CAND_BYTES / (int)sizeof(Vec4<T>), (double)N, density, 0, 0, true, gc_host);
+        rg_choose_grid(lo, ext, radius, (long long)cell_cap, PAIR_CAND_BYTES / (int)sizeof(Vec4<T>), (double)N, density, true, gc_host);
         // A grid over the whole cell that had to take coarser cells to fit the cell capacity (few atoms in a large
         // periodic box) is worse than the grid over the data's own bounding box: that case keeps the device path.
         if (gc_host.res_inv < 0.999 * 1.99 / radius) host_grid = false;
@@ -2002,7 +2012,6 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     }
 
     const int vec_ok = (reinterpret_cast<uintptr_t>(pos_dev) % 16 == 0) ? 1 : 0;
-    const int force_sx = 0, force_sy = 0;  // cells per warp work item: chosen by rg_choose_grid
     const int64_t nb = std::max(N, Nt);
     if (host_grid) {
         rg_wrap_kernel<T, true><<<(unsigned)((N + WRAP_THREADS - 1) / WRAP_THREADS), WRAP_THREADS, 0, stream>>>(
@@ -2017,7 +2026,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
             rg_target_bbox_kernel<T><<<n_tpart, 256, 0, stream>>>(targets, Nt, N, posw, reinterpret_cast<unsigned long long*>(w + L.tpartials));
         }
         rg_grid_kernel<T><<<1, 1024, 0, stream>>>(h, radius, (long long)src_cap, (long long)cell_cap,
-                                                 PAIR_CAND_BYTES / (int)sizeof(Vec4<T>), force_sx, force_sy,
+                                                 PAIR_CAND_BYTES / (int)sizeof(Vec4<T>),
                                                  reinterpret_cast<const unsigned long long*>(w + L.partials),
                                                  (int)((N + WRAP_THREADS - 1) / WRAP_THREADS),
                                                  reinterpret_cast<const unsigned long long*>(w + L.tpartials), n_tpart);
@@ -2045,7 +2054,9 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         rg_group_list_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, tcfill);
     const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
     DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_COUNT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const int grid = sm_count_cached() * 4 * pair_grid_waves();
+    // there are no more groups than cells, and with a target subset no more of interest than targets
+    const int64_t most_groups = std::min(host_grid ? (int64_t)gc_host.ncell_plus1 : cell_cap, targets != nullptr ? Nt : cell_cap);
+    const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * 4 * PAIR_GRID_WAVES, (most_groups + PAIR_WARPS - 1) / PAIR_WARPS);
     rg_pair_kernel<T, MODE_COUNT, true><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, pp_host, nullptr, nullptr, nullptr, 0, GlueArgs{});
     DYNB_CUDA_OK((exclusive_scan<uint32_t, long long>(tcount, toffset, nullptr, Nt + 1, sums64,
                                                        reinterpret_cast<long long*>(&h->E), stream)));
@@ -2056,13 +2067,13 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
 }
 
 template <typename T>
-static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int64_t E, const GlueArgs* glue_opt, cudaStream_t stream)
+static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int64_t E, const GlueArgs* glue_opt, int64_t* total_dev,
+                   bool long_lists, cudaStream_t stream)
 {
     const unsigned char* w = static_cast<const unsigned char*>(ws);
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
-    const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
-    DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_FILL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const int grid = sm_count_cached() * 4 * pair_grid_waves();
+    // a warp for every 32 edges is more than there are groups with targets
+    const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * 4 * PAIR_GRID_WAVES, (E + 32 * PAIR_WARPS - 1) / (32 * PAIR_WARPS));
     GlueArgs glue{};
     if (glue_opt != nullptr) glue = *glue_opt;
     // The edges come from the hit masks of the counting pass; the groups whose candidate list was too long for the masks
@@ -2072,15 +2083,19 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
     auto* d2 = static_cast<T*>(d2out);
     auto launch = [&](auto kernel) -> int {
         DYNB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fsmem));
-        kernel<<<grid, PAIR_THREADS, fsmem, stream>>>(params_dev, ei64, shifts, d2, (long long)E, glue);
+        kernel<<<grid, PAIR_THREADS, fsmem, stream>>>(params_dev, ei64, shifts, d2, (long long)E, glue, reinterpret_cast<long long*>(total_dev));
         return DYNB_OK;
     };
     const int rc = d2 != nullptr ? launch(rg_fillmask_kernel<T, false, true>)
                                  : (glue_opt != nullptr ? launch(rg_fillmask_kernel<T, true, false>) : launch(rg_fillmask_kernel<T, false, false>));
     if (rc) return rc;
-    // this launch usually has nothing to do: two waves keep its cost low
-    const int fgrid = sm_count_cached() * 4 * std::min(2, pair_grid_waves());
-    rg_pair_kernel<T, MODE_FILL, false><<<fgrid, PAIR_THREADS, smem, stream>>>(params_dev, PairParams<T>{}, ei64, shifts, d2, (long long)E, glue);
+    // the groups the counting pass listed; a caller who has read the plan's header knows whether there are any
+    if (long_lists) {
+        const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
+        DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_FILL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        rg_pair_kernel<T, MODE_FILL, false><<<sm_count_cached() * 8, PAIR_THREADS, smem, stream>>>(params_dev, PairParams<T>{}, ei64, shifts, d2,
+                                                                                                   (long long)E, glue);
+    }
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -2092,7 +2107,7 @@ static int rg_halo_mark(const void* ws, HaloArgs ha, int64_t N, int64_t src_cap,
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
     rg_halo_owner_kernel<T><<<(unsigned)((std::max(N, src_cap) + 255) / 256), 256, 0, stream>>>(params_dev, ha, N);
     rg_halo_runs_kernel<T><<<(unsigned)std::min<int64_t>((cell_cap + 255) / 256, (int64_t)sm_count_cached() * 8), 256, 0, stream>>>(params_dev, ha);
-    const int grid = sm_count_cached() * 4 * pair_grid_waves();
+    const int grid = sm_count_cached() * 4 * PAIR_GRID_WAVES;
     if (ha.words == 1) rg_halo_kernel<T, false><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
     else rg_halo_kernel<T, true><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
     DYNB_CUDA_OK(cudaGetLastError());
@@ -2166,38 +2181,43 @@ extern "C" int dynb_rg_bin(const void* pos_dev, int dtype, int64_t n_atoms, cons
                        src_capacity, cell_capacity, nullptr, header_host, true, stream);
 }
 
-extern "C" int dynb_rg_fill(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
-                            void* dist_sq_dev, int64_t E, void* stream)
+static int rg_fill_any(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* shifts_dev, void* dist_sq_dev,
+                       const GlueArgs* glue, int64_t* total_dev, int64_t E, bool long_lists, void* stream)
 {
     if (workspace_dev == nullptr) return fail_arg("null workspace");
     if (E < 0) return fail_arg("E must be non-negative");
     if (E == 0) return DYNB_OK;
-    if (edge_index_dev == nullptr || cell_shifts_dev == nullptr) return fail_arg("null output pointer");
+    if (edge_index_dev == nullptr || shifts_dev == nullptr) return fail_arg("null output pointer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (dtype == DYNB_F32) return rg_fill<float>(workspace_dev, edge_index_dev, cell_shifts_dev, dist_sq_dev, E, nullptr, s);
-    if (dtype == DYNB_F64) return rg_fill<double>(workspace_dev, edge_index_dev, cell_shifts_dev, dist_sq_dev, E, nullptr, s);
+    if (dtype == DYNB_F32) return rg_fill<float>(workspace_dev, edge_index_dev, shifts_dev, dist_sq_dev, E, glue, total_dev, long_lists, s);
+    if (dtype == DYNB_F64) return rg_fill<double>(workspace_dev, edge_index_dev, shifts_dev, dist_sq_dev, E, glue, total_dev, long_lists, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");
+}
+
+extern "C" int dynb_rg_fill(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
+                            void* dist_sq_dev, int64_t E, void* stream)
+{
+    return rg_fill_any(workspace_dev, dtype, edge_index_dev, cell_shifts_dev, dist_sq_dev, nullptr, nullptr, E, true, stream);
+}
+
+extern "C" int dynb_rg_fill_counted(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
+                                    void* dist_sq_dev, int64_t E, int long_lists, int64_t* total_dev, void* stream)
+{
+    return rg_fill_any(workspace_dev, dtype, edge_index_dev, cell_shifts_dev, dist_sq_dev, nullptr, total_dev, E, long_lists != 0, stream);
 }
 
 extern "C" int dynb_rg_fill_glue(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* unit_shifts_dev,
                                  float* cart_shifts_dev, const float* cell_host, int negate_shifts, const int64_t* id_map_dev,
                                  int64_t E, void* stream)
 {
-    if (workspace_dev == nullptr) return fail_arg("null workspace");
-    if (E < 0) return fail_arg("E must be non-negative");
     if (negate_shifts != 0 && negate_shifts != 1) return fail_arg("negate_shifts must be 0 or 1");
     if (cart_shifts_dev != nullptr && cell_host == nullptr) return fail_arg("cell_host is required with cart_shifts_dev");
-    if (E == 0) return DYNB_OK;
-    if (edge_index_dev == nullptr || unit_shifts_dev == nullptr) return fail_arg("null output pointer");
     GlueArgs g{};
     g.cart = cart_shifts_dev;
     g.id_map = reinterpret_cast<const long long*>(id_map_dev);
     g.negate = negate_shifts;
     for (int k = 0; k < 9; k++) g.c[k] = cell_host != nullptr ? cell_host[k] : 0.0f;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (dtype == DYNB_F32) return rg_fill<float>(workspace_dev, edge_index_dev, unit_shifts_dev, nullptr, E, &g, s);
-    if (dtype == DYNB_F64) return rg_fill<double>(workspace_dev, edge_index_dev, unit_shifts_dev, nullptr, E, &g, s);
-    return fail_arg("dtype must be DYNB_F32 or DYNB_F64");
+    return rg_fill_any(workspace_dev, dtype, edge_index_dev, unit_shifts_dev, nullptr, &g, nullptr, E, true, stream);
 }
 
 extern "C" int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,

@@ -89,26 +89,26 @@ class RadiusGraphPlan:
     valid until the next radius-graph call on the same device, which reuses the workspace.
     """
 
-    __slots__ = ("ws", "dtype_code", "E", "M", "counts", "device", "pos_dtype", "max_degree", "grid", "num_groups")
+    __slots__ = ("ws", "dtype_code", "E", "M", "counts", "device", "pos_dtype", "max_degree", "grid", "num_groups", "long_lists")
 
-    def fill(self, want_dist_sq: bool = False):
+    def fill(self, want_dist_sq: bool = False, total: Optional[torch.Tensor] = None):
+        """(edge_index, shifts, squared distances or None); ``total`` (one int64 on the device) receives E."""
         dev = self.device
         E = self.E
         with _lib.on_device(dev):
             edge_index = torch.empty((2, E), dtype=torch.int64, device=dev)
             shifts = torch.empty((E, 3), dtype=torch.float32, device=dev)
             d2 = torch.empty((E,), dtype=self.pos_dtype, device=dev) if want_dist_sq else None
-            self.fill_into(edge_index, shifts, d2)
+            self.fill_into(edge_index, shifts, d2, total)
         return edge_index, shifts, d2
 
-    def fill_into(self, edge_index, shifts, d2=None):
+    def fill_into(self, edge_index, shifts, d2=None, total=None):
         if self.E == 0:
             return
-        stream = torch.cuda.current_stream(self.device)
-        _lib.check(_lib.lib().dynb_rg_fill(self.ws.data_ptr(), self.dtype_code, edge_index.data_ptr(), shifts.data_ptr(),
-                                           d2.data_ptr() if d2 is not None else None, self.E, stream.cuda_stream),
+        _lib.check(_lib.lib().dynb_rg_fill_counted(self.ws.data_ptr(), self.dtype_code, edge_index.data_ptr(), shifts.data_ptr(),
+                                                   d2.data_ptr() if d2 is not None else None, self.E, self.long_lists,
+                                                   total.data_ptr() if total is not None else None, _lib.stream_of(self.device)),
                    "rg_fill")
-
 
     def fill_glue(self, cell: Optional[torch.Tensor], negate_shifts: bool = True, cartesian: bool = True,
                   id_map: Optional[torch.Tensor] = None):
@@ -254,6 +254,7 @@ def plan_radius_graph(pos, cell, pbc, radius, target_indices=None) -> RadiusGrap
     plan.max_degree = int(hdr.max_degree)
     plan.grid = (int(hdr.grid[0]), int(hdr.grid[1]), int(hdr.grid[2]))
     plan.num_groups = int(hdr.num_groups)
+    plan.long_lists = 1 if hdr.reserved[0] else 0
     plan.counts = counts
     plan.device = dev
     plan.pos_dtype = pos.dtype
@@ -278,8 +279,8 @@ def _graph_impl(pos, cell, pbc, radius, target_indices, counts_only, want_dist_s
             plan.counts,
         )
         return out + ((torch.empty(0, dtype=pos.dtype, device=dev),) if want_dist_sq else ())
-    edge_index, shifts, d2 = plan.fill(want_dist_sq)
-    nni = torch.full((1,), plan.E, dtype=torch.int64, device=dev)
+    nni = torch.empty((1,), dtype=torch.int64, device=dev)
+    edge_index, shifts, d2 = plan.fill(want_dist_sq, nni)
     out = (edge_index, shifts, nni, plan.counts)
     return out + ((d2,) if want_dist_sq else ())
 
@@ -308,7 +309,10 @@ def radius_graph_pbc_ex(pos, cell, pbc, radius, max_num_neighbors, enforce_max_s
 def radius_graph_pbc_counts_ex(pos, cell, pbc, radius, target_indices: Optional[torch.Tensor] = None):
     """Per-target degrees only (no edge buffers, no fill pass)."""
     _validate(pos, cell, pbc, float(radius), 0, target_indices)
-    return _graph_impl(pos, cell, pbc, float(radius), target_indices, True)[3]
+    n_target = target_indices.size(0) if target_indices is not None else pos.size(0)
+    if pos.size(0) == 0 or n_target == 0:
+        return torch.zeros((n_target,), dtype=torch.int32, device=pos.device)
+    return plan_radius_graph(pos, cell, pbc, float(radius), target_indices).counts
 
 
 def radius_graph_pbc_with_dist(pos, cell, pbc, radius, target_indices: Optional[torch.Tensor] = None):
@@ -383,12 +387,11 @@ def launches_per_graph(target_subset: bool = False, fully_periodic: bool = True)
     """Kernels one radius_graph_pbc call launches on a fully periodic cell: init (header, counters, degrees), wrap
     (which also counts the images into their cells: the grid follows from the cell), 2 scan kernels (source and
     target cell starts together), scatter, finalize, count pass (degrees included), 2 scan kernels (edge offsets),
-    two edge-writing launches (the one driven by the hit bits of the count pass and the one that recomputes
-    distances; the device decides which of them does the work, the other returns at once; with distances
-    requested only the second is launched).  Two more (grid from the data's bounding box, cell histogram) when a
-    direction is not periodic or a target subset is given, and two more again (the targets' bounding box, the
-    list of groups with targets) with a target subset."""
-    n = 11
+    the edge writer.  One more (the pass that recomputes distances) when a candidate list was too long for its hit
+    bits.  Two more (grid from the data's bounding box, cell histogram) when a direction is not periodic or a target
+    subset is given, and two more again (the targets' bounding box, the list of groups with targets) with a target
+    subset."""
+    n = 10
     if target_subset or not fully_periodic:
         n += 2
     if target_subset:

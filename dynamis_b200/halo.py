@@ -102,7 +102,8 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
         send_mask = torch.empty((max(N, 1), words), dtype=torch.int32, device=dev)
         recv_mask = torch.empty((max(N, 1), words), dtype=torch.int32, device=dev)
         has_remote = torch.empty((max(N, 1),), dtype=torch.uint8, device=dev)
-        bad = torch.zeros((1,), dtype=torch.int32, device=dev)
+        offs_bad = torch.zeros((2 * (W + 1) + 2,), dtype=torch.int64, device=dev)  # the offsets and, behind them, the error word
+        offs, bad = offs_bad[:-1], offs_bad[-1:].view(torch.int32)
         _lib.check(L.dynb_halo_mark_from_edges(edges.data_ptr(), E, pid.data_ptr(), N, R, W, send_mask.data_ptr(),
                                                recv_mask.data_ptr(), has_remote.data_ptr(), bad.data_ptr(), _stream(dev)),
                    "halo_mark_from_edges")
@@ -111,11 +112,10 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_halo_lists_workspace_bytes(N, W, ctypes.byref(nbytes)), "halo_lists_workspace_bytes")
         ws = scratch(dev, "halo_lists", nbytes.value)
-        offs = torch.empty((2 * (W + 1) + 1,), dtype=torch.int64, device=dev)
         _lib.check(L.dynb_halo_lists_plan(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, offs.data_ptr(), ws.data_ptr(),
                                           ws.numel(), _stream(dev)), "halo_lists_plan")
-        offs_h = offs.cpu()
-        if int(bad.item()) != 0:
+        offs_h = offs_bad.cpu()
+        if int(offs_h[-1]) != 0:
             raise RuntimeError("extract_halo_info: an edge endpoint, partition id or my_outer_atoms entry is out of range")
         total_send, total_recv = int(offs_h[W]), int(offs_h[2 * W + 1])
         send_local = torch.empty((total_send,), dtype=torch.int64, device=dev)

@@ -87,6 +87,11 @@ int dynb_rg_plan(const void* pos_dev, int dtype, int64_t n_atoms, const void* ce
 int dynb_rg_fill(const void* workspace_dev, int dtype, int64_t* edge_index_dev /* [2,E] */,
                  float* cell_shifts_dev /* [E,3] */, void* dist_sq_dev /* [E] or NULL */, int64_t E, void* stream);
 
+/* dynb_rg_fill for a caller who has read the plan's header: long_lists = header.reserved[0] != 0 says whether the pass for
+ * long candidate lists has anything to do (0 saves its launch); total_dev (optional, may be NULL) receives E. */
+int dynb_rg_fill_counted(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
+                         void* dist_sq_dev, int64_t E, int long_lists, int64_t* total_dev, void* stream);
+
 /* dynb_rg_fill for the model-side graph glue (dynamis_model/src/dynamis_model/nnp/mace.py:591-608,
  * uma.py:915-948): the models negate the offsets (unit_shifts = -cell_offsets), keep the edges whose
  * destination is an owned atom (edge_index[1] < num_local) and form shifts = unit_shifts @ cell in
