@@ -1031,7 +1031,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
     // behind rg_fillmask_kernel the writing pass has only the groups whose candidate list was too long for the hit bits
     constexpr bool long_only = (MODE == MODE_FILL);
     if (long_only && hp->long_groups == 0u) return;
-    int warp_max_slots = 0, warp_max_degree = 0;
+    int warp_max_slots = 0, max_degree = 0;
     const int nx = hp->nx, ny = hp->ny, nz = hp->nz, S = hp->group_cells, Sy = hp->group_cells_y, pad = hp->pad;
     const uint32_t gx = (uint32_t)hp->gx;
     const uint32_t gy = (uint32_t)((ny + Sy - 1) / Sy);
@@ -1155,6 +1155,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
           if constexpr (MODE == MODE_COUNT) {
             // the targets of both rows of the group as one list, two targets per candidate load
             const uint32_t n0 = te[0] - tb[0], ntot = n0 + (te[1] - tb[1]);
+            int degree = 0;  // lane l collects the degree of target 32 j + l; stored 32 targets at a time
             for (uint32_t k = 0; k < ntot; k += 2) {
                 const bool has2 = (k + 1 < ntot);
                 const uint32_t kb = has2 ? k + 1 : k;
@@ -1202,15 +1203,34 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
                     if (has2) cb += (int)p.tcount[tB];
                     __syncwarp();
                 }
-                if (lane == 0) {
-                    p.tcount[tA] = (uint32_t)ca;
-                    if (has2) p.tcount[tB] = (uint32_t)cb;
-                    if (!more_chunks && p.counts_out != nullptr) {  // degree in caller order (tpos.w = entry)
-                        p.counts_out[__float_as_int(tpA.w)] = ca;
-                        if (has2) p.counts_out[__float_as_int(tpB.w)] = cb;
+                if constexpr (FLOAT_FIRST) {
+                    // (collecting the degrees here costs registers that the double test needs: 0.6 % slower)
+                    if (lane == 0) {
+                        p.tcount[tA] = (uint32_t)ca;
+                        if (has2) p.tcount[tB] = (uint32_t)cb;
+                        if (!more_chunks && p.counts_out != nullptr) {  // in caller order
+                            p.counts_out[__float_as_int(tpA.w)] = ca;
+                            if (has2) p.counts_out[__float_as_int(tpB.w)] = cb;
+                        }
+                    }
+                    if (!more_chunks) max_degree = max(max_degree, max(ca, has2 ? cb : 0));
+                } else {
+                    // stored 32 at a time: one thread's four stores a pair were 1.3 % of the graph of a 1 M liquid
+                    if (lane == (int)(k & 31u)) degree = ca;
+                    if (lane == (int)(k & 31u) + 1) degree = cb;
+                    if ((k & 31u) == 30u || k + 2 >= ntot) {
+                        const uint32_t mine = (k & ~31u) + (uint32_t)lane;
+                        if (mine < ntot) {
+                            const uint32_t t = (mine < n0) ? tb[0] + mine : tb[1] + (mine - n0);
+                            p.tcount[t] = (uint32_t)degree;
+                            if (!more_chunks) {
+                                if (p.counts_out != nullptr) p.counts_out[__float_as_int(p.tscan[t].w)] = degree;  // in caller order
+                                max_degree = max(max_degree, degree);
+                            }
+                        }
+                        __syncwarp();
                     }
                 }
-                if (!more_chunks) warp_max_degree = max(warp_max_degree, max(ca, has2 ? cb : 0));
             }
           } else {
 #pragma unroll
@@ -1299,7 +1319,8 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
         __shared__ int s_max_degree;
         if (threadIdx.x == 0) s_max_degree = 0;
         __syncthreads();
-        if (lane == 0 && warp_max_degree > 0) atomicMax(&s_max_degree, warp_max_degree);
+        max_degree = __reduce_max_sync(0xffffffffu, max_degree);
+        if (lane == 0 && max_degree > 0) atomicMax(&s_max_degree, max_degree);
         __syncthreads();
         if (threadIdx.x == 0 && s_max_degree > 0) atomicMax(&hp->max_degree, (uint32_t)s_max_degree);
     }
