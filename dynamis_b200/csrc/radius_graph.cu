@@ -58,6 +58,9 @@ struct DevHeader {
     int32_t group_cells_y;  // cells per warp work item along y (1 or 2)
     unsigned long long bb_min[3];  // ordered-integer images of the bounding box
     unsigned long long bb_max[3];
+    unsigned long long tb_min[3];  // the same of the wrapped targets (target subsets only)
+    unsigned long long tb_max[3];
+    uint32_t arrived;              // blocks of the pass that chooses the grid that are done
     double gmin[3];
     double res_inv;
     double clip_lo[3];  // source images outside [clip_lo, clip_hi] cannot reach any target and are dropped
@@ -137,7 +140,7 @@ __device__ __forceinline__ uint32_t cell_of(const DevHeader& h, T x, T y, T z)
 constexpr int RG_MASK_SLOTS = 16;  // hit bits kept per lane and target (candidate lists up to 512 records)
 
 // The cell grid of a plan and the shape of a warp's work item.  Chosen on the device from the bounding box of
-// the data (rg_grid_kernel), or on the host from the cell when the box is periodic in all directions and every
+// the data (rg_choose_grid_device), or on the host from the cell when the box is periodic in all directions and every
 // atom is a target (the images then fill a known box and the first two passes run as one).
 struct GridChoice {
     int nx, ny, nz, pad, group_cells, group_cells_y, gx;
@@ -285,6 +288,66 @@ __device__ __forceinline__ void dist2_x2(unsigned long long ax2, unsigned long l
     asm("mov.b64 {%0, %1}, %2;" : "=f"(d_lo), "=f"(d_hi) : "l"(d));
 }
 
+// The grid when the host cannot choose it: from the bounding boxes of the images and, with a target subset, of the targets,
+// by one thread of the block that finishes last of the pass that gathers the last of them.  Cells of edge radius/1.99 scanned
+// +-2 (as the reference, :662,776) unless that would need more than cell_capacity cells; then the cells grow, and once they
+// are wider than the cutoff the scan shrinks to +-1.  As a launch of its own, reducing per-block partial results: 22 us (1.6 M atoms, a subset of 1 M).
+struct GridArgs { double radius; long long src_capacity, cell_capacity; int cand_capacity; };
+template <typename T>
+__device__ void rg_choose_grid_device(DevHeader* h, const GridArgs& a, bool subset)
+{
+    const double radius = a.radius;
+    const long long src_capacity = a.src_capacity, cell_capacity = a.cell_capacity;
+    const int cand_capacity = a.cand_capacity;
+    // written by the atomics of other blocks: read at L2
+    const unsigned long long M = __ldcg(&h->M);
+    const uint32_t status = __ldcg(&h->status);
+    if (M > (unsigned long long)src_capacity) atomicOr(&h->status, DYNB_RG_SRC_OVERFLOW);
+    for (int k = 0; k < 3; k++) { h->clip_lo[k] = -1.0e300; h->clip_hi[k] = 1.0e300; }
+    if (M == 0 || M > (unsigned long long)src_capacity || (status & RG_FATAL)) {
+        h->nx = h->ny = h->nz = 1;
+        h->ncell_plus1 = 2;
+        h->pad = 1;
+        h->group_cells = 1;
+        h->group_cells_y = 1;
+        h->gx = 1;
+        h->num_groups = 0;
+        h->gmin[0] = h->gmin[1] = h->gmin[2] = 0.0;
+        h->res_inv = 1.0;
+        return;
+    }
+    double lo[3], ext[3];
+    for (int k = 0; k < 3; k++) {
+        lo[k] = unordered_any<T>(__ldcg(&h->bb_min[k])) - 0.01;
+        double hi = unordered_any<T>(__ldcg(&h->bb_max[k])) + 0.01;
+        const unsigned long long tmin = __ldcg(&h->tb_min[k]), tmax = __ldcg(&h->tb_max[k]);
+        if (subset && tmin <= tmax) {
+            // clip to the targets' box grown by the cutoff (with slack far above any rounding)
+            const double margin = radius * 1.001 + 0.02;
+            const double tlo = unordered_any<T>(tmin) - margin, thi = unordered_any<T>(tmax) + margin;
+            if (tlo > lo[k]) lo[k] = tlo;
+            if (thi < hi) hi = thi;
+            h->clip_lo[k] = lo[k];
+            h->clip_hi[k] = hi;
+            if (hi < lo[k]) hi = lo[k];
+        }
+        ext[k] = hi - lo[k];
+    }
+    GridChoice gc;
+    rg_choose_grid(lo, ext, radius, cell_capacity, cand_capacity, (double)M, 0.0, !subset, gc);
+    rg_store_grid(*h, gc);
+}
+template <typename T>
+__device__ __forceinline__ void rg_last_block_chooses(DevHeader* h, const GridArgs& a, bool subset)
+{
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (atomicAdd(&h->arrived, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    rg_choose_grid_device<T>(h, a, subset);
+}
+
 constexpr int WRAP_THREADS = 256;
 
 // FUSED: the grid is known before the launch (gc, chosen on the host), so the images and the targets are counted
@@ -292,7 +355,7 @@ constexpr int WRAP_THREADS = 256;
 template <typename T, bool FUSED>
 __global__ void __launch_bounds__(WRAP_THREADS)
 rg_wrap_kernel(const T* __restrict__ pos, int64_t N, Geom<T> g, int vec_ok, Vec4<T>* __restrict__ posw,
-               int4* __restrict__ aff, DevHeader* __restrict__ h, unsigned long long* __restrict__ partials,
+               int4* __restrict__ aff, DevHeader* __restrict__ h, const GridArgs ga, int subset,
                const GridChoice gc, uint32_t* __restrict__ ccount, uint32_t* __restrict__ tccount)
 {
     __shared__ T stage[WRAP_THREADS * 3];
@@ -411,7 +474,7 @@ rg_wrap_kernel(const T* __restrict__ pos, int64_t N, Geom<T> g, int vec_ok, Vec4
     if (lane == 0) {
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            // "no image" stays the 64-bit identity of the minimum that rg_grid_kernel expects
+            // "no image" stays the 64-bit identity of the minimum
             red[k][warp] = (mn[k] == ~(Key)0) ? ~0ull : (unsigned long long)mn[k];
             red[3 + k][warp] = (unsigned long long)mx[k];
         }
@@ -419,40 +482,29 @@ rg_wrap_kernel(const T* __restrict__ pos, int64_t N, Geom<T> g, int vec_ok, Vec4
         if (status) atomicOr(&h->status, status);
     }
     __syncthreads();
-    if (FUSED) {
-        // the bounding box goes straight to the header (it only steers the shape of the work items, which is
-        // settled three launches later): six fire-and-forget atomics per block
-        if (threadIdx.x < 6) {
-            unsigned long long v = red[threadIdx.x][0];
-            for (int w = 1; w < WRAP_THREADS / 32; w++)
-                v = (threadIdx.x < 3) ? min(v, red[threadIdx.x][w]) : max(v, red[threadIdx.x][w]);
-            if (threadIdx.x < 3) atomicMin(&h->bb_min[threadIdx.x], v);
-            else atomicMax(&h->bb_max[threadIdx.x - 3], v);
-        }
-        return;
-    }
-    // per-block partial results (bounding box, image count); rg_grid_kernel reduces them, so that no
-    // block contends for a handful of header words
+    // the bounding box goes straight to the header: six fire-and-forget atomics per block (with a grid chosen on the host it
+    // only steers the shape of the work items, which is settled three launches later)
     if (threadIdx.x < 6) {
         unsigned long long v = red[threadIdx.x][0];
         for (int w = 1; w < WRAP_THREADS / 32; w++)
             v = (threadIdx.x < 3) ? min(v, red[threadIdx.x][w]) : max(v, red[threadIdx.x][w]);
-        partials[(size_t)blockIdx.x * 8 + threadIdx.x] = v;
-    } else if (threadIdx.x == 6) {
+        if (threadIdx.x < 3) atomicMin(&h->bb_min[threadIdx.x], v);
+        else atomicMax(&h->bb_max[threadIdx.x - 3], v);
+    } else if (!FUSED && threadIdx.x == 6) {
         unsigned long long c = 0;
         for (int w = 0; w < WRAP_THREADS / 32; w++) c += red_cnt[w];
-        partials[(size_t)blockIdx.x * 8 + 6] = c;
+        atomicAdd(&h->M, c);
     }
+    if (!FUSED && !subset) rg_last_block_chooses<T>(h, ga, false);
 }
 
-// Bounding box of the wrapped TARGET positions (only when a target subset is given): per-block
-// partials, reduced by rg_grid_kernel.  Sources farther than the cutoff from that box are never
+// Bounding box of the wrapped TARGET positions (only when a target subset is given), then the grid.  Sources farther than the cutoff from that box are never
 // needed, which keeps the grid and the image count small when a rank builds edges for its own
 // atoms only.
 template <typename T>
 __global__ void __launch_bounds__(256)
 rg_target_bbox_kernel(const int64_t* __restrict__ targets, int64_t Nt, int64_t N, const Vec4<T>* __restrict__ posw,
-                      unsigned long long* __restrict__ partials)
+                      DevHeader* __restrict__ h, const GridArgs ga)
 {
     __shared__ unsigned long long red[6][8];
     unsigned long long v[6] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
@@ -479,118 +531,10 @@ rg_target_bbox_kernel(const int64_t* __restrict__ targets, int64_t Nt, int64_t N
     if (threadIdx.x < 6) {
         unsigned long long a = red[threadIdx.x][0];
         for (int w = 1; w < 8; w++) a = (threadIdx.x < 3) ? min(a, red[threadIdx.x][w]) : max(a, red[threadIdx.x][w]);
-        partials[(size_t)blockIdx.x * 8 + threadIdx.x] = a;
+        if (threadIdx.x < 3) atomicMin(&h->tb_min[threadIdx.x], a);
+        else atomicMax(&h->tb_max[threadIdx.x - 3], a);
     }
-}
-
-// ------------------------------------------------------------------------------------------
-// rg_grid: one thread chooses the grid.  Cells of edge radius/1.99 scanned +-2 (as the
-// reference, :662,776) unless that would need more than cell_capacity cells; then the cells
-// grow, and once they are wider than the cutoff the scan shrinks to +-1.
-// ------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(1024)
-rg_grid_kernel(DevHeader* h, double radius, long long src_capacity, long long cell_capacity, int cand_capacity,
-               const unsigned long long* __restrict__ partials, int num_partials,
-               const unsigned long long* __restrict__ tpartials, int num_tpartials)
-{
-    {   // reduce the per-block partials of rg_wrap_kernel into the header
-        __shared__ unsigned long long red[7][32];
-        unsigned long long v[7] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull, 0ull};
-#pragma unroll 4
-        for (int b = threadIdx.x; b < num_partials; b += blockDim.x) {  // independent loads, several in flight
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                v[k] = min(v[k], partials[(size_t)b * 8 + k]);
-                v[3 + k] = max(v[3 + k], partials[(size_t)b * 8 + 3 + k]);
-            }
-            v[6] += partials[(size_t)b * 8 + 6];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                v[k] = min(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-                v[3 + k] = max(v[3 + k], __shfl_xor_sync(0xffffffffu, v[3 + k], o));
-            }
-            v[6] += __shfl_xor_sync(0xffffffffu, v[6], o);
-        }
-        if ((threadIdx.x & 31) == 0)
-            for (int k = 0; k < 7; k++) red[k][threadIdx.x >> 5] = v[k];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int k = 0; k < 7; k++) {
-                unsigned long long a = red[k][0];
-                for (int w = 1; w < (int)(blockDim.x >> 5); w++)
-                    a = (k < 3) ? min(a, red[k][w]) : (k < 6 ? max(a, red[k][w]) : a + red[k][w]);
-                if (k < 3) h->bb_min[k] = a; else if (k < 6) h->bb_max[k - 3] = a; else h->M = a;
-            }
-        }
-    }
-    __shared__ unsigned long long tbox[6];
-    {   // bounding box of the target subset (if any), same block reduction
-        __shared__ unsigned long long tred[6][32];
-        unsigned long long v[6] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
-#pragma unroll 4
-        for (int b = threadIdx.x; b < num_tpartials; b += blockDim.x) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                v[k] = min(v[k], tpartials[(size_t)b * 8 + k]);
-                v[3 + k] = max(v[3 + k], tpartials[(size_t)b * 8 + 3 + k]);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                v[k] = min(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-                v[3 + k] = max(v[3 + k], __shfl_xor_sync(0xffffffffu, v[3 + k], o));
-            }
-        if ((threadIdx.x & 31) == 0)
-            for (int k = 0; k < 6; k++) tred[k][threadIdx.x >> 5] = v[k];
-        __syncthreads();
-        if (threadIdx.x < 6) {
-            unsigned long long a = tred[threadIdx.x][0];
-            for (int w = 1; w < (int)(blockDim.x >> 5); w++)
-                a = (threadIdx.x < 3) ? min(a, tred[threadIdx.x][w]) : max(a, tred[threadIdx.x][w]);
-            tbox[threadIdx.x] = a;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (h->M > (unsigned long long)src_capacity) h->status |= DYNB_RG_SRC_OVERFLOW;
-    for (int k = 0; k < 3; k++) { h->clip_lo[k] = -1.0e300; h->clip_hi[k] = 1.0e300; }
-    if (h->M == 0 || (h->status & RG_FATAL)) {
-        h->nx = h->ny = h->nz = 1;
-        h->ncell_plus1 = 2;
-        h->pad = 1;
-        h->group_cells = 1;
-        h->group_cells_y = 1;
-        h->gx = 1;
-        h->num_groups = 0;
-        h->gmin[0] = h->gmin[1] = h->gmin[2] = 0.0;
-        h->res_inv = 1.0;
-        return;
-    }
-    double lo[3], ext[3];
-    for (int k = 0; k < 3; k++) {
-        lo[k] = unordered_any<T>(h->bb_min[k]) - 0.01;
-        double hi = unordered_any<T>(h->bb_max[k]) + 0.01;
-        if (num_tpartials > 0 && tbox[k] <= tbox[3 + k]) {
-            // clip to the targets' box grown by the cutoff (with slack far above any rounding)
-            const double margin = radius * 1.001 + 0.02;
-            const double tlo = unordered_any<T>(tbox[k]) - margin, thi = unordered_any<T>(tbox[3 + k]) + margin;
-            if (tlo > lo[k]) lo[k] = tlo;
-            if (thi < hi) hi = thi;
-            h->clip_lo[k] = lo[k];
-            h->clip_hi[k] = hi;
-            if (hi < lo[k]) hi = lo[k];
-        }
-        ext[k] = hi - lo[k];
-    }
-    GridChoice gc;
-    rg_choose_grid(lo, ext, radius, cell_capacity, cand_capacity, (double)h->M, 0.0, num_tpartials == 0, gc);
-    rg_store_grid(*h, gc);
+    rg_last_block_chooses<T>(h, ga, true);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1805,7 +1749,7 @@ rg_init_kernel(uint32_t* __restrict__ hdr, const HeaderBlock blk, uint4* __restr
 // host side
 // ------------------------------------------------------------------------------------------
 struct RgLayout {
-    int64_t hdr, partials, tpartials, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, smeta, hitmask, trec, tpos, tscan, tmeta,
+    int64_t hdr, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, smeta, hitmask, trec, tpos, tscan, tmeta,
         tcount, toffset, sums, total;
 };
 
@@ -1816,13 +1760,11 @@ static RgLayout rg_layout(int64_t N, int64_t Nt, int64_t src_cap, int64_t cell_c
     int64_t o = 0;
     auto take = [&](int64_t bytes) { int64_t r = o; o = align_up(o + bytes, 256); return r; };
     L.hdr = take(RG_HEADER_BYTES);
-    // zero-initialised block: cell counters (contiguous so that one memset clears them)
+    // cell counters, cleared in one pass; the fill cursors are written by the prefix sum
     L.ccount = take((cell_cap + 2) * 4);
-    L.cfill = take((cell_cap + 2) * 4);
     L.tccount = take((cell_cap + 2) * 4);
+    L.cfill = take((cell_cap + 2) * 4);
     L.tcfill = take((cell_cap + 2) * 4);
-    L.partials = take(((N + 255) / 256 + 1) * 64);
-    L.tpartials = take(((Nt + 255) / 256 + 1) * 64);
     L.posw = take(N * v4);
     L.aff = take(N * 16);
     const int64_t slot = dtype == DYNB_F64 ? sizeof(SlotRec<double>) : sizeof(SlotRec<float>);
@@ -2008,7 +1950,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     {
         DevHeader hi;
         memset(&hi, 0, sizeof(hi));
-        for (int k = 0; k < 3; k++) { hi.bb_min[k] = ~0ull; hi.bb_max[k] = 0ull; }
+        for (int k = 0; k < 3; k++) { hi.bb_min[k] = hi.tb_min[k] = ~0ull; hi.bb_max[k] = hi.tb_max[k] = 0ull; }
         if (host_grid) {
             rg_store_grid(hi, gc_host);
             for (int k = 0; k < 3; k++) { hi.clip_lo[k] = -1.0e300; hi.clip_hi[k] = 1.0e300; }
@@ -2026,7 +1968,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         HeaderBlock blk;
         memcpy(blk.words, init, sizeof(init));
         // every region of the layout starts on a 256-byte boundary and is padded to one
-        const int64_t n_a16 = (L.partials - L.ccount) / 16, n_b16 = bins_only ? 0 : ((Nt + 1) * 4 + 15) / 16;
+        const int64_t n_a16 = (L.cfill - L.ccount) / 16, n_b16 = bins_only ? 0 : ((Nt + 1) * 4 + 15) / 16;
         rg_init_kernel<<<sm_count_cached() * 4, 256, 0, stream>>>(reinterpret_cast<uint32_t*>(w + L.hdr), blk,
                                                                   reinterpret_cast<uint4*>(w + L.ccount), n_a16,
                                                                   reinterpret_cast<uint4*>(w + L.tcount), n_b16, counts_out, Nt);
@@ -2036,21 +1978,13 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     const int64_t nb = std::max(N, Nt);
     if (host_grid) {
         rg_wrap_kernel<T, true><<<(unsigned)((N + WRAP_THREADS - 1) / WRAP_THREADS), WRAP_THREADS, 0, stream>>>(
-            static_cast<const T*>(pos_dev), N, g, vec_ok, posw, aff, h, nullptr, gc_host, ccount, tccount);
+            static_cast<const T*>(pos_dev), N, g, vec_ok, posw, aff, h, GridArgs{}, 0, gc_host, ccount, tccount);
     } else {
+        const GridArgs ga = {radius, (long long)src_cap, (long long)cell_cap, PAIR_CAND_BYTES / (int)sizeof(Vec4<T>)};
         rg_wrap_kernel<T, false><<<(unsigned)((N + WRAP_THREADS - 1) / WRAP_THREADS), WRAP_THREADS, 0, stream>>>(
-            static_cast<const T*>(pos_dev), N, g, vec_ok, posw, aff, h, reinterpret_cast<unsigned long long*>(w + L.partials), gc_host,
-            nullptr, nullptr);
-        int n_tpart = 0;
-        if (targets != nullptr) {
-            n_tpart = (int)((Nt + 255) / 256);
-            rg_target_bbox_kernel<T><<<n_tpart, 256, 0, stream>>>(targets, Nt, N, posw, reinterpret_cast<unsigned long long*>(w + L.tpartials));
-        }
-        rg_grid_kernel<T><<<1, 1024, 0, stream>>>(h, radius, (long long)src_cap, (long long)cell_cap,
-                                                 PAIR_CAND_BYTES / (int)sizeof(Vec4<T>),
-                                                 reinterpret_cast<const unsigned long long*>(w + L.partials),
-                                                 (int)((N + WRAP_THREADS - 1) / WRAP_THREADS),
-                                                 reinterpret_cast<const unsigned long long*>(w + L.tpartials), n_tpart);
+            static_cast<const T*>(pos_dev), N, g, vec_ok, posw, aff, h, ga, targets != nullptr ? 1 : 0, gc_host, nullptr, nullptr);
+        if (targets != nullptr)
+            rg_target_bbox_kernel<T><<<(unsigned)((Nt + 255) / 256), 256, 0, stream>>>(targets, Nt, N, posw, h, ga);
         rg_bin_kernel<T, false><<<(unsigned)((nb + 255) / 256), 256, 0, stream>>>(
             N, Nt, targets, g, posw, aff, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap, 0);
     }

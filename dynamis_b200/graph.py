@@ -388,12 +388,12 @@ def launches_per_graph(target_subset: bool = False, fully_periodic: bool = True)
     (which also counts the images into their cells: the grid follows from the cell), 2 scan kernels (source and
     target cell starts together), scatter, finalize, count pass (degrees included), 2 scan kernels (edge offsets),
     the edge writer.  One more (the pass that recomputes distances) when a candidate list was too long for its hit
-    bits.  Two more (grid from the data's bounding box, cell histogram) when a direction is not periodic or a target
-    subset is given, and two more again (the targets' bounding box, the list of groups with targets) with a target
-    subset."""
+    bits.  One more (the cell histogram; the grid from the data's bounding box is chosen by the last block of the wrap)
+    when a direction is not periodic or a target subset is given, and two more again (the targets' bounding box, the
+    list of groups with targets) with a target subset."""
     n = 10
     if target_subset or not fully_periodic:
-        n += 2
+        n += 1
     if target_subset:
         n += 2
     return n
