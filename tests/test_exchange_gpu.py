@@ -144,6 +144,14 @@ def test_emulated_ranks_match_oracle(cuda, W, F, dtype):
         e.teardown()
 
 
+@pytest.mark.parametrize("F,dtype", [(1, torch.float32), (8, torch.float32), (16, torch.float32), (20, torch.float32), (64, torch.float32),
+                                     (124, torch.float32), (65, torch.float32), (132, torch.float32), (256, torch.float32),
+                                     (16, torch.float64), (33, torch.float64)])
+def test_row_widths_match_oracle(cuda, F, dtype):
+    """Rows that lie side by side in a warp (fewer than 32 vectors, whether or not they divide 32), exactly 32 and more."""
+    test_emulated_ranks_match_oracle(cuda, 3, F, dtype)
+
+
 def test_wait_budget_expires_with_status_not_a_hang(cuda):
     """A peer that never signals: the bounded wait runs out after its budget, sets the status words,
     and the context stays usable.  The library path reports it by itself: the next push raises

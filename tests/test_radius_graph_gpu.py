@@ -360,6 +360,18 @@ def test_distances_from_hit_bits(cuda, dtype, lists):
     assert float((d2.double() - (vec * vec).sum(dim=1)).abs().max()) <= bound
 
 
+@pytest.mark.parametrize("n_targets", [1, 2, 3, 16, 31, 33])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_few_targets_per_group(cuda, n_targets, dtype):
+    """Odd and even numbers of targets in a group, some without any neighbour: the edge writer takes them two at a time."""
+    rng = np.random.default_rng(n_targets)
+    pos = np.concatenate([rng.random((400, 3)) * 8.0, 20.0 + rng.random((6, 3)) * 15.0]).astype(dtype)
+    cell = (np.eye(3) * 40.0).astype(dtype)
+    targets = np.concatenate([[400], rng.permutation(406)[: n_targets - 1]]).astype(np.int64)
+    _check_vs_oracle(pos, cell, [True] * 3, 3.0, cuda, targets, what=f"{n_targets} targets")
+    _check_vs_oracle(pos[: 400 + n_targets % 6], cell, [True, True, False], 3.0, cuda, what="all")
+
+
 def test_edge_distances_fp32(cuda):
     import dynamis_b200 as D
 
