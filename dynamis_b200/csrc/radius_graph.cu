@@ -5,16 +5,18 @@
 //
 // Pipeline (one stream, no host synchronisation inside the plan):
 //   rg_wrap        wrap positions into the unit cell, classify which periodic images each atom
-//                  needs, per-block bounding box of all images           (ref :596-605, :18-67)
+//                  needs, bounding box of all images                     (ref :596-605, :18-67)
 //   rg_target_bbox bounding box of the targets (only with a target subset)
-//   rg_grid        one block: reduce the boxes, choose the cell grid on the device (ref :662-692)
-//   rg_bin_count   histogram of images / targets per cell (atomics)      (ref :146-171)
+//                  the last block of these two chooses the cell grid, unless the host could (ref :662-692)
+//   rg_bin_count   histogram of images / targets per cell (atomics; part of rg_wrap with a grid from the host)
+//                                                                        (ref :146-171)
 //   scan           cell starts
 //   rg_bin_scatter provisional slot inside each cell (atomic rank)
 //   rg_bin_finalize deterministic order inside each cell, write packed source / target records
 //   rg_pair<COUNT> per-target degree                                     (ref :197-258)
 //   scan           edge offsets + total
-//   rg_pair<FILL>  edges                                                 (ref :282-442)
+//   rg_fillmask    edges from the hit bits of the count pass             (ref :282-442)
+//   rg_pair<FILL>  edges of groups whose candidate list is too long for hit bits
 //
 // The edge SET is fixed by three predicates that are kept expression-for-expression identical to
 // the reference (same operand order, compiled with the same default FMA contraction): the wrap,
