@@ -897,6 +897,7 @@ template <typename T> struct PairParams {
     int32_t* counts_out;      // [Nt] degrees in caller order, or nullptr
     const uint32_t* glist;    // groups that hold at least one target (h->active_groups entries), or nullptr = all groups
     uint32_t* long_list;      // groups whose candidate list exceeds the hit bits (h->long_groups entries, written by COUNT)
+    long long n_targets;
     T r2;
 };
 // The plan stores its PairParams inside the workspace (after the header) so that the fill call
@@ -1505,7 +1506,7 @@ struct HaloArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo, int64_t Nt)
+rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo)
 {
     const PairParams<T> p = *params_dev;
     if (p.h->status & RG_FATAL) return;
@@ -1513,7 +1514,7 @@ rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArg
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t sa = -1, ta = -1;
     if (j < M) sa = (int64_t)p.smeta[j].x;
-    if (j < Nt) ta = (int64_t)p.tmeta[j].x;
+    if (j < p.n_targets) ta = (int64_t)p.tmeta[j].x;  // the plan's, whatever the number of owners
     if (sa >= 0) halo.sown[j] = (unsigned short)halo.owner[sa];
     if (ta >= 0) halo.town[j] = (unsigned short)halo.owner[ta];
 }
@@ -1986,6 +1987,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         // the targets' fill counters are free once the targets are binned: they hold the list of groups with targets
         pp.glist = (targets != nullptr) ? tcfill : nullptr;
         pp.long_list = cfill;   // likewise free once the sources are binned
+        pp.n_targets = Nt;
         memcpy(init + RG_PARAMS_OFFSET, &pp, sizeof(pp));
     }
     {
@@ -2084,7 +2086,7 @@ static int rg_halo_mark(const void* ws, HaloArgs ha, int64_t N, int64_t src_cap,
 {
     const unsigned char* w = static_cast<const unsigned char*>(ws);
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
-    rg_halo_owner_kernel<T><<<(unsigned)((std::max(N, src_cap) + 255) / 256), 256, 0, stream>>>(params_dev, ha, N);
+    rg_halo_owner_kernel<T><<<(unsigned)((std::max(N, src_cap) + 255) / 256), 256, 0, stream>>>(params_dev, ha);
     rg_halo_runs_kernel<T><<<(unsigned)std::min<int64_t>((cell_cap + 255) / 256, (int64_t)sm_count_cached() * 8), 256, 0, stream>>>(params_dev, ha);
     const int grid = sm_count_cached() * 4 * PAIR_GRID_WAVES;
     if (ha.words == 1) rg_halo_kernel<T, false><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);

@@ -346,3 +346,23 @@ def test_select_eq_at_tile_edges(cuda, n):
     src = torch.arange(n, device=cuda) * 7
     assert torch.equal(select_eq(v, 1), torch.nonzero(v == 1).reshape(-1))
     assert torch.equal(select_eq(v, 2, src), src[v == 2])
+
+
+HALO_LISTS = ("send_offsets", "send_local_indices", "recv_offsets", "recv_ghost_indices", "recv_atom_global", "interior_mask")
+
+
+def test_halo_maps_with_owners_of_more_atoms_than_positions(cuda):
+    """Atoms that have an owner but no position have no neighbours: they are in nobody's list, and interior."""
+    pos, cell = _halo_case(17, 1500, 24.0)
+    extra, W = 700, 3
+    owner = np.random.default_rng(4).integers(0, W, pos.shape[0] + extra)
+    g = O.radius_graph(pos, cell, [1, 1, 1], np.float32(5.5))
+    for r in range(W):
+        info = D.PartitionMessagePassingInfo()
+        info.partition_id = torch.as_tensor(owner, device=cuda)
+        st = _state(pos, cuda)
+        st.num_atoms = owner.size
+        D.SFCPartitioner().build_halo_maps(info, st, _env(r, W), _cfg(cell, 5.0, 0.5))
+        ref = O.build_halo_maps(g["src"], g["dst"], owner, r, W)
+        for key in HALO_LISTS:
+            np.testing.assert_array_equal(getattr(info, key).cpu().numpy(), ref[key])
