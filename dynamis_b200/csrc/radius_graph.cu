@@ -898,6 +898,10 @@ template <typename T> struct PairParams {
     const uint32_t* glist;    // groups that hold at least one target (h->active_groups entries), or nullptr = all groups
     uint32_t* long_list;      // groups whose candidate list exceeds the hit bits (h->long_groups entries, written by COUNT)
     long long n_targets;
+    // halo marking only (rg_halo_*): owner of every source record and of every target, and a word for every candidate run
+    unsigned short* sown;     // [M]; lies over the binning slots, which nothing reads behind the plan
+    unsigned short* town;     // [n_targets]; likewise
+    unsigned short* run_owner;  // [gx * ny * nz]
     T r2;
 };
 // The plan stores its PairParams inside the workspace (after the header) so that the fill call
@@ -1495,9 +1499,6 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
 constexpr int HALO_EMPTY = 0x7fff, HALO_MIXED = 0x7ffe, HALO_RANK = 0x8000;
 struct HaloArgs {
     const long long* owner;      // [n_atoms] rank of each atom
-    unsigned short* sown;        // [M] owner of every source record
-    unsigned short* town;        // [Nt] owner of every target
-    unsigned short* run_owner;   // [gx * ny * nz] word of every candidate run
     uint32_t* needed;            // [n_atoms, words]
     unsigned char* has_foreign;  // [n_atoms]
     int words;
@@ -1511,12 +1512,14 @@ rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArg
     const PairParams<T> p = *params_dev;
     if (p.h->status & RG_FATAL) return;
     const int64_t M = (int64_t)p.h->M;
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t sa = -1, ta = -1;
-    if (j < M) sa = (int64_t)p.smeta[j].x;
-    if (j < p.n_targets) ta = (int64_t)p.tmeta[j].x;  // the plan's, whatever the number of owners
-    if (sa >= 0) halo.sown[j] = (unsigned short)halo.owner[sa];
-    if (ta >= 0) halo.town[j] = (unsigned short)halo.owner[ta];
+    const int64_t end = max(M, (int64_t)p.n_targets);  // the plan's targets, whatever the number of owners
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < end; j += (int64_t)gridDim.x * blockDim.x) {
+        int64_t sa = -1, ta = -1;
+        if (j < M) sa = (int64_t)p.smeta[j].x;
+        if (j < p.n_targets) ta = (int64_t)p.tmeta[j].x;
+        if (sa >= 0) p.sown[j] = (unsigned short)halo.owner[sa];
+        if (ta >= 0) p.town[j] = (unsigned short)halo.owner[ta];
+    }
 }
 
 template <typename T>
@@ -1535,12 +1538,12 @@ rg_halo_runs_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs
         int o = HALO_EMPTY;
         bool found = false;
         if (a < e) {
-            o = (int)halo.sown[a];
+            o = (int)p.sown[a];
             found = halo.rank < 0 || o == halo.rank;
             for (uint32_t j = a + 1; j < e && !(found && o == HALO_MIXED); j += 4) {
                 int v[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) v[u] = (int)halo.sown[min(j + u, e - 1)];
+                for (int u = 0; u < 4; u++) v[u] = (int)p.sown[min(j + u, e - 1)];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     if (v[u] != o) o = HALO_MIXED;
@@ -1548,7 +1551,7 @@ rg_halo_runs_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs
                 }
             }
         }
-        halo.run_owner[i] = (unsigned short)(o | (found ? HALO_RANK : 0));
+        p.run_owner[i] = (unsigned short)(o | (found ? HALO_RANK : 0));
     }
 }
 
@@ -1628,7 +1631,7 @@ __device__ __forceinline__ void halo_batch(const PairParams<T>& p, const HaloArg
         if (keep) {
             const int at = near + __popc(m & lt);
             w.cand[at] = c;
-            w.cand_owner[at] = (int)halo.sown[rec];
+            w.cand_owner[at] = (int)p.sown[rec];
         }
         near += __popc(m);
         __syncwarp();
@@ -1669,7 +1672,7 @@ rg_halo_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo
         int run_word;
         {   // nothing to do when all records around the group (its targets' own records among them) have one owner, or
             // when none of them belongs to the rank of interest
-            const int word = has_run ? (int)halo.run_owner[((uint32_t)zz * ny + yy) * gx + ix] : HALO_EMPTY, o = word & 0x7fff;
+            const int word = has_run ? (int)p.run_owner[((uint32_t)zz * ny + yy) * gx + ix] : HALO_EMPTY, o = word & 0x7fff;
             if (!__any_sync(0xffffffffu, word & HALO_RANK)) continue;
             const int lo = __reduce_min_sync(0xffffffffu, o), hi = __reduce_max_sync(0xffffffffu, o == HALO_EMPTY ? 0 : o);
             if (lo == hi && lo != HALO_MIXED) continue;
@@ -1693,7 +1696,7 @@ rg_halo_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo
         for (int q0 = 0; q0 < ntot; q0 += HALO_TARGETS) {
             const int nt = min(HALO_TARGETS, ntot - q0);
             const uint32_t t = (q0 + lane < n0) ? tb0 + q0 + lane : tb1 + (q0 + lane - n0);
-            const int ot = (lane < nt) ? (int)halo.town[t] : 0;
+            const int ot = (lane < nt) ? (int)p.town[t] : 0;
             const int lo = __reduce_min_sync(0xffffffffu, lane < nt ? ot : 0x7fffffff), hi = __reduce_max_sync(0xffffffffu, ot);
             const bool uniform = lo == hi, any_rank = rank < 0 || __any_sync(0xffffffffu, lane < nt && ot == rank);
             HaloBatch b;
@@ -1726,7 +1729,7 @@ rg_halo_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo
             for (int i0 = 0; i0 < longest; i0 += 8) {
                 int o[8];
 #pragma unroll
-                for (int u = 0; u < 8; u++) o[u] = (i0 + u < len) ? (int)halo.sown[run_a + i0 + u] : -1;
+                for (int u = 0; u < 8; u++) o[u] = (i0 + u < len) ? (int)p.sown[run_a + i0 + u] : -1;
                 uint32_t keep = 0;
 #pragma unroll
                 for (int u = 0; u < 8; u++)
@@ -1775,7 +1778,7 @@ rg_init_kernel(uint32_t* __restrict__ hdr, const HeaderBlock blk, uint4* __restr
 // ------------------------------------------------------------------------------------------
 struct RgLayout {
     int64_t hdr, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, smeta, hitmask, trec, tpos, tscan, tmeta,
-        tcount, toffset, sums, total;
+        tcount, toffset, runs, sums, total;
 };
 
 static RgLayout rg_layout(int64_t N, int64_t Nt, int64_t src_cap, int64_t cell_cap, int dtype)
@@ -1804,6 +1807,7 @@ static RgLayout rg_layout(int64_t N, int64_t Nt, int64_t src_cap, int64_t cell_c
     L.tmeta = take(Nt * 16);
     L.tcount = take((Nt + 1) * 4);
     L.toffset = take((Nt + 2) * 8);
+    L.runs = take((cell_cap + 2) * 2);
     const int64_t tiles = std::max<int64_t>(scan_num_tiles(cell_cap + 2), scan_num_tiles(Nt + 2)) + 1;
     L.sums = take(tiles * 8 * 2);
     L.total = o;
@@ -1988,6 +1992,10 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         pp.glist = (targets != nullptr) ? tcfill : nullptr;
         pp.long_list = cfill;   // likewise free once the sources are binned
         pp.n_targets = Nt;
+        static_assert(sizeof(SlotRec<T>) >= sizeof(unsigned short), "owners lie over the binning slots");
+        pp.sown = reinterpret_cast<unsigned short*>(srec);
+        pp.town = reinterpret_cast<unsigned short*>(trec);
+        pp.run_owner = reinterpret_cast<unsigned short*>(w + L.runs);
         memcpy(init + RG_PARAMS_OFFSET, &pp, sizeof(pp));
     }
     {
@@ -2082,12 +2090,13 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
 }
 
 template <typename T>
-static int rg_halo_mark(const void* ws, HaloArgs ha, int64_t N, int64_t src_cap, int64_t cell_cap, cudaStream_t stream)
+static int rg_halo_mark(const void* ws, const HaloArgs& ha, int64_t N, cudaStream_t stream)
 {
     const unsigned char* w = static_cast<const unsigned char*>(ws);
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
-    rg_halo_owner_kernel<T><<<(unsigned)((std::max(N, src_cap) + 255) / 256), 256, 0, stream>>>(params_dev, ha);
-    rg_halo_runs_kernel<T><<<(unsigned)std::min<int64_t>((cell_cap + 255) / 256, (int64_t)sm_count_cached() * 8), 256, 0, stream>>>(params_dev, ha);
+    // the numbers of records and runs are known on the device only: both passes stride
+    rg_halo_owner_kernel<T><<<(unsigned)std::max<int64_t>((N + 255) / 256, (int64_t)sm_count_cached() * 4), 256, 0, stream>>>(params_dev, ha);
+    rg_halo_runs_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, ha);
     const int grid = sm_count_cached() * 4 * PAIR_GRID_WAVES;
     if (ha.words == 1) rg_halo_kernel<T, false><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
     else rg_halo_kernel<T, true><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
@@ -2201,28 +2210,28 @@ extern "C" int dynb_rg_fill_glue(const void* workspace_dev, int dtype, int64_t* 
     return rg_fill_any(workspace_dev, dtype, edge_index_dev, unit_shifts_dev, nullptr, &g, nullptr, E, true, stream);
 }
 
-extern "C" int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
-                                 int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev,
-                                 int64_t src_capacity, int64_t cell_capacity, void* scratch_dev, int64_t scratch_bytes, void* stream)
+extern "C" int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
+                                      int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream)
 {
-    if (workspace_dev == nullptr || owner_dev == nullptr || needed_dev == nullptr || has_foreign_dev == nullptr || scratch_dev == nullptr)
+    if (workspace_dev == nullptr || owner_dev == nullptr || needed_dev == nullptr || has_foreign_dev == nullptr)
         return fail_arg("null pointer");
     if (n_atoms <= 0 || world_size < 1 || world_size > 32000 || rank < -1 || rank >= world_size) return fail_arg("bad sizes");
-    if (src_capacity < 1 || cell_capacity < 1 || scratch_bytes < 2 * (n_atoms + src_capacity + cell_capacity))
-        return fail_arg("scratch must hold 2 * (n_atoms + src_capacity + cell_capacity) bytes");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     HaloArgs ha;
     ha.owner = reinterpret_cast<const long long*>(owner_dev);
-    ha.town = static_cast<unsigned short*>(scratch_dev);
-    ha.sown = ha.town + n_atoms;
-    ha.run_owner = ha.sown + src_capacity;
     ha.needed = needed_dev;
     ha.has_foreign = has_foreign_dev;
     ha.words = (int)((world_size + 31) / 32);
     ha.rank = (int)rank;
     DYNB_CUDA_OK(cudaMemsetAsync(needed_dev, 0, (size_t)n_atoms * ha.words * 4, s));
     DYNB_CUDA_OK(cudaMemsetAsync(has_foreign_dev, 0, (size_t)n_atoms, s));
-    if (dtype == DYNB_F32) return rg_halo_mark<float>(workspace_dev, ha, n_atoms, src_capacity, cell_capacity, s);
-    if (dtype == DYNB_F64) return rg_halo_mark<double>(workspace_dev, ha, n_atoms, src_capacity, cell_capacity, s);
+    if (dtype == DYNB_F32) return rg_halo_mark<float>(workspace_dev, ha, n_atoms, s);
+    if (dtype == DYNB_F64) return rg_halo_mark<double>(workspace_dev, ha, n_atoms, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");
+}
+
+extern "C" int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
+                                 int64_t world_size, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream)
+{
+    return dynb_rg_halo_mark_rank(workspace_dev, dtype, owner_dev, n_atoms, world_size, -1, needed_dev, has_foreign_dev, stream);
 }

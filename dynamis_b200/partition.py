@@ -8,7 +8,7 @@ bound in dynamis_state/src/dynamis_state_bindings.cpp:75-115): ``SFCPartitioner(
 The compute is in libdynb.so: Morton/"Hilbert" keys, a stable radix sort, the label assignment
 (dynb_sfc_partition), bincount / stream compaction (dynb_bincount_i64, dynb_select_eq_i64), and
 for the halo maps one cell-scan pass at cutoff + buffer that marks which rank needs which atom
-(dynb_rg_halo_mark) followed by the assembly of the lists (dynb_halo_lists_plan / _fill).  Unlike the
+(dynb_rg_halo_mark_rank) followed by the assembly of the lists (dynb_halo_lists_plan / _fill).  Unlike the
 reference, no [N, W] bool matrix and no edge list are materialised.
 """
 
@@ -190,10 +190,8 @@ class AbstractPartitioner:
             while True:
                 if bins is not None:
                     bins.launch()
-                    mark = scratch(dev, "halo_owner", 2 * (N + bins.src_capacity + bins.cell_capacity))
-                    _lib.check(L.dynb_rg_halo_mark(bins.ws.data_ptr(), bins.dtype_code, pid.data_ptr(), N, W, R, needed.data_ptr(),
-                                                   has_foreign.data_ptr(), bins.src_capacity, bins.cell_capacity,
-                                                   mark.data_ptr(), mark.numel(), _stream(dev)), "rg_halo_mark")
+                    _lib.check(L.dynb_rg_halo_mark_rank(bins.ws.data_ptr(), bins.dtype_code, pid.data_ptr(), N, W, R, needed.data_ptr(),
+                                                        has_foreign.data_ptr(), _stream(dev)), "rg_halo_mark")
                 _lib.check(L.dynb_halo_lists_plan(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
                                                   ws.numel(), _stream(dev)), "halo_lists_plan")
                 offs_h.copy_(offs, non_blocking=True)

@@ -114,14 +114,16 @@ int dynb_rg_bin(const void* pos_dev, int dtype, int64_t n_atoms, const void* cel
 
 /* Halo marking over a plan (all atoms as targets, radius = cutoff + ghost buffer) or over dynb_rg_bin: for every edge
  * src -> dst whose endpoints have different owners, sets bit owner[dst] of needed_dev[src * words + ...]
- * (words = ceil(world_size / 32)) and has_foreign_dev[dst] = 1.  rank >= 0: only for edges that start or end at an
- * atom of that rank (all its own halo lists need); -1: for every edge.  Both outputs are cleared first.
- * The capacities are those of the plan; scratch_dev holds 2 * (n_atoms + src_capacity + cell_capacity) bytes.
- * This is the edge loop of build_halo_maps (dynamis_state/src/csrc/build_halo_maps.cpp:50-58, 127-138) without
+ * (words = ceil(world_size / 32), world_size at most 32000) and has_foreign_dev[dst] = 1.  Both outputs are cleared
+ * first.  The owners are gathered into parts of the workspace that the fills do not read.  This is the edge loop of build_halo_maps (dynamis_state/src/csrc/build_halo_maps.cpp:50-58, 127-138) without
  * materialising the graph. */
 int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
-                      int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev,
-                      int64_t src_capacity, int64_t cell_capacity, void* scratch_dev, int64_t scratch_bytes, void* stream);
+                      int64_t world_size, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream);
+
+/* The same for the edges that start or end at an atom of `rank`, which are all that the halo lists of that rank need;
+ * rank = -1: every edge, as dynb_rg_halo_mark. */
+int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
+                           int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream);
 
 /* ------------------------------------------------------------------ SFC partition
  * Replaces sfc_partition_cuda (dynamis_state/src/csrc/partition/sfc.cpp:9-33,

@@ -366,3 +366,37 @@ def test_halo_maps_with_owners_of_more_atoms_than_positions(cuda):
         ref = O.build_halo_maps(g["src"], g["dst"], owner, r, W)
         for key in HALO_LISTS:
             np.testing.assert_array_equal(getattr(info, key).cpu().numpy(), ref[key])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("W", [3, 40])
+def test_halo_mark_of_a_plan_through_the_c_entry(cuda, dtype, W):
+    """dynb_rg_halo_mark over a plan marks every edge whose ends have different owners; the plan can be filled afterwards."""
+    from dynamis_b200 import _lib
+    from dynamis_b200.graph import plan_radius_graph
+
+    pos, cell = _halo_case(8, 1300, 22.0)
+    n, words = pos.shape[0], (W + 31) // 32
+    owner = np.random.default_rng(W).integers(0, W, n)
+    real = np.float64 if dtype == torch.float64 else np.float32
+    g = O.radius_graph(pos.astype(real), cell.astype(real), [1, 1, 1], real(5.0))
+    plan = plan_radius_graph(torch.as_tensor(pos, device=cuda).to(dtype), torch.as_tensor(cell).to(dtype), torch.tensor([True] * 3), 5.0)
+    towner = torch.as_tensor(owner, device=cuda)
+    needed = torch.full((n, words), -1, dtype=torch.int32, device=cuda)
+    foreign = torch.full((n,), 9, dtype=torch.uint8, device=cuda)
+    _lib.check(_lib.lib().dynb_rg_halo_mark(plan.ws.data_ptr(), plan.dtype_code, towner.data_ptr(), n, W, needed.data_ptr(),
+                                            foreign.data_ptr(), torch.cuda.current_stream(cuda).cuda_stream), "rg_halo_mark")
+    ei, cs, _ = plan.fill()
+    assert ei.size(1) == g["E"]
+    cross = owner[g["src"]] != owner[g["dst"]]
+    ref = np.zeros((n, W), bool)
+    ref[g["src"][cross], owner[g["dst"][cross]]] = True
+    bits = needed.cpu().numpy().view(np.uint32)
+    ours = (bits[:, np.arange(words * 32) >> 5] >> (np.arange(words * 32) & 31).astype(np.uint32)) & 1
+    np.testing.assert_array_equal(ours[:, :W].astype(bool), ref)
+    assert not ours[:, W:].any()
+    ref_foreign = np.zeros(n, np.uint8)
+    ref_foreign[g["dst"][cross]] = 1
+    np.testing.assert_array_equal(foreign.cpu().numpy(), ref_foreign)
+    ours_e = np.sort(ei[0].cpu().numpy() * n + ei[1].cpu().numpy())
+    np.testing.assert_array_equal(ours_e, np.sort(g["src"].astype(np.int64) * n + g["dst"]))
