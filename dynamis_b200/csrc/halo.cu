@@ -137,7 +137,8 @@ halo_mark_edges_kernel(const int64_t* __restrict__ src, const int64_t* __restric
 // they follow from one "needed by" mask and the owners (build_halo_maps):
 //   S(a) = owner[a] == me ? ranks that need a, without me : {}
 //   R(a) = owner[a] != me and I need a ? {owner[a]} : {}
-// and the own atoms themselves (owner[a] == me, ascending) give the local indices.
+// and the own atoms themselves (owner[a] == me, ascending) give the local indices.  Peers are ranks below W: an owner or a
+// mask bit beyond them is in no set, in the counting and in the writing pass alike.
 //
 // Both lists, the local indices and the interior mask come out of one counting and one writing pass over the masks; most
 // atoms have empty sets, so a warp (128 consecutive atoms, 32 at a time) works on the peers that occur and on no others.
@@ -152,7 +153,7 @@ struct HaloSets {
     const uint32_t* recv_mask;   // masks of R(a); not read when owner != nullptr
     const int64_t* owner;
     int64_t n, me;
-    int words;
+    int words, W;
 };
 
 // the sets of this lane's HL_ROUNDS atoms (base, base + 32, ...) among the 32 peers of one mask word; all loads first
@@ -172,6 +173,7 @@ __device__ __forceinline__ void halo_sets(const HaloSets& h, int64_t base, int w
         o[k] = (live && owners) ? h.owner[a] : -1;
     }
     own = 0u;
+    const uint32_t peers = h.W - 32 * word < 32 ? (1u << (h.W - 32 * word)) - 1u : ~0u;
 #pragma unroll
     for (int k = 0; k < HL_ROUNDS; k++) {
         s[k] = mw[k];
@@ -180,8 +182,10 @@ __device__ __forceinline__ void halo_sets(const HaloSets& h, int64_t base, int w
             const bool mine = o[k] == h.me;
             if (mine) own |= 1u << k;
             s[k] = !mine ? 0u : (word == (int)(h.me >> 5) ? mw[k] & ~(1u << (h.me & 31)) : mw[k]);
-            r[k] = (!mine && (int)(o[k] >> 5) == word && ((mr[k] >> (h.me & 31)) & 1u)) ? 1u << (o[k] & 31) : 0u;
+            r[k] = (!mine && (o[k] >> 5) == word && ((mr[k] >> (h.me & 31)) & 1u)) ? 1u << (o[k] & 31) : 0u;
         }
+        s[k] &= peers;
+        r[k] &= peers;
     }
 }
 
@@ -557,7 +561,7 @@ static int halo_lists_args(const uint32_t* send_mask_dev, const uint32_t* recv_m
     if (n > 0 && (send_mask_dev == nullptr || (owner_dev == nullptr && recv_mask_dev == nullptr))) return fail_arg("null pointer");
     if (owner_dev != nullptr && (R < 0 || R >= W)) return fail_arg("rank out of range");
     if (W > 4096) return fail_arg("world_size above 4096 is not supported");
-    h = HaloSets{send_mask_dev, recv_mask_dev, owner_dev, n, R, (int)((W + 31) / 32)};
+    h = HaloSets{send_mask_dev, recv_mask_dev, owner_dev, n, R, (int)((W + 31) / 32), (int)W};
     return DYNB_OK;
 }
 

@@ -1497,10 +1497,13 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
 // Word of a candidate run: the one owner of its records, or EMPTY or MIXED; HALO_RANK is set when a record belongs to the rank
 // of interest (or when all ranks are of interest).
 constexpr int HALO_EMPTY = 0x7fff, HALO_MIXED = 0x7ffe, HALO_RANK = 0x8000;
+// An owner that has no bit in the masks (below 0, or from 32 * words on) is gathered as the one owner 32 * words, "nobody":
+// its atoms are foreign to every rank.  The number fits the 16 bits below the words above: at most 32000 ranks.
 struct HaloArgs {
     const long long* owner;      // [n_atoms] rank of each atom
     uint32_t* needed;            // [n_atoms, words]
     unsigned char* has_foreign;  // [n_atoms]
+    uint32_t* bad;               // set when an edge of interest ends at an atom of nobody; or nullptr
     int words;
     int rank;                    // -1: all ranks
 };
@@ -1517,8 +1520,9 @@ rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArg
         int64_t sa = -1, ta = -1;
         if (j < M) sa = (int64_t)p.smeta[j].x;
         if (j < p.n_targets) ta = (int64_t)p.tmeta[j].x;
-        if (sa >= 0) p.sown[j] = (unsigned short)halo.owner[sa];
-        if (ta >= 0) p.town[j] = (unsigned short)halo.owner[ta];
+        const unsigned long long nobody = 32ull * (unsigned)halo.words;   // unsigned: negative owners are large
+        if (sa >= 0) p.sown[j] = (unsigned short)min((unsigned long long)halo.owner[sa], nobody);
+        if (ta >= 0) p.town[j] = (unsigned short)min((unsigned long long)halo.owner[ta], nobody);
     }
 }
 
@@ -1586,7 +1590,7 @@ __device__ __forceinline__ void halo_test(const PairParams<T>& p, const HaloArgs
     }
     if (!live) hits = 0;
     uint32_t need = 0;
-    if (b.owner >= 0 && !WIDE) {
+    if (!WIDE && (uint32_t)b.owner < 32u) {
         if (hits) need = 1u << b.owner;
     } else if (hits) {
         const int o = w.cand_owner[first + lane];
@@ -1594,6 +1598,8 @@ __device__ __forceinline__ void halo_test(const PairParams<T>& p, const HaloArgs
             const int q = __ffs((int)left) - 1, ot = real_to_bits(w.tgt[q].w);
             if (o == ot || !(halo.rank < 0 || o == halo.rank || ot == halo.rank)) {
                 hits &= ~(1u << q);
+            } else if (ot >= 32 * halo.words) {
+                if (halo.bad != nullptr) *halo.bad = 1u;
             } else if (!WIDE) {
                 need |= 1u << ot;
             } else {
@@ -1626,7 +1632,7 @@ __device__ __forceinline__ void halo_batch(const PairParams<T>& p, const HaloArg
         const float dx = fmaxf(fmaxf(b.lo[0] - x, x - b.hi[0]), 0.0f), dy = fmaxf(fmaxf(b.lo[1] - y, y - b.hi[1]), 0.0f),
                     dz = fmaxf(fmaxf(b.lo[2] - z, z - b.hi[2]), 0.0f);
         keep = keep && dx * dx + dy * dy + dz * dz <= b.reach2;
-        if (!WIDE && keep && b.owner >= 0 && b.open == 0u) keep = !((halo.needed[real_to_bits(c.w)] >> b.owner) & 1u);
+        if (!WIDE && keep && (uint32_t)b.owner < 32u && b.open == 0u) keep = !((halo.needed[real_to_bits(c.w)] >> b.owner) & 1u);
         const uint32_t m = __ballot_sync(0xffffffffu, keep);
         if (keep) {
             const int at = near + __popc(m & lt);
@@ -2211,7 +2217,7 @@ extern "C" int dynb_rg_fill_glue(const void* workspace_dev, int dtype, int64_t* 
 }
 
 extern "C" int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
-                                      int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream)
+                                      int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev, uint32_t* bad_dev, void* stream)
 {
     if (workspace_dev == nullptr || owner_dev == nullptr || needed_dev == nullptr || has_foreign_dev == nullptr)
         return fail_arg("null pointer");
@@ -2221,10 +2227,12 @@ extern "C" int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, cons
     ha.owner = reinterpret_cast<const long long*>(owner_dev);
     ha.needed = needed_dev;
     ha.has_foreign = has_foreign_dev;
+    ha.bad = bad_dev;
     ha.words = (int)((world_size + 31) / 32);
     ha.rank = (int)rank;
     DYNB_CUDA_OK(cudaMemsetAsync(needed_dev, 0, (size_t)n_atoms * ha.words * 4, s));
     DYNB_CUDA_OK(cudaMemsetAsync(has_foreign_dev, 0, (size_t)n_atoms, s));
+    if (bad_dev != nullptr) DYNB_CUDA_OK(cudaMemsetAsync(bad_dev, 0, 4, s));
     if (dtype == DYNB_F32) return rg_halo_mark<float>(workspace_dev, ha, n_atoms, s);
     if (dtype == DYNB_F64) return rg_halo_mark<double>(workspace_dev, ha, n_atoms, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");
@@ -2233,5 +2241,5 @@ extern "C" int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, cons
 extern "C" int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
                                  int64_t world_size, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream)
 {
-    return dynb_rg_halo_mark_rank(workspace_dev, dtype, owner_dev, n_atoms, world_size, -1, needed_dev, has_foreign_dev, stream);
+    return dynb_rg_halo_mark_rank(workspace_dev, dtype, owner_dev, n_atoms, world_size, -1, needed_dev, has_foreign_dev, nullptr, stream);
 }

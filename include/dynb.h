@@ -121,9 +121,12 @@ int dynb_rg_halo_mark(const void* workspace_dev, int dtype, const int64_t* owner
                       int64_t world_size, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream);
 
 /* The same for the edges that start or end at an atom of `rank`, which are all that the halo lists of that rank need;
- * rank = -1: every edge, as dynb_rg_halo_mark. */
+ * rank = -1: every edge, as dynb_rg_halo_mark.  An owner that has no bit in needed_dev (below 0, or from 32 * words on)
+ * is foreign to every rank; bad_dev (optional, may be NULL) is set to 1 when such an atom is the destination of one of
+ * these edges, else to 0. */
 int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,
-                           int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev, void* stream);
+                           int64_t world_size, int64_t rank, uint32_t* needed_dev, uint8_t* has_foreign_dev,
+                           uint32_t* bad_dev, void* stream);
 
 /* ------------------------------------------------------------------ SFC partition
  * Replaces sfc_partition_cuda (dynamis_state/src/csrc/partition/sfc.cpp:9-33,
@@ -184,7 +187,8 @@ int dynb_halo_mark_from_edges(const int64_t* edges_dev, int64_t E, const int64_t
  * carries two sets of peer ranks; segment p of the send (recv) list holds, ascending in a, the atoms whose send (recv)
  * set contains p.  owner_dev == NULL: the sets are the bits of the two masks ([n, ceil(W/32)] uint32).  owner_dev given:
  * send_mask_dev is the "needed by" mask of dynb_rg_halo_mark (recv_mask_dev is not read), an own atom (owner == R) is sent
- * to the ranks that need it, a foreign one is received from its owner when R needs it.
+ * to the ranks that need it, a foreign one is received from its owner when R needs it.  Mask bits and owners beyond W are
+ * in no list.
  * dynb_halo_lists_plan writes offsets_dev: send [W+1], recv [W+1], number of own atoms.  After reading them the caller
  * allocates the outputs and calls dynb_halo_lists_fill with the same arguments and workspace: send_local_dev (local index
  * of an own atom, or value_map_dev[a] without owners), recv_atom_dev (a), recv_ghost_dev (n_local + place in the list),

@@ -400,3 +400,42 @@ def test_halo_mark_of_a_plan_through_the_c_entry(cuda, dtype, W):
     np.testing.assert_array_equal(foreign.cpu().numpy(), ref_foreign)
     ours_e = np.sort(ei[0].cpu().numpy() * n + ei[1].cpu().numpy())
     np.testing.assert_array_equal(ours_e, np.sort(g["src"].astype(np.int64) * n + g["dst"]))
+
+
+@pytest.mark.parametrize("W,label,accepted", [(3, 5, True), (3, 31, True), (3, 32, False), (3, -1, False), (3, 65537, False),
+                                              (3, 2 ** 37, False), (32, 32, False), (40, 50, True), (40, 64, False), (40, -2, False)])
+def test_labels_that_are_no_ranks(cuda, W, label, accepted):
+    """A label in the unused bits of the last mask word: its atoms are in no list, and foreign to their neighbours.  A label
+    without a bit in the masks: an error, from the partitioner's maps and from extract_halo_info.  The lists with the label
+    as a rank of its own, cut to the first W ranks, are the reference."""
+    pos, cell = _halo_case(23, 1800, 24.0)
+    n = pos.shape[0]
+    owner = np.random.default_rng(W).integers(0, W, n)
+    stray = np.arange(0, n, 11)
+    owner[stray] = label
+    g = O.radius_graph(pos, cell, [1, 1, 1], np.float32(5.5))
+    tp, tc, tb = torch.as_tensor(pos, device=cuda), torch.as_tensor(cell), torch.tensor([True] * 3)
+    pid = torch.as_tensor(owner, device=cuda)
+    for r in (0, W - 1):
+        info = D.PartitionMessagePassingInfo()
+        info.partition_id = pid
+        args = (info, _state(pos, cuda), _env(r, W), _cfg(cell, 5.0, 0.5))
+        mine = torch.nonzero(pid == r).squeeze(-1)
+        edges = D.radius_graph_pbc_ex(tp, tc, tb, float(np.float32(5.5)), 0, False, mine)[0]
+        if not accepted:
+            with pytest.raises(RuntimeError, match="label"):
+                D.SFCPartitioner().build_halo_maps(*args)
+            with pytest.raises(RuntimeError, match="out of range"):
+                D.extract_halo_info(edges, pid, mine, r, W, n)
+            continue
+        D.SFCPartitioner().build_halo_maps(*args)
+        ref = O.build_halo_maps(g["src"], g["dst"], owner, r, label + 1)
+        so, ro = ref["send_offsets"][:W + 1], ref["recv_offsets"][:W + 1]
+        assert ref["send_offsets"][-1] > so[-1]          # the label's atoms are neighbours of this rank's
+        expect = (so, ref["send_local_indices"][:so[-1]], ro, ref["recv_ghost_indices"][:ro[-1]], ref["interior_mask"],
+                  ref["recv_atom_global"][:ro[-1]])
+        ours = (info.send_offsets, info.send_local_indices, info.recv_offsets, info.recv_ghost_indices, info.interior_mask,
+                info.recv_atom_global)
+        for a, b, c in zip(ours, D.extract_halo_info(edges, pid, mine, r, W, n), expect):
+            np.testing.assert_array_equal(a.cpu().numpy(), c)
+            np.testing.assert_array_equal(b.cpu().numpy(), c)
