@@ -208,21 +208,25 @@ class AbstractPartitioner:
             recv_ghost = torch.empty((total_recv,), dtype=torch.int64, device=dev)
             interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
             matrix = info.global_send_recv_matrix
-            if matrix is None or matrix.device != dev or matrix.dtype != torch.int64 or not matrix.is_contiguous() or N == 0:
-                kept, matrix = matrix, torch.zeros((W, W), dtype=torch.int64, device=dev)
-                if kept is not None:
-                    matrix.copy_(kept)
-                info.global_send_recv_matrix = matrix
+            if matrix is None:
+                matrix = info.global_send_recv_matrix = torch.zeros((W, W), dtype=torch.int64, device=dev)
+            # row R is written by the list pass where the matrix is what the partitioner made; any other kind of tensor
+            # (another device, type, shape or stride) and the empty system go through an assignment, which checks them
+            in_place = (N > 0 and matrix.device == dev and matrix.dtype == torch.int64 and matrix.is_contiguous()
+                        and tuple(matrix.shape) == (W, W))
             _lib.check(L.dynb_halo_lists_fill(needed.data_ptr(), None, pid.data_ptr(), N, R, W, None, has_foreign.data_ptr(),
                                               offs.data_ptr(), n_local, send_local.data_ptr(), recv_atom.data_ptr(),
-                                              recv_ghost.data_ptr(), interior.data_ptr(), matrix[R].data_ptr(), ws.data_ptr(),
-                                              _stream(dev)), "halo_lists_fill")
+                                              recv_ghost.data_ptr(), interior.data_ptr(), matrix[R].data_ptr() if in_place else None,
+                                              ws.data_ptr(), _stream(dev)), "halo_lists_fill")
             info.send_offsets = offs[:W + 1]
             info.send_local_indices = send_local
             info.recv_offsets = offs[W + 1:2 * W + 2]
             info.recv_ghost_indices = recv_ghost
             info.recv_atom_global = recv_atom
             info.interior_mask = interior
+            if not in_place:  # build_halo_maps.cpp:150-154
+                matrix[R] = info.send_offsets[1:] - info.send_offsets[:-1]
+                matrix[R, R] = n_local
         info.edge_index_halo = None
         info._edge_index_halo_fn = lambda: radius_graph_pbc(pos32, cell, pbc, ghost_cutoff, HALO_MAX_NUM_NEIGHBORS, False)[0]
 

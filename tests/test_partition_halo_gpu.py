@@ -439,3 +439,33 @@ def test_labels_that_are_no_ranks(cuda, W, label, accepted):
         for a, b, c in zip(ours, D.extract_halo_info(edges, pid, mine, r, W, n), expect):
             np.testing.assert_array_equal(a.cpu().numpy(), c)
             np.testing.assert_array_equal(b.cpu().numpy(), c)
+
+
+def test_halo_maps_write_into_the_matrix_they_are_given(cuda):
+    """The row goes into the caller's matrix, whatever its device and strides; one of another world size is refused by the
+    assignment, and an empty system clears its row."""
+    pos, cell = _halo_case(29, 1100, 20.0)
+    W, R = 3, 1
+    owner = np.random.default_rng(1).integers(0, W, pos.shape[0])
+    g = O.radius_graph(pos, cell, [1, 1, 1], np.float32(5.5))
+    row = O.build_halo_maps(g["src"], g["dst"], owner, R, W)["matrix_row"]
+
+    def run(matrix, n=pos.shape[0]):
+        info = D.PartitionMessagePassingInfo()
+        info.partition_id = torch.as_tensor(owner[:n], device=cuda)
+        info.global_send_recv_matrix = matrix
+        D.SFCPartitioner().build_halo_maps(info, _state(pos[:n], cuda), _env(R, W), _cfg(cell, 5.0, 0.5))
+        return info.global_send_recv_matrix
+
+    fresh = torch.full((W, W), 7, dtype=torch.int64)
+    for matrix in (fresh.to(cuda), fresh.clone(), fresh.to(cuda).t(), fresh.to(cuda, torch.int32), fresh.to(cuda, torch.float64)):
+        out = run(matrix)
+        assert out is matrix
+        expect = np.full((W, W), 7)
+        expect[R] = row
+        np.testing.assert_array_equal(out.cpu().numpy(), expect)
+    assert run(None).device == cuda
+    with pytest.raises((RuntimeError, IndexError)):
+        run(torch.zeros((2, 2), dtype=torch.int64, device=cuda))
+    empty = run(fresh.to(cuda), 0)
+    assert empty[R].tolist() == [0] * W and empty[0].tolist() == [7] * W
