@@ -7,6 +7,7 @@
 //   dynb_halo_lists_plan / _fill             send and recv CSR of build_halo_maps
 //       (dynamis_state/src/csrc/build_halo_maps.cpp:60-125) and of extract_halo_info, from
 //       per-atom rank bit masks instead of the reference's [N, W] bool matrix + nonzero + argsort
+//   dynb_csr_plan / dynb_csr_fill            one such list per call, from one mask
 //   dynb_filter_edges_plan / _fill           filter_edges_to_radius
 //       (dist_graph_ops_kernels.cu:16-43, 62-102)
 //
@@ -360,6 +361,100 @@ halo_lists_fill_kernel(const HaloSets h, int W, int nblocks, const uint32_t* __r
     }
 }
 
+// ------------------------------------------------------------------------------------------ CSR assembly
+// Element a in [0, n) carries a set of peer ranks.  For each peer p, the output segment p lists the
+// elements whose set contains p, ascending in a.  One list per call, every peer walked: the form for C callers that have
+// one mask at a time; the partitioner's and extract_halo_info's two lists come from the halo list passes above.  Modes
+// define the set:
+enum { CSR_SEND = 0, CSR_RECV = 1, CSR_RAW = 2 };
+//   CSR_SEND  owner[a] == R ? bits of mask[a] without R : {}        (needed_by rows of my atoms)
+//   CSR_RECV  owner[a] != R and bit R of mask[a] ? {owner[a]} : {}   (foreign atoms I need)
+//   CSR_RAW   bits of mask[a]
+constexpr int CSR_THREADS = 256;
+constexpr int CSR_WARPS = CSR_THREADS / 32;
+
+__device__ __forceinline__ bool csr_has(const uint32_t* __restrict__ mask, int words, const int64_t* __restrict__ owner,
+                                        int64_t a, int64_t R, int mode, int p)
+{
+    if (mode == CSR_RAW) return (mask[a * words + (p >> 5)] >> (p & 31)) & 1u;
+    const int64_t o = owner[a];
+    if (mode == CSR_SEND) return o == R && p != R && ((mask[a * words + (p >> 5)] >> (p & 31)) & 1u);
+    return o != R && o == p && ((mask[a * words + (R >> 5)] >> (R & 31)) & 1u);
+}
+
+// bsum[p * nblocks + block] = number of elements of this block whose set contains p
+__global__ void __launch_bounds__(CSR_THREADS)
+csr_count_kernel(const uint32_t* __restrict__ mask, int words, const int64_t* __restrict__ owner, int64_t n, int64_t R,
+                 int mode, int W, int nblocks, uint32_t* __restrict__ bsum)
+{
+    __shared__ uint32_t wsum[CSR_WARPS];
+    const int64_t a = (int64_t)blockIdx.x * CSR_THREADS + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int p = 0; p < W; p++) {
+        const bool f = (a < n) && csr_has(mask, words, owner, a, R, mode, p);
+        const uint32_t b = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) wsum[warp] = __popc(b);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t s = 0;
+            for (int w = 0; w < CSR_WARPS; w++) s += wsum[w];
+            bsum[(int64_t)p * nblocks + blockIdx.x] = s;
+        }
+        __syncthreads();
+    }
+}
+
+// One block per peer: exclusive scan of its row of block sums (in place) and the row total.
+__global__ void __launch_bounds__(SCAN_THREADS)
+csr_scan_rows_kernel(uint32_t* __restrict__ bsum, int nblocks, int64_t* __restrict__ totals)
+{
+    __shared__ uint32_t warp_sums[SCAN_THREADS / 32];
+    uint32_t* row = bsum + (int64_t)blockIdx.x * nblocks;
+    uint32_t carry = 0;
+    for (int b0 = 0; b0 < nblocks; b0 += SCAN_THREADS) {
+        const int i = b0 + threadIdx.x;
+        const uint32_t v = (i < nblocks) ? row[i] : 0u;
+        uint32_t tot;
+        const uint32_t ex = block_excl_scan<uint32_t>(v, &tot, warp_sums);
+        if (i < nblocks) row[i] = carry + ex;
+        carry += tot;
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = (int64_t)carry;
+}
+
+__global__ void csr_offsets_kernel(const int64_t* __restrict__ totals, int W, int64_t* __restrict__ offsets)
+{
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        int64_t run = 0;
+        for (int p = 0; p < W; p++) { offsets[p] = run; run += totals[p]; }
+        offsets[W] = run;
+    }
+}
+
+__global__ void __launch_bounds__(CSR_THREADS)
+csr_fill_kernel(const uint32_t* __restrict__ mask, int words, const int64_t* __restrict__ owner, int64_t n, int64_t R,
+                int mode, int W, int nblocks, const uint32_t* __restrict__ bsum, const int64_t* __restrict__ offsets,
+                const int64_t* __restrict__ value_map, int64_t* __restrict__ out)
+{
+    __shared__ uint32_t wsum[CSR_WARPS];
+    const int64_t a = (int64_t)blockIdx.x * CSR_THREADS + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lt = lanemask_lt();
+    for (int p = 0; p < W; p++) {
+        const bool f = (a < n) && csr_has(mask, words, owner, a, R, mode, p);
+        const uint32_t b = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) wsum[warp] = __popc(b);
+        __syncthreads();
+        if (f) {
+            uint32_t before = 0;
+            for (int w = 0; w < warp; w++) before += wsum[w];
+            const int64_t pos = offsets[p] + bsum[(int64_t)p * nblocks + blockIdx.x] + before + __popc(b & lt);
+            out[pos] = value_map ? value_map[a] : a;
+        }
+        __syncthreads();
+    }
+}
+
 __global__ void __launch_bounds__(256)
 gather_not_u8_kernel(const uint8_t* __restrict__ flags, const int64_t* __restrict__ idx, int64_t n, uint8_t* __restrict__ out)
 {
@@ -609,6 +704,57 @@ extern "C" int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_
     const int nb = hl_blocks(n);
     halo_lists_fill_kernel<<<nb, HL_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(h, (int)W, nb, static_cast<const uint32_t*>(workspace_dev),
                                                                                    offsets_dev, out);
+    DYNB_CUDA_OK(cudaGetLastError());
+    return DYNB_OK;
+}
+
+static inline int csr_blocks(int64_t n) { return (int)((n + CSR_THREADS - 1) / CSR_THREADS); }
+
+extern "C" int dynb_csr_workspace_bytes(int64_t n, int64_t W, int64_t* bytes)
+{
+    if (n < 0 || W < 1 || bytes == nullptr) return fail_arg("bad arguments");
+    *bytes = align_up((int64_t)std::max(csr_blocks(n), 1) * W * 4, 256) + align_up(W * 8, 256);
+    return DYNB_OK;
+}
+
+extern "C" int dynb_csr_plan(const uint32_t* mask_dev, const int64_t* owner_dev, int64_t n, int64_t R, int mode, int64_t W,
+                             int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream)
+{
+    if (n < 0 || W < 1 || mode < 0 || mode > 2 || offsets_dev == nullptr) return fail_arg("bad arguments");
+    if (mode != CSR_RAW && owner_dev == nullptr) return fail_arg("owner required");
+    if (W > 4096) return fail_arg("world_size above 4096 is not supported");
+    int64_t need;
+    dynb_csr_workspace_bytes(n, W, &need);
+    if (workspace_dev == nullptr || workspace_bytes < need) return fail_arg("workspace too small (see dynb_csr_workspace_bytes)");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int words = (int)((W + 31) / 32);
+    const int nb = std::max(csr_blocks(n), 1);
+    unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
+    uint32_t* bsum = reinterpret_cast<uint32_t*>(ws);
+    int64_t* totals = reinterpret_cast<int64_t*>(ws + align_up((int64_t)nb * W * 4, 256));
+    if (n == 0) {
+        DYNB_CUDA_OK(cudaMemsetAsync(offsets_dev, 0, (size_t)(W + 1) * 8, s));
+        return DYNB_OK;
+    }
+    csr_count_kernel<<<nb, CSR_THREADS, 0, s>>>(mask_dev, words, owner_dev, n, R, mode, (int)W, nb, bsum);
+    csr_scan_rows_kernel<<<(unsigned)W, SCAN_THREADS, 0, s>>>(bsum, nb, totals);
+    csr_offsets_kernel<<<1, 32, 0, s>>>(totals, (int)W, offsets_dev);
+    DYNB_CUDA_OK(cudaGetLastError());
+    return DYNB_OK;
+}
+
+extern "C" int dynb_csr_fill(const uint32_t* mask_dev, const int64_t* owner_dev, int64_t n, int64_t R, int mode, int64_t W,
+                             const int64_t* value_map_dev, const int64_t* offsets_dev, int64_t* out_dev,
+                             const void* workspace_dev, void* stream)
+{
+    if (n < 0 || W < 1 || mode < 0 || mode > 2) return fail_arg("bad arguments");
+    if (n == 0) return DYNB_OK;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int words = (int)((W + 31) / 32);
+    const int nb = csr_blocks(n);
+    const uint32_t* bsum = reinterpret_cast<const uint32_t*>(workspace_dev);
+    csr_fill_kernel<<<nb, CSR_THREADS, 0, s>>>(mask_dev, words, owner_dev, n, R, mode, (int)W, nb, bsum, offsets_dev,
+                                               value_map_dev, out_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }

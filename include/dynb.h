@@ -201,6 +201,19 @@ int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_t* recv_mas
                          int64_t R, int64_t W, const int64_t* value_map_dev, const uint8_t* has_foreign_dev,
                          const int64_t* offsets_dev, int64_t n_local, int64_t* send_local_dev, int64_t* recv_atom_dev,
                          int64_t* recv_ghost_dev, uint8_t* interior_dev, int64_t* matrix_row_dev, const void* workspace_dev, void* stream);
+/* CSR assembly (build_halo_maps.cpp:60-125; dist_graph_ops_kernels.cu:143-177).  Element a in
+ * [0, n) carries a set of peer ranks; segment p of the output lists, ascending in a, the elements
+ * whose set contains p.  mode 0 (send): owner[a] == R ? mask bits without R : {};
+ * mode 1 (recv): owner[a] != R and bit R of mask[a] ? {owner[a]} : {};  mode 2: the mask bits.
+ * dynb_csr_plan writes offsets_dev [W+1]; after reading offsets[W] the caller allocates out_dev and
+ * calls dynb_csr_fill with the same arguments and workspace (value_map_dev[a] is written instead
+ * of a when given).  dynb_halo_lists_plan / _fill make the send and the recv list of a rank in one pass. */
+int dynb_csr_workspace_bytes(int64_t n, int64_t W, int64_t* bytes);
+int dynb_csr_plan(const uint32_t* mask_dev, const int64_t* owner_dev, int64_t n, int64_t R, int mode, int64_t W,
+                  int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream);
+int dynb_csr_fill(const uint32_t* mask_dev, const int64_t* owner_dev, int64_t n, int64_t R, int mode, int64_t W,
+                  const int64_t* value_map_dev, const int64_t* offsets_dev, int64_t* out_dev,
+                  const void* workspace_dev, void* stream);
 /* interior_mask[i] = !flags[idx[i]] (build_halo_maps.cpp:138). */
 int dynb_gather_not_u8(const uint8_t* flags_dev, const int64_t* idx_dev, int64_t n, uint8_t* out_dev, void* stream);
 /* g2l[idx[i]] = i (dist_graph_ops_kernels.cu:143-144). */

@@ -6,6 +6,8 @@ with the ranks simulated serially on one GPU) and test_dist_graph_builder.py (ex
 bit-exact against build_halo_maps on N = 4000, L = 40, r = 6.5, x-slab partition).
 """
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -469,3 +471,34 @@ def test_halo_maps_write_into_the_matrix_they_are_given(cuda):
         run(torch.zeros((2, 2), dtype=torch.int64, device=cuda))
     empty = run(fresh.to(cuda), 0)
     assert empty[R].tolist() == [0] * W and empty[0].tolist() == [7] * W
+
+
+@pytest.mark.parametrize("n,W", [(1, 1), (255, 3), (257, 32), (3000, 40)])
+def test_csr_c_entries(cuda, n, W):
+    """dynb_csr_plan / dynb_csr_fill: the three sets of an element, with and without a value map."""
+    from dynamis_b200 import _lib
+
+    L = _lib.lib()
+    rng = np.random.default_rng(n + W)
+    words, R = (W + 31) // 32, W // 2
+    mask = rng.integers(0, 2 ** 32, (n, words), dtype=np.uint32)
+    owner = rng.integers(0, W, n)
+    bit = lambda p: (mask[:, p >> 5] >> np.uint32(p & 31)) & 1 == 1
+    sets = {0: lambda p: (owner == R) & bit(p) & (p != R), 1: lambda p: (owner != R) & (owner == p) & bit(R), 2: bit}
+    tm, to = torch.as_tensor(mask.view(np.int32), device=cuda), torch.as_tensor(owner, device=cuda)
+    vmap = torch.arange(n, dtype=torch.int64, device=cuda) * 3
+    st = torch.cuda.current_stream(cuda).cuda_stream
+    nbytes = ctypes.c_int64()
+    _lib.check(L.dynb_csr_workspace_bytes(n, W, ctypes.byref(nbytes)), "csr_workspace_bytes")
+    ws = torch.empty(nbytes.value, dtype=torch.uint8, device=cuda)
+    offs = torch.empty(W + 1, dtype=torch.int64, device=cuda)
+    for mode, member in sets.items():
+        lists = [np.nonzero(member(p))[0] for p in range(W)]
+        _lib.check(L.dynb_csr_plan(tm.data_ptr(), to.data_ptr(), n, R, mode, W, offs.data_ptr(), ws.data_ptr(), ws.numel(), st), "csr_plan")
+        np.testing.assert_array_equal(offs.cpu().numpy(), np.concatenate([[0], np.cumsum([a.size for a in lists])]))
+        for values in (None, vmap):
+            out = torch.full((int(offs[W]) + 1,), -5, dtype=torch.int64, device=cuda)
+            _lib.check(L.dynb_csr_fill(tm.data_ptr(), to.data_ptr(), n, R, mode, W, values.data_ptr() if values is not None else None,
+                                       offs.data_ptr(), out.data_ptr(), ws.data_ptr(), st), "csr_fill")
+            ref = np.concatenate(lists) * (3 if values is not None else 1)
+            np.testing.assert_array_equal(out.cpu().numpy(), np.concatenate([ref, [-5]]))
