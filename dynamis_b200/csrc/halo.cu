@@ -599,7 +599,8 @@ extern "C" int dynb_bincount_i64(const int64_t* a_dev, int64_t n, int64_t W, int
 extern "C" int dynb_select_workspace_bytes(int64_t n, int64_t* bytes)
 {
     if (n < 0 || bytes == nullptr) return fail_arg("bad arguments");
-    *bytes = align_up((n / SELECT_TILE + 1) * 4, 256);
+    // the edge filter takes a workspace of dynb_select_workspace_bytes(2 * E) too
+    *bytes = std::max(align_up((n / SELECT_TILE + 1) * 4, 256), filter_layout(n / 2).total);
     return DYNB_OK;
 }
 

@@ -224,7 +224,8 @@ int dynb_scatter_iota(const int64_t* idx_dev, int64_t n, int64_t N, int64_t* g2l
  * dist_graph_ops_kernels.cu:16-43, 62-102): keeps edge e iff
  * |pos[src] + shift @ cell - pos[dst]|^2 <= radius^2 (float32), order preserving.  The plan writes
  * the number kept to count_dev; the fill compacts edges [2,E] -> [2,E_out] and the shift rows of
- * any element size (shift_row_bytes = 3 * element size). */
+ * any element size (shift_row_bytes = 3 * element size).  Workspace: dynb_filter_edges_workspace_bytes(E), or
+ * dynb_select_workspace_bytes(2 * E), which is no smaller. */
 int dynb_filter_edges_workspace_bytes(int64_t E, int64_t* bytes);
 int dynb_filter_edges_plan(const int64_t* edges_dev, const float* shifts_f32_dev, const float* pos_dev,
                            const float* cell_host, double radius, int64_t E, int64_t* count_dev,

@@ -160,3 +160,15 @@ def test_exchange_plan_over_gloo_world_size_2(tmp_path):
            "--master-port", "29611", str(script), ROOT]
     r = subprocess.run(cmd, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
+
+
+@pytest.mark.parametrize("E", [0, 1, 31, 1023, 1024, 1025, 1_000_003, 3_000_000_001])
+def test_a_select_workspace_holds_the_edge_filters(E):
+    """dynb.h lets a C caller size the filter's workspace by either function."""
+    from dynamis_b200 import _lib
+
+    L = _lib.lib()
+    a, b = ctypes.c_int64(), ctypes.c_int64()
+    assert L.dynb_filter_edges_workspace_bytes(E, ctypes.byref(a)) == 0
+    assert L.dynb_select_workspace_bytes(2 * E, ctypes.byref(b)) == 0
+    assert b.value >= a.value > 0
