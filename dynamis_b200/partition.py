@@ -126,12 +126,12 @@ def bincount_labels(labels: torch.Tensor, W: int) -> torch.Tensor:
 def select_eq(values: torch.Tensor, value: int, gather_src: Optional[torch.Tensor] = None,
               count: Optional[int] = None) -> torch.Tensor:
     """``gather_src[nonzero(values == value)]`` (or the positions themselves), ascending.  One host sync, none when the
-    caller knows how many there are (``count``)."""
+    caller knows how many there are (``count``; the buffer has room for every position all the same)."""
     dev = values.device
     n = values.numel()
     L = _lib.lib()
     with _lib.on_device(dev):
-        out = torch.empty((n if count is None else count,), dtype=torch.int64, device=dev)
+        out = torch.empty((n,), dtype=torch.int64, device=dev)
         cnt = torch.empty((1,), dtype=torch.int64, device=dev)
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_select_workspace_bytes(n, ctypes.byref(nbytes)), "select_workspace_bytes")
@@ -247,8 +247,9 @@ class SFCPartitioner(AbstractPartitioner):
         if config is None:
             labels = sfc_partition_labels(pos32, state.edge_counts, W, int(self.curve_type))
             # equal counts: the first N % W ranks hold one atom more (sfc_kernels.cu:123-134)
-            N = pos32.size(0)
-            n_local = N // W + (1 if int(env.global_rank) < N % W else 0) if state.edge_counts is None else None
+            N, R, n_local = pos32.size(0), int(env.global_rank), None
+            if state.edge_counts is None and 0 <= R < W:
+                n_local = N // W + (1 if R < N % W else 0)
             return _finish_partition(labels, state, env, n_local)
         # mode 3: weights = in-degree at the cutoff; the graph is kept for downstream use
         cutoff = float(np.float32(config.cutoff))

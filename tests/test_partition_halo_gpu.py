@@ -502,3 +502,17 @@ def test_csr_c_entries(cuda, n, W):
                                        offs.data_ptr(), out.data_ptr(), ws.data_ptr(), st), "csr_fill")
             ref = np.concatenate(lists) * (3 if values is not None else 1)
             np.testing.assert_array_equal(out.cpu().numpy(), np.concatenate([ref, [-5]]))
+
+
+@pytest.mark.parametrize("n,W", [(1, 1), (3, 8), (8, 8), (16, 8), (17, 8), (23, 8), (4099, 7)])
+def test_partition_indices_with_the_count_known_beforehand(cuda, n, W):
+    """Equal counts: the partitioner knows how many atoms a rank gets and does not wait for the number; a rank outside the
+    world has none."""
+    from dynamis_b200.partition import select_eq
+
+    pos = (np.random.default_rng(n).random((n, 3)) * 20.0).astype(np.float32)
+    for r in range(W):
+        info = D.SFCPartitioner().partition(_state(pos, cuda), _env(r, W))
+        assert torch.equal(info.partition_indices, select_eq(info.partition_id, r))
+        assert torch.equal(select_eq(info.partition_id, r, None, info.partition_indices.numel()), info.partition_indices)
+    assert D.SFCPartitioner().partition(_state(pos, cuda), _env(-1, W)).partition_indices.numel() == 0
