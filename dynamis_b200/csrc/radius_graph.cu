@@ -2182,9 +2182,12 @@ static int rg_fill_any(const void* workspace_dev, int dtype, int64_t* edge_index
 {
     if (workspace_dev == nullptr) return fail_arg("null workspace");
     if (E < 0) return fail_arg("E must be non-negative");
-    if (E == 0) return DYNB_OK;
-    if (edge_index_dev == nullptr || shifts_dev == nullptr) return fail_arg("null output pointer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (E == 0) {
+        if (total_dev != nullptr) DYNB_CUDA_OK(cudaMemsetAsync(total_dev, 0, sizeof(int64_t), s));
+        return DYNB_OK;
+    }
+    if (edge_index_dev == nullptr || shifts_dev == nullptr) return fail_arg("null output pointer");
     if (dtype == DYNB_F32) return rg_fill<float>(workspace_dev, edge_index_dev, shifts_dev, dist_sq_dev, E, glue, total_dev, long_lists, s);
     if (dtype == DYNB_F64) return rg_fill<double>(workspace_dev, edge_index_dev, shifts_dev, dist_sq_dev, E, glue, total_dev, long_lists, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");

@@ -103,8 +103,6 @@ class RadiusGraphPlan:
         return edge_index, shifts, d2
 
     def fill_into(self, edge_index, shifts, d2=None, total=None):
-        if self.E == 0:
-            return
         _lib.check(_lib.lib().dynb_rg_fill_counted(self.ws.data_ptr(), self.dtype_code, edge_index.data_ptr(), shifts.data_ptr(),
                                                    d2.data_ptr() if d2 is not None else None, self.E, self.long_lists,
                                                    total.data_ptr() if total is not None else None, _lib.stream_of(self.device)),

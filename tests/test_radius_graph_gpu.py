@@ -413,6 +413,20 @@ def test_image_capacity_overflow_is_reported_and_the_plan_repeated(cuda, periodi
         geo.clear()
 
 
+@pytest.mark.parametrize("E", [0, 1, 2])
+def test_fill_reports_the_number_of_edges(cuda, E):
+    """``fill(total=...)`` receives the number of edges, none included."""
+    from dynamis_b200.graph import plan_radius_graph
+
+    pos = torch.zeros((3, 3), device=cuda)
+    pos[1, 0], pos[2, 0] = (2.0 if E else 20.0), 40.0
+    targets = torch.tensor([0], device=cuda) if E == 1 else None
+    plan = plan_radius_graph(pos, torch.eye(3) * 60.0, torch.tensor([False] * 3), 3.0, targets)
+    total = torch.full((1,), 99, dtype=torch.int64, device=cuda)
+    ei, cs, _ = plan.fill(False, total)
+    assert plan.E == E == int(total) and ei.shape == (2, E) and cs.shape == (E, 3)
+
+
 # ------------------------------------------------------------------ against the reference's own kernels
 
 def _run_ref(ref_ops, pos, cell, pbc, r, dev, targets=None):
