@@ -1787,6 +1787,14 @@ struct RgLayout {
         tcount, toffset, runs, sums, total;
 };
 
+// The layout starts at the first 256-byte boundary of the caller's workspace: its records are read and written in pieces
+// of up to 32 bytes, wherever the workspace lies.
+constexpr int64_t RG_WS_ALIGN = 256;
+static unsigned char* rg_base(const void* ws)
+{
+    return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ws) + RG_WS_ALIGN - 1) / RG_WS_ALIGN * RG_WS_ALIGN);
+}
+
 static RgLayout rg_layout(int64_t N, int64_t Nt, int64_t src_cap, int64_t cell_cap, int dtype)
 {
     const int64_t v4 = dtype == DYNB_F64 ? 32 : 16;
@@ -1916,8 +1924,8 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     if (rc) return rc;
     const int dtype = sizeof(T) == 8 ? DYNB_F64 : DYNB_F32;
     const RgLayout L = rg_layout(N, Nt, src_cap, cell_cap, dtype);
-    if (ws_bytes < L.total) return fail_arg("workspace too small (see dynb_rg_workspace_bytes)");
-    unsigned char* w = static_cast<unsigned char*>(ws);
+    unsigned char* w = rg_base(ws);
+    if (ws_bytes < L.total + (w - static_cast<unsigned char*>(ws))) return fail_arg("workspace too small (see dynb_rg_workspace_bytes)");
     DevHeader* h = reinterpret_cast<DevHeader*>(w + L.hdr);
 
     auto* posw = reinterpret_cast<Vec4<T>*>(w + L.posw);
@@ -2065,7 +2073,7 @@ template <typename T>
 static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int64_t E, const GlueArgs* glue_opt, int64_t* total_dev,
                    bool long_lists, cudaStream_t stream)
 {
-    const unsigned char* w = static_cast<const unsigned char*>(ws);
+    const unsigned char* w = rg_base(ws);
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
     // a warp for every 32 edges is more than there are groups with targets
     const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * 4 * PAIR_GRID_WAVES, (E + 32 * PAIR_WARPS - 1) / (32 * PAIR_WARPS));
@@ -2098,7 +2106,7 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
 template <typename T>
 static int rg_halo_mark(const void* ws, const HaloArgs& ha, int64_t N, cudaStream_t stream)
 {
-    const unsigned char* w = static_cast<const unsigned char*>(ws);
+    const unsigned char* w = rg_base(ws);
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
     // the numbers of records and runs are known on the device only: both passes stride
     rg_halo_owner_kernel<T><<<(unsigned)std::max<int64_t>((N + 255) / 256, (int64_t)sm_count_cached() * 4), 256, 0, stream>>>(params_dev, ha);
@@ -2134,7 +2142,7 @@ extern "C" int dynb_rg_workspace_bytes(int64_t n_atoms, int64_t n_targets, int64
     if (dtype != DYNB_F32 && dtype != DYNB_F64) return fail_arg("dtype must be DYNB_F32 or DYNB_F64");
     if (n_atoms >= (1ll << 31) || src_capacity >= (1ll << 31) || n_targets >= (1ll << 31) || cell_capacity >= (1ll << 31) - 8)
         return fail_arg("sizes must stay below 2^31");
-    *bytes = rg_layout(n_atoms, n_targets, src_capacity, cell_capacity, dtype).total;
+    *bytes = rg_layout(n_atoms, n_targets, src_capacity, cell_capacity, dtype).total + RG_WS_ALIGN;
     return DYNB_OK;
 }
 

@@ -72,6 +72,7 @@ typedef struct dynb_rg_header {
 int dynb_rg_suggest_capacity(int64_t n_atoms, const void* cell_host, const uint8_t* pbc_host, double radius,
                              int dtype, int64_t* src_capacity, int64_t* cell_capacity);
 
+/* The workspace may start at any address (the plan uses it from its first 256-byte boundary on). */
 int dynb_rg_workspace_bytes(int64_t n_atoms, int64_t n_targets, int64_t src_capacity, int64_t cell_capacity,
                             int dtype, int64_t* bytes);
 

@@ -7,6 +7,8 @@ add target subsets, positions outside the cell, float64 and a cutoff-tie stress 
 Edge sets are compared bit-exactly after canonical sorting.
 """
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -425,6 +427,39 @@ def test_fill_reports_the_number_of_edges(cuda, E):
     total = torch.full((1,), 99, dtype=torch.int64, device=cuda)
     ei, cs, _ = plan.fill(False, total)
     assert plan.E == E == int(total) and ei.shape == (2, E) and cs.shape == (E, 3)
+
+
+@pytest.mark.parametrize("offset", [0, 16, 40])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_workspace_at_any_address(cuda, dtype, offset):
+    """The C entries take a workspace that starts anywhere inside an allocation: same edges, through a plan and through the
+    capacities and sizes the library itself asks for."""
+    from dynamis_b200 import _lib
+
+    L, code = _lib.lib(), _lib.DYNB_F64 if dtype == torch.float64 else _lib.DYNB_F32
+    pos, cell, pbc = _cubic(900, 22.0, 3)
+    tp = torch.as_tensor(pos, device=cuda).to(dtype)
+    cell_h = np.ascontiguousarray(cell.astype(np.float64 if code == _lib.DYNB_F64 else np.float32))
+    pbc_h = np.ones(3, np.uint8)
+    src, cells, nbytes = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int64()
+    n, r, st = pos.shape[0], 5.0, torch.cuda.current_stream(cuda).cuda_stream
+    _lib.check(L.dynb_rg_suggest_capacity(n, cell_h.ctypes.data, pbc_h.ctypes.data, r, code, ctypes.byref(src), ctypes.byref(cells)), "suggest")
+    _lib.check(L.dynb_rg_workspace_bytes(n, n, src.value, cells.value, code, ctypes.byref(nbytes)), "workspace_bytes")
+    buf = torch.zeros(nbytes.value + 512, dtype=torch.uint8, device=cuda)
+    assert buf.data_ptr() % 256 == 0
+    ws, counts = buf.data_ptr() + offset, torch.empty(n, dtype=torch.int32, device=cuda)
+    hdr_t = torch.zeros(64, dtype=torch.uint8, pin_memory=True)
+    hdr = _lib.RgHeader.from_address(hdr_t.data_ptr())
+    _lib.check(L.dynb_rg_plan(tp.data_ptr(), code, n, cell_h.ctypes.data, pbc_h.ctypes.data, r, None, n, ws, nbytes.value, src.value,
+                              cells.value, counts.data_ptr(), hdr_t.data_ptr(), st), "plan")
+    torch.cuda.synchronize(cuda)
+    assert hdr.status == 0
+    ei = torch.empty((2, hdr.E), dtype=torch.int64, device=cuda)
+    cs = torch.empty((hdr.E, 3), dtype=torch.float32, device=cuda)
+    _lib.check(L.dynb_rg_fill(ws, code, ei.data_ptr(), cs.data_ptr(), None, hdr.E, st), "fill")
+    ref = _run_ours(tp.cpu().numpy(), cell_h, pbc, r, cuda)
+    assert torch.equal(ei, ref[0]) and torch.equal(cs, ref[1]) and torch.equal(counts, ref[3])
+    assert not buf[offset + nbytes.value:].any()
 
 
 # ------------------------------------------------------------------ against the reference's own kernels
