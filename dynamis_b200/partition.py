@@ -170,6 +170,11 @@ class AbstractPartitioner:
             raise RuntimeError("pos must be a CUDA tensor")
         dev = pos.device
         N, W, R = int(global_state.num_atoms), int(env.world_size), int(env.global_rank)
+        # refused before anything is queued: the header and the list sizes are copied into buffers of this call
+        if not 0 <= R < W:
+            raise RuntimeError(f"global_rank must be in [0, world_size), got {R} of {W}")
+        if W > 4096:
+            raise RuntimeError("world_size above 4096 is not supported")
         ghost_cutoff = float(np.float32(config.cutoff + config.ghost_cutoff_buffer))
         pos32 = pos.to(torch.float32).contiguous()
         cell = config.cell.to(torch.float32)

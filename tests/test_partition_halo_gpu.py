@@ -516,3 +516,18 @@ def test_partition_indices_with_the_count_known_beforehand(cuda, n, W):
         assert torch.equal(info.partition_indices, select_eq(info.partition_id, r))
         assert torch.equal(select_eq(info.partition_id, r, None, info.partition_indices.numel()), info.partition_indices)
     assert D.SFCPartitioner().partition(_state(pos, cuda), _env(-1, W)).partition_indices.numel() == 0
+
+
+@pytest.mark.parametrize("rank,W", [(3, 3), (-1, 3), (0, 4097), (0, 0)])
+def test_halo_maps_refuse_ranks_and_worlds_before_any_work(cuda, rank, W, monkeypatch):
+    from dynamis_b200 import partition
+
+    def launched(*_):
+        raise AssertionError("work was queued before the arguments were looked at")
+
+    monkeypatch.setattr(partition, "BinnedAtoms", launched)
+    pos, cell = _halo_case(2, 200, 12.0)
+    info = D.PartitionMessagePassingInfo()
+    info.partition_id = torch.zeros(200, dtype=torch.int64, device=cuda)
+    with pytest.raises(RuntimeError):
+        D.SFCPartitioner().build_halo_maps(info, _state(pos, cuda), _env(rank, W), _cfg(cell, 4.0, 0.5))
