@@ -46,6 +46,11 @@ def scratch(device: torch.device, name: str, nbytes: int) -> torch.Tensor:
 _stream = _lib.stream_of
 
 
+def _single(x) -> float:
+    """x (a number, or a tensor of one element on any device) rounded to single precision."""
+    return float(np.float32(float(x)))
+
+
 class SFCCurveType(enum.IntEnum):
     Morton = 0
     Hilbert = 1
@@ -175,7 +180,7 @@ class AbstractPartitioner:
             raise RuntimeError(f"global_rank must be in [0, world_size), got {R} of {W}")
         if W > 4096:
             raise RuntimeError("world_size above 4096 is not supported")
-        ghost_cutoff = float(np.float32(config.cutoff + config.ghost_cutoff_buffer))
+        ghost_cutoff = _single(config.cutoff + config.ghost_cutoff_buffer)
         pos32 = pos.to(torch.float32).contiguous()
         cell = config.cell.to(torch.float32)
         pbc = config.pbc.to(torch.bool)
@@ -257,7 +262,7 @@ class SFCPartitioner(AbstractPartitioner):
                 n_local = N // W + (1 if R < N % W else 0)
             return _finish_partition(labels, state, env, n_local)
         # mode 3: weights = in-degree at the cutoff; the graph is kept for downstream use
-        cutoff = float(np.float32(config.cutoff))
+        cutoff = _single(config.cutoff)
         cell = config.cell.to(torch.float32)
         ei, _, _, counts = radius_graph_pbc_ex(pos32, cell, config.pbc.to(torch.bool), cutoff, PARTITION_MAX_NUM_NEIGHBORS, False)
         labels = sfc_partition_labels(pos32, counts.to(torch.int64), W, int(self.curve_type))
@@ -313,7 +318,7 @@ class KDTreePartitioner(AbstractPartitioner):
         if config is None:
             labels = kdtree_partition_labels(pos32, state.edge_counts, W)
             return _finish_partition(labels, state, env)
-        cutoff = float(np.float32(config.cutoff))
+        cutoff = _single(config.cutoff)
         cell = config.cell.to(torch.float32)
         ei, _, _, counts = radius_graph_pbc_ex(pos32, cell, config.pbc.to(torch.bool), cutoff, PARTITION_MAX_NUM_NEIGHBORS, False)
         labels = kdtree_partition_labels(pos32, counts.to(torch.int64), W)

@@ -531,3 +531,16 @@ def test_halo_maps_refuse_ranks_and_worlds_before_any_work(cuda, rank, W, monkey
     info.partition_id = torch.zeros(200, dtype=torch.int64, device=cuda)
     with pytest.raises(RuntimeError):
         D.SFCPartitioner().build_halo_maps(info, _state(pos, cuda), _env(rank, W), _cfg(cell, 4.0, 0.5))
+
+
+@pytest.mark.parametrize("device", ["cpu", "cuda:0"])
+def test_cutoffs_may_be_tensors(cuda, device):
+    pos, cell = _halo_case(31, 700, 18.0)
+    as_tensor = _cfg(cell, torch.tensor(5.0, device=device), torch.tensor(0.5, device=device))
+    for part in (D.SFCPartitioner(), D.KDTreePartitioner()):
+        a, b = (part.partition(_state(pos, cuda), _env(1, 3), c) for c in (as_tensor, _cfg(cell, 5.0, 0.5)))
+        assert torch.equal(a.partition_id, b.partition_id) and torch.equal(a.edge_index, b.edge_index)
+        for info, c in ((a, as_tensor), (b, _cfg(cell, 5.0, 0.5))):
+            part.build_halo_maps(info, _state(pos, cuda), _env(1, 3), c)
+        for key in HALO_LISTS:
+            assert torch.equal(getattr(a, key), getattr(b, key))
