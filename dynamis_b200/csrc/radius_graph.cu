@@ -70,7 +70,6 @@ struct DevHeader {
     uint32_t active_groups;  // entries of the list of groups that hold targets (target subsets only)
     float test_near, test_lo, test_hi;  // double positions: thresholds of the float test (float_test)
     uint32_t test_equal_is_near;
-    uint32_t long_groups;    // entries of the list of groups whose candidate list is too long for the hit bits
 };
 static_assert(offsetof(DevHeader, ncell_plus1) == sizeof(dynb_rg_header), "public header prefix mismatch");
 
@@ -896,7 +895,7 @@ template <typename T> struct PairParams {
     const uint2* smeta;       // [M] {atom id, packed shift code} per source record
     int32_t* counts_out;      // [Nt] degrees in caller order, or nullptr
     const uint32_t* glist;    // groups that hold at least one target (h->active_groups entries), or nullptr = all groups
-    uint32_t* long_list;      // groups whose candidate list exceeds the hit bits (h->long_groups entries, written by COUNT)
+    uint32_t* long_list;      // groups whose candidate list exceeds the hit bits (h->reserved[1] entries, written by COUNT)
     long long n_targets;
     // halo marking only (rg_halo_*): owner of every source record and of every target, and a word for every candidate run
     unsigned short* sown;     // [M]; lies over the binning slots, which nothing reads behind the plan
@@ -971,7 +970,8 @@ __device__ __forceinline__ uint32_t exact_hits(const PairParams<T>& p, uint32_t 
 template <typename T, int MODE, bool BYVAL>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
 rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T> params_val, long long* __restrict__ ei,
-               float* __restrict__ shifts, T* __restrict__ d2out, const long long E, const GlueArgs glue)
+               float* __restrict__ shifts, T* __restrict__ d2out, const long long E, const GlueArgs glue, const int all_groups,
+               long long* __restrict__ total)
 {
     // BYVAL: the launch has the record at hand and passes it as a kernel argument; its fields are then operands
     // of the instructions instead of registers loaded (and, under register pressure, reloaded) from the workspace
@@ -1002,13 +1002,14 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
     DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
     // behind rg_fillmask_kernel the writing pass has only the groups whose candidate list was too long for the hit bits
-    constexpr bool long_only = (MODE == MODE_FILL);
-    if (long_only && hp->long_groups == 0u) return;
+    const bool long_only = (MODE == MODE_FILL) && !all_groups;
+    if (long_only && hp->reserved[1] == 0) return;
+    if (MODE == MODE_FILL && total != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *total = E;
     int warp_max_slots = 0, max_degree = 0;
     const int nx = hp->nx, ny = hp->ny, nz = hp->nz, S = hp->group_cells, Sy = hp->group_cells_y, pad = hp->pad;
     const uint32_t gx = (uint32_t)hp->gx;
     const uint32_t gy = (uint32_t)((ny + Sy - 1) / Sy);
-    const uint32_t num_groups = long_only ? hp->long_groups
+    const uint32_t num_groups = long_only ? (uint32_t)hp->reserved[1]
                                           : (p.glist ? hp->active_groups : (uint32_t)hp->num_groups);  // < 2^31: never more groups than cells
     const int Wd = 2 * pad + 1, Wy = Sy + 2 * pad, nrun = Wy * Wd;
     const int lane_dy = (lane % Wy) - pad, lane_dz = (lane / Wy) - pad;
@@ -1058,7 +1059,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
         runs_compact(delta, run_a, run_off, run_len, lt);
         const bool write_masks = (MODE == MODE_COUNT) && nslots_total <= RG_MASK_SLOTS;
         warp_max_slots = max(warp_max_slots, nslots_total);
-        if (MODE == MODE_COUNT && nslots_total > RG_MASK_SLOTS && lane == 0) p.long_list[atomicAdd(&hp->long_groups, 1u)] = grp;
+        if (MODE == MODE_COUNT && nslots_total > RG_MASK_SLOTS && lane == 0) p.long_list[atomicAdd(reinterpret_cast<unsigned long long*>(&hp->reserved[1]), 1ull)] = grp;
 
         for (int cbeg = 0, chunk = 0; cbeg < L; cbeg += CAPX, chunk++) {
             const int clen = min(CAPX, L - cbeg);
@@ -2060,7 +2061,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     // there are no more groups than cells, and with a target subset no more of interest than targets
     const int64_t most_groups = std::min(host_grid ? (int64_t)gc_host.ncell_plus1 : cell_cap, targets != nullptr ? Nt : cell_cap);
     const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * 4 * PAIR_GRID_WAVES, (most_groups + PAIR_WARPS - 1) / PAIR_WARPS);
-    rg_pair_kernel<T, MODE_COUNT, true><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, pp_host, nullptr, nullptr, nullptr, 0, GlueArgs{});
+    rg_pair_kernel<T, MODE_COUNT, true><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, pp_host, nullptr, nullptr, nullptr, 0, GlueArgs{}, 0, nullptr);
     DYNB_CUDA_OK((exclusive_scan<uint32_t, long long>(tcount, toffset, nullptr, Nt + 1, sums64,
                                                        reinterpret_cast<long long*>(&h->E), stream)));
     DYNB_CUDA_OK(cudaGetLastError());
@@ -2069,14 +2070,32 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     return DYNB_OK;
 }
 
+constexpr int64_t RG_GROUPS_UNKNOWN = INT64_MAX / 2;  // for a caller who has not read the plan's header
+// Edges with distances when some lists are too long for the hit bits: one pass that tests every pair again, over all groups,
+// instead of the writer from the bits and that pass over the listed groups behind it?  Liquid of 0.1 atoms per A^3, one pass
+// against two, us (share of listed groups):
+//   200 k atoms, float:  348 / 333 (0.03), 320 / 367 (0.18), 368 / 447 (0.44), 559 / 578 (0.70)
+//   200 k atoms, double: 495 / 371 (0.03), 515 / 455 (0.18), 537 / 574 (0.44), 763 / 778 (0.70)
+//   20 k atoms (10 k groups), two listed groups: 60 / 76 float, 80 / 89 double -- the second pass is then a single warp's
+//   chain over its group, about 15 us with nothing beside it; 74 k groups, 148 listed: 338 / 318 and 474 / 353.
+// The order of the edges is the same.
+constexpr int64_t RG_AT_ONCE_GROUPS = 16384;
+template <typename T> static bool rg_write_at_once(int64_t groups, int64_t long_lists)
+{
+    if (long_lists <= 0 || groups >= RG_GROUPS_UNKNOWN) return false;
+    return groups <= RG_AT_ONCE_GROUPS || long_lists >= groups / (sizeof(T) == 8 ? 4 : 16);
+}
 template <typename T>
 static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int64_t E, const GlueArgs* glue_opt, int64_t* total_dev,
-                   bool long_lists, cudaStream_t stream)
+                   int64_t groups, int64_t long_lists, cudaStream_t stream)
 {
     const unsigned char* w = rg_base(ws);
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
-    // a warp for every 32 edges is more than there are groups with targets
-    const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * 4 * PAIR_GRID_WAVES, (E + 32 * PAIR_WARPS - 1) / (32 * PAIR_WARPS));
+    // A warp per group, up to the waves of PAIR_GRID_WAVES.  The groups are walked whether they hold edges or not, so their
+    // number bounds the launch and the number of edges does not: with E / 256 blocks the writer of a gas of a million atoms
+    // and 8 k edges took 4124 us against 324, of 200 k atoms and 28 k edges 283 against 97.
+    const int64_t full = (int64_t)sm_count_cached() * 4 * PAIR_GRID_WAVES;
+    const int grid = (int)std::max<int64_t>(std::min(full, (groups + PAIR_WARPS - 1) / PAIR_WARPS), 1);
     GlueArgs glue{};
     if (glue_opt != nullptr) glue = *glue_opt;
     // The edges come from the hit masks of the counting pass; the groups whose candidate list was too long for the masks
@@ -2084,6 +2103,14 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
     const int fsmem = PAIR_WARPS * FM_WARP_BYTES;
     auto* ei64 = reinterpret_cast<long long*>(ei);
     auto* d2 = static_cast<T*>(d2out);
+    const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
+    if (long_lists != 0) DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_FILL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (d2 != nullptr && rg_write_at_once<T>(groups, long_lists)) {
+        rg_pair_kernel<T, MODE_FILL, false><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, PairParams<T>{}, ei64, shifts, d2, (long long)E, glue,
+                                                                                 1, reinterpret_cast<long long*>(total_dev));
+        DYNB_CUDA_OK(cudaGetLastError());
+        return DYNB_OK;
+    }
     auto launch = [&](auto kernel) -> int {
         DYNB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fsmem));
         kernel<<<grid, PAIR_THREADS, fsmem, stream>>>(params_dev, ei64, shifts, d2, (long long)E, glue, reinterpret_cast<long long*>(total_dev));
@@ -2093,11 +2120,12 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
                                  : (glue_opt != nullptr ? launch(rg_fillmask_kernel<T, true, false>) : launch(rg_fillmask_kernel<T, false, false>));
     if (rc) return rc;
     // the groups the counting pass listed; a caller who has read the plan's header knows whether there are any
-    if (long_lists) {
-        const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
-        DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_FILL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        rg_pair_kernel<T, MODE_FILL, false><<<sm_count_cached() * 8, PAIR_THREADS, smem, stream>>>(params_dev, PairParams<T>{}, ei64, shifts, d2,
-                                                                                                   (long long)E, glue);
+    if (long_lists != 0) {
+        // Two waves where the caller has not read the header and most likely nothing is listed, else as many as the writer
+        // (200 k atoms at 8 A without distances: 508 against 543 us with two)
+        const int long_grid = (groups == RG_GROUPS_UNKNOWN && d2 == nullptr) ? std::min(grid, sm_count_cached() * 8) : grid;
+        rg_pair_kernel<T, MODE_FILL, false><<<long_grid, PAIR_THREADS, smem, stream>>>(params_dev, PairParams<T>{}, ei64, shifts, d2,
+                                                                                      (long long)E, glue, 0, nullptr);
     }
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
@@ -2186,7 +2214,7 @@ extern "C" int dynb_rg_bin(const void* pos_dev, int dtype, int64_t n_atoms, cons
 }
 
 static int rg_fill_any(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* shifts_dev, void* dist_sq_dev,
-                       const GlueArgs* glue, int64_t* total_dev, int64_t E, bool long_lists, void* stream)
+                       const GlueArgs* glue, int64_t* total_dev, int64_t E, int64_t groups, int64_t long_lists, void* stream)
 {
     if (workspace_dev == nullptr) return fail_arg("null workspace");
     if (E < 0) return fail_arg("E must be non-negative");
@@ -2196,21 +2224,27 @@ static int rg_fill_any(const void* workspace_dev, int dtype, int64_t* edge_index
         return DYNB_OK;
     }
     if (edge_index_dev == nullptr || shifts_dev == nullptr) return fail_arg("null output pointer");
-    if (dtype == DYNB_F32) return rg_fill<float>(workspace_dev, edge_index_dev, shifts_dev, dist_sq_dev, E, glue, total_dev, long_lists, s);
-    if (dtype == DYNB_F64) return rg_fill<double>(workspace_dev, edge_index_dev, shifts_dev, dist_sq_dev, E, glue, total_dev, long_lists, s);
+    if (dtype == DYNB_F32) return rg_fill<float>(workspace_dev, edge_index_dev, shifts_dev, dist_sq_dev, E, glue, total_dev, groups, long_lists, s);
+    if (dtype == DYNB_F64) return rg_fill<double>(workspace_dev, edge_index_dev, shifts_dev, dist_sq_dev, E, glue, total_dev, groups, long_lists, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");
 }
 
 extern "C" int dynb_rg_fill(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
                             void* dist_sq_dev, int64_t E, void* stream)
 {
-    return rg_fill_any(workspace_dev, dtype, edge_index_dev, cell_shifts_dev, dist_sq_dev, nullptr, nullptr, E, true, stream);
+    return rg_fill_any(workspace_dev, dtype, edge_index_dev, cell_shifts_dev, dist_sq_dev, nullptr, nullptr, E, RG_GROUPS_UNKNOWN, 1, stream);
 }
 
 extern "C" int dynb_rg_fill_counted(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
                                     void* dist_sq_dev, int64_t E, int long_lists, int64_t* total_dev, void* stream)
 {
-    return rg_fill_any(workspace_dev, dtype, edge_index_dev, cell_shifts_dev, dist_sq_dev, nullptr, total_dev, E, long_lists != 0, stream);
+    return dynb_rg_fill_groups(workspace_dev, dtype, edge_index_dev, cell_shifts_dev, dist_sq_dev, E, RG_GROUPS_UNKNOWN, long_lists, total_dev, stream);
+}
+
+extern "C" int dynb_rg_fill_groups(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
+                                   void* dist_sq_dev, int64_t E, int64_t groups, int64_t long_lists, int64_t* total_dev, void* stream)
+{
+    return rg_fill_any(workspace_dev, dtype, edge_index_dev, cell_shifts_dev, dist_sq_dev, nullptr, total_dev, E, groups, long_lists, stream);
 }
 
 extern "C" int dynb_rg_fill_glue(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* unit_shifts_dev,
@@ -2224,7 +2258,7 @@ extern "C" int dynb_rg_fill_glue(const void* workspace_dev, int dtype, int64_t* 
     g.id_map = reinterpret_cast<const long long*>(id_map_dev);
     g.negate = negate_shifts;
     for (int k = 0; k < 9; k++) g.c[k] = cell_host != nullptr ? cell_host[k] : 0.0f;
-    return rg_fill_any(workspace_dev, dtype, edge_index_dev, unit_shifts_dev, nullptr, &g, nullptr, E, true, stream);
+    return rg_fill_any(workspace_dev, dtype, edge_index_dev, unit_shifts_dev, nullptr, &g, nullptr, E, RG_GROUPS_UNKNOWN, 1, stream);
 }
 
 extern "C" int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, const int64_t* owner_dev, int64_t n_atoms,

@@ -89,7 +89,8 @@ class RadiusGraphPlan:
     valid until the next radius-graph call on the same device, which reuses the workspace.
     """
 
-    __slots__ = ("ws", "dtype_code", "E", "M", "counts", "device", "pos_dtype", "max_degree", "grid", "num_groups", "long_lists")
+    __slots__ = ("ws", "dtype_code", "E", "M", "counts", "device", "pos_dtype", "max_degree", "grid", "num_groups", "walked",
+                 "long_lists")
 
     def fill(self, want_dist_sq: bool = False, total: Optional[torch.Tensor] = None):
         """(edge_index, shifts, squared distances or None); ``total`` (one int64 on the device) receives E."""
@@ -103,9 +104,9 @@ class RadiusGraphPlan:
         return edge_index, shifts, d2
 
     def fill_into(self, edge_index, shifts, d2=None, total=None):
-        _lib.check(_lib.lib().dynb_rg_fill_counted(self.ws.data_ptr(), self.dtype_code, edge_index.data_ptr(), shifts.data_ptr(),
-                                                   d2.data_ptr() if d2 is not None else None, self.E, self.long_lists,
-                                                   total.data_ptr() if total is not None else None, _lib.stream_of(self.device)),
+        _lib.check(_lib.lib().dynb_rg_fill_groups(self.ws.data_ptr(), self.dtype_code, edge_index.data_ptr(), shifts.data_ptr(),
+                                                  d2.data_ptr() if d2 is not None else None, self.E, self.walked, self.long_lists,
+                                                  total.data_ptr() if total is not None else None, _lib.stream_of(self.device)),
                    "rg_fill")
 
     def fill_glue(self, cell: Optional[torch.Tensor], negate_shifts: bool = True, cartesian: bool = True,
@@ -252,7 +253,8 @@ def plan_radius_graph(pos, cell, pbc, radius, target_indices=None) -> RadiusGrap
     plan.max_degree = int(hdr.max_degree)
     plan.grid = (int(hdr.grid[0]), int(hdr.grid[1]), int(hdr.grid[2]))
     plan.num_groups = int(hdr.num_groups)
-    plan.long_lists = 1 if hdr.reserved[0] else 0
+    plan.walked = plan.num_groups if target_indices is None else min(plan.num_groups, Nt)  # groups the writer looks at
+    plan.long_lists = int(hdr.reserved[1])
     plan.counts = counts
     plan.device = dev
     plan.pos_dtype = pos.dtype

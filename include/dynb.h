@@ -63,7 +63,8 @@ typedef struct dynb_rg_header {
     int32_t group_cells;/* cells per warp work item along x */
     int64_t num_groups;
     int64_t reserved[2]; /* [0]: 0, or the longest candidate list in 32-record slots when one exceeded the 16 slots the
-                          * count pass keeps hit bits for (dynb_rg_fill recomputes the distances of those groups); [1]: unused */
+                          * count pass keeps hit bits for (dynb_rg_fill recomputes the distances of those groups);
+                          * [1]: the number of groups with such a list */
 } dynb_rg_header;
 
 /* Suggested capacities for a system: src_capacity bounds the number of periodic images
@@ -92,6 +93,12 @@ int dynb_rg_fill(const void* workspace_dev, int dtype, int64_t* edge_index_dev /
  * long candidate lists has anything to do (0 saves its launch); total_dev (optional, may be NULL) receives E. */
 int dynb_rg_fill_counted(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
                          void* dist_sq_dev, int64_t E, int long_lists, int64_t* total_dev, void* stream);
+
+/* The same with the launches chosen by what the header says: groups = header.num_groups, or with a target subset the
+ * smaller of that and n_targets; long_lists = header.reserved[1].  (The edges are the same for any number of groups, and
+ * for any number of long lists but a 0 that is not true.) */
+int dynb_rg_fill_groups(const void* workspace_dev, int dtype, int64_t* edge_index_dev, float* cell_shifts_dev,
+                        void* dist_sq_dev, int64_t E, int64_t groups, int64_t long_lists, int64_t* total_dev, void* stream);
 
 /* dynb_rg_fill for the model-side graph glue (dynamis_model/src/dynamis_model/nnp/mace.py:591-608,
  * uma.py:915-948): the models negate the offsets (unit_shifts = -cell_offsets), keep the edges whose

@@ -462,6 +462,36 @@ def test_workspace_at_any_address(cuda, dtype, offset):
     assert not buf[offset + nbytes.value:].any()
 
 
+@pytest.mark.parametrize("case", ["dilute", "liquid", "long lists", "subset"])
+@pytest.mark.parametrize("dist", [False, True])
+def test_edges_do_not_depend_on_the_writers_launch(cuda, case, dist):
+    """The writer's launch is sized by the number of groups: one warp for all of them, one each, or (unknown) all waves give
+    the same edges; so do far more groups than edges and groups whose lists are too long for the hit bits."""
+    from dynamis_b200 import _lib
+    from dynamis_b200.graph import plan_radius_graph
+
+    n, box, r = {"dilute": (3000, 300.0, 5.0), "liquid": (3000, 31.0, 5.0), "long lists": (3000, 24.0, 7.0), "subset": (3000, 31.0, 5.0)}[case]
+    pos, cell, pbc = _cubic(n, box, 11)
+    tp, tb = torch.as_tensor(pos, device=cuda), torch.tensor(pbc)
+    targets = torch.arange(0, n, 50, device=cuda) if case == "subset" else None
+    plan = plan_radius_graph(tp, torch.as_tensor(cell), tb, r, targets)
+    assert bool(plan.long_lists) == (case == "long lists")
+    if case == "dilute":
+        assert plan.E // 256 < plan.num_groups // 64
+    assert plan.walked == (plan.num_groups if targets is None else min(plan.num_groups, targets.numel()))
+    ref = plan.fill(dist)
+    assert_same_edges(canon_t(ref[0], ref[1]), canon_o(O.radius_graph(pos, cell, pbc, r, None if targets is None else targets.cpu().numpy())), case)
+    st = torch.cuda.current_stream(cuda).cuda_stream
+    for groups in (1, 2 ** 40):
+        out = [torch.full_like(t, -1) if t is not None else None for t in ref]
+        total = torch.zeros(1, dtype=torch.int64, device=cuda)
+        _lib.check(_lib.lib().dynb_rg_fill_groups(plan.ws.data_ptr(), plan.dtype_code, out[0].data_ptr(), out[1].data_ptr(),
+                                                  out[2].data_ptr() if dist else None, plan.E, groups, plan.long_lists, total.data_ptr(), st), "fill")
+        assert int(total) == plan.E
+        for a, b in zip(out, ref):
+            assert a is b is None or torch.equal(a, b)
+
+
 # ------------------------------------------------------------------ against the reference's own kernels
 
 def _run_ref(ref_ops, pos, cell, pbc, r, dev, targets=None):
