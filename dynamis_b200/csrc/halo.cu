@@ -44,10 +44,12 @@ bincount_i64_kernel(const int64_t* __restrict__ a, int64_t n, int64_t W, unsigne
     }
 }
 
-// Stream compaction in two launches: matches per tile, then every block adds up the tiles in front of its own (a few
-// thousand values out of L2 at most) and writes its matches.  A warp owns 256 consecutive values, so that the order is
-// kept by ballots alone.
+// Stream compaction in two launches: matches per tile, then every block adds up the tiles in front of its own and writes its
+// matches.  A warp owns 256 consecutive values, so that the order is kept by ballots alone.  Adding up is quadratic in the
+// tiles: above SELECT_FUSED_MAX_TILES (16.8 M values) a prefix sum over the tiles goes between the two (40 M values 160 us
+// either way, 100 M 296 against 412 us without it, 10^9 2.4 against 24.7 ms; a flag and a prefix sum per value took 10.0 ms).
 constexpr int SELECT_TILE = 2048;
+constexpr int64_t SELECT_FUSED_MAX_TILES = 8192;
 
 __global__ void __launch_bounds__(256)
 select_count_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, uint32_t* __restrict__ tile_count)
@@ -71,6 +73,7 @@ select_count_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, uin
     }
 }
 
+template <bool SUMMED>   // tile_count holds the matches in front of each tile already
 __global__ void __launch_bounds__(256)
 select_fill_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, const uint32_t* __restrict__ tile_count,
                    const int64_t* __restrict__ gather_src, int64_t* __restrict__ out, int64_t* __restrict__ count_out)
@@ -82,8 +85,12 @@ select_fill_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, cons
 #pragma unroll
     for (int k = 0; k < 8; k++) v[k] = (base + 32 * k < n) ? a[base + 32 * k] : ~value;
     uint32_t s = 0;
-    for (int i = threadIdx.x; i < (int)blockIdx.x; i += 256) s += tile_count[i];
-    s = __reduce_add_sync(0xffffffffu, s);
+    if (!SUMMED) {
+        for (int i = threadIdx.x; i < (int)blockIdx.x; i += 256) s += tile_count[i];
+        s = __reduce_add_sync(0xffffffffu, s);
+    } else if (threadIdx.x == 0) {
+        s = tile_count[blockIdx.x];
+    }
     uint32_t c = 0;
 #pragma unroll
     for (int k = 0; k < 8; k++) c += (v[k] == value) ? 1u : 0u;
@@ -92,7 +99,7 @@ select_fill_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, cons
     __syncthreads();
     uint32_t at = 0;
     for (int w = 0; w < 8; w++) at += before[w];
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count_out = (int64_t)at + tile_count[blockIdx.x];
+    if (!SUMMED && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count_out = (int64_t)at + tile_count[blockIdx.x];
     for (int w = 0; w < warp; w++) at += wsum[w];
     const uint32_t lt = lanemask_lt();
 #pragma unroll
@@ -596,11 +603,14 @@ extern "C" int dynb_bincount_i64(const int64_t* a_dev, int64_t n, int64_t W, int
     return DYNB_OK;
 }
 
+// workspace of a selection: matches per tile, then the sums of the prefix sum over them
+static int64_t select_sums_at(int64_t n) { return align_up((n / SELECT_TILE + 1) * 4, 256); }
+
 extern "C" int dynb_select_workspace_bytes(int64_t n, int64_t* bytes)
 {
     if (n < 0 || bytes == nullptr) return fail_arg("bad arguments");
     // the edge filter takes a workspace of dynb_select_workspace_bytes(2 * E) too
-    *bytes = std::max(align_up((n / SELECT_TILE + 1) * 4, 256), filter_layout(n / 2).total);
+    *bytes = std::max(select_sums_at(n) + align_up((int64_t)(scan_num_tiles(n / SELECT_TILE + 1) + 1) * 4, 256), filter_layout(n / 2).total);
     return DYNB_OK;
 }
 
@@ -618,7 +628,14 @@ extern "C" int dynb_select_eq_i64(const int64_t* a_dev, int64_t n, int64_t value
     uint32_t* tile_count = static_cast<uint32_t*>(workspace_dev);
     const unsigned tiles = nblk(n, SELECT_TILE);
     select_count_kernel<<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count);
-    select_fill_kernel<<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count, gather_src_dev, out_dev, count_dev);
+    if (tiles <= SELECT_FUSED_MAX_TILES) {
+        select_fill_kernel<false><<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count, gather_src_dev, out_dev, count_dev);
+    } else {
+        uint32_t* sums = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace_dev) + select_sums_at(n));
+        DYNB_CUDA_OK(cudaMemsetAsync(count_dev, 0, 8, s));
+        DYNB_CUDA_OK((exclusive_scan<uint32_t, uint32_t>(tile_count, tile_count, nullptr, tiles, sums, reinterpret_cast<uint32_t*>(count_dev), s)));
+        select_fill_kernel<true><<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count, gather_src_dev, out_dev, count_dev);
+    }
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }

@@ -518,6 +518,18 @@ def test_partition_indices_with_the_count_known_beforehand(cuda, n, W):
     assert D.SFCPartitioner().partition(_state(pos, cuda), _env(-1, W)).partition_indices.numel() == 0
 
 
+@pytest.mark.parametrize("n", [8192 * 2048, 8192 * 2048 + 1, 8193 * 2048 + 77])
+def test_select_eq_of_many_tiles(cuda, n):
+    """Around the number of tiles from which a prefix sum runs between counting and writing."""
+    from dynamis_b200.partition import select_eq
+
+    v = torch.randint(0, 5, (n,), device=cuda, generator=torch.Generator(device=cuda).manual_seed(9))
+    v[-1] = 3
+    ref = torch.nonzero(v == 3).reshape(-1)
+    assert torch.equal(select_eq(v, 3), ref) and int(ref[-1]) == n - 1
+    assert select_eq(v, 7).numel() == 0
+
+
 @pytest.mark.parametrize("rank,W", [(3, 3), (-1, 3), (0, 4097), (0, 0)])
 def test_halo_maps_refuse_ranks_and_worlds_before_any_work(cuda, rank, W, monkeypatch):
     from dynamis_b200 import partition
