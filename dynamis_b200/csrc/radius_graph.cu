@@ -1514,6 +1514,7 @@ __global__ void __launch_bounds__(256)
 rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo)
 {
     const PairParams<T> p = *params_dev;
+    if (halo.bad != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *halo.bad = 0u;  // for the marking behind this launch
     if (p.h->status & RG_FATAL) return;
     const int64_t M = (int64_t)p.h->M;
     const int64_t end = max(M, (int64_t)p.n_targets);  // the plan's targets, whatever the number of owners
@@ -2136,8 +2137,9 @@ static int rg_halo_mark(const void* ws, const HaloArgs& ha, int64_t N, cudaStrea
 {
     const unsigned char* w = rg_base(ws);
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
-    // the numbers of records and runs are known on the device only: both passes stride
-    rg_halo_owner_kernel<T><<<(unsigned)std::max<int64_t>((N + 255) / 256, (int64_t)sm_count_cached() * 4), 256, 0, stream>>>(params_dev, ha);
+    // the numbers of records and runs are known on the device only: both passes stride, the first with a thread for every
+    // record of a system with no more images than atoms
+    rg_halo_owner_kernel<T><<<(unsigned)((2 * N + 255) / 256), 256, 0, stream>>>(params_dev, ha);
     rg_halo_runs_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, ha);
     const int grid = sm_count_cached() * 4 * PAIR_GRID_WAVES;
     if (ha.words == 1) rg_halo_kernel<T, false><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
@@ -2277,7 +2279,6 @@ extern "C" int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, cons
     ha.rank = (int)rank;
     DYNB_CUDA_OK(cudaMemsetAsync(needed_dev, 0, (size_t)n_atoms * ha.words * 4, s));
     DYNB_CUDA_OK(cudaMemsetAsync(has_foreign_dev, 0, (size_t)n_atoms, s));
-    if (bad_dev != nullptr) DYNB_CUDA_OK(cudaMemsetAsync(bad_dev, 0, 4, s));
     if (dtype == DYNB_F32) return rg_halo_mark<float>(workspace_dev, ha, n_atoms, s);
     if (dtype == DYNB_F64) return rg_halo_mark<double>(workspace_dev, ha, n_atoms, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");

@@ -195,7 +195,6 @@ class AbstractPartitioner:
             ws = scratch(dev, "halo_lists", nbytes.value)
             # send offsets, recv offsets, number of own atoms and, behind them, the error word of the marking
             offs = torch.empty((2 * (W + 1) + 2,), dtype=torch.int64, device=dev)
-            bad = offs[-1:].view(torch.int32)
             offs_h = torch.empty((2 * (W + 1) + 2,), dtype=torch.int64, pin_memory=True)
             # everything up to the list sizes is queued before the one wait; the header's status is looked at behind it
             bins = BinnedAtoms(pos32, cell, pbc, ghost_cutoff) if N > 0 else None
@@ -203,16 +202,17 @@ class AbstractPartitioner:
                 if bins is not None:
                     bins.launch()
                     _lib.check(L.dynb_rg_halo_mark_rank(bins.ws.data_ptr(), bins.dtype_code, pid.data_ptr(), N, W, R, needed.data_ptr(),
-                                                        has_foreign.data_ptr(), bad.data_ptr(), _stream(dev)), "rg_halo_mark")
+                                                        has_foreign.data_ptr(), offs.data_ptr() + 8 * (2 * W + 3), _stream(dev)), "rg_halo_mark")
                 _lib.check(L.dynb_halo_lists_plan(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
                                                   ws.numel(), _stream(dev)), "halo_lists_plan")
                 offs_h.copy_(offs, non_blocking=True)
                 torch.cuda.current_stream(dev).synchronize()
                 if bins is None or bins.done():
                     break
-            if bins is not None and int(offs_h[-1:].view(torch.int32)[0]) != 0:
+            sizes = offs_h.tolist()
+            if bins is not None and sizes[2 * W + 3] & 0xFFFFFFFF != 0:
                 raise RuntimeError(f"build_halo_maps: partition_id has a label that is no rank's (world_size is {W})")
-            total_send, total_recv, n_local = int(offs_h[W]), int(offs_h[2 * W + 1]), int(offs_h[2 * W + 2])
+            total_send, total_recv, n_local = sizes[W], sizes[2 * W + 1], sizes[2 * W + 2]
             send_local = torch.empty((total_send,), dtype=torch.int64, device=dev)
             recv_atom = torch.empty((total_recv,), dtype=torch.int64, device=dev)
             recv_ghost = torch.empty((total_recv,), dtype=torch.int64, device=dev)
