@@ -1059,7 +1059,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
         runs_compact(delta, run_a, run_off, run_len, lt);
         const bool write_masks = (MODE == MODE_COUNT) && nslots_total <= RG_MASK_SLOTS;
         warp_max_slots = max(warp_max_slots, nslots_total);
-        if (MODE == MODE_COUNT && nslots_total > RG_MASK_SLOTS && lane == 0) p.long_list[atomicAdd(reinterpret_cast<unsigned long long*>(&hp->reserved[1]), 1ull)] = grp;
+        if (MODE == MODE_COUNT && nslots_total > RG_MASK_SLOTS && lane == 0) p.long_list[atomicAdd(reinterpret_cast<uint32_t*>(&hp->reserved[1]), 1u)] = grp;
 
         for (int cbeg = 0, chunk = 0; cbeg < L; cbeg += CAPX, chunk++) {
             const int clen = min(CAPX, L - cbeg);
