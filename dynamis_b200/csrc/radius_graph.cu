@@ -352,7 +352,7 @@ __device__ __forceinline__ void rg_last_block_chooses(DevHeader* h, const GridAr
 constexpr int WRAP_THREADS = 256;
 
 // FUSED: the grid is known before the launch (gc, chosen on the host), so the images and the targets are counted
-// into their cells here and no bounding box is gathered.
+// into their cells here; the bounding box then only steers the shape of the work items.
 template <typename T, bool FUSED>
 __global__ void __launch_bounds__(WRAP_THREADS)
 rg_wrap_kernel(const T* __restrict__ pos, int64_t N, Geom<T> g, int vec_ok, Vec4<T>* __restrict__ posw,

@@ -365,7 +365,8 @@ def test_distances_from_hit_bits(cuda, dtype, lists):
 @pytest.mark.parametrize("n_targets", [1, 2, 3, 16, 31, 33])
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_few_targets_per_group(cuda, n_targets, dtype):
-    """Odd and even numbers of targets in a group, some without any neighbour: the edge writer takes them two at a time."""
+    """Odd and even numbers of targets in a group, some without any neighbour: the count pass takes them two at a time,
+    the edge writer one after the other."""
     rng = np.random.default_rng(n_targets)
     pos = np.concatenate([rng.random((400, 3)) * 8.0, 20.0 + rng.random((6, 3)) * 15.0]).astype(dtype)
     cell = (np.eye(3) * 40.0).astype(dtype)
