@@ -13,22 +13,22 @@
 //   scan           cell starts
 //   rg_bin_scatter provisional slot inside each cell (atomic rank)
 //   rg_bin_finalize deterministic order inside each cell, write packed source / target records
-//   rg_pair<COUNT> per-target degree                                     (ref :197-258)
+//   rg_count       per-target degree and hit bits                        (ref :197-258)
 //   scan           edge offsets + total
 //   rg_fillmask    edges from the hit bits of the count pass             (ref :282-442)
-//   rg_pair<FILL>  edges of groups whose candidate list is too long for hit bits
+//   rg_pair        edges of groups whose candidate list is too long for hit bits
 //
 // The edge SET is fixed by three predicates that are kept expression-for-expression identical to
 // the reference (same operand order, compiled with the same default FMA contraction): the wrap,
 // the periodic-image test with the image position, and d2 <= r2 && d2 > 1e-8f.  The cell grid
 // only decides which pairs are examined and is free to differ.
 //
-// Work decomposition of rg_pair: one warp owns a group of group_cells x group_cells_y cells (x, y)
+// Work decomposition of the cell scan: one warp owns a group of group_cells x group_cells_y cells (x, y)
 // and all targets inside.  It flattens the contiguous runs of neighbouring source records (one run
-// per (y, z) row, one lane per run) into a dense shared-memory list once, then tests the targets two
-// at a time against the list with one candidate per lane (conflict-free 16-byte shared loads, ballot +
-// popc compaction).  Hits are parked in per-target lists and written out 32 edges at a time so that
-// the 8-byte index stores of a warp cover one contiguous 256-byte run.  With a target subset the
+// per (y, z) row, one lane per run) into one list, the same in every pass.  rg_count tests the targets one at a time against
+// candidates in registers; the writers find the edges in its hit bits; rg_pair tests the targets of long lists two at a time
+// against candidates in shared memory (ballot + popc compaction, hits parked in per-target lists).  Edges are written 32 at
+// a time so that the 8-byte index stores of a warp cover one contiguous 256-byte run.  With a target subset the
 // source images are first clipped to the targets' bounding box grown by the cutoff.
 
 #include "common.cuh"
@@ -275,9 +275,8 @@ __device__ __forceinline__ unsigned long long f32x2_pack(float lo, float hi)
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
     return r;
 }
-__device__ __forceinline__ void dist2_x2(unsigned long long ax2, unsigned long long ay2, unsigned long long az2,
-                                         unsigned long long sx2, unsigned long long sy2, unsigned long long sz2,
-                                         float& d_lo, float& d_hi)
+__device__ __forceinline__ unsigned long long dist2_x2(unsigned long long ax2, unsigned long long ay2, unsigned long long az2,
+                                                       unsigned long long sx2, unsigned long long sy2, unsigned long long sz2)
 {
     unsigned long long dx, dy, dz, d;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dx) : "l"(ax2), "l"(sx2));
@@ -286,7 +285,7 @@ __device__ __forceinline__ void dist2_x2(unsigned long long ax2, unsigned long l
     asm("mul.rn.f32x2 %0, %1, %1;" : "=l"(d) : "l"(dy));
     asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(dx), "l"(d));
     asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(dz), "l"(d));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(d_lo), "=f"(d_hi) : "l"(d));
+    return d;
 }
 
 // The grid when the host cannot choose it: from the bounding boxes of the images and, with a target subset, of the targets,
@@ -696,10 +695,10 @@ __device__ __forceinline__ float scan_coord(double x, double origin) { return (f
 // (conversion, three subtractions, three roundings of the sum); twice that is the margin around r^2 and above the
 // self-distance limit.  The thresholds are rounded outwards, a distance that is not a number is never decided here, and
 // coordinates near the end of the float range are left to the double test altogether.
-// Two records with the same three floats lie within 2 u X of one another along each axis: when that puts them inside the
-// self-distance limit, an undecided pair of equal floats (every target meets itself) is no neighbour and needs no double test.
-// 500 k atoms of silicon, 6 A: 364 -> 228 us (32-byte candidates in chunks of 160 and a double test for each of them before;
-// now all 512 places in one chunk and the packed float test, a double test for about one candidate in 10^5).
+// A float distance of zero means coordinates within 2 u X of one another along each axis (equal floats, or ones so close to
+// zero that the square underflows): when that puts them inside the self-distance limit, the pair (every target meets itself)
+// is no neighbour and needs no double test.  500 k atoms of silicon, 6 A: 364 us with a double test for every candidate, 228
+// with this one.
 __device__ __forceinline__ void float_test(double r2, double X, float& near, float& lo, float& hi, uint32_t& equal_is_near)
 {
     const double u = 5.9604644775390625e-8, eta = 2.0 * u * X, eps = (double)1e-8f;
@@ -723,7 +722,7 @@ __global__ void __launch_bounds__(256)
 rg_bin_finalize_kernel(int64_t Nt, int subset, Geom<T> g, const Vec4<T>* __restrict__ posw, DevHeader* __restrict__ hp,
                        const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ tcstart,
                        const SlotRec<T>* __restrict__ srec, const SlotRec<T>* __restrict__ trec,
-                       Vec4<T>* __restrict__ spos, float* __restrict__ sxyz, long long sxyz_stride,
+                       Vec4<T>* __restrict__ spos, float4* __restrict__ sscan,
                        uint2* __restrict__ smeta, Vec4<T>* __restrict__ tpos, float4* __restrict__ tscan,
                        int4* __restrict__ tmeta, double r2)
 {
@@ -785,9 +784,8 @@ rg_bin_finalize_kernel(int64_t Nt, int subset, Geom<T> g, const Vec4<T>* __restr
         Vec4<T> r;
         r.x = sw.x; r.y = sw.y; r.z = sw.z; r.w = bits_to_real((int32_t)s.id, T());
         spos[at] = r;
-        sxyz[at] = scan_coord(sw.x, hp->gmin[0]);
-        sxyz[sxyz_stride + at] = scan_coord(sw.y, hp->gmin[1]);
-        sxyz[2 * sxyz_stride + at] = scan_coord(sw.z, hp->gmin[2]);
+        if (sizeof(T) == 8)
+            sscan[at] = make_float4(scan_coord(sw.x, hp->gmin[0]), scan_coord(sw.y, hp->gmin[1]), scan_coord(sw.z, hp->gmin[2]), 0.0f);
         smeta[at] = make_uint2(s.id, s.code);
         // its shift is zero: the code is minus the floor
         if (!subset && s.key == center)
@@ -849,12 +847,35 @@ __device__ __forceinline__ int runs_flags(uint32_t* flags, int run_off, int run_
     return __popc(before);
 }
 
-enum { MODE_COUNT = 0, MODE_FILL = 1 };
-
-#ifndef DYNB_COUNT_UNROLL
-#define DYNB_COUNT_UNROLL 1
-#endif
-constexpr int COUNT_UNROLL = DYNB_COUNT_UNROLL;  // unroll factor of the count pass's test loop (tuning knob at build time)
+__device__ __forceinline__ int lane_id()
+{
+    int l;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));  // volatile: kept in a register instead of read again
+    return l;
+}
+// What a warp keeps to find the record behind a place of its candidate list (one chunk of up to 512 places).
+struct RunIndex {
+    int delta[32];                  // per non-empty run: record = delta + place
+    uint32_t flags[RUN_FLAG_WORDS]; // places of the chunk where a run starts
+    uint2 word[RUN_FLAG_WORDS];     // the same word, and the number of runs that start in front of it, minus one
+    // lane r owns run r (run_a = first record, run_off = place in the list); the chunk starts at place cbeg
+    __device__ __forceinline__ void set(int run_a, int run_off, int run_len, int cbeg, int lane, uint32_t lt)
+    {
+        runs_compact(delta, run_a, run_off, run_len, lt);
+        const int before = runs_flags(flags, run_off, run_len, lane, cbeg);
+        const uint32_t f = lane < RUN_FLAG_WORDS ? flags[lane] : 0u;
+        int starts;
+        const int rank = before + warp_excl_scan(__popc(f), lane, &starts);
+        if (lane < RUN_FLAG_WORDS) word[lane] = make_uint2(f, (uint32_t)(rank - 1));
+        __syncwarp();
+    }
+    // record - place, for place 32 s + lane of the chunk
+    __device__ __forceinline__ int record(int s, uint32_t le) const
+    {
+        const uint2 f = word[s];
+        return delta[(int)f.y + __popc(f.x & le)];
+    }
+};
 
 // Optional extras of the edge writers for the model-side glue: the shifts written with the caller's sign
 // and the Cartesian shift of every edge, unit_shift @ cell, rounded like a K = 3 float GEMM
@@ -879,13 +900,57 @@ __device__ __forceinline__ void glue_write(const GlueArgs& g, float* __restrict_
     }
 }
 
+// The grid and the shape of the groups, and one group: its targets (one contiguous run a cell row, at most two rows) and this
+// lane's run of source records.  Both cell-scan kernels keep the grid in shared memory and read it where a group is looked
+// up: in registers it left too few for the loops.
+struct GroupShape { int nx, ny, nz, sx, sy, pad, gx, gy; };
+struct GroupDesc { uint32_t tb0, te0, tb1, te1; int run_a, run_len; };
+__device__ __forceinline__ GroupShape group_shape(const DevHeader* hp)
+{
+    return {hp->nx, hp->ny, hp->nz, hp->group_cells, hp->group_cells_y, hp->pad, hp->gx, (hp->ny + hp->group_cells_y - 1) / hp->group_cells_y};
+}
+// lane r owns run r: (z row, y row) of it, counted from the lowest; -1: no run
+__device__ __forceinline__ int group_lane_run(const GroupShape& g, int lane)
+{
+    const int wy = g.sy + 2 * g.pad;
+    return lane < wy * (2 * g.pad + 1) ? (((lane / wy) << 8) | (lane % wy)) : -1;
+}
+__device__ __forceinline__ GroupDesc fetch_group(const volatile GroupShape& g, const uint32_t* tcstart, const uint32_t* cstart, uint32_t grp, int lane_run)
+{
+    GroupDesc d;
+    const int nx = g.nx, ny = g.ny, pad = g.pad, sx = g.sx, sy = g.sy;
+    const uint32_t gx = (uint32_t)g.gx, gy = (uint32_t)g.gy;
+    const uint32_t row = grp / gx;
+    const int cz = (int)(row / gy), cx0 = (int)(grp - row * gx) * sx, cy0 = (int)(row - (uint32_t)cz * gy) * sy;
+    const int cx1 = min(cx0 + sx, nx) - 1, cy1 = min(cy0 + sy, ny) - 1;
+    const uint32_t* tcell = tcstart + ((uint32_t)cz * ny + cy0) * nx;
+    d.tb0 = tcell[cx0];
+    d.te0 = tcell[cx1 + 1];
+    d.tb1 = d.te1 = 0;
+    if (cy1 > cy0) {
+        d.tb1 = tcell[nx + cx0];
+        d.te1 = tcell[nx + cx1 + 1];
+    }
+    d.run_a = 0;
+    d.run_len = 0;
+    if (lane_run >= 0) {
+        const int yy = cy0 - pad + (lane_run & 255), zz = cz - pad + (lane_run >> 8);
+        if (yy >= 0 && yy < ny && yy <= cy1 + pad && zz >= 0 && zz < g.nz) {
+            const uint32_t* cell = cstart + ((uint32_t)zz * ny + yy) * nx;
+            const uint32_t a = cell[max(cx0 - pad, 0)], e = cell[min(cx1 + pad, nx - 1) + 1];
+            d.run_a = (int)a;
+            d.run_len = (int)(e - a);
+        }
+    }
+    return d;
+}
+
 template <typename T> struct PairParams {
     DevHeader* h;
     const uint32_t* cstart;
     const uint32_t* tcstart;
     const Vec4<T>* spos;
-    const float* sxyz;        // coordinates of the source records as three arrays, each sxyz_stride long (scan_coord)
-    long long sxyz_stride;
+    const float4* sscan;      // the source records' coordinates as the count pass tests them (float: the records themselves)
     const Vec4<T>* tpos;
     const float4* tscan;      // the targets' coordinates as the count pass tests them, and the entry
     const int4* tmeta;
@@ -946,52 +1011,229 @@ rg_group_list_kernel(const PairParams<T>* __restrict__ params_dev, uint32_t* __r
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// rg_count: degrees and hit bits.  Lane l holds the coordinates of candidates l, 32 + l, 64 + l, ... of its warp's list in
+// registers, two candidates to a packed register pair, and the targets pass by one at a time: the test loop reads nothing from
+// memory and is unrolled over the whole list.  (Before: candidates in shared memory, two targets at a time; three of its
+// loads, the shifting of the bit and eight compares with selects for every 64 candidates and two targets.)
+// Bound by the FMA pipe and the issue of instructions (issue slots 64 % busy, 190 M warp instructions for a million atoms of the
+// liquid against 245 M; a packed instruction holds the FMA pipe for two cycles).  Before and after: 300 -> 270 us (liquid, 1 M
+// atoms, 5 A), 357 -> 313 (a rank's 1 M of the 8 M copper atoms), 226 -> 172 (silicon in double precision, 500 k atoms, 6 A).
+// ------------------------------------------------------------------------------------------
+// Seven blocks of four warps: 72 registers.  80 registers and six blocks 276 us, 96 and five 281, 128 and four 293 (liquid).
+// Blocks of two warps, and half or twice the waves: within 2 %.
+constexpr int COUNT_WARPS = 4;
+constexpr int COUNT_BLOCKS = 7;
+constexpr int COUNT_WAVES = 8;
+
+// Thresholds of a distance test, each twice: a bit is set when lo <= d < hi, where lo and hi are the floats behind the bounds of
+// "d > near && d <= upto", and hi >= lo.  A difference of two floats is zero only for equal ones, so the signs of d - lo and
+// d - hi are exact, and that of their product (which keeps it when it underflows) is set between the two.  Two packed
+// subtractions, a packed product and a funnel shift a bit: as compares and selects the bits kept the ALU pipe busier than the
+// distances the FMA pipe (289 us against 276, liquid of a million atoms).
+struct SignTest { unsigned long long lo, hi; };
+__device__ __forceinline__ SignTest sign_test(float near, float upto)
+{
+    const float lo = nextafterf(near, INFINITY), hi = fmaxf(nextafterf(upto, INFINITY), lo);
+    SignTest t;
+    t.lo = f32x2_pack(lo, lo);
+    t.hi = f32x2_pack(hi, hi);
+    return t;
+}
+// bits = bits << 2 with the outcomes for the two distances of d (the upper one first)
+__device__ __forceinline__ void test_x2(unsigned long long d, const SignTest& t, uint32_t& bits)
+{
+    unsigned long long a, b;
+    uint32_t s0, s1;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(d), "l"(t.lo));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(b) : "l"(d), "l"(t.hi));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(s0), "=r"(s1) : "l"(a));
+    bits = __funnelshift_l(s1, bits, 1);
+    bits = __funnelshift_l(s0, bits, 1);
+}
+
 // The undecided candidates of a target (bit s: place 32 s + lane of the staged chunk) by the double test.
 template <typename T>
-__device__ __forceinline__ uint32_t exact_hits(const PairParams<T>& p, uint32_t t, uint32_t undecided, bool equal_is_near, float ax, float ay,
-                                               float az, const float* xs, const int* delta, const uint32_t* flags, const int* wpre, int cbeg,
-                                               int clen, int lane, uint32_t le)
+__device__ __forceinline__ uint32_t exact_hits(const PairParams<T>& p, uint32_t t, uint32_t undecided, const RunIndex& index, int cbeg, int clen,
+                                               int lane, uint32_t le)
 {
-    constexpr int PK = RG_MASK_SLOTS * 32;
     uint32_t hits = 0;
     while (undecided) {
         const int s = __ffs((int)undecided) - 1, j = 32 * s + lane;
         undecided &= undecided - 1;
         if (j >= clen) continue;  // padding
-        const float* x = xs + ((j >> 6) * 64 + lane * 2 + (s & 1));
-        if (equal_is_near && x[0] == ax && x[PK] == ay && x[2 * PK] == az) continue;
-        const Vec4<T> c = p.spos[delta[wpre[s] + __popc(flags[s] & le) - 1] + cbeg + j], a = p.tpos[t];
+        const Vec4<T> c = p.spos[index.record(s, le) + cbeg + j], a = p.tpos[t];
         const T d = dist2<T>(a.x, a.y, a.z, c.x, c.y, c.z);
         if (d <= p.r2 && d > (T)1e-8f) hits |= 1u << s;
     }
     return hits;
 }
 
-template <typename T, int MODE, bool BYVAL>
+struct CountGroup {
+    uint32_t tb0, n0, tb1, ntot;   // targets of the two rows
+    int cbeg, clen;                // chunk of the candidate list
+    bool write_masks, first, last;
+};
+// The targets of a group against the chunk's candidates, at most 64 NB of them and more than 64 FULL.
+template <typename T, int NB, int FULL>
+__device__ __forceinline__ void count_group(const PairParams<T>& p, const RunIndex& index, const CountGroup& g, const SignTest& hit, const SignTest& may,
+                                            const bool all_undecided, int& max_degree, const int lane, const uint32_t le)
+{
+    unsigned long long cx[NB], cy[NB], cz[NB];
+    {
+        const float4* src = p.sscan + g.cbeg;
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+            float4 v[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int s = 2 * b + i;
+                if (b < FULL) {
+                    v[i] = src[index.record(s, le) + 32 * s + lane];
+                } else {
+                    // a padding place reads the last record; x alone keeps it out of every cutoff, its distance is infinite
+                    const int j = min(32 * s + lane, g.clen - 1);
+                    const uint2 f = index.word[j >> 5];
+                    v[i] = src[index.delta[(int)f.y + __popc(f.x & (0xffffffffu >> (31 - (j & 31))))] + j];
+                    if (32 * s + lane >= g.clen) v[i].x = 3.0e38f;
+                }
+            }
+            cx[b] = f32x2_pack(v[0].x, v[1].x);
+            cy[b] = f32x2_pack(v[0].y, v[1].y);
+            cz[b] = f32x2_pack(v[0].z, v[1].z);
+        }
+    }
+    int degree = 0;  // lane l collects the degree of target 32 j + l; stored 32 targets at a time
+    float4 next = p.tscan[g.n0 != 0 ? g.tb0 : g.tb1];  // w = entry
+    uint32_t at = g.n0 != 0 ? g.tb0 : g.tb1;
+#pragma unroll 1
+    for (uint32_t k = 0; k < g.ntot;) {
+        const float4 t = next;
+        const uint32_t mine_at = at;
+        at = (k + 1 == g.n0) ? g.tb1 : at + 1;
+        if (k + 1 >= g.ntot) at = mine_at;
+        next = p.tscan[at];
+        const unsigned long long ax = f32x2_pack(t.x, t.x), ay = f32x2_pack(t.y, t.y), az = f32x2_pack(t.z, t.z);
+        uint32_t bits = 0, maybe = 0;
+#pragma unroll
+        for (int b = NB - 1; b >= 0; b--) {
+            const unsigned long long d = dist2_x2(ax, ay, az, cx[b], cy[b], cz[b]);
+            test_x2(d, hit, bits);
+            if (sizeof(T) == 8) test_x2(d, may, maybe);
+        }
+        if constexpr (sizeof(T) == 8)
+            bits |= exact_hits<T>(p, mine_at, (all_undecided ? 0xffffu >> (16 - 2 * NB) : maybe) & ~bits, index, g.cbeg, g.clen, lane, le);
+        if (g.write_masks) p.hitmask[(size_t)mine_at * 32 + lane] = (unsigned short)bits;
+        int n = __reduce_add_sync(0xffffffffu, __popc(bits));
+        if (!g.first) n += (int)p.tcount[mine_at];
+        if (lane == (int)(k & 31u)) degree = n;
+        k++;
+        if ((k & 31u) == 0u || k == g.ntot) {
+            __syncwarp();
+            const uint32_t mine = ((k - 1) & ~31u) + (uint32_t)lane;
+            if (mine < k) {
+                const uint32_t to = (mine < g.n0) ? g.tb0 + mine : g.tb1 + (mine - g.n0);
+                p.tcount[to] = (uint32_t)degree;
+                if (g.last) {
+                    if (p.counts_out != nullptr) p.counts_out[__float_as_int(p.tscan[to].w)] = degree;  // in caller order
+                    max_degree = max(max_degree, degree);
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(COUNT_WARPS * 32, COUNT_BLOCKS)
+rg_count_kernel(const PairParams<T> p)
+{
+    __shared__ RunIndex indexes[COUNT_WARPS];
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    RunIndex& index = indexes[warp];
+    const uint32_t lt = lanemask_lt(), le = lt | (1u << lane);
+    __shared__ GroupShape shape;
+    DevHeader* hp = p.h;
+    if (hp->status & RG_FATAL) return;
+    int warp_max_slots = 0, max_degree = 0;
+    if (threadIdx.x == 0) shape = group_shape(hp);
+    const uint32_t num_groups = p.glist ? hp->active_groups : (uint32_t)hp->num_groups;  // < 2^31: never more groups than cells
+    __syncthreads();
+    const int lane_run = group_lane_run(shape, lane);
+    const SignTest hit = sizeof(T) == 8 ? sign_test(hp->test_near, hp->test_lo) : sign_test(1e-8f, (float)p.r2);
+    const SignTest may = sizeof(T) == 8 ? sign_test(hp->test_equal_is_near ? 0.0f : -1.0f, hp->test_hi) : hit;
+    const bool all_undecided = sizeof(T) == 8 && hp->test_lo < 0.0f;  // coordinates out of the float test's range (float_test)
+
+    const uint32_t nwarps = gridDim.x * COUNT_WARPS;
+#pragma unroll 1
+    for (uint32_t gi = blockIdx.x * COUNT_WARPS + warp; gi < num_groups; gi += nwarps) {
+        const uint32_t grp = p.glist ? p.glist[gi] : gi;
+        const GroupDesc d = fetch_group(shape, p.tcstart, p.cstart, grp, lane_run);
+        const int run_a = d.run_a, run_len = d.run_len;
+        CountGroup g;
+        g.tb0 = d.tb0;
+        g.tb1 = d.tb1;
+        g.n0 = d.te0 - d.tb0;
+        g.ntot = g.n0 + (d.te1 - d.tb1);
+        if (g.ntot == 0) continue;
+        int L;
+        const int run_off = warp_excl_scan(run_len, lane, &L);
+        const int nslots = (L + 31) >> 5;
+        g.write_masks = nslots <= RG_MASK_SLOTS;
+        warp_max_slots = max(warp_max_slots, nslots);
+        if (nslots > RG_MASK_SLOTS && lane == 0) p.long_list[atomicAdd(reinterpret_cast<uint32_t*>(&hp->reserved[1]), 1u)] = grp;
+#pragma unroll 1
+        for (g.cbeg = 0; g.cbeg < L; g.cbeg += RG_MASK_SLOTS * 32) {
+            g.clen = min(RG_MASK_SLOTS * 32, L - g.cbeg);
+            g.first = g.cbeg == 0;
+            g.last = g.cbeg + RG_MASK_SLOTS * 32 >= L;
+            __syncwarp();
+            index.set(run_a, run_off, run_len, g.cbeg, lane, lt);
+            auto run = [&](auto nb, auto full) {
+                count_group<T, decltype(nb)::value, decltype(full)::value>(p, index, g, hit, may, all_undecided, max_degree, lane, le);
+            };
+            // a copy of the test loop for every length but the shortest: no block of 64 is tested for nothing
+            switch ((g.clen + 63) >> 6) {
+            case 1:
+            case 2: run(std::integral_constant<int, 2>(), std::integral_constant<int, 0>()); break;
+            case 3:
+            case 4: run(std::integral_constant<int, 4>(), std::integral_constant<int, 2>()); break;
+            case 5: run(std::integral_constant<int, 5>(), std::integral_constant<int, 4>()); break;
+            case 6: run(std::integral_constant<int, 6>(), std::integral_constant<int, 5>()); break;
+            case 7: run(std::integral_constant<int, 7>(), std::integral_constant<int, 6>()); break;
+            default: run(std::integral_constant<int, 8>(), std::integral_constant<int, 7>()); break;
+            }
+        }
+        // a group whose neighbourhood holds no source at all still owes its targets a zero
+        if (L == 0)
+            for (uint32_t k = lane; k < g.ntot; k += 32) p.tcount[(k < g.n0) ? g.tb0 + k : g.tb1 + (k - g.n0)] = 0;
+    }
+    {   // largest degree: one atomic per block
+        __shared__ int s_max_degree;
+        if (threadIdx.x == 0) s_max_degree = 0;
+        __syncthreads();
+        max_degree = __reduce_max_sync(0xffffffffu, max_degree);
+        if (lane == 0 && max_degree > 0) atomicMax(&s_max_degree, max_degree);
+        __syncthreads();
+        if (threadIdx.x == 0 && s_max_degree > 0) atomicMax(&hp->max_degree, (uint32_t)s_max_degree);
+    }
+    // a candidate list too long for the hit bits: the edge writer has to recompute distances
+    if (lane == 0 && warp_max_slots > RG_MASK_SLOTS) atomicMax(&hp->reserved[0], (long long)warp_max_slots);
+}
+
+template <typename T>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
-rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T> params_val, long long* __restrict__ ei,
+rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restrict__ ei,
                float* __restrict__ shifts, T* __restrict__ d2out, const long long E, const GlueArgs glue, const int all_groups,
                long long* __restrict__ total)
 {
-    // BYVAL: the launch has the record at hand and passes it as a kernel argument; its fields are then operands
-    // of the instructions instead of registers loaded (and, under register pressure, reloaded) from the workspace
-    PairParams<T> params_loaded;
-    if constexpr (!BYVAL) params_loaded = *params_dev;
-    const PairParams<T>& p = BYVAL ? params_val : params_loaded;
+    const PairParams<T> p = *params_dev;
     extern __shared__ __align__(32) unsigned char smem_raw[];
     constexpr int CAP = PAIR_CAND_BYTES / (int)sizeof(Vec4<T>);
-    // The count pass keeps its candidates as three arrays of float coordinates (no atom ids, no shift codes: the
-    // space of both holds a whole list with hit bits) laid out for the packed distance test: the 8 bytes that
-    // lane l reads for block b hold the coordinate of candidates 64 b + l and 64 b + 32 + l.
-    constexpr bool PACKED = (MODE == MODE_COUNT);
-    constexpr int PK = RG_MASK_SLOTS * 32;
-    constexpr int CAPX = PACKED ? PK : CAP;
-    static_assert(3 * 4 * PK + 4 * RUN_FLAG_WORDS <= PAIR_CAND_BYTES + PAIR_CODE_BYTES, "packed candidates must fit the record and code space");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char* wbase = smem_raw + warp * PAIR_WARP_BYTES;
     Vec4<T>* cand = reinterpret_cast<Vec4<T>*>(wbase);
-    float* xs = reinterpret_cast<float*>(wbase);
-    int* wpre = reinterpret_cast<int*>(wbase + 3 * 4 * PK);  // runs that start in front of each word of flags
     uint32_t* codes = reinterpret_cast<uint32_t*>(wbase + PAIR_CAND_BYTES);
     unsigned short* listA = reinterpret_cast<unsigned short*>(wbase + PAIR_CAND_BYTES + PAIR_CODE_BYTES);
     unsigned short* listB = listA + PAIR_LIST;
@@ -1002,10 +1244,9 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
     DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
     // behind rg_fillmask_kernel the writing pass has only the groups whose candidate list was too long for the hit bits
-    const bool long_only = (MODE == MODE_FILL) && !all_groups;
+    const bool long_only = !all_groups;
     if (long_only && hp->reserved[1] == 0) return;
-    if (MODE == MODE_FILL && total != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *total = E;
-    int warp_max_slots = 0, max_degree = 0;
+    if (total != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *total = E;
     const int nx = hp->nx, ny = hp->ny, nz = hp->nz, S = hp->group_cells, Sy = hp->group_cells_y, pad = hp->pad;
     const uint32_t gx = (uint32_t)hp->gx;
     const uint32_t gy = (uint32_t)((ny + Sy - 1) / Sy);
@@ -1016,10 +1257,6 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
     const T r2 = p.r2;
     const T eps = (T)1e-8f;
     const uint32_t lt = lanemask_lt();
-    constexpr bool FLOAT_FIRST = PACKED && sizeof(T) == 8;
-    const float near = FLOAT_FIRST ? hp->test_near : (float)eps, upto = FLOAT_FIRST ? hp->test_lo : (float)r2;
-    const float beyond = FLOAT_FIRST ? hp->test_hi : 0.0f;
-    const bool equal_is_near = FLOAT_FIRST && hp->test_equal_is_near;
 
     const uint32_t nwarps = gridDim.x * PAIR_WARPS;
     for (uint32_t gi = blockIdx.x * PAIR_WARPS + warp; gi < num_groups; gi += nwarps) {
@@ -1054,50 +1291,16 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
         }
         int L;
         const int run_off = warp_excl_scan(run_len, lane, &L);
-        const int nslots_total = (L + 31) >> 5;
         __syncwarp();
         runs_compact(delta, run_a, run_off, run_len, lt);
-        const bool write_masks = (MODE == MODE_COUNT) && nslots_total <= RG_MASK_SLOTS;
-        warp_max_slots = max(warp_max_slots, nslots_total);
-        if (MODE == MODE_COUNT && nslots_total > RG_MASK_SLOTS && lane == 0) p.long_list[atomicAdd(reinterpret_cast<uint32_t*>(&hp->reserved[1]), 1u)] = grp;
 
-        for (int cbeg = 0, chunk = 0; cbeg < L; cbeg += CAPX, chunk++) {
-            const int clen = min(CAPX, L - cbeg);
+        for (int cbeg = 0, chunk = 0; cbeg < L; cbeg += CAP, chunk++) {
+            const int clen = min(CAP, L - cbeg);
             const int clen32 = (clen + 31) & ~31;
-            const bool more_chunks = cbeg + CAPX < L;
+            const bool more_chunks = cbeg + CAP < L;
             // dense staging: slot j of the list holds flattened candidate cbeg + j; all loads of a chunk are
             // independent
             int rank_base = runs_flags(flags, run_off, run_len, lane, cbeg);
-            if constexpr (FLOAT_FIRST) {
-                int starts;
-                const int before = warp_excl_scan(lane < RUN_FLAG_WORDS ? __popc(flags[lane]) : 0, lane, &starts);
-                if (lane < RUN_FLAG_WORDS) wpre[lane] = rank_base + before;
-            }
-            if constexpr (PACKED) {
-                // Per 64 candidates two rounds; in each the lower half-warp takes 16 candidates of the block's
-                // first 32 and the upper half-warp 16 of its second 32, so that the 32 four-byte stores of a
-                // round fall into 32 different banks and each half-warp reads 64 contiguous bytes per array.
-                const int half = lane >> 4, l16 = lane & 15;
-                for (int blk = 0; blk * 64 < clen; blk++) {
-                    const uint32_t w0 = flags[2 * blk], w1 = flags[2 * blk + 1];
-                    const uint32_t word = half ? w1 : w0;
-                    const int base = rank_base + (half ? __popc(w0) : 0);
-                    rank_base += __popc(w0) + __popc(w1);
-#pragma unroll
-                    for (int i = 0; i < 2; i++) {
-                        const int bitpos = i * 16 + l16;
-                        const int j = blk * 64 + half * 32 + bitpos;
-                        if (j < clen) {
-                            const int r = base + __popc(word & ((2u << bitpos) - 1u)) - 1;
-                            const float* src = p.sxyz + (delta[r] + cbeg + j);
-                            float* dst = &xs[blk * 64 + bitpos * 2 + half];
-                            cp_async<4>(dst, src);
-                            cp_async<4>(dst + PK, src + p.sxyz_stride);
-                            cp_async<4>(dst + 2 * PK, src + 2 * p.sxyz_stride);
-                        }
-                    }
-                }
-            } else {
             for (int j = lane, sw = 0; j < clen32; j += 32, sw++) {
                 const uint32_t word = flags[sw];
                 const int r = rank_base + __popc(word & le) - 1;
@@ -1110,14 +1313,10 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
                         cp_async<16>(&cand[j], &p.spos[gidx]);
                         cp_async<16>(reinterpret_cast<char*>(&cand[j]) + 16, reinterpret_cast<const char*>(&p.spos[gidx]) + 16);
                     }
-                    if (MODE == MODE_FILL) cp_async<4>(&codes[j], &p.smeta[gidx].y);
+                    cp_async<4>(&codes[j], &p.smeta[gidx].y);
                 }
             }
-            }
-            if constexpr (PACKED) {
-                // x alone keeps a padding slot out of every cutoff (its distance is infinite or not a number)
-                for (int j = clen + lane; j < ((clen + 63) & ~63); j += 32) xs[(j >> 6) * 64 + (j & 31) * 2 + ((j >> 5) & 1)] = 3.0e38f;
-            } else if (clen + lane < clen32) {
+            if (clen + lane < clen32) {
                 Vec4<T> c;
                 c.x = c.y = c.z = (T)3.0e38f;  // never within the cutoff
                 c.w = (T)0;
@@ -1126,87 +1325,6 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
             cp_async_wait_all();
             __syncwarp();
 
-          if constexpr (MODE == MODE_COUNT) {
-            // the targets of both rows of the group as one list, two targets per candidate load
-            const uint32_t n0 = te[0] - tb[0], ntot = n0 + (te[1] - tb[1]);
-            int degree = 0;  // lane l collects the degree of target 32 j + l; stored 32 targets at a time
-            for (uint32_t k = 0; k < ntot; k += 2) {
-                const bool has2 = (k + 1 < ntot);
-                const uint32_t kb = has2 ? k + 1 : k;
-                const uint32_t tA = (k < n0) ? tb[0] + k : tb[1] + (k - n0);
-                const uint32_t tB = (kb < n0) ? tb[0] + kb : tb[1] + (kb - n0);
-                const float4 tpA = p.tscan[tA];  // w = entry
-                const float4 tpB = p.tscan[tB];
-                // lane l keeps, for each of its candidates l, 32 + l, 64 + l, ..., one hit bit per target; the
-                // bits are stored so that the edge-writing pass need not repeat the distance tests.  A list too
-                // long for the bits is only counted.
-                unsigned short* mrowA = p.hitmask + (size_t)tA * 32;
-                unsigned short* mrowB = p.hitmask + (size_t)tB * 32;
-                uint32_t bitsA = 0, bitsB = 0, mayA = 0, mayB = 0, bit = 1u;
-                const unsigned long long ax2 = f32x2_pack(tpA.x, tpA.x), ay2 = f32x2_pack(tpA.y, tpA.y), az2 = f32x2_pack(tpA.z, tpA.z);
-                const unsigned long long bx2 = f32x2_pack(tpB.x, tpB.x), by2 = f32x2_pack(tpB.y, tpB.y), bz2 = f32x2_pack(tpB.z, tpB.z);
-                const unsigned long long* x2 = reinterpret_cast<const unsigned long long*>(xs) + lane;
-                const int nblk = (clen + 63) >> 6;
-#pragma unroll COUNT_UNROLL
-                for (int blk = 0; blk < nblk; blk++) {
-                    const unsigned long long sx2 = x2[blk * 32], sy2 = x2[PK / 2 + blk * 32], sz2 = x2[PK + blk * 32];
-                    float a0, a1, b0, b1;
-                    dist2_x2(ax2, ay2, az2, sx2, sy2, sz2, a0, a1);
-                    dist2_x2(bx2, by2, bz2, sx2, sy2, sz2, b0, b1);
-                    const bool ha0 = (a0 <= upto) && (a0 > near), ha1 = (a1 <= upto) && (a1 > near);
-                    const bool hb0 = (b0 <= upto) && (b0 > near), hb1 = (b1 <= upto) && (b1 > near);
-                    bitsA |= (ha0 ? bit : 0u) | (ha1 ? (bit << 1) : 0u);
-                    bitsB |= (hb0 ? bit : 0u) | (hb1 ? (bit << 1) : 0u);
-                    if constexpr (FLOAT_FIRST) {
-                        mayA |= (!(a0 > beyond) ? bit : 0u) | (!(a1 > beyond) ? (bit << 1) : 0u);
-                        mayB |= (!(b0 > beyond) ? bit : 0u) | (!(b1 > beyond) ? (bit << 1) : 0u);
-                    }
-                    bit <<= 2;
-                }
-                if constexpr (FLOAT_FIRST) {
-                    bitsA |= exact_hits<T>(p, tA, mayA & ~bitsA, equal_is_near, tpA.x, tpA.y, tpA.z, xs, delta, flags, wpre, cbeg, clen, lane, le);
-                    bitsB |= exact_hits<T>(p, tB, mayB & ~bitsB, equal_is_near, tpB.x, tpB.y, tpB.z, xs, delta, flags, wpre, cbeg, clen, lane, le);
-                }
-                if (write_masks) {  // the list is one chunk
-                    mrowA[lane] = (unsigned short)bitsA;
-                    if (has2) mrowB[lane] = (unsigned short)bitsB;
-                }
-                int ca = __reduce_add_sync(0xffffffffu, __popc(bitsA)), cb = __reduce_add_sync(0xffffffffu, __popc(bitsB));
-                if (chunk != 0) {
-                    ca += (int)p.tcount[tA];
-                    if (has2) cb += (int)p.tcount[tB];
-                    __syncwarp();
-                }
-                if constexpr (FLOAT_FIRST) {
-                    // (collecting the degrees here costs registers that the double test needs: 0.6 % slower)
-                    if (lane == 0) {
-                        p.tcount[tA] = (uint32_t)ca;
-                        if (has2) p.tcount[tB] = (uint32_t)cb;
-                        if (!more_chunks && p.counts_out != nullptr) {  // in caller order
-                            p.counts_out[__float_as_int(tpA.w)] = ca;
-                            if (has2) p.counts_out[__float_as_int(tpB.w)] = cb;
-                        }
-                    }
-                    if (!more_chunks) max_degree = max(max_degree, max(ca, has2 ? cb : 0));
-                } else {
-                    // stored 32 at a time: one thread's four stores a pair were 1.3 % of the graph of a 1 M liquid
-                    if (lane == (int)(k & 31u)) degree = ca;
-                    if (lane == (int)(k & 31u) + 1) degree = cb;
-                    if ((k & 31u) == 30u || k + 2 >= ntot) {
-                        const uint32_t mine = (k & ~31u) + (uint32_t)lane;
-                        if (mine < ntot) {
-                            const uint32_t t = (mine < n0) ? tb[0] + mine : tb[1] + (mine - n0);
-                            p.tcount[t] = (uint32_t)degree;
-                            if (!more_chunks) {
-                                if (p.counts_out != nullptr) p.counts_out[__float_as_int(p.tscan[t].w)] = degree;  // in caller order
-                                max_degree = max(max_degree, degree);
-                            }
-                        }
-                        __syncwarp();
-                    }
-                }
-            }
-          } else {
 #pragma unroll
           for (int yr = 0; yr < 2; yr++) {
             const uint32_t t0 = tb[yr], t1 = te[yr];
@@ -1282,24 +1400,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, const PairParams<T>
             }
           }
         }
-          }
-        // a group whose neighbourhood holds no source at all still owes its targets a zero
-        if (MODE == MODE_COUNT && L == 0) {
-            for (int yr = 0; yr < 2; yr++)
-                for (uint32_t t = tb[yr] + lane; t < te[yr]; t += 32) p.tcount[t] = 0;
-        }
     }
-    if (MODE == MODE_COUNT) {  // largest degree: one atomic per CTA
-        __shared__ int s_max_degree;
-        if (threadIdx.x == 0) s_max_degree = 0;
-        __syncthreads();
-        max_degree = __reduce_max_sync(0xffffffffu, max_degree);
-        if (lane == 0 && max_degree > 0) atomicMax(&s_max_degree, max_degree);
-        __syncthreads();
-        if (threadIdx.x == 0 && s_max_degree > 0) atomicMax(&hp->max_degree, (uint32_t)s_max_degree);
-    }
-    // a candidate list too long for the hit bits: the edge writer has to recompute distances
-    if (MODE == MODE_COUNT && lane == 0 && warp_max_slots > RG_MASK_SLOTS) atomicMax(&hp->reserved[0], (long long)warp_max_slots);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1785,7 +1886,7 @@ rg_init_kernel(uint32_t* __restrict__ hdr, const HeaderBlock blk, uint4* __restr
 // host side
 // ------------------------------------------------------------------------------------------
 struct RgLayout {
-    int64_t hdr, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sxyz, smeta, hitmask, trec, tpos, tscan, tmeta,
+    int64_t hdr, posw, aff, ccount, cfill, tccount, tcfill, srec, spos, sscan, smeta, hitmask, trec, tpos, tscan, tmeta,
         tcount, toffset, runs, sums, total;
 };
 
@@ -1814,7 +1915,7 @@ static RgLayout rg_layout(int64_t N, int64_t Nt, int64_t src_cap, int64_t cell_c
     const int64_t slot = dtype == DYNB_F64 ? sizeof(SlotRec<double>) : sizeof(SlotRec<float>);
     L.srec = take(src_cap * slot);  // source images in slot order
     L.spos = take(src_cap * v4);
-    L.sxyz = take(src_cap * 12);  // float x[], y[], z[] of the source records for the count pass
+    L.sscan = dtype == DYNB_F64 ? take(src_cap * 16) : L.spos;  // float positions are tested as they are
     L.smeta = take(src_cap * 8);
     L.hitmask = take(Nt * 32 * 2);
     L.trec = take(Nt * slot);     // targets in slot order
@@ -1938,7 +2039,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     auto* tcfill = reinterpret_cast<uint32_t*>(w + L.tcfill);
     auto* srec = reinterpret_cast<SlotRec<T>*>(w + L.srec);
     auto* spos = reinterpret_cast<Vec4<T>*>(w + L.spos);
-    float* sxyz = reinterpret_cast<float*>(w + L.sxyz);
+    auto* sscan = reinterpret_cast<float4*>(w + L.sscan);
     auto* smeta = reinterpret_cast<uint2*>(w + L.smeta);
     auto* hitmask = reinterpret_cast<unsigned short*>(w + L.hitmask);
     auto* trec = reinterpret_cast<SlotRec<T>*>(w + L.trec);
@@ -2002,7 +2103,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         }
         memcpy(init, &hi, sizeof(hi));
         PairParams<T>& pp = pp_host;
-        pp.h = h; pp.cstart = ccount; pp.tcstart = tccount; pp.spos = spos; pp.sxyz = sxyz; pp.sxyz_stride = src_cap; pp.smeta = smeta; pp.hitmask = hitmask; pp.counts_out = counts_out; pp.tpos = tpos;
+        pp.h = h; pp.cstart = ccount; pp.tcstart = tccount; pp.spos = spos; pp.sscan = sscan; pp.smeta = smeta; pp.hitmask = hitmask; pp.counts_out = counts_out; pp.tpos = tpos;
         pp.tscan = tscan; pp.tmeta = tmeta; pp.tcount = tcount; pp.toffset = toffset; pp.r2 = (T)radius * (T)radius;
         // the targets' fill counters are free once the targets are binned: they hold the list of groups with targets
         pp.glist = (targets != nullptr) ? tcfill : nullptr;
@@ -2047,7 +2148,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         host_grid ? PAIR_CAND_BYTES / (int)sizeof(Vec4<T>) : 0);
     const int64_t nf = std::max(src_cap, Nt);
     rg_bin_finalize_kernel<T><<<(unsigned)((nf + 255) / 256), 256, 0, stream>>>(
-        Nt, targets != nullptr ? 1 : 0, g, posw, h, ccount, tccount, srec, trec, spos, sxyz, src_cap, smeta, tpos, tscan, tmeta, (double)pp_host.r2);
+        Nt, targets != nullptr ? 1 : 0, g, posw, h, ccount, tccount, srec, trec, spos, sscan, smeta, tpos, tscan, tmeta, (double)pp_host.r2);
 
     if (bins_only) {
         DYNB_CUDA_OK(cudaGetLastError());
@@ -2057,12 +2158,10 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     }
     if (targets != nullptr)
         rg_group_list_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, tcfill);
-    const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
-    DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_COUNT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     // there are no more groups than cells, and with a target subset no more of interest than targets
     const int64_t most_groups = std::min(host_grid ? (int64_t)gc_host.ncell_plus1 : cell_cap, targets != nullptr ? Nt : cell_cap);
-    const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * 4 * PAIR_GRID_WAVES, (most_groups + PAIR_WARPS - 1) / PAIR_WARPS);
-    rg_pair_kernel<T, MODE_COUNT, true><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, pp_host, nullptr, nullptr, nullptr, 0, GlueArgs{}, 0, nullptr);
+    const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * COUNT_BLOCKS * COUNT_WAVES, (most_groups + COUNT_WARPS - 1) / COUNT_WARPS);
+    rg_count_kernel<T><<<grid, COUNT_WARPS * 32, 0, stream>>>(pp_host);
     DYNB_CUDA_OK((exclusive_scan<uint32_t, long long>(tcount, toffset, nullptr, Nt + 1, sums64,
                                                        reinterpret_cast<long long*>(&h->E), stream)));
     DYNB_CUDA_OK(cudaGetLastError());
@@ -2105,9 +2204,9 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
     auto* ei64 = reinterpret_cast<long long*>(ei);
     auto* d2 = static_cast<T*>(d2out);
     const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
-    if (long_lists != 0) DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T, MODE_FILL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (long_lists != 0) DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (d2 != nullptr && rg_write_at_once<T>(groups, long_lists)) {
-        rg_pair_kernel<T, MODE_FILL, false><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, PairParams<T>{}, ei64, shifts, d2, (long long)E, glue,
+        rg_pair_kernel<T><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, ei64, shifts, d2, (long long)E, glue,
                                                                                  1, reinterpret_cast<long long*>(total_dev));
         DYNB_CUDA_OK(cudaGetLastError());
         return DYNB_OK;
@@ -2125,7 +2224,7 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
         // Two waves where the caller has not read the header and most likely nothing is listed, else as many as the writer
         // (200 k atoms at 8 A without distances: 508 against 543 us with two)
         const int long_grid = (groups == RG_GROUPS_UNKNOWN && d2 == nullptr) ? std::min(grid, sm_count_cached() * 8) : grid;
-        rg_pair_kernel<T, MODE_FILL, false><<<long_grid, PAIR_THREADS, smem, stream>>>(params_dev, PairParams<T>{}, ei64, shifts, d2,
+        rg_pair_kernel<T><<<long_grid, PAIR_THREADS, smem, stream>>>(params_dev, ei64, shifts, d2,
                                                                                       (long long)E, glue, 0, nullptr);
     }
     DYNB_CUDA_OK(cudaGetLastError());
