@@ -1404,21 +1404,304 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restri
 }
 
 // ------------------------------------------------------------------------------------------
-// Edge writer driven by the hit masks of the counting pass, for the groups whose candidate list is not longer
-// than RG_MASK_SLOTS * 32 records (the usual case: about 27 cells of 8-16 atoms): a warp stages {atom id, shift code}
-// of its group's candidates, reads each target's mask words and writes the edge run.  No distance is tested again.
+// Edge writer driven by the hit bits of the counting pass, for the groups whose candidate list is not longer than
+// RG_MASK_SLOTS * 32 records (the usual case: about 27 cells of 8-16 atoms).  No distance is tested again.
+//
+// The 64 bytes of a target are 512 bits: bit 16 l + s belongs to the candidate at place 32 s + l.  The targets of a cell row
+// follow one another, and so do their edges: the bits of a row that are set, in order, ARE its edges.  A lane takes 64 bits
+// (eight lanes a target, both rows of the group in one go), a prefix sum gives it the place of its first edge, and it puts
+// what belongs to its bits into the warp's buffer; the buffer goes out 32 edges at a time.
+// In most groups all candidates have one shift code, and then all shifts are zero (the targets are candidates too): zeros are
+// written 32 bytes a lane, and a group's edges need the two indices only.
+// Bound by the latency of its loads and by instructions (191 M warp instructions, issue slots 53 % busy), not by the 1.47 GB it
+// writes (4.6 TB/s).  Target by target, with a prefix sum, a list and two rounds of 32 edges for each of them, and three
+// stores with a stride of 12 bytes for the shifts: 240 M.  Before and after: 381 -> 320 us (liquid, 1 M atoms), 742 -> 619 (a
+// rank's 1 M of the 8 M copper atoms, with Cartesian shifts), 189 -> 168 (silicon, double precision), 15 -> 14 (1 k atoms, where
+// every group is at the boundary), 25 -> 27 (32 k atoms).  Bulk copies of a block of zeros for the shifts: no gain.
+// ------------------------------------------------------------------------------------------
+constexpr int FM_TABLE = 33 * (RG_MASK_SLOTS * 32 / 32);   // a word of padding every 32 bits: the lanes of a slot fall into 32 banks
+// Seven blocks of four warps: 72 registers and 164 KB of shared memory, which leaves 92 KB of L1 for the records that
+// neighbouring groups share (liquid, 1 M atoms: 320 us; eight blocks 338, six 336; ten blocks of 48 registers and 28 KB of L1, with an
+// earlier form of the loop, 445 against 368).  Small blocks and eight waves of them even out the SMs (four waves 367, eight 350).
+constexpr int EDGE_WARPS = 4, EDGE_BLOCKS = 7, EDGE_WAVES = 8;
+constexpr int FM_EDGES = 384;                              // edges collected before they are written
+struct EdgeWarp {
+    union {
+        uint2 edge[FM_EDGES];             // plain groups: {atom, atom of the target}
+        struct {
+            uint32_t mixed[FM_EDGES];     // others: table place | lane of the target << 16
+            uint32_t code[FM_TABLE];      //         per bit of a target: shift code of the candidate
+        };
+    };
+    uint32_t table[FM_TABLE];             // per bit of a target: atom of the candidate
+    RunIndex index;
+};
+
+__device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t x)
+{
+    // the shuffle's own predicate says whether there is a lane to add
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+        asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 y;\n\tshfl.sync.up.b32 y|q, %0, %1, 0, 0xffffffff;\n\t@q add.u32 %0, %0, y;\n\t}" : "+r"(x) : "r"(o));
+    return x;
+}
+// The highest set bit s of `bits`, if there is one: table word s goes in front of `at` (bytes of shared memory), which moves back.
+__device__ __forceinline__ void put_edge(uint32_t& bits, uint32_t& at, uint32_t table, uint32_t tag)
+{
+    asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 s, m, a, v;\n\t"
+                 "setp.ne.u32 q, %0, 0;\n\t"
+                 "bfind.u32 s, %0;\n\t"
+                 "shl.b32 m, 1, s;\n\t"
+                 "xor.b32 %0, %0, m;\n\t"
+                 "mad.lo.u32 a, s, 4, %2;\n\t"
+                 "@q ld.shared.u32 v, [a];\n\t"
+                 "@q add.u32 %1, %1, -8;\n\t"
+                 "@q st.shared.v2.u32 [%1], {v, %3};\n\t}"
+                 : "+r"(bits), "+r"(at) : "r"(table), "r"(tag) : "memory");
+}
+// The same with s itself in place of what the table holds.
+__device__ __forceinline__ void put_mixed(uint32_t& bits, uint32_t& at, uint32_t tag)
+{
+    asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 s, m;\n\t"
+                 "setp.ne.u32 q, %0, 0;\n\t"
+                 "bfind.u32 s, %0;\n\t"
+                 "shl.b32 m, 1, s;\n\t"
+                 "xor.b32 %0, %0, m;\n\t"
+                 "add.u32 s, s, %2;\n\t"
+                 "@q add.u32 %1, %1, -4;\n\t"
+                 "@q st.shared.u32 [%1], s;\n\t}"
+                 : "+r"(bits), "+r"(at) : "r"(tag) : "memory");
+}
+// n floats of zero: whole 32-byte sectors, single words at the ends
+__device__ __forceinline__ void zero_floats(float* at, int n, int lane)
+{
+    const int head = min((int)((0u - (uint32_t)(reinterpret_cast<uintptr_t>(at) >> 2)) & 7u), n);
+    const int body = (n - head) & ~7, tail = n - head - body;
+    if (lane < head) at[lane] = 0.0f;
+    at += head;
+#pragma unroll 1
+    for (int i = 8 * lane; i < body; i += 256)
+        asm volatile("st.global.v8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"l"(at + i), "r"(0u) : "memory");
+    if (lane < tail) at[body + lane] = 0.0f;
+}
+
+template <typename T, bool GLUE>
+__global__ void __launch_bounds__(EDGE_WARPS * 32, EDGE_BLOCKS)
+rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restrict__ ei, float* __restrict__ shifts, const long long E,
+                const GlueArgs glue, long long* __restrict__ total)
+{
+    // the plan's pointers are read where they are used, too
+    __shared__ PairParams<T> params;
+    __shared__ GroupShape shape;
+    const DevHeader* hp = params_dev->h;
+    if (hp->status & RG_FATAL) return;
+    for (int i = threadIdx.x; i < (int)(sizeof(PairParams<T>) / 4); i += EDGE_WARPS * 32)
+        reinterpret_cast<uint32_t*>(&params)[i] = reinterpret_cast<const uint32_t*>(params_dev)[i];
+    if (threadIdx.x == 0) shape = group_shape(hp);
+    const uint32_t num_groups = params_dev->glist ? hp->active_groups : (uint32_t)hp->num_groups;
+    __syncthreads();
+    const volatile PairParams<T>& p = params;
+    extern __shared__ __align__(32) unsigned char smem_raw[];
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    EdgeWarp& w = reinterpret_cast<EdgeWarp*>(smem_raw)[warp];
+    const uint32_t lt = lanemask_lt(), le = lt | (1u << lane);
+
+    if (total != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *total = E;
+    const int lane_run = group_lane_run(shape, lane);
+    // Candidates of one shift code: the targets, which are among them, have it too, and every shift of the group is zero.
+    // Left out: mapped ids, and Cartesian shifts of which a zero is a negative zero (a column of the cell that is all negative).
+    bool may_be_plain = true;
+    if constexpr (GLUE) {
+        may_be_plain = glue.id_map == nullptr;
+        if (glue.cart != nullptr) {
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                may_be_plain = may_be_plain && __float_as_uint(__fmaf_rn(0.0f, glue.c[6 + k], __fmaf_rn(0.0f, glue.c[3 + k], __fmul_rn(0.0f, glue.c[k])))) == 0u;
+        }
+    }
+    // this lane's place in the table as a lane of the candidate list, and as the holder of 64 bits
+    uint32_t* const my_table = w.table + 33 * (lane >> 1) + 16 * (lane & 1);
+    const uint32_t my_bits = (uint32_t)__cvta_generic_to_shared(w.table) + 4u * 66u * (uint32_t)(lane & 7);
+    const uint32_t edges_at = (uint32_t)__cvta_generic_to_shared(w.edge);
+
+    // the next group is looked up while the current one is written, so that one round trip to memory per group (the candidate
+    // records) stays exposed
+    auto fetch = [&](uint32_t i) { return fetch_group(shape, p.tcstart, p.cstart, p.glist ? p.glist[i] : i, lane_run); };
+
+    const uint32_t nwarps = gridDim.x * EDGE_WARPS;
+    uint32_t gi = blockIdx.x * EDGE_WARPS + warp;
+    if (gi >= num_groups) return;
+    GroupDesc nd = fetch(gi);
+#pragma unroll 1
+    for (; gi < num_groups; gi += nwarps) {
+        const GroupDesc d = nd;
+        if (gi + nwarps < num_groups) nd = fetch(gi + nwarps);
+        const int n0 = (int)(d.te0 - d.tb0), pieces = 8 * (n0 + (int)(d.te1 - d.tb1));
+        if (pieces == 0) continue;
+        // the first bits and the rows' places in the output do not depend on the candidate records: ask for them now
+        const uint32_t second = d.tb1 - (uint32_t)n0;   // + number of a target of the second row among all
+        auto target = [&](int i) { return (uint32_t)(i >> 3) + ((i >> 3) < n0 ? d.tb0 : second); };
+        uint2 next_bits = make_uint2(0u, 0u);
+        int next_dst = 0;
+        if (lane < pieces) {
+            const uint32_t t = target(lane);
+            next_bits = reinterpret_cast<const uint2*>(p.hitmask + (size_t)t * 32)[lane & 7];
+            next_dst = p.tmeta[t].x;
+        }
+        const long long base0 = p.toffset[d.tb0], base1 = p.toffset[d.tb1];
+        const int edges0 = (int)(p.toffset[d.te0] - base0), edges1 = (int)(p.toffset[d.te1] - base1);
+        int L;
+        const int run_off = warp_excl_scan(d.run_len, lane, &L);
+        const int nslots = (L + 31) >> 5;
+        if (nslots == 0 || nslots > RG_MASK_SLOTS) continue;  // a longer list has no hit bits: rg_pair_kernel writes that group
+
+        __syncwarp();
+        w.index.set(d.run_a, run_off, d.run_len, 0, lane, lt);
+        // four slots at a time: the four gathers are in flight together before the first is stored
+        uint32_t all = 0xffffffffu, any = 0u;
+#pragma unroll 1
+        for (int s0 = 0; s0 < nslots; s0 += 4) {
+            uint2 m[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int j = (s0 + u) * 32 + lane;
+                if (j < L) {
+                    m[u] = p.smeta[w.index.record(s0 + u, le) + j];
+                    all &= m[u].y;
+                    any |= m[u].y;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if ((s0 + u) * 32 + lane < L) my_table[s0 + u] = m[u].x;
+        }
+        const bool plain = may_be_plain && __reduce_and_sync(0xffffffffu, all) == __reduce_or_sync(0xffffffffu, any);
+        if (plain) {
+            zero_floats(shifts + 3 * base0, 3 * edges0, lane);
+            zero_floats(shifts + 3 * base1, 3 * edges1, lane);
+            if (GLUE && glue.cart != nullptr) {
+                zero_floats(glue.cart + 3 * base0, 3 * edges0, lane);
+                zero_floats(glue.cart + 3 * base1, 3 * edges1, lane);
+            }
+        } else {
+            uint32_t* const my_code = w.code + (my_table - w.table);
+#pragma unroll 1
+            for (int s0 = 0; s0 < nslots; s0 += 4) {
+                uint32_t m[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if ((s0 + u) * 32 + lane < L) m[u] = p.smeta[w.index.record(s0 + u, le) + (s0 + u) * 32 + lane].y;
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if ((s0 + u) * 32 + lane < L) my_code[s0 + u] = m[u];
+            }
+        }
+        __syncwarp();
+
+        int written = 0;   // edges of the group in front of this step
+#pragma unroll 1
+        for (int i0 = 0; i0 < pieces; i0 += 32) {
+            uint32_t lo = next_bits.x, hi = next_bits.y;
+            const int dst = next_dst;
+            next_bits = make_uint2(0u, 0u);
+            if (i0 + 32 + lane < pieces) {
+                const uint32_t t = target(i0 + 32 + lane);
+                next_bits = reinterpret_cast<const uint2*>(p.hitmask + (size_t)t * 32)[lane & 7];
+                next_dst = p.tmeta[t].x;
+            }
+            const uint32_t clo = (uint32_t)__popc(lo), chi = (uint32_t)__popc(hi);
+            const uint32_t incl = warp_incl_scan_u32(clo + chi);
+            const int ntot = (int)__shfl_sync(0xffffffffu, incl, 31);
+            int4 tm = make_int4(dst, 0, 0, 0);
+            if (!plain && i0 + lane < pieces) tm = p.tmeta[target(i0 + lane)];
+#pragma unroll 1
+            for (int win = 0; win < ntot; win += FM_EDGES) {
+                if (ntot > FM_EDGES) {
+                    // more than the buffer holds: the part that begins at win
+                    uint32_t at = incl - clo - chi - (uint32_t)win;
+                    auto put = [&](uint32_t place) {
+                        if (at < (uint32_t)FM_EDGES) {
+                            if (plain) w.edge[at] = make_uint2(w.table[place], (uint32_t)dst);
+                            else w.mixed[at] = place | ((uint32_t)lane << 16);
+                        }
+                        at++;
+                    };
+                    for (uint32_t b = lo; b; b &= b - 1) put(66 * (lane & 7) + __ffs((int)b) - 1);
+                    for (uint32_t b = hi; b; b &= b - 1) put(66 * (lane & 7) + 33 + __ffs((int)b) - 1);
+                } else if (plain) {
+                    uint32_t ahi = edges_at + 8u * incl, alo = ahi - 8u * chi;
+                    do {
+                        put_edge(lo, alo, my_bits, (uint32_t)dst);
+                        put_edge(hi, ahi, my_bits + 4u * 33u, (uint32_t)dst);
+                    } while (__any_sync(0xffffffffu, (lo | hi) != 0u));
+                } else {
+                    const uint32_t tag = (uint32_t)(66 * (lane & 7)) | ((uint32_t)lane << 16);
+                    uint32_t ahi = edges_at + 4u * incl, alo = ahi - 4u * chi;
+                    do {
+                        put_mixed(lo, alo, tag);
+                        put_mixed(hi, ahi, tag + 33u);
+                    } while (__any_sync(0xffffffffu, (lo | hi) != 0u));
+                }
+                __syncwarp();
+                const int n = min(FM_EDGES, ntot - win), first = written + win;
+                // edges [0, mid) of the buffer belong to the first row, the others to the second
+                const int mid = max(0, min(n, edges0 - first));
+#pragma unroll 1
+                for (int r = 0; r < 2; r++) {
+                    const int a = r ? mid : 0, b = r ? n : mid;
+                    const long long e0 = (r ? base1 - edges0 : base0) + first;
+                    if (plain) {
+                        long long *src = ei + e0, *to = src + E;
+#pragma unroll 1
+                        for (int i = a + lane; i < b; i += 32) {
+                            const uint2 v = w.edge[i];
+                            src[i] = (long long)v.x;
+                            to[i] = (long long)v.y;
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int i32 = a; i32 < b; i32 += 32) {
+                            const int i = i32 + lane;
+                            const uint32_t v = w.mixed[min(i, b - 1)], id = w.table[v & 0xffffu], code = w.code[v & 0xffffu];
+                            const int from = (int)(v >> 16);
+                            const int td = __shfl_sync(0xffffffffu, tm.x, from), tx = __shfl_sync(0xffffffffu, tm.y, from),
+                                      ty = __shfl_sync(0xffffffffu, tm.z, from), tz = __shfl_sync(0xffffffffu, tm.w, from);
+                            if (i < b) {
+                                const long long e = e0 + i;
+                                const int sx = (int)(code & 1023u) - 512 + tx, sy = (int)((code >> 10) & 1023u) - 512 + ty, sz = (int)((code >> 20) & 1023u) - 512 + tz;
+                                ei[e] = (GLUE && glue.id_map) ? glue.id_map[id] : (long long)id;
+                                ei[E + e] = (GLUE && glue.id_map) ? glue.id_map[td] : (long long)td;
+                                if (GLUE) {
+                                    glue_write(glue, shifts, e, sx, sy, sz);
+                                } else {
+                                    shifts[3 * e + 0] = (float)sx;
+                                    shifts[3 * e + 1] = (float)sy;
+                                    shifts[3 * e + 2] = (float)sz;
+                                }
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            written += ntot;
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// The same with squared distances: a warp stages {record number, shift code} of its group's candidates and reads each target's
+// mask words; the position and the atom id of a hit come from the cell-sorted records (a group's few hundred records stay in
+// L1), and the edges of a target are ordered by candidate place, as rg_pair_kernel writes them: a slot's hits are placed by one
+// ballot.  131 k atoms, 6.9 M edges: 158 us when every pair was tested again by that kernel, 115 us from the hit bits.
 // ------------------------------------------------------------------------------------------
 constexpr int FM_META = RG_MASK_SLOTS * 32;                       // staged candidate records per warp
 constexpr int FM_WARP_BYTES = FM_META * 8 + FM_META * 2 + RUN_INDEX_BYTES;    // records + one parked slot per possible hit
 
-// With DIST the squared distances are written too: the staged record is {record number, shift code}, the position and
-// the atom id of a hit come from the cell-sorted records (a group's few hundred records stay in L1), and the edges of a
-// target are ordered by candidate place, as rg_pair_kernel<FILL> writes them: a slot's hits are placed by one ballot.
-// 131 k atoms, 6.9 M edges: 158 us when every pair was tested again by that kernel, 115 us from the hit bits.
-template <typename T, bool GLUE, bool DIST>
+template <typename T>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
-rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restrict__ ei, float* __restrict__ shifts,
-                   T* __restrict__ d2out, const long long E, const GlueArgs glue, long long* __restrict__ total)
+rg_fillmask_dist_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restrict__ ei, float* __restrict__ shifts,
+                   T* __restrict__ d2out, const long long E, long long* __restrict__ total)
 {
     const PairParams<T> p = *params_dev;
     extern __shared__ __align__(32) unsigned char smem_raw[];
@@ -1510,8 +1793,7 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
                 const uint32_t word = (sw < nslots) ? flags[sw] : 0u;
                 const int r = rank_base + __popc(word & le) - 1;
                 rank_base += __popc(word);
-                if constexpr (DIST) mv[u] = (j < L) ? make_uint2((uint32_t)(delta[r] + j), p.smeta[delta[r] + j].y) : make_uint2(0u, 0u);
-                else mv[u] = (j < L) ? p.smeta[delta[r] + j] : make_uint2(0u, 0u);
+                mv[u] = (j < L) ? make_uint2((uint32_t)(delta[r] + j), p.smeta[delta[r] + j].y) : make_uint2(0u, 0u);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -1522,60 +1804,39 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
         __syncwarp();
 
         // Targets of both rows as one list, one at a time; the words of the next target are requested
-        // before the current one is written.  Lane l holds the hit bits of candidates l, 32 + l, ...:
-        // a warp scan of the bit counts gives every lane the place of its first edge, so the edges of a
-        // target are ordered by (candidate mod 32, candidate / 32).
+        // before the current one is written.  Lane l holds the hit bits of candidates l, 32 + l, ...
         const int n0 = (int)(te[0] - tb[0]), nT = n0 + (int)(te[1] - tb[1]);
         for (int q = 0; q < nT; q++) {
             const int4 tm = ntm;
             const long long base = nbase;
             uint32_t w = nw;
-            Vec4<T> tp{};
-            if constexpr (DIST) tp = p.tpos[q < n0 ? tb[0] + q : tb[1] + (q - n0)];
+            const Vec4<T> tp = p.tpos[q < n0 ? tb[0] + q : tb[1] + (q - n0)];
             if (q + 1 < nT) {
                 const int qa = q + 1;
                 const uint32_t t = qa < n0 ? tb[0] + qa : tb[1] + (qa - n0);
                 ntm = p.tmeta[t]; nbase = p.toffset[t]; nw = p.hitmask[(size_t)t * 32 + lane];
             }
             int cnt = 0;
-            if constexpr (DIST) {
-                __syncwarp();
-                for (int slot = 0; slot < nslots; slot++) {
-                    const bool hit = (w >> slot) & 1u;
-                    const uint32_t m = __ballot_sync(0xffffffffu, hit);
-                    if (hit) list[cnt + __popc(m & lt)] = (unsigned short)(slot * 32 + lane);
-                    cnt += __popc(m);
-                }
-            } else {
-                int pos = warp_excl_scan(__popc(w), lane, &cnt);
-                __syncwarp();
-                while (w) {
-                    const int sbit = __ffs((int)w) - 1;
-                    w &= w - 1;
-                    list[pos++] = (unsigned short)(sbit * 32 + lane);
-                }
+            __syncwarp();
+            for (int slot = 0; slot < nslots; slot++) {
+                const bool hit = (w >> slot) & 1u;
+                const uint32_t m = __ballot_sync(0xffffffffu, hit);
+                if (hit) list[cnt + __popc(m & lt)] = (unsigned short)(slot * 32 + lane);
+                cnt += __popc(m);
             }
             __syncwarp();
             const int sx = tm.y - 512, sy = tm.z - 512, sz = tm.w - 512;
-            const long long dst_id = (GLUE && glue.id_map) ? glue.id_map[tm.x] : (long long)tm.x;
             for (int i = lane; i < cnt; i += 32) {
-                uint2 m = meta[list[i]];
+                const uint2 m = meta[list[i]];
                 const uint32_t code = m.y;
                 const long long e = base + i;
-                if constexpr (DIST) {
-                    const Vec4<T> c = p.spos[m.x];
-                    m.x = (uint32_t)real_to_bits(c.w);
-                    d2out[e] = dist2<T>(tp.x, tp.y, tp.z, c.x, c.y, c.z);
-                }
-                ei[e] = (GLUE && glue.id_map) ? glue.id_map[m.x] : (long long)m.x;
-                ei[E + e] = dst_id;
-                if (GLUE) {
-                    glue_write(glue, shifts, e, (int)(code & 1023u) + sx, (int)((code >> 10) & 1023u) + sy, (int)((code >> 20) & 1023u) + sz);
-                } else {
-                    shifts[3 * e + 0] = (float)((int)(code & 1023u) + sx);
-                    shifts[3 * e + 1] = (float)((int)((code >> 10) & 1023u) + sy);
-                    shifts[3 * e + 2] = (float)((int)((code >> 20) & 1023u) + sz);
-                }
+                const Vec4<T> c = p.spos[m.x];
+                d2out[e] = dist2<T>(tp.x, tp.y, tp.z, c.x, c.y, c.z);
+                ei[e] = (long long)real_to_bits(c.w);
+                ei[E + e] = (long long)tm.x;
+                shifts[3 * e + 0] = (float)((int)(code & 1023u) + sx);
+                shifts[3 * e + 1] = (float)((int)((code >> 10) & 1023u) + sy);
+                shifts[3 * e + 2] = (float)((int)((code >> 20) & 1023u) + sz);
             }
         }
     }
@@ -2200,7 +2461,6 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
     if (glue_opt != nullptr) glue = *glue_opt;
     // The edges come from the hit masks of the counting pass; the groups whose candidate list was too long for the masks
     // (listed on the device by the counting pass; usually none) are written by the distance-recomputing pass behind it.
-    const int fsmem = PAIR_WARPS * FM_WARP_BYTES;
     auto* ei64 = reinterpret_cast<long long*>(ei);
     auto* d2 = static_cast<T*>(d2out);
     const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
@@ -2211,13 +2471,16 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
         DYNB_CUDA_OK(cudaGetLastError());
         return DYNB_OK;
     }
-    auto launch = [&](auto kernel) -> int {
-        DYNB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fsmem));
-        kernel<<<grid, PAIR_THREADS, fsmem, stream>>>(params_dev, ei64, shifts, d2, (long long)E, glue, reinterpret_cast<long long*>(total_dev));
+    auto launch = [&](auto kernel, int blocks, int warps, int bytes, auto... out) -> int {
+        DYNB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        kernel<<<blocks, warps * 32, bytes, stream>>>(params_dev, ei64, shifts, out..., reinterpret_cast<long long*>(total_dev));
         return DYNB_OK;
     };
-    const int rc = d2 != nullptr ? launch(rg_fillmask_kernel<T, false, true>)
-                                 : (glue_opt != nullptr ? launch(rg_fillmask_kernel<T, true, false>) : launch(rg_fillmask_kernel<T, false, false>));
+    const int esmem = EDGE_WARPS * (int)sizeof(EdgeWarp);
+    const int egrid = (int)std::max<int64_t>(std::min<int64_t>((int64_t)sm_count_cached() * EDGE_BLOCKS * EDGE_WAVES, (groups + EDGE_WARPS - 1) / EDGE_WARPS), 1);
+    const int rc = d2 != nullptr ? launch(rg_fillmask_dist_kernel<T>, grid, PAIR_WARPS, PAIR_WARPS * FM_WARP_BYTES, d2, (long long)E)
+                                 : (glue_opt != nullptr ? launch(rg_fillmask_kernel<T, true>, egrid, EDGE_WARPS, esmem, (long long)E, glue)
+                                                        : launch(rg_fillmask_kernel<T, false>, egrid, EDGE_WARPS, esmem, (long long)E, glue));
     if (rc) return rc;
     // the groups the counting pass listed; a caller who has read the plan's header knows whether there are any
     if (long_lists != 0) {
