@@ -37,31 +37,53 @@ struct KdSeg {            // per segment of the current level
     int32_t pad;
 };
 
-// starts[s] = atoms in segments before s (sorted order puts segments in id order); boxes reset
-__global__ void kd_level_init_kernel(int S, const long long* __restrict__ seg_size, long long* __restrict__ seg_start,
-                                     uint32_t* __restrict__ box)
+// Sizes of a segment's children when its cut has m atoms in front.
+__device__ __forceinline__ void kd_child_sizes(const KdSeg& g, long long sz, long long m, long long* __restrict__ next_size)
+{
+    if (g.child_left == g.child_right) {
+        next_size[g.child_left] = sz;
+    } else {
+        next_size[g.child_left] = m;
+        next_size[g.child_right] = sz - m;
+    }
+}
+
+// starts[s] = atoms in segments before s (sorted order puts segments in id order); `reset` boxes emptied.  With thresholds
+// (equal counts) also the cuts: 1 + atoms in front of the cut, in sorted order, and the sizes of the next level's segments.
+__global__ void __launch_bounds__(256)
+kd_level_init_kernel(int S, const KdSeg* __restrict__ seg, const long long* __restrict__ seg_size, long long* __restrict__ seg_start,
+                     uint32_t* __restrict__ box, int reset, long long* __restrict__ next_size, long long* __restrict__ thresholds)
 {
     if (threadIdx.x == 0) {
         long long acc = 0;
         for (int s = 0; s < S; s++) { seg_start[s] = acc; acc += seg_size[s]; }
         seg_start[S] = acc;
     }
-    for (int k = threadIdx.x; k < S * 6; k += blockDim.x) box[k] = ((k % 6) < 3) ? 0xffffffffu : 0u;
+    for (int k = threadIdx.x; k < reset * 6; k += blockDim.x) box[k] = ((k % 6) < 3) ? 0xffffffffu : 0u;
+    if (thresholds == nullptr) return;
+    __syncthreads();
+    for (int s = threadIdx.x; s < S; s += blockDim.x) {
+        const KdSeg g = seg[s];
+        const long long sz = seg_size[s];
+        // kdtree_kernels.cu:110-111, 135-138: a segment that is not cut goes to the left child
+        const long long m = (g.parts <= 1 || sz <= 1) ? sz : min(max(sz / 2, 1ll), sz - 1);
+        thresholds[s] = seg_start[s] + m + 1;
+        kd_child_sizes(g, sz, m, next_size);
+    }
 }
 
 // box[s*6 + 0..2] = min, +3..5 = max of the ordered-integer images of the coordinates
-__global__ void __launch_bounds__(256)
-kd_bbox_kernel(const float* __restrict__ pos, const int32_t* __restrict__ seg_id, int64_t n, int S, uint32_t* __restrict__ box)
-{
-    __shared__ uint32_t sbox[KD_MAX_SEGS_SMEM * 6];
-    const bool in_smem = S <= KD_MAX_SEGS_SMEM;
-    if (in_smem) {
-        for (int k = threadIdx.x; k < S * 6; k += blockDim.x) sbox[k] = ((k % 6) < 3) ? 0xffffffffu : 0u;
+struct KdBoxes {
+    uint32_t sbox[KD_MAX_SEGS_SMEM * 6];
+    __device__ __forceinline__ void begin(int S)
+    {
+        if (S <= KD_MAX_SEGS_SMEM)
+            for (int k = threadIdx.x; k < S * 6; k += blockDim.x) sbox[k] = ((k % 6) < 3) ? 0xffffffffu : 0u;
         __syncthreads();
     }
-    uint32_t* tgt = in_smem ? sbox : box;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int s = seg_id[i];
+    __device__ __forceinline__ void add(const float* __restrict__ pos, int64_t i, int s, int S, uint32_t* __restrict__ box)
+    {
+        uint32_t* tgt = S <= KD_MAX_SEGS_SMEM ? sbox : box;
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             const uint32_t o = ordered_u32(pos[3 * i + d]);
@@ -70,13 +92,25 @@ kd_bbox_kernel(const float* __restrict__ pos, const int32_t* __restrict__ seg_id
             if (o > tgt[s * 6 + 3 + d]) atomicMax(&tgt[s * 6 + 3 + d], o);
         }
     }
-    if (in_smem) {
+    __device__ __forceinline__ void end(int S, uint32_t* __restrict__ box)
+    {
         __syncthreads();
+        if (S > KD_MAX_SEGS_SMEM) return;
         for (int k = threadIdx.x; k < S * 6; k += blockDim.x) {
             if ((k % 6) < 3) { if (sbox[k] != 0xffffffffu) atomicMin(&box[k], sbox[k]); }
             else if (sbox[k] != 0u) atomicMax(&box[k], sbox[k]);
         }
     }
+};
+
+__global__ void __launch_bounds__(256)
+kd_bbox_kernel(const float* __restrict__ pos, const int32_t* __restrict__ seg_id, int64_t n, int S, uint32_t* __restrict__ box)
+{
+    __shared__ KdBoxes boxes;
+    boxes.begin(S);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        boxes.add(pos, i, seg_id[i], S, box);
+    boxes.end(S, box);
 }
 
 // widest axis of the segment (kdtree_kernels.cu:58-70: strict '>' keeps the first axis on ties)
@@ -115,8 +149,7 @@ kd_gather_weights_kernel(const int64_t* __restrict__ w, const uint32_t* __restri
 // exclusive prefix of the sorted weights, excl[n] = total.
 __global__ void __launch_bounds__(256)
 kd_split_kernel(int S, const KdSeg* __restrict__ seg, const long long* __restrict__ seg_size, const long long* __restrict__ seg_start,
-                const long long* __restrict__ excl, long long* __restrict__ mid, long long* __restrict__ next_size,
-                long long* __restrict__ thresholds /* or nullptr: 1 + atoms in front of the cut, in sorted order */)
+                const long long* __restrict__ excl, long long* __restrict__ mid, long long* __restrict__ next_size)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S) return;
@@ -139,13 +172,7 @@ kd_split_kernel(int S, const KdSeg* __restrict__ seg, const long long* __restric
         m = min(max(lo, 1ll), sz - 1);
     }
     mid[s] = m;
-    if (thresholds != nullptr) thresholds[s] = seg_start[s] + m + 1;
-    if (g.child_left == g.child_right) {
-        next_size[g.child_left] = sz;
-    } else {
-        next_size[g.child_left] = m;
-        next_size[g.child_right] = sz - m;
-    }
+    kd_child_sizes(g, sz, m, next_size);
 }
 
 __global__ void __launch_bounds__(256)
@@ -159,20 +186,33 @@ kd_assign_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__
     new_seg_id[vals[q]] = (q - seg_start[s] < mid[s]) ? g.child_left : g.child_right;
 }
 
-// equal counts without a sort: an atom goes right when its (coordinate, index) is not in front of its segment's cut
+// equal counts without a sort: an atom goes right when its (coordinate, index) is not in front of its segment's cut.  The pass
+// also finds the boxes of the next level's S segments (S > 0), or writes the labels (behind the last cut).  Bound by the latency of
+// its two loads (10 us for a million atoms); a launch for each of the two, for the sizes of the cuts and for every level's
+// part of the tree made the call of a million atoms on 8 ranks 305 us instead of 278.
 __global__ void __launch_bounds__(256)
-kd_assign_select_kernel(const uint64_t* __restrict__ keys, int64_t n, int idx_bits, const SelSplit* __restrict__ cut,
-                        const KdSeg* __restrict__ seg, int32_t* __restrict__ new_seg_id)
+kd_assign_select_kernel(const float* __restrict__ pos, const uint64_t* __restrict__ keys, int64_t n, int idx_bits, const SelSplit* __restrict__ cut,
+                        const KdSeg* __restrict__ seg, int32_t* __restrict__ new_seg_id, int S, uint32_t* __restrict__ box,
+                        const int64_t* __restrict__ base_label, int64_t* __restrict__ labels)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint64_t key = keys[i];
-    const int s = (int)(key >> 32);
-    const SelSplit c = cut[s];
-    const u128 C = ((u128)key << idx_bits) | (u128)(uint64_t)i;
-    const bool right = !c.dead && C >= sel_prefix(c);
-    const KdSeg g = seg[s];
-    new_seg_id[i] = right ? g.child_right : g.child_left;
+    __shared__ KdBoxes boxes;
+    if (S > 0) boxes.begin(S);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint64_t key = keys[i];
+        const int s = (int)(key >> 32);
+        const SelSplit c = cut[s];
+        const u128 C = ((u128)key << idx_bits) | (u128)(uint64_t)i;
+        const bool right = !c.dead && C >= sel_prefix(c);
+        const KdSeg g = seg[s];
+        const int child = right ? g.child_right : g.child_left;
+        if (S > 0) {
+            new_seg_id[i] = child;
+            boxes.add(pos, i, child, S, box);
+        } else {
+            labels[i] = base_label[child];
+        }
+    }
+    if (S > 0) boxes.end(S, box);
 }
 
 __global__ void __launch_bounds__(256)
@@ -197,13 +237,13 @@ static KdLayout kd_layout(int64_t n, int64_t W)
     L.sorted_w = take(n * 8);
     L.excl = take((n + 1) * 8);
     L.sums = take((int64_t)(scan_num_tiles(n + 1) + 1) * 8);
-    L.tree = take(W * (int64_t)sizeof(KdSeg));
+    L.tree = take((2 * W + 64) * (int64_t)sizeof(KdSeg));   // all levels
     L.size_a = take((W + 1) * 8);
     L.size_b = take((W + 1) * 8);
     L.start = take((W + 2) * 8);
     L.mid = take((W + 1) * 8);
     L.thr = take((W + 1) * 8);
-    L.box = take(W * 6 * 4);
+    L.box = take(2 * W * 6 * 4);   // of this level's and of the next level's segments
     L.base_label = take((W + 1) * 8);
     L.rs = take(rs_bytes);
     L.sel_state = take(2 * SEL_MAX_SPLITS * (int64_t)sizeof(SelSplit));
@@ -257,50 +297,65 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
     long long* thr = reinterpret_cast<long long*>(ws + L.thr);
     const bool by_selection = (weights_dev == nullptr) && W <= SEL_MAX_SPLITS && method == 0;
     uint32_t* box = reinterpret_cast<uint32_t*>(ws + L.box);
+    uint32_t* box_next = box + W * 6;
     int64_t* base_label = reinterpret_cast<int64_t*>(ws + L.base_label);
     int64_t rs_bytes = 0;
     dynb_radix_sort_workspace_bytes(n, &rs_bytes);
 
-    // the tree of part counts, level by level (kdtree_kernels.cu:215-262)
+    // the tree of part counts, level by level (kdtree_kernels.cu:215-262), and the labels of its leaves
     int levels = 0;
     for (int64_t v = 1; v < W; v <<= 1) levels++;
-    std::vector<int32_t> cur_parts = {(int32_t)W};
-    DYNB_CUDA_OK(cudaMemsetAsync(seg_cur, 0, (size_t)n * 4, s));
+    std::vector<KdSeg> segs;
+    std::vector<int64_t> first(levels + 1, 0);   // of a level's segments
+    std::vector<int32_t> parts = {(int32_t)W};
+    for (int l = 0; l < levels; l++) {
+        first[l] = (int64_t)segs.size();
+        std::vector<int32_t> next;
+        for (const int32_t k : parts) {
+            KdSeg g;
+            g.parts = k;
+            g.pad = 0;
+            g.child_left = g.child_right = (int32_t)next.size();
+            const int32_t lp = k > 1 ? k / 2 : k;
+            next.push_back(lp);
+            if (k > 1) {
+                g.child_right = (int32_t)next.size();
+                next.push_back(k - lp);
+            }
+            segs.push_back(g);
+        }
+        parts.swap(next);
+    }
+    first[levels] = (int64_t)segs.size();
+    std::vector<int64_t> base(parts.size());
+    int64_t label = 0;
+    for (size_t k = 0; k < parts.size(); k++) { base[k] = label; label += parts[k]; }
+    // small pageable sources: staged by cudaMemcpyAsync before it returns
     const long long n_ll = n;
     DYNB_CUDA_OK(cudaMemcpyAsync(size_cur, &n_ll, 8, cudaMemcpyHostToDevice, s));
+    DYNB_CUDA_OK(cudaMemcpyAsync(tree, segs.data(), segs.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, s));
+    DYNB_CUDA_OK(cudaMemcpyAsync(base_label, base.data(), base.size() * 8, cudaMemcpyHostToDevice, s));
+    DYNB_CUDA_OK(cudaMemsetAsync(seg_cur, 0, (size_t)n * 4, s));
     const int grid_stride = (int)std::min<int64_t>(nbk, (int64_t)sm_count_cached() * 8);
     for (int l = 0; l < levels; l++) {
-        const int S = (int)cur_parts.size();
-        std::vector<KdSeg> segs(S);
-        std::vector<int32_t> next_parts;
-        for (int k = 0; k < S; k++) {
-            segs[k].parts = cur_parts[k];
-            segs[k].pad = 0;
-            if (cur_parts[k] <= 1) {
-                segs[k].child_left = segs[k].child_right = (int32_t)next_parts.size();
-                next_parts.push_back(cur_parts[k]);
-            } else {
-                const int32_t lp = cur_parts[k] / 2;
-                segs[k].child_left = (int32_t)next_parts.size();
-                next_parts.push_back(lp);
-                segs[k].child_right = (int32_t)next_parts.size();
-                next_parts.push_back(cur_parts[k] - lp);
-            }
+        const int S = (int)(first[l + 1] - first[l]), S_next = l + 1 < levels ? (int)(first[l + 2] - first[l + 1]) : 0;
+        const KdSeg* level_tree = tree + first[l];
+        if (l == 0 || !by_selection) {
+            kd_level_init_kernel<<<1, 256, 0, s>>>(S, nullptr, size_cur, start, box, S, nullptr, nullptr);
+            kd_bbox_kernel<<<grid_stride, 256, 0, s>>>(pos_dev, seg_cur, n, S, box);
         }
-        // small pageable source: staged by cudaMemcpyAsync before it returns
-        DYNB_CUDA_OK(cudaMemcpyAsync(tree, segs.data(), (size_t)S * sizeof(KdSeg), cudaMemcpyHostToDevice, s));
-        kd_level_init_kernel<<<1, 256, 0, s>>>(S, size_cur, start, box);
-        kd_bbox_kernel<<<grid_stride, 256, 0, s>>>(pos_dev, seg_cur, n, S, box);
         kd_keys_kernel<<<nbk, 256, 0, s>>>(pos_dev, seg_cur, n, box, keys, vals);
         int seg_bits = 0;
         while ((1 << seg_bits) < S) seg_bits++;
         if (by_selection) {
-            kd_split_kernel<<<(S + 255) / 256, 256, 0, s>>>(S, tree, size_cur, start, nullptr, mid, size_next, thr);
+            kd_level_init_kernel<<<1, 256, 0, s>>>(S, level_tree, size_cur, start, box_next, S_next, size_next, thr);
             int idx_bits = 0;
             const SelSplit* cut = nullptr;
             int rc = sel_select_splits(keys, 32 + seg_bits, nullptr, n, S, W, thr, ws + L.sel_state, ws + L.sel_hist, &idx_bits, &cut, true, s);
             if (rc) return rc;
-            kd_assign_select_kernel<<<nbk, 256, 0, s>>>(keys, n, idx_bits, cut, tree, seg_next);
+            kd_assign_select_kernel<<<grid_stride, 256, 0, s>>>(pos_dev, keys, n, idx_bits, cut, level_tree, seg_next, S_next, box_next, base_label,
+                                                                labels_dev);
+            std::swap(box, box_next);
         } else {
             const int end_bit = std::min(64, ((32 + seg_bits + 7) / 8) * 8);
             int rc = dynb_radix_sort_pairs(keys, vals, n, 0, end_bit, ws + L.rs, rs_bytes, s);
@@ -311,18 +366,13 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
                 DYNB_CUDA_OK((exclusive_scan<long long, long long>(reinterpret_cast<long long*>(sorted_w), excl, nullptr, n, sums, excl + n, s)));
                 excl_arg = excl;
             }
-            kd_split_kernel<<<(S + 255) / 256, 256, 0, s>>>(S, tree, size_cur, start, excl_arg, mid, size_next, nullptr);
-            kd_assign_kernel<<<nbk, 256, 0, s>>>(keys, vals, n, tree, start, mid, seg_next);
+            kd_split_kernel<<<(S + 255) / 256, 256, 0, s>>>(S, level_tree, size_cur, start, excl_arg, mid, size_next);
+            kd_assign_kernel<<<nbk, 256, 0, s>>>(keys, vals, n, level_tree, start, mid, seg_next);
         }
         std::swap(seg_cur, seg_next);
         std::swap(size_cur, size_next);
-        cur_parts.swap(next_parts);
     }
-    std::vector<int64_t> base(cur_parts.size());
-    int64_t label = 0;
-    for (size_t k = 0; k < cur_parts.size(); k++) { base[k] = label; label += cur_parts[k]; }
-    DYNB_CUDA_OK(cudaMemcpyAsync(base_label, base.data(), base.size() * 8, cudaMemcpyHostToDevice, s));
-    kd_label_kernel<<<nbk, 256, 0, s>>>(seg_cur, base_label, labels_dev, n);
+    if (!by_selection) kd_label_kernel<<<nbk, 256, 0, s>>>(seg_cur, base_label, labels_dev, n);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }

@@ -14,7 +14,7 @@ struct SelSplit {           // one per split point and level parity
     unsigned long long pre_hi, pre_lo;  // C >> (bits not yet decided)
     long long residual;                 // weight still to cover among the atoms that share the prefix
     int dead;                           // its threshold lies beyond the total weight: no atom reaches it
-    int pad;
+    int atoms;                          // unit weights: atoms that share the prefix (0: not counted)
 };
 
 __device__ __forceinline__ u128 sel_prefix(const SelSplit& s) { return ((u128)s.pre_hi << 64) | (u128)s.pre_lo; }

@@ -369,8 +369,8 @@ __device__ int sel_groups(const SelSplit* __restrict__ st, int nsplit, u128* gli
 }
 
 // A warp finds, among up to 256 counters at p, the first whose inclusive prefix reaches R: returns its
-// index to all lanes (-1 if the sum stays below R), *before = weight in front of it, *total = sum of all.
-__device__ int sel_warp_cross(const unsigned long long* p, int count, long long R, long long* before, long long* total)
+// index to all lanes (-1 if the sum stays below R), *before = weight in front of it, *total = sum of all, *value = its own.
+__device__ int sel_warp_cross(const unsigned long long* p, int count, long long R, long long* before, long long* total, long long* value)
 {
     const int lane = threadIdx.x & 31;
     long long v[8];
@@ -392,14 +392,15 @@ __device__ int sel_warp_cross(const unsigned long long* p, int count, long long 
     const unsigned m = __ballot_sync(0xffffffffu, mine);
     if (m == 0u) return -1;
     int idx = -1;
-    long long bef = 0, c = x - local;
+    long long bef = 0, val = 0, c = x - local;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        if (idx < 0 && c + v[k] >= R) { idx = lane * 8 + k; bef = c; }
+        if (idx < 0 && c + v[k] >= R) { idx = lane * 8 + k; bef = c; val = v[k]; }
         c += v[k];
     }
     const int src = __ffs((int)m) - 1;
     *before = __shfl_sync(0xffffffffu, bef, src);
+    *value = __shfl_sync(0xffffffffu, val, src);
     return __shfl_sync(0xffffffffu, idx, src);
 }
 
@@ -413,7 +414,7 @@ __device__ void sel_pick_warp(int s, const SelSplit* __restrict__ st_in, SelSpli
     SelSplit me;
     int g = 0;
     if (level == 0) {
-        me.pre_hi = me.pre_lo = 0; me.residual = 0; me.dead = 0; me.pad = 0;
+        me.pre_hi = me.pre_lo = 0; me.residual = 0; me.dead = 0; me.atoms = 0;
     } else {
         me = st_in[s];
         g = gid[s];
@@ -427,11 +428,11 @@ __device__ void sel_pick_warp(int s, const SelSplit* __restrict__ st_in, SelSpli
     const int fbits = min(width, 8);
     const int nc = 1 << (width - fbits);  // coarse counters in use (<= 256)
     long long R = me.residual;
-    long long before_c = 0, before_f = 0, total = 0;
+    long long before_c = 0, before_f = 0, total = 0, value = 0;
     int cb;
     if (level == 0) {
         // the total first: thresholds of sfc_kernels.cu:123-134 (equal counts) and :165-170 (weights)
-        sel_warp_cross(coarse, nc, 0x7fffffffffffffffll, &before_c, &total);
+        sel_warp_cross(coarse, nc, 0x7fffffffffffffffll, &before_c, &total, &value);
         const long long p = s + 1;
         long long T;
         if (thresholds != nullptr) {
@@ -451,9 +452,9 @@ __device__ void sel_pick_warp(int s, const SelSplit* __restrict__ st_in, SelSpli
             return;
         }
     }
-    cb = sel_warp_cross(coarse, nc, R, &before_c, &total);
+    cb = sel_warp_cross(coarse, nc, R, &before_c, &total, &value);
     if (cb < 0) return;  // cannot happen: the threshold lies inside this group
-    const int fb = sel_warp_cross(fine + ((size_t)cb << fbits), 1 << fbits, R - before_c, &before_f, &total);
+    const int fb = sel_warp_cross(fine + ((size_t)cb << fbits), 1 << fbits, R - before_c, &before_f, &total, &value);
     if (fb < 0) return;
     if (lane == 0) {
         const unsigned digit = ((unsigned)cb << fbits) | (unsigned)fb;
@@ -461,6 +462,7 @@ __device__ void sel_pick_warp(int s, const SelSplit* __restrict__ st_in, SelSpli
         me.pre_hi = (unsigned long long)(P >> 64);
         me.pre_lo = (unsigned long long)P;
         me.residual = R - before_c - before_f;
+        me.atoms = weighted ? 0 : (int)min(value, 0x7fffffffll);
         st_out[s] = me;
     }
 }
@@ -471,7 +473,8 @@ __device__ void sel_pick_warp(int s, const SelSplit* __restrict__ st_in, SelSpli
 // from that list at once: the split atom of a group is the listed atom with the smallest composite number whose
 // inclusive prefix weight inside the group reaches the split point's residual.  The remaining levels then return
 // at once.  A list that overflows, or a group with more than SEL_FINISH_GROUP_MAX atoms, leaves the level as it
-// was and the next level tries again.
+// was and the next level tries again.  With unit weights the level in front has counted the atoms (SelSplit::atoms): a list that
+// would overflow is not begun (the second pass of a KD-tree level: 20 -> 14 us, a million atoms).
 struct SelCand { unsigned long long hi, lo; long long w; int g; int pad; };
 static_assert(sizeof(SelCand) == sizeof(SelSplit), "candidates share the unused split-point slots");
 constexpr int SEL_FINISH_SPLITS = 16;        // the fused path's limit on split points
@@ -583,7 +586,8 @@ sel_hist_kernel(const uint64_t* __restrict__ keys, const int64_t* __restrict__ w
     __shared__ int gid[SEL_MAX_SPLITS];
     __shared__ unsigned long long s_coarse[256];  // weighted; 64-bit shared additions are compare-and-swap loops
     __shared__ unsigned int s_coarse_unit[256];   // unit weights
-    __shared__ bool s_last;
+    __shared__ bool s_last, s_listed;
+    bool listing = false;   // this level lists its atoms
     // cand != nullptr: the early finish is in use (see above); finished: set by the level that settled the split points
     if (cand != nullptr && __ldcg(finished) != 0u) return;
     // clear the table the next level accumulates into (its last reader, the previous pick, has finished)
@@ -601,58 +605,78 @@ sel_hist_kernel(const uint64_t* __restrict__ keys, const int64_t* __restrict__ w
         __syncthreads();
     } else {
         ng = sel_groups(st, nsplit, glist, gid);
+        if (cand != nullptr && threadIdx.x == 0) {
+            long long atoms = 0;
+            for (int k = 0; k < nsplit; k++)
+                if (gid[k] >= 0 && (k == 0 || gid[k] != gid[k - 1])) atoms += st[k].atoms;
+            s_listed = atoms <= (long long)SEL_CAND_CAP;
+        }
+        __syncthreads();
+        listing = cand != nullptr && s_listed;
     }
     const u128 dmask = ((u128)1 << width) - 1;
     if (ng > 0) {
-        // warp-uniform trip count (all 32 lanes take part in the vote below); lanes past the end carry no counter
-        const int64_t warp_base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
-        for (int64_t base = warp_base; base < n; base += (int64_t)gridDim.x * blockDim.x) {
-            const int64_t i = base + (threadIdx.x & 31);
-            unsigned long long w = 0ull;
-            size_t slot = ~(size_t)0;  // counter of this atom, or none
-            unsigned digit = 0;
-            int lo = 0;
-            u128 C = 0;
-            if (i < n) {
-                C = ((u128)keys[i] << idx_bits) | (u128)(uint64_t)i;
-                const u128 P = C >> (shift + width);
-                int hi = ng;  // first group with prefix >= P
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (glist[mid] < P) lo = mid + 1; else hi = mid;
-                }
-                if (lo < ng && glist[lo] == P) {
-                    w = weights ? (unsigned long long)weights[i] : 1ull;
-                    if (w) {
-                        digit = (unsigned)((C >> shift) & dmask);
-                        slot = ((size_t)lo << dbits) + digit;
+        // warp-uniform trip count (all 32 lanes take part in the vote below); lanes past the end carry no counter.  Four keys of
+        // a lane are in flight together: one by one the half-dozen rounds of a million keys were as many trips to L2.
+        constexpr int U = 4;
+        const int64_t warp_base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31), stride = (int64_t)gridDim.x * blockDim.x;
+        for (int64_t base = warp_base; base < n; base += U * stride) {
+            uint64_t key[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int64_t i = base + u * stride + (threadIdx.x & 31);
+                key[u] = i < n ? keys[i] : 0ull;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int64_t i = base + u * stride + (threadIdx.x & 31);
+                if (base + u * stride >= n) break;
+                unsigned long long w = 0ull;
+                size_t slot = ~(size_t)0;  // counter of this atom, or none
+                unsigned digit = 0;
+                int lo = 0;
+                u128 C = 0;
+                if (i < n) {
+                    C = ((u128)key[u] << idx_bits) | (u128)(uint64_t)i;
+                    const u128 P = C >> (shift + width);
+                    int hi = ng;  // first group with prefix >= P
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (glist[mid] < P) lo = mid + 1; else hi = mid;
+                    }
+                    if (lo < ng && glist[lo] == P) {
+                        w = weights ? (unsigned long long)weights[i] : 1ull;
+                        if (w) {
+                            digit = (unsigned)((C >> shift) & dmask);
+                            slot = ((size_t)lo << dbits) + digit;
+                        }
                     }
                 }
-            }
-            if (cand != nullptr && level > 0) {
-                // the atoms counted at this level, listed for the early finish (one atomic per warp round)
-                const bool listed = (slot != ~(size_t)0);
-                const unsigned lm = __ballot_sync(0xffffffffu, listed);
-                if (lm) {
-                    const int leader = __ffs((int)lm) - 1;
-                    unsigned at = 0;
-                    if ((int)(threadIdx.x & 31) == leader) at = atomicAdd(cand_count, (unsigned)__popc(lm));
-                    at = __shfl_sync(0xffffffffu, at, leader) + (unsigned)__popc(lm & lanemask_lt());
-                    if (listed && at < (unsigned)SEL_CAND_CAP) {
-                        SelCand c;
-                        c.hi = (unsigned long long)(C >> 64); c.lo = (unsigned long long)C; c.w = (long long)w; c.g = lo; c.pad = 0;
-                        cand[at] = c;
+                if (listing) {
+                    // the atoms counted at this level, listed for the early finish (one atomic per warp round)
+                    const bool listed = (slot != ~(size_t)0);
+                    const unsigned lm = __ballot_sync(0xffffffffu, listed);
+                    if (lm) {
+                        const int leader = __ffs((int)lm) - 1;
+                        unsigned at = 0;
+                        if ((int)(threadIdx.x & 31) == leader) at = atomicAdd(cand_count, (unsigned)__popc(lm));
+                        at = __shfl_sync(0xffffffffu, at, leader) + (unsigned)__popc(lm & lanemask_lt());
+                        if (listed && at < (unsigned)SEL_CAND_CAP) {
+                            SelCand c;
+                            c.hi = (unsigned long long)(C >> 64); c.lo = (unsigned long long)C; c.w = (long long)w; c.g = lo; c.pad = 0;
+                            cand[at] = c;
+                        }
                     }
                 }
-            }
-            if (w) {
-                if (fine_private) {
-                    atomicAdd(&s_fine[digit], 1u);
-                } else {
-                    atomicAdd(&hist[slot], w);
-                    if (level > 0) atomicAdd(&coarse[((size_t)lo << 8) + (digit >> fbits)], w);
-                    else if (weights) atomicAdd(&s_coarse[digit >> fbits], w);
-                    else atomicAdd(&s_coarse_unit[digit >> fbits], 1u);
+                if (w) {
+                    if (fine_private) {
+                        atomicAdd(&s_fine[digit], 1u);
+                    } else {
+                        atomicAdd(&hist[slot], w);
+                        if (level > 0) atomicAdd(&coarse[((size_t)lo << 8) + (digit >> fbits)], w);
+                        else if (weights) atomicAdd(&s_coarse[digit >> fbits], w);
+                        else atomicAdd(&s_coarse_unit[digit >> fbits], 1u);
+                    }
                 }
             }
         }
