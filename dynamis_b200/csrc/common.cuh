@@ -73,6 +73,18 @@ int fail_cuda(cudaError_t e, const char* what);
 int fail_arg(const char* what);
 void set_last_error(const char* msg);
 
+// Where the device can write to `host` (16-byte aligned pinned memory), or nullptr.
+static inline void* device_view_of_host(void* host)
+{
+    if (reinterpret_cast<uintptr_t>(host) % 16 != 0) return nullptr;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
+
 static inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 static inline int sm_count_cached()
 {

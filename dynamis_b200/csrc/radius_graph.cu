@@ -724,8 +724,10 @@ rg_bin_finalize_kernel(int64_t Nt, int subset, Geom<T> g, const Vec4<T>* __restr
                        const SlotRec<T>* __restrict__ srec, const SlotRec<T>* __restrict__ trec,
                        Vec4<T>* __restrict__ spos, float4* __restrict__ sscan,
                        uint2* __restrict__ smeta, Vec4<T>* __restrict__ tpos, float4* __restrict__ tscan,
-                       int4* __restrict__ tmeta, double r2)
+                       int4* __restrict__ tmeta, double r2, uint4* header_host)
 {
+    // a plan that ends here: its header is complete
+    if (header_host != nullptr && blockIdx.x == 0 && threadIdx.x == 0) publish_64_bytes(reinterpret_cast<const uint4*>(hp), header_host);
     if (hp->status & RG_FATAL) return;
     if (sizeof(T) == 8 && blockIdx.x == 0 && threadIdx.x == 0)
         float_test(r2, 1.01 * (double)max(hp->nx, max(hp->ny, hp->nz)) / hp->res_inv + 0.02, hp->test_near, hp->test_lo, hp->test_hi,
@@ -2313,6 +2315,11 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     auto* sums64 = reinterpret_cast<long long*>(w + L.sums);
     auto* params_dev = reinterpret_cast<PairParams<T>*>(w + L.hdr + RG_PARAMS_OFFSET);
 
+    // The last kernel of the plan writes the header to the host itself where the caller's copy lies in pinned memory (a copy
+    // behind it is a launch of another engine: 8 to 10 us of a call with a thousand atoms).
+    static_assert(sizeof(dynb_rg_header) == 64, "the header is published in four pieces of 16 bytes");
+    uint4* header_written = nullptr;
+    if (header_host != nullptr && (bins_only || scan_publishes(Nt + 1))) header_written = static_cast<uint4*>(device_view_of_host(header_host));
     static_assert(sizeof(DevHeader) <= RG_PARAMS_OFFSET, "header overlaps params");
     static_assert(RG_PARAMS_OFFSET + sizeof(PairParams<T>) <= RG_HEADER_BYTES, "params overflow header block");
     unsigned char init[RG_HEADER_BYTES];
@@ -2409,11 +2416,11 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         host_grid ? PAIR_CAND_BYTES / (int)sizeof(Vec4<T>) : 0);
     const int64_t nf = std::max(src_cap, Nt);
     rg_bin_finalize_kernel<T><<<(unsigned)((nf + 255) / 256), 256, 0, stream>>>(
-        Nt, targets != nullptr ? 1 : 0, g, posw, h, ccount, tccount, srec, trec, spos, sscan, smeta, tpos, tscan, tmeta, (double)pp_host.r2);
+        Nt, targets != nullptr ? 1 : 0, g, posw, h, ccount, tccount, srec, trec, spos, sscan, smeta, tpos, tscan, tmeta, (double)pp_host.r2, bins_only ? header_written : nullptr);
 
     if (bins_only) {
         DYNB_CUDA_OK(cudaGetLastError());
-        if (header_host != nullptr)
+        if (header_host != nullptr && header_written == nullptr)
             DYNB_CUDA_OK(cudaMemcpyAsync(header_host, h, sizeof(dynb_rg_header), cudaMemcpyDeviceToHost, stream));
         return DYNB_OK;
     }
@@ -2424,9 +2431,10 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * COUNT_BLOCKS * COUNT_WAVES, (most_groups + COUNT_WARPS - 1) / COUNT_WARPS);
     rg_count_kernel<T><<<grid, COUNT_WARPS * 32, 0, stream>>>(pp_host);
     DYNB_CUDA_OK((exclusive_scan<uint32_t, long long>(tcount, toffset, nullptr, Nt + 1, sums64,
-                                                       reinterpret_cast<long long*>(&h->E), stream)));
+                                                       reinterpret_cast<long long*>(&h->E), stream,
+                                                       ScanPublish{reinterpret_cast<const uint4*>(h), header_written})));
     DYNB_CUDA_OK(cudaGetLastError());
-    if (header_host != nullptr)
+    if (header_host != nullptr && header_written == nullptr)
         DYNB_CUDA_OK(cudaMemcpyAsync(header_host, h, sizeof(dynb_rg_header), cudaMemcpyDeviceToHost, stream));
     return DYNB_OK;
 }

@@ -196,9 +196,21 @@ scan_apply_pair_kernel(const TIn* in0, TOut* out0, const TIn* in1, TOut* out1, c
                                blockIdx.y ? copy1 : copy0);
 }
 
+// 64 bytes that the thread which writes the grand total copies behind it (dst == nullptr: none): a header that holds the total,
+// to host memory.
+struct ScanPublish { const uint4* src; uint4* dst; };
+__device__ __forceinline__ void publish_64_bytes(const uint4* src, uint4* dst)
+{
+    uint4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = __ldcg(src + k);
+#pragma unroll
+    for (int k = 0; k < 4; k++) dst[k] = v[k];
+}
+
 // sum of sums[0 .. blockIdx.x) by the whole block (and, from the last block, the grand total)
 template <typename TOut>
-__device__ __forceinline__ TOut scan_prefix_of_sums(const TOut* __restrict__ sums, int num_tiles, TOut* __restrict__ total_out)
+__device__ __forceinline__ TOut scan_prefix_of_sums(const TOut* __restrict__ sums, int num_tiles, TOut* total_out, const ScanPublish& publish = {})
 {
     __shared__ TOut part[SCAN_THREADS / 32];
     __shared__ TOut result;
@@ -214,7 +226,13 @@ __device__ __forceinline__ TOut scan_prefix_of_sums(const TOut* __restrict__ sum
 #pragma unroll
         for (int w = 0; w < SCAN_THREADS / 32; w++) t += part[w];
         result = t;
-        if (total_out != nullptr && mine == num_tiles - 1) *total_out = t + sums[mine];
+        if (total_out != nullptr && mine == num_tiles - 1) {
+            *total_out = t + sums[mine];
+            if (publish.dst != nullptr) {
+                __threadfence();
+                publish_64_bytes(publish.src, publish.dst);
+            }
+        }
     }
     __syncthreads();
     return result;
@@ -223,13 +241,13 @@ __device__ __forceinline__ TOut scan_prefix_of_sums(const TOut* __restrict__ sum
 template <typename TIn, typename TOut>
 __device__ __forceinline__ void scan_apply_fused_body(const TIn* in, const uint32_t* __restrict__ n_dev, int64_t n_host,
                                                       const TOut* __restrict__ sums, int num_tiles, TOut* out, TOut* total_out,
-                                                      TOut* out_copy = nullptr)
+                                                      TOut* out_copy = nullptr, const ScanPublish& publish = {})
 {
     __shared__ TOut warp_sums[SCAN_THREADS / 32];
     const int64_t n = scan_count(n_dev, n_host);
     // a tile past the (device-side) end has nothing to write; only the last block still adds up all sums for the total
     if ((int64_t)blockIdx.x * SCAN_TILE >= n && (int)blockIdx.x != num_tiles - 1) return;
-    const TOut before = scan_prefix_of_sums<TOut>(sums, num_tiles, total_out);
+    const TOut before = scan_prefix_of_sums<TOut>(sums, num_tiles, total_out, publish);
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
     TOut v[SCAN_ITEMS];
     scan_load_items<TIn, TOut>(in, base, n, v);
@@ -245,9 +263,9 @@ __device__ __forceinline__ void scan_apply_fused_body(const TIn* in, const uint3
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_apply_fused_kernel(const TIn* in, const uint32_t* __restrict__ n_dev, int64_t n_host, const TOut* __restrict__ sums,
-                        TOut* out, TOut* total_out)
+                        TOut* out, TOut* total_out, const ScanPublish publish)
 {
-    scan_apply_fused_body<TIn, TOut>(in, n_dev, n_host, sums, gridDim.x, out, total_out);
+    scan_apply_fused_body<TIn, TOut>(in, n_dev, n_host, sums, gridDim.x, out, total_out, nullptr, publish);
 }
 
 template <typename TIn, typename TOut>
@@ -264,11 +282,14 @@ constexpr int SCAN_FUSED_MAX_TILES = 8192;  // above this the per-block summing 
 
 static inline int scan_num_tiles(int64_t n_host) { return (int)((n_host + SCAN_TILE - 1) / SCAN_TILE); }
 
-// `sums` must hold scan_num_tiles(n_host) elements of TOut.  `total_out` (device, may be null)
-// receives the sum of all elements.
+// Whether exclusive_scan honours `publish` for this many elements.
+static inline bool scan_publishes(int64_t n_host) { return n_host > 0 && scan_num_tiles(n_host) <= SCAN_FUSED_MAX_TILES; }
+
+// `sums` must hold scan_num_tiles(n_host) elements of TOut.  `total_out` (device, or host memory that the device can write; may
+// be null) receives the sum of all elements.
 template <typename TIn, typename TOut>
 static inline cudaError_t exclusive_scan(const TIn* in, TOut* out, const uint32_t* n_dev, int64_t n_host,
-                                         TOut* sums, TOut* total_out, cudaStream_t stream)
+                                         TOut* sums, TOut* total_out, cudaStream_t stream, ScanPublish publish = {})
 {
     if (n_host <= 0) {
         if (total_out) return cudaMemsetAsync(total_out, 0, sizeof(TOut), stream);
@@ -277,7 +298,7 @@ static inline cudaError_t exclusive_scan(const TIn* in, TOut* out, const uint32_
     const int tiles = scan_num_tiles(n_host);
     scan_tile_sums_kernel<TIn, TOut><<<tiles, SCAN_THREADS, 0, stream>>>(in, n_dev, n_host, sums);
     if (tiles <= SCAN_FUSED_MAX_TILES) {
-        scan_apply_fused_kernel<TIn, TOut><<<tiles, SCAN_THREADS, 0, stream>>>(in, n_dev, n_host, sums, out, total_out);
+        scan_apply_fused_kernel<TIn, TOut><<<tiles, SCAN_THREADS, 0, stream>>>(in, n_dev, n_host, sums, out, total_out, publish);
     } else {
         scan_sums_kernel<TOut><<<1, SCAN_THREADS, 0, stream>>>(sums, tiles, total_out);
         scan_apply_kernel<TIn, TOut><<<tiles, SCAN_THREADS, 0, stream>>>(in, n_dev, n_host, sums, out);

@@ -49,7 +49,7 @@ int dynb_version(void);
  *
  * Two phases, because the number of edges is only known after counting:
  *   dynb_rg_plan   wrap -> periodic images -> cell binning -> per-target degrees -> offsets;
- *                  copies a dynb_rg_header into header_host asynchronously.
+ *                  writes a dynb_rg_header into header_host asynchronously (pinned memory: by its last kernel).
  *   (caller synchronises the stream, reads header.E, allocates the outputs)
  *   dynb_rg_fill   writes edge_index [2,E] int64 and cell_shifts [E,3] float32.
  * The workspace carries the plan between the two calls and must not be touched in between.
