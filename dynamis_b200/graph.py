@@ -22,6 +22,7 @@ import torch
 from . import _lib
 
 _STATE: dict = {}
+HOST_WORDS = 64
 
 
 def _dev_state(device: torch.device) -> dict:
@@ -31,8 +32,10 @@ def _dev_state(device: torch.device) -> dict:
     key = (index, _lib.stream_of(device))
     st = _STATE.get(key)
     if st is None:
-        pinned = torch.empty(64, dtype=torch.uint8).pin_memory()
-        st = {"ws": None, "hdr_t": pinned, "hdr": _lib.RgHeader.from_address(pinned.data_ptr()), "geo": {}}
+        # pinned: the plan's header, and words for the counts of other calls; every call waits for what it has written there
+        pinned = torch.empty(64 + 8 * HOST_WORDS, dtype=torch.uint8).pin_memory()
+        st = {"ws": None, "hdr_t": pinned, "hdr": _lib.RgHeader.from_address(pinned.data_ptr()), "geo": {}, "bytes": {},
+              "words": pinned[64:].view(torch.int64)}
         _STATE[key] = st
     return st
 
@@ -82,6 +85,26 @@ def _empty_result(pos, n_target):
     )
 
 
+def host_words(device: torch.device, count: int) -> torch.Tensor:
+    """Pinned int64 words of the current stream of ``device``, for counts that a kernel writes or a copy brings and the caller
+    waits for before it returns; a buffer of its own for more than ``HOST_WORDS``."""
+    if count > HOST_WORDS:
+        return torch.empty((count,), dtype=torch.int64, pin_memory=True)
+    return _dev_state(device)["words"][:count]
+
+
+def _plan_bytes(st: dict, n_atoms: int, n_targets: int, src_cap: int, cell_cap: int, dtype_code: int) -> int:
+    key = (n_atoms, n_targets, src_cap, cell_cap, dtype_code)
+    nbytes = st["bytes"].get(key)
+    if nbytes is None:
+        out = ctypes.c_int64()
+        _lib.check(_lib.lib().dynb_rg_workspace_bytes(n_atoms, n_targets, src_cap, cell_cap, dtype_code, ctypes.byref(out)), "rg_workspace_bytes")
+        if len(st["bytes"]) > 64:
+            st["bytes"].clear()
+        nbytes = st["bytes"][key] = out.value
+    return nbytes
+
+
 class RadiusGraphPlan:
     """Result of the counting phase: degrees are known, the edge buffers are not written yet.
 
@@ -90,7 +113,7 @@ class RadiusGraphPlan:
     """
 
     __slots__ = ("ws", "dtype_code", "E", "M", "counts", "device", "pos_dtype", "max_degree", "grid", "num_groups", "walked",
-                 "long_lists")
+                 "long_lists", "total")
 
     def fill(self, want_dist_sq: bool = False, total: Optional[torch.Tensor] = None):
         """(edge_index, shifts, squared distances or None); ``total`` (one int64 on the device) receives E."""
@@ -139,7 +162,7 @@ class RadiusGraphPlan:
 def _geometry(st: dict, cell_np, pbc_np, radius: float, N: int, dtype_code: int):
     """Host-side conversions and capacities of a geometry, kept by value of (cell, pbc, radius, sizes):
     (key, (cell, pbc, radius, source capacity, cell capacity))."""
-    key = (cell_np.tobytes(), str(cell_np.dtype), pbc_np.tobytes(), float(radius), N, dtype_code)
+    key = (cell_np.tobytes(), cell_np.dtype.num, pbc_np.tobytes(), pbc_np.dtype.num, float(radius), N, dtype_code)
     geo = st["geo"].get(key)
     if geo is None:
         np_real = np.float64 if dtype_code == _lib.DYNB_F64 else np.float32
@@ -177,8 +200,7 @@ class BinnedAtoms:
         self.pos = pos.contiguous()
         self.dtype_code = _lib.DYNB_F64 if pos.dtype == torch.float64 else _lib.DYNB_F32
         self.st = _dev_state(pos.device)
-        self.hdr_t = torch.empty((64,), dtype=torch.uint8, pin_memory=True)
-        self.hdr = _lib.RgHeader.from_address(self.hdr_t.data_ptr())
+        self.hdr_t, self.hdr = self.st["hdr_t"], self.st["hdr"]
         self.key, geo = _geometry(self.st, cell.detach().to("cpu").numpy(), pbc.detach().to("cpu").numpy(), radius, pos.size(0),
                                   self.dtype_code)
         self.cell_h, self.pbc_h, self.radius, self.src_capacity, self.cell_capacity = geo
@@ -187,10 +209,7 @@ class BinnedAtoms:
 
     def launch(self) -> None:
         L, N, dev = _lib.lib(), self.pos.size(0), self.pos.device
-        nbytes = ctypes.c_int64()
-        _lib.check(L.dynb_rg_workspace_bytes(N, N, self.src_capacity, self.cell_capacity, self.dtype_code, ctypes.byref(nbytes)),
-                   "rg_workspace_bytes")
-        self.ws = _workspace(self.st, nbytes.value, dev)
+        self.ws = _workspace(self.st, _plan_bytes(self.st, N, N, self.src_capacity, self.cell_capacity, self.dtype_code), dev)
         self.attempts += 1
         _lib.check(L.dynb_rg_bin(self.pos.data_ptr(), self.dtype_code, N, self.cell_h.ctypes.data, self.pbc_h.ctypes.data, self.radius,
                                  self.ws.data_ptr(), self.ws.numel(), self.src_capacity, self.cell_capacity, self.hdr_t.data_ptr(),
@@ -206,9 +225,10 @@ class BinnedAtoms:
         return True
 
 
-def plan_radius_graph(pos, cell, pbc, radius, target_indices=None) -> RadiusGraphPlan:
+def plan_radius_graph(pos, cell, pbc, radius, target_indices=None, want_total: bool = False) -> RadiusGraphPlan:
     """Counting phase (wrap, periodic images, cell binning, degrees, offsets).  Synchronises the
-    current stream once to learn the number of edges.  ``pos`` must be non-empty."""
+    current stream once to learn the number of edges.  ``pos`` must be non-empty.  What does not depend on that number
+    (``want_total``: the word on the device that is to receive it) is made before the wait."""
     pos = pos.contiguous()
     N = pos.size(0)
     if target_indices is not None:
@@ -226,18 +246,23 @@ def plan_radius_graph(pos, cell, pbc, radius, target_indices=None) -> RadiusGrap
         st = _dev_state(dev)
         geo_key, (cell_h, pbc_h, radius, src_cap, cell_cap) = _geometry(st, cell_np, pbc_np, radius, N, dtype_code)
         counts = torch.empty((Nt,), dtype=torch.int32, device=dev)
-        stream = torch.cuda.current_stream(dev)
+        stream = _lib.stream_of(dev)
         hdr = st["hdr"]
+        plan = None
         for attempt in range(3):
-            nbytes = ctypes.c_int64()
-            _lib.check(L.dynb_rg_workspace_bytes(N, Nt, src_cap, cell_cap, dtype_code, ctypes.byref(nbytes)),
-                       "rg_workspace_bytes")
-            ws = _workspace(st, nbytes.value, dev)
+            ws = _workspace(st, _plan_bytes(st, N, Nt, src_cap, cell_cap, dtype_code), dev)
             _lib.check(L.dynb_rg_plan(pos.data_ptr(), dtype_code, N, cell_h.ctypes.data, pbc_h.ctypes.data, radius,
                                       target_indices.data_ptr() if target_indices is not None else None, Nt,
                                       ws.data_ptr(), ws.numel(), src_cap, cell_cap, counts.data_ptr(),
-                                      st["hdr_t"].data_ptr(), stream.cuda_stream), "rg_plan")
-            stream.synchronize()
+                                      st["hdr_t"].data_ptr(), stream), "rg_plan")
+            if plan is None:
+                plan = RadiusGraphPlan()
+                plan.dtype_code = dtype_code
+                plan.counts = counts
+                plan.device = dev
+                plan.pos_dtype = pos.dtype
+                plan.total = torch.empty((1,), dtype=torch.int64, device=dev) if want_total else None
+            torch.cuda.current_stream(dev).synchronize()
             status = int(hdr.status)
             if status & _lib.RG_SRC_OVERFLOW and attempt < 2:
                 src_cap = max(int(hdr.M) + 1024, 2 * src_cap)
@@ -245,19 +270,14 @@ def plan_radius_graph(pos, cell, pbc, radius, target_indices=None) -> RadiusGrap
                 continue
             break
     _raise_status(status)
-    plan = RadiusGraphPlan()
     plan.ws = ws
-    plan.dtype_code = dtype_code
     plan.E = int(hdr.E)
     plan.M = int(hdr.M)
     plan.max_degree = int(hdr.max_degree)
-    plan.grid = (int(hdr.grid[0]), int(hdr.grid[1]), int(hdr.grid[2]))
+    plan.grid = tuple(hdr.grid)
     plan.num_groups = int(hdr.num_groups)
     plan.walked = plan.num_groups if target_indices is None else min(plan.num_groups, Nt)  # groups the writer looks at
     plan.long_lists = int(hdr.reserved[1])
-    plan.counts = counts
-    plan.device = dev
-    plan.pos_dtype = pos.dtype
     return plan
 
 
@@ -269,7 +289,7 @@ def _graph_impl(pos, cell, pbc, radius, target_indices, counts_only, want_dist_s
     if N == 0 or Nt == 0:  # reference: radius_graph_kernels.cu:499-509
         out = _empty_result(pos, Nt)
         return out + ((torch.empty(0, dtype=pos.dtype, device=pos.device),) if want_dist_sq else ())
-    plan = plan_radius_graph(pos, cell, pbc, radius, target_indices)
+    plan = plan_radius_graph(pos, cell, pbc, radius, target_indices, want_total=not counts_only)
     dev = pos.device
     if counts_only or plan.E == 0:  # reference: :802-811, :828-840
         out = (
@@ -279,9 +299,8 @@ def _graph_impl(pos, cell, pbc, radius, target_indices, counts_only, want_dist_s
             plan.counts,
         )
         return out + ((torch.empty(0, dtype=pos.dtype, device=dev),) if want_dist_sq else ())
-    nni = torch.empty((1,), dtype=torch.int64, device=dev)
-    edge_index, shifts, d2 = plan.fill(want_dist_sq, nni)
-    out = (edge_index, shifts, nni, plan.counts)
+    edge_index, shifts, d2 = plan.fill(want_dist_sq, plan.total)
+    out = (edge_index, shifts, plan.total, plan.counts)
     return out + ((d2,) if want_dist_sq else ())
 
 

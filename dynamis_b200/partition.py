@@ -22,11 +22,12 @@ import numpy as np
 import torch
 
 from . import _lib
-from .graph import BinnedAtoms, radius_graph_pbc, radius_graph_pbc_ex
+from .graph import BinnedAtoms, host_words, radius_graph_pbc, radius_graph_pbc_ex
 from .state import DistEnvironment, MolecularInfo, PartitionMessagePassingInfo, SimulationConfig
 
 PARTITION_MAX_NUM_NEIGHBORS = 1000
 HALO_MAX_NUM_NEIGHBORS = 1000
+SELECT_HOST_COUNT = 8192 * 2048   # SELECT_FUSED_MAX_TILES tiles of SELECT_TILE values (csrc/halo.cu)
 
 _SCRATCH: dict = {}
 
@@ -137,13 +138,19 @@ def select_eq(values: torch.Tensor, value: int, gather_src: Optional[torch.Tenso
     L = _lib.lib()
     with _lib.on_device(dev):
         out = torch.empty((n,), dtype=torch.int64, device=dev)
-        cnt = torch.empty((1,), dtype=torch.int64, device=dev)
+        # a count that is waited for is written to the host by the kernel (up to 16.7 M values: its tiles then need no prefix sum)
+        waited = count is None and 0 < n <= SELECT_HOST_COUNT
+        cnt = host_words(dev, 1) if waited else torch.empty((1,), dtype=torch.int64, device=dev)
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_select_workspace_bytes(n, ctypes.byref(nbytes)), "select_workspace_bytes")
         ws = scratch(dev, "select", nbytes.value)
         _lib.check(L.dynb_select_eq_i64(values.data_ptr(), n, int(value), gather_src.data_ptr() if gather_src is not None else None,
                                         out.data_ptr(), cnt.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev)), "select_eq")
-        k = int(cnt.item()) if count is None else count
+        if waited:
+            torch.cuda.current_stream(dev).synchronize()
+            k = int(cnt[0])
+        else:
+            k = int(cnt.item()) if count is None else count
     return out[:k]
 
 
@@ -160,7 +167,7 @@ def _finish_partition(labels: torch.Tensor, state: MolecularInfo, env: DistEnvir
     vn = vn.to(device=dev, dtype=torch.int64).contiguous() if vn is not None else None
     info.partition_indices = select_eq(labels, R, vn, n_local)
     m = torch.zeros((W, W), dtype=torch.int64, device=dev)
-    m[R, R] = info.partition_indices.numel()
+    m[R, R].fill_(info.partition_indices.numel())   # (an assignment copies the number from pageable memory)
     info.global_send_recv_matrix = m
     return info
 
@@ -195,7 +202,7 @@ class AbstractPartitioner:
             ws = scratch(dev, "halo_lists", nbytes.value)
             # send offsets, recv offsets, number of own atoms and, behind them, the error word of the marking
             offs = torch.empty((2 * (W + 1) + 2,), dtype=torch.int64, device=dev)
-            offs_h = torch.empty((2 * (W + 1) + 2,), dtype=torch.int64, pin_memory=True)
+            offs_h = host_words(dev, 2 * (W + 1) + 2)
             # everything up to the list sizes is queued before the one wait; the header's status is looked at behind it
             bins = BinnedAtoms(pos32, cell, pbc, ghost_cutoff) if N > 0 else None
             while True:
