@@ -855,6 +855,14 @@ __device__ __forceinline__ int lane_id()
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));  // volatile: kept in a register instead of read again
     return l;
 }
+__device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t x)
+{
+    // the shuffle's own predicate says whether there is a lane to add
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+        asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 y;\n\tshfl.sync.up.b32 y|q, %0, %1, 0, 0xffffffff;\n\t@q add.u32 %0, %0, y;\n\t}" : "+r"(x) : "r"(o));
+    return x;
+}
 // What a warp keeps to find the record behind a place of its candidate list (one chunk of up to 512 places).
 struct RunIndex {
     int delta[32];                  // per non-empty run: record = delta + place
@@ -866,9 +874,8 @@ struct RunIndex {
         runs_compact(delta, run_a, run_off, run_len, lt);
         const int before = runs_flags(flags, run_off, run_len, lane, cbeg);
         const uint32_t f = lane < RUN_FLAG_WORDS ? flags[lane] : 0u;
-        int starts;
-        const int rank = before + warp_excl_scan(__popc(f), lane, &starts);
-        if (lane < RUN_FLAG_WORDS) word[lane] = make_uint2(f, (uint32_t)(rank - 1));
+        const uint32_t own = (uint32_t)__popc(f), rank = (uint32_t)before + warp_incl_scan_u32(own) - own;
+        if (lane < RUN_FLAG_WORDS) word[lane] = make_uint2(f, rank - 1u);
         __syncwarp();
     }
     // record - place, for place 32 s + lane of the chunk
@@ -905,11 +912,21 @@ __device__ __forceinline__ void glue_write(const GlueArgs& g, float* __restrict_
 // The grid and the shape of the groups, and one group: its targets (one contiguous run a cell row, at most two rows) and this
 // lane's run of source records.  Both cell-scan kernels keep the grid in shared memory and read it where a group is looked
 // up: in registers it left too few for the loops.
-struct GroupShape { int nx, ny, nz, sx, sy, pad, gx, gy; };
-struct GroupDesc { uint32_t tb0, te0, tb1, te1; int run_a, run_len; };
+struct GroupShape { int nx, ny, nz, sx, sy, pad, gx, gy; uint32_t by_gx, by_gy; };
+struct GroupDesc { uint32_t tb0, te0, tb1, te1; int run_a, run_e; };   // as loaded: nothing waits for the loads until the group's turn
 __device__ __forceinline__ GroupShape group_shape(const DevHeader* hp)
 {
-    return {hp->nx, hp->ny, hp->nz, hp->group_cells, hp->group_cells_y, hp->pad, hp->gx, (hp->ny + hp->group_cells_y - 1) / hp->group_cells_y};
+    const int gx = hp->gx, gy = (hp->ny + hp->group_cells_y - 1) / hp->group_cells_y;
+    return {hp->nx, hp->ny, hp->nz, hp->group_cells, hp->group_cells_y, hp->pad, gx, gy, 0xffffffffu / (uint32_t)gx, 0xffffffffu / (uint32_t)gy};
+}
+// v / d and the remainder, from by_d = floor((2^32 - 1) / d) >= 2^32 / d - 1: v by_d / 2^32 lies above v / d - 1, so the upper half
+// of the product is the quotient or one less.  (The compiler's division is three times as many instructions.)
+__device__ __forceinline__ uint32_t group_divide(uint32_t v, uint32_t d, uint32_t by_d, uint32_t& rest)
+{
+    uint32_t q = __umulhi(v, by_d);
+    rest = v - q * d;
+    if (rest >= d) { rest -= d; q++; }
+    return q;
 }
 // lane r owns run r: (z row, y row) of it, counted from the lowest; -1: no run
 __device__ __forceinline__ int group_lane_run(const GroupShape& g, int lane)
@@ -922,8 +939,9 @@ __device__ __forceinline__ GroupDesc fetch_group(const volatile GroupShape& g, c
     GroupDesc d;
     const int nx = g.nx, ny = g.ny, pad = g.pad, sx = g.sx, sy = g.sy;
     const uint32_t gx = (uint32_t)g.gx, gy = (uint32_t)g.gy;
-    const uint32_t row = grp / gx;
-    const int cz = (int)(row / gy), cx0 = (int)(grp - row * gx) * sx, cy0 = (int)(row - (uint32_t)cz * gy) * sy;
+    uint32_t ix, iy;
+    const uint32_t row = group_divide(grp, gx, g.by_gx, ix);
+    const int cz = (int)group_divide(row, gy, g.by_gy, iy), cx0 = (int)ix * sx, cy0 = (int)iy * sy;
     const int cx1 = min(cx0 + sx, nx) - 1, cy1 = min(cy0 + sy, ny) - 1;
     const uint32_t* tcell = tcstart + ((uint32_t)cz * ny + cy0) * nx;
     d.tb0 = tcell[cx0];
@@ -933,15 +951,13 @@ __device__ __forceinline__ GroupDesc fetch_group(const volatile GroupShape& g, c
         d.tb1 = tcell[nx + cx0];
         d.te1 = tcell[nx + cx1 + 1];
     }
-    d.run_a = 0;
-    d.run_len = 0;
+    d.run_a = d.run_e = 0;
     if (lane_run >= 0) {
         const int yy = cy0 - pad + (lane_run & 255), zz = cz - pad + (lane_run >> 8);
         if (yy >= 0 && yy < ny && yy <= cy1 + pad && zz >= 0 && zz < g.nz) {
             const uint32_t* cell = cstart + ((uint32_t)zz * ny + yy) * nx;
-            const uint32_t a = cell[max(cx0 - pad, 0)], e = cell[min(cx1 + pad, nx - 1) + 1];
-            d.run_a = (int)a;
-            d.run_len = (int)(e - a);
+            d.run_a = (int)cell[max(cx0 - pad, 0)];
+            d.run_e = (int)cell[min(cx1 + pad, nx - 1) + 1];
         }
     }
     return d;
@@ -1019,8 +1035,8 @@ rg_group_list_kernel(const PairParams<T>* __restrict__ params_dev, uint32_t* __r
 // memory and is unrolled over the whole list.  (Before: candidates in shared memory, two targets at a time; three of its
 // loads, the shifting of the bit and eight compares with selects for every 64 candidates and two targets.)
 // Bound by the FMA pipe and the issue of instructions (issue slots 64 % busy, 190 M warp instructions for a million atoms of the
-// liquid against 245 M; a packed instruction holds the FMA pipe for two cycles).  Before and after: 300 -> 270 us (liquid, 1 M
-// atoms, 5 A), 357 -> 313 (a rank's 1 M of the 8 M copper atoms), 226 -> 172 (silicon in double precision, 500 k atoms, 6 A).
+// liquid against 245 M; a packed instruction holds the FMA pipe for two cycles).  Before and after: 300 -> 262 us (liquid, 1 M
+// atoms, 5 A), 357 -> 302 (a rank's 1 M of the 8 M copper atoms), 226 -> 171 (silicon in double precision, 500 k atoms, 6 A).
 // ------------------------------------------------------------------------------------------
 // Seven blocks of four warps: 72 registers.  80 registers and six blocks 276 us, 96 and five 281, 128 and four 293 (liquid).
 // Blocks of two warps, and half or twice the waves: within 2 %.
@@ -1172,15 +1188,14 @@ rg_count_kernel(const PairParams<T> p)
     for (uint32_t gi = blockIdx.x * COUNT_WARPS + warp; gi < num_groups; gi += nwarps) {
         const uint32_t grp = p.glist ? p.glist[gi] : gi;
         const GroupDesc d = fetch_group(shape, p.tcstart, p.cstart, grp, lane_run);
-        const int run_a = d.run_a, run_len = d.run_len;
+        const int run_a = d.run_a, run_len = d.run_e - d.run_a;
         CountGroup g;
         g.tb0 = d.tb0;
         g.tb1 = d.tb1;
         g.n0 = d.te0 - d.tb0;
         g.ntot = g.n0 + (d.te1 - d.tb1);
         if (g.ntot == 0) continue;
-        int L;
-        const int run_off = warp_excl_scan(run_len, lane, &L);
+        const int run_end = (int)warp_incl_scan_u32((uint32_t)run_len), run_off = run_end - run_len, L = __shfl_sync(0xffffffffu, run_end, 31);
         const int nslots = (L + 31) >> 5;
         g.write_masks = nslots <= RG_MASK_SLOTS;
         warp_max_slots = max(warp_max_slots, nslots);
@@ -1416,10 +1431,12 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restri
 // In most groups all candidates have one shift code, and then all shifts are zero (the targets are candidates too): zeros are
 // written 32 bytes a lane, and a group's edges need the two indices only.
 // Bound by the latency of its loads and by instructions (191 M warp instructions, issue slots 53 % busy), not by the 1.47 GB it
-// writes (4.6 TB/s).  Target by target, with a prefix sum, a list and two rounds of 32 edges for each of them, and three
-// stores with a stride of 12 bytes for the shifts: 240 M.  Before and after: 381 -> 320 us (liquid, 1 M atoms), 742 -> 619 (a
-// rank's 1 M of the 8 M copper atoms, with Cartesian shifts), 189 -> 168 (silicon, double precision), 15 -> 14 (1 k atoms, where
-// every group is at the boundary), 25 -> 27 (32 k atoms).  Bulk copies of a block of zeros for the shifts: no gain.
+// writes (4.8 TB/s).  Target by target, with a prefix sum, a list and two rounds of 32 edges for each of them, and three
+// stores with a stride of 12 bytes for the shifts: 240 M.  Before and after: 381 -> 308 us (liquid, 1 M atoms), 742 -> 611 (a
+// rank's 1 M of the 8 M copper atoms, with Cartesian shifts), 189 -> 160 (silicon, double precision), 15 -> 13 (1 k atoms, where
+// every group is at the boundary), 25 -> 25 (32 k atoms).  What is loaded ahead is not touched until its turn: a subtraction
+// behind the loads of the next group's runs or of the rows' places in the output waits for them (322 -> 308 us).
+// Bulk copies of a block of zeros for the shifts: no gain.
 // ------------------------------------------------------------------------------------------
 constexpr int FM_TABLE = 33 * (RG_MASK_SLOTS * 32 / 32);   // a word of padding every 32 bits: the lanes of a slot fall into 32 banks
 // Seven blocks of four warps: 72 registers and 164 KB of shared memory, which leaves 92 KB of L1 for the records that
@@ -1439,14 +1456,6 @@ struct EdgeWarp {
     RunIndex index;
 };
 
-__device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t x)
-{
-    // the shuffle's own predicate says whether there is a lane to add
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
-        asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 y;\n\tshfl.sync.up.b32 y|q, %0, %1, 0, 0xffffffff;\n\t@q add.u32 %0, %0, y;\n\t}" : "+r"(x) : "r"(o));
-    return x;
-}
 // The highest set bit s of `bits`, if there is one: table word s goes in front of `at` (bytes of shared memory), which moves back.
 __device__ __forceinline__ void put_edge(uint32_t& bits, uint32_t& at, uint32_t table, uint32_t tag)
 {
@@ -1550,15 +1559,13 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
             next_bits = reinterpret_cast<const uint2*>(p.hitmask + (size_t)t * 32)[lane & 7];
             next_dst = p.tmeta[t].x;
         }
-        const long long base0 = p.toffset[d.tb0], base1 = p.toffset[d.tb1];
-        const int edges0 = (int)(p.toffset[d.te0] - base0), edges1 = (int)(p.toffset[d.te1] - base1);
-        int L;
-        const int run_off = warp_excl_scan(d.run_len, lane, &L);
+        const long long base0 = p.toffset[d.tb0], base1 = p.toffset[d.tb1], end0 = p.toffset[d.te0], end1 = p.toffset[d.te1];
+        const int run_len = d.run_e - d.run_a, run_end = (int)warp_incl_scan_u32((uint32_t)run_len), run_off = run_end - run_len, L = __shfl_sync(0xffffffffu, run_end, 31);
         const int nslots = (L + 31) >> 5;
         if (nslots == 0 || nslots > RG_MASK_SLOTS) continue;  // a longer list has no hit bits: rg_pair_kernel writes that group
 
         __syncwarp();
-        w.index.set(d.run_a, run_off, d.run_len, 0, lane, lt);
+        w.index.set(d.run_a, run_off, run_len, 0, lane, lt);
         // four slots at a time: the four gathers are in flight together before the first is stored
         uint32_t all = 0xffffffffu, any = 0u;
 #pragma unroll 1
@@ -1578,6 +1585,7 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
                 if ((s0 + u) * 32 + lane < L) my_table[s0 + u] = m[u].x;
         }
         const bool plain = may_be_plain && __reduce_and_sync(0xffffffffu, all) == __reduce_or_sync(0xffffffffu, any);
+        const int edges0 = (int)(end0 - base0), edges1 = (int)(end1 - base1);
         if (plain) {
             zero_floats(shifts + 3 * base0, 3 * edges0, lane);
             zero_floats(shifts + 3 * base1, 3 * edges1, lane);
