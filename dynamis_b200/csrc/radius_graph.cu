@@ -68,6 +68,7 @@ struct DevHeader {
     double clip_lo[3];  // source images outside [clip_lo, clip_hi] cannot reach any target and are dropped
     double clip_hi[3];
     uint32_t active_groups;  // entries of the list of groups that hold targets (target subsets only)
+    uint32_t halo_groups;    // halo marking: entries of halo_list
     float test_near, test_lo, test_hi;  // double positions: thresholds of the float test (float_test)
     uint32_t test_equal_is_near;
 };
@@ -984,6 +985,7 @@ template <typename T> struct PairParams {
     unsigned short* sown;     // [M]; lies over the binning slots, which nothing reads behind the plan
     unsigned short* town;     // [n_targets]; likewise
     unsigned short* run_owner;  // [gx * ny * nz]
+    uint32_t* halo_list;        // [n_targets] groups that can hold an edge of interest (h->halo_groups entries); behind sown
     T r2;
 };
 // The plan stores its PairParams inside the workspace (after the header) so that the fill call
@@ -1860,11 +1862,11 @@ rg_fillmask_dist_kernel(const PairParams<T>* __restrict__ params_dev, long long*
 //
 // What matters is what is not tested: most of the volume lies inside one subdomain.  The owners of the cell-sorted records
 // and targets are gathered once, and every candidate run (one per group column and (y, z) row) gets a word that says whether
-// all its records have one owner; from these words, one per lane, a warp drops the groups that cannot hold an edge of
-// interest (at 1 M atoms, 8 ranks: nine of ten).  The others list the candidates that can matter to one of their targets and
+// all its records have one owner; from these words the groups that can hold an edge of interest are listed (at 1 M
+// atoms, 8 ranks: one of ten).  A warp lists a group's candidates that can matter to one of their targets and
 // test distances for these alone — lane = candidate, targets broadcast from shared memory, one hit bit per target in a
-// register of the lane, one atomic per candidate and group.  A million atoms, 8 ranks, 6 A, one rank's edges: 17 + 9 + 130 us
-// (owners, runs, marking) for 59 M warp instructions; the same with one list of owners per group and no words took 338 us,
+// register of the lane, one atomic per candidate and group.  A million atoms, 8 ranks, 6 A, one rank's edges:
+// 17 + 6 + 14 + 79 us (owners, runs, list, marking); without the list of groups 126 us for the last two, the same with one list of owners per group and no words took 338 us,
 // and the pass that tested every pair for every rank 1034 us.
 // ------------------------------------------------------------------------------------------
 // Word of a candidate run: the one owner of its records, or EMPTY or MIXED; HALO_RANK is set when a record belongs to the rank
@@ -1886,7 +1888,10 @@ __global__ void __launch_bounds__(256)
 rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo)
 {
     const PairParams<T> p = *params_dev;
-    if (halo.bad != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *halo.bad = 0u;  // for the marking behind this launch
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // for the marking behind this launch
+        if (halo.bad != nullptr) *halo.bad = 0u;
+        p.h->halo_groups = 0u;
+    }
     if (p.h->status & RG_FATAL) return;
     const int64_t M = (int64_t)p.h->M;
     const int64_t end = max(M, (int64_t)p.n_targets);  // the plan's targets, whatever the number of owners
@@ -1930,6 +1935,54 @@ rg_halo_runs_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs
             }
         }
         p.run_owner[i] = (unsigned short)(o | (found ? HALO_RANK : 0));
+    }
+}
+
+// The groups that the marking has to look at, as a list: those whose runs have several owners (the targets' own records are among
+// them), with a record of the rank of interest, and with targets.  They lie together along the subdomains' boundary, one in ten
+// of all: spread over the warps by their numbers some warps had several and most had none.  A lane takes a group; the words
+// of its runs lie beside those of the lanes next to it.  A million atoms, 8 ranks, 6 A: marking 126 -> 14 (this pass, bound by the
+// latency of its loads) + 79 us; with a warp a group here 31 us.
+template <typename T>
+__global__ void __launch_bounds__(128)
+rg_halo_list_kernel(const PairParams<T>* __restrict__ params_dev)
+{
+    const PairParams<T> p = *params_dev;
+    DevHeader* hp = p.h;
+    if (hp->status & RG_FATAL) return;
+    const int nx = hp->nx, ny = hp->ny, nz = hp->nz, S = hp->group_cells, Sy = hp->group_cells_y, pad = hp->pad;
+    const uint32_t gx = (uint32_t)hp->gx, gy = (uint32_t)((ny + Sy - 1) / Sy), num_groups = (uint32_t)hp->num_groups;
+    for (uint32_t g0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; g0 < num_groups; g0 += gridDim.x * blockDim.x) {
+        const uint32_t grp = g0 + (threadIdx.x & 31);
+        bool wanted = false;
+        if (grp < num_groups) {
+            const uint32_t row = grp / gx;
+            const int ix = (int)(grp - row * gx);
+            const int cz = (int)(row / gy), iy = (int)(row - (uint32_t)cz * gy);
+            const int cy0 = iy * Sy, cy1 = min(cy0 + Sy, ny) - 1;
+            int lo = HALO_EMPTY, hi = 0;
+            bool rank = false;
+            for (int zz = max(cz - pad, 0); zz <= min(cz + pad, nz - 1); zz++) {
+                const unsigned short* word = p.run_owner + ((uint32_t)zz * ny) * gx + ix;
+#pragma unroll 6
+                for (int yy = max(cy0 - pad, 0); yy <= min(cy1 + pad, ny - 1); yy++) {
+                    const int w = (int)word[(uint32_t)yy * gx], o = w & 0x7fff;
+                    rank = rank || (w & HALO_RANK);
+                    lo = min(lo, o);
+                    hi = max(hi, o == HALO_EMPTY ? 0 : o);
+                }
+            }
+            if (rank && (lo != hi || lo == HALO_MIXED)) {
+                const int cx0 = ix * S, cx1 = min(cx0 + S, nx) - 1;
+                const uint32_t* tcell = p.tcstart + ((uint32_t)cz * ny + cy0) * nx;
+                wanted = tcell[cx0] != tcell[cx1 + 1] || (cy1 > cy0 && tcell[nx + cx0] != tcell[nx + cx1 + 1]);
+            }
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, wanted);
+        uint32_t base = 0;
+        if ((threadIdx.x & 31) == 0 && m) base = atomicAdd(&hp->halo_groups, (uint32_t)__popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (wanted) p.halo_list[base + __popc(m & lanemask_lt())] = grp;
     }
 }
 
@@ -2034,7 +2087,7 @@ rg_halo_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo
     const DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
     const int nx = hp->nx, ny = hp->ny, nz = hp->nz, S = hp->group_cells, Sy = hp->group_cells_y, pad = hp->pad;
-    const uint32_t gx = (uint32_t)hp->gx, gy = (uint32_t)((ny + Sy - 1) / Sy), num_groups = (uint32_t)hp->num_groups;
+    const uint32_t gx = (uint32_t)hp->gx, gy = (uint32_t)((ny + Sy - 1) / Sy), num_groups = hp->halo_groups;
     const int Wd = 2 * pad + 1, Wy = Sy + 2 * pad, nrun = Wy * Wd;
     const int lane_dy = (lane % Wy) - pad, lane_dz = (lane / Wy) - pad;
     const uint32_t lt = lanemask_lt();
@@ -2042,22 +2095,15 @@ rg_halo_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo
     const float reach0 = sqrtf((float)p.r2) * 1.002f;
 
     const uint32_t nwarps = gridDim.x * PAIR_WARPS;
-    for (uint32_t grp = blockIdx.x * PAIR_WARPS + warp; grp < num_groups; grp += nwarps) {
+    for (uint32_t gi = blockIdx.x * PAIR_WARPS + warp; gi < num_groups; gi += nwarps) {
+        const uint32_t grp = p.halo_list[gi];
         const uint32_t row = grp / gx;
         const int ix = (int)(grp - row * gx);
         const int cz = (int)(row / gy), iy = (int)(row - (uint32_t)cz * gy);
         const int cy0 = iy * Sy, cy1 = min(cy0 + Sy, ny) - 1;
         const int yy = cy0 + lane_dy, zz = cz + lane_dz;
         const bool has_run = lane < nrun && yy >= 0 && yy < ny && yy <= cy1 + pad && zz >= 0 && zz < nz;
-        int run_word;
-        {   // nothing to do when all records around the group (its targets' own records among them) have one owner, or
-            // when none of them belongs to the rank of interest
-            const int word = has_run ? (int)p.run_owner[((uint32_t)zz * ny + yy) * gx + ix] : HALO_EMPTY, o = word & 0x7fff;
-            if (!__any_sync(0xffffffffu, word & HALO_RANK)) continue;
-            const int lo = __reduce_min_sync(0xffffffffu, o), hi = __reduce_max_sync(0xffffffffu, o == HALO_EMPTY ? 0 : o);
-            if (lo == hi && lo != HALO_MIXED) continue;
-            run_word = o;
-        }
+        const int run_word = has_run ? (int)p.run_owner[((uint32_t)zz * ny + yy) * gx + ix] & 0x7fff : HALO_EMPTY;
         const int cx0 = ix * S, cx1 = min(cx0 + S, nx) - 1;
         const uint32_t tb0 = p.tcstart[((uint32_t)cz * ny + cy0) * nx + cx0], te0 = p.tcstart[((uint32_t)cz * ny + cy0) * nx + cx1 + 1];
         uint32_t tb1 = 0, te1 = 0;
@@ -2389,6 +2435,9 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         pp.sown = reinterpret_cast<unsigned short*>(srec);
         pp.town = reinterpret_cast<unsigned short*>(trec);
         pp.run_owner = reinterpret_cast<unsigned short*>(w + L.runs);
+        // a listed group holds targets: no more groups than targets, and no more of those than source records
+        static_assert(sizeof(SlotRec<T>) >= sizeof(unsigned short) + sizeof(uint32_t), "the list lies behind the owners over the binning slots");
+        pp.halo_list = reinterpret_cast<uint32_t*>(srec) + (src_cap + 1) / 2;
         memcpy(init + RG_PARAMS_OFFSET, &pp, sizeof(pp));
     }
     {
@@ -2520,6 +2569,7 @@ static int rg_halo_mark(const void* ws, const HaloArgs& ha, int64_t N, cudaStrea
     rg_halo_owner_kernel<T><<<(unsigned)((2 * N + 255) / 256), 256, 0, stream>>>(params_dev, ha);
     rg_halo_runs_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, ha);
     const int grid = sm_count_cached() * 4 * PAIR_GRID_WAVES;
+    rg_halo_list_kernel<T><<<sm_count_cached() * 8, 128, 0, stream>>>(params_dev);
     if (ha.words == 1) rg_halo_kernel<T, false><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
     else rg_halo_kernel<T, true><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
     DYNB_CUDA_OK(cudaGetLastError());
