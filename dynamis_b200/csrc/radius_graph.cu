@@ -815,6 +815,7 @@ constexpr int PAIR_LIST = 128;         // parked hits per target (uint16 each, t
 // all drain their share at the same speed, and a static one-wave split left the slowest SM 20-30 %
 // behind the average; with several short waves the block scheduler evens that out.
 constexpr int PAIR_GRID_WAVES = 8;
+constexpr int PAIR_SHARE = 8;          // warps that share a listed group's targets when few groups are listed
 constexpr int RUN_FLAG_WORDS = 16;     // run-start bitmap of one staged chunk (up to 512 records)
 constexpr int RUN_INDEX_BYTES = 32 * 4 + RUN_FLAG_WORDS * 4;
 constexpr int PAIR_WARP_BYTES = PAIR_CAND_BYTES + PAIR_CODE_BYTES + PAIR_LIST * 4 + RUN_INDEX_BYTES;
@@ -1278,7 +1279,11 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restri
     const uint32_t lt = lanemask_lt();
 
     const uint32_t nwarps = gridDim.x * PAIR_WARPS;
-    for (uint32_t gi = blockIdx.x * PAIR_WARPS + warp; gi < num_groups; gi += nwarps) {
+    // A few listed groups leave the chip idle but for the chain of one warp each: then eight warps share a group's targets (graph
+    // calls of a liquid at 6 A, where one list in some hundred is long: 8 k atoms 166 -> 117 us, 20 k 179 -> 129, 60 k 160 -> 153).
+    const uint32_t parts = long_only && num_groups * (uint32_t)PAIR_SHARE <= nwarps ? (uint32_t)PAIR_SHARE : 1u;
+    for (uint32_t item = blockIdx.x * PAIR_WARPS + warp; item < num_groups * parts; item += nwarps) {
+        const uint32_t gi = item / parts, part = item - gi * parts;
         const uint32_t grp = long_only ? p.long_list[gi] : (p.glist ? p.glist[gi] : gi);
         const uint32_t row = grp / gx;
         const int ix = (int)(grp - row * gx);
@@ -1348,7 +1353,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restri
           for (int yr = 0; yr < 2; yr++) {
             const uint32_t t0 = tb[yr], t1 = te[yr];
             // two targets share every candidate load
-            for (uint32_t t = t0; t < t1; t += 2) {
+            for (uint32_t t = t0 + 2 * part; t < t1; t += 2 * parts) {
                 const bool has2 = (t + 1 < t1);
                 const Vec4<T> tpA = p.tpos[t];
                 const Vec4<T> tpB = p.tpos[has2 ? t + 1 : t];
@@ -1441,11 +1446,11 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restri
 // Bulk copies of a block of zeros for the shifts: no gain.
 // ------------------------------------------------------------------------------------------
 constexpr int FM_TABLE = 33 * (RG_MASK_SLOTS * 32 / 32);   // a word of padding every 32 bits: the lanes of a slot fall into 32 banks
-// Seven blocks of four warps: 72 registers and 164 KB of shared memory, which leaves 92 KB of L1 for the records that
-// neighbouring groups share (liquid, 1 M atoms: 320 us; eight blocks 338, six 336; ten blocks of 48 registers and 28 KB of L1, with an
-// earlier form of the loop, 445 against 368).  Small blocks and eight waves of them even out the SMs (four waves 367, eight 350).
+// Seven blocks of four warps: 72 registers, and 177 of the 228 KB of shared memory, which leaves L1 for the records that neighbouring
+// groups share (liquid, 1 M atoms: 320 us; eight blocks 338, six 336; ten blocks of 48 registers and hardly any L1, with an earlier
+// form of the loop, 445 against 368).  Small blocks and eight waves of them even out the SMs (four waves 367, eight 350).
 constexpr int EDGE_WARPS = 4, EDGE_BLOCKS = 7, EDGE_WAVES = 8;
-constexpr int FM_EDGES = 384;                              // edges collected before they are written
+constexpr int FM_EDGES = 384;                              // edges collected before they are written (512: 315 us against 306)
 struct EdgeWarp {
     union {
         uint2 edge[FM_EDGES];             // plain groups: {atom, atom of the target}
@@ -1565,6 +1570,9 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
         const int run_len = d.run_e - d.run_a, run_end = (int)warp_incl_scan_u32((uint32_t)run_len), run_off = run_end - run_len, L = __shfl_sync(0xffffffffu, run_end, 31);
         const int nslots = (L + 31) >> 5;
         if (nslots == 0 || nslots > RG_MASK_SLOTS) continue;  // a longer list has no hit bits: rg_pair_kernel writes that group
+        // one or two targets are often without neighbours (a gas of a million atoms, 0.001 per A^3: 433 us without this line, 357
+        // with it, 399 target by target); more of them hardly ever are, and the test waits for the bits
+        if (pieces <= 16 && !__any_sync(0xffffffffu, (next_bits.x | next_bits.y) != 0u)) continue;
 
         __syncwarp();
         w.index.set(d.run_a, run_off, run_len, 0, lane, lt);
@@ -1626,10 +1634,32 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
             const int ntot = (int)__shfl_sync(0xffffffffu, incl, 31);
             int4 tm = make_int4(dst, 0, 0, 0);
             if (!plain && i0 + lane < pieces) tm = p.tmeta[target(i0 + lane)];
+            // In one go, or two targets and two targets, or (targets with more neighbours than that) piece by piece.  Piece by
+            // piece in place of two and two: 1043 us against 1021 a graph call (liquid of 1 M atoms, 6 A: 90 neighbours).
+            const int half = (int)__shfl_sync(0xffffffffu, incl, 15);
+            const bool whole = ntot <= FM_EDGES, halves = !whole && max(half, ntot - half) <= FM_EDGES;
+            int n;
 #pragma unroll 1
-            for (int win = 0; win < ntot; win += FM_EDGES) {
-                if (ntot > FM_EDGES) {
-                    // more than the buffer holds: the part that begins at win
+            for (int win = 0; win < ntot; win += n) {
+                n = whole ? ntot : (halves ? (win == 0 ? half : ntot - half) : min(FM_EDGES, ntot - win));
+                if (whole || halves) {
+                    const bool mine = whole || (lane < 16) == (win == 0);
+                    uint32_t l = mine ? lo : 0u, h = mine ? hi : 0u;
+                    if (plain) {
+                        uint32_t ahi = edges_at + 8u * (incl - (uint32_t)win), alo = ahi - 8u * chi;
+                        do {
+                            put_edge(l, alo, my_bits, (uint32_t)dst);
+                            put_edge(h, ahi, my_bits + 4u * 33u, (uint32_t)dst);
+                        } while (__any_sync(0xffffffffu, (l | h) != 0u));
+                    } else {
+                        const uint32_t tag = (uint32_t)(66 * (lane & 7)) | ((uint32_t)lane << 16);
+                        uint32_t ahi = edges_at + 4u * (incl - (uint32_t)win), alo = ahi - 4u * chi;
+                        do {
+                            put_mixed(l, alo, tag);
+                            put_mixed(h, ahi, tag + 33u);
+                        } while (__any_sync(0xffffffffu, (l | h) != 0u));
+                    }
+                } else {
                     uint32_t at = incl - clo - chi - (uint32_t)win;
                     auto put = [&](uint32_t place) {
                         if (at < (uint32_t)FM_EDGES) {
@@ -1640,22 +1670,9 @@ rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __re
                     };
                     for (uint32_t b = lo; b; b &= b - 1) put(66 * (lane & 7) + __ffs((int)b) - 1);
                     for (uint32_t b = hi; b; b &= b - 1) put(66 * (lane & 7) + 33 + __ffs((int)b) - 1);
-                } else if (plain) {
-                    uint32_t ahi = edges_at + 8u * incl, alo = ahi - 8u * chi;
-                    do {
-                        put_edge(lo, alo, my_bits, (uint32_t)dst);
-                        put_edge(hi, ahi, my_bits + 4u * 33u, (uint32_t)dst);
-                    } while (__any_sync(0xffffffffu, (lo | hi) != 0u));
-                } else {
-                    const uint32_t tag = (uint32_t)(66 * (lane & 7)) | ((uint32_t)lane << 16);
-                    uint32_t ahi = edges_at + 4u * incl, alo = ahi - 4u * chi;
-                    do {
-                        put_mixed(lo, alo, tag);
-                        put_mixed(hi, ahi, tag + 33u);
-                    } while (__any_sync(0xffffffffu, (lo | hi) != 0u));
                 }
                 __syncwarp();
-                const int n = min(FM_EDGES, ntot - win), first = written + win;
+                const int first = written + win;
                 // edges [0, mid) of the buffer belong to the first row, the others to the second
                 const int mid = max(0, min(n, edges0 - first));
 #pragma unroll 1

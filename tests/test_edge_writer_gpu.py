@@ -29,6 +29,10 @@ def _system(kind, dtype):
             pos += rng.integers(-3, 4, (n, 3)) * length
         elif kind == "moved":      # all atoms three cells away: one code, which is not that of a shift of zero
             pos += 3.0 * length
+        elif kind == "halves":     # the edges of four targets often exceed the buffer, those of two never do
+            r = 6.1
+        elif kind == "few_long":   # some groups have lists without hit bits: warps share their targets
+            pos[:700] = pos[0] + rng.random((700, 3)) * 2.5
         elif kind == "columns":    # few targets a row
             pos[:, 1:] *= 0.3
             r = 2.0
@@ -36,7 +40,7 @@ def _system(kind, dtype):
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
-@pytest.mark.parametrize("kind", ["dense", "dense_codes", "wrapped", "unwrapped", "moved", "columns"])
+@pytest.mark.parametrize("kind", ["dense", "dense_codes", "wrapped", "unwrapped", "moved", "columns", "halves", "few_long"])
 def test_edges(cuda, kind, dtype):
     pos, cell, pbc, r = _system(kind, dtype)
     g = O.radius_graph(pos, cell, pbc, r, None)
