@@ -425,75 +425,90 @@ halo_backward_end_kernel(dynb_halo_ctx c, uint32_t gen, unsigned long long budge
                          const V* __restrict__ recv, const int64_t* __restrict__ inv_offsets,
                          const uint32_t* __restrict__ inv_entries, V* __restrict__ out)
 {
-    // one warp per listed row (rows of fewer than 32 columns side by side), R rows in flight; lanes walk the row's V-wide
-    // columns.  What does not depend on the peers — the rows' ids and their places in the inverse CSR — is requested before
-    // the wait for the warp's first step, so that behind the wait the gradient rows and the received rows are one round of
-    // independent loads.  500 k rows, both ranks' whole exchange: 256 -> 171 us at 16 floats, 131 -> 96 us at 3.
-    constexpr int R = 4;
+    // Two listed rows per warp and step (rows of fewer than 32 columns side by side), 16 bytes of each row per lane.  Bound by
+    // HBM and by the chain row id -> place in the inverse CSR -> row; so each step's loads are issued together: the rows of
+    // this step, the places of the next, the ids of the one after, and only the ids and places of a warp's first step come
+    // before the wait for the peers.  Blocks stay (four per SM, 64 registers): 150 k of 500 k rows at 128 floats 57 -> 48 us,
+    // 64 floats 36 -> 28, 130 (scalar loads) 75 -> 64, 16 floats 15 -> 12, 700 rows 4.6 -> 3.4.  Four rows a step 59 us with
+    // three blocks per SM (spills with four) and 64 us with two; three rows 54; one row and six blocks 50; eight blocks' grid 50.
+    constexpr int R = 2, C = NARROW ? 1 : 16 / (VW * (int)sizeof(T));
     const int lane = threadIdx.x & 31;
     const int per = NARROW ? 32 / (int)q : 1, sub = NARROW ? lane / (int)q : 0, c0 = NARROW ? lane % (int)q : lane;
     const int wpb = blockDim.x >> 5;
     const int64_t nw = (int64_t)gridDim.x * wpb, w = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5);
-    struct Step { int64_t row[R]; uint32_t b[R], e[R], first[R]; };   // list places fit 32 bits (dynb_inverse_csr)
-    auto request = [&](int64_t r0, Step& s) {
+    auto ids = [&](int64_t r0, int64_t (&row)[R]) {
 #pragma unroll
         for (int k = 0; k < R; k++) {
-            s.row[k] = -1;
-            s.first[k] = 0;
             const int64_t r = r0 + k * per + sub;
-            if ((!NARROW || sub < per) && r < n_rows) {
-                s.row[k] = rows[r];
-                if (row_first != nullptr) s.first[k] = row_first[r];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < R; k++) {
-            s.b[k] = s.e[k] = 0;
-            if (s.row[k] >= 0) {
-                s.b[k] = (uint32_t)inv_offsets[s.row[k]];
-                s.e[k] = (uint32_t)inv_offsets[s.row[k] + 1];
-            }
+            row[k] = (!NARROW || sub < per) && r < n_rows ? rows[r] : -1;
         }
     };
-    Step cur;
+    // the number of received rows of each row and the first of them (list places fit 32 bits, dynb_inverse_csr)
+    auto places = [&](int64_t r0, const int64_t (&row)[R], uint32_t (&count)[R], uint32_t (&first)[R]) {
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            count[k] = first[k] = 0;
+            if (row[k] < 0) continue;
+            const int64_t b = inv_offsets[row[k]];
+            count[k] = (uint32_t)(inv_offsets[row[k] + 1] - b);
+            if (row_first != nullptr) first[k] = row_first[r0 + k * per + sub];
+            else if (count[k] > 0) first[k] = inv_entries[b];
+        }
+    };
+    auto add_row = [](V& to, const V& from) {
+        T* a = reinterpret_cast<T*>(&to);
+        const T* b = reinterpret_cast<const T*>(&from);
+#pragma unroll
+        for (int cc = 0; cc < VW; cc++) a[cc] += b[cc];
+    };
+    int64_t row[R], row1[R], row2[R];
+    uint32_t count[R], first[R], count1[R], first1[R];
     const int64_t step = nw * R * per;
     int64_t r0 = w * R * per;
-    if (r0 < n_rows) request(r0, cur);
+    ids(r0, row);
+    ids(r0 + step, row1);
+    places(r0, row, count, first);
     wait_all(c, 1, gen, budget_ns);
     if (blockIdx.x == 0) drift_or(c, 1, gen);
-    while (r0 < n_rows) {
-        for (int64_t col = c0; col < q; col += 32) {
-            V v[R], f[R];
-            bool hf[R];
+    for (; r0 < n_rows; r0 += step) {
+        for (int64_t col = c0; col < q; col += 32 * C) {
+            V v[R][C], f[R][C];
 #pragma unroll
             for (int k = 0; k < R; k++) {
-                hf[k] = false;
-                if (cur.row[k] >= 0) {
-                    v[k] = g[cur.row[k] * q + col];
-                    hf[k] = cur.b[k] < cur.e[k];
-                    if (hf[k]) f[k] = recv[(int64_t)(row_first != nullptr ? cur.first[k] : inv_entries[cur.b[k]]) * q + col];
-                }
+                if (row[k] < 0) continue;
+#pragma unroll
+                for (int u = 0; u < C; u++)
+                    if (u == 0 || col + 32 * u < q) {
+                        v[k][u] = g[row[k] * q + col + 32 * u];
+                        if (count[k] > 0) f[k][u] = recv[(int64_t)first[k] * q + col + 32 * u];
+                    }
+            }
+            if (col == c0) {
+                places(r0 + step, row1, count1, first1);
+                ids(r0 + 2 * step, row2);
             }
 #pragma unroll
             for (int k = 0; k < R; k++) {
-                if (cur.row[k] < 0) continue;
-                T* a = reinterpret_cast<T*>(&v[k]);
-                if (hf[k]) {
-                    const T* fr = reinterpret_cast<const T*>(&f[k]);
+                if (row[k] < 0) continue;
+                if (count[k] > 0) {
 #pragma unroll
-                    for (int cc = 0; cc < VW; cc++) a[cc] += fr[cc];
+                    for (int u = 0; u < C; u++)
+                        if (u == 0 || col + 32 * u < q) add_row(v[k][u], f[k][u]);
                 }
-                for (uint32_t j = cur.b[k] + 1; j < cur.e[k]; j++) {
-                    const V xx = recv[(int64_t)inv_entries[j] * q + col];
-                    const T* xr = reinterpret_cast<const T*>(&xx);
+                if (count[k] > 1) {
+                    const uint32_t b = (uint32_t)inv_offsets[row[k]], e = b + count[k];
+                    for (uint32_t j = b + 1; j < e; j++)
 #pragma unroll
-                    for (int cc = 0; cc < VW; cc++) a[cc] += xr[cc];
+                        for (int u = 0; u < C; u++)
+                            if (u == 0 || col + 32 * u < q) add_row(v[k][u], recv[(int64_t)inv_entries[j] * q + col + 32 * u]);
                 }
-                out[cur.row[k] * q + col] = v[k];
+#pragma unroll
+                for (int u = 0; u < C; u++)
+                    if (u == 0 || col + 32 * u < q) out[row[k] * q + col + 32 * u] = v[k][u];
             }
         }
-        r0 += step;
-        if (r0 < n_rows) request(r0, cur);
+#pragma unroll
+        for (int k = 0; k < R; k++) { row[k] = row1[k]; row1[k] = row2[k]; count[k] = count1[k]; first[k] = first1[k]; }
     }
 }
 
@@ -700,7 +715,8 @@ extern "C" int dynb_halo_backward_end(const dynb_halo_ctx* ctx, uint32_t gen, in
     const bool narrow = q < 32;
     auto launch = [&](auto kernel, auto* g, auto* recv, auto* out) {
         const int64_t warps = narrow ? (n_rows * q + 31) / 32 : n_rows;
-        kernel<<<grid_for(warps * 32), 256, 0, s>>>(*ctx, gen, bud, g, rows_dev, row_first_dev, n_rows, q, recv, inv_offsets_dev, inv_entries_dev, out);
+        const unsigned blocks = std::min<unsigned>(grid_for(warps * 32), sm_count_cached() * 4);
+        kernel<<<blocks, 256, 0, s>>>(*ctx, gen, bud, g, rows_dev, row_first_dev, n_rows, q, recv, inv_offsets_dev, inv_entries_dev, out);
     };
     auto run = [&](auto wide_kernel, auto narrow_kernel, auto* g, auto* recv, auto* out) {
         if (narrow) launch(narrow_kernel, g, recv, out);
