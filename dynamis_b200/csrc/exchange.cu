@@ -225,32 +225,51 @@ __device__ void copy_span(unsigned char* __restrict__ dst, const unsigned char* 
     }
 }
 
-// Rows of q 16-byte units whose flag is zero.  A warp reads 32 flags in one load and copies the rows behind them with eight
-// loads per lane in flight; rows shorter than a warp's 32 units lie side by side.
-// 500 k rows, reverse first half: 117 -> 113 us at 128 floats (four rows of a warp in flight, flags read one by one before).
+// Rows of q 16-byte units whose flag is zero.  A warp reads the flags of 16 rows (32 where rows shorter than its 32 units lie
+// side by side) one step ahead and copies the rows behind the zeros with eight loads per lane in flight; the warps' pieces
+// interleave like copy_span's.  With the grid of one wave, reverse first half
+// of 500 k rows with 150 k flagged: 105 -> 98 us at 128 floats, 61 -> 54 at 64, 100 against 107 at 256 (250 k rows); all 300 k rows
+// flagged 96 -> 77; 50 k rows 29 -> 21.
 __device__ void copy_rows_unflagged(uint4* __restrict__ dst, const uint4* __restrict__ src, const uint8_t* __restrict__ flag,
                                     int64_t rows, int64_t q, int64_t part, int64_t parts)
 {
-    constexpr int R = 8;
+    constexpr int R = 8, T = 16;
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     const int64_t nw = parts * wpb, w = part * wpb + (threadIdx.x >> 5);
-    const int64_t lo = rows * w / nw, hi = rows * (w + 1) / nw;
-    const int per = q >= 32 ? 1 : 32 / (int)q;   // rows side by side
-    const int sub = q >= 32 ? 0 : lane / (int)q, c0 = q >= 32 ? lane : lane % (int)q;
-    for (int64_t r0 = lo; r0 < hi; r0 += 32) {
-        const uint32_t todo = __ballot_sync(0xffffffffu, r0 + lane < hi && flag[r0 + lane] == 0);
-        for (int t = sub; t - sub < 32; t += R * per) {
+    const bool wide = q >= 32;
+    const int per = wide ? 1 : 32 / (int)q;   // rows side by side
+    const int sub = wide ? 0 : lane / (int)q, c0 = wide ? lane : lane % (int)q;
+    const int tile = wide ? T : 32;
+    const int64_t step = nw * tile;
+    auto read_flag = [&](int64_t r) { return lane < tile && r + lane < rows ? flag[r + lane] : (uint8_t)1; };
+    int64_t r0 = w * tile;
+    uint8_t next = read_flag(r0);
+    for (; r0 < rows; r0 += step) {
+        uint32_t todo = __ballot_sync(0xffffffffu, next == 0);
+        next = read_flag(r0 + step);
+        const int passes = wide ? (__popc(todo) + R - 1) / R : (32 + R * per - 1) / (R * per);
+        for (int p = 0; p < passes; p++) {
             bool ok[R];
+            int at[R];
 #pragma unroll
-            for (int k = 0; k < R; k++) ok[k] = sub < per && t + k * per < 32 && ((todo >> ((t + k * per) & 31)) & 1u);
+            for (int k = 0; k < R; k++) {
+                if (wide) {
+                    ok[k] = todo != 0u;
+                    at[k] = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                } else {
+                    at[k] = (p * R + k) * per + sub;
+                    ok[k] = sub < per && at[k] < 32 && ((todo >> (at[k] & 31)) & 1u);
+                }
+            }
             for (int64_t c = c0; c < q; c += 32) {
                 uint4 v[R];
 #pragma unroll
                 for (int k = 0; k < R; k++)
-                    if (ok[k]) v[k] = __ldcs(src + (r0 + t + k * per) * q + c);
+                    if (ok[k]) v[k] = __ldcs(src + (r0 + at[k]) * q + c);
 #pragma unroll
                 for (int k = 0; k < R; k++)
-                    if (ok[k]) dst[(r0 + t + k * per) * q + c] = v[k];
+                    if (ok[k]) dst[(r0 + at[k]) * q + c] = v[k];
             }
         }
     }
@@ -355,11 +374,13 @@ halo_forward_begin_kernel(dynb_halo_ctx c, const V* __restrict__ x, int64_t n_lo
     // Even blocks push first and copy second, odd blocks the other way round: measured on four GPUs (2 M rows
     // of 512 bytes copied, 395 k pushed) 0.52 ms against 0.51 ms for the push alone and 0.37 ms for the copy
     // alone; alternating the two inside every warp gave 0.58 ms, blocks with a fixed role 0.54-0.87 ms.
+    // The pieces of the push are dealt from the last block on: the blocks that get one piece more of it are not those that get one
+    // more of the copy.
     if (b & 1) {
         if (out_head != nullptr) copy_span(out_head, xs, head_bytes, head_vb, b, G);
-        push_units<V, true>(c, x, n_local, q, send_local, 0, seg, c.world_size, P, b, G, stride);
+        push_units<V, true>(c, x, n_local, q, send_local, 0, seg, c.world_size, P, G - 1 - b, G, stride);
     } else {
-        push_units<V, true>(c, x, n_local, q, send_local, 0, seg, c.world_size, P, b, G, stride);
+        push_units<V, true>(c, x, n_local, q, send_local, 0, seg, c.world_size, P, G - 1 - b, G, stride);
         if (out_head != nullptr) copy_span(out_head, xs, head_bytes, head_vb, b, G);
     }
     last_block_signals(c, 0, gen, announce);
@@ -407,9 +428,9 @@ halo_backward_begin_kernel(dynb_halo_ctx c, const V* __restrict__ g, int64_t n_l
     if (b & 1) {
         if (has_recv == nullptr) copy_span(out, gs, own_bytes, out_vb, b, G);
         else copy_rows_unflagged(reinterpret_cast<uint4*>(out), reinterpret_cast<const uint4*>(g), has_recv, n_local, row_bytes >> 4, b, G);
-        push_units<V, false>(c, g, n_local + n_ghost, q, nullptr, n_local, seg, c.world_size, P, b, G, stride);
+        push_units<V, false>(c, g, n_local + n_ghost, q, nullptr, n_local, seg, c.world_size, P, G - 1 - b, G, stride);
     } else {
-        push_units<V, false>(c, g, n_local + n_ghost, q, nullptr, n_local, seg, c.world_size, P, b, G, stride);
+        push_units<V, false>(c, g, n_local + n_ghost, q, nullptr, n_local, seg, c.world_size, P, G - 1 - b, G, stride);
         if (has_recv == nullptr) copy_span(out, gs, own_bytes, out_vb, b, G);
         else copy_rows_unflagged(reinterpret_cast<uint4*>(out), reinterpret_cast<const uint4*>(g), has_recv, n_local, row_bytes >> 4, b, G);
     }
@@ -633,10 +654,12 @@ static inline int span_vb(const void* a, const void* b, int64_t)
     return (u % 16 == 0) ? 16 : (u % 4 == 0) ? 4 : 1;
 }
 
+// One wave of three blocks per SM: every block has its share of the push and of the copy, and a second wave began while the first
+// one's stores drained (50 k rows of 128 floats, one of two ranks: forward 26 -> 23 us, reverse 29 -> 21; 500 k rows 119 and 120).
 static inline unsigned fused_grid(int64_t units16)
 {
     const int64_t blocks = (units16 + 256 * 8 - 1) / (256 * 8);
-    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)sm_count_cached() * 6));  // two waves of 3 CTAs per SM
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)sm_count_cached() * 3));
 }
 
 extern "C" int dynb_halo_forward_begin(const dynb_halo_ctx* ctx, const void* x_dev, int64_t n_local, int64_t row_bytes,
