@@ -33,7 +33,7 @@ def _dev_state(device: torch.device) -> dict:
     st = _STATE.get(key)
     if st is None:
         # pinned: the plan's header, and words for the counts of other calls; every call waits for what it has written there
-        pinned = torch.empty(64 + 8 * HOST_WORDS, dtype=torch.uint8).pin_memory()
+        pinned = torch.empty(64 + 8 * HOST_WORDS, dtype=torch.uint8, device="cpu").pin_memory()
         st = {"ws": None, "hdr_t": pinned, "hdr": _lib.RgHeader.from_address(pinned.data_ptr()), "geo": {}, "bytes": {},
               "words": pinned[64:].view(torch.int64)}
         _STATE[key] = st
@@ -89,7 +89,7 @@ def host_words(device: torch.device, count: int) -> torch.Tensor:
     """Pinned int64 words of the current stream of ``device``, for counts that a kernel writes or a copy brings and the caller
     waits for before it returns; a buffer of its own for more than ``HOST_WORDS``."""
     if count > HOST_WORDS:
-        return torch.empty((count,), dtype=torch.int64, pin_memory=True)
+        return torch.empty((count,), dtype=torch.int64, device="cpu", pin_memory=True)
     return _dev_state(device)["words"][:count]
 
 
