@@ -33,9 +33,11 @@ def _dev_state(device: torch.device) -> dict:
     st = _STATE.get(key)
     if st is None:
         # pinned: the plan's header, and words for the counts of other calls; every call waits for what it has written there
-        pinned = torch.empty(64 + 8 * HOST_WORDS, dtype=torch.uint8, device="cpu").pin_memory()
+        with torch.inference_mode(False):   # a tensor made in that mode cannot be copied to outside it
+            pinned = torch.empty(64 + 8 * HOST_WORDS, dtype=torch.uint8, device="cpu").pin_memory()
+            words = pinned[64:].view(torch.int64)
         st = {"ws": None, "hdr_t": pinned, "hdr": _lib.RgHeader.from_address(pinned.data_ptr()), "geo": {}, "bytes": {},
-              "words": pinned[64:].view(torch.int64)}
+              "words": words}
         _STATE[key] = st
     return st
 

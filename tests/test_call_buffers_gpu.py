@@ -37,3 +37,12 @@ def test_counts_under_another_default_device(cuda, fresh_state):
     with torch.device(cuda):
         assert torch.equal(select_eq(values, 3), torch.nonzero(values == 3).reshape(-1))
         _check_halo(cuda)
+
+
+def test_counts_first_read_in_inference_mode(cuda, fresh_state):
+    """What the first call leaves for later ones can be written outside the mode it was made in."""
+    with torch.inference_mode():
+        _check_halo(cuda)
+    _check_halo(cuda)
+    with torch.inference_mode():
+        _check_halo(cuda)
