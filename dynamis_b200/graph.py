@@ -22,7 +22,9 @@ import torch
 from . import _lib
 
 _STATE: dict = {}
-HOST_WORDS = 64
+HOST_WORDS = 64          # words of a pinned buffer for counts
+HOST_WORDS_KEPT = 16     # buffers that are kept when no call holds them
+_HOST_WORDS: list = []
 
 
 def _dev_state(device: torch.device) -> dict:
@@ -32,12 +34,8 @@ def _dev_state(device: torch.device) -> dict:
     key = (index, _lib.stream_of(device))
     st = _STATE.get(key)
     if st is None:
-        # pinned: the plan's header, and words for the counts of other calls; every call waits for what it has written there
-        with torch.inference_mode(False):   # a tensor made in that mode cannot be copied to outside it
-            pinned = torch.empty(64 + 8 * HOST_WORDS, dtype=torch.uint8, device="cpu").pin_memory()
-            words = pinned[64:].view(torch.int64)
-        st = {"ws": None, "hdr_t": pinned, "hdr": _lib.RgHeader.from_address(pinned.data_ptr()), "geo": {}, "bytes": {},
-              "words": words}
+        pinned = torch.empty(64, dtype=torch.uint8, device="cpu").pin_memory()
+        st = {"ws": None, "hdr_t": pinned, "hdr": _lib.RgHeader.from_address(pinned.data_ptr()), "geo": {}, "bytes": {}}
         _STATE[key] = st
     return st
 
@@ -87,12 +85,22 @@ def _empty_result(pos, n_target):
     )
 
 
-def host_words(device: torch.device, count: int) -> torch.Tensor:
-    """Pinned int64 words of the current stream of ``device``, for counts that a kernel writes or a copy brings and the caller
-    waits for before it returns; a buffer of its own for more than ``HOST_WORDS``."""
-    if count > HOST_WORDS:
-        return torch.empty((count,), dtype=torch.int64, device="cpu", pin_memory=True)
-    return _dev_state(device)["words"][:count]
+def take_host_words(count: int) -> torch.Tensor:
+    """Pinned int64 words, at least ``count`` of them, for counts that a kernel writes or a copy brings.  They are this call's
+    alone until it gives them back, behind its wait: the wait lets other threads run, and these may use the same stream.
+    A call that raises in between drops them."""
+    if count <= HOST_WORDS:
+        try:
+            return _HOST_WORDS.pop()
+        except IndexError:
+            pass
+    with torch.inference_mode(False):   # a tensor made in that mode cannot be copied to outside it
+        return torch.empty((max(count, HOST_WORDS),), dtype=torch.int64, device="cpu", pin_memory=True)
+
+
+def give_host_words(words: torch.Tensor) -> None:
+    if words.numel() == HOST_WORDS and len(_HOST_WORDS) < HOST_WORDS_KEPT:
+        _HOST_WORDS.append(words)
 
 
 def _plan_bytes(st: dict, n_atoms: int, n_targets: int, src_cap: int, cell_cap: int, dtype_code: int) -> int:

@@ -22,7 +22,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .graph import BinnedAtoms, host_words, radius_graph_pbc, radius_graph_pbc_ex
+from .graph import BinnedAtoms, give_host_words, radius_graph_pbc, radius_graph_pbc_ex, take_host_words
 from .state import DistEnvironment, MolecularInfo, PartitionMessagePassingInfo, SimulationConfig
 
 PARTITION_MAX_NUM_NEIGHBORS = 1000
@@ -140,7 +140,7 @@ def select_eq(values: torch.Tensor, value: int, gather_src: Optional[torch.Tenso
         out = torch.empty((n,), dtype=torch.int64, device=dev)
         # a count that is waited for is written to the host by the kernel (up to 16.7 M values: its tiles then need no prefix sum)
         waited = count is None and 0 < n <= SELECT_HOST_COUNT
-        cnt = host_words(dev, 1) if waited else torch.empty((1,), dtype=torch.int64, device=dev)
+        cnt = take_host_words(1) if waited else torch.empty((1,), dtype=torch.int64, device=dev)
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_select_workspace_bytes(n, ctypes.byref(nbytes)), "select_workspace_bytes")
         ws = scratch(dev, "select", nbytes.value)
@@ -149,6 +149,7 @@ def select_eq(values: torch.Tensor, value: int, gather_src: Optional[torch.Tenso
         if waited:
             torch.cuda.current_stream(dev).synchronize()
             k = int(cnt[0])
+            give_host_words(cnt)
         else:
             k = int(cnt.item()) if count is None else count
     return out[:k]
@@ -202,7 +203,8 @@ class AbstractPartitioner:
             ws = scratch(dev, "halo_lists", nbytes.value)
             # send offsets, recv offsets, number of own atoms and, behind them, the error word of the marking
             offs = torch.empty((2 * (W + 1) + 2,), dtype=torch.int64, device=dev)
-            offs_h = host_words(dev, 2 * (W + 1) + 2)
+            offs_h = take_host_words(2 * (W + 1) + 2)
+            sizes_h = offs_h[:2 * (W + 1) + 2]
             # everything up to the list sizes is queued before the one wait; the header's status is looked at behind it
             bins = BinnedAtoms(pos32, cell, pbc, ghost_cutoff) if N > 0 else None
             while True:
@@ -212,11 +214,12 @@ class AbstractPartitioner:
                                                         has_foreign.data_ptr(), offs.data_ptr() + 8 * (2 * W + 3), _stream(dev)), "rg_halo_mark")
                 _lib.check(L.dynb_halo_lists_plan(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
                                                   ws.numel(), _stream(dev)), "halo_lists_plan")
-                offs_h.copy_(offs, non_blocking=True)
+                sizes_h.copy_(offs, non_blocking=True)
                 torch.cuda.current_stream(dev).synchronize()
                 if bins is None or bins.done():
                     break
-            sizes = offs_h.tolist()
+            sizes = sizes_h.tolist()
+            give_host_words(offs_h)
             if bins is not None and sizes[2 * W + 3] & 0xFFFFFFFF != 0:
                 raise RuntimeError(f"build_halo_maps: partition_id has a label that is no rank's (world_size is {W})")
             total_send, total_recv, n_local = sizes[W], sizes[2 * W + 1], sizes[2 * W + 2]

@@ -1,4 +1,7 @@
-"""The host buffers of the calls that wait for a count, whatever the modes and threads around them."""
+"""The host buffers of the calls that wait for a count, whatever the modes and threads around them.  The wait lets go of the
+interpreter: another thread may make a call on the same stream before the waiting one reads its count."""
+
+import threading
 
 import pytest
 import torch
@@ -14,6 +17,33 @@ pytestmark = pytest.mark.gpu
 def fresh_state(monkeypatch):
     """No buffers left by earlier calls."""
     monkeypatch.setattr(G, "_STATE", {})
+    monkeypatch.setattr(G, "_HOST_WORDS", [])
+
+
+class _Wait:
+    """A stream behind whose first wait another thread makes a call on the same stream, before the waiting one goes on."""
+
+    def __init__(self, stream, pending):
+        self.stream, self.pending = stream, pending
+
+    def __getattr__(self, name):
+        return getattr(self.stream, name)
+
+    def synchronize(self):
+        self.stream.synchronize()
+        if self.pending:
+            t = threading.Thread(target=self.pending.pop())
+            t.start()
+            t.join()
+
+
+@pytest.fixture
+def behind_the_wait(monkeypatch):
+    """behind_the_wait(call): ``call`` runs in another thread right behind the next wait of this one."""
+    pending, me, real = [], threading.get_ident(), torch.cuda.current_stream
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: _Wait(real(dev), pending) if threading.get_ident() == me else real(dev))
+    yield pending.append
+    assert not pending, "the call did not wait"
 
 
 def _halo_edges(dev):
@@ -46,3 +76,41 @@ def test_counts_first_read_in_inference_mode(cuda, fresh_state):
     _check_halo(cuda)
     with torch.inference_mode():
         _check_halo(cuda)
+
+
+def test_count_of_a_selection(cuda, behind_the_wait):
+    values = (torch.arange(5000, device=cuda) % 7).to(torch.int64)
+    others = torch.ones(3000, dtype=torch.int64, device=cuda)
+    got = []
+    behind_the_wait(lambda: got.append(select_eq(others, 1)))
+    mine = select_eq(values, 3)
+    assert torch.equal(mine, torch.nonzero(values == 3).reshape(-1))
+    assert torch.equal(got[0], torch.arange(3000, device=cuda))
+
+
+def test_count_of_filtered_edges(cuda, behind_the_wait):
+    pos = torch.zeros((400, 3), device=cuda)
+    pos[:, 0] = torch.arange(400, device=cuda)
+    src = torch.arange(399, device=cuda)
+    edges = torch.cat([torch.stack([src, src + 1]), torch.stack([src[:-1], src[:-1] + 2])], dim=1).contiguous()
+    shifts = torch.zeros((edges.size(1), 3), device=cuda)
+    others = torch.ones(900, dtype=torch.int64, device=cuda)
+    behind_the_wait(lambda: select_eq(others, 1))
+    kept, kept_shifts = D.filter_edges_to_radius(edges, shifts, pos, torch.eye(3) * 500.0, 1.5)
+    assert torch.equal(kept, edges[:, :399]) and kept_shifts.shape == (399, 3)
+
+
+def test_sizes_of_halo_lists(cuda, behind_the_wait):
+    others = torch.ones(900, dtype=torch.int64, device=cuda)
+    behind_the_wait(lambda: [select_eq(others, 1) for _ in range(3)])
+    _check_halo(cuda)
+
+
+def test_words_are_one_calls_and_bounded(cuda, fresh_state):
+    held = [G.take_host_words(n) for n in [1, G.HOST_WORDS, G.HOST_WORDS + 1] + [2] * (G.HOST_WORDS_KEPT + 3)]
+    assert len({w.data_ptr() for w in held}) == len(held) and all(w.is_pinned() for w in held)
+    assert held[2].numel() == G.HOST_WORDS + 1
+    for w in held:
+        G.give_host_words(w)
+    assert len(G._HOST_WORDS) == G.HOST_WORDS_KEPT and all(w.numel() == G.HOST_WORDS for w in G._HOST_WORDS)
+    assert G.take_host_words(3).data_ptr() in {w.data_ptr() for w in held}
