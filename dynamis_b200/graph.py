@@ -210,7 +210,9 @@ class BinnedAtoms:
         self.pos = pos.contiguous()
         self.dtype_code = _lib.DYNB_F64 if pos.dtype == torch.float64 else _lib.DYNB_F32
         self.st = _dev_state(pos.device)
-        self.hdr_t, self.hdr = self.st["hdr_t"], self.st["hdr"]
+        # a header of its own: a graph call on the same stream, before done(), writes the stream's
+        self.hdr_t = torch.empty((64,), dtype=torch.uint8, device="cpu", pin_memory=True)
+        self.hdr = _lib.RgHeader.from_address(self.hdr_t.data_ptr())
         self.key, geo = _geometry(self.st, cell.detach().to("cpu").numpy(), pbc.detach().to("cpu").numpy(), radius, pos.size(0),
                                   self.dtype_code)
         self.cell_h, self.pbc_h, self.radius, self.src_capacity, self.cell_capacity = geo

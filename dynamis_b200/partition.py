@@ -183,7 +183,7 @@ class AbstractPartitioner:
             raise RuntimeError("pos must be a CUDA tensor")
         dev = pos.device
         N, W, R = int(global_state.num_atoms), int(env.world_size), int(env.global_rank)
-        # refused before anything is queued: the header and the list sizes are copied into buffers of this call
+        # refused before anything is queued: the header and the list sizes are written to buffers of this call
         if not 0 <= R < W:
             raise RuntimeError(f"global_rank must be in [0, world_size), got {R} of {W}")
         if W > 4096:

@@ -1,13 +1,16 @@
 """The host buffers of the calls that wait for a count, whatever the modes and threads around them.  The wait lets go of the
-interpreter: another thread may make a call on the same stream before the waiting one reads its count."""
+interpreter: another thread may make a call on the same stream before the waiting one reads its count.  And the header of a binning
+pass, which outlives a graph call."""
 
 import threading
 
+import numpy as np
 import pytest
 import torch
 
 import dynamis_b200 as D
 from dynamis_b200 import graph as G
+from dynamis_b200.graph import BinnedAtoms
 from dynamis_b200.partition import select_eq
 
 pytestmark = pytest.mark.gpu
@@ -114,3 +117,20 @@ def test_words_are_one_calls_and_bounded(cuda, fresh_state):
         G.give_host_words(w)
     assert len(G._HOST_WORDS) == G.HOST_WORDS_KEPT and all(w.numel() == G.HOST_WORDS for w in G._HOST_WORDS)
     assert G.take_host_words(3).data_ptr() in {w.data_ptr() for w in held}
+
+
+@pytest.mark.parametrize("periodic", [True, False])
+def test_header_of_a_binning_pass(cuda, periodic):
+    """The status of a pass whose image capacity was too small outlives a graph call made before it is looked at."""
+    rng = np.random.default_rng(8)
+    pos = torch.as_tensor((rng.random((4000, 3)) * 30.0).astype(np.float32), device=cuda)
+    cell, pbc = torch.eye(3) * 30.0, torch.tensor([True, True, periodic])
+    bins = BinnedAtoms(pos, cell, pbc, 5.0)
+    bins.src_capacity = 1000   # fewer slots than atoms: reported, nothing is written behind them
+    bins.launch()
+    D.radius_graph_pbc_ex(pos[:500].contiguous(), cell, pbc, 4.0, 0, False)
+    torch.cuda.synchronize()
+    assert bins.done() is False and bins.src_capacity > 4000
+    bins.launch()
+    torch.cuda.synchronize()
+    assert bins.done() is True and int(bins.hdr.M) >= 4000
