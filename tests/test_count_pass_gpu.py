@@ -1,4 +1,4 @@
-"""The count pass keeps the candidates of a group in registers, 64 to a block, with a copy of its loop for every number of blocks:
+"""The count pass keeps the candidates of a group in registers, 64 to a block, with copies of its loop for 2, 4, 5, 6, 7 and 8 blocks:
 candidate lists whose lengths lie at the edges of the blocks and of the 512 places that have hit bits, against the oracle."""
 
 import numpy as np
@@ -11,7 +11,7 @@ from oracle import cpu_oracle as O
 
 pytestmark = pytest.mark.gpu
 
-LENGTHS = [1, 2, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 319, 320, 321, 384, 385, 448, 449, 511, 512, 513, 1024, 1025]
+LENGTHS = [1, 2, 31, 32, 33, 63, 64, 65, 127, 128, 129, 191, 192, 193, 255, 256, 257, 319, 320, 321, 384, 385, 448, 449, 511, 512, 513, 1024, 1025]
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])

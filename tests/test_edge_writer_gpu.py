@@ -49,8 +49,9 @@ def test_edges(cuda, kind, dtype):
     assert_same_edges(canon_t(ei, cs), canon_o(g), kind)
     assert int(nni) == g["E"]
     # the targets' runs: as long as the degrees say, each target once
-    runs = ei[1][torch.cat([torch.ones(1, dtype=torch.bool, device=cuda), ei[1][1:] != ei[1][:-1]])]
+    runs, lengths = torch.unique_consecutive(ei[1], return_counts=True)
     assert runs.numel() == int((counts > 0).sum()) == runs.unique().numel()
+    assert torch.equal(lengths, counts[runs].to(torch.int64))
     # the model-side form: the opposite sign and the Cartesian shift
     e2, unit, cart = D.owned_graph(tp, tc, tb, r, pos.shape[0])
     assert torch.equal(e2, ei) and torch.equal(unit, -cs) and torch.equal(cart, torch.matmul(unit, tc.to(cuda, torch.float32)))
@@ -80,3 +81,100 @@ def test_negative_zero_shifts(cuda):
     _, unit, cart = D.owned_graph(pos, cell, torch.tensor([True] * 3), 4.0, 2000)
     still = (unit == 0).all(dim=1)
     assert still.any() and torch.signbit(cart[still]).all()
+
+
+class _Plan:
+    """What a plan leaves in its workspace, read on the host: the grid, the records in the order of the cells, the hit bits."""
+
+    POINTERS = ["h", "cstart", "tcstart", "spos", "sscan", "tpos", "tscan", "tmeta", "tcount", "toffset", "hitmask", "smeta"]
+
+    def __init__(self, plan, n):
+        base = plan.ws.data_ptr()
+        raw = plan.ws.cpu().numpy()
+        start = -base % 256
+        at = {k: int(v) - base for k, v in zip(self.POINTERS, raw[start + 512:start + 512 + 8 * len(self.POINTERS)].view(np.uint64))}
+        assert at["h"] == start
+
+        def view(name, dtype, count):
+            return raw[at[name]:at[name] + count * np.dtype(dtype).itemsize].view(dtype)
+
+        self.nx, self.ny, self.nz, self.sx = (int(v) for v in raw[start + 24:start + 40].view(np.int32))
+        self.pad, self.gx, self.sy = (int(v) for v in raw[start + 68:start + 80].view(np.int32))
+        assert (self.nx, self.ny, self.nz) == plan.grid
+        cells = self.nx * self.ny * self.nz
+        self.cstart, self.tcstart = view("cstart", np.uint32, cells + 1).astype(int), view("tcstart", np.uint32, cells + 1).astype(int)
+        self.smeta = view("smeta", np.uint32, 2 * plan.M).reshape(-1, 2).astype(int)
+        self.tmeta = view("tmeta", np.int32, 4 * n).reshape(-1, 4).astype(int)
+        self.toffset = view("toffset", np.int64, n + 1)
+        self.hitmask = view("hitmask", np.uint16, 32 * n).reshape(-1, 32)
+
+    def groups(self):
+        """(targets, records of the candidate list) of every group with targets."""
+        for cz in range(self.nz):
+            for cy0 in range(0, self.ny, self.sy):
+                cy1 = min(cy0 + self.sy, self.ny) - 1
+                for cx0 in range(0, self.nx, self.sx):
+                    cx1 = min(cx0 + self.sx, self.nx) - 1
+                    targets = [t for cy in range(cy0, cy1 + 1)
+                               for t in range(self.tcstart[(cz * self.ny + cy) * self.nx + cx0], self.tcstart[(cz * self.ny + cy) * self.nx + cx1 + 1])]
+                    if not targets:
+                        continue
+                    records = []
+                    for zz in range(max(cz - self.pad, 0), min(cz + self.pad, self.nz - 1) + 1):
+                        for yy in range(max(cy0 - self.pad, 0), min(cy1 + self.pad, self.ny - 1) + 1):
+                            row = (zz * self.ny + yy) * self.nx
+                            records += range(self.cstart[row + max(cx0 - self.pad, 0)], self.cstart[row + min(cx1 + self.pad, self.nx - 1) + 1])
+                    yield targets, np.array(records, dtype=int)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", ["dense", "dense_codes", "wrapped", "unwrapped", "halves", "columns", "few_long"])
+def test_order_of_the_edges(cuda, kind, dtype):
+    """The order is part of the result.  Targets follow one another cell by cell.  The edges of a target come by (place mod 32,
+    place / 32) of their candidates in the group's list where it has at most 512 places, and by place in longer lists and
+    wherever distances are asked for."""
+    pos, cell, pbc, r = _system(kind, dtype)
+    n = len(pos)
+    plan = G.plan_radius_graph(torch.as_tensor(pos, device=cuda), torch.as_tensor(cell), torch.tensor(pbc), r)
+    p = _Plan(plan, n)
+    edges = {d: [a.cpu().numpy() for a in plan.fill(d)[:2]] for d in (False, True)}
+    degrees, lists = plan.counts.cpu().numpy(), set()
+    assert plan.E == p.toffset[-1] == degrees.sum()
+    seen = 0
+    for targets, records in p.groups():
+        short = len(records) <= 512
+        lists.add(short)
+        codes = p.smeta[records, 1]
+        atoms, moved = p.smeta[records, 0], np.stack([(codes >> k & 1023) - 512 for k in (0, 10, 20)], axis=1)
+        for t in targets:
+            seen += 1
+            at = slice(int(p.toffset[t]), int(p.toffset[t + 1]))
+            atom, shifts = p.tmeta[t, 0], moved + p.tmeta[t, 1:]
+            assert at.stop - at.start == degrees[atom]
+            place_of = {(a, *s): k for k, (a, s) in enumerate(zip(atoms.tolist(), shifts.tolist()))}
+            assert len(place_of) == len(records)
+            for dist, (ei, cs) in edges.items():
+                places = [place_of[(a, *s)] for a, s in zip(ei[0, at].tolist(), cs[at].astype(int).tolist())]
+                assert (ei[1, at] == atom).all()
+                if short and not dist:
+                    bits = p.hitmask[t][:, None] >> np.arange(16) & 1
+                    assert places == [32 * s + lane for lane, s in zip(*np.nonzero(bits))]
+                else:
+                    assert places == sorted(set(places)), "by place"
+    assert seen == n
+    assert True in lists and (kind != "few_long" or False in lists)
+
+
+# boxes a few cells wide along two axes or one, so that a row or a column of groups is one, two, three, 63 to 65 or hundreds long
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("length,other", [(L, 8.0) for L in (8.0, 12.0, 16.0, 25.0, *np.arange(240.0, 268.0, 4.0), *np.arange(480.0, 528.0, 4.0), 2500.0)] + [(260.0, 260.0)])
+def test_look_up_of_a_group_in_thin_boxes(cuda, length, other, axis, periodic):
+    """The kernels divide a group's number by the lengths of the rows and of the columns of groups."""
+    box = np.array([length, other, 8.0] if axis == 0 else [other, length, 8.0])
+    pos = (np.random.default_rng(int(length)).random((int(0.04 * box.prod()) + 2, 3)) * box).astype(np.float32)
+    cell, pbc = np.diag(box).astype(np.float32), [periodic] * 3
+    g = O.radius_graph(pos, cell, pbc, 4.0, None)
+    ei, cs, nni, counts = D.radius_graph_pbc_ex(torch.as_tensor(pos, device=cuda), torch.as_tensor(cell), torch.tensor(pbc), 4.0, 0, False)
+    np.testing.assert_array_equal(counts.cpu().numpy(), g["counts"])
+    assert_same_edges(canon_t(ei, cs), canon_o(g), f"{box}")

@@ -1,5 +1,6 @@
-"""The division by a plan's number of groups (group_divide in csrc/radius_graph.cu), restated: from floor((2^32 - 1) / d) the upper half
-of the product is the quotient or one less, for every 32-bit dividend."""
+"""The arithmetic behind the look-up of a group (group_divide in csrc/radius_graph.cu), restated: from floor((2^32 - 1) / d) the upper
+half of the product is the quotient or one less, for every 32-bit dividend.  The kernels' own division is run, in boxes of many
+shapes, by test_look_up_of_a_group_in_thin_boxes."""
 
 import numpy as np
 import pytest

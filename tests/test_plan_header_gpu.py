@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from dynamis_b200 import _lib
+from dynamis_b200.graph import plan_radius_graph
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +45,16 @@ def test_header(cuda, memory, bins_only, n):
     assert h.E == (0 if bins_only else int(counts.sum()))
     before, behind = at - host.data_ptr(), at + 64 - host.data_ptr()
     assert (host[:before] == 255).all() and (host[behind:] == 255).all()
+
+
+@pytest.mark.parametrize("n", [8192 * 2048 - 1, 8192 * 2048])
+def test_header_of_the_largest_scans(cuda, n):
+    """Up to 8192 tiles of degrees (one more than targets) the scan writes the header itself; beyond that it is copied."""
+    gen = torch.Generator(device=cuda).manual_seed(1)
+    length = (n / 0.02) ** (1.0 / 3.0)
+    pos = torch.rand(n, 3, generator=gen, device=cuda) * length
+    plan = plan_radius_graph(pos, torch.eye(3) * length, torch.tensor([True] * 3), 2.0)
+    base = (-plan.ws.data_ptr()) % 256
+    E, M = plan.ws[base:base + 16].view(torch.int64).tolist()
+    assert plan.E == E == int(plan.counts.sum(dtype=torch.int64)) > 0 and plan.M == M >= n
+    assert plan.max_degree == int(plan.counts.max())
