@@ -227,9 +227,9 @@ __device__ void copy_span(unsigned char* __restrict__ dst, const unsigned char* 
 
 // Rows of q 16-byte units whose flag is zero.  A warp reads the flags of 16 rows (32 where rows shorter than its 32 units lie
 // side by side) one step ahead and copies the rows behind the zeros with eight loads per lane in flight; the warps' pieces
-// interleave like copy_span's.  With the grid of one wave, reverse first half
-// of 500 k rows with 150 k flagged: 105 -> 98 us at 128 floats, 61 -> 54 at 64, 100 against 107 at 256 (250 k rows); all 300 k rows
-// flagged 96 -> 77; 50 k rows 29 -> 21.
+// interleave like copy_span's.  With the grid of one wave, before and after, reverse first half: 500 k rows with 150 k flagged 105 -> 98 us
+// at 128 floats and 61 -> 54 at 64; 250 k rows of 256 floats 107 -> 100; all 300 k rows flagged 96 -> 77; 50 k rows 29 -> 21 (two ranks
+// on one GPU).
 __device__ void copy_rows_unflagged(uint4* __restrict__ dst, const uint4* __restrict__ src, const uint8_t* __restrict__ flag,
                                     int64_t rows, int64_t q, int64_t part, int64_t parts)
 {
@@ -373,7 +373,8 @@ halo_forward_begin_kernel(dynb_halo_ctx c, const V* __restrict__ x, int64_t n_lo
     const int64_t head_bytes = n_local * row_bytes;
     // Even blocks push first and copy second, odd blocks the other way round: measured on four GPUs (2 M rows
     // of 512 bytes copied, 395 k pushed) 0.52 ms against 0.51 ms for the push alone and 0.37 ms for the copy
-    // alone; alternating the two inside every warp gave 0.58 ms, blocks with a fixed role 0.54-0.87 ms.
+    // alone; alternating the two inside every warp gave 0.58 ms, blocks with a fixed role 0.54-0.87 ms (all with the grid of two
+    // waves that fused_grid gave then).
     // The pieces of the push are dealt from the last block on: the blocks that get one piece more of it are not those that get one
     // more of the copy.
     if (b & 1) {
@@ -656,6 +657,8 @@ static inline int span_vb(const void* a, const void* b, int64_t)
 
 // One wave of three blocks per SM: every block has its share of the push and of the copy, and a second wave began while the first
 // one's stores drained (50 k rows of 128 floats, one of two ranks: forward 26 -> 23 us, reverse 29 -> 21; 500 k rows 119 and 120).
+// Measured with two ranks on one GPU, where a peer's buffer lies in the same memory.  Not measured over NVLink, whose stores take longer
+// to drain: there two waves may be the better choice again.
 static inline unsigned fused_grid(int64_t units16)
 {
     const int64_t blocks = (units16 + 256 * 8 - 1) / (256 * 8);

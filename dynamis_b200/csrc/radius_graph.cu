@@ -974,13 +974,13 @@ template <typename T> struct PairParams {
     const Vec4<T>* tpos;
     const float4* tscan;      // the targets' coordinates as the count pass tests them, and the entry
     const int4* tmeta;
-    uint32_t* tcount;         // [Nt+1] degree per sorted target; running cursor in FILL
+    uint32_t* tcount;         // [Nt+1] degree per sorted target; running cursor of rg_pair_kernel
     const long long* toffset; // [Nt+1]
-    unsigned short* hitmask;  // [Nt, 32] per lane: bit s set if candidate 32 s + lane is a neighbour (written by COUNT)
+    unsigned short* hitmask;  // [Nt, 32] per lane: bit s set if candidate 32 s + lane is a neighbour (written by rg_count_kernel)
     const uint2* smeta;       // [M] {atom id, packed shift code} per source record
     int32_t* counts_out;      // [Nt] degrees in caller order, or nullptr
     const uint32_t* glist;    // groups that hold at least one target (h->active_groups entries), or nullptr = all groups
-    uint32_t* long_list;      // groups whose candidate list exceeds the hit bits (h->reserved[1] entries, written by COUNT)
+    uint32_t* long_list;      // groups whose candidate list exceeds the hit bits (h->reserved[1] entries, written by rg_count_kernel)
     long long n_targets;
     // halo marking only (rg_halo_*): owner of every source record and of every target, and a word for every candidate run
     unsigned short* sown;     // [M]; lies over the binning slots, which nothing reads behind the plan
@@ -1037,11 +1037,13 @@ rg_group_list_kernel(const PairParams<T>* __restrict__ params_dev, uint32_t* __r
 // registers, two candidates to a packed register pair, and the targets pass by one at a time: the test loop reads nothing from
 // memory and is unrolled over the whole list.  (Before: candidates in shared memory, two targets at a time; three of its
 // loads, the shifting of the bit and eight compares with selects for every 64 candidates and two targets.)
-// Bound by the FMA pipe and the issue of instructions (issue slots 64 % busy, 190 M warp instructions for a million atoms of the
+// Bound by the FMA pipe and the issue of instructions (issue slots 65 % busy, 191 M warp instructions for a million atoms of the
 // liquid against 245 M; a packed instruction holds the FMA pipe for two cycles).  Before and after: 300 -> 262 us (liquid, 1 M
 // atoms, 5 A), 357 -> 302 (a rank's 1 M of the 8 M copper atoms), 226 -> 171 (silicon in double precision, 500 k atoms, 6 A).
 // ------------------------------------------------------------------------------------------
-// Seven blocks of four warps: 72 registers.  80 registers and six blocks 276 us, 96 and five 281, 128 and four 293 (liquid).
+// Seven blocks of four warps: 72 registers, with spills (a stack of 88 bytes, 116 bytes of stores and 124 of loads; in double, which keeps
+// two words of bits a target, 120, 220 and 332).  Fewer spills did not pay: 80 registers and six blocks 276 us, 96 and five 281, 128 and
+// four 293 (liquid in single precision; double takes the same shape, which was not measured against others there).
 // Blocks of two warps, and half or twice the waves: within 2 %.
 constexpr int COUNT_WARPS = 4;
 constexpr int COUNT_BLOCKS = 7;
@@ -1213,7 +1215,7 @@ rg_count_kernel(const PairParams<T> p)
             auto run = [&](auto nb, auto full) {
                 count_group<T, decltype(nb)::value, decltype(full)::value>(p, index, g, hit, may, all_undecided, max_degree, lane, le);
             };
-            // a copy of the test loop for every length but the shortest: no block of 64 is tested for nothing
+            // copies of the test loop for 2, 4, 5, 6, 7 and 8 blocks of 64; one block is tested as two and three as four, with padding
             switch ((g.clen + 63) >> 6) {
             case 1:
             case 2: run(std::integral_constant<int, 2>(), std::integral_constant<int, 0>()); break;
@@ -1437,7 +1439,7 @@ rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restri
 // what belongs to its bits into the warp's buffer; the buffer goes out 32 edges at a time.
 // In most groups all candidates have one shift code, and then all shifts are zero (the targets are candidates too): zeros are
 // written 32 bytes a lane, and a group's edges need the two indices only.
-// Bound by the latency of its loads and by instructions (191 M warp instructions, issue slots 53 % busy), not by the 1.47 GB it
+// Bound by the latency of its loads and by instructions (192 M warp instructions, issue slots 57 % busy), not by the 1.47 GB it
 // writes (4.8 TB/s).  Target by target, with a prefix sum, a list and two rounds of 32 edges for each of them, and three
 // stores with a stride of 12 bytes for the shifts: 240 M.  Before and after: 381 -> 308 us (liquid, 1 M atoms), 742 -> 611 (a
 // rank's 1 M of the 8 M copper atoms, with Cartesian shifts), 189 -> 160 (silicon, double precision), 15 -> 13 (1 k atoms, where
@@ -1807,7 +1809,7 @@ rg_fillmask_dist_kernel(const PairParams<T>* __restrict__ params_dev, long long*
         int L;
         const int run_off = warp_excl_scan(run_len, lane, &L);
         const int nslots = (L + 31) >> 5;
-        if (nslots == 0 || nslots > RG_MASK_SLOTS) continue;  // a longer list has no hit bits: rg_pair_kernel<FILL> writes that group
+        if (nslots == 0 || nslots > RG_MASK_SLOTS) continue;  // a longer list has no hit bits: rg_pair_kernel writes that group
 
         __syncwarp();
         runs_compact(delta, run_a, run_off, run_len, lt);

@@ -176,7 +176,8 @@ int dynb_radix_sort_pairs(uint64_t* keys_dev, uint32_t* vals_dev, int64_t n, int
  * atom_counts = bincount(labels) and partition_indices = vertex_numbers[nonzero(labels == R)]
  * (dynamis_state/src/csrc/partition/sfc_partitioner.cpp:166-176).  bad_dev: one uint32, non-zero
  * when a value fell outside [0, W).  dynb_select_eq_i64 writes at most n values to out_dev
- * (ascending positions; gather_src_dev[i] instead of i when given) and the count to count_dev. */
+ * (ascending positions; gather_src_dev[i] instead of i when given) and the count to count_dev, which may be
+ * pinned host memory that the device can write to (read it behind a wait for the stream). */
 int dynb_bincount_i64(const int64_t* a_dev, int64_t n, int64_t W, int64_t* counts_dev, uint32_t* bad_dev, void* stream);
 int dynb_select_workspace_bytes(int64_t n, int64_t* bytes);
 int dynb_select_eq_i64(const int64_t* a_dev, int64_t n, int64_t value, const int64_t* gather_src_dev,
@@ -231,7 +232,8 @@ int dynb_scatter_iota(const int64_t* idx_dev, int64_t n, int64_t N, int64_t* g2l
  * filter_edges_to_radius (dynamis_state/src/csrc/graph/dist_graph_ops.cpp:5-37,
  * dist_graph_ops_kernels.cu:16-43, 62-102): keeps edge e iff
  * |pos[src] + shift @ cell - pos[dst]|^2 <= radius^2 (float32), order preserving.  The plan writes
- * the number kept to count_dev; the fill compacts edges [2,E] -> [2,E_out] and the shift rows of
+ * the number kept to count_dev (device memory, or pinned host memory that the device can write to);
+ * the fill compacts edges [2,E] -> [2,E_out] and the shift rows of
  * any element size (shift_row_bytes = 3 * element size).  Workspace: dynb_filter_edges_workspace_bytes(E), or
  * dynb_select_workspace_bytes(2 * E), which is no smaller. */
 int dynb_filter_edges_workspace_bytes(int64_t E, int64_t* bytes);
