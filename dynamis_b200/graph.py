@@ -29,7 +29,8 @@ _HOST_WORDS: list = []
 
 def _dev_state(device: torch.device) -> dict:
     """Plan workspace and pinned header of one (device, stream): calls on different streams of a device get
-    workspaces of their own and so cannot race on one; calls on one stream are ordered by the stream."""
+    workspaces of their own and so cannot race on one; the work of calls on one stream is ordered by the stream, and
+    one thread at a time makes them."""
     index = device.index if device.index is not None else torch.cuda.current_device()
     key = (index, _lib.stream_of(device))
     st = _STATE.get(key)
@@ -119,7 +120,7 @@ class RadiusGraphPlan:
     """Result of the counting phase: degrees are known, the edge buffers are not written yet.
 
     ``fill()`` may be called more than once (the benchmark times it in isolation); the plan stays
-    valid until the next radius-graph call on the same device, which reuses the workspace.
+    valid until the next radius-graph call on the same stream, which reuses the workspace.
     """
 
     __slots__ = ("ws", "dtype_code", "E", "M", "counts", "device", "pos_dtype", "max_degree", "grid", "num_groups", "walked",
