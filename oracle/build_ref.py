@@ -36,7 +36,7 @@ TIMING_CONFIG = "#pragma once\n/* #undef DYNAMIS_TIMING */\n"
 
 
 def build(reference: str = DEFAULT_REFERENCE, force: bool = False) -> str | None:
-    if not os.path.isdir(reference):
+    if not os.path.isdir(os.path.join(reference, "dynamis_state")):
         return SO if os.path.exists(SO) else None
     if os.path.exists(SO) and not force:
         return SO

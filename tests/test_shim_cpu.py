@@ -49,7 +49,7 @@ for name in ["feature_push_forward", "feature_push_backward", "supports_fabric_h
 env = dynamis_state.TorchDistEnv(is_distributed=False)
 assert env.world_size == 1 and env.dist_env.world_size == 1
 
-if os.path.isdir(ref):
+if os.path.isdir(os.path.join(ref, "dynamis_model")):
     def load(name, rel):
         spec = importlib.util.spec_from_file_location(name, os.path.join(ref, rel))
         mod = importlib.util.module_from_spec(spec)
@@ -87,5 +87,5 @@ def test_shim_packages_resolve_and_reference_callers_load():
     r = subprocess.run([sys.executable, "-c", _CHILD, ROOT, REF], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
     assert "shim ok" in r.stdout
-    if os.path.isdir(REF):
+    if os.path.isdir(os.path.join(REF, "dynamis_model")):
         assert "reference callers loaded" in r.stdout
