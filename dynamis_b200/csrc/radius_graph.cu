@@ -71,6 +71,7 @@ struct DevHeader {
     uint32_t halo_groups;    // halo marking: entries of halo_list
     float test_near, test_lo, test_hi;  // double positions: thresholds of the float test (float_test)
     uint32_t test_equal_is_near;
+    uint32_t count_next;      // count pass: groups taken behind every warp's first
 };
 static_assert(offsetof(DevHeader, ncell_plus1) == sizeof(dynb_rg_header), "public header prefix mismatch");
 
@@ -276,13 +277,14 @@ __device__ __forceinline__ unsigned long long f32x2_pack(float lo, float hi)
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
     return r;
 }
+// The candidate comes negated: a - s = a + (-s).
 __device__ __forceinline__ unsigned long long dist2_x2(unsigned long long ax2, unsigned long long ay2, unsigned long long az2,
-                                                       unsigned long long sx2, unsigned long long sy2, unsigned long long sz2)
+                                                       unsigned long long minus_sx2, unsigned long long minus_sy2, unsigned long long minus_sz2)
 {
     unsigned long long dx, dy, dz, d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dx) : "l"(ax2), "l"(sx2));
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dy) : "l"(ay2), "l"(sy2));
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dz) : "l"(az2), "l"(sz2));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(dx) : "l"(ax2), "l"(minus_sx2));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(dy) : "l"(ay2), "l"(minus_sy2));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(dz) : "l"(az2), "l"(minus_sz2));
     asm("mul.rn.f32x2 %0, %1, %1;" : "=l"(d) : "l"(dy));
     asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(dx), "l"(d));
     asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(dz), "l"(d));
@@ -915,7 +917,7 @@ __device__ __forceinline__ void glue_write(const GlueArgs& g, float* __restrict_
 // lane's run of source records.  Both cell-scan kernels keep the grid in shared memory and read it where a group is looked
 // up: in registers it left too few for the loops.
 struct GroupShape { int nx, ny, nz, sx, sy, pad, gx, gy; uint32_t by_gx, by_gy; };
-struct GroupDesc { uint32_t tb0, te0, tb1, te1; int run_a, run_e; };   // as loaded: nothing waits for the loads until the group's turn
+struct GroupDesc { uint32_t tb0, te0, tb1, te1; int run_a, run_e, cy0, cy1, cz; };   // as loaded: nothing waits for the loads until the group's turn
 __device__ __forceinline__ GroupShape group_shape(const DevHeader* hp)
 {
     const int gx = hp->gx, gy = (hp->ny + hp->group_cells_y - 1) / hp->group_cells_y;
@@ -945,6 +947,9 @@ __device__ __forceinline__ GroupDesc fetch_group(const volatile GroupShape& g, c
     const uint32_t row = group_divide(grp, gx, g.by_gx, ix);
     const int cz = (int)group_divide(row, gy, g.by_gy, iy), cx0 = (int)ix * sx, cy0 = (int)iy * sy;
     const int cx1 = min(cx0 + sx, nx) - 1, cy1 = min(cy0 + sy, ny) - 1;
+    d.cy0 = cy0;
+    d.cy1 = cy1;
+    d.cz = cz;
     const uint32_t* tcell = tcstart + ((uint32_t)cz * ny + cy0) * nx;
     d.tb0 = tcell[cx0];
     d.te0 = tcell[cx1 + 1];
@@ -1034,137 +1039,243 @@ rg_group_list_kernel(const PairParams<T>* __restrict__ params_dev, uint32_t* __r
 
 // ------------------------------------------------------------------------------------------
 // rg_count: degrees and hit bits.  Lane l holds the coordinates of candidates l, 32 + l, 64 + l, ... of its warp's list in
-// registers, two candidates to a packed register pair, and the targets pass by one at a time: the test loop reads nothing from
-// memory and is unrolled over the whole list.  (Before: candidates in shared memory, two targets at a time; three of its
-// loads, the shifting of the bit and eight compares with selects for every 64 candidates and two targets.)
-// Bound by the FMA pipe and the issue of instructions (issue slots 65 % busy, 191 M warp instructions for a million atoms of the
-// liquid against 245 M; a packed instruction holds the FMA pipe for two cycles).  Before and after: 300 -> 262 us (liquid, 1 M
-// atoms, 5 A), 357 -> 302 (a rank's 1 M of the 8 M copper atoms), 226 -> 171 (silicon in double precision, 500 k atoms, 6 A).
+// registers, two candidates to a packed register pair, and the targets pass by one at a time, from shared memory: the test loop is
+// unrolled over the whole list.  A warp takes the next group when it is done with one.
+// Two tests a pair: d <= r^2, and d above the self-distance limit.  The second is made for the two blocks of 64 candidates only that
+// hold the records of the targets' own cell rows, for records elsewhere are further away (targets next to the faces of these rows are
+// tested again in full); for these two blocks to be the same registers in every group the blocks are loaded in turned order.
+// The bits of a target go to shared memory and leave it, with the degrees, for 16 targets together.
+// Bound by the latency of its loads, its issue slots (60 % busy) and the FMA pipe (40 %): 162 instructions a target of the liquid, 56 of
+// them tests; 207 without the items above.  Before and after: 266 -> 207 us (liquid, 1 M atoms, 5 A), 309 -> 259 (a rank's 1 M of the
+// 8 M copper atoms), 177 -> 163 (silicon in double precision, 500 k atoms, 6 A), 46 -> 39 (liquid, 131 k), 9.5 -> 8.3 (1 k).
+// Distances from the matrix units (halves of split coordinates, pairs near the cutoff again) took 482 us: operand moves and the
+// 8 cycles of an m16n8k16.  The next group's look-up, or its candidates, copied ahead to shared memory: 218 and 231 us.
 // ------------------------------------------------------------------------------------------
-// Seven blocks of four warps: 72 registers, with spills (a stack of 88 bytes, 116 bytes of stores and 124 of loads; in double, which keeps
-// two words of bits a target, 120, 220 and 332).  Fewer spills did not pay: 80 registers and six blocks 276 us, 96 and five 281, 128 and
-// four 293 (liquid in single precision; double takes the same shape, which was not measured against others there).
-// Blocks of two warps, and half or twice the waves: within 2 %.
+// Five blocks of four warps: 96 registers, hardly any spills.  Six and 80: 213 us, 284 for the rank's copper.  Eight waves of blocks in
+// place of the counter: 222.
 constexpr int COUNT_WARPS = 4;
-constexpr int COUNT_BLOCKS = 7;
-constexpr int COUNT_WAVES = 8;
+constexpr int COUNT_BLOCKS = 5;
+constexpr int COUNT_TARGETS = 16;   // staged together
 
-// Thresholds of a distance test, each twice: a bit is set when lo <= d < hi, where lo and hi are the floats behind the bounds of
-// "d > near && d <= upto", and hi >= lo.  A difference of two floats is zero only for equal ones, so the signs of d - lo and
+// A pair as the result of an instruction: pairs that are copies (of two words of different loads, of one word twice, of a
+// uniform register) are made again in front of every use, two moves each time: 8 of 19 instructions a block.  nothing: {-0, -0}
+__device__ __forceinline__ unsigned long long f32x2_kept(float lo, float hi, unsigned long long nothing)
+{
+    unsigned long long r = f32x2_pack(lo, hi);
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(r) : "l"(nothing));
+    return r;
+}
+
+// Thresholds of a distance test, negated and twice: a bit is set when lo <= d < hi, where lo and hi are the floats behind the bounds
+// of "d > near && d <= upto", and hi >= lo.  A difference of two floats is zero only for equal ones, so the signs of d - lo and
 // d - hi are exact, and that of their product (which keeps it when it underflows) is set between the two.  Two packed
-// subtractions, a packed product and a funnel shift a bit: as compares and selects the bits kept the ALU pipe busier than the
+// additions, a packed product and a funnel shift a bit: as compares and selects the bits kept the ALU pipe busier than the
 // distances the FMA pipe (289 us against 276, liquid of a million atoms).
-struct SignTest { unsigned long long lo, hi; };
+struct SignTest { float2 lo, hi; };
 __device__ __forceinline__ SignTest sign_test(float near, float upto)
 {
     const float lo = nextafterf(near, INFINITY), hi = fmaxf(nextafterf(upto, INFINITY), lo);
-    SignTest t;
-    t.lo = f32x2_pack(lo, lo);
-    t.hi = f32x2_pack(hi, hi);
-    return t;
+    return {make_float2(-lo, -lo), make_float2(-hi, -hi)};
 }
-// bits = bits << 2 with the outcomes for the two distances of d (the upper one first)
-__device__ __forceinline__ void test_x2(unsigned long long d, const SignTest& t, uint32_t& bits)
+// From shared memory, every time: registers are short in the test loop.
+__device__ __forceinline__ unsigned long long f32x2_load(const float2& at)
 {
-    unsigned long long a, b;
+    unsigned long long r;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(r) : "r"((uint32_t)__cvta_generic_to_shared(&at)));
+    return r;
+}
+__device__ __forceinline__ unsigned long long f32x2_add(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// bits = bits << 2 with the signs of the two halves of a (the upper one first)
+__device__ __forceinline__ void push_signs(unsigned long long a, uint32_t& bits)
+{
     uint32_t s0, s1;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(d), "l"(t.lo));
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(b) : "l"(d), "l"(t.hi));
-    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
     asm("mov.b64 {%0, %1}, %2;" : "=r"(s0), "=r"(s1) : "l"(a));
     bits = __funnelshift_l(s1, bits, 1);
     bits = __funnelshift_l(s0, bits, 1);
 }
-
-// The undecided candidates of a target (bit s: place 32 s + lane of the staged chunk) by the double test.
-template <typename T>
-__device__ __forceinline__ uint32_t exact_hits(const PairParams<T>& p, uint32_t t, uint32_t undecided, const RunIndex& index, int cbeg, int clen,
-                                               int lane, uint32_t le)
+__device__ __forceinline__ void test_x2(unsigned long long d, unsigned long long lo, unsigned long long hi, uint32_t& bits)
 {
-    uint32_t hits = 0;
-    while (undecided) {
-        const int s = __ffs((int)undecided) - 1, j = 32 * s + lane;
-        undecided &= undecided - 1;
-        if (j >= clen) continue;  // padding
-        const Vec4<T> c = p.spos[index.record(s, le) + cbeg + j], a = p.tpos[t];
-        const T d = dist2<T>(a.x, a.y, a.z, c.x, c.y, c.z);
-        if (d <= p.r2 && d > (T)1e-8f) hits |= 1u << s;
-    }
-    return hits;
+    unsigned long long a = f32x2_add(d, lo);
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(f32x2_add(d, hi)));
+    push_signs(a, bits);
 }
 
+struct CountTests {
+    SignTest hit;                // single precision: decides; double: d decided to be a neighbour
+    SignTest may;                // double: d may be one
+    float2 middle;               // double: minus the middle of the undecided distances around the cutoff
+    float half;                  //         and their reach on both sides
+};
+// What a warp keeps of its group, in shared memory.
 struct CountGroup {
     uint32_t tb0, n0, tb1, ntot;   // targets of the two rows
     int cbeg, clen;                // chunk of the candidate list
-    bool write_masks, first, last;
+    int turn;                      // block of 64 that the first registers hold
+    float ylo, yhi, zlo, zhi;      // where a target's cell coordinates are clear of the faces of its rows
+    int write_masks, first, last, all_exact;
+    __device__ __forceinline__ uint32_t target(uint32_t k) const volatile { return k < n0 ? tb0 + k : tb1 + (k - n0); }
 };
-// The targets of a group against the chunk's candidates, at most 64 NB of them and more than 64 FULL.
-template <typename T, int NB, int FULL>
-__device__ __forceinline__ void count_group(const PairParams<T>& p, const RunIndex& index, const CountGroup& g, const SignTest& hit, const SignTest& may,
-                                            const bool all_undecided, int& max_degree, const int lane, const uint32_t le)
+struct CountWarp {
+    float4 target[COUNT_TARGETS][2];            // {x, x, y, y}, {z, z, entry, -}
+    unsigned short mask[COUNT_TARGETS][32];
+    RunIndex index;
+    CountGroup group;
+    int pad;
+};
+struct CountCells { float gmin_y, gmin_z, res_inv; };
+
+// The candidates of a target given by `which` (bit s: place 32 s + lane of the chunk) by the expression that decides.
+template <typename T>
+__device__ __forceinline__ uint32_t exact_hits(const Vec4<T>* spos, const Vec4<T>* target, const T r2, uint32_t which, const RunIndex& index, int cbeg, int clen,
+                                               int lane, uint32_t le)
 {
+    uint32_t hits = 0;
+    while (which) {
+        const int s = __ffs((int)which) - 1, j = 32 * s + lane;
+        which &= which - 1;
+        if (j >= clen) continue;  // padding
+        const Vec4<T> c = spos[index.record(s, le) + cbeg + j], a = *target;
+        const T d = dist2<T>(a.x, a.y, a.z, c.x, c.y, c.z);
+        if (d <= r2 && d > (T)1e-8f) hits |= 1u << s;
+    }
+    return hits;
+}
+// Out of line in double, where it is called for every target with an undecided candidate: the copies of the test loop overran the
+// instruction cache (176 us against 160, silicon of 500 k atoms).  In single precision the call costs more (207 against 224, liquid of 1 M).
+__device__ __noinline__ uint32_t exact_hits_call(const Vec4<double>* spos, const Vec4<double>* target, const double r2, uint32_t which, const RunIndex& index,
+                                                 int cbeg, int clen)
+{
+    const int lane = lane_id();
+    return exact_hits<double>(spos, target, r2, which, index, cbeg, clen, lane, 0xffffffffu >> (31 - lane));
+}
+
+// The targets of a group against the chunk's candidates, at most 64 NB of them.  FULL: both tests for all blocks.
+template <typename T, int NB, bool FULL>
+__device__ __forceinline__ void count_group(const PairParams<T>& p, CountWarp& w, const volatile CountCells& cells, const CountTests& test, int& max_degree, const int lane,
+                                            const uint32_t le)
+{
+    const volatile CountGroup& g = w.group;
+    constexpr int OWN = FULL ? NB : 2;
+    constexpr uint32_t ALL_BITS = 0xffffu >> (16 - 2 * NB);
     unsigned long long cx[NB], cy[NB], cz[NB];
     {
-        const float4* src = p.sscan + g.cbeg;
+        const float4* const src = p.sscan + g.cbeg;
+        int b0 = g.turn;
+        const int clen = g.clen;
+        const unsigned long long nothing = 0x8000000080000000ull;
 #pragma unroll
         for (int b = 0; b < NB; b++) {
             float4 v[2];
 #pragma unroll
             for (int i = 0; i < 2; i++) {
-                const int s = 2 * b + i;
-                if (b < FULL) {
-                    v[i] = src[index.record(s, le) + 32 * s + lane];
-                } else {
-                    // a padding place reads the last record; x alone keeps it out of every cutoff, its distance is infinite
-                    const int j = min(32 * s + lane, g.clen - 1);
-                    const uint2 f = index.word[j >> 5];
-                    v[i] = src[index.delta[(int)f.y + __popc(f.x & (0xffffffffu >> (31 - (j & 31))))] + j];
-                    if (32 * s + lane >= g.clen) v[i].x = 3.0e38f;
-                }
+                // a padding place reads the last record; x alone keeps it out of every cutoff, its distance is infinite
+                const int j = 64 * b0 + 32 * i + lane;
+                v[i] = src[w.index.record(2 * b0 + i, le) + min(j, clen - 1)];
+                if (j >= clen) v[i].x = 3.0e38f;
             }
-            cx[b] = f32x2_pack(v[0].x, v[1].x);
-            cy[b] = f32x2_pack(v[0].y, v[1].y);
-            cz[b] = f32x2_pack(v[0].z, v[1].z);
+            cx[b] = f32x2_kept(-v[0].x, -v[1].x, nothing);
+            cy[b] = f32x2_kept(-v[0].y, -v[1].y, nothing);
+            cz[b] = f32x2_kept(-v[0].z, -v[1].z, nothing);
+            b0 = b0 + 1 == NB ? 0 : b0 + 1;
         }
     }
-    int degree = 0;  // lane l collects the degree of target 32 j + l; stored 32 targets at a time
-    float4 next = p.tscan[g.n0 != 0 ? g.tb0 : g.tb1];  // w = entry
-    uint32_t at = g.n0 != 0 ? g.tb0 : g.tb1;
+    const unsigned long long upto = f32x2_load(sizeof(T) == 8 ? test.middle : test.hit.hi);
+    const int turn = 2 * (NB - g.turn);
 #pragma unroll 1
-    for (uint32_t k = 0; k < g.ntot;) {
-        const float4 t = next;
-        const uint32_t mine_at = at;
-        at = (k + 1 == g.n0) ? g.tb1 : at + 1;
-        if (k + 1 >= g.ntot) at = mine_at;
-        next = p.tscan[at];
-        const unsigned long long ax = f32x2_pack(t.x, t.x), ay = f32x2_pack(t.y, t.y), az = f32x2_pack(t.z, t.z);
-        uint32_t bits = 0, maybe = 0;
-#pragma unroll
-        for (int b = NB - 1; b >= 0; b--) {
-            const unsigned long long d = dist2_x2(ax, ay, az, cx[b], cy[b], cz[b]);
-            test_x2(d, hit, bits);
-            if (sizeof(T) == 8) test_x2(d, may, maybe);
-        }
-        if constexpr (sizeof(T) == 8)
-            bits |= exact_hits<T>(p, mine_at, (all_undecided ? 0xffffu >> (16 - 2 * NB) : maybe) & ~bits, index, g.cbeg, g.clen, lane, le);
-        if (g.write_masks) p.hitmask[(size_t)mine_at * 32 + lane] = (unsigned short)bits;
-        int n = __reduce_add_sync(0xffffffffu, __popc(bits));
-        if (!g.first) n += (int)p.tcount[mine_at];
-        if (lane == (int)(k & 31u)) degree = n;
-        k++;
-        if ((k & 31u) == 0u || k == g.ntot) {
+    for (uint32_t k0 = 0; k0 < g.ntot; k0 += COUNT_TARGETS) {
+        const int n = (int)min(g.ntot - k0, (uint32_t)COUNT_TARGETS);
+        uint32_t again = 0;   // targets to be tested again in full
+        {
+            const float4 v = p.tscan[g.target(k0 + min(lane, n - 1))];   // w = entry
             __syncwarp();
-            const uint32_t mine = ((k - 1) & ~31u) + (uint32_t)lane;
-            if (mine < k) {
-                const uint32_t to = (mine < g.n0) ? g.tb0 + mine : g.tb1 + (mine - g.n0);
-                p.tcount[to] = (uint32_t)degree;
-                if (g.last) {
-                    if (p.counts_out != nullptr) p.counts_out[__float_as_int(p.tscan[to].w)] = degree;  // in caller order
-                    max_degree = max(max_degree, degree);
+            if (lane < n) {
+                w.target[lane][0] = make_float4(v.x, v.x, v.y, v.y);
+                w.target[lane][1] = make_float4(v.z, v.z, v.w, 0.0f);
+            }
+            const float fy = (v.y - cells.gmin_y) * cells.res_inv, fz = (v.z - cells.gmin_z) * cells.res_inv;
+            const bool clear = fy > g.ylo && fy < g.yhi && fz > g.zlo && fz < g.zhi;
+            again = __ballot_sync(0xffffffffu, lane < n && (g.all_exact || (!FULL && !clear)));
+            __syncwarp();
+        }
+#pragma unroll 1
+        for (int k = 0; k < n; k++) {
+            const ulonglong2 axy = *reinterpret_cast<const ulonglong2*>(&w.target[k][0]);
+            const unsigned long long az = *reinterpret_cast<const unsigned long long*>(&w.target[k][1]);
+            uint32_t bits = 0, maybe = 0;
+            float closest = INFINITY;
+            const unsigned long long lo = f32x2_load(test.hit.lo);
+            unsigned long long hi = 0, may_lo = 0, may_hi = 0;
+            if (sizeof(T) == 8) {
+                hi = f32x2_load(test.hit.hi);
+                may_lo = f32x2_load(test.may.lo);
+                may_hi = f32x2_load(test.may.hi);
+            }
+#pragma unroll
+            for (int b = NB - 1; b >= 0; b--) {
+                const unsigned long long d = dist2_x2(axy.x, axy.y, az, cx[b], cy[b], cz[b]);
+                if (b < OWN) {
+                    test_x2(d, lo, sizeof(T) == 8 ? hi : upto, bits);
+                    if (sizeof(T) == 8) test_x2(d, may_lo, may_hi, maybe);
+                } else {
+                    const unsigned long long a = f32x2_add(d, upto);
+                    push_signs(a, bits);
+                    if (sizeof(T) == 8) {
+                        float a0, a1;
+                        asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
+                        asm("min.f32 %0, %0, %1, %2;" : "+f"(closest) : "f"(fabsf(a0)), "f"(fabsf(a1)));
+                    }
                 }
             }
+            // bit 2 b + i of the registers is bit 2 (b + turn mod NB) + i of the list
+            auto turned = [&](uint32_t v) { return ((v | (v << (2 * NB))) >> turn) & ALL_BITS; };
+            bits = turned(bits);
+            if constexpr (sizeof(T) == 8) {
+                if (!g.all_exact) {
+                    const uint32_t undecided = turned(maybe) & ~bits & turned(0xffffu >> (16 - 2 * OWN));
+                    if (undecided) bits |= exact_hits_call(p.spos, p.tpos + g.target(k0 + k), p.r2, undecided, w.index, g.cbeg, g.clen);
+                }
+                if (!FULL && closest <= test.half) again |= 1u << k;
+            }
+            w.mask[k][lane] = (unsigned short)bits;
+        }
+        __syncwarp();
+        if (sizeof(T) == 8) again = __reduce_or_sync(0xffffffffu, again);
+#pragma unroll 1
+        for (; again; again &= again - 1) {
+            const int k = __ffs((int)again) - 1;
+            uint32_t bits;
+            if constexpr (sizeof(T) == 8) bits = exact_hits_call(p.spos, p.tpos + g.target(k0 + k), p.r2, ALL_BITS, w.index, g.cbeg, g.clen);
+            else bits = exact_hits<T>(p.spos, p.tpos + g.target(k0 + k), p.r2, ALL_BITS, w.index, g.cbeg, g.clen, lane, le);
+            w.mask[k][lane] = (unsigned short)bits;
             __syncwarp();
         }
+        // degrees, and the bits to memory: four lanes a target
+#pragma unroll 1
+        for (int i0 = 0; i0 < 4 * n; i0 += 32) {
+            const int i = i0 + lane, k = min(i >> 2, n - 1);
+            const uint4 m = reinterpret_cast<const uint4*>(w.mask[k])[i & 3];
+            const uint32_t t = g.target(k0 + k);
+            int degree = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+            degree += __shfl_xor_sync(0xffffffffu, degree, 1);
+            degree += __shfl_xor_sync(0xffffffffu, degree, 2);
+            if (i < 4 * n) {
+                if (g.write_masks) reinterpret_cast<uint4*>(p.hitmask + (size_t)t * 32)[i & 3] = m;
+                if ((i & 3) == 0) {
+                    if (!g.first) degree += (int)p.tcount[t];
+                    p.tcount[t] = (uint32_t)degree;
+                    if (g.last) {
+                        if (p.counts_out != nullptr) p.counts_out[__float_as_int(w.target[k][1].z)] = degree;  // in caller order
+                        max_degree = max(max_degree, degree);
+                    }
+                }
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -1172,75 +1283,114 @@ template <typename T>
 __global__ void __launch_bounds__(COUNT_WARPS * 32, COUNT_BLOCKS)
 rg_count_kernel(const PairParams<T> p)
 {
-    __shared__ RunIndex indexes[COUNT_WARPS];
-    const int lane = lane_id(), warp = threadIdx.x >> 5;
-    RunIndex& index = indexes[warp];
-    const uint32_t lt = lanemask_lt(), le = lt | (1u << lane);
+    __shared__ CountWarp warps[COUNT_WARPS];
     __shared__ GroupShape shape;
+    __shared__ CountCells cells;
+    __shared__ CountTests test;
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    CountWarp& w = warps[warp];
+    const uint32_t lt = lanemask_lt(), le = lt | (1u << lane);
     DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
     int warp_max_slots = 0, max_degree = 0;
-    if (threadIdx.x == 0) shape = group_shape(hp);
+    if (threadIdx.x == 0) {
+        shape = group_shape(hp);
+        // double positions are scanned relative to the grid's origin
+        cells.gmin_y = sizeof(T) == 8 ? 0.0f : (float)hp->gmin[1];
+        cells.gmin_z = sizeof(T) == 8 ? 0.0f : (float)hp->gmin[2];
+        cells.res_inv = (float)hp->res_inv;
+    }
+    if (threadIdx.x == 32) {
+        test.hit = sizeof(T) == 8 ? sign_test(hp->test_near, hp->test_lo) : sign_test(1e-8f, (float)p.r2);
+        test.may = sizeof(T) == 8 ? sign_test(hp->test_equal_is_near ? 0.0f : -1.0f, hp->test_hi) : test.hit;
+        const float middle = 0.5f * (hp->test_lo + hp->test_hi);
+        test.middle = make_float2(-middle, -middle);
+        test.half = 1.001f * fmaxf(middle - hp->test_lo, hp->test_hi - middle);
+    }
     const uint32_t num_groups = p.glist ? hp->active_groups : (uint32_t)hp->num_groups;  // < 2^31: never more groups than cells
     __syncthreads();
     const int lane_run = group_lane_run(shape, lane);
-    const SignTest hit = sizeof(T) == 8 ? sign_test(hp->test_near, hp->test_lo) : sign_test(1e-8f, (float)p.r2);
-    const SignTest may = sizeof(T) == 8 ? sign_test(hp->test_equal_is_near ? 0.0f : -1.0f, hp->test_hi) : hit;
-    const bool all_undecided = sizeof(T) == 8 && hp->test_lo < 0.0f;  // coordinates out of the float test's range (float_test)
+    const bool all_exact = sizeof(T) == 8 && hp->test_lo < 0.0f;  // coordinates out of the float test's range (float_test)
+    // Records within the self-distance limit of a target (1e-4, or what the float test calls near) lie in the target's cell row
+    // but for targets this close to its faces, in cells: the distance, and the rounding of the two cell coordinates.
+    const float skin = 1.01f * sqrtf(sizeof(T) == 8 ? hp->test_near : 1e-8f) * (float)hp->res_inv + 1e-6f * (float)(16 + max(hp->ny, hp->nz));
 
     const uint32_t nwarps = gridDim.x * COUNT_WARPS;
+    uint32_t gi = blockIdx.x * COUNT_WARPS + warp;
 #pragma unroll 1
-    for (uint32_t gi = blockIdx.x * COUNT_WARPS + warp; gi < num_groups; gi += nwarps) {
+    while (gi < num_groups) {
         const uint32_t grp = p.glist ? p.glist[gi] : gi;
+        uint32_t following = 0;
+        if (lane == 0) following = nwarps + atomicAdd(&hp->count_next, 1u);
         const GroupDesc d = fetch_group(shape, p.tcstart, p.cstart, grp, lane_run);
         const int run_a = d.run_a, run_len = d.run_e - d.run_a;
-        CountGroup g;
-        g.tb0 = d.tb0;
-        g.tb1 = d.tb1;
-        g.n0 = d.te0 - d.tb0;
-        g.ntot = g.n0 + (d.te1 - d.tb1);
-        if (g.ntot == 0) continue;
-        const int run_end = (int)warp_incl_scan_u32((uint32_t)run_len), run_off = run_end - run_len, L = __shfl_sync(0xffffffffu, run_end, 31);
-        const int nslots = (L + 31) >> 5;
-        g.write_masks = nslots <= RG_MASK_SLOTS;
-        warp_max_slots = max(warp_max_slots, nslots);
-        if (nslots > RG_MASK_SLOTS && lane == 0) p.long_list[atomicAdd(reinterpret_cast<uint32_t*>(&hp->reserved[1]), 1u)] = grp;
-#pragma unroll 1
-        for (g.cbeg = 0; g.cbeg < L; g.cbeg += RG_MASK_SLOTS * 32) {
-            g.clen = min(RG_MASK_SLOTS * 32, L - g.cbeg);
-            g.first = g.cbeg == 0;
-            g.last = g.cbeg + RG_MASK_SLOTS * 32 >= L;
+        volatile CountGroup& g = w.group;   // all lanes write the same
+        const uint32_t n0 = d.te0 - d.tb0, ntot = n0 + (d.te1 - d.tb1);
+        if (ntot != 0) {
             __syncwarp();
-            index.set(run_a, run_off, run_len, g.cbeg, lane, lt);
-            auto run = [&](auto nb, auto full) {
-                count_group<T, decltype(nb)::value, decltype(full)::value>(p, index, g, hit, may, all_undecided, max_degree, lane, le);
-            };
-            // copies of the test loop for 2, 4, 5, 6, 7 and 8 blocks of 64; one block is tested as two and three as four, with padding
-            switch ((g.clen + 63) >> 6) {
-            case 1:
-            case 2: run(std::integral_constant<int, 2>(), std::integral_constant<int, 0>()); break;
-            case 3:
-            case 4: run(std::integral_constant<int, 4>(), std::integral_constant<int, 2>()); break;
-            case 5: run(std::integral_constant<int, 5>(), std::integral_constant<int, 4>()); break;
-            case 6: run(std::integral_constant<int, 6>(), std::integral_constant<int, 5>()); break;
-            case 7: run(std::integral_constant<int, 7>(), std::integral_constant<int, 6>()); break;
-            default: run(std::integral_constant<int, 8>(), std::integral_constant<int, 7>()); break;
+            g.tb0 = d.tb0;
+            g.tb1 = d.tb1;
+            g.n0 = n0;
+            g.ntot = ntot;
+            const int run_end = (int)warp_incl_scan_u32((uint32_t)run_len), run_off = run_end - run_len, L = __shfl_sync(0xffffffffu, run_end, 31);
+            const int nslots = (L + 31) >> 5;
+            g.write_masks = nslots <= RG_MASK_SLOTS;
+            g.all_exact = all_exact;
+            warp_max_slots = max(warp_max_slots, nslots);
+            if (nslots > RG_MASK_SLOTS && lane == 0) p.long_list[atomicAdd(reinterpret_cast<uint32_t*>(&hp->reserved[1]), 1u)] = grp;
+            g.ylo = (float)d.cy0 + skin;
+            g.yhi = (float)(d.cy1 + 1) - skin;
+            g.zlo = (float)d.cz + skin;
+            g.zhi = (float)(d.cz + 1) - skin;
+            int own_beg, own_end;
+            {
+                // the runs that hold the targets' own rows
+                const volatile GroupShape& f = shape;
+                const int own = f.pad * (f.sy + 2 * f.pad) + f.pad;
+                own_beg = __shfl_sync(0xffffffffu, run_off, own);
+                own_end = __shfl_sync(0xffffffffu, run_end, own + d.cy1 - d.cy0);
             }
+#pragma unroll 1
+            for (int cbeg = 0; cbeg < L; cbeg += RG_MASK_SLOTS * 32) {
+                const int clen = min(RG_MASK_SLOTS * 32, L - cbeg);
+                // both tests everywhere where the own records are not in two blocks, and in lists of several chunks
+                const bool everywhere = L > RG_MASK_SLOTS * 32 || ((own_end - 1) >> 6) - (own_beg >> 6) > 1;
+                __syncwarp();
+                g.cbeg = cbeg;
+                g.clen = clen;
+                g.first = cbeg == 0;
+                g.last = cbeg + RG_MASK_SLOTS * 32 >= L;
+                g.turn = everywhere ? 0 : own_beg >> 6;
+                w.index.set(run_a, run_off, run_len, cbeg, lane, lt);
+                auto run = [&](auto nb, auto full) {
+                    count_group<T, decltype(nb)::value, decltype(full)::value>(p, w, cells, test, max_degree, lane, le);
+                };
+                // Copies of the test loop for 2, 4, 5, 6, 7 and 8 blocks of 64; one block is tested as two and three as four, with
+                // padding
+                if (everywhere) {
+                    run(std::integral_constant<int, 8>(), std::true_type());
+                } else {
+                    switch ((clen + 63) >> 6) {
+                    case 1:
+                    case 2: run(std::integral_constant<int, 2>(), std::false_type()); break;
+                    case 3:
+                    case 4: run(std::integral_constant<int, 4>(), std::false_type()); break;
+                    case 5: run(std::integral_constant<int, 5>(), std::false_type()); break;
+                    case 6: run(std::integral_constant<int, 6>(), std::false_type()); break;
+                    case 7: run(std::integral_constant<int, 7>(), std::false_type()); break;
+                    default: run(std::integral_constant<int, 8>(), std::false_type()); break;
+                    }
+                }
+            }
+            // a group whose neighbourhood holds no source at all still owes its targets a zero
+            if (L == 0)
+                for (uint32_t k = lane; k < ntot; k += 32) p.tcount[g.target(k)] = 0;
         }
-        // a group whose neighbourhood holds no source at all still owes its targets a zero
-        if (L == 0)
-            for (uint32_t k = lane; k < g.ntot; k += 32) p.tcount[(k < g.n0) ? g.tb0 + k : g.tb1 + (k - g.n0)] = 0;
+        gi = __shfl_sync(0xffffffffu, following, 0);
     }
-    {   // largest degree: one atomic per block
-        __shared__ int s_max_degree;
-        if (threadIdx.x == 0) s_max_degree = 0;
-        __syncthreads();
-        max_degree = __reduce_max_sync(0xffffffffu, max_degree);
-        if (lane == 0 && max_degree > 0) atomicMax(&s_max_degree, max_degree);
-        __syncthreads();
-        if (threadIdx.x == 0 && s_max_degree > 0) atomicMax(&hp->max_degree, (uint32_t)s_max_degree);
-    }
-    // a candidate list too long for the hit bits: the edge writer has to recompute distances
+    // largest degree; a candidate list too long for the hit bits: the edge writer has to recompute distances
+    max_degree = __reduce_max_sync(0xffffffffu, max_degree);
+    if (lane == 0 && max_degree > (int)__ldcg(&hp->max_degree)) atomicMax(&hp->max_degree, (uint32_t)max_degree);
     if (lane == 0 && warp_max_slots > RG_MASK_SLOTS) atomicMax(&hp->reserved[0], (long long)warp_max_slots);
 }
 
@@ -2504,7 +2654,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         rg_group_list_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, tcfill);
     // there are no more groups than cells, and with a target subset no more of interest than targets
     const int64_t most_groups = std::min(host_grid ? (int64_t)gc_host.ncell_plus1 : cell_cap, targets != nullptr ? Nt : cell_cap);
-    const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * COUNT_BLOCKS * COUNT_WAVES, (most_groups + COUNT_WARPS - 1) / COUNT_WARPS);
+    const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * COUNT_BLOCKS, (most_groups + COUNT_WARPS - 1) / COUNT_WARPS);
     rg_count_kernel<T><<<grid, COUNT_WARPS * 32, 0, stream>>>(pp_host);
     DYNB_CUDA_OK((exclusive_scan<uint32_t, long long>(tcount, toffset, nullptr, Nt + 1, sums64,
                                                        reinterpret_cast<long long*>(&h->E), stream,
