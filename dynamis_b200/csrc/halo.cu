@@ -22,9 +22,10 @@ namespace dynb {
 
 // ------------------------------------------------------------------------------------------ bincount / select
 __global__ void __launch_bounds__(256)
-bincount_i64_kernel(const int64_t* __restrict__ a, int64_t n, int64_t W, unsigned long long* __restrict__ counts,
-                    uint32_t* __restrict__ bad)
+bincount_i64_kernel(const int64_t* a, int64_t n, int64_t W, unsigned long long* counts,
+                    uint32_t* bad)
 {
+    chain_begin();
     extern __shared__ uint32_t hist[];
     const bool use_smem = W <= 4096;
     if (use_smem) {
@@ -52,8 +53,9 @@ constexpr int SELECT_TILE = 2048;
 constexpr int64_t SELECT_FUSED_MAX_TILES = 8192;
 
 __global__ void __launch_bounds__(256)
-select_count_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, uint32_t* __restrict__ tile_count)
+select_count_kernel(const int64_t* a, int64_t n, int64_t value, uint32_t* tile_count)
 {
+    chain_begin();
     __shared__ uint32_t wsum[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t base = (int64_t)blockIdx.x * SELECT_TILE + warp * 256 + lane;
@@ -75,9 +77,10 @@ select_count_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, uin
 
 template <bool SUMMED>   // tile_count holds the matches in front of each tile already
 __global__ void __launch_bounds__(256)
-select_fill_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, const uint32_t* __restrict__ tile_count,
-                   const int64_t* __restrict__ gather_src, int64_t* __restrict__ out, int64_t* __restrict__ count_out)
+select_fill_kernel(const int64_t* a, int64_t n, int64_t value, const uint32_t* tile_count,
+                   const int64_t* gather_src, int64_t* out, int64_t* count_out)
 {
+    chain_begin();
     __shared__ uint32_t wsum[8], before[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t base = (int64_t)blockIdx.x * SELECT_TILE + warp * 256 + lane;
@@ -119,11 +122,12 @@ select_fill_kernel(const int64_t* __restrict__ a, int64_t n, int64_t value, cons
 // owned by a peer p, that peer must send src to me (recv side) and I must send dst to p (send
 // side, by the symmetry of the radius graph).
 __global__ void __launch_bounds__(256)
-halo_mark_edges_kernel(const int64_t* __restrict__ src, const int64_t* __restrict__ dst, int64_t E,
-                       const int64_t* __restrict__ pid, int64_t N, int64_t my_rank, int words,
-                       uint32_t* __restrict__ send_mask, uint32_t* __restrict__ recv_mask,
-                       uint8_t* __restrict__ has_remote, uint32_t* __restrict__ bad)
+halo_mark_edges_kernel(const int64_t* src, const int64_t* dst, int64_t E,
+                       const int64_t* pid, int64_t N, int64_t my_rank, int words,
+                       uint32_t* send_mask, uint32_t* recv_mask,
+                       uint8_t* has_remote, uint32_t* bad)
 {
+    chain_begin();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= E) return;
     const int64_t s = src[e], d = dst[e];
@@ -211,8 +215,9 @@ __device__ __forceinline__ uint32_t halo_count_sets(uint32_t set, int lane)
 
 // rows of bsum (nblocks entries each): send peers 0..W-1, recv peers 0..W-1, own atoms
 __global__ void __launch_bounds__(HL_THREADS)
-halo_lists_count_kernel(const HaloSets h, int W, int nblocks, uint32_t* __restrict__ bsum)
+halo_lists_count_kernel(const HaloSets h, int W, int nblocks, uint32_t* bsum)
 {
+    chain_begin();
     __shared__ uint32_t ws[HL_WARPS][2][32];
     __shared__ uint32_t wown[HL_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -247,9 +252,10 @@ halo_lists_count_kernel(const HaloSets h, int W, int nblocks, uint32_t* __restri
 // One block per row: exclusive scan of the row of block sums (in place) and its total; the block that finishes last turns
 // the totals into offsets [send W + 1 | recv W + 1 | number of own atoms].
 __global__ void __launch_bounds__(SCAN_THREADS)
-halo_lists_scan_kernel(uint32_t* __restrict__ bsum, int nblocks, int W, int64_t* __restrict__ totals, uint32_t* __restrict__ arrived,
-                       int64_t* __restrict__ offsets)
+halo_lists_scan_kernel(uint32_t* bsum, int nblocks, int W, int64_t* totals, uint32_t* arrived,
+                       int64_t* offsets)
 {
+    chain_begin();
     __shared__ uint32_t warp_sums[SCAN_THREADS / 32];
     __shared__ bool last;
     uint32_t* row = bsum + (int64_t)blockIdx.x * nblocks;
@@ -299,9 +305,10 @@ struct HaloListsOut {
 };
 
 __global__ void __launch_bounds__(HL_THREADS)
-halo_lists_fill_kernel(const HaloSets h, int W, int nblocks, const uint32_t* __restrict__ bsum, const int64_t* __restrict__ offsets,
+halo_lists_fill_kernel(const HaloSets h, int W, int nblocks, const uint32_t* bsum, const int64_t* offsets,
                        const HaloListsOut out)
 {
+    chain_begin();
     __shared__ uint32_t ws[HL_WARPS][2][32];
     __shared__ uint32_t wown[HL_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -463,15 +470,17 @@ csr_fill_kernel(const uint32_t* __restrict__ mask, int words, const int64_t* __r
 }
 
 __global__ void __launch_bounds__(256)
-gather_not_u8_kernel(const uint8_t* __restrict__ flags, const int64_t* __restrict__ idx, int64_t n, uint8_t* __restrict__ out)
+gather_not_u8_kernel(const uint8_t* flags, const int64_t* idx, int64_t n, uint8_t* out)
 {
+    chain_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = flags[idx[i]] ? 0 : 1;
 }
 
 __global__ void __launch_bounds__(256)
-scatter_iota_kernel(const int64_t* __restrict__ idx, int64_t n, int64_t N, int64_t* __restrict__ g2l, uint32_t* __restrict__ bad)
+scatter_iota_kernel(const int64_t* idx, int64_t n, int64_t N, int64_t* g2l, uint32_t* bad)
 {
+    chain_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t a = idx[i];
@@ -493,10 +502,11 @@ constexpr int FILTER_TILE = 256 * FILTER_ROUNDS;       // 32 words of 32 edges
 static_assert(FILTER_TILE == 1024, "a warp reads a tile's words in one load");
 
 __global__ void __launch_bounds__(256)
-edge_keep_bits_kernel(const int64_t* __restrict__ src, const int64_t* __restrict__ dst, const float* __restrict__ shifts,
-                      const float* __restrict__ pos, Cell9 cell, float r2, int64_t E, uint32_t* __restrict__ bits,
-                      uint32_t* __restrict__ tile_count)
+edge_keep_bits_kernel(const int64_t* src, const int64_t* dst, const float* shifts,
+                      const float* pos, Cell9 cell, float r2, int64_t E, uint32_t* bits,
+                      uint32_t* tile_count)
 {
+    chain_begin();
     __shared__ uint32_t warp_count[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t e0 = (int64_t)blockIdx.x * FILTER_TILE + threadIdx.x;
@@ -540,10 +550,11 @@ edge_keep_bits_kernel(const int64_t* __restrict__ src, const int64_t* __restrict
 }
 
 __global__ void __launch_bounds__(256)
-edge_compact_kernel(const int64_t* __restrict__ edges, const unsigned char* __restrict__ shifts_raw, int shift_row_bytes,
-                    const uint32_t* __restrict__ bits, const long long* __restrict__ tile_first, int64_t E, int64_t E_out,
-                    int64_t* __restrict__ edges_out, unsigned char* __restrict__ shifts_out)
+edge_compact_kernel(const int64_t* edges, const unsigned char* shifts_raw, int shift_row_bytes,
+                    const uint32_t* bits, const long long* tile_first, int64_t E, int64_t E_out,
+                    int64_t* edges_out, unsigned char* shifts_out)
 {
+    chain_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t mine = bits[(int64_t)blockIdx.x * 32 + lane];
     int total;
@@ -598,7 +609,7 @@ extern "C" int dynb_bincount_i64(const int64_t* a_dev, int64_t n, int64_t W, int
     if (n == 0) return DYNB_OK;
     const int grid = (int)std::min<int64_t>(nblk(n), (int64_t)sm_count_cached() * 8);
     const size_t smem = W <= 4096 ? (size_t)W * 4 : 0;
-    bincount_i64_kernel<<<grid, 256, smem, s>>>(a_dev, n, W, reinterpret_cast<unsigned long long*>(counts_dev), bad_dev);
+    launch_chained(bincount_i64_kernel, grid, 256, smem, s, a_dev, n, W, reinterpret_cast<unsigned long long*>(counts_dev), bad_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -627,14 +638,14 @@ extern "C" int dynb_select_eq_i64(const int64_t* a_dev, int64_t n, int64_t value
     if (workspace_dev == nullptr || workspace_bytes < need) return fail_arg("workspace too small (see dynb_select_workspace_bytes)");
     uint32_t* tile_count = static_cast<uint32_t*>(workspace_dev);
     const unsigned tiles = nblk(n, SELECT_TILE);
-    select_count_kernel<<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count);
+    launch_chained(select_count_kernel, tiles, 256, 0, s, a_dev, n, value, tile_count);
     if (tiles <= SELECT_FUSED_MAX_TILES) {
-        select_fill_kernel<false><<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count, gather_src_dev, out_dev, count_dev);
+        launch_chained(select_fill_kernel<false>, tiles, 256, 0, s, a_dev, n, value, tile_count, gather_src_dev, out_dev, count_dev);
     } else {
         uint32_t* sums = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace_dev) + select_sums_at(n));
         DYNB_CUDA_OK(cudaMemsetAsync(count_dev, 0, 8, s));
         DYNB_CUDA_OK((exclusive_scan<uint32_t, uint32_t>(tile_count, tile_count, nullptr, tiles, sums, reinterpret_cast<uint32_t*>(count_dev), s)));
-        select_fill_kernel<true><<<tiles, 256, 0, s>>>(a_dev, n, value, tile_count, gather_src_dev, out_dev, count_dev);
+        launch_chained(select_fill_kernel<true>, tiles, 256, 0, s, a_dev, n, value, tile_count, gather_src_dev, out_dev, count_dev);
     }
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
@@ -652,7 +663,7 @@ extern "C" int dynb_halo_mark_from_edges(const int64_t* edges_dev, int64_t E, co
     DYNB_CUDA_OK(cudaMemsetAsync(has_remote_dev, 0, (size_t)N, s));
     DYNB_CUDA_OK(cudaMemsetAsync(bad_dev, 0, 4, s));
     if (E == 0) return DYNB_OK;
-    halo_mark_edges_kernel<<<nblk(E), 256, 0, s>>>(edges_dev, edges_dev + E, E, pid_dev, N, my_rank, words, send_mask_dev,
+    launch_chained(halo_mark_edges_kernel, nblk(E), 256, 0, s, edges_dev, edges_dev + E, E, pid_dev, N, my_rank, words, send_mask_dev,
                                                    recv_mask_dev, has_remote_dev, bad_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
@@ -699,8 +710,8 @@ extern "C" int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_
     int64_t* totals = reinterpret_cast<int64_t*>(ws + align_up((int64_t)nb * (2 * W + 1) * 4, 256));
     uint32_t* arrived = reinterpret_cast<uint32_t*>(ws + need - 256);
     DYNB_CUDA_OK(cudaMemsetAsync(arrived, 0, 4, s));
-    halo_lists_count_kernel<<<nb, HL_THREADS, 0, s>>>(h, (int)W, nb, bsum);
-    halo_lists_scan_kernel<<<(unsigned)(2 * W + 1), SCAN_THREADS, 0, s>>>(bsum, nb, (int)W, totals, arrived, offsets_dev);
+    launch_chained(halo_lists_count_kernel, nb, HL_THREADS, 0, s, h, (int)W, nb, bsum);
+    launch_chained(halo_lists_scan_kernel, (unsigned)(2 * W + 1), SCAN_THREADS, 0, s, bsum, nb, (int)W, totals, arrived, offsets_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -720,7 +731,7 @@ extern "C" int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_
         return fail_arg("null pointer");
     const HaloListsOut out{value_map_dev, has_foreign_dev, send_local_dev, recv_atom_dev, recv_ghost_dev, interior_dev, matrix_row_dev, n_local};
     const int nb = hl_blocks(n);
-    halo_lists_fill_kernel<<<nb, HL_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(h, (int)W, nb, static_cast<const uint32_t*>(workspace_dev),
+    launch_chained(halo_lists_fill_kernel, nb, HL_THREADS, 0, static_cast<cudaStream_t>(stream), h, (int)W, nb, static_cast<const uint32_t*>(workspace_dev),
                                                                                    offsets_dev, out);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
@@ -781,7 +792,7 @@ extern "C" int dynb_gather_not_u8(const uint8_t* flags_dev, const int64_t* idx_d
 {
     if (n < 0) return fail_arg("bad arguments");
     if (n == 0) return DYNB_OK;
-    gather_not_u8_kernel<<<nblk(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(flags_dev, idx_dev, n, out_dev);
+    launch_chained(gather_not_u8_kernel, nblk(n), 256, 0, static_cast<cudaStream_t>(stream), flags_dev, idx_dev, n, out_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -790,7 +801,7 @@ extern "C" int dynb_scatter_iota(const int64_t* idx_dev, int64_t n, int64_t N, i
 {
     if (n < 0 || N < 0) return fail_arg("bad arguments");
     if (n == 0) return DYNB_OK;
-    scatter_iota_kernel<<<nblk(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(idx_dev, n, N, g2l_dev, bad_dev);
+    launch_chained(scatter_iota_kernel, nblk(n), 256, 0, static_cast<cudaStream_t>(stream), idx_dev, n, N, g2l_dev, bad_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -818,7 +829,7 @@ extern "C" int dynb_filter_edges_plan(const int64_t* edges_dev, const float* shi
     Cell9 c;
     for (int i = 0; i < 9; i++) c.c[i] = cell_host[i];
     const float r2 = static_cast<float>(radius * radius);  // dist_graph_ops_kernels.cu:84
-    edge_keep_bits_kernel<<<(unsigned)L.tiles, 256, 0, s>>>(edges_dev, edges_dev + E, shifts_f32_dev, pos_dev, c, r2, E, bits, count);
+    launch_chained(edge_keep_bits_kernel, (unsigned)L.tiles, 256, 0, s, edges_dev, edges_dev + E, shifts_f32_dev, pos_dev, c, r2, E, bits, count);
     DYNB_CUDA_OK((exclusive_scan<uint32_t, long long>(count, reinterpret_cast<long long*>(ws + L.first), nullptr, L.tiles,
                                                        reinterpret_cast<long long*>(ws + L.sums), reinterpret_cast<long long*>(count_dev), s)));
     DYNB_CUDA_OK(cudaGetLastError());
@@ -833,8 +844,7 @@ extern "C" int dynb_filter_edges_fill(const int64_t* edges_dev, const void* shif
     if (E == 0 || E_out == 0) return DYNB_OK;
     const unsigned char* ws = static_cast<const unsigned char*>(workspace_dev);
     const FilterLayout L = filter_layout(E);
-    edge_compact_kernel<<<(unsigned)L.tiles, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        edges_dev, static_cast<const unsigned char*>(shifts_raw_dev), shift_row_bytes, reinterpret_cast<const uint32_t*>(ws + L.bits),
+    launch_chained(edge_compact_kernel, (unsigned)L.tiles, 256, 0, static_cast<cudaStream_t>(stream), edges_dev, static_cast<const unsigned char*>(shifts_raw_dev), shift_row_bytes, reinterpret_cast<const uint32_t*>(ws + L.bits),
         reinterpret_cast<const long long*>(ws + L.first), E, E_out, edges_out_dev,
         static_cast<unsigned char*>(shifts_out_dev));
     DYNB_CUDA_OK(cudaGetLastError());

@@ -51,9 +51,10 @@ __device__ __forceinline__ void kd_child_sizes(const KdSeg& g, long long sz, lon
 // starts[s] = atoms in segments before s (sorted order puts segments in id order); `reset` boxes emptied.  With thresholds
 // (equal counts) also the cuts: 1 + atoms in front of the cut, in sorted order, and the sizes of the next level's segments.
 __global__ void __launch_bounds__(256)
-kd_level_init_kernel(int S, const KdSeg* __restrict__ seg, const long long* __restrict__ seg_size, long long* __restrict__ seg_start,
-                     uint32_t* __restrict__ box, int reset, long long* __restrict__ next_size, long long* __restrict__ thresholds)
+kd_level_init_kernel(int S, const KdSeg* seg, const long long* seg_size, long long* seg_start,
+                     uint32_t* box, int reset, long long* next_size, long long* thresholds)
 {
+    chain_begin();
     if (threadIdx.x == 0) {
         long long acc = 0;
         for (int s = 0; s < S; s++) { seg_start[s] = acc; acc += seg_size[s]; }
@@ -104,8 +105,9 @@ struct KdBoxes {
 };
 
 __global__ void __launch_bounds__(256)
-kd_bbox_kernel(const float* __restrict__ pos, const int32_t* __restrict__ seg_id, int64_t n, int S, uint32_t* __restrict__ box)
+kd_bbox_kernel(const float* pos, const int32_t* seg_id, int64_t n, int S, uint32_t* box)
 {
+    chain_begin();
     __shared__ KdBoxes boxes;
     boxes.begin(S);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -127,9 +129,10 @@ __device__ __forceinline__ int kd_axis(const uint32_t* __restrict__ box, int s)
 }
 
 __global__ void __launch_bounds__(256)
-kd_keys_kernel(const float* __restrict__ pos, const int32_t* __restrict__ seg_id, int64_t n, const uint32_t* __restrict__ box,
-               uint64_t* __restrict__ keys, uint32_t* __restrict__ vals)
+kd_keys_kernel(const float* pos, const int32_t* seg_id, int64_t n, const uint32_t* box,
+               uint64_t* keys, uint32_t* vals)
 {
+    chain_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int s = seg_id[i];
@@ -191,10 +194,11 @@ kd_assign_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__
 // its two loads (10 us for a million atoms); a launch for each of the two, for the sizes of the cuts and for every level's
 // part of the tree made the call of a million atoms on 8 ranks 305 us instead of 278.
 __global__ void __launch_bounds__(256)
-kd_assign_select_kernel(const float* __restrict__ pos, const uint64_t* __restrict__ keys, int64_t n, int idx_bits, const SelSplit* __restrict__ cut,
-                        const KdSeg* __restrict__ seg, int32_t* __restrict__ new_seg_id, int S, uint32_t* __restrict__ box,
-                        const int64_t* __restrict__ base_label, int64_t* __restrict__ labels)
+kd_assign_select_kernel(const float* pos, const uint64_t* keys, int64_t n, int idx_bits, const SelSplit* cut,
+                        const KdSeg* seg, int32_t* new_seg_id, int S, uint32_t* box,
+                        const int64_t* base_label, int64_t* labels)
 {
+    chain_begin();
     __shared__ KdBoxes boxes;
     if (S > 0) boxes.begin(S);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -341,19 +345,19 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
         const int S = (int)(first[l + 1] - first[l]), S_next = l + 1 < levels ? (int)(first[l + 2] - first[l + 1]) : 0;
         const KdSeg* level_tree = tree + first[l];
         if (l == 0 || !by_selection) {
-            kd_level_init_kernel<<<1, 256, 0, s>>>(S, nullptr, size_cur, start, box, S, nullptr, nullptr);
-            kd_bbox_kernel<<<grid_stride, 256, 0, s>>>(pos_dev, seg_cur, n, S, box);
+            launch_chained(kd_level_init_kernel, 1, 256, 0, s, S, nullptr, size_cur, start, box, S, nullptr, nullptr);
+            launch_chained(kd_bbox_kernel, grid_stride, 256, 0, s, pos_dev, seg_cur, n, S, box);
         }
-        kd_keys_kernel<<<nbk, 256, 0, s>>>(pos_dev, seg_cur, n, box, keys, vals);
+        launch_chained(kd_keys_kernel, nbk, 256, 0, s, pos_dev, seg_cur, n, box, keys, vals);
         int seg_bits = 0;
         while ((1 << seg_bits) < S) seg_bits++;
         if (by_selection) {
-            kd_level_init_kernel<<<1, 256, 0, s>>>(S, level_tree, size_cur, start, box_next, S_next, size_next, thr);
+            launch_chained(kd_level_init_kernel, 1, 256, 0, s, S, level_tree, size_cur, start, box_next, S_next, size_next, thr);
             int idx_bits = 0;
             const SelSplit* cut = nullptr;
             int rc = sel_select_splits(keys, 32 + seg_bits, nullptr, n, S, W, thr, ws + L.sel_state, ws + L.sel_hist, &idx_bits, &cut, true, s);
             if (rc) return rc;
-            kd_assign_select_kernel<<<grid_stride, 256, 0, s>>>(pos_dev, keys, n, idx_bits, cut, level_tree, seg_next, S_next, box_next, base_label,
+            launch_chained(kd_assign_select_kernel, grid_stride, 256, 0, s, pos_dev, keys, n, idx_bits, cut, level_tree, seg_next, S_next, box_next, base_label,
                                                                 labels_dev);
             std::swap(box, box_next);
         } else {

@@ -357,10 +357,11 @@ constexpr int WRAP_THREADS = 256;
 // into their cells here; the bounding box then only steers the shape of the work items.
 template <typename T, bool FUSED>
 __global__ void __launch_bounds__(WRAP_THREADS)
-rg_wrap_kernel(const T* __restrict__ pos, int64_t N, Geom<T> g, int vec_ok, Vec4<T>* __restrict__ posw,
-               int4* __restrict__ aff, DevHeader* __restrict__ h, const GridArgs ga, int subset,
-               const GridChoice gc, uint32_t* __restrict__ ccount, uint32_t* __restrict__ tccount)
+rg_wrap_kernel(const T* pos, int64_t N, Geom<T> g, int vec_ok, Vec4<T>* posw,
+               int4* aff, DevHeader* h, const GridArgs ga, int subset,
+               const GridChoice gc, uint32_t* ccount, uint32_t* tccount)
 {
+    chain_begin();
     __shared__ T stage[WRAP_THREADS * 3];
     __shared__ unsigned long long red[6][WRAP_THREADS / 32];
     __shared__ unsigned int red_cnt[WRAP_THREADS / 32];
@@ -506,9 +507,10 @@ rg_wrap_kernel(const T* __restrict__ pos, int64_t N, Geom<T> g, int vec_ok, Vec4
 // atoms only.
 template <typename T>
 __global__ void __launch_bounds__(256)
-rg_target_bbox_kernel(const int64_t* __restrict__ targets, int64_t Nt, int64_t N, const Vec4<T>* __restrict__ posw,
-                      DevHeader* __restrict__ h, const GridArgs ga)
+rg_target_bbox_kernel(const int64_t* targets, int64_t Nt, int64_t N, const Vec4<T>* posw,
+                      DevHeader* h, const GridArgs ga)
 {
+    chain_begin();
     __shared__ unsigned long long red[6][8];
     unsigned long long v[6] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -569,12 +571,13 @@ __device__ __forceinline__ void store_slot(SlotRec<double>* at, uint32_t key, ui
 }
 template <typename T, bool SCATTER>
 __global__ void __launch_bounds__(256, 4)
-rg_bin_kernel(int64_t N, int64_t Nt, const int64_t* __restrict__ targets, Geom<T> g,
-              const Vec4<T>* __restrict__ posw, const int4* __restrict__ aff, DevHeader* __restrict__ hp,
-              uint32_t* __restrict__ ccount, uint32_t* __restrict__ cfill,
-              uint32_t* __restrict__ tccount, uint32_t* __restrict__ tcfill,
-              SlotRec<T>* __restrict__ srec, SlotRec<T>* __restrict__ trec, long long src_capacity, int shape_cand_capacity)
+rg_bin_kernel(int64_t N, int64_t Nt, const int64_t* targets, Geom<T> g,
+              const Vec4<T>* posw, const int4* aff, DevHeader* hp,
+              uint32_t* ccount, uint32_t* cfill,
+              uint32_t* tccount, uint32_t* tcfill,
+              SlotRec<T>* srec, SlotRec<T>* trec, long long src_capacity, int shape_cand_capacity)
 {
+    chain_begin();
     const DevHeader h = *hp;
     // the counting pass still runs when only the image capacity is short (it writes nothing but the cell counters): the
     // prefix sum's total then leaves the true number of images in header.M for the caller's second attempt
@@ -722,13 +725,14 @@ __device__ __forceinline__ void float_test(double r2, double X, float& near, flo
 // Deterministic order inside each cell (ascending key) and the packed records.
 template <typename T>
 __global__ void __launch_bounds__(256)
-rg_bin_finalize_kernel(int64_t Nt, int subset, Geom<T> g, const Vec4<T>* __restrict__ posw, DevHeader* __restrict__ hp,
-                       const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ tcstart,
-                       const SlotRec<T>* __restrict__ srec, const SlotRec<T>* __restrict__ trec,
-                       Vec4<T>* __restrict__ spos, float4* __restrict__ sscan,
-                       uint2* __restrict__ smeta, Vec4<T>* __restrict__ tpos, float4* __restrict__ tscan,
-                       int4* __restrict__ tmeta, double r2, uint4* header_host)
+rg_bin_finalize_kernel(int64_t Nt, int subset, Geom<T> g, const Vec4<T>* posw, DevHeader* hp,
+                       const uint32_t* cstart, const uint32_t* tcstart,
+                       const SlotRec<T>* srec, const SlotRec<T>* trec,
+                       Vec4<T>* spos, float4* sscan,
+                       uint2* smeta, Vec4<T>* tpos, float4* tscan,
+                       int4* tmeta, double r2, uint4* header_host)
 {
+    chain_begin();
     // a plan that ends here: its header is complete
     if (header_host != nullptr && blockIdx.x == 0 && threadIdx.x == 0) publish_64_bytes(reinterpret_cast<const uint4*>(hp), header_host);
     if (hp->status & RG_FATAL) return;
@@ -1006,8 +1010,9 @@ constexpr int64_t RG_HEADER_BYTES = 1024;
 // output place is fixed by the offsets).
 template <typename T>
 __global__ void __launch_bounds__(256)
-rg_group_list_kernel(const PairParams<T>* __restrict__ params_dev, uint32_t* __restrict__ glist)
+rg_group_list_kernel(const PairParams<T>* params_dev, uint32_t* glist)
 {
+    chain_begin();
     const PairParams<T> p = *params_dev;
     DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
@@ -1283,6 +1288,7 @@ template <typename T>
 __global__ void __launch_bounds__(COUNT_WARPS * 32, COUNT_BLOCKS)
 rg_count_kernel(const PairParams<T> p)
 {
+    chain_begin();
     __shared__ CountWarp warps[COUNT_WARPS];
     __shared__ GroupShape shape;
     __shared__ CountCells cells;
@@ -1396,10 +1402,11 @@ rg_count_kernel(const PairParams<T> p)
 
 template <typename T>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
-rg_pair_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restrict__ ei,
-               float* __restrict__ shifts, T* __restrict__ d2out, const long long E, const GlueArgs glue, const int all_groups,
-               long long* __restrict__ total)
+rg_pair_kernel(const PairParams<T>* params_dev, long long* ei,
+               float* shifts, T* d2out, const long long E, const GlueArgs glue, const int all_groups,
+               long long* total)
 {
+    chain_begin();
     const PairParams<T> p = *params_dev;
     extern __shared__ __align__(32) unsigned char smem_raw[];
     constexpr int CAP = PAIR_CAND_BYTES / (int)sizeof(Vec4<T>);
@@ -1657,9 +1664,10 @@ __device__ __forceinline__ void zero_floats(float* at, int n, int lane)
 
 template <typename T, bool GLUE>
 __global__ void __launch_bounds__(EDGE_WARPS * 32, EDGE_BLOCKS)
-rg_fillmask_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restrict__ ei, float* __restrict__ shifts, const long long E,
-                const GlueArgs glue, long long* __restrict__ total)
+rg_fillmask_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts, const long long E,
+                const GlueArgs glue, long long* total)
 {
+    chain_begin();
     // the plan's pointers are read where they are used, too
     __shared__ PairParams<T> params;
     __shared__ GroupShape shape;
@@ -1881,9 +1889,10 @@ constexpr int FM_WARP_BYTES = FM_META * 8 + FM_META * 2 + RUN_INDEX_BYTES;    //
 
 template <typename T>
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
-rg_fillmask_dist_kernel(const PairParams<T>* __restrict__ params_dev, long long* __restrict__ ei, float* __restrict__ shifts,
-                   T* __restrict__ d2out, const long long E, long long* __restrict__ total)
+rg_fillmask_dist_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts,
+                   T* d2out, const long long E, long long* total)
 {
+    chain_begin();
     const PairParams<T> p = *params_dev;
     extern __shared__ __align__(32) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2054,8 +2063,9 @@ struct HaloArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo)
+rg_halo_owner_kernel(const PairParams<T>* params_dev, const HaloArgs halo)
 {
+    chain_begin();
     const PairParams<T> p = *params_dev;
     if (blockIdx.x == 0 && threadIdx.x == 0) {  // for the marking behind this launch
         if (halo.bad != nullptr) *halo.bad = 0u;
@@ -2076,8 +2086,9 @@ rg_halo_owner_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArg
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-rg_halo_runs_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo)
+rg_halo_runs_kernel(const PairParams<T>* params_dev, const HaloArgs halo)
 {
+    chain_begin();
     const PairParams<T> p = *params_dev;
     const DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
@@ -2114,8 +2125,9 @@ rg_halo_runs_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs
 // latency of its loads) + 79 us; with a warp a group here 31 us.
 template <typename T>
 __global__ void __launch_bounds__(128)
-rg_halo_list_kernel(const PairParams<T>* __restrict__ params_dev)
+rg_halo_list_kernel(const PairParams<T>* params_dev)
 {
+    chain_begin();
     const PairParams<T> p = *params_dev;
     DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
@@ -2247,8 +2259,9 @@ __device__ __forceinline__ void halo_batch(const PairParams<T>& p, const HaloArg
 
 template <typename T, bool WIDE>   // WIDE: more than 32 ranks, several words per atom
 __global__ void __launch_bounds__(PAIR_THREADS, 4)
-rg_halo_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo)
+rg_halo_kernel(const PairParams<T>* params_dev, const HaloArgs halo)
 {
+    chain_begin();
     const PairParams<T> p = *params_dev;
     __shared__ HaloWarp<T> warps[PAIR_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2356,9 +2369,10 @@ rg_halo_kernel(const PairParams<T>* __restrict__ params_dev, const HaloArgs halo
 // buffer), the cell counters, the degree counters and the caller's degree array in one pass.
 struct HeaderBlock { uint32_t words[RG_HEADER_BYTES / 4]; };
 __global__ void __launch_bounds__(256)
-rg_init_kernel(uint32_t* __restrict__ hdr, const HeaderBlock blk, uint4* __restrict__ zero_a, int64_t n_a16,
-               uint4* __restrict__ zero_b, int64_t n_b16, int32_t* __restrict__ counts_out, int64_t Nt)
+rg_init_kernel(uint32_t* hdr, const HeaderBlock blk, uint4* zero_a, int64_t n_a16,
+               uint4* zero_b, int64_t n_b16, int32_t* counts_out, int64_t Nt)
 {
+    chain_begin();
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
     if (i0 < RG_HEADER_BYTES / 4) hdr[i0] = blk.words[i0];
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
@@ -2614,7 +2628,7 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         memcpy(blk.words, init, sizeof(init));
         // every region of the layout starts on a 256-byte boundary and is padded to one
         const int64_t n_a16 = (L.cfill - L.ccount) / 16, n_b16 = bins_only ? 0 : ((Nt + 1) * 4 + 15) / 16;
-        rg_init_kernel<<<sm_count_cached() * 4, 256, 0, stream>>>(reinterpret_cast<uint32_t*>(w + L.hdr), blk,
+        launch_chained(rg_init_kernel, sm_count_cached() * 4, 256, 0, stream, reinterpret_cast<uint32_t*>(w + L.hdr), blk,
                                                                   reinterpret_cast<uint4*>(w + L.ccount), n_a16,
                                                                   reinterpret_cast<uint4*>(w + L.tcount), n_b16, counts_out, Nt);
     }
@@ -2622,27 +2636,22 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
     const int vec_ok = (reinterpret_cast<uintptr_t>(pos_dev) % 16 == 0) ? 1 : 0;
     const int64_t nb = std::max(N, Nt);
     if (host_grid) {
-        rg_wrap_kernel<T, true><<<(unsigned)((N + WRAP_THREADS - 1) / WRAP_THREADS), WRAP_THREADS, 0, stream>>>(
-            static_cast<const T*>(pos_dev), N, g, vec_ok, posw, aff, h, GridArgs{}, 0, gc_host, ccount, tccount);
+        launch_chained(rg_wrap_kernel<T, true>, (unsigned)((N + WRAP_THREADS - 1) / WRAP_THREADS), WRAP_THREADS, 0, stream, static_cast<const T*>(pos_dev), N, g, vec_ok, posw, aff, h, GridArgs{}, 0, gc_host, ccount, tccount);
     } else {
         const GridArgs ga = {radius, (long long)src_cap, (long long)cell_cap, PAIR_CAND_BYTES / (int)sizeof(Vec4<T>)};
-        rg_wrap_kernel<T, false><<<(unsigned)((N + WRAP_THREADS - 1) / WRAP_THREADS), WRAP_THREADS, 0, stream>>>(
-            static_cast<const T*>(pos_dev), N, g, vec_ok, posw, aff, h, ga, targets != nullptr ? 1 : 0, gc_host, nullptr, nullptr);
+        launch_chained(rg_wrap_kernel<T, false>, (unsigned)((N + WRAP_THREADS - 1) / WRAP_THREADS), WRAP_THREADS, 0, stream, static_cast<const T*>(pos_dev), N, g, vec_ok, posw, aff, h, ga, targets != nullptr ? 1 : 0, gc_host, nullptr, nullptr);
         if (targets != nullptr)
-            rg_target_bbox_kernel<T><<<(unsigned)((Nt + 255) / 256), 256, 0, stream>>>(targets, Nt, N, posw, h, ga);
-        rg_bin_kernel<T, false><<<(unsigned)((nb + 255) / 256), 256, 0, stream>>>(
-            N, Nt, targets, g, posw, aff, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap, 0);
+            launch_chained(rg_target_bbox_kernel<T>, (unsigned)((Nt + 255) / 256), 256, 0, stream, targets, Nt, N, posw, h, ga);
+        launch_chained(rg_bin_kernel<T, false>, (unsigned)((nb + 255) / 256), 256, 0, stream, N, Nt, targets, g, posw, aff, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap, 0);
     }
     // cell starts of sources and targets in the same two launches (which also set the fill cursors); the total of the source counts is the
     // number of source images actually binned (<= the count of rg_wrap when clipping): it becomes header.M
     DYNB_CUDA_OK((exclusive_scan_pair<uint32_t, uint32_t>(ccount, ccount, reinterpret_cast<uint32_t*>(&h->M), tccount, tccount, nullptr,
                                                            &h->ncell_plus1, cell_cap + 1, sums32, stream, cfill, tcfill)));
-    rg_bin_kernel<T, true><<<(unsigned)((nb + 255) / 256), 256, 0, stream>>>(
-        N, Nt, targets, g, posw, aff, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap,
+    launch_chained(rg_bin_kernel<T, true>, (unsigned)((nb + 255) / 256), 256, 0, stream, N, Nt, targets, g, posw, aff, h, ccount, cfill, tccount, tcfill, srec, trec, (long long)src_cap,
         host_grid ? PAIR_CAND_BYTES / (int)sizeof(Vec4<T>) : 0);
     const int64_t nf = std::max(src_cap, Nt);
-    rg_bin_finalize_kernel<T><<<(unsigned)((nf + 255) / 256), 256, 0, stream>>>(
-        Nt, targets != nullptr ? 1 : 0, g, posw, h, ccount, tccount, srec, trec, spos, sscan, smeta, tpos, tscan, tmeta, (double)pp_host.r2, bins_only ? header_written : nullptr);
+    launch_chained(rg_bin_finalize_kernel<T>, (unsigned)((nf + 255) / 256), 256, 0, stream, Nt, targets != nullptr ? 1 : 0, g, posw, h, ccount, tccount, srec, trec, spos, sscan, smeta, tpos, tscan, tmeta, (double)pp_host.r2, bins_only ? header_written : nullptr);
 
     if (bins_only) {
         DYNB_CUDA_OK(cudaGetLastError());
@@ -2651,11 +2660,11 @@ static int rg_plan(const void* pos_dev, int64_t N, const void* cell_host, const 
         return DYNB_OK;
     }
     if (targets != nullptr)
-        rg_group_list_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, tcfill);
+        launch_chained(rg_group_list_kernel<T>, sm_count_cached() * 8, 256, 0, stream, params_dev, tcfill);
     // there are no more groups than cells, and with a target subset no more of interest than targets
     const int64_t most_groups = std::min(host_grid ? (int64_t)gc_host.ncell_plus1 : cell_cap, targets != nullptr ? Nt : cell_cap);
     const int grid = (int)std::min<int64_t>((int64_t)sm_count_cached() * COUNT_BLOCKS, (most_groups + COUNT_WARPS - 1) / COUNT_WARPS);
-    rg_count_kernel<T><<<grid, COUNT_WARPS * 32, 0, stream>>>(pp_host);
+    launch_chained(rg_count_kernel<T>, grid, COUNT_WARPS * 32, 0, stream, pp_host);
     DYNB_CUDA_OK((exclusive_scan<uint32_t, long long>(tcount, toffset, nullptr, Nt + 1, sums64,
                                                        reinterpret_cast<long long*>(&h->E), stream,
                                                        ScanPublish{reinterpret_cast<const uint4*>(h), header_written})));
@@ -2700,14 +2709,14 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
     const int smem = PAIR_WARPS * PAIR_WARP_BYTES;
     if (long_lists != 0) DYNB_CUDA_OK(cudaFuncSetAttribute(rg_pair_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (d2 != nullptr && rg_write_at_once<T>(groups, long_lists)) {
-        rg_pair_kernel<T><<<grid, PAIR_THREADS, smem, stream>>>(params_dev, ei64, shifts, d2, (long long)E, glue,
+        launch_chained(rg_pair_kernel<T>, grid, PAIR_THREADS, smem, stream, params_dev, ei64, shifts, d2, (long long)E, glue,
                                                                                  1, reinterpret_cast<long long*>(total_dev));
         DYNB_CUDA_OK(cudaGetLastError());
         return DYNB_OK;
     }
     auto launch = [&](auto kernel, int blocks, int warps, int bytes, auto... out) -> int {
         DYNB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        kernel<<<blocks, warps * 32, bytes, stream>>>(params_dev, ei64, shifts, out..., reinterpret_cast<long long*>(total_dev));
+        launch_chained(kernel, blocks, warps * 32, bytes, stream, params_dev, ei64, shifts, out..., reinterpret_cast<long long*>(total_dev));
         return DYNB_OK;
     };
     const int esmem = EDGE_WARPS * (int)sizeof(EdgeWarp);
@@ -2721,7 +2730,7 @@ static int rg_fill(const void* ws, int64_t* ei, float* shifts, void* d2out, int6
         // Two waves where the caller has not read the header and most likely nothing is listed, else as many as the writer
         // (200 k atoms at 8 A without distances: 508 against 543 us with two)
         const int long_grid = (groups == RG_GROUPS_UNKNOWN && d2 == nullptr) ? std::min(grid, sm_count_cached() * 8) : grid;
-        rg_pair_kernel<T><<<long_grid, PAIR_THREADS, smem, stream>>>(params_dev, ei64, shifts, d2,
+        launch_chained(rg_pair_kernel<T>, long_grid, PAIR_THREADS, smem, stream, params_dev, ei64, shifts, d2,
                                                                                       (long long)E, glue, 0, nullptr);
     }
     DYNB_CUDA_OK(cudaGetLastError());
@@ -2735,12 +2744,12 @@ static int rg_halo_mark(const void* ws, const HaloArgs& ha, int64_t N, cudaStrea
     const auto* params_dev = reinterpret_cast<const PairParams<T>*>(w + RG_PARAMS_OFFSET);
     // the numbers of records and runs are known on the device only: both passes stride, the first with a thread for every
     // record of a system with no more images than atoms
-    rg_halo_owner_kernel<T><<<(unsigned)((2 * N + 255) / 256), 256, 0, stream>>>(params_dev, ha);
-    rg_halo_runs_kernel<T><<<sm_count_cached() * 8, 256, 0, stream>>>(params_dev, ha);
+    launch_chained(rg_halo_owner_kernel<T>, (unsigned)((2 * N + 255) / 256), 256, 0, stream, params_dev, ha);
+    launch_chained(rg_halo_runs_kernel<T>, sm_count_cached() * 8, 256, 0, stream, params_dev, ha);
     const int grid = sm_count_cached() * 4 * PAIR_GRID_WAVES;
-    rg_halo_list_kernel<T><<<sm_count_cached() * 8, 128, 0, stream>>>(params_dev);
-    if (ha.words == 1) rg_halo_kernel<T, false><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
-    else rg_halo_kernel<T, true><<<grid, PAIR_THREADS, 0, stream>>>(params_dev, ha);
+    launch_chained(rg_halo_list_kernel<T>, sm_count_cached() * 8, 128, 0, stream, params_dev);
+    if (ha.words == 1) launch_chained(rg_halo_kernel<T, false>, grid, PAIR_THREADS, 0, stream, params_dev, ha);
+    else launch_chained(rg_halo_kernel<T, true>, grid, PAIR_THREADS, 0, stream, params_dev, ha);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }

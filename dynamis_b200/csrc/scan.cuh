@@ -115,18 +115,20 @@ __device__ __forceinline__ void scan_tile_sums_body(const TIn* __restrict__ in, 
 
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_tile_sums_kernel(const TIn* __restrict__ in, const uint32_t* __restrict__ n_dev, int64_t n_host,
-                      TOut* __restrict__ sums)
+scan_tile_sums_kernel(const TIn* in, const uint32_t* n_dev, int64_t n_host,
+                      TOut* sums)
 {
+    chain_begin();
     scan_tile_sums_body<TIn, TOut>(in, n_dev, n_host, sums);
 }
 
 // two arrays of the same length in one launch: blockIdx.y picks the array, sums holds 2 x tiles entries
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_tile_sums_pair_kernel(const TIn* __restrict__ in0, const TIn* __restrict__ in1, const uint32_t* __restrict__ n_dev,
-                           int64_t n_host, TOut* __restrict__ sums)
+scan_tile_sums_pair_kernel(const TIn* in0, const TIn* in1, const uint32_t* n_dev,
+                           int64_t n_host, TOut* sums)
 {
+    chain_begin();
     scan_tile_sums_body<TIn, TOut>(blockIdx.y ? in1 : in0, n_dev, n_host, sums + (size_t)blockIdx.y * gridDim.x);
 }
 
@@ -262,18 +264,20 @@ __device__ __forceinline__ void scan_apply_fused_body(const TIn* in, const uint3
 
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
-scan_apply_fused_kernel(const TIn* in, const uint32_t* __restrict__ n_dev, int64_t n_host, const TOut* __restrict__ sums,
+scan_apply_fused_kernel(const TIn* in, const uint32_t* n_dev, int64_t n_host, const TOut* sums,
                         TOut* out, TOut* total_out, const ScanPublish publish)
 {
+    chain_begin();
     scan_apply_fused_body<TIn, TOut>(in, n_dev, n_host, sums, gridDim.x, out, total_out, nullptr, publish);
 }
 
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_apply_fused_pair_kernel(const TIn* in0, TOut* out0, TOut* total0, const TIn* in1, TOut* out1, TOut* total1,
-                             const uint32_t* __restrict__ n_dev, int64_t n_host, const TOut* __restrict__ sums, TOut* copy0,
+                             const uint32_t* n_dev, int64_t n_host, const TOut* sums, TOut* copy0,
                              TOut* copy1)
 {
+    chain_begin();
     scan_apply_fused_body<TIn, TOut>(blockIdx.y ? in1 : in0, n_dev, n_host, sums + (size_t)blockIdx.y * gridDim.x, gridDim.x,
                                      blockIdx.y ? out1 : out0, blockIdx.y ? total1 : total0, blockIdx.y ? copy1 : copy0);
 }
@@ -296,9 +300,9 @@ static inline cudaError_t exclusive_scan(const TIn* in, TOut* out, const uint32_
         return cudaSuccess;
     }
     const int tiles = scan_num_tiles(n_host);
-    scan_tile_sums_kernel<TIn, TOut><<<tiles, SCAN_THREADS, 0, stream>>>(in, n_dev, n_host, sums);
+    launch_chained(scan_tile_sums_kernel<TIn, TOut>, tiles, SCAN_THREADS, 0, stream, in, n_dev, n_host, sums);
     if (tiles <= SCAN_FUSED_MAX_TILES) {
-        scan_apply_fused_kernel<TIn, TOut><<<tiles, SCAN_THREADS, 0, stream>>>(in, n_dev, n_host, sums, out, total_out, publish);
+        launch_chained(scan_apply_fused_kernel<TIn, TOut>, tiles, SCAN_THREADS, 0, stream, in, n_dev, n_host, sums, out, total_out, publish);
     } else {
         scan_sums_kernel<TOut><<<1, SCAN_THREADS, 0, stream>>>(sums, tiles, total_out);
         scan_apply_kernel<TIn, TOut><<<tiles, SCAN_THREADS, 0, stream>>>(in, n_dev, n_host, sums, out);
@@ -315,9 +319,9 @@ static inline cudaError_t exclusive_scan_pair(const TIn* in0, TOut* out0, TOut* 
 {
     if (n_host <= 0) return cudaSuccess;
     const int tiles = scan_num_tiles(n_host);
-    scan_tile_sums_pair_kernel<TIn, TOut><<<dim3(tiles, 2), SCAN_THREADS, 0, stream>>>(in0, in1, n_dev, n_host, sums);
+    launch_chained(scan_tile_sums_pair_kernel<TIn, TOut>, dim3(tiles, 2), SCAN_THREADS, 0, stream, in0, in1, n_dev, n_host, sums);
     if (tiles <= SCAN_FUSED_MAX_TILES) {
-        scan_apply_fused_pair_kernel<TIn, TOut><<<dim3(tiles, 2), SCAN_THREADS, 0, stream>>>(in0, out0, total0, in1, out1, total1, n_dev,
+        launch_chained(scan_apply_fused_pair_kernel<TIn, TOut>, dim3(tiles, 2), SCAN_THREADS, 0, stream, in0, out0, total0, in1, out1, total1, n_dev,
                                                                                           n_host, sums, copy0, copy1);
     } else {
         scan_sums_pair_kernel<TOut><<<2, SCAN_THREADS, 0, stream>>>(sums, tiles, total0, total1);

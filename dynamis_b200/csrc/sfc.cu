@@ -39,8 +39,9 @@ __device__ __forceinline__ void stage_positions(const float* __restrict__ pos, i
 }
 
 __global__ void __launch_bounds__(256)
-sfc_minmax_kernel(const float* __restrict__ pos, int64_t n, int vec_ok, SfcBounds* __restrict__ b)
+sfc_minmax_kernel(const float* pos, int64_t n, int vec_ok, SfcBounds* b)
 {
+    chain_begin();
     __shared__ __align__(16) float stage[768];
     uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
     for (int64_t base = (int64_t)blockIdx.x * 256; base < n; base += (int64_t)gridDim.x * 256) {
@@ -101,9 +102,10 @@ __device__ __forceinline__ uint64_t spread_bits_21(uint32_t v)
 
 template <int CURVE>
 __global__ void __launch_bounds__(256)
-sfc_keys_kernel(const float* __restrict__ pos, int64_t n, int vec_ok, const SfcBounds* __restrict__ b,
-                uint64_t* __restrict__ keys, uint32_t* __restrict__ idx)
+sfc_keys_kernel(const float* pos, int64_t n, int vec_ok, const SfcBounds* b,
+                uint64_t* keys, uint32_t* idx)
 {
+    chain_begin();
     __shared__ __align__(16) float stage[768];
     const int64_t base = (int64_t)blockIdx.x * 256;
     stage_positions(pos, n, base, vec_ok, stage);
@@ -567,13 +569,14 @@ __device__ bool sel_finish_warp(const SelSplit& me, int g, const SelCand* cand, 
 // With done_counter != nullptr the block that finishes last also advances the split points (one warp
 // each), which saves a launch per level; used while there are few split points.
 __global__ void __launch_bounds__(256, 4)   // four blocks per SM for the histogram pass; the rare finish may spill
-sel_hist_kernel(const uint64_t* __restrict__ keys, const int64_t* __restrict__ weights, int64_t n, int idx_bits,
-                int shift, int width, int dbits, const SelSplit* st, SelSplit* __restrict__ st_out, int nsplit,
-                int level, int64_t W, const long long* __restrict__ thresholds, unsigned long long* __restrict__ hist,
-                unsigned long long* __restrict__ hist_next, int64_t table_words, unsigned int* __restrict__ done_counter,
-                int fine_private, SelCand* __restrict__ cand, unsigned int* __restrict__ cand_count,
-                unsigned int* __restrict__ finished, SelSplit* st_other /* the buffer st points into: no restrict */)
+sel_hist_kernel(const uint64_t* keys, const int64_t* weights, int64_t n, int idx_bits,
+                int shift, int width, int dbits, const SelSplit* st, SelSplit* st_out, int nsplit,
+                int level, int64_t W, const long long* thresholds, unsigned long long* hist,
+                unsigned long long* hist_next, int64_t table_words, unsigned int* done_counter,
+                int fine_private, SelCand* cand, unsigned int* cand_count,
+                unsigned int* finished, SelSplit* st_other /* the buffer st points into: no restrict */)
 {
+    chain_begin();
     // fine_private (first level, unit weights, width <= 14 only): the digit counters of this block are kept in
     // shared memory and added to the table once at the end -- for keys that crowd into a few digits (the
     // ordered bits of float coordinates) a million atomics on a handful of addresses took 90-150 us.
@@ -737,10 +740,11 @@ sel_hist_kernel(const uint64_t* __restrict__ keys, const int64_t* __restrict__ w
 
 // the same step as its own launch, eight split points per block (many split points)
 __global__ void __launch_bounds__(256)
-sel_pick_kernel(const SelSplit* __restrict__ st_in, SelSplit* __restrict__ st_out, int nsplit, int level, int width, int dbits,
-                int64_t n, int64_t W, int weighted, const long long* __restrict__ thresholds,
-                const unsigned long long* __restrict__ hist)
+sel_pick_kernel(const SelSplit* st_in, SelSplit* st_out, int nsplit, int level, int width, int dbits,
+                int64_t n, int64_t W, int weighted, const long long* thresholds,
+                const unsigned long long* hist)
 {
+    chain_begin();
     __shared__ u128 glist[SEL_MAX_SPLITS];
     __shared__ int gid[SEL_MAX_SPLITS];
     if (level > 0) sel_groups(st_in, nsplit, glist, gid);
@@ -749,9 +753,10 @@ sel_pick_kernel(const SelSplit* __restrict__ st_in, SelSplit* __restrict__ st_ou
 }
 
 __global__ void __launch_bounds__(256)
-sel_label_kernel(const uint64_t* __restrict__ keys, int64_t n, int idx_bits, const SelSplit* __restrict__ st, int nsplit,
-                 int64_t* __restrict__ labels)
+sel_label_kernel(const uint64_t* keys, int64_t n, int idx_bits, const SelSplit* st, int nsplit,
+                 int64_t* labels)
 {
+    chain_begin();
     __shared__ u128 cs[SEL_MAX_SPLITS];
     __shared__ int s_live;
     if (threadIdx.x == 0) s_live = nsplit;
@@ -822,11 +827,11 @@ int sel_select_splits(const uint64_t* keys, int key_bits, const int64_t* weights
         const size_t dyn = priv ? ((size_t)4 << width) : 0;
         // static + dynamic shared memory beyond 48 KB needs the opt-in
         if (dyn > 0) DYNB_CUDA_OK(cudaFuncSetAttribute(sel_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        sel_hist_kernel<<<hgrid, 256, dyn, s>>>(keys, weights_dev, n, idx_bits, shift, width, dbits, st_in, st_out, nsplit, l, W,
+        launch_chained(sel_hist_kernel, hgrid, 256, dyn, s, keys, weights_dev, n, idx_bits, shift, width, dbits, st_in, st_out, nsplit, l, W,
                                                 thresholds_dev, h_cur, h_other, table_words, done, priv, cand, cand_counts + l, finished,
                                                 const_cast<SelSplit*>(st_in));
         if (!fused)
-            sel_pick_kernel<<<(nsplit + 7) / 8, 256, 0, s>>>(st_in, st_out, nsplit, l, width, dbits, n, W,
+            launch_chained(sel_pick_kernel, (nsplit + 7) / 8, 256, 0, s, st_in, st_out, nsplit, l, width, dbits, n, W,
                                                              weights_dev != nullptr ? 1 : 0, thresholds_dev, h_cur);
     }
     DYNB_CUDA_OK(cudaGetLastError());
@@ -865,10 +870,10 @@ static int sfc_keys_into(const float* pos, int64_t n, int curve, unsigned char* 
     DYNB_CUDA_OK(cudaMemsetAsync(b->mx, 0, sizeof(SfcBounds) - sizeof(b->mn), stream));
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count_cached() * 4);
     const int vec_ok = (reinterpret_cast<uintptr_t>(pos) % 16 == 0) ? 1 : 0;
-    sfc_minmax_kernel<<<grid, 256, 0, stream>>>(pos, n, vec_ok, b);
+    launch_chained(sfc_minmax_kernel, grid, 256, 0, stream, pos, n, vec_ok, b);
     const unsigned nbk = (unsigned)((n + 255) / 256);
-    if (curve == 0) sfc_keys_kernel<0><<<nbk, 256, 0, stream>>>(pos, n, vec_ok, b, keys, idx);
-    else sfc_keys_kernel<1><<<nbk, 256, 0, stream>>>(pos, n, vec_ok, b, keys, idx);
+    if (curve == 0) launch_chained(sfc_keys_kernel<0>, nbk, 256, 0, stream, pos, n, vec_ok, b, keys, idx);
+    else launch_chained(sfc_keys_kernel<1>, nbk, 256, 0, stream, pos, n, vec_ok, b, keys, idx);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -947,7 +952,7 @@ extern "C" int dynb_sfc_minmax(const float* pos_dev, int64_t n_atoms, float* min
     DYNB_CUDA_OK(cudaMemsetAsync(b->mx, 0, sizeof(b->mx), s));
     if (n_atoms > 0) {
         const int grid = (int)std::min<int64_t>((n_atoms + 255) / 256, (int64_t)sm_count_cached() * 4);
-        sfc_minmax_kernel<<<grid, 256, 0, s>>>(pos_dev, n_atoms, (reinterpret_cast<uintptr_t>(pos_dev) % 16 == 0) ? 1 : 0, b);
+        launch_chained(sfc_minmax_kernel, grid, 256, 0, s, pos_dev, n_atoms, (reinterpret_cast<uintptr_t>(pos_dev) % 16 == 0) ? 1 : 0, b);
     }
     sfc_bounds_to_float_kernel<<<1, 32, 0, s>>>(b, minmax_dev);
     DYNB_CUDA_OK(cudaGetLastError());
@@ -966,8 +971,8 @@ extern "C" int dynb_sfc_keys_from_bounds(const float* pos_dev, int64_t n_atoms, 
     sfc_bounds_from_float_kernel<<<1, 32, 0, s>>>(minmax_dev, b);
     const unsigned nbk = (unsigned)((n_atoms + 255) / 256);
     const int vec_ok = (reinterpret_cast<uintptr_t>(pos_dev) % 16 == 0) ? 1 : 0;
-    if (curve_type == 0) sfc_keys_kernel<0><<<nbk, 256, 0, s>>>(pos_dev, n_atoms, vec_ok, b, reinterpret_cast<uint64_t*>(keys_dev), nullptr);
-    else sfc_keys_kernel<1><<<nbk, 256, 0, s>>>(pos_dev, n_atoms, vec_ok, b, reinterpret_cast<uint64_t*>(keys_dev), nullptr);
+    if (curve_type == 0) launch_chained(sfc_keys_kernel<0>, nbk, 256, 0, s, pos_dev, n_atoms, vec_ok, b, reinterpret_cast<uint64_t*>(keys_dev), nullptr);
+    else launch_chained(sfc_keys_kernel<1>, nbk, 256, 0, s, pos_dev, n_atoms, vec_ok, b, reinterpret_cast<uint64_t*>(keys_dev), nullptr);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -1018,7 +1023,7 @@ extern "C" int dynb_sfc_partition(const float* pos_dev, int64_t n_atoms, const i
                                &idx_bits, &splits, false, s);
         if (rc) return rc;
         const int hgrid = (int)std::min<int64_t>((n_atoms + 255) / 256, (int64_t)sm_count_cached() * 4);
-        sel_label_kernel<<<hgrid, 256, 0, s>>>(keys, n_atoms, idx_bits, splits, nsplit, labels_dev);
+        launch_chained(sel_label_kernel, hgrid, 256, 0, s, keys, n_atoms, idx_bits, splits, nsplit, labels_dev);
         DYNB_CUDA_OK(cudaGetLastError());
         return DYNB_OK;
     }
