@@ -16,6 +16,7 @@
 // ascending id, so nothing is sorted.
 
 #include "common.cuh"
+#include "clear.cuh"
 #include "scan.cuh"
 
 namespace dynb {
@@ -604,8 +605,7 @@ extern "C" int dynb_bincount_i64(const int64_t* a_dev, int64_t n, int64_t W, int
 {
     if (n < 0 || W < 1 || counts_dev == nullptr || bad_dev == nullptr) return fail_arg("bad arguments");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    DYNB_CUDA_OK(cudaMemsetAsync(counts_dev, 0, (size_t)W * 8, s));
-    DYNB_CUDA_OK(cudaMemsetAsync(bad_dev, 0, 4, s));
+    DYNB_CUDA_OK(clear_ranges(s, {counts_dev, W * 8, 0}, {bad_dev, 4, 0}));
     if (n == 0) return DYNB_OK;
     const int grid = (int)std::min<int64_t>(nblk(n), (int64_t)sm_count_cached() * 8);
     const size_t smem = W <= 4096 ? (size_t)W * 4 : 0;
@@ -658,10 +658,7 @@ extern "C" int dynb_halo_mark_from_edges(const int64_t* edges_dev, int64_t E, co
     if (E < 0 || N < 0 || world_size < 1 || my_rank < 0 || my_rank >= world_size) return fail_arg("bad arguments");
     const int words = (int)((world_size + 31) / 32);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    DYNB_CUDA_OK(cudaMemsetAsync(send_mask_dev, 0, (size_t)N * words * 4, s));
-    DYNB_CUDA_OK(cudaMemsetAsync(recv_mask_dev, 0, (size_t)N * words * 4, s));
-    DYNB_CUDA_OK(cudaMemsetAsync(has_remote_dev, 0, (size_t)N, s));
-    DYNB_CUDA_OK(cudaMemsetAsync(bad_dev, 0, 4, s));
+    DYNB_CUDA_OK(clear_ranges(s, {send_mask_dev, N * words * 4, 0}, {recv_mask_dev, N * words * 4, 0}, {has_remote_dev, N, 0}, {bad_dev, 4, 0}));
     if (E == 0) return DYNB_OK;
     launch_chained(halo_mark_edges_kernel, nblk(E), 256, 0, s, edges_dev, edges_dev + E, E, pid_dev, N, my_rank, words, send_mask_dev,
                                                    recv_mask_dev, has_remote_dev, bad_dev);
@@ -709,7 +706,7 @@ extern "C" int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_
     uint32_t* bsum = reinterpret_cast<uint32_t*>(ws);
     int64_t* totals = reinterpret_cast<int64_t*>(ws + align_up((int64_t)nb * (2 * W + 1) * 4, 256));
     uint32_t* arrived = reinterpret_cast<uint32_t*>(ws + need - 256);
-    DYNB_CUDA_OK(cudaMemsetAsync(arrived, 0, 4, s));
+    DYNB_CUDA_OK(clear_ranges(s, {arrived, 4, 0}));
     launch_chained(halo_lists_count_kernel, nb, HL_THREADS, 0, s, h, (int)W, nb, bsum);
     launch_chained(halo_lists_scan_kernel, (unsigned)(2 * W + 1), SCAN_THREADS, 0, s, bsum, nb, (int)W, totals, arrived, offsets_dev);
     DYNB_CUDA_OK(cudaGetLastError());

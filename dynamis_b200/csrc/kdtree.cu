@@ -20,9 +20,12 @@
 // of select.cuh on (segment, coordinate, index); an atom goes right when it is not in front of its
 // segment's cut.  Weighted cuts keep the sorted path (they need ranks for the clamp).
 
+#include <string.h>
+
 #include <vector>
 
 #include "common.cuh"
+#include "clear.cuh"
 #include "scan.cuh"
 #include "select.cuh"
 
@@ -46,6 +49,25 @@ __device__ __forceinline__ void kd_child_sizes(const KdSeg& g, long long sz, lon
         next_size[g.child_left] = m;
         next_size[g.child_right] = sz - m;
     }
+}
+
+// What the levels need before the first: the tree and the labels of its leaves (as a kernel argument while they fit; three copies from
+// host memory and a memset: 242 us a call of 1 M atoms against 233), the one segment's size, and every atom in that segment (the
+// array is padded to 16 bytes in the workspace).
+constexpr int KD_SETUP_BYTES = 3072;
+struct KdSetup { __align__(8) unsigned char bytes[KD_SETUP_BYTES]; };
+__global__ void __launch_bounds__(256)
+kd_setup_kernel(const KdSetup setup, int tree_words, int label_words, uint2* tree, uint2* base_label, long long* size, int64_t n, uint4* seg_id)
+{
+    chain_begin();
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    const uint2* const words = reinterpret_cast<const uint2*>(setup.bytes);
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < tree_words; i += blockDim.x) tree[i] = words[i];
+        for (int i = threadIdx.x; i < label_words; i += blockDim.x) base_label[i] = words[tree_words + i];
+        if (threadIdx.x == 0) *size = n;
+    }
+    for (int64_t i = i0; i < (n + 3) / 4; i += stride) seg_id[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // starts[s] = atoms in segments before s (sorted order puts segments in id order); `reset` boxes emptied.  With thresholds
@@ -334,12 +356,22 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
     std::vector<int64_t> base(parts.size());
     int64_t label = 0;
     for (size_t k = 0; k < parts.size(); k++) { base[k] = label; label += parts[k]; }
-    // small pageable sources: staged by cudaMemcpyAsync before it returns
-    const long long n_ll = n;
-    DYNB_CUDA_OK(cudaMemcpyAsync(size_cur, &n_ll, 8, cudaMemcpyHostToDevice, s));
-    DYNB_CUDA_OK(cudaMemcpyAsync(tree, segs.data(), segs.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, s));
-    DYNB_CUDA_OK(cudaMemcpyAsync(base_label, base.data(), base.size() * 8, cudaMemcpyHostToDevice, s));
-    DYNB_CUDA_OK(cudaMemsetAsync(seg_cur, 0, (size_t)n * 4, s));
+    const int64_t tree_bytes = (int64_t)(segs.size() * sizeof(KdSeg)), label_bytes = (int64_t)base.size() * 8;
+    if (tree_bytes + label_bytes <= KD_SETUP_BYTES) {
+        KdSetup setup;
+        memcpy(setup.bytes, segs.data(), (size_t)tree_bytes);
+        memcpy(setup.bytes + tree_bytes, base.data(), (size_t)label_bytes);
+        const unsigned blocks = (unsigned)std::min<int64_t>((n + 1023) / 1024, (int64_t)sm_count_cached() * 4);
+        launch_chained(kd_setup_kernel, blocks, 256, 0, s, setup, (int)(tree_bytes / 8), (int)(label_bytes / 8), reinterpret_cast<uint2*>(tree),
+                       reinterpret_cast<uint2*>(base_label), size_cur, n, reinterpret_cast<uint4*>(seg_cur));
+    } else {
+        // small pageable sources: staged by cudaMemcpyAsync before it returns
+        const long long n_ll = n;
+        DYNB_CUDA_OK(cudaMemcpyAsync(size_cur, &n_ll, 8, cudaMemcpyHostToDevice, s));
+        DYNB_CUDA_OK(cudaMemcpyAsync(tree, segs.data(), (size_t)tree_bytes, cudaMemcpyHostToDevice, s));
+        DYNB_CUDA_OK(cudaMemcpyAsync(base_label, base.data(), (size_t)label_bytes, cudaMemcpyHostToDevice, s));
+        DYNB_CUDA_OK(clear_ranges(s, {seg_cur, n * 4, 0}));
+    }
     const int grid_stride = (int)std::min<int64_t>(nbk, (int64_t)sm_count_cached() * 8);
     for (int l = 0; l < levels; l++) {
         const int S = (int)(first[l + 1] - first[l]), S_next = l + 1 < levels ? (int)(first[l + 2] - first[l + 1]) : 0;

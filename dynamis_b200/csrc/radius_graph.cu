@@ -32,6 +32,7 @@
 // source images are first clipped to the targets' bounding box grown by the cutoff.
 
 #include "common.cuh"
+#include "clear.cuh"
 #include "scan.cuh"
 
 #include <math.h>
@@ -2883,8 +2884,7 @@ extern "C" int dynb_rg_halo_mark_rank(const void* workspace_dev, int dtype, cons
     ha.bad = bad_dev;
     ha.words = (int)((world_size + 31) / 32);
     ha.rank = (int)rank;
-    DYNB_CUDA_OK(cudaMemsetAsync(needed_dev, 0, (size_t)n_atoms * ha.words * 4, s));
-    DYNB_CUDA_OK(cudaMemsetAsync(has_foreign_dev, 0, (size_t)n_atoms, s));
+    DYNB_CUDA_OK(clear_ranges(s, {needed_dev, n_atoms * ha.words * 4, 0}, {has_foreign_dev, n_atoms, 0}));
     if (dtype == DYNB_F32) return rg_halo_mark<float>(workspace_dev, ha, n_atoms, s);
     if (dtype == DYNB_F64) return rg_halo_mark<double>(workspace_dev, ha, n_atoms, s);
     return fail_arg("dtype must be DYNB_F32 or DYNB_F64");

@@ -10,6 +10,7 @@
 // (the reference's at::sort leaves that order unspecified).
 
 #include "common.cuh"
+#include "clear.cuh"
 #include "scan.cuh"
 #include "select.cuh"
 
@@ -806,7 +807,7 @@ int sel_select_splits(const uint64_t* keys, int key_bits, const int64_t* weights
     const int64_t table_words = ((int64_t)nsplit << dbits) + ((int64_t)nsplit << 8);  // digit + coarse counters of a level
     // the first table and, behind it, one arrival counter per level
     unsigned int* counters = reinterpret_cast<unsigned int*>(hist + table_words);
-    DYNB_CUDA_OK(cudaMemsetAsync(hist, 0, (size_t)table_words * 8 + 256, s));
+    DYNB_CUDA_OK(clear_ranges(s, {hist, table_words * 8 + 256, 0}));
     const bool fused = nsplit <= SEL_FINISH_SPLITS;  // two rounds of eight warps in the last block
     // early finish (fused path only): candidates in the split-point slots of state buffer 0 that no level uses,
     // one list counter per level behind the arrival counters, then the "finished" word
@@ -866,8 +867,7 @@ static int sfc_keys_into(const float* pos, int64_t n, int curve, unsigned char* 
 {
     // extrema start at +max / 0 in the ordered-integer image; set on the device (no copy from host memory)
     SfcBounds* b = reinterpret_cast<SfcBounds*>(ws + L.bounds);
-    DYNB_CUDA_OK(cudaMemsetAsync(b->mn, 0xff, sizeof(b->mn), stream));
-    DYNB_CUDA_OK(cudaMemsetAsync(b->mx, 0, sizeof(SfcBounds) - sizeof(b->mn), stream));
+    DYNB_CUDA_OK(clear_ranges(stream, {b->mn, sizeof(b->mn), 0xff}, {b->mx, sizeof(SfcBounds) - sizeof(b->mn), 0}));
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count_cached() * 4);
     const int vec_ok = (reinterpret_cast<uintptr_t>(pos) % 16 == 0) ? 1 : 0;
     launch_chained(sfc_minmax_kernel, grid, 256, 0, stream, pos, n, vec_ok, b);
@@ -948,8 +948,7 @@ extern "C" int dynb_sfc_minmax(const float* pos_dev, int64_t n_atoms, float* min
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // the 24 bytes behind the six floats are the scratch for the ordered-integer extrema
     SfcBounds* b = reinterpret_cast<SfcBounds*>(minmax_dev + 8);
-    DYNB_CUDA_OK(cudaMemsetAsync(b->mn, 0xff, sizeof(b->mn), s));
-    DYNB_CUDA_OK(cudaMemsetAsync(b->mx, 0, sizeof(b->mx), s));
+    DYNB_CUDA_OK(clear_ranges(s, {b->mn, sizeof(b->mn), 0xff}, {b->mx, sizeof(b->mx), 0}));
     if (n_atoms > 0) {
         const int grid = (int)std::min<int64_t>((n_atoms + 255) / 256, (int64_t)sm_count_cached() * 4);
         launch_chained(sfc_minmax_kernel, grid, 256, 0, s, pos_dev, n_atoms, (reinterpret_cast<uintptr_t>(pos_dev) % 16 == 0) ? 1 : 0, b);
