@@ -921,12 +921,15 @@ __device__ __forceinline__ void glue_write(const GlueArgs& g, float* __restrict_
 // The grid and the shape of the groups, and one group: its targets (one contiguous run a cell row, at most two rows) and this
 // lane's run of source records.  Both cell-scan kernels keep the grid in shared memory and read it where a group is looked
 // up: in registers it left too few for the loops.
-struct GroupShape { int nx, ny, nz, sx, sy, pad, gx, gy; uint32_t by_gx, by_gy; };
-struct GroupDesc { uint32_t tb0, te0, tb1, te1; int run_a, run_e, cy0, cy1, cz; };   // as loaded: nothing waits for the loads until the group's turn
+struct __align__(16) GroupShape { uint32_t gx, by_gx, gy, by_gy; int nx, ny, nz, sx; int sy, pad, unused[2]; };
+// As loaded (nothing waits for the loads until the group's turn): lanes below 30 have their run of source records, the two last lanes the
+// targets of the group's two rows.
+struct GroupDesc { int run_a, run_e; };
+constexpr int GROUP_ROW_LANE = 30;
 __device__ __forceinline__ GroupShape group_shape(const DevHeader* hp)
 {
-    const int gx = hp->gx, gy = (hp->ny + hp->group_cells_y - 1) / hp->group_cells_y;
-    return {hp->nx, hp->ny, hp->nz, hp->group_cells, hp->group_cells_y, hp->pad, gx, gy, 0xffffffffu / (uint32_t)gx, 0xffffffffu / (uint32_t)gy};
+    const uint32_t gx = (uint32_t)hp->gx, gy = (uint32_t)((hp->ny + hp->group_cells_y - 1) / hp->group_cells_y);
+    return {gx, 0xffffffffu / gx, gy, 0xffffffffu / gy, hp->nx, hp->ny, hp->nz, hp->group_cells, hp->group_cells_y, hp->pad, {0, 0}};
 }
 // v / d and the remainder, from by_d = floor((2^32 - 1) / d) >= 2^32 / d - 1: v by_d / 2^32 lies above v / d - 1, so the upper half
 // of the product is the quotient or one less.  (The compiler's division is three times as many instructions.)
@@ -937,17 +940,54 @@ __device__ __forceinline__ uint32_t group_divide(uint32_t v, uint32_t d, uint32_
     if (rest >= d) { rest -= d; q++; }
     return q;
 }
-// lane r owns run r: (z row, y row) of it, counted from the lowest; -1: no run
+// Which cells a lane looks up: (y, z) row relative to the group's first, and how far beyond the group along x; -1: none
+__device__ __forceinline__ int group_lane(const GroupShape& g, int lane)
+{
+    const int wy = g.sy + 2 * g.pad;
+    if (lane >= GROUP_ROW_LANE) return (8 + lane - GROUP_ROW_LANE) | (8 << 8);
+    return lane < wy * (2 * g.pad + 1) ? ((8 + lane % wy - g.pad) | ((8 + lane / wy - g.pad) << 8) | (g.pad << 16)) : -1;
+}
+__device__ __forceinline__ uint4 shared_words(const void* at)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"((uint32_t)__cvta_generic_to_shared(at)));
+    return v;
+}
+// cells: first records of the cells, of the sources, for the two last lanes of the targets.  Two loads a lane, and none of the
+// branches that a row outside the grid would need: its lane reads an empty run.  Edge writer, before (every lane loaded the rows'
+// targets, ten words of the grid were read one by one) and after: 309 -> 298 us (liquid, 1 M atoms), 162 -> 153 (silicon in double
+// precision, 500 k), 25.3 -> 23.1 (copper, 32 k), 12.8 -> 10.7 (1 k), 605 -> 605 (a rank's copper with Cartesian shifts).
+__device__ __forceinline__ GroupDesc fetch_group(const GroupShape& shape, const uint32_t* cells, uint32_t grp, int which)
+{
+    const uint4 g = shared_words(&shape.gx), n = shared_words(&shape.nx), s = shared_words(&shape.sy);
+    const int nx = (int)n.x, ny = (int)n.y, nz = (int)n.z;
+    uint32_t ix, iy;
+    const uint32_t row = group_divide(grp, g.x, g.y, ix);
+    const int cz = (int)group_divide(row, g.z, g.w, iy), cy0 = (int)(iy * s.x), cy1 = min(cy0 + (int)s.x, ny) - 1;
+    GroupDesc d;
+    const int cx0 = (int)(ix * n.w), cx1 = min(cx0 + (int)n.w, nx) - 1;
+    const int beyond = which >> 16, yy = cy0 + (which & 255) - 8, zz = cz + ((which >> 8) & 255) - 8;
+    const bool there = which >= 0 && yy >= 0 && yy <= min(cy1 + beyond, ny - 1) && zz >= 0 && zz < nz;
+    const uint32_t first = ((uint32_t)zz * (uint32_t)ny + (uint32_t)yy) * (uint32_t)nx;
+    const uint32_t a = there ? first + (uint32_t)max(cx0 - beyond, 0) : 0u, e = there ? first + (uint32_t)min(cx1 + beyond, nx - 1) + 1u : 0u;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(d.run_a) : "l"(cells + a));
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(d.run_e) : "l"(cells + e));
+    return d;
+}
+
+// The same for the count pass, which does not load ahead: every lane loads the rows' targets, and nothing is handed round behind the
+// loads (a rank's copper: 265 us with this one, 270 with the other; the liquid 209 and 211).
+struct GroupRows { uint32_t tb0, te0, tb1, te1; int run_a, run_e, cy0, cy1, cz; };
 __device__ __forceinline__ int group_lane_run(const GroupShape& g, int lane)
 {
     const int wy = g.sy + 2 * g.pad;
     return lane < wy * (2 * g.pad + 1) ? (((lane / wy) << 8) | (lane % wy)) : -1;
 }
-__device__ __forceinline__ GroupDesc fetch_group(const volatile GroupShape& g, const uint32_t* tcstart, const uint32_t* cstart, uint32_t grp, int lane_run)
+__device__ __forceinline__ GroupRows fetch_group_rows(const volatile GroupShape& g, const uint32_t* tcstart, const uint32_t* cstart, uint32_t grp, int lane_run)
 {
-    GroupDesc d;
+    GroupRows d;
     const int nx = g.nx, ny = g.ny, pad = g.pad, sx = g.sx, sy = g.sy;
-    const uint32_t gx = (uint32_t)g.gx, gy = (uint32_t)g.gy;
+    const uint32_t gx = g.gx, gy = g.gy;
     uint32_t ix, iy;
     const uint32_t row = group_divide(grp, gx, g.by_gx, ix);
     const int cz = (int)group_divide(row, gy, g.by_gy, iy), cx0 = (int)ix * sx, cy0 = (int)iy * sy;
@@ -1329,7 +1369,7 @@ rg_count_kernel(const PairParams<T> p)
         const uint32_t grp = p.glist ? p.glist[gi] : gi;
         uint32_t following = 0;
         if (lane == 0) following = nwarps + atomicAdd(&hp->count_next, 1u);
-        const GroupDesc d = fetch_group(shape, p.tcstart, p.cstart, grp, lane_run);
+        const GroupRows d = fetch_group_rows(shape, p.tcstart, p.cstart, grp, lane_run);
         const int run_a = d.run_a, run_len = d.run_e - d.run_a;
         volatile CountGroup& g = w.group;   // all lanes write the same
         const uint32_t n0 = d.te0 - d.tb0, ntot = n0 + (d.te1 - d.tb1);
@@ -1686,7 +1726,7 @@ rg_fillmask_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts
     const uint32_t lt = lanemask_lt(), le = lt | (1u << lane);
 
     if (total != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *total = E;
-    const int lane_run = group_lane_run(shape, lane);
+    const int which = group_lane(shape, lane);
     // Candidates of one shift code: the targets, which are among them, have it too, and every shift of the group is zero.
     // Left out: mapped ids, and Cartesian shifts of which a zero is a negative zero (a column of the cell that is all negative).
     bool may_be_plain = true;
@@ -1705,7 +1745,11 @@ rg_fillmask_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts
 
     // the next group is looked up while the current one is written, so that one round trip to memory per group (the candidate
     // records) stays exposed
-    auto fetch = [&](uint32_t i) { return fetch_group(shape, p.tcstart, p.cstart, p.glist ? p.glist[i] : i, lane_run); };
+    static_assert(offsetof(PairParams<T>, tcstart) == offsetof(PairParams<T>, cstart) + sizeof(void*), "read as a pair");
+    auto fetch = [&](uint32_t i) {
+        const uint32_t* cells = reinterpret_cast<const uint32_t* const volatile*>(&params.cstart)[lane >= GROUP_ROW_LANE ? 1 : 0];
+        return fetch_group(shape, cells, p.glist ? p.glist[i] : i, which);
+    };
 
     const uint32_t nwarps = gridDim.x * EDGE_WARPS;
     uint32_t gi = blockIdx.x * EDGE_WARPS + warp;
@@ -1715,11 +1759,13 @@ rg_fillmask_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts
     for (; gi < num_groups; gi += nwarps) {
         const GroupDesc d = nd;
         if (gi + nwarps < num_groups) nd = fetch(gi + nwarps);
-        const int n0 = (int)(d.te0 - d.tb0), pieces = 8 * (n0 + (int)(d.te1 - d.tb1));
+        const uint32_t tb0 = __shfl_sync(0xffffffffu, (uint32_t)d.run_a, GROUP_ROW_LANE), te0 = __shfl_sync(0xffffffffu, (uint32_t)d.run_e, GROUP_ROW_LANE);
+        const uint32_t tb1 = __shfl_sync(0xffffffffu, (uint32_t)d.run_a, GROUP_ROW_LANE + 1), te1 = __shfl_sync(0xffffffffu, (uint32_t)d.run_e, GROUP_ROW_LANE + 1);
+        const int n0 = (int)(te0 - tb0), pieces = 8 * (n0 + (int)(te1 - tb1));
         if (pieces == 0) continue;
         // the first bits and the rows' places in the output do not depend on the candidate records: ask for them now
-        const uint32_t second = d.tb1 - (uint32_t)n0;   // + number of a target of the second row among all
-        auto target = [&](int i) { return (uint32_t)(i >> 3) + ((i >> 3) < n0 ? d.tb0 : second); };
+        const uint32_t second = tb1 - (uint32_t)n0;   // + number of a target of the second row among all
+        auto target = [&](int i) { return (uint32_t)(i >> 3) + ((i >> 3) < n0 ? tb0 : second); };
         uint2 next_bits = make_uint2(0u, 0u);
         int next_dst = 0;
         if (lane < pieces) {
@@ -1727,8 +1773,8 @@ rg_fillmask_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts
             next_bits = reinterpret_cast<const uint2*>(p.hitmask + (size_t)t * 32)[lane & 7];
             next_dst = p.tmeta[t].x;
         }
-        const long long base0 = p.toffset[d.tb0], base1 = p.toffset[d.tb1], end0 = p.toffset[d.te0], end1 = p.toffset[d.te1];
-        const int run_len = d.run_e - d.run_a, run_end = (int)warp_incl_scan_u32((uint32_t)run_len), run_off = run_end - run_len, L = __shfl_sync(0xffffffffu, run_end, 31);
+        const long long base0 = p.toffset[tb0], base1 = p.toffset[tb1], end0 = p.toffset[te0], end1 = p.toffset[te1];
+        const int run_len = lane < GROUP_ROW_LANE ? d.run_e - d.run_a : 0, run_end = (int)warp_incl_scan_u32((uint32_t)run_len), run_off = run_end - run_len, L = __shfl_sync(0xffffffffu, run_end, 31);
         const int nslots = (L + 31) >> 5;
         if (nslots == 0 || nslots > RG_MASK_SLOTS) continue;  // a longer list has no hit bits: rg_pair_kernel writes that group
         // one or two targets are often without neighbours (a gas of a million atoms, 0.001 per A^3: 433 us without this line, 357
