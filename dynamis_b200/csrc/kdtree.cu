@@ -138,9 +138,9 @@ kd_bbox_kernel(const float* pos, const int32_t* seg_id, int64_t n, int S, uint32
 }
 
 // widest axis of the segment (kdtree_kernels.cu:58-70: strict '>' keeps the first axis on ties)
-__device__ __forceinline__ int kd_axis(const uint32_t* __restrict__ box, int s)
+__device__ __forceinline__ int kd_axis(const uint32_t* __restrict__ box, int s, float& best)
 {
-    float best = -1.0f;
+    best = -1.0f;
     int axis = 0;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -150,17 +150,32 @@ __device__ __forceinline__ int kd_axis(const uint32_t* __restrict__ box, int s)
     return axis;
 }
 
+// Selection: the place of the coordinate in its segment's box, in equal cells, stands in front of the coordinate's own bits
+// (place_bits of them).  The place does not fall where the coordinate rises (a difference with the box's end and a product with
+// one positive number, both rounded, cut off and clamped; zero for all where the extent is no number to divide by), so the order is that of
+// the coordinates, but the leading digit of the selection spreads evenly: it leaves 60 of a million atoms where sign, exponent and
+// five bits of the mantissa left 30 thousand, and the second digit's pass settles the cuts in place of the third's.  A call of a
+// million atoms on 8 ranks: 233 us before, 200 with places.
+constexpr int KD_PLACE_BITS = 14;
 __global__ void __launch_bounds__(256)
 kd_keys_kernel(const float* pos, const int32_t* seg_id, int64_t n, const uint32_t* box,
-               uint64_t* keys, uint32_t* vals)
+               uint64_t* keys, uint32_t* vals, int place_bits)
 {
     chain_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int s = seg_id[i];
-    const int axis = kd_axis(box, s);
-    keys[i] = ((uint64_t)(uint32_t)s << 32) | (uint64_t)ordered_u32(pos[3 * i + axis]);
-    vals[i] = (uint32_t)i;
+    float extent;
+    const int axis = kd_axis(box, s, extent);
+    const float x = pos[3 * i + axis];
+    uint64_t segment = (uint64_t)(uint32_t)s;
+    if (place_bits > 0) {
+        const float cells = (float)(1 << place_bits), scale = extent > 0.0f && extent < INFINITY ? cells / extent : 0.0f;
+        const uint32_t place = (uint32_t)((x - unordered_f32(box[s * 6 + axis])) * scale);
+        segment = (segment << place_bits) | (uint64_t)min(place, (1u << place_bits) - 1u);
+    }
+    keys[i] = (segment << 32) | (uint64_t)ordered_u32(x);
+    if (vals != nullptr) vals[i] = (uint32_t)i;
 }
 
 __global__ void __launch_bounds__(256)
@@ -216,7 +231,7 @@ kd_assign_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__
 // its two loads (10 us for a million atoms); a launch for each of the two, for the sizes of the cuts and for every level's
 // part of the tree made the call of a million atoms on 8 ranks 305 us instead of 278.
 __global__ void __launch_bounds__(256)
-kd_assign_select_kernel(const float* pos, const uint64_t* keys, int64_t n, int idx_bits, const SelSplit* cut,
+kd_assign_select_kernel(const float* pos, const uint64_t* keys, int64_t n, int idx_bits, int segment_shift, const SelSplit* cut,
                         const KdSeg* seg, int32_t* new_seg_id, int S, uint32_t* box,
                         const int64_t* base_label, int64_t* labels)
 {
@@ -225,7 +240,7 @@ kd_assign_select_kernel(const float* pos, const uint64_t* keys, int64_t n, int i
     if (S > 0) boxes.begin(S);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t key = keys[i];
-        const int s = (int)(key >> 32);
+        const int s = (int)(key >> segment_shift);
         const SelSplit c = cut[s];
         const u128 C = ((u128)key << idx_bits) | (u128)(uint64_t)i;
         const bool right = !c.dead && C >= sel_prefix(c);
@@ -373,6 +388,7 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
         DYNB_CUDA_OK(clear_ranges(s, {seg_cur, n * 4, 0}));
     }
     const int grid_stride = (int)std::min<int64_t>(nbk, (int64_t)sm_count_cached() * 8);
+    const int place_bits = by_selection ? KD_PLACE_BITS : 0;
     for (int l = 0; l < levels; l++) {
         const int S = (int)(first[l + 1] - first[l]), S_next = l + 1 < levels ? (int)(first[l + 2] - first[l + 1]) : 0;
         const KdSeg* level_tree = tree + first[l];
@@ -380,16 +396,16 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
             launch_chained(kd_level_init_kernel, 1, 256, 0, s, S, nullptr, size_cur, start, box, S, nullptr, nullptr);
             launch_chained(kd_bbox_kernel, grid_stride, 256, 0, s, pos_dev, seg_cur, n, S, box);
         }
-        launch_chained(kd_keys_kernel, nbk, 256, 0, s, pos_dev, seg_cur, n, box, keys, vals);
+        launch_chained(kd_keys_kernel, nbk, 256, 0, s, pos_dev, seg_cur, n, box, keys, by_selection ? nullptr : vals, place_bits);
         int seg_bits = 0;
         while ((1 << seg_bits) < S) seg_bits++;
         if (by_selection) {
             launch_chained(kd_level_init_kernel, 1, 256, 0, s, S, level_tree, size_cur, start, box_next, S_next, size_next, thr);
             int idx_bits = 0;
             const SelSplit* cut = nullptr;
-            int rc = sel_select_splits(keys, 32 + seg_bits, nullptr, n, S, W, thr, ws + L.sel_state, ws + L.sel_hist, &idx_bits, &cut, true, s);
+            int rc = sel_select_splits(keys, 32 + place_bits + seg_bits, nullptr, n, S, W, thr, ws + L.sel_state, ws + L.sel_hist, &idx_bits, &cut, s);
             if (rc) return rc;
-            launch_chained(kd_assign_select_kernel, grid_stride, 256, 0, s, pos_dev, keys, n, idx_bits, cut, level_tree, seg_next, S_next, box_next, base_label,
+            launch_chained(kd_assign_select_kernel, grid_stride, 256, 0, s, pos_dev, keys, n, idx_bits, 32 + place_bits, cut, level_tree, seg_next, S_next, box_next, base_label,
                                                                 labels_dev);
             std::swap(box, box_next);
         } else {

@@ -24,10 +24,9 @@ __device__ __forceinline__ u128 sel_prefix(const SelSplit& s) { return ((u128)s.
 // composite of the split atom (or dead).  thresholds_dev == nullptr: the thresholds of the W-way
 // partition (equal counts, or weights_dev); else thresholds_dev[s] = 1 + number of atoms in front of
 // split atom s in (key, index) order, non-decreasing in s.  state_ws: 2 * SEL_MAX_SPLITS SelSplit,
-// hist_ws: 2 * SEL_HIST_BYTES.  crowded_keys: the keys fall into few values of their leading digit (float
-// coordinates): the first level then counts in shared memory first.
+// hist_ws: 2 * SEL_HIST_BYTES.  Keys whose leading digits spread over many values are settled in two passes.
 int sel_select_splits(const uint64_t* keys_dev, int key_bits, const int64_t* weights_dev, int64_t n, int nsplit, int64_t W,
                       const long long* thresholds_dev, unsigned char* state_ws, unsigned char* hist_ws, int* idx_bits_out,
-                      const SelSplit** final_out, bool crowded_keys, cudaStream_t stream);
+                      const SelSplit** final_out, cudaStream_t stream);
 
 }  // namespace dynb

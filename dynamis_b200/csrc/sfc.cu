@@ -574,18 +574,10 @@ sel_hist_kernel(const uint64_t* keys, const int64_t* weights, int64_t n, int idx
                 int shift, int width, int dbits, const SelSplit* st, SelSplit* st_out, int nsplit,
                 int level, int64_t W, const long long* thresholds, unsigned long long* hist,
                 unsigned long long* hist_next, int64_t table_words, unsigned int* done_counter,
-                int fine_private, SelCand* cand, unsigned int* cand_count,
+                SelCand* cand, unsigned int* cand_count,
                 unsigned int* finished, SelSplit* st_other /* the buffer st points into: no restrict */)
 {
     chain_begin();
-    // fine_private (first level, unit weights, width <= 14 only): the digit counters of this block are kept in
-    // shared memory and added to the table once at the end -- for keys that crowd into a few digits (the
-    // ordered bits of float coordinates) a million atomics on a handful of addresses took 90-150 us.
-    // Every atom adds a constant one to a 32-bit shared counter (a native operation that also takes lanes on one address
-    // together) and the coarse counters are summed from the digit counters at the end: 118, 90 and 77 -> 22, 26 and 25 us for the
-    // first digits of the three levels of a KD-tree of a million atoms.  Before, lanes were grouped by a warp match and a
-    // 64-bit coarse counter, one of two or three in use, was added to in shared memory for every group.
-    extern __shared__ unsigned int s_fine[];
     __shared__ u128 glist[SEL_MAX_SPLITS];
     __shared__ int gid[SEL_MAX_SPLITS];
     __shared__ unsigned long long s_coarse[256];  // weighted; 64-bit shared additions are compare-and-swap loops
@@ -604,8 +596,6 @@ sel_hist_kernel(const uint64_t* keys, const int64_t* weights, int64_t n, int idx
         if (threadIdx.x == 0) glist[0] = 0;
         s_coarse[threadIdx.x] = 0ull;  // one group, every atom counts: coarse counters through shared memory
         s_coarse_unit[threadIdx.x] = 0u;
-        if (fine_private)
-            for (int k = threadIdx.x; k < (1 << width); k += blockDim.x) s_fine[k] = 0u;
         __syncthreads();
     } else {
         ng = sel_groups(st, nsplit, glist, gid);
@@ -672,37 +662,31 @@ sel_hist_kernel(const uint64_t* keys, const int64_t* weights, int64_t n, int idx
                         }
                     }
                 }
+                // Unit weights: a warp whose atoms all fall on one counter adds them together.  Keys of a system with an outlier crowd
+                // into a few first digits, and a million additions to one address take 90 us and more.
+                unsigned together = 0u;
+                if (weights == nullptr) {
+                    const unsigned counted = __ballot_sync(0xffffffffu, w != 0ull);
+                    int same = 0;
+                    if (w) __match_all_sync(counted, (unsigned)slot, &same);
+                    if (w && same) together = counted;
+                }
+                if (together != 0u) {
+                    w = (together & lanemask_lt()) == 0u ? (unsigned long long)__popc(together) : 0ull;
+                }
                 if (w) {
-                    if (fine_private) {
-                        atomicAdd(&s_fine[digit], 1u);
-                    } else {
-                        atomicAdd(&hist[slot], w);
-                        if (level > 0) atomicAdd(&coarse[((size_t)lo << 8) + (digit >> fbits)], w);
-                        else if (weights) atomicAdd(&s_coarse[digit >> fbits], w);
-                        else atomicAdd(&s_coarse_unit[digit >> fbits], 1u);
-                    }
+                    atomicAdd(&hist[slot], w);
+                    if (level > 0) atomicAdd(&coarse[((size_t)lo << 8) + (digit >> fbits)], w);
+                    else if (weights) atomicAdd(&s_coarse[digit >> fbits], w);
+                    else atomicAdd(&s_coarse_unit[digit >> fbits], (unsigned)w);
                 }
             }
         }
     }
     if (level == 0) {
         __syncthreads();
-        if (fine_private) {
-            const int lane = threadIdx.x & 31;
-            for (int c = threadIdx.x >> 5; c < (1 << (width - fbits)); c += (int)(blockDim.x >> 5)) {
-                unsigned int sum = 0;
-                for (int k = (c << fbits) + lane; k < ((c + 1) << fbits); k += 32) {
-                    const unsigned int v = s_fine[k];
-                    if (v) atomicAdd(&hist[k], (unsigned long long)v);
-                    sum += v;
-                }
-                sum = __reduce_add_sync(0xffffffffu, sum);
-                if (lane == 0 && sum) atomicAdd(&coarse[c], (unsigned long long)sum);
-            }
-        } else {
-            const unsigned long long v = weights ? s_coarse[threadIdx.x] : (unsigned long long)s_coarse_unit[threadIdx.x];
-            if (v) atomicAdd(&coarse[threadIdx.x], v);
-        }
+        const unsigned long long v = weights ? s_coarse[threadIdx.x] : (unsigned long long)s_coarse_unit[threadIdx.x];
+        if (v) atomicAdd(&coarse[threadIdx.x], v);
     }
     if (done_counter == nullptr) return;
     __threadfence();
@@ -793,7 +777,7 @@ static int sel_digit_bits(int64_t groups, int total_bits)
 
 int sel_select_splits(const uint64_t* keys, int key_bits, const int64_t* weights_dev, int64_t n, int nsplit, int64_t W,
                       const long long* thresholds_dev, unsigned char* state_ws, unsigned char* hist_ws, int* idx_bits_out,
-                      const SelSplit** final_out, bool crowded_keys, cudaStream_t s)
+                      const SelSplit** final_out, cudaStream_t s)
 {
     if (nsplit < 1 || nsplit > SEL_MAX_SPLITS) return fail_arg("number of split points out of range");
     int idx_bits = 1;
@@ -824,12 +808,8 @@ int sel_select_splits(const uint64_t* keys, int key_bits, const int64_t* weights
         unsigned long long* h_cur = hist + (size_t)(l & 1) * hist_words;
         unsigned long long* h_other = hist + (size_t)((l + 1) & 1) * hist_words;
         unsigned int* done = fused ? counters + l : nullptr;
-        const int priv = (crowded_keys && l == 0 && weights_dev == nullptr && width <= 14) ? 1 : 0;
-        const size_t dyn = priv ? ((size_t)4 << width) : 0;
-        // static + dynamic shared memory beyond 48 KB needs the opt-in
-        if (dyn > 0) DYNB_CUDA_OK(cudaFuncSetAttribute(sel_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        launch_chained(sel_hist_kernel, hgrid, 256, dyn, s, keys, weights_dev, n, idx_bits, shift, width, dbits, st_in, st_out, nsplit, l, W,
-                                                thresholds_dev, h_cur, h_other, table_words, done, priv, cand, cand_counts + l, finished,
+        launch_chained(sel_hist_kernel, hgrid, 256, 0, s, keys, weights_dev, n, idx_bits, shift, width, dbits, st_in, st_out, nsplit, l, W,
+                                                thresholds_dev, h_cur, h_other, table_words, done, cand, cand_counts + l, finished,
                                                 const_cast<SelSplit*>(st_in));
         if (!fused)
             launch_chained(sel_pick_kernel, (nsplit + 7) / 8, 256, 0, s, st_in, st_out, nsplit, l, width, dbits, n, W,
@@ -1019,7 +999,7 @@ extern "C" int dynb_sfc_partition(const float* pos_dev, int64_t n_atoms, const i
         int idx_bits = 0;
         const SelSplit* splits = nullptr;
         rc = sel_select_splits(keys, curve_type == 0 ? 63 : 21, weights_dev, n_atoms, nsplit, W, nullptr, ws + L.sel_state, ws + L.sel_hist,
-                               &idx_bits, &splits, false, s);
+                               &idx_bits, &splits, s);
         if (rc) return rc;
         const int hgrid = (int)std::min<int64_t>((n_atoms + 255) / 256, (int64_t)sm_count_cached() * 4);
         launch_chained(sel_label_kernel, hgrid, 256, 0, s, keys, n_atoms, idx_bits, splits, nsplit, labels_dev);
