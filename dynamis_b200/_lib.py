@@ -102,6 +102,8 @@ SIGNATURES = {
     "dynb_halo_mark_from_edges": (_i32, [_p, _i64, _p, _i64, _i64, _i64, _p, _p, _p, _p, _p]),
     "dynb_halo_lists_workspace_bytes": (_i32, [_i64, _i64, ctypes.POINTER(_i64)]),
     "dynb_halo_lists_plan": (_i32, [_p, _p, _p, _i64, _i64, _i64, _p, _p, _i64, _p]),
+    "dynb_halo_lists_plan_words": (_i32, [_p, _p, _p, _i64, _i64, _i64, _p, _p, _i64, _p, _i64, _p]),
+    "dynb_fill_bytes": (_i32, [_p, _i64, _i32, _p]),
     "dynb_halo_lists_fill": (_i32, [_p, _p, _p, _i64, _i64, _i64, _p, _p, _p, _i64, _p, _p, _p, _p, _p, _p, _p]),
     "dynb_csr_workspace_bytes": (_i32, [_i64, _i64, ctypes.POINTER(_i64)]),
     "dynb_csr_plan": (_i32, [_p, _p, _i64, _i64, _i32, _i64, _p, _p, _i64, _p]),

@@ -254,7 +254,7 @@ halo_lists_count_kernel(const HaloSets h, int W, int nblocks, uint32_t* bsum)
 // the totals into offsets [send W + 1 | recv W + 1 | number of own atoms].
 __global__ void __launch_bounds__(SCAN_THREADS)
 halo_lists_scan_kernel(uint32_t* bsum, int nblocks, int W, int64_t* totals, uint32_t* arrived,
-                       int64_t* offsets)
+                       int64_t* offsets, int64_t* words_host, int n_words)
 {
     chain_begin();
     __shared__ uint32_t warp_sums[SCAN_THREADS / 32];
@@ -281,17 +281,23 @@ halo_lists_scan_kernel(uint32_t* bsum, int nblocks, int W, int64_t* totals, uint
         last = atomicAdd(arrived, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
-    __threadfence();
-    for (int which = 0; which < 2; which++) {
-        int64_t run = 0;
-        for (int p = 0; p < W; p++) {
-            offsets[which * (W + 1) + p] = run;
-            run += __ldcg(reinterpret_cast<const long long*>(totals) + which * W + p);
+    if (!last) return;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        for (int which = 0; which < 2; which++) {
+            int64_t run = 0;
+            for (int p = 0; p < W; p++) {
+                offsets[which * (W + 1) + p] = run;
+                run += __ldcg(reinterpret_cast<const long long*>(totals) + which * W + p);
+            }
+            offsets[which * (W + 1) + W] = run;
         }
-        offsets[which * (W + 1) + W] = run;
+        offsets[2 * (W + 1)] = __ldcg(reinterpret_cast<const long long*>(totals) + 2 * W);
     }
-    offsets[2 * (W + 1)] = __ldcg(reinterpret_cast<const long long*>(totals) + 2 * W);
+    // to the caller's pinned memory from here: a copy behind this launch is one of another engine, 10 us
+    if (words_host == nullptr) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_words; i += blockDim.x) words_host[i] = __ldcg(reinterpret_cast<const long long*>(offsets) + i);
 }
 
 struct HaloListsOut {
@@ -689,16 +695,26 @@ static int halo_lists_args(const uint32_t* send_mask_dev, const uint32_t* recv_m
 extern "C" int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
                                     int64_t R, int64_t W, int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream)
 {
+    return dynb_halo_lists_plan_words(send_mask_dev, recv_mask_dev, owner_dev, n, R, W, offsets_dev, workspace_dev, workspace_bytes, nullptr, 0, stream);
+}
+
+extern "C" int dynb_halo_lists_plan_words(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
+                                          int64_t R, int64_t W, int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes,
+                                          int64_t* words_host, int64_t n_words, void* stream)
+{
     HaloSets h;
     int rc = halo_lists_args(send_mask_dev, recv_mask_dev, owner_dev, n, R, W, h);
     if (rc) return rc;
     int64_t need;
     dynb_halo_lists_workspace_bytes(n, W, &need);
     if (offsets_dev == nullptr) return fail_arg("null pointer");
+    if (words_host != nullptr && (n_words < 0 || n_words > 2 * (W + 1) + 2)) return fail_arg("n_words out of range");
     if (workspace_dev == nullptr || workspace_bytes < need) return fail_arg("workspace too small (see dynb_halo_lists_workspace_bytes)");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int64_t* words_view = words_host != nullptr ? static_cast<int64_t*>(device_view_of_host(words_host)) : nullptr;
     if (n == 0) {
         DYNB_CUDA_OK(cudaMemsetAsync(offsets_dev, 0, (size_t)(2 * (W + 1) + 1) * 8, s));
+        if (words_host != nullptr) DYNB_CUDA_OK(cudaMemcpyAsync(words_host, offsets_dev, (size_t)n_words * 8, cudaMemcpyDeviceToHost, s));
         return DYNB_OK;
     }
     const int nb = hl_blocks(n);
@@ -708,8 +724,10 @@ extern "C" int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_
     uint32_t* arrived = reinterpret_cast<uint32_t*>(ws + need - 256);
     DYNB_CUDA_OK(clear_ranges(s, {arrived, 4, 0}));
     launch_chained(halo_lists_count_kernel, nb, HL_THREADS, 0, s, h, (int)W, nb, bsum);
-    launch_chained(halo_lists_scan_kernel, (unsigned)(2 * W + 1), SCAN_THREADS, 0, s, bsum, nb, (int)W, totals, arrived, offsets_dev);
+    launch_chained(halo_lists_scan_kernel, (unsigned)(2 * W + 1), SCAN_THREADS, 0, s, bsum, nb, (int)W, totals, arrived, offsets_dev, words_view, (int)n_words);
     DYNB_CUDA_OK(cudaGetLastError());
+    if (words_host != nullptr && words_view == nullptr)
+        DYNB_CUDA_OK(cudaMemcpyAsync(words_host, offsets_dev, (size_t)n_words * 8, cudaMemcpyDeviceToHost, s));
     return DYNB_OK;
 }
 
@@ -791,6 +809,13 @@ extern "C" int dynb_gather_not_u8(const uint8_t* flags_dev, const int64_t* idx_d
     if (n == 0) return DYNB_OK;
     launch_chained(gather_not_u8_kernel, nblk(n), 256, 0, static_cast<cudaStream_t>(stream), flags_dev, idx_dev, n, out_dev);
     DYNB_CUDA_OK(cudaGetLastError());
+    return DYNB_OK;
+}
+
+extern "C" int dynb_fill_bytes(void* at_dev, int64_t bytes, int byte, void* stream)
+{
+    if (bytes < 0 || (bytes > 0 && at_dev == nullptr)) return fail_arg("bad arguments");
+    DYNB_CUDA_OK(clear_ranges(static_cast<cudaStream_t>(stream), {at_dev, bytes, (uint32_t)byte}));
     return DYNB_OK;
 }
 

@@ -155,34 +155,47 @@ class RadiusGraphPlan:
             unit = torch.empty((E, 3), dtype=torch.float32, device=dev)
             cart = torch.empty((E, 3), dtype=torch.float32, device=dev) if cartesian else None
             if E:
-                cell_h = None
-                if cartesian:
-                    cell_h = np.ascontiguousarray(cell.detach().to("cpu").reshape(3, 3).numpy().astype(np.float32))
+                cell_h = host_cell(cell.reshape(3, 3)) if cartesian else None
                 if id_map is not None:
                     if id_map.dtype != torch.int64 or not id_map.is_contiguous() or id_map.device != dev:
                         raise RuntimeError("id_map must be a contiguous int64 tensor on the graph's device")
-                stream = torch.cuda.current_stream(dev)
                 _lib.check(_lib.lib().dynb_rg_fill_glue(self.ws.data_ptr(), self.dtype_code, edge_index.data_ptr(), unit.data_ptr(),
                                                         cart.data_ptr() if cart is not None else None,
-                                                        cell_h.ctypes.data if cell_h is not None else None,
+                                                        cell_h,
                                                         1 if negate_shifts else 0, id_map.data_ptr() if id_map is not None else None,
-                                                        E, stream.cuda_stream), "rg_fill_glue")
+                                                        E, _lib.stream_of(dev)), "rg_fill_glue")
         return edge_index, unit, cart
 
 
-def _geometry(st: dict, cell_np, pbc_np, radius: float, N: int, dtype_code: int):
+def _host_bytes(t: torch.Tensor) -> bytes:
+    """The values of a small tensor; without array objects in between where it lies on the CPU in one piece (each of these costs
+    about a microsecond, a graph call of a thousand atoms has 80)."""
+    if t.is_cpu and t.is_contiguous() and not t.is_neg() and type(t) is torch.Tensor:
+        return ctypes.string_at(t.data_ptr(), t.numel() * t.element_size())
+    return t.detach().to("cpu").numpy().tobytes()
+
+
+def host_cell(cell: torch.Tensor):
+    """A 3 x 3 cell as nine floats for the library."""
+    if cell.dtype == torch.float32:
+        return (ctypes.c_float * 9).from_buffer_copy(_host_bytes(cell))
+    return (ctypes.c_float * 9).from_buffer_copy(np.ascontiguousarray(cell.detach().to("cpu", torch.float32).numpy()))
+
+
+def _geometry(st: dict, cell: torch.Tensor, pbc: torch.Tensor, radius: float, N: int, dtype_code: int):
     """Host-side conversions and capacities of a geometry, kept by value of (cell, pbc, radius, sizes):
     (key, (cell, pbc, radius, source capacity, cell capacity))."""
-    key = (cell_np.tobytes(), cell_np.dtype.num, pbc_np.tobytes(), pbc_np.dtype.num, float(radius), N, dtype_code)
+    key = (_host_bytes(cell), cell.dtype, _host_bytes(pbc), pbc.dtype, float(radius), N, dtype_code)
     geo = st["geo"].get(key)
     if geo is None:
+        cell_np, pbc_np = cell.detach().to("cpu").numpy(), pbc.detach().to("cpu").numpy()
         np_real = np.float64 if dtype_code == _lib.DYNB_F64 else np.float32
-        cell_h = np.ascontiguousarray(cell_np.astype(np_real))
-        pbc_h = np.ascontiguousarray(pbc_np.astype(bool).astype(np.uint8))
+        cell_h = (ctypes.c_char * (9 * np.dtype(np_real).itemsize)).from_buffer_copy(np.ascontiguousarray(cell_np.astype(np_real)))
+        pbc_h = (ctypes.c_char * 3).from_buffer_copy(np.ascontiguousarray(pbc_np.astype(bool).astype(np.uint8)))
         radius_h = float(np.float32(radius)) if dtype_code == _lib.DYNB_F32 else float(radius)
         src_cap = ctypes.c_int64()
         cell_cap = ctypes.c_int64()
-        _lib.check(_lib.lib().dynb_rg_suggest_capacity(N, cell_h.ctypes.data, pbc_h.ctypes.data, radius_h, dtype_code,
+        _lib.check(_lib.lib().dynb_rg_suggest_capacity(N, cell_h, pbc_h, radius_h, dtype_code,
                                                        ctypes.byref(src_cap), ctypes.byref(cell_cap)), "rg_suggest_capacity")
         if len(st["geo"]) > 64:
             st["geo"].clear()
@@ -211,11 +224,11 @@ class BinnedAtoms:
         self.pos = pos.contiguous()
         self.dtype_code = _lib.DYNB_F64 if pos.dtype == torch.float64 else _lib.DYNB_F32
         self.st = _dev_state(pos.device)
-        # a header of its own: a graph call on the same stream, before done(), writes the stream's
+        # a header of its own: a graph call on the same stream, before done(), writes the stream's.  Pinned words of this object until
+        # it goes; they are not given back, for the launch that writes them may still be queued then.
         self.hdr_t = torch.empty((64,), dtype=torch.uint8, device="cpu", pin_memory=True)
         self.hdr = _lib.RgHeader.from_address(self.hdr_t.data_ptr())
-        self.key, geo = _geometry(self.st, cell.detach().to("cpu").numpy(), pbc.detach().to("cpu").numpy(), radius, pos.size(0),
-                                  self.dtype_code)
+        self.key, geo = _geometry(self.st, cell, pbc, radius, pos.size(0), self.dtype_code)
         self.cell_h, self.pbc_h, self.radius, self.src_capacity, self.cell_capacity = geo
         self.attempts = 0
         self.ws = None
@@ -224,7 +237,7 @@ class BinnedAtoms:
         L, N, dev = _lib.lib(), self.pos.size(0), self.pos.device
         self.ws = _workspace(self.st, _plan_bytes(self.st, N, N, self.src_capacity, self.cell_capacity, self.dtype_code), dev)
         self.attempts += 1
-        _lib.check(L.dynb_rg_bin(self.pos.data_ptr(), self.dtype_code, N, self.cell_h.ctypes.data, self.pbc_h.ctypes.data, self.radius,
+        _lib.check(L.dynb_rg_bin(self.pos.data_ptr(), self.dtype_code, N, self.cell_h, self.pbc_h, self.radius,
                                  self.ws.data_ptr(), self.ws.numel(), self.src_capacity, self.cell_capacity, self.hdr_t.data_ptr(),
                                  _lib.stream_of(dev)), "rg_bin")
 
@@ -252,19 +265,17 @@ def plan_radius_graph(pos, cell, pbc, radius, target_indices=None, want_total: b
     L = _lib.lib()
     dev = pos.device
     dtype_code = _lib.DYNB_F64 if pos.dtype == torch.float64 else _lib.DYNB_F32
-    cell_np = cell.detach().to("cpu").numpy()
-    pbc_np = pbc.detach().to("cpu").numpy()
 
     with _lib.on_device(dev):
         st = _dev_state(dev)
-        geo_key, (cell_h, pbc_h, radius, src_cap, cell_cap) = _geometry(st, cell_np, pbc_np, radius, N, dtype_code)
+        geo_key, (cell_h, pbc_h, radius, src_cap, cell_cap) = _geometry(st, cell, pbc, radius, N, dtype_code)
         counts = torch.empty((Nt,), dtype=torch.int32, device=dev)
         stream = _lib.stream_of(dev)
         hdr = st["hdr"]
         plan = None
         for attempt in range(3):
             ws = _workspace(st, _plan_bytes(st, N, Nt, src_cap, cell_cap, dtype_code), dev)
-            _lib.check(L.dynb_rg_plan(pos.data_ptr(), dtype_code, N, cell_h.ctypes.data, pbc_h.ctypes.data, radius,
+            _lib.check(L.dynb_rg_plan(pos.data_ptr(), dtype_code, N, cell_h, pbc_h, radius,
                                       target_indices.data_ptr() if target_indices is not None else None, Nt,
                                       ws.data_ptr(), ws.numel(), src_cap, cell_cap, counts.data_ptr(),
                                       st["hdr_t"].data_ptr(), stream), "rg_plan")

@@ -9,11 +9,10 @@ from __future__ import annotations
 
 import ctypes
 
-import numpy as np
 import torch
 
 from . import _lib
-from .graph import give_host_words, take_host_words
+from .graph import give_host_words, host_cell, take_host_words
 from .partition import _stream, scratch
 
 
@@ -48,7 +47,7 @@ def filter_edges_to_radius(edges: torch.Tensor, cell_shifts: torch.Tensor, pos: 
     cell_shifts = cell_shifts.contiguous()
     pos = pos.contiguous()
     dev = pos.device
-    cell_h = np.ascontiguousarray(cell.detach().to("cpu", torch.float32).numpy())
+    cell_h = host_cell(cell)
     shifts_f = cell_shifts if cell_shifts.dtype == torch.float32 else cell_shifts.to(torch.float32)
     L = _lib.lib()
     with _lib.on_device(dev):
@@ -56,7 +55,7 @@ def filter_edges_to_radius(edges: torch.Tensor, cell_shifts: torch.Tensor, pos: 
         _lib.check(L.dynb_filter_edges_workspace_bytes(E, ctypes.byref(nbytes)), "filter_edges_workspace_bytes")
         ws = scratch(dev, "filter", nbytes.value)
         cnt = take_host_words(1)   # written by the plan's last kernel
-        _lib.check(L.dynb_filter_edges_plan(edges.data_ptr(), shifts_f.data_ptr(), pos.data_ptr(), cell_h.ctypes.data,
+        _lib.check(L.dynb_filter_edges_plan(edges.data_ptr(), shifts_f.data_ptr(), pos.data_ptr(), cell_h,
                                             float(radius), E, cnt.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev)),
                    "filter_edges_plan")
         torch.cuda.current_stream(dev).synchronize()
@@ -105,24 +104,26 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
         send_mask = torch.empty((max(N, 1), words), dtype=torch.int32, device=dev)
         recv_mask = torch.empty((max(N, 1), words), dtype=torch.int32, device=dev)
         has_remote = torch.empty((max(N, 1),), dtype=torch.uint8, device=dev)
-        offs_bad = torch.zeros((2 * (W + 1) + 2,), dtype=torch.int64, device=dev)  # the offsets and, behind them, the error word
-        offs, bad = offs_bad[:-1], offs_bad[-1:].view(torch.int32)
+        n_words = 2 * (W + 1) + 2
+        offs = torch.empty((n_words,), dtype=torch.int64, device=dev)   # the offsets and, behind them, the error word
+        bad = offs.data_ptr() + 8 * (n_words - 1)
         _lib.check(L.dynb_halo_mark_from_edges(edges.data_ptr(), E, pid.data_ptr(), N, R, W, send_mask.data_ptr(),
-                                               recv_mask.data_ptr(), has_remote.data_ptr(), bad.data_ptr(), _stream(dev)),
+                                               recv_mask.data_ptr(), has_remote.data_ptr(), bad, _stream(dev)),
                    "halo_mark_from_edges")
-        g2l = torch.full((max(N, 1),), -1, dtype=torch.int64, device=dev)
-        _lib.check(L.dynb_scatter_iota(mine.data_ptr(), n_local, N, g2l.data_ptr(), bad.data_ptr(), _stream(dev)), "scatter_iota")
+        g2l = torch.empty((max(N, 1),), dtype=torch.int64, device=dev)
+        _lib.check(L.dynb_fill_bytes(g2l.data_ptr(), 8 * g2l.numel(), 0xFF, _stream(dev)), "fill_bytes")   # -1
+        _lib.check(L.dynb_scatter_iota(mine.data_ptr(), n_local, N, g2l.data_ptr(), bad, _stream(dev)), "scatter_iota")
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_halo_lists_workspace_bytes(N, W, ctypes.byref(nbytes)), "halo_lists_workspace_bytes")
         ws = scratch(dev, "halo_lists", nbytes.value)
-        _lib.check(L.dynb_halo_lists_plan(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, offs.data_ptr(), ws.data_ptr(),
-                                          ws.numel(), _stream(dev)), "halo_lists_plan")
-        offs_h = take_host_words(2 * (W + 1) + 2)
-        offs_h[:2 * (W + 1) + 2].copy_(offs_bad, non_blocking=True)
+        offs_h = take_host_words(n_words)
+        _lib.check(L.dynb_halo_lists_plan_words(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, offs.data_ptr(), ws.data_ptr(),
+                                                ws.numel(), offs_h.data_ptr(), n_words, _stream(dev)), "halo_lists_plan")
+        interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
         torch.cuda.current_stream(dev).synchronize()
-        sizes = offs_h[:2 * (W + 1) + 2].tolist()
+        sizes = offs_h[:n_words].tolist()
         give_host_words(offs_h)
-        if sizes[-1] != 0:
+        if sizes[-1] & 0xFFFFFFFF != 0:
             raise RuntimeError("extract_halo_info: an edge endpoint, partition id or my_outer_atoms entry is out of range")
         total_send, total_recv = sizes[W], sizes[2 * W + 1]
         send_local = torch.empty((total_send,), dtype=torch.int64, device=dev)
@@ -131,7 +132,6 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
         _lib.check(L.dynb_halo_lists_fill(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, g2l.data_ptr(), None,
                                           offs.data_ptr(), n_local, send_local.data_ptr(), recv_atom.data_ptr(), recv_ghost.data_ptr(),
                                           None, None, ws.data_ptr(), _stream(dev)), "halo_lists_fill")
-        interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
         _lib.check(L.dynb_gather_not_u8(has_remote.data_ptr(), mine.data_ptr(), n_local, interior.data_ptr(), _stream(dev)),
                    "gather_not_u8")
         return offs[:W + 1], send_local, offs[W + 1:2 * W + 2], recv_ghost, interior, recv_atom

@@ -204,7 +204,6 @@ class AbstractPartitioner:
             # send offsets, recv offsets, number of own atoms and, behind them, the error word of the marking
             offs = torch.empty((2 * (W + 1) + 2,), dtype=torch.int64, device=dev)
             offs_h = take_host_words(2 * (W + 1) + 2)
-            sizes_h = offs_h[:2 * (W + 1) + 2]
             # everything up to the list sizes is queued before the one wait; the header's status is looked at behind it
             bins = BinnedAtoms(pos32, cell, pbc, ghost_cutoff) if N > 0 else None
             while True:
@@ -212,13 +211,12 @@ class AbstractPartitioner:
                     bins.launch()
                     _lib.check(L.dynb_rg_halo_mark_rank(bins.ws.data_ptr(), bins.dtype_code, pid.data_ptr(), N, W, R, needed.data_ptr(),
                                                         has_foreign.data_ptr(), offs.data_ptr() + 8 * (2 * W + 3), _stream(dev)), "rg_halo_mark")
-                _lib.check(L.dynb_halo_lists_plan(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
-                                                  ws.numel(), _stream(dev)), "halo_lists_plan")
-                sizes_h.copy_(offs, non_blocking=True)
+                _lib.check(L.dynb_halo_lists_plan_words(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
+                                                        ws.numel(), offs_h.data_ptr(), 2 * (W + 1) + 2, _stream(dev)), "halo_lists_plan")
                 torch.cuda.current_stream(dev).synchronize()
                 if bins is None or bins.done():
                     break
-            sizes = sizes_h.tolist()
+            sizes = offs_h[:2 * (W + 1) + 2].tolist()
             give_host_words(offs_h)
             if bins is not None and sizes[2 * W + 3] & 0xFFFFFFFF != 0:
                 raise RuntimeError(f"build_halo_maps: partition_id has a label that is no rank's (world_size is {W})")

@@ -206,6 +206,14 @@ int dynb_halo_mark_from_edges(const int64_t* edges_dev, int64_t E, const int64_t
 int dynb_halo_lists_workspace_bytes(int64_t n, int64_t W, int64_t* bytes);
 int dynb_halo_lists_plan(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
                          int64_t R, int64_t W, int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes, void* stream);
+/* The same; the first n_words of offsets_dev (at most 2 (W + 1) + 2: the offsets, the number of own atoms and one word behind them,
+ * which an earlier launch may have written) go to words_host, too: from the plan's last kernel where that is 16-byte aligned pinned
+ * memory, else by a copy behind it. */
+int dynb_halo_lists_plan_words(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
+                               int64_t R, int64_t W, int64_t* offsets_dev, void* workspace_dev, int64_t workspace_bytes,
+                               int64_t* words_host, int64_t n_words, void* stream);
+/* Every byte of [at_dev, at_dev + bytes) set to `byte`, as a launch of the chain that the library's other kernels form. */
+int dynb_fill_bytes(void* at_dev, int64_t bytes, int byte, void* stream);
 int dynb_halo_lists_fill(const uint32_t* send_mask_dev, const uint32_t* recv_mask_dev, const int64_t* owner_dev, int64_t n,
                          int64_t R, int64_t W, const int64_t* value_map_dev, const uint8_t* has_foreign_dev,
                          const int64_t* offsets_dev, int64_t n_local, int64_t* send_local_dev, int64_t* recv_atom_dev,
