@@ -122,6 +122,9 @@ select_fill_kernel(const int64_t* a, int64_t n, int64_t value, const uint32_t* t
 // For every edge src -> dst of one rank's edge list (dst owned by my_rank): when the source is
 // owned by a peer p, that peer must send src to me (recv side) and I must send dst to p (send
 // side, by the symmetry of the radius graph).
+// Four edges a thread: bound by the latency of an edge's ends and then its owner, which are in flight for all four (5.6 M edges, one edge
+// a thread: 40 us with what it waits for, four 36).
+constexpr int MARK_EDGES = 4;
 __global__ void __launch_bounds__(256)
 halo_mark_edges_kernel(const int64_t* src, const int64_t* dst, int64_t E,
                        const int64_t* pid, int64_t N, int64_t my_rank, int words,
@@ -129,19 +132,36 @@ halo_mark_edges_kernel(const int64_t* src, const int64_t* dst, int64_t E,
                        uint8_t* has_remote, uint32_t* bad)
 {
     chain_begin();
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    const int64_t s = src[e], d = dst[e];
-    if (s < 0 || s >= N || d < 0 || d >= N) { atomicOr(bad, 1u); return; }
-    const int64_t p = pid[s];
-    if (p == my_rank) return;
-    if (p < 0 || p >= (int64_t)words * 32) { atomicOr(bad, 2u); return; }
-    const uint32_t bit = 1u << (p & 31);
-    uint32_t* rw = &recv_mask[s * words + (p >> 5)];
-    if (!(*rw & bit)) atomicOr(rw, bit);
-    uint32_t* sw = &send_mask[d * words + (p >> 5)];
-    if (!(*sw & bit)) atomicOr(sw, bit);
-    has_remote[d] = 1;
+    const int64_t e0 = (int64_t)blockIdx.x * (MARK_EDGES * 256) + threadIdx.x;
+    int64_t s[MARK_EDGES], d[MARK_EDGES], owner[MARK_EDGES];
+#pragma unroll
+    for (int k = 0; k < MARK_EDGES; k++) {
+        const bool in = e0 + 256 * k < E;
+        s[k] = in ? src[e0 + 256 * k] : 0;
+        d[k] = in ? dst[e0 + 256 * k] : 0;
+    }
+    // my_rank: nothing to do
+    uint32_t wrong = 0u;
+#pragma unroll
+    for (int k = 0; k < MARK_EDGES; k++) {
+        owner[k] = my_rank;
+        if (e0 + 256 * k >= E) continue;
+        if (s[k] < 0 || s[k] >= N || d[k] < 0 || d[k] >= N) wrong |= 1u;
+        else owner[k] = pid[s[k]];
+    }
+#pragma unroll
+    for (int k = 0; k < MARK_EDGES; k++) {
+        const int64_t p = owner[k];
+        if (p == my_rank) continue;
+        if (p < 0 || p >= (int64_t)words * 32) { wrong |= 2u; continue; }
+        const uint32_t bit = 1u << (p & 31);
+        uint32_t* rw = &recv_mask[s[k] * words + (p >> 5)];
+        if (!(*rw & bit)) atomicOr(rw, bit);
+        uint32_t* sw = &send_mask[d[k] * words + (p >> 5)];
+        if (!(*sw & bit)) atomicOr(sw, bit);
+        has_remote[d[k]] = 1;
+    }
+    if (wrong) atomicOr(bad, wrong);
 }
 
 // ------------------------------------------------------------------------------------------ halo lists
@@ -567,19 +587,37 @@ edge_compact_kernel(const int64_t* edges, const unsigned char* shifts_raw, int s
     int total;
     const int before = warp_excl_scan(__popc(mine), lane, &total);
     const int64_t first = tile_first[blockIdx.x];
+    // all edges of the thread are asked for before the first is written (one by one 51 us for 5.6 M edges, together 33)
+    int64_t from[FILTER_ROUNDS], to[FILTER_ROUNDS], place[FILTER_ROUNDS];
+    float h[FILTER_ROUNDS][3];
+    const bool floats = shift_row_bytes == 12;
 #pragma unroll
     for (int k = 0; k < FILTER_ROUNDS; k++) {
         const uint32_t word = __shfl_sync(0xffffffffu, mine, 8 * k + warp);
         const int64_t o = first + __shfl_sync(0xffffffffu, before, 8 * k + warp) + __popc(word & lanemask_lt());
-        if (!((word >> lane) & 1u)) continue;
         const int64_t e = (int64_t)blockIdx.x * FILTER_TILE + 256 * k + threadIdx.x;
-        edges_out[o] = edges[e];
-        edges_out[E_out + o] = edges[E + e];
-        if (shift_row_bytes == 12) {
+        place[k] = ((word >> lane) & 1u) ? o : -1;
+        if (place[k] < 0) continue;
+        from[k] = edges[e];
+        to[k] = edges[E + e];
+        if (floats) {
             const float* a = reinterpret_cast<const float*>(shifts_raw) + 3 * e;
+#pragma unroll
+            for (int c = 0; c < 3; c++) h[k][c] = a[c];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < FILTER_ROUNDS; k++) {
+        const int64_t o = place[k];
+        if (o < 0) continue;
+        edges_out[o] = from[k];
+        edges_out[E_out + o] = to[k];
+        if (floats) {
             float* b = reinterpret_cast<float*>(shifts_out) + 3 * o;
-            b[0] = a[0]; b[1] = a[1]; b[2] = a[2];
+#pragma unroll
+            for (int c = 0; c < 3; c++) b[c] = h[k][c];
         } else {
+            const int64_t e = (int64_t)blockIdx.x * FILTER_TILE + 256 * k + threadIdx.x;
             for (int i = 0; i < shift_row_bytes; i++) shifts_out[o * shift_row_bytes + i] = shifts_raw[e * shift_row_bytes + i];
         }
     }
@@ -666,7 +704,7 @@ extern "C" int dynb_halo_mark_from_edges(const int64_t* edges_dev, int64_t E, co
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     DYNB_CUDA_OK(clear_ranges(s, {send_mask_dev, N * words * 4, 0}, {recv_mask_dev, N * words * 4, 0}, {has_remote_dev, N, 0}, {bad_dev, 4, 0}));
     if (E == 0) return DYNB_OK;
-    launch_chained(halo_mark_edges_kernel, nblk(E), 256, 0, s, edges_dev, edges_dev + E, E, pid_dev, N, my_rank, words, send_mask_dev,
+    launch_chained(halo_mark_edges_kernel, nblk(E, MARK_EDGES * 256), 256, 0, s, edges_dev, edges_dev + E, E, pid_dev, N, my_rank, words, send_mask_dev,
                                                    recv_mask_dev, has_remote_dev, bad_dev);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
