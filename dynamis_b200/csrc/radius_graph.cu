@@ -1929,9 +1929,16 @@ rg_fillmask_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts
 // The same with squared distances: a warp stages {record number, shift code} of its group's candidates and reads each target's
 // mask words; the position and the atom id of a hit come from the cell-sorted records (a group's few hundred records stay in
 // L1), and the edges of a target are ordered by candidate place, as rg_pair_kernel writes them: a slot's hits are placed by one
-// ballot.  131 k atoms, 6.9 M edges: 158 us when every pair was tested again by that kernel, 115 us from the hit bits.
+// ballot and a predicated store.  Bound by instructions (the loop over the slots) and the latency of the records.  131 k atoms, 6.9 M
+// edges: 158 us when every pair
+// was tested again by that kernel, 118 us from the hit bits with a branch a slot and the lane mask read again every time, 96 now.
 // ------------------------------------------------------------------------------------------
 constexpr int FM_META = RG_MASK_SLOTS * 32;                       // staged candidate records per warp
+// A place of the list at `at` (shared memory) if there is a hit: a predicated store, no branch.
+__device__ __forceinline__ void put_place(uint32_t hit, uint32_t at, uint32_t place)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.u16 [%1], %2;\n\t}" ::"r"(hit), "r"(at), "h"((unsigned short)place) : "memory");
+}
 constexpr int FM_WARP_BYTES = FM_META * 8 + FM_META * 2 + RUN_INDEX_BYTES;    // records + one parked slot per possible hit
 
 template <typename T>
@@ -1942,13 +1949,15 @@ rg_fillmask_dist_kernel(const PairParams<T>* params_dev, long long* ei, float* s
     chain_begin();
     const PairParams<T> p = *params_dev;
     extern __shared__ __align__(32) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
     unsigned char* wbase = smem_raw + warp * FM_WARP_BYTES;
     uint2* meta = reinterpret_cast<uint2*>(wbase);
     unsigned short* list = reinterpret_cast<unsigned short*>(wbase + FM_META * 8);
     int* delta = reinterpret_cast<int*>(wbase + FM_META * 8 + FM_META * 2);
     uint32_t* flags = reinterpret_cast<uint32_t*>(delta + 32);
-    const uint32_t le = lanemask_lt() | (1u << (threadIdx.x & 31));
+    uint32_t lt;
+    asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));   // volatile: kept in a register instead of read again
+    const uint32_t le = lt | (1u << lane), list_at = (uint32_t)__cvta_generic_to_shared(list);
 
     const DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
@@ -1959,7 +1968,6 @@ rg_fillmask_dist_kernel(const PairParams<T>* params_dev, long long* ei, float* s
     const uint32_t num_groups = p.glist ? hp->active_groups : (uint32_t)hp->num_groups;
     const int Wd = 2 * pad + 1, Wy = Sy + 2 * pad, nrun = Wy * Wd;
     const int lane_dy = (lane % Wy) - pad, lane_dz = (lane / Wy) - pad;
-    const uint32_t lt = lanemask_lt();
 
     // target ranges and source run of a group; the next group's are requested while the current group
     // is written, so that one round trip to memory per group (the candidate records) stays exposed
@@ -2053,27 +2061,61 @@ rg_fillmask_dist_kernel(const PairParams<T>* params_dev, long long* ei, float* s
                 const uint32_t t = qa < n0 ? tb[0] + qa : tb[1] + (qa - n0);
                 ntm = p.tmeta[t]; nbase = p.toffset[t]; nw = p.hitmask[(size_t)t * 32 + lane];
             }
-            int cnt = 0;
             __syncwarp();
-            for (int slot = 0; slot < nslots; slot++) {
-                const bool hit = (w >> slot) & 1u;
-                const uint32_t m = __ballot_sync(0xffffffffu, hit);
-                if (hit) list[cnt + __popc(m & lt)] = (unsigned short)(slot * 32 + lane);
-                cnt += __popc(m);
+            // the hits slot by slot, four slots a step: the mask has no bits behind the list's end
+            uint32_t at = list_at, place = (uint32_t)lane;
+#pragma unroll 1
+            for (int s0 = 0; s0 < nslots; s0 += 4) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint32_t hit = w & (1u << u), m = __ballot_sync(0xffffffffu, hit != 0u);
+                    put_place(hit, at + 2u * (uint32_t)__popc(m & lt), place + 32u * u);
+                    at += 2u * (uint32_t)__popc(m);
+                }
+                w >>= 4;
+                place += 128u;
             }
+            const int cnt = (int)(at - list_at) >> 1;
             __syncwarp();
             const int sx = tm.y - 512, sy = tm.z - 512, sz = tm.w - 512;
-            for (int i = lane; i < cnt; i += 32) {
-                const uint2 m = meta[list[i]];
-                const uint32_t code = m.y;
-                const long long e = base + i;
-                const Vec4<T> c = p.spos[m.x];
-                d2out[e] = dist2<T>(tp.x, tp.y, tp.z, c.x, c.y, c.z);
-                ei[e] = (long long)real_to_bits(c.w);
-                ei[E + e] = (long long)tm.x;
-                shifts[3 * e + 0] = (float)((int)(code & 1023u) + sx);
-                shifts[3 * e + 1] = (float)((int)((code >> 10) & 1023u) + sy);
-                shifts[3 * e + 2] = (float)((int)((code >> 20) & 1023u) + sz);
+            if (sizeof(T) == 4 && cnt > 32) {
+                // two rounds of 32 edges, both rounds' records asked for before the first edge is written (103 -> 96 us; up to 32 edges
+                // it is a round for nothing, and in double, with twice the registers to a record, 994 -> 1009 us a call of 500 k atoms at 5.5 A)
+                for (int i0 = 0; i0 < cnt; i0 += 64) {
+                    uint2 m[2];
+                    Vec4<T> c[2];
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        m[k] = meta[list[min(i0 + 32 * k + lane, cnt - 1)]];
+                        c[k] = p.spos[m[k].x];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        const int i = i0 + 32 * k + lane;
+                        if (i >= cnt) break;
+                        const uint32_t code = m[k].y;
+                        const long long e = base + i;
+                        d2out[e] = dist2<T>(tp.x, tp.y, tp.z, c[k].x, c[k].y, c[k].z);
+                        ei[e] = (long long)real_to_bits(c[k].w);
+                        ei[E + e] = (long long)tm.x;
+                        shifts[3 * e + 0] = (float)((int)(code & 1023u) + sx);
+                        shifts[3 * e + 1] = (float)((int)((code >> 10) & 1023u) + sy);
+                        shifts[3 * e + 2] = (float)((int)((code >> 20) & 1023u) + sz);
+                    }
+                }
+            } else {
+                for (int i = lane; i < cnt; i += 32) {
+                    const uint2 m = meta[list[i]];
+                    const uint32_t code = m.y;
+                    const long long e = base + i;
+                    const Vec4<T> c = p.spos[m.x];
+                    d2out[e] = dist2<T>(tp.x, tp.y, tp.z, c.x, c.y, c.z);
+                    ei[e] = (long long)real_to_bits(c.w);
+                    ei[E + e] = (long long)tm.x;
+                    shifts[3 * e + 0] = (float)((int)(code & 1023u) + sx);
+                    shifts[3 * e + 1] = (float)((int)((code >> 10) & 1023u) + sy);
+                    shifts[3 * e + 2] = (float)((int)((code >> 20) & 1023u) + sz);
+                }
             }
         }
     }
