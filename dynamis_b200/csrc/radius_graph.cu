@@ -1930,8 +1930,8 @@ rg_fillmask_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts
 // mask words; the position and the atom id of a hit come from the cell-sorted records (a group's few hundred records stay in
 // L1), and the edges of a target are ordered by candidate place, as rg_pair_kernel writes them: a slot's hits are placed by one
 // ballot and a predicated store.  Bound by instructions (the loop over the slots) and the latency of the records.  131 k atoms, 6.9 M
-// edges: 158 us when every pair
-// was tested again by that kernel, 118 us from the hit bits with a branch a slot and the lane mask read again every time, 96 now.
+// edges: 158 us when every pair was tested again by that kernel, 118 us from the hit bits with a branch a slot and the lane mask read
+// again every time, 96 now.
 // ------------------------------------------------------------------------------------------
 constexpr int FM_META = RG_MASK_SLOTS * 32;                       // staged candidate records per warp
 // A place of the list at `at` (shared memory) if there is a hit: a predicated store, no branch.
