@@ -858,6 +858,13 @@ __device__ __forceinline__ int runs_flags(uint32_t* flags, int run_off, int run_
     return __popc(before);
 }
 
+// The mask of the lanes below, likewise: read again where it is used it was 24 of 530 instructions a target.
+__device__ __forceinline__ uint32_t lanes_below()
+{
+    uint32_t m;
+    asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    return m;
+}
 __device__ __forceinline__ int lane_id()
 {
     int l;
@@ -1091,7 +1098,7 @@ rg_group_list_kernel(const PairParams<T>* params_dev, uint32_t* glist)
 // hold the records of the targets' own cell rows, for records elsewhere are further away (targets next to the faces of these rows are
 // tested again in full); for these two blocks to be the same registers in every group the blocks are loaded in turned order.
 // The bits of a target go to shared memory and leave it, with the degrees, for 16 targets together.
-// Bound by the latency of its loads, its issue slots (60 % busy) and the FMA pipe (40 %): 162 instructions a target of the liquid, 56 of
+// Bound by the latency of its loads, its issue slots (60 % busy) and the FMA pipe (40 %): 156 instructions a target of the liquid, 56 of
 // them tests; 207 without the items above.  Before and after: 266 -> 207 us (liquid, 1 M atoms, 5 A), 309 -> 259 (a rank's 1 M of the
 // 8 M copper atoms), 177 -> 163 (silicon in double precision, 500 k atoms, 6 A), 46 -> 39 (liquid, 131 k), 9.5 -> 8.3 (1 k).
 // Distances from the matrix units (halves of split coordinates, pairs near the cutoff again) took 482 us: operand moves and the
@@ -1931,7 +1938,7 @@ rg_fillmask_kernel(const PairParams<T>* params_dev, long long* ei, float* shifts
 // L1), and the edges of a target are ordered by candidate place, as rg_pair_kernel writes them: a slot's hits are placed by one
 // ballot and a predicated store.  Bound by instructions (the loop over the slots) and the latency of the records.  131 k atoms, 6.9 M
 // edges: 158 us when every pair was tested again by that kernel, 118 us from the hit bits with a branch a slot and the lane mask read
-// again every time, 96 now.
+// again every time, 96 without, 89 with the look-up by two loads a lane.
 // ------------------------------------------------------------------------------------------
 constexpr int FM_META = RG_MASK_SLOTS * 32;                       // staged candidate records per warp
 // A place of the list at `at` (shared memory) if there is a hit: a predicated store, no branch.
@@ -1955,52 +1962,20 @@ rg_fillmask_dist_kernel(const PairParams<T>* params_dev, long long* ei, float* s
     unsigned short* list = reinterpret_cast<unsigned short*>(wbase + FM_META * 8);
     int* delta = reinterpret_cast<int*>(wbase + FM_META * 8 + FM_META * 2);
     uint32_t* flags = reinterpret_cast<uint32_t*>(delta + 32);
-    uint32_t lt;
-    asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));   // volatile: kept in a register instead of read again
-    const uint32_t le = lt | (1u << lane), list_at = (uint32_t)__cvta_generic_to_shared(list);
+    const uint32_t lt = lanes_below(), le = lt | (1u << lane), list_at = (uint32_t)__cvta_generic_to_shared(list);
 
     const DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
     if (total != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *total = E;
-    const int nx = hp->nx, ny = hp->ny, nz = hp->nz, S = hp->group_cells, Sy = hp->group_cells_y, pad = hp->pad;
-    const uint32_t gx = (uint32_t)hp->gx;
-    const uint32_t gy = (uint32_t)((ny + Sy - 1) / Sy);
+    __shared__ GroupShape shape;
+    if (threadIdx.x == 0) shape = group_shape(hp);
     const uint32_t num_groups = p.glist ? hp->active_groups : (uint32_t)hp->num_groups;
-    const int Wd = 2 * pad + 1, Wy = Sy + 2 * pad, nrun = Wy * Wd;
-    const int lane_dy = (lane % Wy) - pad, lane_dz = (lane / Wy) - pad;
-
-    // target ranges and source run of a group; the next group's are requested while the current group
-    // is written, so that one round trip to memory per group (the candidate records) stays exposed
-    struct GroupDesc { uint32_t tb0, te0, tb1, te1; int run_a, run_len; };
-    auto fetch = [&](uint32_t gi) -> GroupDesc {
-        GroupDesc d;
-        const uint32_t grp = p.glist ? p.glist[gi] : gi;
-        const uint32_t row = grp / gx;
-        const int ix = (int)(grp - row * gx);
-        const int cz = (int)(row / gy), iy = (int)(row - (uint32_t)cz * gy);
-        const int cx0 = ix * S, cx1 = min(cx0 + S, nx) - 1;
-        const int cy0 = iy * Sy, cy1 = min(cy0 + Sy, ny) - 1;
-        d.tb0 = p.tcstart[((uint32_t)cz * ny + cy0) * nx + cx0];
-        d.te0 = p.tcstart[((uint32_t)cz * ny + cy0) * nx + cx1 + 1];
-        d.tb1 = d.te1 = 0;
-        if (cy1 > cy0) {
-            d.tb1 = p.tcstart[((uint32_t)cz * ny + cy1) * nx + cx0];
-            d.te1 = p.tcstart[((uint32_t)cz * ny + cy1) * nx + cx1 + 1];
-        }
-        d.run_a = 0;
-        d.run_len = 0;
-        if (lane < nrun) {
-            const int yy = cy0 + lane_dy, zz = cz + lane_dz;
-            if (yy >= 0 && yy < ny && yy <= cy1 + pad && zz >= 0 && zz < nz) {
-                const uint32_t b = ((uint32_t)zz * ny + yy) * nx;
-                const uint32_t a = p.cstart[b + max(cx0 - pad, 0)];
-                const uint32_t e = p.cstart[b + min(cx1 + pad, nx - 1) + 1];
-                d.run_a = (int)a;
-                d.run_len = (int)(e - a);
-            }
-        }
-        return d;
-    };
+    __syncthreads();
+    // the next group is looked up while the current one is written, so that one round trip to memory per group (the candidate
+    // records) stays exposed
+    const int which = group_lane(shape, lane);
+    const uint32_t* const cells = lane >= GROUP_ROW_LANE ? p.tcstart : p.cstart;
+    auto fetch = [&](uint32_t i) { return fetch_group(shape, cells, p.glist ? p.glist[i] : i, which); };
 
     const uint32_t nwarps = gridDim.x * PAIR_WARPS;
     uint32_t grp = blockIdx.x * PAIR_WARPS + warp;
@@ -2009,9 +1984,10 @@ rg_fillmask_dist_kernel(const PairParams<T>* params_dev, long long* ei, float* s
     for (; grp < num_groups; grp += nwarps) {
         const GroupDesc d = nd;
         if (grp + nwarps < num_groups) nd = fetch(grp + nwarps);
-        uint32_t tb[2] = {d.tb0, d.tb1}, te[2] = {d.te0, d.te1};
+        const uint32_t tb[2] = {__shfl_sync(0xffffffffu, (uint32_t)d.run_a, GROUP_ROW_LANE), __shfl_sync(0xffffffffu, (uint32_t)d.run_a, GROUP_ROW_LANE + 1)};
+        const uint32_t te[2] = {__shfl_sync(0xffffffffu, (uint32_t)d.run_e, GROUP_ROW_LANE), __shfl_sync(0xffffffffu, (uint32_t)d.run_e, GROUP_ROW_LANE + 1)};
         if (tb[0] == te[0] && tb[1] == te[1]) continue;
-        const int run_a = d.run_a, run_len = d.run_len;
+        const int run_a = d.run_a, run_len = lane < GROUP_ROW_LANE ? d.run_e - d.run_a : 0;
         // the first target's words do not depend on the candidate records: ask for them now
         int4 ntm;
         long long nbase;
