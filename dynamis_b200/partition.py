@@ -58,12 +58,12 @@ class SFCCurveType(enum.IntEnum):
 
 
 def launches_per_partition() -> int:
-    """Kernels one Morton partition of a million atoms into 8 labels launches (labels only): bounds (1),
-    keys (1), 6 digit levels (histogram; its last block advances the split points; once the remaining atoms are few
-    the last block settles the split points and the later levels return at once), labels (1).  With the
-    curve-order permutation requested the sorted path runs instead: bounds, keys, 8 radix passes x
-    (histogram + 2 scan kernels + scatter), assignment."""
-    return 1 + 1 + 6 + 1
+    """Kernels one Morton partition of a million atoms into 8 labels launches (labels only): bounds (2, the first
+    clears them), keys (1), 6 digit levels (the first behind a launch that clears its table; histogram; its last block
+    advances the split points; once the remaining atoms are few the last block settles the split points and the later
+    levels return at once), labels (1).  With the curve-order permutation requested the sorted path runs instead: bounds,
+    keys, 8 radix passes x (histogram + 2 scan kernels + scatter), assignment."""
+    return 2 + 1 + 1 + 6 + 1
 
 
 def sfc_partition_labels(pos: torch.Tensor, weights: Optional[torch.Tensor], W: int, curve_type: int = 0,
