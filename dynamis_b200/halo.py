@@ -116,10 +116,10 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_halo_lists_workspace_bytes(N, W, ctypes.byref(nbytes)), "halo_lists_workspace_bytes")
         ws = scratch(dev, "halo_lists", nbytes.value)
-        offs_h = take_host_words(n_words)
+        interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
+        offs_h = take_host_words(n_words)   # nothing that can raise between the launch that writes them and the wait
         _lib.check(L.dynb_halo_lists_plan_words(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, offs.data_ptr(), ws.data_ptr(),
                                                 ws.numel(), offs_h.data_ptr(), n_words, _stream(dev)), "halo_lists_plan")
-        interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
         torch.cuda.current_stream(dev).synchronize()
         sizes = offs_h[:n_words].tolist()
         give_host_words(offs_h)
