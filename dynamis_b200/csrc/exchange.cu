@@ -347,11 +347,10 @@ __device__ unsigned long long scatter_stride(int64_t total, int64_t piece)
 // that NVLink stores and the HBM copy run side by side.
 template <typename V>
 __global__ void __launch_bounds__(256, 3)
-halo_forward_begin_kernel(dynb_halo_ctx c, const V* x, int64_t n_local, int64_t q, int64_t row_bytes,
-                          const int64_t* send_local, int64_t total_send, unsigned char* out_head,
+halo_forward_begin_kernel(dynb_halo_ctx c, const V* __restrict__ x, int64_t n_local, int64_t q, int64_t row_bytes,
+                          const int64_t* __restrict__ send_local, int64_t total_send, unsigned char* __restrict__ out_head,
                           int head_vb, uint32_t gen, uint32_t announce, int skip_push)
 {
-    chain_begin();
     __shared__ PeerSeg seg[PUSH_MAX_TARGETS];
     for (int k = threadIdx.x; k < c.world_size; k += blockDim.x) {
         const dynb_halo_peer p = c.peers[k];
@@ -392,10 +391,9 @@ halo_forward_begin_kernel(dynb_halo_ctx c, const V* x, int64_t n_local, int64_t 
 // and — when the rows arrived in the staging buffer rather than in the result itself — their copy into
 // the result's tail.
 __global__ void __launch_bounds__(256)
-halo_forward_end_kernel(dynb_halo_ctx c, uint32_t gen, unsigned long long budget_ns, const unsigned char* stage,
-                        unsigned char* out_tail, int64_t tail_bytes, int tail_vb)
+halo_forward_end_kernel(dynb_halo_ctx c, uint32_t gen, unsigned long long budget_ns, const unsigned char* __restrict__ stage,
+                        unsigned char* __restrict__ out_tail, int64_t tail_bytes, int tail_vb)
 {
-    chain_begin();
     wait_all(c, 0, gen, budget_ns);
     if (blockIdx.x == 0) drift_or(c, 0, gen);
     if (out_tail != nullptr && tail_bytes > 0) copy_span(out_tail, stage, tail_bytes, tail_vb, blockIdx.x, gridDim.x);
@@ -405,11 +403,10 @@ halo_forward_end_kernel(dynb_halo_ctx c, uint32_t gen, unsigned long long budget
 // gradient rows of owned atoms that receive nothing -> result (has_recv == nullptr: all owned rows); signal.
 template <typename V>
 __global__ void __launch_bounds__(256, 3)
-halo_backward_begin_kernel(dynb_halo_ctx c, const V* g, int64_t n_local, int64_t n_ghost, int64_t q,
-                           int64_t row_bytes, const uint8_t* has_recv, unsigned char* out, int out_vb,
+halo_backward_begin_kernel(dynb_halo_ctx c, const V* __restrict__ g, int64_t n_local, int64_t n_ghost, int64_t q,
+                           int64_t row_bytes, const uint8_t* __restrict__ has_recv, unsigned char* __restrict__ out, int out_vb,
                            uint32_t gen)
 {
-    chain_begin();
     __shared__ PeerSeg seg[PUSH_MAX_TARGETS];
     for (int k = threadIdx.x; k < c.world_size; k += blockDim.x) {
         const dynb_halo_peer p = c.peers[k];
@@ -445,12 +442,11 @@ halo_backward_begin_kernel(dynb_halo_ctx c, const V* g, int64_t n_local, int64_t
 // out[row] = g[row] + the received rows that name it, in the fixed order of inv_entries.
 template <typename T, typename V, int VW, bool NARROW>   // NARROW: fewer than 32 columns, several rows side by side
 __global__ void __launch_bounds__(256, 4)
-halo_backward_end_kernel(dynb_halo_ctx c, uint32_t gen, unsigned long long budget_ns, const V* g,
-                         const int64_t* rows, const uint32_t* row_first, int64_t n_rows, int64_t q,
-                         const V* recv, const int64_t* inv_offsets,
-                         const uint32_t* inv_entries, V* out)
+halo_backward_end_kernel(dynb_halo_ctx c, uint32_t gen, unsigned long long budget_ns, const V* __restrict__ g,
+                         const int64_t* __restrict__ rows, const uint32_t* __restrict__ row_first, int64_t n_rows, int64_t q,
+                         const V* __restrict__ recv, const int64_t* __restrict__ inv_offsets,
+                         const uint32_t* __restrict__ inv_entries, V* __restrict__ out)
 {
-    chain_begin();
     // Two listed rows per warp and step (rows of fewer than 32 columns side by side), 16 bytes of each row per lane.  Bound by
     // HBM and by the chain row id -> place in the inverse CSR -> row; so each step's loads are issued together: the rows of
     // this step, the places of the next, the ids of the one after, and only the ids and places of a warp's first step come
@@ -682,9 +678,9 @@ extern "C" int dynb_halo_forward_begin(const dynb_halo_ctx* ctx, const void* x_d
     const int hv = span_vb(x_dev, out_head_dev, 0);
     const unsigned g = fused_grid((total_send + (out_head_dev ? n_local : 0)) * row_bytes / 16 + 1);
     unsigned char* oh = static_cast<unsigned char*>(out_head_dev);
-    if (vb == 16) launch_chained(halo_forward_begin_kernel<uint4>, g, 256, 0, s, *ctx, static_cast<const uint4*>(x_dev), n_local, q, row_bytes, send_local_dev, total_send, oh, hv, gen, announce_slot, skip_push);
-    else if (vb == 4) launch_chained(halo_forward_begin_kernel<uint32_t>, g, 256, 0, s, *ctx, static_cast<const uint32_t*>(x_dev), n_local, q, row_bytes, send_local_dev, total_send, oh, hv, gen, announce_slot, skip_push);
-    else launch_chained(halo_forward_begin_kernel<uint8_t>, g, 256, 0, s, *ctx, static_cast<const uint8_t*>(x_dev), n_local, q, row_bytes, send_local_dev, total_send, oh, hv, gen, announce_slot, skip_push);
+    if (vb == 16) halo_forward_begin_kernel<uint4><<<g, 256, 0, s>>>(*ctx, static_cast<const uint4*>(x_dev), n_local, q, row_bytes, send_local_dev, total_send, oh, hv, gen, announce_slot, skip_push);
+    else if (vb == 4) halo_forward_begin_kernel<uint32_t><<<g, 256, 0, s>>>(*ctx, static_cast<const uint32_t*>(x_dev), n_local, q, row_bytes, send_local_dev, total_send, oh, hv, gen, announce_slot, skip_push);
+    else halo_forward_begin_kernel<uint8_t><<<g, 256, 0, s>>>(*ctx, static_cast<const uint8_t*>(x_dev), n_local, q, row_bytes, send_local_dev, total_send, oh, hv, gen, announce_slot, skip_push);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -697,7 +693,8 @@ extern "C" int dynb_halo_forward_end(const dynb_halo_ctx* ctx, uint32_t gen, int
     if (out_tail_dev != nullptr && tail_bytes > 0 && stage_dev == nullptr) return fail_arg("null pointer");
     const bool copy = out_tail_dev != nullptr && tail_bytes > 0;
     const unsigned g = copy ? fused_grid(tail_bytes / 16 + 1) : 1u;
-    launch_chained(halo_forward_end_kernel, g, 256, 0, static_cast<cudaStream_t>(stream), *ctx, gen, (unsigned long long)timeout_ns, static_cast<const unsigned char*>(stage_dev),
+    halo_forward_end_kernel<<<g, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        *ctx, gen, (unsigned long long)timeout_ns, static_cast<const unsigned char*>(stage_dev),
         static_cast<unsigned char*>(out_tail_dev), tail_bytes, span_vb(stage_dev, out_tail_dev, 0));
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
@@ -716,9 +713,9 @@ extern "C" int dynb_halo_backward_begin(const dynb_halo_ctx* ctx, const void* gr
     const uint8_t* hr = (vb == 16 && ov == 16 && row_bytes >= 64) ? has_recv_dev : nullptr;  // short rows: plain copy
     const unsigned g = fused_grid((n_local + n_ghost) * row_bytes / 16 + 1);
     unsigned char* o = static_cast<unsigned char*>(out_dev);
-    if (vb == 16) launch_chained(halo_backward_begin_kernel<uint4>, g, 256, 0, s, *ctx, static_cast<const uint4*>(grad_dev), n_local, n_ghost, q, row_bytes, hr, o, ov, gen);
-    else if (vb == 4) launch_chained(halo_backward_begin_kernel<uint32_t>, g, 256, 0, s, *ctx, static_cast<const uint32_t*>(grad_dev), n_local, n_ghost, q, row_bytes, hr, o, ov, gen);
-    else launch_chained(halo_backward_begin_kernel<uint8_t>, g, 256, 0, s, *ctx, static_cast<const uint8_t*>(grad_dev), n_local, n_ghost, q, row_bytes, hr, o, ov, gen);
+    if (vb == 16) halo_backward_begin_kernel<uint4><<<g, 256, 0, s>>>(*ctx, static_cast<const uint4*>(grad_dev), n_local, n_ghost, q, row_bytes, hr, o, ov, gen);
+    else if (vb == 4) halo_backward_begin_kernel<uint32_t><<<g, 256, 0, s>>>(*ctx, static_cast<const uint32_t*>(grad_dev), n_local, n_ghost, q, row_bytes, hr, o, ov, gen);
+    else halo_backward_begin_kernel<uint8_t><<<g, 256, 0, s>>>(*ctx, static_cast<const uint8_t*>(grad_dev), n_local, n_ghost, q, row_bytes, hr, o, ov, gen);
     DYNB_CUDA_OK(cudaGetLastError());
     return DYNB_OK;
 }
@@ -745,7 +742,7 @@ extern "C" int dynb_halo_backward_end(const dynb_halo_ctx* ctx, uint32_t gen, in
     auto launch = [&](auto kernel, auto* g, auto* recv, auto* out) {
         const int64_t warps = narrow ? (n_rows * q + 31) / 32 : n_rows;
         const unsigned blocks = std::min<unsigned>(grid_for(warps * 32), sm_count_cached() * 4);
-        launch_chained(kernel, blocks, 256, 0, s, *ctx, gen, bud, g, rows_dev, row_first_dev, n_rows, q, recv, inv_offsets_dev, inv_entries_dev, out);
+        kernel<<<blocks, 256, 0, s>>>(*ctx, gen, bud, g, rows_dev, row_first_dev, n_rows, q, recv, inv_offsets_dev, inv_entries_dev, out);
     };
     auto run = [&](auto wide_kernel, auto narrow_kernel, auto* g, auto* recv, auto* out) {
         if (narrow) launch(narrow_kernel, g, recv, out);
