@@ -1644,12 +1644,12 @@ rg_pair_kernel(const PairParams<T>* params_dev, long long* ei,
 // what belongs to its bits into the warp's buffer; the buffer goes out 32 edges at a time.
 // In most groups all candidates have one shift code, and then all shifts are zero (the targets are candidates too): zeros are
 // written 32 bytes a lane, and a group's edges need the two indices only.
-// Bound by the latency of its loads and by instructions (192 M warp instructions, issue slots 57 % busy), not by the 1.47 GB it
-// writes (4.8 TB/s).  Target by target, with a prefix sum, a list and two rounds of 32 edges for each of them, and three
+// Bound by the latency of its loads and by instructions (4 an edge, issue slots 57 % busy), not by the 1.47 GB it writes (4.9 TB/s).  Target by target, with a prefix sum, a list and two rounds of 32 edges for each of them, and three
 // stores with a stride of 12 bytes for the shifts: 240 M.  Before and after: 381 -> 308 us (liquid, 1 M atoms), 742 -> 611 (a
 // rank's 1 M of the 8 M copper atoms, with Cartesian shifts), 189 -> 160 (silicon, double precision), 15 -> 13 (1 k atoms, where
 // every group is at the boundary), 25 -> 25 (32 k atoms).  What is loaded ahead is not touched until its turn: a subtraction
-// behind the loads of the next group's runs or of the rows' places in the output waits for them (322 -> 308 us).
+// behind the loads of the next group's runs or of the rows' places in the output waits for them (322 -> 308 us).  298 with the look-up by
+// two loads a lane (fetch_group).
 // Bulk copies of a block of zeros for the shifts: no gain.
 // ------------------------------------------------------------------------------------------
 constexpr int FM_TABLE = 33 * (RG_MASK_SLOTS * 32 / 32);   // a word of padding every 32 bits: the lanes of a slot fall into 32 banks
