@@ -1419,21 +1419,23 @@ rg_count_kernel(const PairParams<T> p)
                 auto run = [&](auto nb, auto full) {
                     count_group<T, decltype(nb)::value, decltype(full)::value>(p, w, cells, test, max_degree, lane, le);
                 };
-                // Copies of the test loop for 2, 4, 5, 6, 7 and 8 blocks of 64; one block is tested as two and three as four, with
-                // padding
-                if (everywhere) {
-                    run(std::integral_constant<int, 8>(), std::true_type());
-                } else {
-                    switch ((clen + 63) >> 6) {
-                    case 1:
-                    case 2: run(std::integral_constant<int, 2>(), std::false_type()); break;
-                    case 3:
-                    case 4: run(std::integral_constant<int, 4>(), std::false_type()); break;
-                    case 5: run(std::integral_constant<int, 5>(), std::false_type()); break;
-                    case 6: run(std::integral_constant<int, 6>(), std::false_type()); break;
-                    case 7: run(std::integral_constant<int, 7>(), std::false_type()); break;
-                    default: run(std::integral_constant<int, 8>(), std::false_type()); break;
-                    }
+                // Copies of the test loop for 2, 4, 5, 6, 7 and 8 blocks of 64, with both tests everywhere for 2, 4 and 8; a chunk takes the
+                // smallest that holds it, with padding.  The last chunk of a list is often short: 200 k atoms of the liquid, degrees
+                // alone, at 7 A (512 + 32 places) 222 us with the copy for 8 blocks for all chunks and 199 so, at 9 A (512 + 512 + 131) 247
+                // and 224.  No copies for 5, 6 and 7: what the loop saves the instruction cache loses (8 A, 512 + 300: 212 us with
+                // one for 5, 207 without; in double 287 and 266; 245 and 355 with the copy for 8 inlined twice).
+                const int blocks = (clen + 63) >> 6;
+                switch (everywhere && blocks > 2 ? (blocks > 4 ? 10 : 9) : blocks) {
+                case 1:
+                case 2: run(std::integral_constant<int, 2>(), std::true_type()); break;
+                case 3:
+                case 4: run(std::integral_constant<int, 4>(), std::false_type()); break;
+                case 5: run(std::integral_constant<int, 5>(), std::false_type()); break;
+                case 6: run(std::integral_constant<int, 6>(), std::false_type()); break;
+                case 7: run(std::integral_constant<int, 7>(), std::false_type()); break;
+                case 8: run(std::integral_constant<int, 8>(), std::false_type()); break;
+                case 9: run(std::integral_constant<int, 4>(), std::true_type()); break;
+                default: run(std::integral_constant<int, 8>(), std::true_type()); break;
                 }
             }
             // a group whose neighbourhood holds no source at all still owes its targets a zero
