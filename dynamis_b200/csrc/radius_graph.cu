@@ -1104,8 +1104,10 @@ rg_group_list_kernel(const PairParams<T>* params_dev, uint32_t* glist)
 // Distances from the matrix units (halves of split coordinates, pairs near the cutoff again) took 482 us: operand moves and the
 // 8 cycles of an m16n8k16.  The next group's look-up, or its candidates, copied ahead to shared memory: 218 and 231 us.
 // ------------------------------------------------------------------------------------------
-// Five blocks of four warps: 96 registers, hardly any spills.  Six and 80: 213 us, 284 for the rank's copper.  Eight waves of blocks in
-// place of the counter: 222.
+// Five blocks of four warps: 96 registers; float without spills, double with 104 bytes of stores and 112 of loads.  Six and 80: 213 us, 284 for
+// the rank's copper.  Eight waves of blocks in place of the counter: 222.  Double with four, five, six and seven blocks, degrees of 200 k
+// atoms of the liquid, whole call: 219, 222, 219 and 217 us at 6 A, 254, 259, 269 and 274 at 7 A; the crystal on a shell (exact_hits_call)
+// 428, 400, 401 and 360.
 constexpr int COUNT_WARPS = 4;
 constexpr int COUNT_BLOCKS = 5;
 constexpr int COUNT_TARGETS = 16;   // staged together
@@ -1171,6 +1173,7 @@ struct CountGroup {
     int turn;                      // block of 64 that the first registers hold
     float ylo, yhi, zlo, zhi;      // where a target's cell coordinates are clear of the faces of its rows
     int write_masks, first, last, all_exact;
+    uint32_t unsettled;            // double: targets that the float tests outside the own rows (FULL: anywhere) leave open
     __device__ __forceinline__ uint32_t target(uint32_t k) const volatile { return k < n0 ? tb0 + k : tb1 + (k - n0); }
 };
 struct CountWarp {
@@ -1183,28 +1186,42 @@ struct CountWarp {
 struct CountCells { float gmin_y, gmin_z, res_inv; };
 
 // The candidates of a target given by `which` (bit s: place 32 s + lane of the chunk) by the expression that decides.
-template <typename T>
-__device__ __forceinline__ uint32_t exact_hits(const Vec4<T>* spos, const Vec4<T>* target, const T r2, uint32_t which, const RunIndex& index, int cbeg, int clen,
-                                               int lane, uint32_t le)
+__device__ __forceinline__ uint32_t exact_hits(const Vec4<float>* spos, const Vec4<float>* target, const float r2, uint32_t which, const RunIndex& index, int cbeg,
+                                               int clen, int lane, uint32_t le)
 {
     uint32_t hits = 0;
     while (which) {
         const int s = __ffs((int)which) - 1, j = 32 * s + lane;
         which &= which - 1;
         if (j >= clen) continue;  // padding
-        const Vec4<T> c = spos[index.record(s, le) + cbeg + j], a = *target;
-        const T d = dist2<T>(a.x, a.y, a.z, c.x, c.y, c.z);
-        if (d <= r2 && d > (T)1e-8f) hits |= 1u << s;
+        const Vec4<float> c = spos[index.record(s, le) + cbeg + j], a = *target;
+        const float d = dist2<float>(a.x, a.y, a.z, c.x, c.y, c.z);
+        if (d <= r2 && d > 1e-8f) hits |= 1u << s;
     }
     return hits;
 }
 // Out of line in double, where it is called for every target with an undecided candidate: the copies of the test loop overran the
 // instruction cache (176 us against 160, silicon of 500 k atoms).  In single precision the call costs more (207 against 224, liquid of 1 M).
+// Two records in flight: the crystal with its cutoff on a shell, below, takes 430 us with one, 402 with two, 418 with three, 446 with four.
 __device__ __noinline__ uint32_t exact_hits_call(const Vec4<double>* spos, const Vec4<double>* target, const double r2, uint32_t which, const RunIndex& index,
                                                  int cbeg, int clen)
 {
     const int lane = lane_id();
-    return exact_hits<double>(spos, target, r2, which, index, cbeg, clen, lane, 0xffffffffu >> (31 - lane));
+    const uint32_t le = 0xffffffffu >> (31 - lane);
+    const Vec4<double> a = *target;
+    uint32_t hits = 0;
+    while (which) {
+        // the second may be the first again; a padding place reads the last record
+        const int s0 = __ffs((int)which) - 1;
+        which &= which - 1;
+        const int s1 = which ? __ffs((int)which) - 1 : s0, j0 = 32 * s0 + lane, j1 = 32 * s1 + lane;
+        which &= which - 1;
+        const Vec4<double> c0 = spos[index.record(s0, le) + cbeg + min(j0, clen - 1)], c1 = spos[index.record(s1, le) + cbeg + min(j1, clen - 1)];
+        const double d0 = dist2<double>(a.x, a.y, a.z, c0.x, c0.y, c0.z), d1 = dist2<double>(a.x, a.y, a.z, c1.x, c1.y, c1.z);
+        if (j0 < clen && d0 <= r2 && d0 > (double)1e-8f) hits |= 1u << s0;
+        if (j1 < clen && d1 <= r2 && d1 > (double)1e-8f) hits |= 1u << s1;
+    }
+    return hits;
 }
 
 // The targets of a group against the chunk's candidates, at most 64 NB of them.  FULL: both tests for all blocks.
@@ -1212,7 +1229,7 @@ template <typename T, int NB, bool FULL>
 __device__ __forceinline__ void count_group(const PairParams<T>& p, CountWarp& w, const volatile CountCells& cells, const CountTests& test, int& max_degree, const int lane,
                                             const uint32_t le)
 {
-    const volatile CountGroup& g = w.group;
+    volatile CountGroup& g = w.group;
     constexpr int OWN = FULL ? NB : 2;
     constexpr uint32_t ALL_BITS = 0xffffu >> (16 - 2 * NB);
     unsigned long long cx[NB], cy[NB], cz[NB];
@@ -1288,22 +1305,26 @@ __device__ __forceinline__ void count_group(const PairParams<T>& p, CountWarp& w
             auto turned = [&](uint32_t v) { return ((v | (v << (2 * NB))) >> turn) & ALL_BITS; };
             bits = turned(bits);
             if constexpr (sizeof(T) == 8) {
+                const uint32_t undecided = turned(maybe) & ~bits & turned(0xffffu >> (16 - 2 * OWN));
                 if (!g.all_exact) {
-                    const uint32_t undecided = turned(maybe) & ~bits & turned(0xffffu >> (16 - 2 * OWN));
                     if (undecided) bits |= exact_hits_call(p.spos, p.tpos + g.target(k0 + k), p.r2, undecided, w.index, g.cbeg, g.clen);
                 }
-                if (!FULL && closest <= test.half) again |= 1u << k;
+                if (FULL ? undecided != 0u : closest <= test.half) again |= 1u << k;
             }
             w.mask[k][lane] = (unsigned short)bits;
         }
         __syncwarp();
-        if (sizeof(T) == 8) again = __reduce_or_sync(0xffffffffu, again);
+        if (sizeof(T) == 8) {
+            again = __reduce_or_sync(0xffffffffu, again);
+            if (again && lane == 0) g.unsettled = g.unsettled + __popc(again);
+            if (FULL && !g.all_exact) again = 0u;
+        }
 #pragma unroll 1
         for (; again; again &= again - 1) {
             const int k = __ffs((int)again) - 1;
             uint32_t bits;
             if constexpr (sizeof(T) == 8) bits = exact_hits_call(p.spos, p.tpos + g.target(k0 + k), p.r2, ALL_BITS, w.index, g.cbeg, g.clen);
-            else bits = exact_hits<T>(p.spos, p.tpos + g.target(k0 + k), p.r2, ALL_BITS, w.index, g.cbeg, g.clen, lane, le);
+            else bits = exact_hits(p.spos, p.tpos + g.target(k0 + k), p.r2, ALL_BITS, w.index, g.cbeg, g.clen, lane, le);
             w.mask[k][lane] = (unsigned short)bits;
             __syncwarp();
         }
@@ -1347,6 +1368,7 @@ rg_count_kernel(const PairParams<T> p)
     DevHeader* hp = p.h;
     if (hp->status & RG_FATAL) return;
     int warp_max_slots = 0, max_degree = 0;
+    if (lane == 0) w.group.unsettled = w.group.ntot = 0u;
     if (threadIdx.x == 0) {
         shape = group_shape(hp);
         // double positions are scanned relative to the grid's origin
@@ -1381,7 +1403,12 @@ rg_count_kernel(const PairParams<T> p)
         volatile CountGroup& g = w.group;   // all lanes write the same
         const uint32_t n0 = d.te0 - d.tb0, ntot = n0 + (d.te1 - d.tb1);
         if (ntot != 0) {
+            // Double: a target that is tested again takes three or four times the loop (all places of its list by the deciding expression), so both tests
+            // everywhere where more than one in 16 of the warp's group before were.  Degrees of 512 k atoms of an ideal silicon crystal with the cutoff on
+            // a shell of neighbours, whole call: 865 us without this line, 402 with it (253 off the shell, with and without).
+            const bool unsettled = sizeof(T) == 8 && 16u * g.unsettled > g.ntot;
             __syncwarp();
+            if (sizeof(T) == 8) g.unsettled = 0u;
             g.tb0 = d.tb0;
             g.tb1 = d.tb1;
             g.n0 = n0;
@@ -1408,7 +1435,7 @@ rg_count_kernel(const PairParams<T> p)
             for (int cbeg = 0; cbeg < L; cbeg += RG_MASK_SLOTS * 32) {
                 const int clen = min(RG_MASK_SLOTS * 32, L - cbeg);
                 // both tests everywhere where the own records are not in two blocks, and in lists of several chunks
-                const bool everywhere = L > RG_MASK_SLOTS * 32 || ((own_end - 1) >> 6) - (own_beg >> 6) > 1;
+                const bool everywhere = unsettled || L > RG_MASK_SLOTS * 32 || ((own_end - 1) >> 6) - (own_beg >> 6) > 1;
                 __syncwarp();
                 g.cbeg = cbeg;
                 g.clen = clen;
