@@ -894,6 +894,15 @@ struct RunIndex {
         if (lane < RUN_FLAG_WORDS) word[lane] = make_uint2(f, rank - 1u);
         __syncwarp();
     }
+    // the same for a list of up to 64 places: its first two words, from registers (that gas: 826 -> 800 us)
+    __device__ __forceinline__ void set_short(int run_a, int run_off, int run_len, int lane, uint32_t lt)
+    {
+        runs_compact(delta, run_a, run_off, run_len, lt);
+        const uint32_t start = run_len > 0 ? 1u << (run_off & 31) : 0u;
+        const uint32_t f0 = __reduce_or_sync(0xffffffffu, run_off < 32 ? start : 0u), f1 = __reduce_or_sync(0xffffffffu, run_off < 32 ? 0u : start);
+        if (lane < 2) word[lane] = lane == 0 ? make_uint2(f0, 0xffffffffu) : make_uint2(f1, (uint32_t)__popc(f0) - 1u);
+        __syncwarp();
+    }
     // record - place, for place 32 s + lane of the chunk
     __device__ __forceinline__ int record(int s, uint32_t le) const
     {
@@ -1267,9 +1276,12 @@ __device__ __forceinline__ void count_group(const PairParams<T>& p, CountWarp& w
                 w.target[lane][0] = make_float4(v.x, v.x, v.y, v.y);
                 w.target[lane][1] = make_float4(v.z, v.z, v.w, 0.0f);
             }
-            const float fy = (v.y - cells.gmin_y) * cells.res_inv, fz = (v.z - cells.gmin_z) * cells.res_inv;
-            const bool clear = fy > g.ylo && fy < g.yhi && fz > g.zlo && fz < g.zhi;
-            again = __ballot_sync(0xffffffffu, lane < n && (g.all_exact || (!FULL && !clear)));
+            if constexpr (!FULL) {
+                const float fy = (v.y - cells.gmin_y) * cells.res_inv, fz = (v.z - cells.gmin_z) * cells.res_inv;
+                const bool clear = fy > g.ylo && fy < g.yhi && fz > g.zlo && fz < g.zhi;
+                again = __ballot_sync(0xffffffffu, lane < n && !clear);
+            }
+            if (sizeof(T) == 8 && g.all_exact) again = 0xffffu >> (COUNT_TARGETS - n);
             __syncwarp();
         }
 #pragma unroll 1
@@ -1320,7 +1332,7 @@ __device__ __forceinline__ void count_group(const PairParams<T>& p, CountWarp& w
             if (FULL && !g.all_exact) again = 0u;
         }
 #pragma unroll 1
-        for (; again; again &= again - 1) {
+        for (; !(FULL && sizeof(T) == 4) && again; again &= again - 1) {
             const int k = __ffs((int)again) - 1;
             uint32_t bits;
             if constexpr (sizeof(T) == 8) bits = exact_hits_call(p.spos, p.tpos + g.target(k0 + k), p.r2, ALL_BITS, w.index, g.cbeg, g.clen);
@@ -1384,6 +1396,10 @@ rg_count_kernel(const PairParams<T> p)
         test.half = 1.001f * fmaxf(middle - hp->test_lo, hp->test_hi - middle);
     }
     const uint32_t num_groups = p.glist ? hp->active_groups : (uint32_t)hp->num_groups;  // < 2^31: never more groups than cells
+    // Groups are taken one by one, or, from 128 a warp on, several in a row (a power of two, 64 to 128 takings a warp): every taking is an
+    // addition to one address, and a thin gas has a group for every atom or two.  Degrees of 1 M atoms, 0.001 per A^3, 5 A, whole call: 937 us one by
+    // one, 876 so; 300 k atoms in dense pockets of a gas 402 and 295.
+    if (threadIdx.x == 0) shape.unused[0] = 1 << (31 - __clz((int)max(num_groups / (64u * COUNT_WARPS * gridDim.x), 1u)));
     __syncthreads();
     const int lane_run = group_lane_run(shape, lane);
     const bool all_exact = sizeof(T) == 8 && hp->test_lo < 0.0f;  // coordinates out of the float test's range (float_test)
@@ -1392,12 +1408,16 @@ rg_count_kernel(const PairParams<T> p)
     const float skin = 1.01f * sqrtf(sizeof(T) == 8 ? hp->test_near : 1e-8f) * (float)hp->res_inv + 1e-6f * (float)(16 + max(hp->ny, hp->nz));
 
     const uint32_t nwarps = gridDim.x * COUNT_WARPS;
-    uint32_t gi = blockIdx.x * COUNT_WARPS + warp;
+    const volatile int& in_a_row = shape.unused[0];
+    uint32_t gi = (blockIdx.x * COUNT_WARPS + warp) * (uint32_t)in_a_row;
 #pragma unroll 1
     while (gi < num_groups) {
         const uint32_t grp = p.glist ? p.glist[gi] : gi;
-        uint32_t following = 0;
-        if (lane == 0) following = nwarps + atomicAdd(&hp->count_next, 1u);
+        uint32_t following = gi + 1u;
+        if (lane == 0) {
+            const uint32_t taken = (uint32_t)in_a_row;
+            if ((following & (taken - 1u)) == 0u) following = nwarps * taken + atomicAdd(&hp->count_next, taken);
+        }
         const GroupRows d = fetch_group_rows(shape, p.tcstart, p.cstart, grp, lane_run);
         const int run_a = d.run_a, run_len = d.run_e - d.run_a;
         volatile CountGroup& g = w.group;   // all lanes write the same
@@ -1442,18 +1462,19 @@ rg_count_kernel(const PairParams<T> p)
                 g.first = cbeg == 0;
                 g.last = cbeg + RG_MASK_SLOTS * 32 >= L;
                 g.turn = everywhere ? 0 : own_beg >> 6;
-                w.index.set(run_a, run_off, run_len, cbeg, lane, lt);
+                if (L <= 64) w.index.set_short(run_a, run_off, run_len, lane, lt);
+                else w.index.set(run_a, run_off, run_len, cbeg, lane, lt);
                 auto run = [&](auto nb, auto full) {
                     count_group<T, decltype(nb)::value, decltype(full)::value>(p, w, cells, test, max_degree, lane, le);
                 };
-                // Copies of the test loop for 2, 4, 5, 6, 7 and 8 blocks of 64, with both tests everywhere for 2, 4 and 8; a chunk takes the
+                // Copies of the test loop for 1, 2, 4, 5, 6, 7 and 8 blocks of 64, with both tests everywhere for 1, 2, 4 and 8; a chunk takes the
                 // smallest that holds it, with padding.  The last chunk of a list is often short: 200 k atoms of the liquid, degrees
                 // alone, at 7 A (512 + 32 places) 222 us with the copy for 8 blocks for all chunks and 199 so, at 9 A (512 + 512 + 131) 247
                 // and 224.  No copies for 5, 6 and 7: what the loop saves the instruction cache loses (8 A, 512 + 300: 212 us with
-                // one for 5, 207 without; in double 287 and 266; 245 and 355 with the copy for 8 inlined twice).
+                // one for 5, 207 without; in double 287 and 266; 245 and 355 with the copy for 8 inlined twice).  The one for 1: that gas 876 -> 826.
                 const int blocks = (clen + 63) >> 6;
                 switch (everywhere && blocks > 2 ? (blocks > 4 ? 10 : 9) : blocks) {
-                case 1:
+                case 1: run(std::integral_constant<int, 1>(), std::true_type()); break;
                 case 2: run(std::integral_constant<int, 2>(), std::true_type()); break;
                 case 3:
                 case 4: run(std::integral_constant<int, 4>(), std::false_type()); break;
