@@ -1374,6 +1374,7 @@ rg_count_kernel(const PairParams<T> p)
     __shared__ GroupShape shape;
     __shared__ CountCells cells;
     __shared__ CountTests test;
+    constexpr bool ONE_BLOCK = sizeof(T) == 4;   // a copy of the loop for one block of 64
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     CountWarp& w = warps[warp];
     const uint32_t lt = lanemask_lt(), le = lt | (1u << lane);
@@ -1462,19 +1463,20 @@ rg_count_kernel(const PairParams<T> p)
                 g.first = cbeg == 0;
                 g.last = cbeg + RG_MASK_SLOTS * 32 >= L;
                 g.turn = everywhere ? 0 : own_beg >> 6;
-                if (L <= 64) w.index.set_short(run_a, run_off, run_len, lane, lt);
+                if (ONE_BLOCK && L <= 64) w.index.set_short(run_a, run_off, run_len, lane, lt);   // no more than its two words are read below
                 else w.index.set(run_a, run_off, run_len, cbeg, lane, lt);
                 auto run = [&](auto nb, auto full) {
                     count_group<T, decltype(nb)::value, decltype(full)::value>(p, w, cells, test, max_degree, lane, le);
                 };
-                // Copies of the test loop for 1, 2, 4, 5, 6, 7 and 8 blocks of 64, with both tests everywhere for 1, 2, 4 and 8; a chunk takes the
+                // Copies of the test loop for 1 (float), 2, 4, 5, 6, 7 and 8 blocks of 64, with both tests everywhere for 1, 2, 4 and 8; a chunk takes the
                 // smallest that holds it, with padding.  The last chunk of a list is often short: 200 k atoms of the liquid, degrees
                 // alone, at 7 A (512 + 32 places) 222 us with the copy for 8 blocks for all chunks and 199 so, at 9 A (512 + 512 + 131) 247
                 // and 224.  No copies for 5, 6 and 7: what the loop saves the instruction cache loses (8 A, 512 + 300: 212 us with
-                // one for 5, 207 without; in double 287 and 266; 245 and 355 with the copy for 8 inlined twice).  The one for 1: that gas 876 -> 826.
+                // one for 5, 207 without; in double 287 and 266; 245 and 355 with the copy for 8 inlined twice).  The one for 1, that gas: 876 ->
+                // 826; in double it costs the others (jittered silicon of 500 k atoms 268 -> 278 us).
                 const int blocks = (clen + 63) >> 6;
                 switch (everywhere && blocks > 2 ? (blocks > 4 ? 10 : 9) : blocks) {
-                case 1: run(std::integral_constant<int, 1>(), std::true_type()); break;
+                case 1: if constexpr (ONE_BLOCK) { run(std::integral_constant<int, 1>(), std::true_type()); break; }
                 case 2: run(std::integral_constant<int, 2>(), std::true_type()); break;
                 case 3:
                 case 4: run(std::integral_constant<int, 4>(), std::false_type()); break;
