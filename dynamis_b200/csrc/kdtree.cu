@@ -52,8 +52,8 @@ __device__ __forceinline__ void kd_child_sizes(const KdSeg& g, long long sz, lon
 }
 
 // What the levels need before the first: the tree and the labels of its leaves (as a kernel argument while they fit; three copies from
-// host memory and a memset: 242 us a call of 1 M atoms against 233), the one segment's size, and every atom in that segment (the
-// array is padded to 16 bytes in the workspace).
+// host memory and a memset: 242 us a call of 1 M atoms against 233), the one segment's size, and every atom in that segment (16 bytes a
+// store: the array starts on such a boundary where the workspace does, and is padded to one).
 constexpr int KD_SETUP_BYTES = 3072;
 struct KdSetup { __align__(8) unsigned char bytes[KD_SETUP_BYTES]; };
 __global__ void __launch_bounds__(256)
@@ -320,6 +320,7 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
         return DYNB_OK;
     }
     if (workspace_dev == nullptr) return fail_arg("null workspace");
+    if (reinterpret_cast<uintptr_t>(workspace_dev) % 8 != 0) return fail_arg("the workspace must start on an 8-byte boundary");
     const KdLayout L = kd_layout(n, W);
     if (workspace_bytes < L.total) return fail_arg("workspace too small (see dynb_kdtree_workspace_bytes)");
     unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
@@ -372,7 +373,7 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
     int64_t label = 0;
     for (size_t k = 0; k < parts.size(); k++) { base[k] = label; label += parts[k]; }
     const int64_t tree_bytes = (int64_t)(segs.size() * sizeof(KdSeg)), label_bytes = (int64_t)base.size() * 8;
-    if (tree_bytes + label_bytes <= KD_SETUP_BYTES) {
+    if (tree_bytes + label_bytes <= KD_SETUP_BYTES && reinterpret_cast<uintptr_t>(seg_cur) % 16 == 0) {
         KdSetup setup;
         memcpy(setup.bytes, segs.data(), (size_t)tree_bytes);
         memcpy(setup.bytes + tree_bytes, base.data(), (size_t)label_bytes);

@@ -818,7 +818,8 @@ int sel_select_splits(const uint64_t* keys, int key_bits, const int64_t* weights
     const bool fused = nsplit <= SEL_FINISH_SPLITS;  // two rounds of eight warps in the last block
     // early finish (fused path only): candidates in the split-point slots of state buffer 0 that no level uses,
     // one list counter per level behind the arrival counters, then the "finished" word
-    SelCand* cand = fused ? reinterpret_cast<SelCand*>(st + SEL_FINISH_SPLITS) : nullptr;
+    // (the records are read 16 bytes at a time: a workspace off such a boundary goes through all levels instead)
+    SelCand* cand = fused && reinterpret_cast<uintptr_t>(st) % 16 == 0 ? reinterpret_cast<SelCand*>(st + SEL_FINISH_SPLITS) : nullptr;
     unsigned int* cand_counts = counters + 16;
     unsigned int* finished = counters + 48;
     if (levels > 16) return fail_arg("too many digit levels");

@@ -407,7 +407,8 @@ int dynb_drift_flag(const float* cur_dev, const float* ref_dev, const float* vel
  * counts).  Atoms with equal coordinates are ordered by ascending index; weights are summed exactly
  * (the reference uses a float32 cumulative sum, identical while the sums stay below 2^24).
  * method 0: equal-count cuts by selection (no sort), weighted cuts by a stable sort; method 1: sorted
- * cuts for both (same labels; kept so that the two routes can be checked against each other). */
+ * cuts for both (same labels; kept so that the two routes can be checked against each other).  The workspace starts on an
+ * 8-byte boundary, better on a 16-byte one: off these the selection takes all its levels and the tree is copied from the host. */
 int dynb_kdtree_workspace_bytes(int64_t n_atoms, int64_t W, int64_t* bytes);
 int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, const int64_t* weights_dev, int64_t W,
                           int64_t* labels_dev, int method, void* workspace_dev, int64_t workspace_bytes, void* stream);
