@@ -343,16 +343,20 @@ __global__ void __launch_bounds__(256) u32_to_i64_kernel(const uint32_t* a, int6
 
 // Distinct prefixes of the live split points (they are non-decreasing) into glist (loaded by the whole
 // block, compacted in place).  All threads of the block call this; returns the number of groups.
-__device__ int sel_groups(const SelSplit* __restrict__ st, int nsplit, u128* glist, int* gid_of_split)
+__device__ int sel_groups(const SelSplit* __restrict__ st, int nsplit, u128* glist, int* gid_of_split, unsigned* atoms = nullptr)
 {
     __shared__ int s_ng;
     __shared__ int s_live;
-    if (threadIdx.x == 0) s_live = nsplit;
+    if (threadIdx.x == 0) {
+        s_live = nsplit;
+        if (atoms != nullptr) *atoms = 0u;
+    }
     __syncthreads();
     for (int s = threadIdx.x; s < nsplit; s += blockDim.x) {
         const SelSplit v = st[s];
         glist[s] = sel_prefix(v);
         if (v.dead) atomicMin(&s_live, s);  // dead split points are the last ones
+        else if (atoms != nullptr) atomicAdd(atoms, (unsigned)v.atoms);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -564,6 +568,35 @@ __device__ bool sel_finish_warp(const SelSplit& me, int g, const SelCand* cand, 
     return true;
 }
 
+// Counters of a block for additions of one to a table in memory: the first counter that meets each place is kept here, the others are
+// added to where they are.  Additions of a block to a few counters leave the SM as one each.
+template <unsigned N>
+struct SelKept {
+    static constexpr unsigned NONE = 0xffffffffu;
+    unsigned which[N], count[N];
+    __device__ __forceinline__ void begin()
+    {
+        for (unsigned k = threadIdx.x; k < N; k += 256) { which[k] = NONE; count[k] = 0u; }
+    }
+    __device__ __forceinline__ void add(unsigned long long* table, unsigned at)
+    {
+        const unsigned place = (at ^ (at >> 8)) % N;
+        unsigned kept = *static_cast<volatile unsigned*>(&which[place]);
+        if (kept == NONE) {
+            kept = atomicCAS(&which[place], NONE, at);
+            if (kept == NONE) kept = at;
+        }
+        if (kept == at) atomicAdd(&count[place], 1u);
+        else atomicAdd(&table[at], 1ull);
+    }
+    __device__ __forceinline__ void end(unsigned long long* table)
+    {
+        for (unsigned k = threadIdx.x; k < N; k += 256)
+            if (count[k]) atomicAdd(&table[which[k]], (unsigned long long)count[k]);
+    }
+};
+constexpr unsigned SEL_KEEP_FROM = 32768;   // atoms that a level behind the first counts: fewer are added to the table as they come
+
 // Table of one level: per group 2^dbits digit counters ("fine"), followed by per group 256 coarse
 // counters, one per run of 2^fbits consecutive digits (fbits = min(width, 8)), so that a split point is
 // located by reading 256 + 256 counters instead of the whole digit range.
@@ -583,8 +616,21 @@ sel_hist_kernel(const uint64_t* keys, const int64_t* weights, int64_t n, int idx
     __shared__ int gid[SEL_MAX_SPLITS];
     __shared__ unsigned long long s_coarse[256];  // weighted; 64-bit shared additions are compare-and-swap loops
     __shared__ unsigned int s_coarse_unit[256];   // unit weights
-    __shared__ bool s_last, s_listed;
+    // Unit weights: digits, and behind the first level runs of digits, of keys that crowd into a few of them (an outlier, clusters far from
+    // one another): additions of a million atoms to a few addresses of memory take 90 us and more a level.  KD-tree of 1 M atoms on 8 ranks: even
+    // 215 us, without these counters 215; one atom at 1e6 253 and 1250; two clusters 292 and 1917; twelve 309 and 787; the curve of
+    // 1 M atoms with that atom 120 and 783.
+    // They lie behind the prefixes of fewer split points than there may be: with 4 KB more a block the next kernel of the chain finds no room beside four
+    // blocks of this one (a curve of 1 M atoms, 64 labels: 198 -> 220 us).
+    constexpr int ROOM = 256;   // split points that they take the places of
+    static_assert(sizeof(SelKept<512>) <= ROOM * sizeof(u128) && sizeof(SelKept<256>) <= ROOM * sizeof(unsigned long long), "room for the counters");
+    SelKept<512>& s_digits = *reinterpret_cast<SelKept<512>*>(glist + SEL_MAX_SPLITS - ROOM);
+    SelKept<256>& s_runs = *reinterpret_cast<SelKept<256>*>(glist64 + SEL_MAX_SPLITS - ROOM);
+    const bool may_keep = weights == nullptr && nsplit <= SEL_MAX_SPLITS - ROOM;
+    __shared__ unsigned s_atoms;   // that this level counts
+    __shared__ bool s_last;
     bool listing = false;   // this level lists its atoms
+    bool keep = may_keep;
     // cand != nullptr: the early finish is in use (see above); finished: set by the level that settled the split points
     if (cand != nullptr && __ldcg(finished) != 0u) return;
     // clear the table the next level accumulates into (its last reader, the previous pick, has finished)
@@ -597,17 +643,24 @@ sel_hist_kernel(const uint64_t* keys, const int64_t* weights, int64_t n, int idx
         if (threadIdx.x == 0) glist[0] = 0;
         s_coarse[threadIdx.x] = 0ull;  // one group, every atom counts: coarse counters through shared memory
         s_coarse_unit[threadIdx.x] = 0u;
+        if (keep) s_digits.begin();
         __syncthreads();
     } else {
-        ng = sel_groups(st, nsplit, glist, gid);
+        ng = sel_groups(st, nsplit, glist, gid, &s_atoms);
         if (cand != nullptr && threadIdx.x == 0) {
             long long atoms = 0;
             for (int k = 0; k < nsplit; k++)
                 if (gid[k] >= 0 && (k == 0 || gid[k] != gid[k - 1])) atoms += st[k].atoms;
-            s_listed = atoms <= (long long)SEL_CAND_CAP;
+            s_atoms = (unsigned)atoms;
         }
         __syncthreads();
-        listing = cand != nullptr && s_listed;
+        listing = cand != nullptr && s_atoms <= (unsigned)SEL_CAND_CAP;
+        keep = may_keep && s_atoms > SEL_KEEP_FROM;
+        if (keep) {
+            s_digits.begin();
+            s_runs.begin();
+            __syncthreads();
+        }
     }
     const u128 dmask = ((u128)1 << width) - 1;
     // A level above the index's bits: prefix and digit are of the key alone, in 64 bits (a million keys, a KD-tree of a million atoms: 208 us with 128-bit prefixes everywhere, 201 so).
@@ -685,26 +738,26 @@ sel_hist_kernel(const uint64_t* keys, const int64_t* weights, int64_t n, int idx
                         }
                     }
                 }
-                // Unit weights: a warp whose atoms all fall on one counter adds them together.  Keys of a system with an outlier crowd
-                // into a few first digits, and a million additions to one address take 90 us and more.
-                unsigned together = 0u;
-                if (weights == nullptr) {
-                    const unsigned counted = __ballot_sync(0xffffffffu, w != 0ull);
-                    int same = 0;
-                    if (w) __match_all_sync(counted, (unsigned)slot, &same);
-                    if (w && same) together = counted;
-                }
-                if (together != 0u) {
-                    w = (together & lanemask_lt()) == 0u ? (unsigned long long)__popc(together) : 0ull;
-                }
                 if (w) {
-                    atomicAdd(&hist[slot], w);
-                    if (level > 0) atomicAdd(&coarse[((size_t)lo << 8) + (digit >> fbits)], w);
-                    else if (weights) atomicAdd(&s_coarse[digit >> fbits], w);
-                    else atomicAdd(&s_coarse_unit[digit >> fbits], (unsigned)w);
+                    const unsigned run = ((unsigned)lo << 8) + (digit >> fbits);
+                    if (keep) s_digits.add(hist, (unsigned)slot);
+                    else atomicAdd(&hist[slot], w);
+                    if (level > 0) {
+                        if (keep) s_runs.add(coarse, run);
+                        else atomicAdd(&coarse[run], w);
+                    } else if (weights) {
+                        atomicAdd(&s_coarse[run], w);
+                    } else {
+                        atomicAdd(&s_coarse_unit[run], 1u);
+                    }
                 }
             }
         }
+    }
+    if (keep) {
+        __syncthreads();
+        s_digits.end(hist);
+        if (level > 0) s_runs.end(coarse);
     }
     if (level == 0) {
         __syncthreads();
