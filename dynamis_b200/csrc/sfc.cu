@@ -484,7 +484,6 @@ __device__ void sel_pick_warp(int s, const SelSplit* __restrict__ st_in, SelSpli
 // would overflow is not begun (the second pass of a KD-tree level: 20 -> 14 us, a million atoms).
 struct SelCand { unsigned long long hi, lo; long long w; int g; int pad; };
 static_assert(sizeof(SelCand) == sizeof(SelSplit), "candidates share the unused split-point slots");
-constexpr int SEL_FINISH_SPLITS = 16;        // the fused path's limit on split points
 constexpr int SEL_CAND_CAP = SEL_MAX_SPLITS - SEL_FINISH_SPLITS;   // records behind the split points of state buffer 0
 constexpr int SEL_FINISH_GROUP_MAX = 128;
 
