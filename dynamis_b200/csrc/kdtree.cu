@@ -156,7 +156,7 @@ __device__ __forceinline__ int kd_axis(const uint32_t* __restrict__ box, int s, 
 // the coordinates, but the leading digit of the selection spreads evenly: it leaves 60 of a million atoms where sign, exponent and
 // five bits of the mantissa left 30 thousand, and the second digit's pass settles the cuts in place of the third's.  A call of a
 // million atoms on 8 ranks: 233 us before, 200 with places.
-constexpr int KD_PLACE_BITS = 14;
+constexpr int KD_PLACE_BITS = 14, KD_PLACE_BITS_MOST = 18;   // for a million atoms, and for more
 __global__ void __launch_bounds__(256)
 kd_keys_kernel(const float* pos, const int32_t* seg_id, int64_t n, const uint32_t* box,
                uint64_t* keys, uint32_t* vals, int place_bits)
@@ -392,9 +392,12 @@ extern "C" int dynb_kdtree_partition(const float* pos_dev, int64_t n_atoms, cons
     for (int l = 0; l < levels; l++) {
         const int S = (int)(first[l + 1] - first[l]), S_next = l + 1 < levels ? (int)(first[l + 2] - first[l + 1]) : 0;
         const KdSeg* level_tree = tree + first[l];
-        // places where the selection ends early; with more cuts all its digits are passed over, and longer keys are one more pass a level
-        // (1 M atoms, 64 ranks: 549 us with places at all levels, 530 so; 256 ranks 990 and 928)
-        const int place_bits = by_selection && S <= SEL_FINISH_SPLITS ? KD_PLACE_BITS : 0;
+        // Places where the selection ends early; with more cuts all its digits are passed over, and longer keys are one more pass a level
+        // (1 M atoms, 64 ranks: 549 us with places at all levels, 530 so; 256 ranks 990 and 928).  No more than 64 atoms a place, up to 18
+        // bits, for a prefix with more than 128 takes one more pass (8 ranks, 2 M atoms: 345 us with 14 bits, 340 so; 4 M 591 and 525; 8 M 1062 and 870).
+        int place_bits = KD_PLACE_BITS;
+        while (place_bits < KD_PLACE_BITS_MOST && (n >> place_bits) > 64) place_bits++;
+        if (!by_selection || S > SEL_FINISH_SPLITS) place_bits = 0;
         if (l == 0 || !by_selection) {
             launch_chained(kd_level_init_kernel, 1, 256, 0, s, S, nullptr, size_cur, start, box, S, nullptr, nullptr);
             launch_chained(kd_bbox_kernel, grid_stride, 256, 0, s, pos_dev, seg_cur, n, S, box);

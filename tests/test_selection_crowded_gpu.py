@@ -30,6 +30,13 @@ def test_kdtree_labels(cuda, name, n, W):
     assert torch.equal(D.kdtree_partition_labels(pos, None, W), D.kdtree_partition_labels(pos, None, W, sorted_cuts=True))
 
 
+@pytest.mark.parametrize("name", ["uniform", "two"])
+@pytest.mark.parametrize("n, W", [((65 << 14) - 1, 8), (65 << 14, 8), (2_200_003, 16), (4_300_007, 3)])
+def test_kdtree_labels_with_finer_places(cuda, name, n, W):
+    pos = system(name, n, cuda)
+    assert torch.equal(D.kdtree_partition_labels(pos, None, W), D.kdtree_partition_labels(pos, None, W, sorted_cuts=True))
+
+
 @pytest.mark.parametrize("name", ["uniform", "outlier", "two", "many", "equal"])
 @pytest.mark.parametrize("n, W", [(120_011, 2), (120_011, 17), (120_011, 18), (120_011, 769), (120_011, 770), (300_007, 8)])
 def test_curve_labels(cuda, name, n, W):
