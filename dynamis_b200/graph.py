@@ -89,7 +89,7 @@ def _empty_result(pos, n_target):
 def take_host_words(count: int) -> torch.Tensor:
     """Pinned int64 words, at least ``count`` of them, for counts that a kernel writes or a copy brings.  They are this call's
     alone until it gives them back, behind its wait: the wait lets other threads run, and these may use the same stream.
-    A call that raises in between drops them."""
+    PyTorch's cache of pinned memory, to which dropped words go, knows nothing of the kernels that write them: see HostWords."""
     if count <= HOST_WORDS:
         try:
             return _HOST_WORDS.pop()
@@ -102,6 +102,30 @@ def take_host_words(count: int) -> torch.Tensor:
 def give_host_words(words: torch.Tensor) -> None:
     if words.numel() == HOST_WORDS and len(_HOST_WORDS) < HOST_WORDS_KEPT:
         _HOST_WORDS.append(words)
+
+
+class HostWords:
+    """``with HostWords(count, device) as words``: pinned words around the launches that write them and the wait for these.  Where the
+    block raises in between, the current stream is waited for before the words, and what the block alone held, can have another owner."""
+
+    __slots__ = ("count", "dev", "words")
+    _LOST: list = []   # words that could not be waited for
+
+    def __init__(self, count: int, dev: torch.device):
+        self.count, self.dev = count, dev
+
+    def __enter__(self) -> torch.Tensor:
+        self.words = take_host_words(self.count)
+        return self.words
+
+    def __exit__(self, kind, *_) -> None:
+        if kind is not None:
+            try:
+                torch.cuda.current_stream(self.dev).synchronize()
+            except RuntimeError:   # the block's own exception goes on
+                self._LOST.append(self.words)
+                return
+        give_host_words(self.words)
 
 
 def _plan_bytes(st: dict, n_atoms: int, n_targets: int, src_cap: int, cell_cap: int, dtype_code: int) -> int:
@@ -224,8 +248,8 @@ class BinnedAtoms:
         self.pos = pos.contiguous()
         self.dtype_code = _lib.DYNB_F64 if pos.dtype == torch.float64 else _lib.DYNB_F32
         self.st = _dev_state(pos.device)
-        # a header of its own: a graph call on the same stream, before done(), writes the stream's.  Pinned words of this object until
-        # it goes; they are not given back, for the launch that writes them may still be queued then.
+        # A header of its own: a graph call on the same stream, before done(), writes the stream's.  It goes with this object, which
+        # must not go before the stream was waited for.
         self.hdr_t = torch.empty((64,), dtype=torch.uint8, device="cpu", pin_memory=True)
         self.hdr = _lib.RgHeader.from_address(self.hdr_t.data_ptr())
         self.key, geo = _geometry(self.st, cell, pbc, radius, pos.size(0), self.dtype_code)

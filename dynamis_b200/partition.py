@@ -22,7 +22,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .graph import BinnedAtoms, give_host_words, radius_graph_pbc, radius_graph_pbc_ex, take_host_words
+from .graph import BinnedAtoms, HostWords, radius_graph_pbc, radius_graph_pbc_ex
 from .state import DistEnvironment, MolecularInfo, PartitionMessagePassingInfo, SimulationConfig
 
 PARTITION_MAX_NUM_NEIGHBORS = 1000
@@ -140,17 +140,22 @@ def select_eq(values: torch.Tensor, value: int, gather_src: Optional[torch.Tenso
         out = torch.empty((n,), dtype=torch.int64, device=dev)
         # a count that is waited for is written to the host by the kernel (up to 16.7 M values: its tiles then need no prefix sum)
         waited = count is None and 0 < n <= SELECT_HOST_COUNT
-        cnt = take_host_words(1) if waited else torch.empty((1,), dtype=torch.int64, device=dev)
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_select_workspace_bytes(n, ctypes.byref(nbytes)), "select_workspace_bytes")
         ws = scratch(dev, "select", nbytes.value)
-        _lib.check(L.dynb_select_eq_i64(values.data_ptr(), n, int(value), gather_src.data_ptr() if gather_src is not None else None,
-                                        out.data_ptr(), cnt.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev)), "select_eq")
+
+        def launch(cnt):
+            _lib.check(L.dynb_select_eq_i64(values.data_ptr(), n, int(value), gather_src.data_ptr() if gather_src is not None else None,
+                                            out.data_ptr(), cnt.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev)), "select_eq")
+
         if waited:
-            torch.cuda.current_stream(dev).synchronize()
-            k = int(cnt[0])
-            give_host_words(cnt)
+            with HostWords(1, dev) as cnt:
+                launch(cnt)
+                torch.cuda.current_stream(dev).synchronize()
+                k = int(cnt[0])
         else:
+            cnt = torch.empty((1,), dtype=torch.int64, device=dev)
+            launch(cnt)
             k = int(cnt.item()) if count is None else count
     return out[:k]
 
@@ -203,21 +208,20 @@ class AbstractPartitioner:
             ws = scratch(dev, "halo_lists", nbytes.value)
             # send offsets, recv offsets, number of own atoms and, behind them, the error word of the marking
             offs = torch.empty((2 * (W + 1) + 2,), dtype=torch.int64, device=dev)
-            offs_h = take_host_words(2 * (W + 1) + 2)
             # everything up to the list sizes is queued before the one wait; the header's status is looked at behind it
             bins = BinnedAtoms(pos32, cell, pbc, ghost_cutoff) if N > 0 else None
-            while True:
-                if bins is not None:
-                    bins.launch()
-                    _lib.check(L.dynb_rg_halo_mark_rank(bins.ws.data_ptr(), bins.dtype_code, pid.data_ptr(), N, W, R, needed.data_ptr(),
-                                                        has_foreign.data_ptr(), offs.data_ptr() + 8 * (2 * W + 3), _stream(dev)), "rg_halo_mark")
-                _lib.check(L.dynb_halo_lists_plan_words(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
-                                                        ws.numel(), offs_h.data_ptr(), 2 * (W + 1) + 2, _stream(dev)), "halo_lists_plan")
-                torch.cuda.current_stream(dev).synchronize()
-                if bins is None or bins.done():
-                    break
-            sizes = offs_h[:2 * (W + 1) + 2].tolist()
-            give_host_words(offs_h)
+            with HostWords(2 * (W + 1) + 2, dev) as offs_h:   # and the header of the bins
+                while True:
+                    if bins is not None:
+                        bins.launch()
+                        _lib.check(L.dynb_rg_halo_mark_rank(bins.ws.data_ptr(), bins.dtype_code, pid.data_ptr(), N, W, R, needed.data_ptr(),
+                                                            has_foreign.data_ptr(), offs.data_ptr() + 8 * (2 * W + 3), _stream(dev)), "rg_halo_mark")
+                    _lib.check(L.dynb_halo_lists_plan_words(needed.data_ptr(), None, pid.data_ptr(), N, R, W, offs.data_ptr(), ws.data_ptr(),
+                                                            ws.numel(), offs_h.data_ptr(), 2 * (W + 1) + 2, _stream(dev)), "halo_lists_plan")
+                    torch.cuda.current_stream(dev).synchronize()
+                    if bins is None or bins.done():
+                        break
+                sizes = offs_h[:2 * (W + 1) + 2].tolist()
             if bins is not None and sizes[2 * W + 3] & 0xFFFFFFFF != 0:
                 raise RuntimeError(f"build_halo_maps: partition_id has a label that is no rank's (world_size is {W})")
             total_send, total_recv, n_local = sizes[W], sizes[2 * W + 1], sizes[2 * W + 2]
