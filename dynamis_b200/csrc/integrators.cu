@@ -67,7 +67,8 @@ __device__ __forceinline__ void drift_atom(const float (&x)[3], const float (&v)
 
 // A atoms a thread: with four of them an array's twelve numbers are three loads of 16 bytes (arrays that start on such a boundary; the
 // up to three atoms behind the last four go one by one), else one atom and loads that lie 12 bytes apart.  Bound by HBM
-// and, where the arrays stay in it, L2.  A Langevin step of 1 M atoms, both halves, drift word with the first: 31 us before, 25 now.
+// and, where the arrays stay in it, L2.  A Langevin step of 1 M atoms, both halves, drift word with the first, arrays out of L2: 42.2 us as
+// two launches that wait for one another, 28.1 as a chain.
 template <int KIND, bool DRIFT, int A>
 __global__ void __launch_bounds__(256)
 integrate_kernel(float* pos, float* vel, const float* frc, const float* mass, const float* noise, int64_t n, float dt, float gamma,
@@ -170,6 +171,8 @@ integrate_kernel(float* pos, float* vel, const float* frc, const float* mass, co
     }
 }
 
+constexpr int64_t INT_L2_BYTES = 126ll << 20;
+
 template <int KIND>
 static int launch_integrator(float* pos, float* vel, const float* frc, const float* mass, const float* noise, int64_t n,
                              float dt, float gamma, float kT, const DriftArgs* da, cudaStream_t s)
@@ -177,8 +180,13 @@ static int launch_integrator(float* pos, float* vel, const float* frc, const flo
     uintptr_t at = reinterpret_cast<uintptr_t>(pos) | reinterpret_cast<uintptr_t>(vel) | reinterpret_cast<uintptr_t>(frc) | reinterpret_cast<uintptr_t>(mass) |
                    reinterpret_cast<uintptr_t>(noise);
     if (da != nullptr) at |= reinterpret_cast<uintptr_t>(da->ref) | reinterpret_cast<uintptr_t>(da->prev_vel);
-    // four atoms a thread once these fill the chip: below, more threads with fewer loads each
-    const bool wide = at % 16 == 0 && n >= 4 * 256 * (int64_t)sm_count_cached();
+    // Four atoms a thread where the arrays outgrow L2, more threads with fewer loads each below.  One atom a thread and four, us a step with its arrays
+    // in L2 / out of it: Langevin, both halves, drift word with the first (76 and 40 B an atom) 300 k atoms 14.8, 16.0 / 12.6, 12.5, 700 k
+    // 20.3, 24.8 / 20.9, 22.5, 1 M 25.1, 30.9 / 28.1, 30.0, 2 M 56.2, 54.6 / 56.0, 53.7, 4 M 115.8, 111.2 / 113.2, 109.2; Euler (40 B)
+    // 1 M 11.7, 14.1 / 12.4, 12.3, 2 M 17.7, 22.2 / 24.1, 21.9, 4 M 51.2, 47.9 / 47.8, 44.7.
+    constexpr bool MOVES = KIND == INT_EULER || KIND == INT_VERLET1 || KIND == INT_LANGEVIN1, NOISE = KIND == INT_LANGEVIN1 || KIND == INT_LANGEVIN2;
+    const int arrays = 2 + (MOVES ? 1 : 0) + (NOISE ? 1 : 0) + (da != nullptr ? 2 : 0);
+    const bool wide = at % 16 == 0 && n * (12 * arrays + 4) >= INT_L2_BYTES;
     const int64_t threads = wide ? (n + 3) / 4 : n;
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((threads + 255) / 256, (int64_t)sm_count_cached() * 8));
     auto run = [&](auto drift, auto atoms) {
