@@ -89,7 +89,7 @@ def _empty_result(pos, n_target):
 def take_host_words(count: int) -> torch.Tensor:
     """Pinned int64 words, at least ``count`` of them, for counts that a kernel writes or a copy brings.  They are this call's
     alone until it gives them back, behind its wait: the wait lets other threads run, and these may use the same stream.
-    PyTorch's cache of pinned memory, to which dropped words go, knows nothing of the kernels that write them: see HostWords."""
+    PyTorch's cache of pinned memory, to which dropped words go, knows nothing of the kernels that write them: see lose_host_words."""
     if count <= HOST_WORDS:
         try:
             return _HOST_WORDS.pop()
@@ -104,28 +104,18 @@ def give_host_words(words: torch.Tensor) -> None:
         _HOST_WORDS.append(words)
 
 
-class HostWords:
-    """``with HostWords(count, device) as words``: pinned words around the launches that write them and the wait for these.  Where the
-    block raises in between, the current stream is waited for before the words, and what the block alone held, can have another owner."""
+_LOST_WORDS: list = []   # words that could not be waited for
 
-    __slots__ = ("count", "dev", "words")
-    _LOST: list = []   # words that could not be waited for
 
-    def __init__(self, count: int, dev: torch.device):
-        self.count, self.dev = count, dev
-
-    def __enter__(self) -> torch.Tensor:
-        self.words = take_host_words(self.count)
-        return self.words
-
-    def __exit__(self, kind, *_) -> None:
-        if kind is not None:
-            try:
-                torch.cuda.current_stream(self.dev).synchronize()
-            except RuntimeError:   # the block's own exception goes on
-                self._LOST.append(self.words)
-                return
-        give_host_words(self.words)
+def lose_host_words(words: torch.Tensor, dev: torch.device) -> None:
+    """For a call that raises between a launch that writes its words and the wait for it: the current stream is waited for before
+    the words, and what the call alone held, can have another owner."""
+    try:
+        torch.cuda.current_stream(dev).synchronize()
+    except RuntimeError:   # the call's own exception goes on
+        _LOST_WORDS.append(words)
+    else:
+        give_host_words(words)
 
 
 def _plan_bytes(st: dict, n_atoms: int, n_targets: int, src_cap: int, cell_cap: int, dtype_code: int) -> int:

@@ -12,7 +12,7 @@ import ctypes
 import torch
 
 from . import _lib
-from .graph import HostWords, host_cell
+from .graph import give_host_words, host_cell, lose_host_words, take_host_words
 from .partition import _stream, scratch
 
 
@@ -54,12 +54,17 @@ def filter_edges_to_radius(edges: torch.Tensor, cell_shifts: torch.Tensor, pos: 
         nbytes = ctypes.c_int64()
         _lib.check(L.dynb_filter_edges_workspace_bytes(E, ctypes.byref(nbytes)), "filter_edges_workspace_bytes")
         ws = scratch(dev, "filter", nbytes.value)
-        with HostWords(1, dev) as cnt:   # written by the plan's last kernel
+        cnt = take_host_words(1)   # written by the plan's last kernel
+        try:
             _lib.check(L.dynb_filter_edges_plan(edges.data_ptr(), shifts_f.data_ptr(), pos.data_ptr(), cell_h,
                                                 float(radius), E, cnt.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev)),
                        "filter_edges_plan")
             torch.cuda.current_stream(dev).synchronize()
-            E_out = int(cnt[0])
+        except BaseException:
+            lose_host_words(cnt, dev)
+            raise
+        E_out = int(cnt[0])
+        give_host_words(cnt)
         edges_out = torch.empty((2, E_out), dtype=torch.int64, device=dev)
         shifts_out = torch.empty((E_out, 3), dtype=cell_shifts.dtype, device=dev)
         _lib.check(L.dynb_filter_edges_fill(edges.data_ptr(), cell_shifts.data_ptr(), 3 * cell_shifts.element_size(), E, E_out,
@@ -116,11 +121,16 @@ def extract_halo_info(edges: torch.Tensor, pid_outer: torch.Tensor, my_outer_ato
         _lib.check(L.dynb_halo_lists_workspace_bytes(N, W, ctypes.byref(nbytes)), "halo_lists_workspace_bytes")
         ws = scratch(dev, "halo_lists", nbytes.value)
         interior = torch.empty((n_local,), dtype=torch.bool, device=dev)
-        with HostWords(n_words, dev) as offs_h:
+        offs_h = take_host_words(n_words)
+        try:
             _lib.check(L.dynb_halo_lists_plan_words(send_mask.data_ptr(), recv_mask.data_ptr(), None, N, R, W, offs.data_ptr(), ws.data_ptr(),
                                                     ws.numel(), offs_h.data_ptr(), n_words, _stream(dev)), "halo_lists_plan")
             torch.cuda.current_stream(dev).synchronize()
-            sizes = offs_h[:n_words].tolist()
+        except BaseException:
+            lose_host_words(offs_h, dev)
+            raise
+        sizes = offs_h[:n_words].tolist()
+        give_host_words(offs_h)
         if sizes[-1] & 0xFFFFFFFF != 0:
             raise RuntimeError("extract_halo_info: an edge endpoint, partition id or my_outer_atoms entry is out of range")
         total_send, total_recv = sizes[W], sizes[2 * W + 1]

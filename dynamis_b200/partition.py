@@ -22,7 +22,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .graph import BinnedAtoms, HostWords, radius_graph_pbc, radius_graph_pbc_ex
+from .graph import BinnedAtoms, give_host_words, lose_host_words, radius_graph_pbc, radius_graph_pbc_ex, take_host_words
 from .state import DistEnvironment, MolecularInfo, PartitionMessagePassingInfo, SimulationConfig
 
 PARTITION_MAX_NUM_NEIGHBORS = 1000
@@ -144,18 +144,20 @@ def select_eq(values: torch.Tensor, value: int, gather_src: Optional[torch.Tenso
         _lib.check(L.dynb_select_workspace_bytes(n, ctypes.byref(nbytes)), "select_workspace_bytes")
         ws = scratch(dev, "select", nbytes.value)
 
-        def launch(cnt):
+        cnt = take_host_words(1) if waited else torch.empty((1,), dtype=torch.int64, device=dev)
+        try:
             _lib.check(L.dynb_select_eq_i64(values.data_ptr(), n, int(value), gather_src.data_ptr() if gather_src is not None else None,
                                             out.data_ptr(), cnt.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev)), "select_eq")
-
-        if waited:
-            with HostWords(1, dev) as cnt:
-                launch(cnt)
+            if waited:
                 torch.cuda.current_stream(dev).synchronize()
-                k = int(cnt[0])
+        except BaseException:
+            if waited:
+                lose_host_words(cnt, dev)
+            raise
+        if waited:
+            k = int(cnt[0])
+            give_host_words(cnt)
         else:
-            cnt = torch.empty((1,), dtype=torch.int64, device=dev)
-            launch(cnt)
             k = int(cnt.item()) if count is None else count
     return out[:k]
 
@@ -210,7 +212,8 @@ class AbstractPartitioner:
             offs = torch.empty((2 * (W + 1) + 2,), dtype=torch.int64, device=dev)
             # everything up to the list sizes is queued before the one wait; the header's status is looked at behind it
             bins = BinnedAtoms(pos32, cell, pbc, ghost_cutoff) if N > 0 else None
-            with HostWords(2 * (W + 1) + 2, dev) as offs_h:   # and the header of the bins
+            offs_h = take_host_words(2 * (W + 1) + 2)
+            try:
                 while True:
                     if bins is not None:
                         bins.launch()
@@ -221,7 +224,11 @@ class AbstractPartitioner:
                     torch.cuda.current_stream(dev).synchronize()
                     if bins is None or bins.done():
                         break
-                sizes = offs_h[:2 * (W + 1) + 2].tolist()
+            except BaseException:   # the header of the bins waits as well
+                lose_host_words(offs_h, dev)
+                raise
+            sizes = offs_h[:2 * (W + 1) + 2].tolist()
+            give_host_words(offs_h)
             if bins is not None and sizes[2 * W + 3] & 0xFFFFFFFF != 0:
                 raise RuntimeError(f"build_halo_maps: partition_id has a label that is no rank's (world_size is {W})")
             total_send, total_recv, n_local = sizes[W], sizes[2 * W + 1], sizes[2 * W + 2]

@@ -7,7 +7,7 @@ from dynamis_b200 import graph as G
 
 
 class Stream:
-    def __init__(self, log, fails=False):
+    def __init__(self, log, fails):
         self.log, self.fails = log, fails
 
     def synchronize(self):
@@ -16,33 +16,12 @@ class Stream:
             raise RuntimeError("CUDA error")
 
 
-@pytest.fixture
-def log(monkeypatch):
-    log = []
-    words = torch.zeros(G.HOST_WORDS, dtype=torch.int64)
-    monkeypatch.setattr(G, "take_host_words", lambda count: words)
+@pytest.mark.parametrize("fails", [False, True])
+def test_waited_for_and_given_back_or_kept(monkeypatch, fails):
+    log, words = [], torch.zeros(G.HOST_WORDS, dtype=torch.int64)
     monkeypatch.setattr(G, "give_host_words", lambda w: log.append("given" if w is words else "others given"))
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream(log))
-    monkeypatch.setattr(G.HostWords, "_LOST", [])
-    return log
-
-
-def test_given_back_behind_the_callers_own_wait(log):
-    with G.HostWords(3, torch.device("cuda", 0)) as words:
-        assert words.numel() >= 3
-    assert log == ["given"]
-
-
-def test_a_call_that_raises_waits_first(log):
-    with pytest.raises(RuntimeError, match="behind the launch"):
-        with G.HostWords(3, torch.device("cuda", 0)):
-            raise RuntimeError("behind the launch")
-    assert log == ["wait", "given"]
-
-
-def test_words_that_cannot_be_waited_for_are_kept(log, monkeypatch):
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream(log, fails=True))
-    with pytest.raises(ValueError, match="behind the launch"):
-        with G.HostWords(3, torch.device("cuda", 0)):
-            raise ValueError("behind the launch")
-    assert log == ["wait"] and len(G.HostWords._LOST) == 1
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream(log, fails))
+    monkeypatch.setattr(G, "_LOST_WORDS", [])
+    G.lose_host_words(words, torch.device("cuda", 0))
+    assert log == (["wait"] if fails else ["wait", "given"])
+    assert [w is words for w in G._LOST_WORDS] == ([True] if fails else [])
