@@ -594,7 +594,7 @@ struct SelKept {
             if (count[k]) atomicAdd(&table[which[k]], (unsigned long long)count[k]);
     }
 };
-constexpr unsigned SEL_KEEP_FROM = 32768;   // atoms that a level behind the first counts: fewer are added to the table as they come
+constexpr unsigned SEL_KEEP_FROM = 32768;   // atoms that a level counts: fewer are added to the table as they come (30 k even ones on 4 ranks: 80 us either way)
 
 // Table of one level: per group 2^dbits digit counters ("fine"), followed by per group 256 coarse
 // counters, one per run of 2^fbits consecutive digits (fbits = min(width, 8)), so that a split point is
@@ -625,7 +625,7 @@ sel_hist_kernel(const uint64_t* keys, const int64_t* weights, int64_t n, int idx
     static_assert(sizeof(SelKept<512>) <= ROOM * sizeof(u128) && sizeof(SelKept<256>) <= ROOM * sizeof(unsigned long long), "room for the counters");
     SelKept<512>& s_digits = *reinterpret_cast<SelKept<512>*>(glist + SEL_MAX_SPLITS - ROOM);
     SelKept<256>& s_runs = *reinterpret_cast<SelKept<256>*>(glist64 + SEL_MAX_SPLITS - ROOM);
-    const bool may_keep = weights == nullptr && nsplit <= SEL_MAX_SPLITS - ROOM;
+    const bool may_keep = weights == nullptr && n > SEL_KEEP_FROM && nsplit <= SEL_MAX_SPLITS - ROOM;
     __shared__ unsigned s_atoms;   // that this level counts
     __shared__ bool s_last;
     bool listing = false;   // this level lists its atoms
@@ -875,7 +875,10 @@ int sel_select_splits(const uint64_t* keys, int key_bits, const int64_t* weights
     unsigned int* cand_counts = counters + 16;
     unsigned int* finished = counters + 48;
     if (levels > 16) return fail_arg("too many digit levels");
-    const int hgrid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count_cached() * 4);  // one wave
+    // One wave at most, and four keys a thread (read together) while every SM has a block: a block's counters are a microsecond of its own.  KD-tree
+    // on 8 ranks, a thread a key / so: 60 k atoms 133 / 118 us, 100 k 132 / 123, 300 k 156 / 152.
+    const int64_t sms = sm_count_cached();
+    const int hgrid = (int)std::min<int64_t>(std::max<int64_t>((n + 1023) / 1024, std::min<int64_t>((n + 255) / 256, sms)), sms * 4);
     for (int l = 0; l < levels; l++) {
         const int width = std::min(dbits, B - l * dbits);
         const int shift = B - l * dbits - width;
