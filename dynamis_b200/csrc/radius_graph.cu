@@ -1105,7 +1105,8 @@ rg_group_list_kernel(const PairParams<T>* params_dev, uint32_t* glist)
 // unrolled over the whole list.  A warp takes the next group when it is done with one.
 // Two tests a pair: d <= r^2, and d above the self-distance limit.  The second is made for the two blocks of 64 candidates only that
 // hold the records of the targets' own cell rows, for records elsewhere are further away (targets next to the faces of these rows are
-// tested again in full); for these two blocks to be the same registers in every group the blocks are loaded in turned order.
+// tested again in full; lists whose own records touch three blocks, and lists of several chunks, take both tests everywhere); for these
+// two blocks to be the same registers in every group the blocks are loaded in turned order.
 // The bits of a target go to shared memory and leave it, with the degrees, for 16 targets together.
 // Bound by the latency of its loads, its issue slots (60 % busy) and the FMA pipe (40 %): 156 instructions a target of the liquid, 56 of
 // them tests; 207 without the items above.  Before and after: 266 -> 207 us (liquid, 1 M atoms, 5 A), 309 -> 259 (a rank's 1 M of the
