@@ -1476,9 +1476,7 @@ rg_count_kernel(const PairParams<T> p)
                 // one for 5, 207 without; in double 287 and 266; 245 and 355 with the copy for 8 inlined twice).  The one for 1, that gas: 876 ->
                 // 826; in double it costs the others (jittered silicon of 500 k atoms 268 -> 278 us).
                 const int blocks = (clen + 63) >> 6;
-                const bool both = everywhere && blocks > 2;
-                // (the hint puts the copies with one test first: liquid of 4 M atoms 1190 -> 1187 us; in double jittered silicon 265 -> 273)
-                switch ((sizeof(T) == 4 ? __builtin_expect(both, false) : both) ? (blocks > 4 ? 10 : 9) : blocks) {
+                switch (everywhere && blocks > 2 ? (blocks > 4 ? 10 : 9) : blocks) {
                 case 1: if constexpr (ONE_BLOCK) { run(std::integral_constant<int, 1>(), std::true_type()); break; }
                 case 2: run(std::integral_constant<int, 2>(), std::true_type()); break;
                 case 3:
